@@ -21,7 +21,7 @@ import torch
 import torch.distributed as dist
 
 from .config import COMPUTE_BATCH_SIZES, Config, topk_idx_t
-from .engine import EPEngine, LayerHandle
+from .engine import EPEngine, LayerHandle, LocalHandle
 from .low_latency import LowLatencyMixin
 from .parallel.world import EPWorld
 from .utils.events import EventHandle, EventOverlap
@@ -42,6 +42,14 @@ def _rows_from_bf16(rows: torch.Tensor, dtype: torch.dtype, cols: int) -> torch.
     raw = rows.contiguous().view(torch.uint8).reshape(rows.shape[0], rows.shape[1] * rows.element_size())
     nbytes = cols * torch.empty((), dtype=dtype).element_size()
     return raw[:, :nbytes].contiguous().view(dtype)
+
+
+def _leaves(v):
+    if isinstance(v, (tuple, list)):
+        for x in v:
+            yield from _leaves(x)
+    else:
+        yield v
 
 
 class _TeraMoEFunction(torch.autograd.Function):
@@ -138,6 +146,8 @@ class Buffer(LowLatencyMixin):
         self._world = (EPWorld.from_group(group, self.device, use_fabric=self.use_fabric) if group is not None
                        else EPWorld.single(self.device, use_fabric=self.use_fabric))
         self._engine = EPEngine(self._world)
+        # one rank on a GPU: the un-fused and low-latency calls have nothing to send and run as kernels between the caller's tensors
+        self._local = self._world.ext.LocalExchange() if self.device.type == "cuda" and self.group_size == 1 else None
         self._comm_stream = torch.cuda.Stream(self.device, priority=-1) if self.device.type == "cuda" else None
         if self.device.type == "cuda" and num_nvl_bytes > 0:
             self._world.ensure_data(num_nvl_bytes)
@@ -274,18 +284,30 @@ class Buffer(LowLatencyMixin):
         cur = self._enter(previous_event, allocate_on_comm_stream)
         with torch.cuda.stream(self._comm_stream):
             res = fn()
-        flat = res if isinstance(res, (tuple, list)) else (res,)
-        return res, self._leave(cur, async_finish, flat)
+        return res, self._leave(cur, async_finish, list(_leaves(res)))
+
+    def _run_local(self, fn: Callable, previous_event, async_finish):
+        """A call of the one-rank paths.  It touches no arena, so it needs no order against other calls on this buffer: unless
+        the caller asks for the asynchronous protocol, it goes straight to the current stream."""
+        if self._destroyed:
+            raise RuntimeError("Buffer was destroyed")
+        self._world.poll_status()
+        if async_finish or previous_event is not None:
+            return self._on_comm_stream(fn, previous_event, async_finish, False)
+        return fn(), EventOverlap(None)
 
     # ------------------------------------------------------------------ layout / dispatch / combine
     def get_dispatch_layout(self, topk_idx: torch.Tensor, num_experts: int, previous_event: Optional[EventOverlap] = None,
                             async_finish: bool = False, allocate_on_comm_stream: bool = False):
         """-> (num_tokens_per_rank [ranks] i32, None, num_tokens_per_expert [E] i32, is_token_in_rank [T,ranks] bool, event)."""
         N = self.group_size
+        if self._local is not None and topk_idx.is_cuda:
+            (per_rank, per_expert, in_rank), ev = self._run_local(lambda: self._world.ext.local_counts(topk_idx, num_experts), previous_event,
+                                                                  async_finish)
+            return per_rank, None, per_expert, in_rank, ev
 
         def run():
             T, K = topk_idx.shape
-            El = num_experts // N
             if topk_idx.is_cuda:
                 # two kernels, nothing else: per-chunk histograms (which also write is_token_in_rank), then their column sums
                 ext = self._world.ext
@@ -323,6 +345,9 @@ class Buffer(LowLatencyMixin):
         no host synchronisation happens.  `num_worst_tokens > 0` gives fixed-shape outputs (padded rows are
         zero, expert id -1, empty per-expert list) without any host wait: the tables are sized for that many rows
         and the layout sizes stay on the device (`_dispatch_fixed_shape`)."""
+        if self._local is not None and (x[0] if isinstance(x, tuple) else x).is_cuda:
+            return self._dispatch_local(x, handle, num_tokens_per_expert, topk_idx, topk_weights, expert_alignment, num_worst_tokens,
+                                        previous_event, async_finish, num_experts)
         if isinstance(x, tuple):
             # FP8 payload (x_e4m3 [T,H], scales [T,H/128] fp32), teramoe/buffer.py:344-346: both parts travel as raw
             # bytes through the same kernels (the second with the cached handle) and come back as a tuple
@@ -380,6 +405,36 @@ class Buffer(LowLatencyMixin):
         res, ev = self._on_comm_stream(run, previous_event, async_finish, allocate_on_comm_stream)
         return (*res, ev)
 
+    def _dispatch_local(self, x, handle, num_tokens_per_expert, topk_idx, topk_weights, expert_alignment, worst, previous_event, async_finish,
+                        num_experts):
+        """`deepep_dispatch` on one rank (csrc/local.cu): the rows of the tokens that go anywhere, straight from the caller's
+        tensors into the results.  Both parts of an FP8 payload move in the same launch."""
+        parts = list(x) if isinstance(x, tuple) else [x]
+        if not isinstance(x, tuple) and x.dtype != torch.bfloat16:
+            raise RuntimeError("x must be a bf16 CUDA tensor (or a tuple of payload and scales)")
+        if handle is not None:
+            rows = handle.num_rows()
+            recv, ev = self._run_local(lambda: self._world.ext.local_scatter(parts, handle.send_row, rows), previous_event, async_finish)
+            return (tuple(recv) if isinstance(x, tuple) else recv[0]), None, None, None, handle, ev
+        if topk_idx is None or topk_weights is None:
+            raise ValueError("topk_idx and topk_weights are required without a cached handle")
+        E = num_experts if num_experts is not None else (int(num_tokens_per_expert.numel()) if num_tokens_per_expert is not None else None)
+        if E is None:
+            raise ValueError("pass num_tokens_per_expert (from get_dispatch_layout) or num_experts")
+        if worst > 0 and parts[0].shape[0] > worst:
+            raise ValueError(f"{parts[0].shape[0]} tokens exceed num_worst_tokens={worst}")
+        topk_idx = topk_idx.contiguous()
+        (recv, recv_idx, recv_w, counts, rows, send_row, totals), ev = self._run_local(
+            lambda: self._local.dispatch(parts, topk_idx, topk_weights, E, worst, expert_alignment), previous_event, async_finish)
+        h = LocalHandle(topk_idx.shape[0], topk_idx.shape[1], E, topk_idx, send_row, totals, rows)
+        return (tuple(recv) if isinstance(x, tuple) else recv[0]), recv_idx, recv_w, counts, h, ev
+
+    def _combine_local(self, x, handle, topk_weights):
+        rows = handle.num_rows()
+        if x.shape[0] < rows:
+            raise ValueError(f"expected {rows} rows (one per received token), got {x.shape[0]}")
+        return self._world.ext.local_combine(x, handle.send_row, handle.topk_idx, handle.E, topk_weights)
+
     def _dispatch_fixed_shape(self, x, topk_idx, topk_weights, E, worst):
         """Dispatch with `num_worst_tokens` rows of output and NO host wait (csrc/kernels/intranode.cu:521-531 in the
         reference): the receive tables are sized for `worst` rows, the layout sizes stay on the device, rows past the
@@ -409,18 +464,24 @@ class Buffer(LowLatencyMixin):
                        allocate_on_comm_stream: bool = False):
         """Un-fused combine: un-weighted sum over ranks of the rows given for each token (+ up to two
         bias tensors).  -> (combined_x [T,H], combined_topk_weights [T,K] or None, event)."""
-        h = handle
+        local = isinstance(handle, LocalHandle)
 
         def run():
-            out, cw = self._drive(self._engine.combine_rows_gen(h, x, topk_weights))
-            self._release()
+            if local:
+                out, cw = self._combine_local(x, handle, topk_weights)
+            else:
+                out, cw = self._drive(self._engine.combine_rows_gen(handle, x, topk_weights))
+                self._release()
             if bias is not None:
                 for b in (bias if isinstance(bias, (tuple, list)) else (bias,)):
                     if b is not None:
                         out = (out.float() + b.float()).to(out.dtype)
             return out, cw
 
-        res, ev = self._on_comm_stream(run, previous_event, async_finish, allocate_on_comm_stream)
+        if local:
+            res, ev = self._run_local(run, previous_event, async_finish)
+        else:
+            res, ev = self._on_comm_stream(run, previous_event, async_finish, allocate_on_comm_stream)
         return (*res, ev)
 
     # reference aliases (teramoe/buffer.py:453-454)

@@ -169,7 +169,8 @@ void gemm_wgrad(torch::Tensor a, torch::Tensor b, torch::Tensor dw, torch::Tenso
 
 }  // namespace
 
-void register_more(pybind11::module_& m);  // routing / comm / runtime bindings (bindings_more.cpp)
+void register_more(pybind11::module_& m);   // routing / comm / runtime bindings (bindings_more.cpp)
+void register_local(pybind11::module_& m);  // one-rank paths (bindings_local.cpp)
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.doc() = "teramoe_b200 native kernels (sm_100a)";
@@ -182,4 +183,5 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("gemm_has_gather4", &tmoe::gemm_has_gather4);
     m.def("launch_count", [] { return tmoe::launch_counter().load(); });
     register_more(m);
+    register_local(m);
 }

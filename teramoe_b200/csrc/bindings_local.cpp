@@ -1,0 +1,253 @@
+// Bindings of the one-rank paths.  They allocate their results and launch in one call, so that a call costs the host a few
+// allocations and launches instead of a Python pipeline.
+#include <ATen/cuda/CUDAContext.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <pybind11/stl.h>
+#include <torch/extension.h>
+
+#include <mutex>
+
+#include "launch_count.h"
+#include "local.h"
+#include "lowlat.h"
+
+namespace {
+
+#define TM_CHECK_CUDA(call)                                                                          \
+    do {                                                                                             \
+        tmoe::count_launch();                                                                        \
+        cudaError_t _e = (call);                                                                     \
+        TORCH_CHECK(_e == cudaSuccess, "teramoe_b200: ", #call, " failed: ", cudaGetErrorString(_e)); \
+    } while (0)
+
+cudaStream_t cur_stream() { return at::cuda::getCurrentCUDAStream().stream(); }
+
+struct TopK {
+    const void* ptr;
+    int is64, T, K;
+};
+TopK topk_of(const torch::Tensor& idx) {
+    TORCH_CHECK(idx.is_cuda() && idx.is_contiguous() && idx.dim() == 2, "topk_idx must be a contiguous [T,K] CUDA tensor");
+    TORCH_CHECK(idx.scalar_type() == torch::kInt64 || idx.scalar_type() == torch::kInt32, "topk_idx must be int64 or int32");
+    TORCH_CHECK(idx.size(1) <= 32, "top-k must be <= 32");
+    return TopK{idx.data_ptr(), idx.scalar_type() == torch::kInt64 ? 1 : 0, (int)idx.size(0), (int)idx.size(1)};
+}
+torch::Tensor weights_of(const torch::Tensor& w) {
+    auto f = w.scalar_type() == torch::kFloat32 ? w : w.to(torch::kFloat32);
+    return f.contiguous();
+}
+torch::TensorOptions on(const torch::Tensor& like, torch::ScalarType t) { return torch::TensorOptions().dtype(t).device(like.device()); }
+
+// ------------------------------------------------------------------------------------------------ low latency
+tmoe::LowLatLayout local_layout(int64_t E, int64_t M, int64_t H, int wire, bool logfmt) {
+    tmoe::LowLatLayout l{};
+    l.num_ranks = 1; l.num_experts = (int)E; l.max_tokens = (int)M; l.hidden = (int)H;
+    l.use_fp8 = wire > 0; l.round_scale = wire > 1; l.use_ue8m0 = wire > 2; l.use_logfmt = logfmt ? 1 : 0;
+    l.d_msg_bytes = 16; l.c_row_bytes = 16;
+    return l;
+}
+
+// wire: 0 bf16, 1 e4m3 + fp32 scales, 2 power-of-two scales, 3 scales packed as UE8M0 bytes
+// -> (recv_x [E,M,H], scales (transposed view of [E,groups,M]) or None, count [E], src_info [E,M], layout_range [E,1], entry_row [T,K])
+std::tuple<torch::Tensor, c10::optional<torch::Tensor>, torch::Tensor, torch::Tensor, torch::Tensor, torch::Tensor>
+ll_local_dispatch(torch::Tensor x, torch::Tensor topk_idx, int64_t M, int64_t E, int64_t wire, c10::optional<torch::Tensor> expert_stats) {
+    c10::cuda::CUDAGuard guard(x.device());
+    x = x.contiguous();
+    topk_idx = topk_idx.contiguous();
+    const TopK tk = topk_of(topk_idx);
+    TORCH_CHECK(x.is_cuda() && x.scalar_type() == torch::kBFloat16 && x.dim() == 2 && x.size(0) == tk.T, "x must be a bf16 [T, hidden] CUDA tensor");
+    int* stats = nullptr;
+    if (expert_stats.has_value()) {
+        TORCH_CHECK(expert_stats->is_cuda() && expert_stats->scalar_type() == torch::kInt32 && expert_stats->is_contiguous() &&
+                    expert_stats->numel() >= E, "expert_stats must be a contiguous int32 CUDA tensor of one word per expert");
+        stats = expert_stats->data_ptr<int>();
+    }
+    const int64_t H = x.size(1), G = H / 128;
+    auto recv = torch::empty({E, M, H}, on(x, wire > 0 ? torch::kFloat8_e4m3fn : torch::kBFloat16));
+    c10::optional<torch::Tensor> scales;
+    if (wire > 0) scales = wire == 3 ? torch::empty({E, G / 4, M}, on(x, torch::kInt32)) : torch::empty({E, G, M}, on(x, torch::kFloat32));
+    auto count = torch::empty({E}, on(x, torch::kInt32));
+    auto src_info = torch::empty({E, M}, on(x, torch::kInt32));
+    auto range = torch::empty({E, 1}, on(x, torch::kInt64));
+    auto entry = torch::empty({tk.T, tk.K}, on(x, torch::kInt32));
+    TM_CHECK_CUDA(tmoe::ll_local_dispatch(local_layout(E, M, H, (int)wire, false), x.data_ptr(), tk.ptr, tk.is64, tk.T, tk.K, recv.data_ptr(),
+                                          scales.has_value() ? scales->data_ptr() : nullptr, src_info.data_ptr<int>(),
+                                          reinterpret_cast<long long*>(range.data_ptr<int64_t>()), count.data_ptr<int>(), stats,
+                                          entry.data_ptr<int>(), cur_stream()));
+    if (scales.has_value()) scales = scales->transpose(1, 2);
+    return {recv, scales, count, src_info, range, entry};
+}
+
+torch::Tensor ll_local_combine(torch::Tensor x, torch::Tensor topk_idx, torch::Tensor topk_weights, torch::Tensor entry_row, int64_t M, int64_t E,
+                               int64_t H, bool logfmt, c10::optional<torch::Tensor> out) {
+    c10::cuda::CUDAGuard guard(x.device());
+    x = x.contiguous();
+    topk_idx = topk_idx.contiguous();
+    const TopK tk = topk_of(topk_idx);
+    const auto w = weights_of(topk_weights);
+    TORCH_CHECK(x.is_cuda() && x.scalar_type() == torch::kBFloat16 && x.numel() == E * M * H, "x must be bf16 [E_local, ranks*max_tokens, hidden]");
+    TORCH_CHECK(w.is_cuda() && w.numel() == (int64_t)tk.T * tk.K, "topk_weights must have one weight per entry");
+    if (!out.has_value()) out = torch::empty({tk.T, H}, on(x, torch::kBFloat16));
+    TORCH_CHECK(out->is_cuda() && out->scalar_type() == torch::kBFloat16 && out->is_contiguous() && out->dim() == 2 && out->size(0) == tk.T &&
+                out->size(1) == H, "out must be a contiguous bf16 [T, hidden] CUDA tensor");
+    TM_CHECK_CUDA(tmoe::ll_local_combine(local_layout(E, M, H, 0, logfmt), x.data_ptr(), tk.ptr, tk.is64, w.data_ptr<float>(),
+                                         entry_row.data_ptr<int>(), tk.T, tk.K, (int)entry_row.size(0), (int)entry_row.size(1), out->data_ptr(),
+                                         cur_stream()));
+    return *out;
+}
+
+// ------------------------------------------------------------------------------------------------ un-fused exchange
+struct Scratch {
+    torch::Tensor all;
+    int *totals, *row_local, *chunk_base;
+};
+Scratch route_scratch(const torch::Tensor& idx, const TopK& tk, int64_t E) {
+    const int64_t chunks = std::max<int64_t>(1, (tk.T + tmoe::kLocalChunk - 1) / tmoe::kLocalChunk);
+    Scratch s;
+    s.all = torch::empty({E + 2 + tk.T + chunks}, on(idx, torch::kInt32));
+    s.totals = s.all.data_ptr<int>();
+    s.row_local = s.totals + E + 2;
+    s.chunk_base = s.row_local + tk.T;
+    return s;
+}
+
+tmoe::LocalPart part(const torch::Tensor& src, const torch::Tensor& dst) {
+    return tmoe::LocalPart{src.data_ptr(), dst.data_ptr(), (uint32_t)(src.size(1) * src.element_size())};
+}
+
+// -> (tokens [1], tokens per expert [E], is_token_in_rank [T,1])
+std::tuple<torch::Tensor, torch::Tensor, torch::Tensor> local_counts(torch::Tensor topk_idx, int64_t E) {
+    c10::cuda::CUDAGuard guard(topk_idx.device());
+    topk_idx = topk_idx.contiguous();
+    const TopK tk = topk_of(topk_idx);
+    const auto s = route_scratch(topk_idx, tk, E);
+    auto in_rank = torch::empty({tk.T, 1}, on(topk_idx, torch::kBool));
+    TM_CHECK_CUDA(tmoe::local_route(tk.ptr, tk.is64, tk.T, tk.K, (int)E, s.totals, s.row_local, s.chunk_base,
+                                    reinterpret_cast<uint8_t*>(in_rank.data_ptr<bool>()), nullptr, cur_stream()));
+    return {s.all.narrow(0, E, 1), s.all.narrow(0, 0, E), in_rank};
+}
+
+// The one piece of host state: a pinned block that local_route writes the counts into, and the event behind it.
+class LocalExchange {
+  public:
+    ~LocalExchange() {
+        if (event_ != nullptr) cudaEventDestroy(event_);
+    }
+
+    // -> (received payloads, recv_idx, recv_w, counts per expert rounded up to `alignment` (empty with worst_rows), rows (-1: not read),
+    //     send_row [T], totals: device [E+1], entries per expert and rows)
+    py::tuple dispatch(std::vector<torch::Tensor> parts, torch::Tensor topk_idx, torch::Tensor topk_weights, int64_t E, int64_t worst_rows,
+                       int64_t alignment) {
+        std::vector<torch::Tensor> recv;
+        torch::Tensor idx_out, w_out, send_row, totals;
+        std::vector<int64_t> counts;
+        int64_t rows = -1;
+        {
+            py::gil_scoped_release nogil;
+            c10::cuda::CUDAGuard guard(topk_idx.device());
+            std::lock_guard<std::mutex> lock(mutex_);
+            const cudaStream_t stream = cur_stream();
+            topk_idx = topk_idx.contiguous();
+            const TopK tk = topk_of(topk_idx);
+            const auto w = weights_of(topk_weights);
+            TORCH_CHECK(w.is_cuda() && w.numel() == (int64_t)tk.T * tk.K, "topk_weights must have one weight per entry");
+            TORCH_CHECK(!parts.empty() && parts.size() <= tmoe::kLocalMaxParts, "one or two payloads");
+            const auto s = route_scratch(topk_idx, tk, E);
+            const int64_t cap = worst_rows > 0 ? worst_rows : tk.T;
+            std::vector<tmoe::LocalPart> lp;
+            for (auto& p : parts) {
+                p = p.contiguous();
+                TORCH_CHECK(p.is_cuda() && p.dim() == 2 && p.size(0) == tk.T, "payloads must be [T, C] CUDA tensors");
+                recv.push_back(torch::empty({cap, p.size(1)}, p.options()));
+                lp.push_back(part(p, recv.back()));
+            }
+            idx_out = torch::empty({cap, tk.K}, topk_idx.options());
+            w_out = torch::empty({cap, tk.K}, w.options());
+            send_row = torch::empty({tk.T}, on(topk_idx, torch::kInt32));
+            const bool wait = worst_rows <= 0;
+            if (wait) host_block(E + 1);
+            TM_CHECK_CUDA(tmoe::local_route(tk.ptr, tk.is64, tk.T, tk.K, (int)E, s.totals, s.row_local, s.chunk_base, nullptr,
+                                            wait ? host_.data_ptr<int>() : nullptr, stream));
+            if (wait) TORCH_CHECK(cudaEventRecord(event_, stream) == cudaSuccess, "teramoe_b200: cudaEventRecord failed");
+            TM_CHECK_CUDA(tmoe::local_dispatch(lp.data(), (int)lp.size(), tk.ptr, tk.is64, w.data_ptr<float>(), tk.T, tk.K, (int)E, s.totals,
+                                               s.row_local, s.chunk_base, send_row.data_ptr<int>(), idx_out.data_ptr(), w_out.data_ptr<float>(),
+                                               (int)std::max<int64_t>(worst_rows, 0), stream));
+            totals = s.all.narrow(0, 0, E + 1);
+            if (wait) {
+                // the rows are being copied while the host waits for the counts
+                const cudaError_t e = cudaEventSynchronize(event_);
+                TORCH_CHECK(e == cudaSuccess, "teramoe_b200: dispatch failed: ", cudaGetErrorString(e));
+                const int* h = host_.data_ptr<int>();
+                rows = h[0];
+                counts.resize(E);
+                for (int64_t e2 = 0; e2 < E; ++e2) counts[e2] = (h[1 + e2] + alignment - 1) / alignment * alignment;
+                if (rows < cap) {
+                    for (auto& r : recv) r = r.narrow(0, 0, rows);
+                    idx_out = idx_out.narrow(0, 0, rows);
+                    w_out = w_out.narrow(0, 0, rows);
+                }
+            }
+        }
+        return py::make_tuple(recv, idx_out, w_out, counts, rows, send_row, totals);
+    }
+
+  private:
+    void host_block(int64_t n) {
+        if (event_ == nullptr)
+            TORCH_CHECK(cudaEventCreateWithFlags(&event_, cudaEventDisableTiming) == cudaSuccess, "teramoe_b200: cudaEventCreate failed");
+        if (!host_.defined() || host_.numel() < n)
+            host_ = torch::empty({n}, torch::TensorOptions().dtype(torch::kInt32).pinned_memory(true));
+    }
+    std::mutex mutex_;
+    torch::Tensor host_;
+    cudaEvent_t event_ = nullptr;
+};
+
+// A dispatch whose layout is known: payload rows of the tokens that have a row.
+std::vector<torch::Tensor> local_scatter(std::vector<torch::Tensor> parts, torch::Tensor send_row, int64_t rows) {
+    c10::cuda::CUDAGuard guard(send_row.device());
+    std::vector<torch::Tensor> recv;
+    std::vector<tmoe::LocalPart> lp;
+    const int64_t T = send_row.numel();
+    TORCH_CHECK(!parts.empty() && parts.size() <= tmoe::kLocalMaxParts, "one or two payloads");
+    for (auto& p : parts) {
+        p = p.contiguous();
+        TORCH_CHECK(p.is_cuda() && p.dim() == 2 && p.size(0) == T, "payloads must be [T, C] CUDA tensors");
+        recv.push_back(torch::empty({rows, p.size(1)}, p.options()));
+        lp.push_back(part(p, recv.back()));
+    }
+    TM_CHECK_CUDA(tmoe::local_move(lp.data(), (int)lp.size(), send_row.data_ptr<int>(), (int)T, 1, nullptr, 0, 0, 0, nullptr, nullptr,
+                                   cur_stream()));
+    return recv;
+}
+
+// out[t] = row send_row[t] of x (zeros for tokens that went nowhere) and, with weights [rows, K], the entries' weights [T, K]
+std::tuple<torch::Tensor, c10::optional<torch::Tensor>> local_combine(torch::Tensor x, torch::Tensor send_row, torch::Tensor topk_idx, int64_t E,
+                                                                      c10::optional<torch::Tensor> weights) {
+    c10::cuda::CUDAGuard guard(x.device());
+    x = x.contiguous();
+    const TopK tk = topk_of(topk_idx);
+    TORCH_CHECK(x.is_cuda() && x.scalar_type() == torch::kBFloat16 && x.dim() == 2, "x must be a bf16 [rows, H] CUDA tensor");
+    auto out = torch::empty({tk.T, x.size(1)}, x.options());
+    c10::optional<torch::Tensor> w_out;
+    torch::Tensor w;
+    if (weights.has_value()) {
+        w = weights_of(*weights);
+        w_out = torch::empty({tk.T, tk.K}, w.options());
+    }
+    const tmoe::LocalPart p = part(x, out);
+    TM_CHECK_CUDA(tmoe::local_move(&p, 1, send_row.data_ptr<int>(), tk.T, 0, tk.ptr, tk.is64, tk.K, (int)E, w.defined() ? w.data_ptr<float>() : nullptr,
+                                   w_out.has_value() ? w_out->data_ptr<float>() : nullptr, cur_stream()));
+    return {out, w_out};
+}
+
+}  // namespace
+
+void register_local(pybind11::module_& m) {
+    m.def("ll_local_dispatch", &ll_local_dispatch);
+    m.def("ll_local_combine", &ll_local_combine);
+    m.def("local_counts", &local_counts);
+    m.def("local_scatter", &local_scatter);
+    m.def("local_combine", &local_combine);
+    py::class_<LocalExchange>(m, "LocalExchange").def(py::init<>()).def("dispatch", &LocalExchange::dispatch);
+}

@@ -1,0 +1,238 @@
+// Un-fused dispatch / combine on one rank, see local.h.
+//
+//   local_route     counts per expert and the row of every token: one launch, the last block to finish scans the chunks
+//   local_dispatch  rows, expert ids and weights of the tokens that go anywhere, in token order
+//   local_move      the repeat of a dispatch with a known layout, and the combine
+//
+// All are bound by memory traffic: every row is read once and written once.  A warp moves 2 KB of a row (four 16-byte loads in
+// flight per lane), so that a few hundred rows already fill the SMs.  Through the symmetric arena the same dispatch took a
+// push into the arena, a copy out of it, nine table copies and two waits of the host.  Measured through the API, hidden 7168,
+// top-8, 32 experts: layout + dispatch + combine + cached dispatch + combine with weights at 4096 tokens 1175 -> 99 us (77 launches
+// before), layout + FP8 dispatch + combine at 1003 tokens 718 -> 52 us.
+#include "local.h"
+
+#include "ptx.cuh"
+
+namespace tmoe {
+
+namespace {
+
+constexpr uint32_t kSegBytes = 2048;
+
+struct Parts {
+    LocalPart p[kLocalMaxParts];
+    int n;
+    int segs[kLocalMaxParts];
+    int total_segs;
+};
+
+__device__ __forceinline__ long long load_entry(const void* idx, int is64, long i) {
+    return is64 ? reinterpret_cast<const long long*>(idx)[i] : (long long) reinterpret_cast<const int*>(idx)[i];
+}
+
+__global__ void __launch_bounds__(kLocalChunk)
+local_route_kernel(const void* topk_idx, int is64, int T, int K, int E, int* totals, int* row_local, int* chunk_base, uint8_t* in_rank,
+                   int* host_out) {
+    extern __shared__ int hist[];
+    __shared__ int warp_rows[kLocalChunk / 32];
+    __shared__ int last;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    for (int e = tid; e < E; e += kLocalChunk) hist[e] = 0;
+    __syncthreads();
+    const int t = blockIdx.x * kLocalChunk + tid;
+    bool any = false;
+    if (t < T) {
+        for (int k = 0; k < K; ++k) {
+            const long long e = load_entry(topk_idx, is64, (long)t * K + k);
+            if (e >= 0 && e < E) {
+                atomicAdd(&hist[(int)e], 1);
+                any = true;
+            }
+        }
+        if (in_rank != nullptr) in_rank[t] = any ? 1 : 0;
+    }
+    const uint32_t b = __ballot_sync(0xffffffffu, any);
+    if (lane == 0) warp_rows[warp] = __popc(b);
+    __syncthreads();
+    int before = 0, rows = 0;
+    for (int w = 0; w < kLocalChunk / 32; ++w) {
+        if (w < warp) before += warp_rows[w];
+        rows += warp_rows[w];
+    }
+    if (t < T) row_local[t] = any ? before + __popc(b & ((1u << lane) - 1u)) : -1;
+    for (int e = tid; e < E; e += kLocalChunk)
+        if (hist[e] != 0) atomicAdd(totals + e, hist[e]);
+    if (tid == 0) {
+        chunk_base[blockIdx.x] = rows;
+        atomicAdd(totals + E, rows);
+    }
+    // the last block to arrive sees every count: it turns the chunk counts into chunk bases
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) last = atomicAdd(totals + E + 1, 1) == (int)gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    if (warp == 0) {
+        int run = 0;
+        for (int c0 = 0; c0 < (int)gridDim.x; c0 += 32) {
+            const int c = c0 + lane;
+            const int v = c < (int)gridDim.x ? __ldcg(chunk_base + c) : 0;
+            int incl = v;
+            for (int s = 1; s < 32; s <<= 1) {
+                const int u = __shfl_up_sync(0xffffffffu, incl, s);
+                if (lane >= s) incl += u;
+            }
+            if (c < (int)gridDim.x) chunk_base[c] = run + incl - v;
+            run += __shfl_sync(0xffffffffu, incl, 31);
+        }
+    }
+    if (host_out != nullptr) {
+        if (tid == 0) host_out[0] = __ldcg(totals + E);
+        for (int e = tid; e < E; e += kLocalChunk) host_out[1 + e] = __ldcg(totals + e);
+        __threadfence_system();
+    }
+}
+
+// up to kSegBytes of one row, by one warp; src == nullptr writes zeros
+__device__ __forceinline__ void move_segment(uint8_t* dst, const uint8_t* src, uint32_t bytes, int lane) {
+    const uintptr_t align = (reinterpret_cast<uintptr_t>(dst) | reinterpret_cast<uintptr_t>(src) | bytes) & 15u;
+    if (align == 0) {
+        const int nvec = (int)(bytes / 16);
+        int4* d = reinterpret_cast<int4*>(dst);
+        const int4* s = reinterpret_cast<const int4*>(src);
+        int4 v[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            v[i] = make_int4(0, 0, 0, 0);
+            if (src != nullptr && lane + 32 * i < nvec) v[i] = ld_nc_v4(s + lane + 32 * i);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (lane + 32 * i < nvec) d[lane + 32 * i] = v[i];
+    } else {
+        for (uint32_t i = lane; i < bytes; i += 32) dst[i] = src != nullptr ? src[i] : (uint8_t)0;
+    }
+}
+
+__device__ __forceinline__ void move_row_segment(const Parts& ps, int seg, long dst_row, long src_row, int lane) {
+    int i = 0;
+    if (ps.n > 1 && seg >= ps.segs[0]) {
+        seg -= ps.segs[0];
+        i = 1;
+    }
+    const LocalPart& p = ps.p[i];
+    const uint32_t off = (uint32_t)seg * kSegBytes;
+    const uint32_t bytes = min(kSegBytes, p.row_bytes - off);
+    const uint8_t* src = src_row < 0 ? nullptr : static_cast<const uint8_t*>(p.src) + (size_t)src_row * p.row_bytes + off;
+    move_segment(static_cast<uint8_t*>(p.dst) + (size_t)dst_row * p.row_bytes + off, src, bytes, lane);
+}
+
+__global__ void __launch_bounds__(256)
+local_dispatch_kernel(const __grid_constant__ Parts ps, const void* topk_idx, int is64, const float* topk_w, int T, int K, int E,
+                      const int* totals, const int* row_local, const int* chunk_base, int* send_row, void* recv_idx, float* recv_w,
+                      int worst_rows) {
+    const int lane = threadIdx.x & 31;
+    const long warps = (long)gridDim.x * (blockDim.x >> 5);
+    const int filled = worst_rows > 0 ? min(totals[E], worst_rows) : 0;
+    const long work = (long)(T + (worst_rows > 0 ? worst_rows - filled : 0)) * ps.total_segs;
+    for (long i = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < work; i += warps) {
+        const long t = i / ps.total_segs;
+        const int seg = (int)(i - t * ps.total_segs);
+        long row, src = t;
+        if (t < T) {
+            const int r = row_local[t];
+            row = r >= 0 ? (long)chunk_base[t / kLocalChunk] + r : -1;
+            if (seg == 0 && lane == 0) send_row[t] = (int)row;
+            if (row < 0) continue;
+        } else {
+            row = filled + (t - T);
+            src = -1;
+        }
+        move_row_segment(ps, seg, row, src, lane);
+        if (seg == 0 && lane < K) {
+            long long e = -1;
+            if (src >= 0) e = load_entry(topk_idx, is64, t * K + lane);
+            if (e >= E) e = -1;
+            if (is64) static_cast<long long*>(recv_idx)[row * K + lane] = e < 0 ? -1 : e;
+            else static_cast<int*>(recv_idx)[row * K + lane] = e < 0 ? -1 : (int)e;
+            recv_w[row * K + lane] = e < 0 ? 0.f : topk_w[t * K + lane];
+        }
+    }
+}
+
+__global__ void __launch_bounds__(256)
+local_move_kernel(const __grid_constant__ Parts ps, const int* send_row, int T, int to_rows, const void* topk_idx, int is64, int K, int E,
+                  const float* weights, float* weights_out) {
+    const int lane = threadIdx.x & 31;
+    const long warps = (long)gridDim.x * (blockDim.x >> 5);
+    const long work = (long)T * ps.total_segs;
+    for (long i = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < work; i += warps) {
+        const long t = i / ps.total_segs;
+        const int seg = (int)(i - t * ps.total_segs);
+        const long row = send_row[t];
+        if (to_rows) {
+            if (row >= 0) move_row_segment(ps, seg, row, t, lane);
+            continue;
+        }
+        move_row_segment(ps, seg, t, row, lane);
+        if (weights != nullptr && seg == 0 && lane < K) {
+            const long long e = load_entry(topk_idx, is64, t * K + lane);
+            weights_out[t * K + lane] = (row >= 0 && e >= 0 && e < E) ? weights[row * K + lane] : 0.f;
+        }
+    }
+}
+
+bool make_parts(const LocalPart* parts, int n, Parts& ps) {
+    if (n < 1 || n > kLocalMaxParts) return false;
+    ps.n = n;
+    ps.total_segs = 0;
+    for (int i = 0; i < n; ++i) {
+        if (parts[i].row_bytes == 0) return false;
+        ps.p[i] = parts[i];
+        ps.segs[i] = (int)((parts[i].row_bytes + kSegBytes - 1) / kSegBytes);
+        ps.total_segs += ps.segs[i];
+    }
+    return true;
+}
+
+int move_grid(long rows, int segs) {
+    const long blocks = (rows * segs + 7) / 8;
+    return (int)(blocks < 1 ? 1 : blocks > 148 * 16 ? 148 * 16 : blocks);
+}
+
+}  // namespace
+
+cudaError_t local_route(const void* topk_idx, int is64, int T, int K, int E, int* totals, int* row_local, int* chunk_base, uint8_t* in_rank,
+                        int* host_out, cudaStream_t stream) {
+    const size_t smem = (size_t)E * sizeof(int);
+    if (E < 1 || smem > 40 * 1024) return cudaErrorInvalidValue;
+    cudaError_t e = cudaMemsetAsync(totals, 0, (size_t)(E + 2) * sizeof(int), stream);
+    if (e != cudaSuccess) return e;
+    const int chunks = T > 0 ? (T + kLocalChunk - 1) / kLocalChunk : 1;
+    local_route_kernel<<<chunks, kLocalChunk, smem, stream>>>(topk_idx, is64, T, K, E, totals, row_local, chunk_base, in_rank, host_out);
+    return cudaGetLastError();
+}
+
+cudaError_t local_dispatch(const LocalPart* parts, int num_parts, const void* topk_idx, int is64, const float* topk_w, int T, int K, int E,
+                           const int* totals, const int* row_local, const int* chunk_base, int* send_row, void* recv_idx, float* recv_w,
+                           int worst_rows, cudaStream_t stream) {
+    Parts ps{};
+    if (!make_parts(parts, num_parts, ps) || K > 32) return cudaErrorInvalidValue;
+    const long rows = T > worst_rows ? T : worst_rows;
+    if (rows == 0) return cudaSuccess;
+    local_dispatch_kernel<<<move_grid(rows, ps.total_segs), 256, 0, stream>>>(ps, topk_idx, is64, topk_w, T, K, E, totals, row_local, chunk_base,
+                                                                             send_row, recv_idx, recv_w, worst_rows);
+    return cudaGetLastError();
+}
+
+cudaError_t local_move(const LocalPart* parts, int num_parts, const int* send_row, int T, int to_rows, const void* topk_idx, int is64, int K,
+                       int E, const float* weights, float* weights_out, cudaStream_t stream) {
+    Parts ps{};
+    if (!make_parts(parts, num_parts, ps) || K > 32) return cudaErrorInvalidValue;
+    if (T == 0) return cudaSuccess;
+    local_move_kernel<<<move_grid(T, ps.total_segs), 256, 0, stream>>>(ps, send_row, T, to_rows, topk_idx, is64, K, E, weights, weights_out);
+    return cudaGetLastError();
+}
+
+}  // namespace tmoe

@@ -55,6 +55,15 @@ cudaError_t ll_combine_recv(const LowLatLayout& lay, const void* arena_local, co
                             int T, int K, void* out, long long* wait_stats, long long call_seq, int* mask, int shrink, uint64_t limit_ns,
                             int* status, cudaStream_t stream);
 
+// One rank (num_ranks == 1, no mask): dispatch straight into the packed receive tensors (same contents and row order as
+// ll_dispatch_send + ll_dispatch_recv) and combine straight from the expert outputs.  entry_row: int [T, K], the packed row
+// (expert * max_tokens + row) of every entry, -1 where there is none; the combine takes it back with its sizes.
+cudaError_t ll_local_dispatch(const LowLatLayout& lay, const void* x, const void* topk_idx, int idx_is64, int T, int K, void* recv_x,
+                              void* recv_scales, int* src_info, long long* layout_range, int* recv_count, int* expert_stats, int* entry_row,
+                              cudaStream_t stream);
+cudaError_t ll_local_combine(const LowLatLayout& lay, const void* x, const void* topk_idx, int idx_is64, const float* topk_weights,
+                             const int* entry_row, int T, int K, int entry_t, int entry_k, void* out, cudaStream_t stream);
+
 // Rank-mask maintenance (reference: query / update / clean mask buffer kernels).
 cudaError_t ll_mask_update(int* mask, int num_ranks, int rank, int value, cudaStream_t stream);
 cudaError_t ll_mask_query(const int* mask, int num_ranks, int* out, cudaStream_t stream);

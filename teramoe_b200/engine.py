@@ -188,6 +188,23 @@ class LayerHandle:
 
 
 @dataclass
+class LocalHandle:
+    """Layout of an un-fused dispatch on one rank (csrc/local.cu): which row every token got."""
+    T: int
+    K: int
+    E: int
+    topk_idx: torch.Tensor
+    send_row: torch.Tensor       # [T] row of the token, -1 if it went nowhere
+    totals: torch.Tensor         # [E+1] on the device: entries per expert, number of rows
+    rows: int                    # number of rows, -1 while only the device knows it (fixed-shape dispatch)
+
+    def num_rows(self) -> int:
+        if self.rows < 0:
+            self.rows = int(self.totals[self.E])
+        return self.rows
+
+
+@dataclass
 class SavedForBackward:
     handle: LayerHandle
     saved_x: torch.Tensor        # [rows, H]

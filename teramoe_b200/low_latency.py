@@ -37,6 +37,7 @@ class LowLatencyHandle:
     src_info: Optional[torch.Tensor] = None       # [E_local, ranks*max_tokens] token index at the source
     layout_range: Optional[torch.Tensor] = None   # [E_local, ranks] int64: rows << 32 | first row
     seq: int = 0                                  # call number the flags of this dispatch / its combine carry
+    entry_row: Optional[torch.Tensor] = None      # one rank: [T,K] packed row of every entry (-1: none)
 
 
 def _ll_geometry(N: int, rank: int, E: int, M: int, H: int, use_fp8: bool, use_ue8m0: bool, round_scale: bool, use_logfmt: bool):
@@ -117,6 +118,10 @@ def _flatten(v):
     return list(v) if isinstance(v, tuple) else [v]
 
 
+def _nothing() -> None:
+    """Receive hook of a call that has nothing left to receive."""
+
+
 class LowLatencyMixin:
     """Methods mixed into `Buffer` (they use its `_engine`, `_drive`, `_world`, `group_size`)."""
 
@@ -182,6 +187,9 @@ class LowLatencyMixin:
         if T > M:
             raise ValueError(f"{T} tokens exceed num_max_dispatch_tokens_per_rank={M}")
         El = num_experts // N
+        if x.is_cuda and self._local is not None and not self.enable_shrink:
+            return self._ll_dispatch_local(x, topk_idx, M, num_experts, cumulative_local_expert_recv_stats, use_fp8, round_scale, use_ue8m0,
+                                           async_finish, return_recv_hook)
         if x.is_cuda:
             return self._ll_dispatch_cuda(x, topk_idx, M, num_experts, cumulative_local_expert_recv_stats, dispatch_wait_recv_cost_stats,
                                           use_fp8, round_scale, use_ue8m0, async_finish, return_recv_hook)
@@ -225,6 +233,33 @@ class LowLatencyMixin:
         hook: Optional[Callable] = (lambda: None) if return_recv_hook else None
         return recv, counts, handle, ev, hook
 
+    # ------------------------------------------------------------------ one rank (csrc/lowlat.cu, ll_local_*)
+    # Nothing crosses a link: the call is one kernel on the caller's stream, into tensors of its own.  Nothing is awaited
+    # either, so with `return_recv_hook` the work is done when the call returns and the hook has nothing left to do.
+    @staticmethod
+    def _ll_check(H, use_fp8, round_scale, use_ue8m0):
+        if H % 256 != 0:
+            raise ValueError("the low-latency kernels need hidden % 256 == 0")
+        if use_ue8m0 and not (use_fp8 and round_scale and H % 512 == 0):
+            raise ValueError("UE8M0 scales need use_fp8, round_scale and hidden % 512 == 0")
+
+    def _ll_dispatch_local(self, x, topk_idx, M, num_experts, expert_stats, use_fp8, round_scale, use_ue8m0, async_finish, return_recv_hook):
+        H = x.shape[1]
+        self._ll_check(H, use_fp8, round_scale, use_ue8m0)
+        wire = 0 if not use_fp8 else 3 if use_ue8m0 else 2 if round_scale else 1
+        (recv, scales, count, src_info, layout_range, entry_row), ev = self._run_local(
+            lambda: self._world.ext.ll_local_dispatch(x, topk_idx, M, num_experts, wire, expert_stats), None, async_finish and not return_recv_hook)
+        handle = LowLatencyHandle(None, M, H, num_experts, src_info=src_info, layout_range=layout_range, entry_row=entry_row)
+        return ((recv, scales) if use_fp8 else recv), count, handle, ev, (_nothing if return_recv_hook else None)
+
+    def _ll_combine_local(self, x, topk_idx, topk_weights, handle, use_logfmt, async_finish, return_recv_hook, out):
+        if topk_idx.shape[0] > handle.max_tokens:
+            raise ValueError(f"{topk_idx.shape[0]} tokens exceed num_max_dispatch_tokens_per_rank={handle.max_tokens}")
+        res, ev = self._run_local(
+            lambda: self._world.ext.ll_local_combine(x, topk_idx, topk_weights, handle.entry_row, handle.max_tokens, handle.num_experts,
+                                                     handle.hidden, use_logfmt, out), None, async_finish and not return_recv_hook)
+        return res, ev, (_nothing if return_recv_hook else None)
+
     # ------------------------------------------------------------------ kernel path (csrc/lowlat.cu)
     def _ll_prepare(self, M, H, E, use_fp8, use_ue8m0, round_scale, use_logfmt):
         """Geometry of the windows for these sizes; on a change (or after other users of the arena) the flag words are
@@ -249,10 +284,7 @@ class LowLatencyMixin:
         w, ext = self._world, self._world.ext
         N, T, H = self.group_size, x.shape[0], x.shape[1]
         El, G = num_experts // N, x.shape[1] // 128
-        if H % 256 != 0:
-            raise ValueError("the low-latency kernels need hidden % 256 == 0")
-        if use_ue8m0 and not (use_fp8 and round_scale and H % 512 == 0):
-            raise ValueError("UE8M0 scales need use_fp8, round_scale and hidden % 512 == 0")
+        self._ll_check(H, use_fp8, round_scale, use_ue8m0)
         mask = self._ll_mask_tensor() if self.enable_shrink else None
         dev = x.device
 
@@ -360,6 +392,8 @@ class LowLatencyMixin:
         """Weighted reduce at the token's rank: out[t] = sum_k topk_weights[t,k] * x[row of (t,k)].
         -> (combined_x [T,H], event, hook)."""
         src = self.get_next_low_latency_combine_buffer(handle) if zero_copy else x
+        if handle.entry_row is not None:
+            return self._ll_combine_local(src, topk_idx, topk_weights, handle, use_logfmt, async_finish, return_recv_hook, out)
         if handle.src_info is not None:
             return self._ll_combine_cuda(src, topk_idx, topk_weights, handle, use_logfmt, async_finish, return_recv_hook, out,
                                          combine_wait_recv_cost_stats)

@@ -1,0 +1,104 @@
+"""The one-rank kernels of the low-latency calls (csrc/lowlat.cu, ll_local_*) and of the un-fused exchange (csrc/local.cu),
+against the window kernels that several ranks use (a buffer with a rank mask takes them on one rank too) and against
+plain indexing."""
+import pytest
+import torch
+
+import teramoe_b200 as tm
+
+pytestmark = pytest.mark.gpu
+
+
+def _routing(T, E, K, seed, dtype=torch.int64, drop=0.2):
+    g = torch.Generator().manual_seed(seed)
+    idx = torch.stack([torch.randperm(E, generator=g)[:K] for _ in range(T)]) if T else torch.zeros(0, K, dtype=torch.int64)
+    gone = torch.rand(T, K, generator=g) < drop
+    if T > 2:
+        gone[2] = True                      # a token that goes nowhere
+    idx = idx.masked_fill(gone, -1)
+    w = torch.rand(T, K, generator=g)
+    return idx.to(dtype).cuda(), w.cuda()
+
+
+# one token; a token per block; fewer tokens than blocks wanted; more; hidden sizes of 1, 2 and 28 channel steps; top-k of 1, 8, 9 and 32
+@pytest.mark.parametrize("T,H,E,K,M", [(1, 256, 4, 1, 1), (0, 512, 4, 2, 8), (3, 512, 8, 8, 4), (77, 7168, 32, 8, 128), (300, 1024, 40, 9, 300),
+                                       (40, 2560, 64, 32, 64)])
+@pytest.mark.parametrize("wire", ["bf16", "fp8", "pow2", "ue8m0"])
+def test_low_latency_local_kernels_match_window_kernels(T, H, E, K, M, wire):
+    if wire == "ue8m0" and H % 512:
+        pytest.skip("UE8M0 scales are packed four groups to a word")
+    idx, w = _routing(T, E, K, seed=T + K, dtype=torch.int32 if K == 9 else torch.int64)
+    x = (torch.randn(T, H, generator=torch.Generator().manual_seed(T)) * 0.3).to(torch.bfloat16).cuda()
+    y = (torch.randn(E, M, H, generator=torch.Generator().manual_seed(H)) * 0.2).to(torch.bfloat16).cuda()
+    y[:, :, :128] *= 8.0                    # groups that LogFMT leaves as they are
+    got = []
+    for shrink in (False, True):            # local kernels, window kernels
+        buf = tm.Buffer(None, 0, low_latency_mode=True, explicitly_destroy=True, enable_shrink=shrink)
+        stats = torch.zeros(E, dtype=torch.int32, device="cuda")
+        recv, count, handle, _, hook = buf.low_latency_dispatch(x, idx, M, E, cumulative_local_expert_recv_stats=stats, use_fp8=wire != "bf16",
+                                                                round_scale=wire in ("pow2", "ue8m0"), use_ue8m0=wire == "ue8m0",
+                                                                return_recv_hook=True)
+        hook()
+        assert (handle.entry_row is None) == shrink
+        rows, scales = recv if isinstance(recv, tuple) else (recv, None)
+        valid = torch.arange(M, device="cuda").view(1, -1) < count.view(-1, 1)
+        outs = [count, stats, handle.layout_range, handle.src_info[valid], rows.view(torch.uint8)[valid]]
+        if scales is not None:
+            outs.append(scales[valid])
+        for logfmt in (False, True):
+            outs.append(buf.low_latency_combine(y, idx, w, handle, use_logfmt=logfmt)[0])
+        # routing with entries removed: their rows are left out
+        fewer = idx.masked_fill(torch.arange(K, device="cuda").view(1, -1) % 3 == 1, -1)
+        outs.append(buf.low_latency_combine(y, fewer, w, handle)[0])
+        torch.cuda.synchronize()
+        buf.check_status()
+        got.append(outs)
+        buf.destroy()
+    for i, (a, b) in enumerate(zip(*got)):
+        assert torch.equal(a, b), f"output {i} differs"
+
+
+# chunks of 128 tokens: one, a full one, one more token, several; rows of 2 KB segments: a short one, several, odd byte counts (fp8 scales)
+@pytest.mark.parametrize("T,H,E,K", [(0, 256, 4, 2), (1, 128, 4, 1), (128, 1024, 8, 4), (129, 1032, 300, 8), (1003, 7168, 32, 8), (5000, 256, 40, 32)])
+@pytest.mark.parametrize("fp8", [False, True])
+def test_unfused_exchange_matches_plain_indexing(T, H, E, K, fp8):
+    idx, w = _routing(T, E, K, seed=T + H, dtype=torch.int32 if T == 1003 else torch.int64)
+    g = torch.Generator().manual_seed(1)
+    x = torch.randn(T, H, generator=g).to(torch.bfloat16).cuda()
+    payload = (x.to(torch.float8_e4m3fn), torch.randn(T, max(1, H // 128), generator=g).cuda()) if fp8 else x
+    parts = payload if fp8 else (x,)
+    buf = tm.Buffer(None, 0, explicitly_destroy=True)
+    valid = idx >= 0
+    goes = valid.any(1)
+    n = int(goes.sum())
+    per_rank, _, per_expert, in_rank, _ = buf.get_dispatch_layout(idx, E)
+    want_counts = torch.bincount(idx[valid].long(), minlength=E)
+    assert per_rank.tolist() == [n] and torch.equal(per_expert.long(), want_counts) and torch.equal(in_rank[:, 0], goes)
+    recv, recv_idx, recv_w, counts, handle, _ = buf.deepep_dispatch(payload, topk_idx=idx, topk_weights=w, num_tokens_per_expert=per_expert,
+                                                                    expert_alignment=16)
+    assert counts == ((want_counts + 15) // 16 * 16).tolist() and recv_idx.dtype == idx.dtype
+    assert torch.equal(recv_idx, idx[goes]) and torch.equal(recv_w, torch.where(valid, w, torch.zeros_like(w))[goes])
+    for a, b in zip(recv if fp8 else (recv,), parts):
+        assert a.dtype == b.dtype and torch.equal(a.contiguous().view(torch.uint8), b[goes].contiguous().view(torch.uint8))
+    again = buf.deepep_dispatch(payload, handle=handle)[0]
+    for a, b in zip(again if fp8 else (again,), recv if fp8 else (recv,)):
+        assert torch.equal(a.contiguous().view(torch.uint8), b.contiguous().view(torch.uint8))
+    y = torch.randn(n, H, generator=g).to(torch.bfloat16).cuda()
+    out, cw, _ = buf.deepep_combine(y, handle, topk_weights=recv_w)
+    want = torch.zeros(T, H, dtype=torch.bfloat16, device="cuda")
+    want[goes] = y
+    assert torch.equal(out, want) and torch.equal(cw, torch.where(valid, w, torch.zeros_like(w)))
+    # fixed-shape outputs: rows past the received count are "nothing", and no host wait happens before the combine asks
+    worst = T + 5
+    recv, recv_idx, recv_w, counts, fixed, ev = buf.deepep_dispatch(payload, topk_idx=idx, topk_weights=w, num_tokens_per_expert=per_expert,
+                                                                    num_worst_tokens=worst, async_finish=True)
+    ev.current_stream_wait()
+    assert counts == [] and fixed.rows == -1 and recv_idx.shape == (worst, K)
+    assert torch.equal(recv_idx[:n], idx[goes]) and bool((recv_idx[n:] == -1).all()) and bool((recv_w[n:] == 0).all())
+    for a, b in zip(recv if fp8 else (recv,), parts):
+        a = a.view(torch.uint8)
+        assert a.shape[0] == worst and torch.equal(a[:n], b[goes].contiguous().view(torch.uint8)) and not bool(a[n:].any())
+    if n:
+        with pytest.raises(ValueError, match="expected"):
+            buf.deepep_combine(y[:-1], fixed)
+    buf.destroy()
