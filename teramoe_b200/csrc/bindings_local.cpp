@@ -5,10 +5,12 @@
 #include <pybind11/stl.h>
 #include <torch/extension.h>
 
+#include <array>
 #include <mutex>
 
 #include "launch_count.h"
 #include "local.h"
+#include "local_layer.h"
 #include "lowlat.h"
 
 namespace {
@@ -241,11 +243,124 @@ std::tuple<torch::Tensor, c10::optional<torch::Tensor>> local_combine(torch::Ten
     return {out, w_out};
 }
 
+// ------------------------------------------------------------------------------------------------ layer
+int64_t layer_rows(const tmoe::LocalLayerPlan& plan) { return std::max(plan.slots_cap, 128); }
+
+// bytes of the arena that a call with these sizes uses: rows in slot order and expert outputs in slot order
+int64_t local_layer_arena_bytes(int64_t T, int64_t K, int64_t E, int64_t H) {
+    return 2 * layer_rows(tmoe::local_layer_plan((int)T, (int)K, (int)E, (int)H, 64, 0)) * H * 2;
+}
+
+void check_layer_weights(const torch::Tensor& wg, const torch::Tensor& wd, int64_t E, int64_t H, int64_t I) {
+    TORCH_CHECK(wg.is_cuda() && wg.scalar_type() == torch::kBFloat16 && wg.is_contiguous() && wg.dim() == 3 && wg.size(0) == E &&
+                wg.size(1) == 2 * I && wg.size(2) == H, "W_gateup must be a contiguous bf16 [E, 2I, H] CUDA tensor");
+    TORCH_CHECK(wd.is_cuda() && wd.scalar_type() == torch::kBFloat16 && wd.is_contiguous() && wd.dim() == 3 && wd.size(0) == E &&
+                wd.size(1) == H && wd.size(2) == I, "W_down must be a contiguous bf16 [E, H, I] CUDA tensor");
+}
+
+void set_arena(tmoe::LocalLayerParams& p, int64_t rows, int64_t arena, int64_t arena_bytes) {
+    const int64_t half = rows * p.plan.H * 2;
+    TORCH_CHECK(2 * half <= arena_bytes, "the arena is too small for this call");
+    p.out_rows = (int)rows;
+    p.slot_x = reinterpret_cast<void*>(arena);
+    p.y = reinterpret_cast<void*>(arena + half);
+}
+
+// schedule: [group_units, lag_percent, min_lag_items, dispatch_pairs, num_sms]
+// -> (out [T,H], workspace, preact [rows,2I] or None, saved_x [T,H] or None)
+std::tuple<torch::Tensor, torch::Tensor, c10::optional<torch::Tensor>, c10::optional<torch::Tensor>>
+local_layer_forward(torch::Tensor x, torch::Tensor topk_idx, torch::Tensor topk_w, torch::Tensor w_gateup, torch::Tensor w_down,
+                    std::array<int64_t, 5> schedule, bool keep, int64_t arena, int64_t arena_bytes, torch::Tensor status) {
+    c10::cuda::CUDAGuard guard(x.device());
+    const TopK tk = topk_of(topk_idx);
+    const int64_t E = w_gateup.size(0), H = x.size(1), I = w_gateup.size(1) / 2;
+    TORCH_CHECK(x.is_cuda() && x.scalar_type() == torch::kBFloat16 && x.is_contiguous() && x.dim() == 2 && x.size(0) == tk.T, "x must be a contiguous bf16 [T, H] CUDA tensor");
+    TORCH_CHECK(topk_w.is_cuda() && topk_w.scalar_type() == torch::kFloat32 && topk_w.is_contiguous() && topk_w.numel() == (int64_t)tk.T * tk.K,
+                "topk_weights must be a contiguous fp32 [T, K] CUDA tensor");
+    check_layer_weights(w_gateup, w_down, E, H, I);
+    tmoe::LocalLayerParams p{};
+    p.plan = tmoe::local_layer_plan(tk.T, tk.K, (int)E, (int)H, (int)I, keep ? 1 : 0);
+    const int64_t rows = layer_rows(p.plan);
+    set_arena(p, rows, arena, arena_bytes);
+    auto ws = torch::empty({p.plan.words}, on(x, torch::kInt32));
+    auto out = torch::empty({tk.T, H}, x.options());
+    auto act = torch::empty({rows, I}, x.options());
+    c10::optional<torch::Tensor> preact, saved_x;
+    if (keep) {
+        preact = torch::empty({rows, 2 * I}, x.options());
+        saved_x = torch::empty({tk.T, H}, x.options());
+        p.aux = preact->data_ptr();
+        p.saved_x = saved_x->data_ptr();
+    }
+    p.ws = ws.data_ptr<int>();
+    p.topk_idx = tk.ptr; p.idx_is64 = tk.is64; p.topk_w = topk_w.data_ptr<float>();
+    p.group_units = (int)schedule[0]; p.lag_percent = (int)schedule[1]; p.min_lag_items = (int)schedule[2];
+    p.dispatch_pairs = (int)schedule[3]; p.num_sms = (int)schedule[4];
+    p.x = x.data_ptr(); p.w_gateup = w_gateup.data_ptr(); p.w_down = w_down.data_ptr();
+    p.act = act.data_ptr(); p.out = out.data_ptr();
+    p.status = status.data_ptr<int>();
+    const cudaStream_t stream = cur_stream();
+    tmoe::count_launch();
+    TM_CHECK_CUDA(tmoe::local_layer_route(p, stream));
+    TM_CHECK_CUDA(tmoe::local_layer_launch(p, stream));
+    return {out, ws, preact, saved_x};
+}
+
+// -> (dx [T,H], d(topk_weights) [T,K], dW_gateup, dW_down)
+std::tuple<torch::Tensor, torch::Tensor, torch::Tensor, torch::Tensor>
+local_layer_backward(torch::Tensor grad_out, torch::Tensor ws, torch::Tensor preact, torch::Tensor saved_x, torch::Tensor w_gateup,
+                     torch::Tensor w_down, int64_t K, std::array<int64_t, 5> schedule, int64_t arena, int64_t arena_bytes, torch::Tensor status) {
+    c10::cuda::CUDAGuard guard(grad_out.device());
+    const int64_t E = w_gateup.size(0), T = saved_x.size(0), H = saved_x.size(1), I = w_gateup.size(1) / 2;
+    TORCH_CHECK(grad_out.is_cuda() && grad_out.scalar_type() == torch::kBFloat16 && grad_out.is_contiguous() && grad_out.dim() == 2 &&
+                grad_out.size(0) == T && grad_out.size(1) == H, "grad_out must be a contiguous bf16 [T, H] CUDA tensor");
+    check_layer_weights(w_gateup, w_down, E, H, I);
+    tmoe::LocalLayerParams p{};
+    p.plan = tmoe::local_layer_plan((int)T, (int)K, (int)E, (int)H, (int)I, 1);
+    const int64_t rows = layer_rows(p.plan);
+    TORCH_CHECK(ws.numel() == p.plan.words && preact.size(0) == rows && preact.size(1) == 2 * I, "saved tensors of another call");
+    set_arena(p, rows, arena, arena_bytes);
+    auto act_w = torch::empty({rows, I}, grad_out.options());
+    auto dgu = torch::empty({rows, 2 * I}, grad_out.options());
+    auto xperm = torch::empty({rows, H}, grad_out.options());
+    auto parts = torch::empty({rows, 2 * ((I + 255) / 256)}, on(grad_out, torch::kFloat32));
+    auto dx = torch::empty({T, H}, grad_out.options());
+    auto dw = torch::empty({T, K}, on(grad_out, torch::kFloat32));
+    auto dwg = torch::empty({E, 2 * I, H}, grad_out.options());
+    auto dwd = torch::empty({E, H, I}, grad_out.options());
+    p.ws = ws.data_ptr<int>();
+    p.group_units = (int)schedule[0]; p.lag_percent = (int)schedule[1]; p.min_lag_items = (int)schedule[2];
+    p.dispatch_pairs = (int)schedule[3]; p.num_sms = (int)schedule[4];
+    p.bwd = 1;
+    p.x = grad_out.data_ptr(); p.w_gateup = w_gateup.data_ptr(); p.w_down = w_down.data_ptr();
+    p.act = act_w.data_ptr(); p.aux = dgu.data_ptr(); p.saved_x = saved_x.data_ptr(); p.out = dx.data_ptr();
+    p.preact = preact.data_ptr(); p.droute_part = parts.data_ptr<float>(); p.xperm = xperm.data_ptr();
+    p.dw_topk = dw.data_ptr<float>(); p.dw_gateup = dwg.data_ptr(); p.dw_down = dwd.data_ptr();
+    p.status = status.data_ptr<int>();
+    TM_CHECK_CUDA(tmoe::local_layer_launch(p, cur_stream()));
+    return {dx, dw, dwg, dwd};
+}
+
+// word offsets inside the workspace that the host may read: statistics of the two directions, entries per expert, slots in use
+py::dict local_layer_words(int64_t T, int64_t K, int64_t E, int64_t H, int64_t I, bool keep) {
+    const auto p = tmoe::local_layer_plan((int)T, (int)K, (int)E, (int)H, (int)I, keep ? 1 : 0);
+    py::dict d;
+    d["stats"] = py::make_tuple(p.stats[0], keep ? p.stats[1] : -1);
+    d["totals"] = p.totals;
+    d["meta"] = p.meta;
+    d["slots_cap"] = p.slots_cap;
+    return d;
+}
+
 }  // namespace
 
 void register_local(pybind11::module_& m) {
     m.def("ll_local_dispatch", &ll_local_dispatch);
     m.def("ll_local_combine", &ll_local_combine);
+    m.def("local_layer_arena_bytes", &local_layer_arena_bytes);
+    m.def("local_layer_forward", &local_layer_forward);
+    m.def("local_layer_backward", &local_layer_backward);
+    m.def("local_layer_words", &local_layer_words);
     m.def("local_counts", &local_counts);
     m.def("local_scatter", &local_scatter);
     m.def("local_combine", &local_combine);

@@ -1,0 +1,1363 @@
+// The MoE layer on one rank, see local_layer.h.  Roles of the persistent kernel (74 CTA pairs, 12 warps per CTA):
+//
+//   dispatch   the first pairs copy the routed rows into slot order (bulk copies through shared memory), then join
+//   producer   claims items of the work list, hands them to the pair, loads operand tiles by TMA
+//   issuer     tcgen05 cta_group::2, 256x256 tiles, two accumulators in tensor memory
+//   epilogue   8 warps: SwiGLU / dSwiGLU / store.  A warp packs 32 rows x 64 columns into shared memory (128-byte swizzle) and
+//              hands them to one TMA store.
+//   gather     warps 2 and 3, joined by the epilogue warps at the end of the list: keep a copy of x (forward), rebuild x in slot
+//              order and clear padding (backward), and sum every token's expert rows as soon as the units that hold them
+//              are finished.  Tokens are visited in the order of their last expert, which is the order in which they become ready.
+//
+// The work list, the 256x256x64 tiles and the order of every sum are those of layer.cu.  What is different because there is one
+// rank: rows are copied by slot instead of pushed by entry, expert rows stay in slot order (one TMA box per 32 rows instead
+// of 32 bulk copies to landing rows), the sum of a token waits for its own units instead of for every rank's completion
+// flag, counters have GPU scope, and no host read, table copy or padding kernel is left around the kernel.
+//
+// Forward + backward through the API, before (several-rank kernels, 30 to 38 launches and one host wait per step) -> after:
+//   512 tokens, H=512 I=256, 4 experts, top-2            905 ->   149 us   (was host work and launches)
+//   4096, H=2048 I=2048, 16 experts, top-8              2847 ->  2509 us
+//   8192, H=2048 I=3072, 16 experts, top-6              6047 ->  5383 us
+//   8192, H=7168 I=2048, 32 experts, top-8             16561 -> 15588 us
+//   forward only, 32 tokens of that layer                773 ->   630 us
+// Large layers are bound by the power cap: the issuer counts 5.63 M cycles for the forward at 8192 tokens, of which the tiles need 5.35 M,
+// while the clock drops to 1.24 GHz.
+#include "local_layer.h"
+
+#include "gemm_common.cuh"
+#include "layer.h"
+
+namespace tmoe {
+
+using namespace detail;
+
+namespace {
+
+constexpr int kStagesP = 6;
+constexpr int kBHalfBytesP = (BN / 2) * BK * 2;
+constexpr int kStageBytesP = kAStageBytes + kBHalfBytesP;                 // 32 KB
+constexpr int kPipeBytesP = kStagesP * kStageBytesP;                      // 192 KB
+constexpr int kBoxBytes = 32 * 128;                                       // 32 rows x 64 bf16 columns
+constexpr int kEpiBytes = kEpiWarps * kBoxBytes;                          // 32 KB: one box per epilogue warp
+constexpr int kBarOffsetP = kPipeBytesP + kEpiBytes;
+constexpr int kSmemBytesP = kBarOffsetP + 512 + 1024;
+constexpr int kCopyChunk = 8192;                                          // dispatch: two buffers per warp
+constexpr int kPublishBatch = 4;
+constexpr int kRingDepth = 4;
+constexpr int kGatherTasks = 16384;                                       // least number of (token, columns) tasks of the gather role
+constexpr uint32_t kOffTmem = 496, kOffCopyBar = 128, kOffRingFull = 320, kOffRingEmpty = 352, kOffItems = 384;
+constexpr uint32_t kRingConsumers = 2 * kEpiWarps + 2;
+static_assert((kThreads / 32) * 2 * kCopyChunk <= kBarOffsetP, "dispatch staging exceeds the operand stages + store staging");
+static_assert(8 * (2 * kStagesP + 4) <= (int)kOffCopyBar && kOffItems + 16 * kRingDepth <= kOffTmem && kOffTmem + 8 <= 512, "barrier block");
+static_assert(kSmemBytesP <= 232448, "shared memory");
+
+// words of the sync block
+enum { kSyncItem = 0, kSyncUnits = 1, kSyncToken = 2, kSyncCopy = 3, kSyncExpand = 4, kSyncExpanded = 5, kSyncWords = 16 };
+// words of the meta block
+enum { kMetaUnits = 0, kMetaSlots = 1, kMetaWork = 2 };
+
+constexpr int kRouteThreads = 256;
+constexpr int kRouteWarps = kRouteThreads / 32;
+
+__device__ __forceinline__ int load_expert(const void* idx, int is64, long i, int E) {
+    const long long e = is64 ? reinterpret_cast<const long long*>(idx)[i] : (long long) reinterpret_cast<const int*>(idx)[i];
+    return e >= 0 && e < E ? (int)e : -1;
+}
+
+// -------------------------------------------------------------------------------------------------
+// Routing.  A chunk is 256 tokens (a warp per 32); slots are ordered by (expert, 32-token group, k, lane) as in routing.cu.
+// count: histograms of a chunk's entries over experts and of its tokens over their LAST expert, plus the totals.
+// assign: every block derives the segment table from the totals and its own bases from the chunk histograms before it, so
+// no block waits for another and no scan kernel sits in between.
+// -------------------------------------------------------------------------------------------------
+struct RouteArgs {
+    LocalLayerPlan p;
+    int* ws;
+    const void* topk_idx;
+    int is64;
+    const float* topk_w;
+    int nb1[2], nb2, mu_wd, nb_wd, mu_wg, nb_wg;
+    int group_units, lag_percent, min_lag_items;
+};
+
+__global__ void __launch_bounds__(kRouteThreads) local_route_count_kernel(const RouteArgs a) {
+    extern __shared__ int sh[];
+    const int E = a.p.E, K = a.p.K, tid = threadIdx.x;
+    int* hist = sh;
+    int* last = sh + E;
+    for (int i = tid; i < 2 * E + 1; i += kRouteThreads) sh[i] = 0;
+    __syncthreads();
+    const int t = blockIdx.x * kRouteThreads + tid;
+    if (t < a.p.T) {
+        int m = -1;
+        for (int k = 0; k < K; ++k) {
+            const int e = load_expert(a.topk_idx, a.is64, (long)t * K + k, E);
+            if (e >= 0) atomicAdd(&hist[e], 1);
+            m = max(m, e);
+        }
+        atomicAdd(&last[m + 1], 1);
+    }
+    __syncthreads();
+    int* ch = a.ws + a.p.chunk_hist + (long)blockIdx.x * E;
+    int* cl = a.ws + a.p.chunk_last + (long)blockIdx.x * (E + 1);
+    for (int e = tid; e < E; e += kRouteThreads) {
+        ch[e] = hist[e];
+        if (hist[e] != 0) atomicAdd(a.ws + a.p.totals + e, hist[e]);
+    }
+    for (int e = tid; e <= E; e += kRouteThreads) {
+        cl[e] = last[e];
+        if (last[e] != 0) atomicAdd(a.ws + a.p.last_hist + e, last[e]);
+    }
+}
+
+// largest e with base[e] <= v < base[e + 1]
+__device__ __forceinline__ int find_segment(const int* base, int E, int v) {
+    int lo = 0, hi = E;
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (base[mid] <= v) lo = mid;
+        else hi = mid;
+    }
+    return lo;
+}
+
+__global__ void __launch_bounds__(kRouteThreads) local_route_assign_kernel(const RouteArgs a) {
+    extern __shared__ int sh[];
+    const int E = a.p.E, K = a.p.K, T = a.p.T, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    int* seg = sh;                           // [E + 1] first slot
+    int* ub = seg + E + 1;                   // [E + 1] first unit
+    int* ob = ub + E + 1;                    // [E + 1] first place in the token order, by last expert
+    int* cnt = ob + E + 1;                   // [warps][E] next slot
+    int* lst = cnt + kRouteWarps * E;        // [warps][E + 1] next place in the token order
+    const int* totals = a.ws + a.p.totals;
+    if (warp == 0) {
+        int run_s = 0, run_u = 0;
+        for (int e0 = 0; e0 < E; e0 += 32) {
+            const int e = e0 + lane;
+            const int blocks = e < E ? (totals[e] + 127) / 128 : 0;
+            int s = blocks * 128, u = (blocks + 1) / 2;
+            const int s_own = s, u_own = u;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int sv = __shfl_up_sync(0xffffffffu, s, o), uv = __shfl_up_sync(0xffffffffu, u, o);
+                if (lane >= o) {
+                    s += sv;
+                    u += uv;
+                }
+            }
+            if (e < E) {
+                seg[e] = run_s + s - s_own;
+                ub[e] = run_u + u - u_own;
+            }
+            run_s += __shfl_sync(0xffffffffu, s, 31);
+            run_u += __shfl_sync(0xffffffffu, u, 31);
+        }
+        if (lane == 0) {
+            seg[E] = run_s;
+            ub[E] = run_u;
+        }
+    }
+    if (warp == 1) {
+        int run = 0;
+        for (int e0 = 0; e0 <= E; e0 += 32) {
+            const int own = e0 + lane <= E ? a.ws[a.p.last_hist + e0 + lane] : 0;
+            int v = own;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int u = __shfl_up_sync(0xffffffffu, v, o);
+                if (lane >= o) v += u;
+            }
+            if (e0 + lane <= E) ob[e0 + lane] = run + v - own;
+            run += __shfl_sync(0xffffffffu, v, 31);
+        }
+    }
+    for (int i = tid; i < kRouteWarps * (2 * E + 1); i += kRouteThreads) cnt[i] = 0;
+    __syncthreads();
+    const int U = ub[E], S = seg[E];
+    const int gtid = blockIdx.x * kRouteThreads + tid, gthreads = gridDim.x * kRouteThreads;
+    // ---- tables
+    int* meta = a.ws + a.p.meta;
+    int* slot_tk = a.ws + a.p.slot_tk;
+    float* slot_w = reinterpret_cast<float*>(a.ws + a.p.slot_w);
+    if (blockIdx.x == 0) {
+        for (int e = tid; e <= E; e += kRouteThreads) a.ws[a.p.seg + e] = seg[e];
+        if (tid == 0) {
+            meta[kMetaUnits] = U;
+            meta[kMetaSlots] = S;
+        }
+    }
+    for (int e = blockIdx.x; e < E; e += gridDim.x)
+        for (int s = seg[e] + totals[e] + tid; s < seg[e + 1]; s += kRouteThreads) {
+            slot_tk[s] = -1;
+            slot_w[s] = 0.f;
+        }
+    // ---- work lists: the order that layer.cu's scheduler writes (see there), with units in slot order
+    const int SG = max(1, a.group_units), NG = (U + SG - 1) / SG;
+    for (int dir = 0; dir < (a.p.keep ? 2 : 1); ++dir) {
+        int4* work = reinterpret_cast<int4*>(a.ws + a.p.work[dir]);
+        const int cap = a.p.work_cap[dir], nb1 = a.nb1[dir], nb2 = a.nb2;
+        auto gsize = [&](int g) { return min(SG, U - g * SG); };
+        auto emit = [&](int pos, int kind, int g, int r) {
+            const int s = gsize(g), n_blk = r / s, u = g * SG + (r - n_blk * s);
+            const int e = find_segment(ub, E, u);
+            const int blk0 = seg[e] / 128 + 2 * (u - ub[e]);
+            const int two = (blk0 + 1) * 128 < seg[e + 1] ? 1 : 0;
+            const int end = seg[e] + totals[e];
+            const int need0 = max(0, min(128, end - blk0 * 128)), need1 = two ? max(0, min(128, end - (blk0 + 1) * 128)) : 0;
+            if (pos < cap) work[pos] = make_int4(kind | (two << 4) | (e << 8), u, n_blk | (need0 << 16) | (need1 << 24), blk0);
+        };
+        const int full1 = SG * nb1, full2 = SG * nb2;
+        const int lag_items = max((int)(((long)full1 * a.lag_percent + 99) / 100), a.min_lag_items);
+        const int lg = max(1, (lag_items + full1 - 1) / full1);
+        const int head_full = min(full1, max(0, lag_items - (lg - 1) * full1));
+        for (int g = blockIdx.x; g < NG + lg && NG > 0; g += gridDim.x) {
+            const int g2 = g - lg;
+            const int c2 = min(max(g2, 0), NG);
+            const int off = (g < NG ? g * full1 : U * nb1) + (c2 < NG ? c2 * full2 : U * nb2);
+            const int n1 = g < NG ? gsize(g) * nb1 : 0;
+            const int n2 = (g2 >= 0 && g2 < NG) ? gsize(g2) * nb2 : 0;
+            const int head = min(n1, head_full);
+            for (int i = tid; i < n1 + n2; i += kRouteThreads) {
+                if (i < head) emit(off + i, kWorkGemm1, g, i);
+                else if (i < head + n2) emit(off + i, kWorkGemm2, g2, i - head);
+                else emit(off + i, kWorkGemm1, g, i - n2);
+            }
+        }
+        int pos = U * (nb1 + nb2);
+        if (dir == 1) {
+            const int per_wd = a.mu_wd * a.nb_wd, per_wg = a.mu_wg * a.nb_wg;
+            for (int i = gtid; i < E * (per_wd + per_wg); i += gthreads) {
+                const bool down = i < E * per_wd;
+                const int j = down ? i : i - E * per_wd;
+                const int per = down ? per_wd : per_wg, mu = down ? a.mu_wd : a.mu_wg;
+                const int e = j / per, r = j - e * per, n_blk = r / mu;
+                if (pos + i < cap)
+                    work[pos + i] = make_int4((down ? kWorkWgradDown : kWorkWgradGateup) | (e << 8), seg[e], n_blk | ((r - n_blk * mu) << 16),
+                                              (totals[e] + BK - 1) / BK);       // blocks of padding add nothing
+            }
+            pos += E * (per_wd + per_wg);
+        }
+        if (gtid == 0) meta[kMetaWork + dir] = min(pos, cap);
+    }
+    // ---- slots of this chunk's entries, places of its tokens in the token order
+    if ((int)blockIdx.x >= a.p.chunks) return;
+    const int t = blockIdx.x * kRouteThreads + tid;
+    int m = -1;
+    if (t < T) {
+        for (int k = 0; k < K; ++k) {
+            const int e = load_expert(a.topk_idx, a.is64, (long)t * K + k, E);
+            if (e >= 0) atomicAdd(&cnt[warp * E + e], 1);
+            m = max(m, e);
+        }
+        atomicAdd(&lst[warp * (E + 1) + m + 1], 1);
+    }
+    __syncthreads();
+    const int* ch = a.ws + a.p.chunk_hist;
+    const int* cl = a.ws + a.p.chunk_last;
+    for (int i = tid; i < 2 * E + 1; i += kRouteThreads) {
+        const bool slots = i < E;
+        const int e = slots ? i : i - E, cols = slots ? E : E + 1;
+        const int* h = slots ? ch : cl;
+        int run = slots ? seg[e] : ob[e];
+#pragma unroll 8
+        for (int c = 0; c < (int)blockIdx.x; ++c) run += h[(long)c * cols + e];
+        int* w = slots ? cnt : lst;
+        for (int v = 0; v < kRouteWarps; ++v) {
+            const int n = w[v * cols + e];
+            w[v * cols + e] = run;
+            run += n;
+        }
+    }
+    __syncthreads();
+    const uint32_t before = (1u << lane) - 1u;
+    int* my = cnt + warp * E;
+    long place = 0;
+    {
+        const int bucket = t < T ? m + 1 : -1;
+        const uint32_t same = __match_any_sync(0xffffffffu, bucket);
+        if (t < T) {
+            place = lst[warp * (E + 1) + bucket] + __popc(same & before);
+            a.ws[a.p.token_order + place] = t;
+        }
+    }
+    for (int k = 0; k < K; ++k) {
+        const int e = t < T ? load_expert(a.topk_idx, a.is64, (long)t * K + k, E) : -1;
+        const uint32_t same = __match_any_sync(0xffffffffu, e);
+        int slot = -1;
+        if (e >= 0) {
+            slot = my[e] + __popc(same & before);
+            slot_tk[slot] = t * K + k;
+            slot_w[slot] = a.topk_w[(long)t * K + k];
+        }
+        __syncwarp();
+        if (e >= 0 && (same & before) == 0) my[e] += __popc(same);
+        __syncwarp();
+        if (t < T) a.ws[a.p.order_slot + place * K + k] = slot;
+    }
+}
+
+// -------------------------------------------------------------------------------------------------
+// The layer kernel
+// -------------------------------------------------------------------------------------------------
+struct Phase {
+    alignas(64) CUtensorMap map_a;
+    alignas(64) CUtensorMap map_b;
+    int nk, b_group_rows, num_n_blocks, n_total, m_total;
+};
+
+struct LayerArgsP {
+    Phase ph[4];
+    alignas(64) CUtensorMap st_act;      // stores: [out_rows, I] (backward: boxes of 32 columns), [out_rows, 2I], [out_rows, H] and
+    alignas(64) CUtensorMap st_aux;      // [E, rows, cols] of the weight gradients, in boxes of 32 rows x 64 columns
+    alignas(64) CUtensorMap st_y;
+    alignas(64) CUtensorMap st_dwd;
+    alignas(64) CUtensorMap st_dwg;
+    int T, K, H, I, E;
+    int dispatch_pairs, keep, out_rows;
+    const uint8_t* x;
+    uint8_t* slot_x;
+    const __nv_bfloat16* y;
+    __nv_bfloat16* saved_x;
+    __nv_bfloat16* xperm;
+    __nv_bfloat16* out;
+    const __nv_bfloat16* preact;
+    float* droute_part;
+    int n_parts;
+    float* dw_topk;
+    const int* meta;
+    const int* seg;
+    const int* totals;
+    const int* slot_tk;
+    const float* slot_w;
+    const int* token_order;              // tokens by their last expert
+    const int* order_slot;               // [T, K] slots of the tokens in that order
+    const int4* work;
+    int max_work, max_units;
+    int* sync;
+    int* done1;                          // per unit: epilogue warps that finished a tile of the first GEMM
+    int* done2;                          // per 128-row block: the same for the second GEMM
+    int* arrived;                        // per 128-row block: rows in place
+    unsigned long long* stats;
+    int* status;
+};
+
+__device__ __forceinline__ void red_add_relaxed_gpu(int* p, int v) {
+    asm volatile("red.relaxed.gpu.global.add.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+__device__ __forceinline__ int atom_add_acq_rel(int* p, int v) {
+    int old;
+    asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
+    return old;
+}
+__device__ __forceinline__ int4 ld_cg_v4_ordered(const void* p) {
+    int4 v;
+    // volatile keeps it behind the acquire loads that precede it; no memory clobber, so that many can be in flight
+    asm volatile("ld.global.cg.v4.s32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ void tma_store_3d(const CUtensorMap* map, uint32_t src_smem, int c0, int c1, int c2) {
+    asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];"
+                 ::"l"(reinterpret_cast<uint64_t>(map)), "r"(src_smem), "r"(c0), "r"(c1), "r"(c2)
+                 : "memory");
+}
+__device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+// Bounded wait until *flag >= target (counters that other SMs bump).
+__device__ __forceinline__ bool wait_count(const int* flag, int target, int* status, int site, uint32_t pause_ns) {
+    if (ld_acquire_gpu(flag) >= target) return true;
+    const uint64_t limit_ns = peer_wait_limit_ns(status);
+    const uint64_t t0 = globaltimer_ns();
+#pragma unroll 1
+    while (true) {
+#pragma unroll 1
+        for (int i = 0; i < 32; ++i) {
+            if (ld_acquire_gpu(flag) >= target) return true;
+            __nanosleep(pause_ns);
+        }
+        if (status != nullptr && ld_relaxed_sys(status) != 0) return false;
+        if (globaltimer_ns() - t0 > limit_ns) {
+            report_status(status, kStatusFlagTimeout, site, target);
+            return false;
+        }
+    }
+}
+
+// Warp-wide row copy with 16 loads in flight per lane (8 KB per warp): two warps per SM have to keep HBM busy.
+__device__ __forceinline__ void copy_row_deep(int4* dst, const int4* src, int nvec, int lane) {
+    for (int b = 0; b < nvec; b += 512) {
+        int4 v[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = ld_nc_v4(src + min(b + 32 * i + lane, nvec - 1));
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+            if (b + 32 * i + lane < nvec) dst[b + 32 * i + lane] = v[i];
+    }
+}
+
+struct Item {
+    int kind, n_blk, group, k0, nk, m0, unit, need;
+    bool live;          // this CTA's 128 rows are real
+    int m_in_group;     // weight gradients: first row of dW inside the expert
+};
+
+__device__ __forceinline__ void decode_item(const LayerArgsP& L, const int4& it, uint32_t rank, Item& q) {
+    q.kind = it.x & 15;
+    q.group = (it.x >> 8) & 0xfffff;
+    q.n_blk = it.z & 0xffff;
+    if (q.kind <= kWorkGemm2) {
+        q.unit = it.y;
+        q.need = rank == 0 ? ((it.z >> 16) & 0xff) : ((it.z >> 24) & 0xff);
+        q.live = (rank == 0) || ((it.x >> 4) & 1);
+        q.m0 = (it.w + (int)rank) * BM;
+        q.k0 = 0;
+        q.nk = L.ph[q.kind].nk;
+        q.m_in_group = 0;
+    } else {
+        q.unit = -1;
+        q.need = 0;
+        q.live = true;
+        q.m_in_group = ((it.z >> 16) * 2 + (int)rank) * BM;
+        q.m0 = q.m_in_group;
+        q.k0 = it.y;
+        q.nk = it.w;
+    }
+}
+
+// Store staging of one epilogue warp: a box of 32 rows x 128 bytes, swizzled as the tensor maps expect.  One box per warp, because the
+// 32 KB that a second one would take are worth more as a sixth operand stage; the wait until the store has read the box
+// is hidden behind the mainloop of the next tile.
+struct Staging {
+    uint32_t base;      // 1024-byte aligned
+    int lane;
+    // 16 bytes at 16-byte column `chunk` of this lane's row
+    __device__ __forceinline__ void put(int chunk, uint32_t a, uint32_t b, uint32_t c, uint32_t d) const {
+        st_shared_v4(base + lane * 128 + ((chunk ^ (lane & 7)) << 4), a, b, c, d);
+    }
+    __device__ __forceinline__ void put32(int half, const uint32_t (&acc)[32]) const {
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+            const uint32_t* p = acc + 8 * v;
+            put(4 * half + v, pack_bf16x2(__uint_as_float(p[0]), __uint_as_float(p[1])), pack_bf16x2(__uint_as_float(p[2]), __uint_as_float(p[3])),
+                pack_bf16x2(__uint_as_float(p[4]), __uint_as_float(p[5])), pack_bf16x2(__uint_as_float(p[6]), __uint_as_float(p[7])));
+        }
+    }
+    // the same in a box of 32 rows x 64 bytes (64-byte swizzle)
+    __device__ __forceinline__ void put_narrow(int chunk, uint32_t a, uint32_t b, uint32_t c, uint32_t d) const {
+        st_shared_v4(base + lane * 64 + ((chunk ^ ((lane >> 1) & 3)) << 4), a, b, c, d);
+    }
+    // wait until this warp's last store has been read out of shared memory
+    __device__ __forceinline__ void reuse() const {
+        if (lane == 0) tma_store_wait_read<0>();
+        __syncwarp();
+    }
+    __device__ __forceinline__ void store(bool wanted, const CUtensorMap* map, int c0, int c1) const {
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0 && wanted) {
+            tma_store_2d(map, base, c0, c1);
+            tma_store_commit();
+        }
+    }
+    __device__ __forceinline__ void store3(bool wanted, const CUtensorMap* map, int c0, int c1, int c2) const {
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0 && wanted) {
+            tma_store_3d(map, base, c0, c1, c2);
+            tma_store_commit();
+        }
+    }
+};
+
+// First GEMM, forward: accumulator columns (2j, 2j+1) = (gate_j, up_j).  act = silu(g) * u * w; the pre-activation is kept for
+// backward (from a second read of tensor memory, which costs less than 32 registers to hold the activation).
+__device__ __forceinline__ void epilogue_swiglu(const LayerArgsP& L, const Staging& st, uint32_t taddr, int row0, bool live, int n0) {
+    const float w = live ? L.slot_w[row0 + st.lane] : 0.f;
+    const int n_total = 2 * L.I;
+    st.reuse();
+#pragma unroll 1
+    for (int c = 0; c < 4; ++c) {
+        uint32_t acc[32];
+        tmem_ld_x32(taddr + (uint32_t)(c * 32), acc);
+        tmem_ld_wait();
+        uint32_t o[8];
+#pragma unroll
+        for (int p = 0; p < 8; ++p) {
+            float v[2];
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const float gt = __uint_as_float(acc[4 * p + 2 * e]), up = __uint_as_float(acc[4 * p + 2 * e + 1]);
+                v[e] = __fdividef(gt, 1.f + __expf(-gt)) * up * w;
+            }
+            o[p] = pack_bf16x2(v[0], v[1]);
+        }
+        st.put(2 * c, o[0], o[1], o[2], o[3]);
+        st.put(2 * c + 1, o[4], o[5], o[6], o[7]);
+    }
+    st.store(live && n0 < n_total, &L.st_act, n0 >> 1, row0);
+    if (!L.keep) return;
+#pragma unroll 1
+    for (int h = 0; h < 2; ++h) {
+        uint32_t a0[32], a1[32];
+        tmem_ld_x32(taddr + (uint32_t)(h * 64), a0);
+        tmem_ld_x32(taddr + (uint32_t)(h * 64 + 32), a1);
+        tmem_ld_wait();
+        st.reuse();
+        st.put32(0, a0);
+        st.put32(1, a1);
+        st.store(live && n0 + h * 64 < n_total, &L.st_aux, n0 + h * 64, row0);
+    }
+}
+
+// First GEMM, backward: accumulator column j = d act_j.  Padding rows give zeros whatever the operands hold there: dGU and
+// act x route are operands of the weight gradients, which sum over whole 64-row blocks.
+__device__ __forceinline__ void epilogue_dswiglu(const LayerArgsP& L, const Staging& st, uint32_t taddr, int row0, bool live, int n0, int part) {
+    const long row = row0 + st.lane;
+    const bool real = live && L.slot_tk[row] >= 0;
+    const float w = real ? L.slot_w[row] : 0.f;
+    float droute = 0.f;
+#pragma unroll 1
+    for (int c = 0; c < 4; ++c) {
+        const int col = n0 + c * 32;
+        const bool in = live && col < L.I;
+        int4 pre[8];
+#pragma unroll
+        for (int v = 0; v < 8; ++v) pre[v] = make_int4(0, 0, 0, 0);
+        if (real && in) {
+            // issued before the tensor-memory load so that their latencies overlap
+            const int4* pp = reinterpret_cast<const int4*>(L.preact + row * (2l * L.I) + 2 * col);
+#pragma unroll
+            for (int v = 0; v < 8; ++v) pre[v] = ld_nc_v4(pp + v);
+        }
+        uint32_t acc[32];
+        tmem_ld_x32(taddr + (uint32_t)(c * 32), acc);
+        tmem_ld_wait();
+        st.reuse();
+        uint32_t act[16];
+#pragma unroll
+        for (int v = 0; v < 8; ++v) {
+            const uint32_t pr[4] = {(uint32_t)pre[v].x, (uint32_t)pre[v].y, (uint32_t)pre[v].z, (uint32_t)pre[v].w};
+            uint32_t dgu[4];
+            float av[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float2 gu = unpack_bf16x2(pr[e]);
+                const float ga = real ? __uint_as_float(acc[4 * v + e]) : 0.f;
+                const float sig = __fdividef(1.f, 1.f + __expf(-gu.x));
+                const float s = gu.x * sig;
+                const float a = s * gu.y;
+                const float gaw = ga * w;
+                const float d_up = s * gaw;
+                const float d_gate = (sig - s * sig + s) * gaw * gu.y;
+                dgu[e] = pack_bf16x2(d_gate, d_up);
+                av[e] = a * w;
+                droute += ga * a;
+            }
+            st.put(v, dgu[0], dgu[1], dgu[2], dgu[3]);
+            act[2 * v] = pack_bf16x2(av[0], av[1]);
+            act[2 * v + 1] = pack_bf16x2(av[2], av[3]);
+        }
+        st.store(in, &L.st_aux, 2 * col, row0);
+        st.reuse();
+#pragma unroll
+        for (int v = 0; v < 4; ++v) st.put_narrow(v, act[4 * v], act[4 * v + 1], act[4 * v + 2], act[4 * v + 3]);
+        st.store(in, &L.st_act, col, row0);
+    }
+    if (live) L.droute_part[row * L.n_parts + part] = droute;
+}
+
+// 128 accumulator columns as two boxes; store_box(first column)
+template <typename F>
+__device__ __forceinline__ void epilogue_plain(const Staging& st, uint32_t taddr, bool zero, F store_box) {
+#pragma unroll 1
+    for (int h = 0; h < 2; ++h) {
+        uint32_t a0[32], a1[32];
+        tmem_ld_x32(taddr + (uint32_t)(h * 64), a0);
+        tmem_ld_x32(taddr + (uint32_t)(h * 64 + 32), a1);
+        tmem_ld_wait();
+        if (zero) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) a0[i] = a1[i] = 0u;
+        }
+        st.reuse();
+        st.put32(0, a0);
+        st.put32(1, a1);
+        store_box(h * 64);
+    }
+}
+
+template <bool BWD>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
+local_layer_kernel(const __grid_constant__ LayerArgsP L) {
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
+    const uint32_t bar_base = smem_base + kBarOffsetP;
+    auto full_bar = [&](int s) { return bar_base + 8u * s; };
+    auto empty_bar = [&](int s) { return bar_base + 8u * (kStagesP + s); };
+    auto tfull_bar = [&](int s) { return bar_base + 8u * (2 * kStagesP + s); };
+    auto tempty_bar = [&](int s) { return bar_base + 8u * (2 * kStagesP + 2 + s); };
+    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + kBarOffsetP + kOffTmem);
+    volatile uint32_t* abort_flag = tmem_slot + 1;
+    auto copy_bar = [&](int w, uint32_t b) { return bar_base + kOffCopyBar + 8u * (2u * w + b); };
+    auto ring_full = [&](int e) { return bar_base + kOffRingFull + 8u * e; };
+    auto ring_empty = [&](int e) { return bar_base + kOffRingEmpty + 8u * e; };
+
+    const int warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31;
+    const uint32_t rank = cluster_ctarank();
+    const int pair = blockIdx.x >> 1;
+
+    if (threadIdx.x == 0) {
+        *abort_flag = 0u;
+        for (int s = 0; s < kStagesP; ++s) {
+            mbar_init(full_bar(s), 2);
+            mbar_init(empty_bar(s), 1);
+        }
+        for (int s = 0; s < 2; ++s) {
+            mbar_init(tfull_bar(s), 1);
+            mbar_init(tempty_bar(s), 2 * kEpiWarps);
+        }
+        for (int w = 0; w < kThreads / 32; ++w) {
+            mbar_init(copy_bar(w, 0), 1);
+            mbar_init(copy_bar(w, 1), 1);
+        }
+        for (int e = 0; e < kRingDepth; ++e) {
+            mbar_init(ring_full(e), 1);
+            mbar_init(ring_empty(e), kRingConsumers);
+        }
+        fence_mbar_init();
+#pragma unroll
+        for (int p = 0; p < (BWD ? 4 : 2); ++p) {
+            tma_prefetch_desc(&L.ph[p].map_a);
+            tma_prefetch_desc(&L.ph[p].map_b);
+        }
+    }
+    if (warp == 2) tmem_alloc_2cta(smem_u32((const void*)tmem_slot), kTmemCols);
+    tcgen05_fence_before();
+    cluster_sync_all();
+    tcgen05_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+
+    const int num_units = min(L.meta[kMetaUnits], L.max_units);
+    const int num_slots = L.meta[kMetaSlots];
+    const int target1 = 2 * kEpiWarps * L.ph[0].num_n_blocks;         // epilogue warps that finish a unit's first GEMM,
+    const int target2 = kEpiWarps * L.ph[1].num_n_blocks;             // a block's second GEMM
+
+    if (pair < L.dispatch_pairs) {
+        // ------------------------------------------------------------------ dispatch role (all 12 warps)
+        // A warp's leader streams rows through its two 8 KB buffers (in the operand stages, which nobody uses yet): global -> shared
+        // completes on the buffer's mbarrier, shared -> slot row joins a bulk group; the load of a chunk runs while the one
+        // before it is stored.  Rows are counted into their block in batches behind one completed group and one fence.
+        if (lane == 0) {
+            const int warps_total = L.dispatch_pairs * 2 * (kThreads / 32);
+            const int wid = (pair * 2 + (int)rank) * (kThreads / 32) + warp;
+            const uint32_t buf0 = smem_base + (uint32_t)warp * (2 * kCopyChunk);
+            const uint32_t row_bytes = (uint32_t)L.H * 2u;
+            uint32_t ph0 = 0, ph1 = 0, nchunk = 0;
+            bool ok = true, pend = false, pend_last = false;
+            uint64_t pend_dst = 0;
+            uint32_t pend_bytes = 0, pend_b = 0;
+            int pend_blk = 0, pub[kPublishBatch], npub = 0;
+            auto publish = [&]() {
+                if (npub == 0) return;
+                tma_store_wait<0>();
+                fence_proxy_async_all();
+                fence_acq_rel_gpu();
+#pragma unroll
+                for (int i = 0; i < kPublishBatch; ++i)
+                    if (i < npub) red_add_relaxed_gpu(L.arrived + pub[i], 1);
+                npub = 0;
+            };
+            auto store_pending = [&]() -> bool {
+                if (!pend) return true;
+                if (!mbar_wait(copy_bar(warp, pend_b), pend_b ? ph1 : ph0, abort_flag, L.status, 640)) return false;
+                if (pend_b) ph1 ^= 1u; else ph0 ^= 1u;
+                bulk_store_1d(pend_dst, buf0 + pend_b * kCopyChunk, pend_bytes);
+                tma_store_commit();
+                pend = false;
+                if (pend_last) {
+#pragma unroll
+                    for (int i = 0; i < kPublishBatch; ++i)
+                        if (i == npub) pub[i] = pend_blk;
+                    if (++npub == kPublishBatch) publish();
+                }
+                return true;
+            };
+            int next_tk = wid < num_slots ? L.slot_tk[wid] : -1;
+            for (int s = wid; ok && s < num_slots; s += warps_total) {
+                const int tk = next_tk;
+                next_tk = s + warps_total < num_slots ? L.slot_tk[s + warps_total] : -1;
+                if (tk < 0) continue;
+                const uint8_t* src = L.x + (size_t)(tk / L.K) * row_bytes;
+                const uint64_t dst = reinterpret_cast<uint64_t>(L.slot_x) + (uint64_t)s * row_bytes;
+                for (uint32_t off = 0; off < row_bytes; off += kCopyChunk) {
+                    const uint32_t chunk = min((uint32_t)kCopyChunk, row_bytes - off);
+                    const uint32_t b = nchunk & 1u;
+                    tma_store_wait_read<0>();
+                    mbar_arrive_expect_tx(copy_bar(warp, b), chunk);
+                    bulk_load_1d(buf0 + b * kCopyChunk, src + off, chunk, copy_bar(warp, b));
+                    ++nchunk;
+                    if (!(ok = store_pending())) break;
+                    pend = true;
+                    pend_b = b;
+                    pend_dst = dst + off;
+                    pend_bytes = chunk;
+                    pend_last = off + kCopyChunk >= row_bytes;
+                    pend_blk = s >> 7;
+                }
+            }
+            if (ok) ok = store_pending();
+            if (ok) publish();
+            tma_store_wait<0>();
+        }
+        __syncwarp();
+        cluster_sync_all();                   // both CTAs of the pair are done with the staging buffers: they become operand stages
+    }
+
+    // ---------------------------------------------------------------------- gather role
+    const int nvec = L.H / 8;
+    auto clear_padding = [&](int s) {
+        int4* row = reinterpret_cast<int4*>(L.slot_x) + (long)s * nvec;
+        for (int i = lane; i < nvec; i += 32) row[i] = make_int4(0, 0, 0, 0);
+    };
+    auto clear_all_padding = [&]() {
+        // Forward: what stands in padding rows reaches no result, so nothing waits for this.  But the tensor cores multiply these
+        // rows too, and multiplying leftovers of earlier calls costs power, which is what limits large layers.
+        const int warps = gridDim.x * 2, gw = blockIdx.x * 2 + (warp - 2);
+        const int share = max(1, warps / L.E);
+        for (int e = gw / share; e < L.E; e += (warps + share - 1) / share)
+            for (int s = L.seg[e] + L.totals[e] + gw % share; s < L.seg[e + 1]; s += share) clear_padding(s);
+    };
+    auto copy_x_loop = [&]() {
+        // forward: backward's copy of x, eight rows per claim
+        while (true) {
+            int t0 = 0;
+            if (lane == 0) t0 = atomicAdd(L.sync + kSyncCopy, 8);
+            t0 = __shfl_sync(0xffffffffu, t0, 0);
+            if (t0 >= L.T) break;
+            for (int t = t0; t < min(t0 + 8, L.T); ++t)
+                copy_row_deep(reinterpret_cast<int4*>(L.saved_x + (long)t * L.H), reinterpret_cast<const int4*>(L.x) + (long)t * nvec, nvec, lane);
+        }
+    };
+    auto expand_loop = [&]() {
+        // backward: x in slot order (operand of dW_gateup) and zeros in the padding rows of both slot-order operands
+        while (true) {
+            int s0 = 0;
+            if (lane == 0) s0 = atomicAdd(L.sync + kSyncExpand, 8);
+            s0 = __shfl_sync(0xffffffffu, s0, 0);
+            if (s0 >= num_slots) break;
+            const int s1 = min(s0 + 8, num_slots);
+            for (int s = s0; s < s1; ++s) {
+                const int tk = L.slot_tk[s];
+                int4* dst = reinterpret_cast<int4*>(L.xperm + (long)s * L.H);
+                if (tk >= 0) {
+                    copy_row_deep(dst, reinterpret_cast<const int4*>(L.saved_x + (long)(tk / L.K) * L.H), nvec, lane);
+                } else {
+                    for (int i = lane; i < nvec; i += 32) dst[i] = make_int4(0, 0, 0, 0);
+                    clear_padding(s);
+                }
+            }
+            __syncwarp();
+            if (lane == 0) {
+                fence_acq_rel_gpu();
+                red_add_release_gpu(L.sync + kSyncExpanded, s1 - s0);
+            }
+        }
+    };
+    // Rows [k0, k0 + n) of a token's entries, columns v and v + 32: all loads are issued before the first is used (16 in flight
+    // per lane; a load behind a lane-dependent branch would be waited for one at a time, so out-of-range columns are clamped
+    // and only their stores are left out).
+    auto add_rows = [&](const int (&slots)[8], int n, uint32_t valid, int v0, int v1, float (&a0)[8], float (&a1)[8]) {
+        int4 r0[8], r1[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            if (j < n) {
+                const int4* row = reinterpret_cast<const int4*>(L.y) + (long)slots[j] * nvec;
+                r0[j] = ld_cg_v4_ordered(row + v0);
+                r1[j] = ld_cg_v4_ordered(row + v1);
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            if (j < n && ((valid >> j) & 1u)) {
+                const uint32_t p0[4] = {(uint32_t)r0[j].x, (uint32_t)r0[j].y, (uint32_t)r0[j].z, (uint32_t)r0[j].w};
+                const uint32_t p1[4] = {(uint32_t)r1[j].x, (uint32_t)r1[j].y, (uint32_t)r1[j].z, (uint32_t)r1[j].w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float2 f0 = unpack_bf16x2(p0[i]), f1 = unpack_bf16x2(p1[i]);
+                    a0[2 * i] += f0.x;
+                    a0[2 * i + 1] += f0.y;
+                    a1[2 * i] += f1.x;
+                    a1[2 * i + 1] += f1.y;
+                }
+            }
+        }
+    };
+    auto gather_loop = [&]() {
+        // A task is (token, part of its columns).  Most tokens become ready in the last few percent of the kernel, so the tail
+        // is as long as the last tasks: about eleven for each of the 1480 warps that take part by then, down to 512 columns.
+        // The order of a sum (k ascending) does not depend on it.
+        const int K = L.K;
+        const int steps = (nvec + 63) / 64;
+        const int parts = max(1, min(steps, kGatherTasks / max(L.T, 1)));
+        const int part_steps = (steps + parts - 1) / parts;
+        const int tasks = L.T * parts;
+        uint64_t waited = 0;
+        bool stamped = false;
+        const bool stamps = L.stats != nullptr && lane == 0;
+        // claimed one task ahead, with the token's slots, so that a task starts with the test of its counters
+        int next_i = tasks, next_t = 0, next_slot = -1;
+        auto claim = [&]() {
+            if (lane == 0) next_i = atomicAdd(L.sync + kSyncToken, 1);
+            next_i = __shfl_sync(0xffffffffu, next_i, 0);
+            if (next_i < tasks) {
+                next_t = L.token_order[next_i / parts];
+                next_slot = lane < K ? L.order_slot[(long)(next_i / parts) * K + lane] : -1;
+            }
+        };
+        if (L.T > 0) claim();
+        while (next_i < tasks) {
+            const int part = next_i % parts, t = next_t, slot = next_slot;
+            claim();
+            const uint32_t valid = __ballot_sync(0xffffffffu, slot >= 0);
+            bool ready = true;
+            if (slot >= 0) {
+                const int* flag = L.done2 + (slot >> 7);
+                if (ld_acquire_gpu(flag) < target2) {
+                    const uint64_t w0 = globaltimer_ns();
+                    ready = wait_count(flag, target2, L.status, 660, 500);
+                    waited += globaltimer_ns() - w0;
+                }
+            }
+            if (!__all_sync(0xffffffffu, ready)) return;                  // reported: unwind
+            __syncwarp();                                                 // every lane reads behind the other lanes' acquires
+            if (stamps && !stamped) {
+                stamped = true;
+                atomicMax(L.stats + kStatKindFirst + kWorkReduce, ~globaltimer_ns());
+            }
+            if constexpr (BWD) {
+                if (part == 0 && lane < K && slot < 0) L.dw_topk[(long)t * K + lane] = 0.f;
+            }
+            int4* dst = reinterpret_cast<int4*>(L.out + (long)t * L.H);
+            int sl[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) sl[j] = max(0, __shfl_sync(0xffffffffu, slot, j));
+            const int step1 = min(steps, (part + 1) * part_steps);
+            for (int step = part * part_steps; step < step1; ++step) {
+                const int c0 = step * 64 + lane, c1 = c0 + 32;
+                const int v0 = min(c0, nvec - 1), v1 = min(c1, nvec - 1);
+                float a0[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+                float a1[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+                add_rows(sl, min(K, 8), valid, v0, v1, a0, a1);
+                for (int k0 = 8; k0 < K; k0 += 8) {
+                    int more[8];
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) more[j] = max(0, __shfl_sync(0xffffffffu, slot, (k0 + j) & 31));
+                    add_rows(more, min(K - k0, 8), valid >> k0, v0, v1, a0, a1);
+                }
+                if (c0 < nvec)
+                    dst[c0] = make_int4((int)pack_bf16x2(a0[0], a0[1]), (int)pack_bf16x2(a0[2], a0[3]), (int)pack_bf16x2(a0[4], a0[5]),
+                                        (int)pack_bf16x2(a0[6], a0[7]));
+                if (c1 < nvec)
+                    dst[c1] = make_int4((int)pack_bf16x2(a1[0], a1[1]), (int)pack_bf16x2(a1[2], a1[3]), (int)pack_bf16x2(a1[4], a1[5]),
+                                        (int)pack_bf16x2(a1[6], a1[7]));
+            }
+        }
+        if (stamps) {
+            atomicMax(L.stats + kStatKindLast + kWorkReduce, globaltimer_ns());
+            if (waited) atomicAdd(L.stats + kStatWaitLanded, waited);
+        }
+    };
+
+    // ---------------------------------------------------------------------- worker roles
+    {
+        const int total_items = min(L.meta[kMetaWork + (BWD ? 1 : 0)], L.max_work);
+        const uint32_t ring_addr = bar_base + kOffItems;
+        volatile int* ring = reinterpret_cast<volatile int*>(smem_gen + kBarOffsetP + kOffItems);
+        // consumer side of the item ring (see layer.cu: the second CTA's entries arrive through the async proxy)
+        auto next_item = [&](int& ss, uint32_t& sph, int site, int4& it) -> bool {
+            if (!mbar_wait(ring_full(ss), sph, abort_flag, L.status, site)) return false;
+            it = make_int4(ring[4 * ss], ring[4 * ss + 1], ring[4 * ss + 2], ring[4 * ss + 3]);
+            __syncwarp();
+            if (lane == 0) {
+                if (rank == 0) mbar_arrive(ring_empty(ss));
+                else mbar_arrive_cluster(mapa_shared(ring_empty(ss), 0));
+            }
+            if (++ss == kRingDepth) { ss = 0; sph ^= 1u; }
+            return true;
+        };
+
+        if (warp == 0) {
+            // -------------------------------------------------------------- item fetch (first CTA) + TMA producer
+            if (elect_one()) {
+                int stage = 0;
+                uint32_t phase = 0;
+                bool ok = true;
+                int ss = 0;
+                uint32_t sph = 0;
+                // Both producers look at the NEXT item while the loads of the current one are in flight: they fetch it and test what
+                // its operands wait for, so that between two items there is normally nothing to wait for.
+                int claim = (rank == 0) ? atomicAdd(L.sync + kSyncItem, 1) : 0;
+                unsigned long long w_arrive = 0, w_unit = 0, w_wgrad = 0;
+                bool wgrad_ready = false, wgrad_fenced = false;
+                int4 cur = make_int4(-1, 0, 0, 0), nxt = cur;
+                bool have = false, nxt_ready = false;
+                // 1: got an item, 0: none yet (non-blocking form, second CTA), -1: a wait ran out
+                auto get_item = [&](int4& it, bool blocking) -> int {
+                    if (rank == 0) {
+                        it = (claim < total_items) ? L.work[claim] : make_int4(-1, 0, 0, 0);
+                        if (it.x >= 0) claim = atomicAdd(L.sync + kSyncItem, 1);      // needed when the next item is fetched
+                        if (!mbar_wait(ring_empty(ss), sph ^ 1u, abort_flag, L.status, 650)) return -1;
+                        ring[4 * ss] = it.x; ring[4 * ss + 1] = it.y; ring[4 * ss + 2] = it.z; ring[4 * ss + 3] = it.w;
+                        mbar_arrive(ring_full(ss));
+                        const uint32_t remote_bar = mapa_shared(ring_full(ss), 1);
+                        mbar_arrive_expect_tx_cluster(remote_bar, 16u);
+                        st_async_v4_cluster(mapa_shared(ring_addr + 16u * ss, 1), it, remote_bar);
+                    } else {
+                        if (blocking) {
+                            if (!mbar_wait(ring_full(ss), sph, abort_flag, L.status, 651)) return -1;
+                        } else if (!mbar_try_wait(ring_full(ss), sph)) {
+                            return 0;
+                        }
+                        it = make_int4(ring[4 * ss], ring[4 * ss + 1], ring[4 * ss + 2], ring[4 * ss + 3]);
+                        mbar_arrive_cluster(mapa_shared(ring_empty(ss), 0));
+                    }
+                    if (++ss == kRingDepth) { ss = 0; sph ^= 1u; }
+                    return 1;
+                };
+                auto counted = [&](const int* flag, int target, bool block, int site, unsigned long long& waited) -> int {
+                    if (ld_acquire_gpu(flag) >= target) return 1;
+                    if (!block) return 0;
+                    const uint64_t t0 = globaltimer_ns();
+                    const bool got = wait_count(flag, target, L.status, site, 64);
+                    waited += globaltimer_ns() - t0;
+                    return got ? 1 : -1;
+                };
+                // what the operands of an item wait for; `block`: wait (bounded) instead of only looking
+                auto operands_ready = [&](const Item& q, bool block) -> int {
+                    if (q.kind == kWorkGemm1) return (!q.live || q.need == 0) ? 1 : counted(L.arrived + q.m0 / BM, q.need, block, 600, w_arrive);
+                    if (q.kind == kWorkGemm2) return counted(L.done1 + q.unit, target1, block, 601, w_unit);
+                    // the weight gradients sit behind all first GEMMs in the list: one check per pair is enough
+                    if (wgrad_ready) return 1;
+                    const int a = counted(L.sync + kSyncExpanded, num_slots, block, 603, w_wgrad);
+                    const int b = a == 1 ? counted(L.sync + kSyncUnits, num_units, block, 602, w_wgrad) : a;
+                    wgrad_ready = b == 1;
+                    return b;
+                };
+                auto look_ahead = [&]() -> bool {            // false: a wait ran out
+                    const int r = get_item(nxt, false);
+                    if (r < 0) return false;
+                    if (r == 0) return true;
+                    have = true;
+                    nxt_ready = false;
+                    if (nxt.x >= 0) {
+                        Item qn;
+                        decode_item(L, nxt, rank, qn);
+                        nxt_ready = operands_ready(qn, false) == 1;
+                    }
+                    return true;
+                };
+                while (ok) {
+                    bool cur_ready = false;
+                    if (have) {
+                        cur = nxt;
+                        cur_ready = nxt_ready;
+                        have = false;
+                    } else if (get_item(cur, true) < 0) {
+                        ok = false;
+                        break;
+                    }
+                    if (cur.x < 0) break;
+                    Item q;
+                    decode_item(L, cur, rank, q);
+                    const Phase& P = L.ph[q.kind];
+                    if (!cur_ready && operands_ready(q, true) != 1) { *abort_flag = 1u; ok = false; break; }
+                    // stores of other SMs -> async-proxy reads; the weight gradients acquire once, so they need the fence once
+                    if (q.kind <= kWorkGemm2 || !wgrad_fenced) fence_proxy_async_all();
+                    if (q.kind > kWorkGemm2) wgrad_fenced = true;
+                    const int n0 = q.n_blk * BN + (int)rank * (BN / 2);
+                    const int look_kb = min(kStagesP - 1, q.nk - 1);   // all stages are in flight: a pause of this thread costs nothing
+                    for (int kb = 0; kb < q.nk; ++kb) {
+                        if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag, L.status, 610)) { ok = false; break; }
+                        const uint32_t a_dst = smem_base + stage * kStageBytesP;
+                        const uint32_t b_dst = a_dst + kAStageBytes;
+                        const uint32_t bar = mapa_shared(full_bar(stage), 0);
+                        if (rank == 0) mbar_arrive_expect_tx(full_bar(stage), 2 * kStageBytesP);
+                        else mbar_arrive_cluster(bar);
+                        const int k = q.k0 + kb * BK;
+                        if (q.kind <= kWorkGemm2) {
+                            tma_load_2d_2cta(a_dst, &P.map_a, bar, k, q.live ? q.m0 : L.out_rows);     // no rows: past the end reads zeros
+                            if constexpr (!BWD) {
+                                tma_load_2d_2cta(b_dst, &P.map_b, bar, k, q.group * P.b_group_rows + n0);
+                            } else {
+                                const int krow = q.group * P.b_group_rows + k;
+#pragma unroll
+                                for (int a = 0; a < BN / 128; ++a) tma_load_2d_2cta(b_dst + a * kAtomBytes, &P.map_b, bar, n0 + 64 * a, krow);
+                            }
+                        } else {
+#pragma unroll
+                            for (int a = 0; a < BM / 64; ++a) tma_load_2d_2cta(a_dst + a * kAtomBytes, &P.map_a, bar, q.m0 + 64 * a, k);
+#pragma unroll
+                            for (int a = 0; a < BN / 128; ++a) tma_load_2d_2cta(b_dst + a * kAtomBytes, &P.map_b, bar, n0 + 64 * a, k);
+                        }
+                        if (++stage == kStagesP) { stage = 0; phase ^= 1u; }
+                        // (the second CTA keeps looking until the first one has published the item)
+                        if (kb >= look_kb && !have && (kb == look_kb || rank != 0) && !look_ahead()) { ok = false; break; }
+                    }
+                }
+                if (L.stats != nullptr) {
+                    if (w_arrive) atomicAdd(L.stats + kStatWaitArrival, w_arrive);
+                    if (w_unit) atomicAdd(L.stats + kStatWaitFirstGemm, w_unit);
+                    if (w_wgrad) atomicAdd(L.stats + kStatWaitWgrad, w_wgrad);
+                }
+            }
+        } else if (warp == 1 && rank == 0) {
+            // -------------------------------------------------------------- UMMA issuer
+            int stage = 0;
+            uint32_t phase = 0;
+            bool ok = true;
+            int ss = 0;
+            uint32_t sph = 0;
+            int iter = 0;
+            while (ok) {
+                int4 it;
+                if (!next_item(ss, sph, 652, it) || it.x < 0) break;
+                Item q;
+                decode_item(L, it, rank, q);
+                const bool a_mn = q.kind >= kWorkWgradDown;
+                const uint32_t idesc = BWD ? (a_mn ? make_idesc_bf16(2 * BM, BN, true, true) : make_idesc_bf16(2 * BM, BN, false, true))
+                                           : make_idesc_bf16(2 * BM, BN, false, false);
+                const int as = iter & 1;
+                const uint32_t aphase = (iter >> 1) & 1;
+                ++iter;
+                if (!mbar_wait(tempty_bar(as), aphase ^ 1u, abort_flag, L.status, 620)) { ok = false; break; }
+                tcgen05_fence_after();
+                const uint32_t d_tmem = tmem_base + (uint32_t)(as * BN);
+                for (int kb = 0; kb < q.nk; ++kb) {
+                    if (!mbar_wait(full_bar(stage), phase, abort_flag, L.status, 621)) { ok = false; break; }
+                    tcgen05_fence_after();
+                    if (elect_one()) {
+                        const uint32_t a_addr = smem_base + stage * kStageBytesP;
+                        const uint32_t b_addr = a_addr + kAStageBytes;
+#pragma unroll
+                        for (int k = 0; k < BK / UK; ++k) {
+                            const uint64_t a_desc = a_mn ? make_smem_desc_sw128(a_addr + k * (UK * 128), kAtomBytes, 1024)
+                                                         : make_smem_desc_sw128(a_addr + k * (UK * 2), 0, 1024);
+                            const uint64_t b_desc = BWD ? make_smem_desc_sw128(b_addr + k * (UK * 128), kAtomBytes, 1024)
+                                                        : make_smem_desc_sw128(b_addr + k * (UK * 2), 0, 1024);
+                            umma_bf16_ss_2cta(d_tmem, a_desc, b_desc, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+                        }
+                        umma_commit_2cta(empty_bar(stage), 3u);
+                        if (kb == q.nk - 1) umma_commit_2cta(tfull_bar(as), 3u);
+                    }
+                    __syncwarp();
+                    if (++stage == kStagesP) { stage = 0; phase ^= 1u; }
+                }
+                if (ok && q.nk == 0) {                       // an expert without rows: the epilogue stores zeros
+                    if (elect_one()) umma_commit_2cta(tfull_bar(as), 3u);
+                    __syncwarp();
+                }
+            }
+        } else if (warp >= 4) {
+            // -------------------------------------------------------------- epilogue, then gather
+            const int qd = warp & 3;
+            const int hh = (warp - 4) >> 2;
+            const Staging st{smem_base + kPipeBytesP + (uint32_t)(warp - 4) * kBoxBytes, lane};
+            bool ok = true;
+            int ss = 0;
+            uint32_t sph = 0;
+            int iter = 0;
+            int owed_kind = -1, owed_at = 0;        // tile whose stores are not yet counted as complete
+            // Count the tile of the previous item: done right before this warp would wait for the next accumulator, when its stores
+            // have normally completed.  (Never behind that wait: the next item may be the one that waits for this count.)
+            auto flush = [&]() {
+                if (owed_kind < 0) return;
+                __syncwarp();
+                if (lane == 0) {
+                    tma_store_wait<0>();
+                    fence_proxy_async_all();
+                    fence_acq_rel_gpu();
+                    if (owed_kind == kWorkGemm1) {
+                        if (atom_add_acq_rel(L.done1 + owed_at, 1) == target1 - 1) red_add_release_gpu(L.sync + kSyncUnits, 1);
+                    } else {
+                        red_add_release_gpu(L.done2 + owed_at, 1);
+                    }
+                }
+                owed_kind = -1;
+            };
+            while (ok) {
+                int4 it;
+                flush();
+                if (!next_item(ss, sph, 653, it) || it.x < 0) break;
+                const bool stamps = L.stats != nullptr && warp == 4 && lane == 0 && rank == 0;
+                Item q;
+                decode_item(L, it, rank, q);
+                if (stamps) atomicMax(L.stats + kStatKindFirst + q.kind, ~globaltimer_ns());
+                const int as = iter & 1;
+                const uint32_t aphase = (iter >> 1) & 1;
+                ++iter;
+                if (!mbar_wait(tfull_bar(as), aphase, abort_flag, L.status, 630)) { ok = false; break; }
+                tcgen05_fence_after();
+                const uint32_t taddr = tmem_base + ((uint32_t)(qd * 32) << 16) + (uint32_t)(as * BN + hh * (BN / 2));
+                const int n0 = q.n_blk * BN + hh * (BN / 2);
+                const int row0 = q.m0 + qd * 32;
+                if (q.kind == kWorkGemm1) {
+                    if constexpr (BWD) epilogue_dswiglu(L, st, taddr, row0, q.live, n0, q.n_blk * 2 + hh);
+                    else epilogue_swiglu(L, st, taddr, row0, q.live, n0);
+                } else if (q.kind == kWorkGemm2) {
+                    epilogue_plain(st, taddr, false, [&](int c) {
+                        st.store(q.live && n0 + c < L.H, &L.st_y, n0 + c, row0);
+                    });
+                    if constexpr (BWD) {
+                        if (q.live && q.n_blk == 0 && hh == 0) {
+                            // this row's d(route weight): the sum of the first GEMM's partials
+                            const long row = row0 + lane;
+                            const int tk = L.slot_tk[row];
+                            if (tk >= 0) {
+                                float v = 0.f;
+                                for (int p = 0; p < L.n_parts; ++p) v += __ldcg(L.droute_part + row * L.n_parts + p);
+                                L.dw_topk[tk] = v;
+                            }
+                        }
+                    }
+                } else {
+                    if constexpr (BWD) {
+                        const Phase& P = L.ph[q.kind];
+                        const CUtensorMap* map = q.kind == kWorkWgradDown ? &L.st_dwd : &L.st_dwg;
+                        const int m = q.m_in_group + qd * 32;
+                        epilogue_plain(st, taddr, q.nk == 0, [&](int c) {
+                            st.store3(m < P.m_total && n0 + c < P.n_total, map, n0 + c, m, q.group);
+                        });
+                    }
+                }
+                tcgen05_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive_cluster(mapa_shared(tempty_bar(as), 0));
+                if (stamps) atomicMax(L.stats + kStatKindLast + q.kind, globaltimer_ns());
+                if (q.kind == kWorkGemm1 || (q.kind == kWorkGemm2 && q.live)) {
+                    owed_kind = q.kind;
+                    owed_at = q.kind == kWorkGemm1 ? q.unit : q.m0 / BM;
+                }
+            }
+            flush();
+            if (lane == 0) tma_store_wait<0>();
+            __syncwarp();
+            if (ok) gather_loop();            // the list is done: help with the sums
+        } else if (warp >= 2) {
+            if constexpr (BWD) {
+                expand_loop();
+            } else {
+                clear_all_padding();
+                if (L.saved_x != nullptr) copy_x_loop();
+            }
+            gather_loop();
+        }
+    }
+
+    tcgen05_fence_before();
+    cluster_sync_all();
+    if (warp == 2) {
+        tcgen05_fence_after();
+        tmem_dealloc_2cta(tmem_base, kTmemCols);
+    }
+}
+
+// [rows, cols] bf16, boxes of 32 rows x 32 columns, 64-byte swizzle
+cudaError_t make_map_narrow(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols) {
+    EncodeTiledFn fn = get_encode_fn();
+    if (fn == nullptr) return cudaErrorNotSupported;
+    if ((reinterpret_cast<uintptr_t>(base) & 15u) != 0) return cudaErrorInvalidValue;
+    cuuint64_t dims[2] = {cols, rows};
+    cuuint64_t strides[1] = {cols * 2};
+    cuuint32_t box[2] = {32, 32};
+    cuuint32_t estr[2] = {1, 1};
+    const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
+                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
+}
+
+// [groups, rows, cols] bf16, boxes of 32 rows x 64 columns of one group; rows and columns outside a group are not written
+cudaError_t make_store_map3(CUtensorMap* map, const void* base, uint64_t groups, uint64_t rows, uint64_t cols) {
+    EncodeTiledFn fn = get_encode_fn();
+    if (fn == nullptr) return cudaErrorNotSupported;
+    if ((reinterpret_cast<uintptr_t>(base) & 15u) != 0) return cudaErrorInvalidValue;
+    cuuint64_t dims[3] = {cols, rows, groups};
+    cuuint64_t strides[2] = {cols * 2, rows * cols * 2};
+    cuuint32_t box[3] = {64, 32, 1};
+    cuuint32_t estr[3] = {1, 1, 1};
+    const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
+                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
+}
+
+template <bool BWD>
+cudaError_t launch(const LayerArgsP& L, int num_sms, cudaStream_t stream) {
+    auto kern = local_layer_kernel<BWD>;
+    static bool configured[64] = {};
+    if (cudaError_t e = ensure_smem_limit(kern, kSmemBytesP, configured); e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(num_sms & ~1);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = kSmemBytesP;
+    cfg.stream = stream;
+    // workers wait for rows that the dispatch pairs copy and for tiles of other pairs: all of them have to be resident
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, L);
+}
+
+}  // namespace
+
+LocalLayerPlan local_layer_plan(int T, int K, int E, int H, int I, int keep) {
+    LocalLayerPlan p{};
+    p.T = T; p.K = K; p.E = E; p.H = H; p.I = I; p.keep = keep;
+    p.chunks = (T + kRouteThreads - 1) / kRouteThreads;
+    const long entries = (long)T * K, segs = entries < E ? entries : E;
+    p.blocks_cap = (int)((entries + 127 * segs) / 128);
+    p.slots_cap = p.blocks_cap * 128;
+    p.units_cap = (int)((p.blocks_cap + segs) / 2);
+    const int nbH = (H + BN - 1) / BN, nbI = (I + BN - 1) / BN, nb2I = (2 * I + BN - 1) / BN;
+    p.work_cap[0] = p.units_cap * (nb2I + nbH);
+    p.work_cap[1] = keep ? p.units_cap * (nbI + nbH) + E * (((H + 2 * BM - 1) / (2 * BM)) * nbI + ((2 * I + 2 * BM - 1) / (2 * BM)) * nbH) : 0;
+    long at = 0;
+    auto take = [&](long n) {
+        const long o = at;
+        at += (n + 3) / 4 * 4;
+        return o;
+    };
+    const int dirs = keep ? 2 : 1;
+    for (int d = 0; d < dirs; ++d) {
+        p.stats[d] = take(2 * kLayerStatWords);
+        p.sync[d] = take(kSyncWords);
+        p.done1[d] = take(p.units_cap);
+        p.done2[d] = take(p.blocks_cap);
+        p.arrived[d] = take(p.blocks_cap);
+    }
+    p.totals = take(E);
+    p.last_hist = take(E + 1);
+    p.zero_words = at;
+    p.meta = take(4);
+    p.seg = take(E + 1);
+    p.slot_tk = take(p.slots_cap);
+    p.slot_w = take(p.slots_cap);
+    p.token_order = take(T);
+    p.order_slot = take(entries);
+    p.chunk_hist = take((long)p.chunks * E);
+    p.chunk_last = take((long)p.chunks * (E + 1));
+    for (int d = 0; d < dirs; ++d) p.work[d] = take(4l * p.work_cap[d]);
+    p.words = at;
+    return p;
+}
+
+cudaError_t local_layer_route(const LocalLayerParams& q, cudaStream_t stream) {
+    const LocalLayerPlan& p = q.plan;
+    if (p.E < 1 || p.E > kLocalMaxExperts || p.K < 1 || p.K > 32 || q.group_units <= 0 || q.lag_percent < 0 || q.lag_percent > 100)
+        return cudaErrorInvalidValue;
+    RouteArgs a{};
+    a.p = p;
+    a.ws = q.ws; a.topk_idx = q.topk_idx; a.is64 = q.idx_is64; a.topk_w = q.topk_w;
+    a.nb1[0] = (2 * p.I + BN - 1) / BN;
+    a.nb1[1] = (p.I + BN - 1) / BN;
+    a.nb2 = (p.H + BN - 1) / BN;
+    a.mu_wd = (p.H + 2 * BM - 1) / (2 * BM); a.nb_wd = (p.I + BN - 1) / BN;
+    a.mu_wg = (2 * p.I + 2 * BM - 1) / (2 * BM); a.nb_wg = (p.H + BN - 1) / BN;
+    a.group_units = q.group_units; a.lag_percent = q.lag_percent; a.min_lag_items = q.min_lag_items > 0 ? q.min_lag_items : 0;
+    cudaError_t e = cudaMemsetAsync(q.ws, 0, (size_t)p.zero_words * sizeof(int), stream);
+    if (e != cudaSuccess) return e;
+    if (p.chunks > 0) {
+        local_route_count_kernel<<<p.chunks, kRouteThreads, (2 * p.E + 1) * sizeof(int), stream>>>(a);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    }
+    // 64 blocks at least: the lists (tens of thousands of items for a large layer) are written by all blocks
+    const int grid = p.chunks > 64 ? p.chunks : 64;
+    local_route_assign_kernel<<<grid, kRouteThreads, (3 * (p.E + 1) + kRouteWarps * (2 * p.E + 1)) * sizeof(int), stream>>>(a);
+    return cudaGetLastError();
+}
+
+cudaError_t local_layer_launch(const LocalLayerParams& q, cudaStream_t stream) {
+    const LocalLayerPlan& p = q.plan;
+    const int H = p.H, I = p.I, E = p.E, dir = q.bwd ? 1 : 0;
+    if (H % BK != 0 || I % BK != 0 || q.out_rows % BM != 0 || q.out_rows < BM || q.out_rows < p.slots_cap || p.K < 1 || p.K > 32 || (q.bwd && !p.keep))
+        return cudaErrorInvalidValue;
+    if (reinterpret_cast<uintptr_t>(q.x) % 16 != 0 || reinterpret_cast<uintptr_t>(q.slot_x) % 16 != 0) return cudaErrorInvalidValue;
+    const uint64_t R = (uint64_t)q.out_rows;
+    LayerArgsP L{};
+    cudaError_t e;
+    // The tensor-map encoder wants a current context; a thread that has not used the device yet (an autograd worker whose
+    // allocations were all served from the cache) has none until the runtime binds it.
+    int dev = 0;
+    if ((e = cudaGetDevice(&dev)) != cudaSuccess || (e = cudaSetDevice(dev)) != cudaSuccess) return e;
+    Phase& g1 = L.ph[kWorkGemm1];
+    Phase& g2 = L.ph[kWorkGemm2];
+    g1.nk = H / BK;
+    g2.n_total = H; g2.num_n_blocks = (H + BN - 1) / BN;
+    if ((e = make_map(&g1.map_a, q.slot_x, R, H, BK, BM)) != cudaSuccess) return e;
+    if ((e = q.bwd ? make_map_narrow(&L.st_act, q.act, R, I) : make_map(&L.st_act, q.act, R, I, 64, 32)) != cudaSuccess) return e;
+    if ((e = make_map(&L.st_y, q.y, R, H, 64, 32)) != cudaSuccess) return e;
+    if (!q.bwd) {
+        // gate_up: A = rows in slot order, B = W_gateup [E*2I, H] K-major;  down: A = act, B = W_down [E*H, I] K-major
+        if ((e = make_map(&g1.map_b, q.w_gateup, (uint64_t)E * 2 * I, H, BK, BN / 2)) != cudaSuccess) return e;
+        if ((e = make_map(&g2.map_a, q.act, R, I, BK, BM)) != cudaSuccess) return e;
+        if ((e = make_map(&g2.map_b, q.w_down, (uint64_t)E * H, I, BK, BN / 2)) != cudaSuccess) return e;
+        g1.n_total = 2 * I; g1.b_group_rows = 2 * I;
+        g2.nk = I / BK; g2.b_group_rows = H;
+        if (p.keep && (e = make_map(&L.st_aux, q.aux, R, 2 * I, 64, 32)) != cudaSuccess) return e;
+    } else {
+        // grad_act: A = dY, B = W_down MN-major;  dX: A = dGU, B = W_gateup MN-major
+        if ((e = make_map(&g1.map_b, q.w_down, (uint64_t)E * H, I, 64, BK)) != cudaSuccess) return e;
+        if ((e = make_map(&g2.map_a, q.aux, R, 2 * I, BK, BM)) != cudaSuccess) return e;
+        if ((e = make_map(&g2.map_b, q.w_gateup, (uint64_t)E * 2 * I, H, 64, BK)) != cudaSuccess) return e;
+        g1.n_total = I; g1.b_group_rows = H;
+        g2.nk = 2 * I / BK; g2.b_group_rows = 2 * I;
+        if ((e = make_map(&L.st_aux, q.aux, R, 2 * I, 64, 32)) != cudaSuccess) return e;
+        // dW_down[e] = dY[seg]^T . act_w[seg]  ([H, I]);  dW_gateup[e] = dGU[seg]^T . X[seg]  ([2I, H])
+        Phase& gd = L.ph[kWorkWgradDown];
+        Phase& gg = L.ph[kWorkWgradGateup];
+        if ((e = make_map(&gd.map_a, q.slot_x, R, H, 64, BK)) != cudaSuccess) return e;
+        if ((e = make_map(&gd.map_b, q.act, R, I, 64, BK)) != cudaSuccess) return e;
+        if ((e = make_map(&gg.map_a, q.aux, R, 2 * I, 64, BK)) != cudaSuccess) return e;
+        if ((e = make_map(&gg.map_b, q.xperm, R, H, 64, BK)) != cudaSuccess) return e;
+        gd.m_total = H; gd.n_total = I; gd.num_n_blocks = (I + BN - 1) / BN;
+        gg.m_total = 2 * I; gg.n_total = H; gg.num_n_blocks = (H + BN - 1) / BN;
+        if ((e = make_store_map3(&L.st_dwd, q.dw_down, E, H, I)) != cudaSuccess) return e;
+        if ((e = make_store_map3(&L.st_dwg, q.dw_gateup, E, 2 * I, H)) != cudaSuccess) return e;
+    }
+    g1.num_n_blocks = (g1.n_total + BN - 1) / BN;
+    L.T = p.T; L.K = p.K; L.H = H; L.I = I; L.E = E; L.keep = p.keep; L.out_rows = q.out_rows;
+    L.x = static_cast<const uint8_t*>(q.x);
+    L.slot_x = static_cast<uint8_t*>(q.slot_x);
+    L.y = static_cast<const __nv_bfloat16*>(q.y);
+    L.saved_x = static_cast<__nv_bfloat16*>(q.saved_x);
+    L.xperm = static_cast<__nv_bfloat16*>(q.xperm);
+    L.out = static_cast<__nv_bfloat16*>(q.out);
+    L.preact = static_cast<const __nv_bfloat16*>(q.preact);
+    L.droute_part = q.droute_part;
+    L.n_parts = 2 * ((I + BN - 1) / BN);
+    L.dw_topk = q.dw_topk;
+    L.meta = q.ws + p.meta;
+    L.seg = q.ws + p.seg;
+    L.totals = q.ws + p.totals;
+    L.slot_tk = q.ws + p.slot_tk;
+    L.slot_w = reinterpret_cast<const float*>(q.ws + p.slot_w);
+    L.token_order = q.ws + p.token_order;
+    L.order_slot = q.ws + p.order_slot;
+    L.work = reinterpret_cast<const int4*>(q.ws + p.work[dir]);
+    L.max_work = p.work_cap[dir];
+    L.max_units = p.units_cap;
+    L.sync = q.ws + p.sync[dir];
+    L.done1 = q.ws + p.done1[dir];
+    L.done2 = q.ws + p.done2[dir];
+    L.arrived = q.ws + p.arrived[dir];
+    L.stats = reinterpret_cast<unsigned long long*>(q.ws + p.stats[dir]);
+    L.status = q.status;
+    const int sms = default_sms(q.num_sms) & ~1;
+    if (sms < 4) return cudaErrorInvalidConfiguration;
+    L.dispatch_pairs = q.dispatch_pairs < 1 ? 1 : q.dispatch_pairs > sms / 2 - 1 ? sms / 2 - 1 : q.dispatch_pairs;
+    return q.bwd ? launch<true>(L, sms, stream) : launch<false>(L, sms, stream);
+}
+
+}  // namespace tmoe

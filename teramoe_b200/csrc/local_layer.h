@@ -1,0 +1,59 @@
+// The MoE layer on one rank (local_layer.cu): routing preparation in two launches, then ONE cooperative persistent kernel per
+// direction.  Same work list, tiles and summation orders as the kernel for several ranks (layer.h), so both give the same
+// bits; what differs is everything that only a second rank needs (peer tables, completion flags, landing rows).
+#pragma once
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+namespace tmoe {
+
+constexpr int kLocalMaxExperts = 512;    // the routing kernels keep 19 words per expert in shared memory
+
+// Word offsets of the tables of one call inside its int32 workspace.  Capacities follow from the sizes alone (T * K entries in
+// at most min(E, T * K) segments padded to 128 rows), so the host never has to read the layout back.
+struct LocalLayerPlan {
+    int T, K, E, H, I, keep;             // keep: tables of the backward pass too
+    int chunks;                          // blocks of the routing kernels
+    int slots_cap, blocks_cap, units_cap;
+    int work_cap[2];                     // items of the forward / backward list
+    // zero-filled by local_layer_route
+    long stats[2], sync[2], totals, last_hist, done1[2], done2[2], arrived[2], zero_words;
+    // written by it
+    long meta, seg, slot_tk, slot_w, token_order, order_slot, chunk_hist, chunk_last, work[2], words;
+};
+LocalLayerPlan local_layer_plan(int T, int K, int E, int H, int I, int keep);
+
+struct LocalLayerParams {
+    LocalLayerPlan plan;
+    int* ws;                             // plan.words int32
+    const void* topk_idx;
+    int idx_is64;
+    const float* topk_w;                 // forward
+    // schedule
+    int group_units, lag_percent, min_lag_items, dispatch_pairs, num_sms;
+    int bwd;
+    const void* x;                       // [T, H] forward x, backward grad_out
+    const void* w_gateup;
+    const void* w_down;
+    void* slot_x;                        // [out_rows, H] rows in slot order
+    void* y;                             // [out_rows, H] second GEMM's output in slot order
+    int out_rows;                        // rows of the slot-order tensors: max(slots_cap, 128)
+    void* act;                           // forward act, backward act x route [out_rows, I]
+    void* aux;                           // forward preact (may be null without keep), backward dGU [out_rows, 2I]
+    void* saved_x;                       // [T, H] copy of x: written by forward (may be null), read by backward
+    void* out;                           // [T, H]
+    // backward
+    const void* preact;
+    float* droute_part;                  // [out_rows, 2 * ceil(I / 256)]
+    void* xperm;                         // [out_rows, H]
+    float* dw_topk;                      // [T, K]
+    void* dw_gateup;
+    void* dw_down;
+    int* status;
+};
+
+// Routing tables and both work lists (p: plan, ws, topk_*, schedule).
+cudaError_t local_layer_route(const LocalLayerParams& p, cudaStream_t stream);
+cudaError_t local_layer_launch(const LocalLayerParams& p, cudaStream_t stream);
+
+}  // namespace tmoe

@@ -127,6 +127,10 @@ LAUNCH_AHEAD = os.environ.get("TERAMOE_LAUNCH_AHEAD", "1") == "1"
 LAYER_WIRE = os.environ.get("TERAMOE_WIRE", "entry")
 if LAYER_WIRE not in ("entry", "rank"):
     raise ValueError(f"TERAMOE_WIRE must be 'entry' or 'rank', not {LAYER_WIRE!r}")
+# One rank: the routing kernels and the layer kernel of csrc/local_layer.cu, launched by one native call per direction
+# ("0": the kernels that several ranks use).
+_LOCAL_LAYER_MODE = os.environ.get("TERAMOE_LOCAL_LAYER", "auto")
+LOCAL_LAYER_MAX_EXPERTS = 512    # csrc/local_layer.h kLocalMaxExperts
 LAYER_REDUCE_CHUNK = 64          # tokens per reduce item
 LAYER_MIN_LAG_PER_PAIR = float(os.environ.get("TERAMOE_LAYER_MIN_LAG", "2"))
 
@@ -205,6 +209,30 @@ class LocalHandle:
 
 
 @dataclass
+class LocalLayerHandle:
+    """What backward needs of a one-rank layer call: its int32 workspace (csrc/local_layer.h) and its sizes."""
+    T: int
+    K: int
+    E: int
+    H: int
+    I: int
+    ws: torch.Tensor
+    schedule: list
+
+
+class _LazyStats(dict):
+    """Per-call numbers that are read back from the device when somebody asks for them."""
+
+    def __init__(self, read):
+        super().__init__()
+        self._read = read
+
+    def __missing__(self, key):
+        self.update(self._read())
+        return dict.__getitem__(self, key)
+
+
+@dataclass
 class SavedForBackward:
     handle: LayerHandle
     saved_x: torch.Tensor        # [rows, H]
@@ -239,6 +267,7 @@ class EPEngine:
         self.world = world
         self.is_cuda = world.is_cuda
         self.ext = world.ext if self.is_cuda else None
+        self._num_sms = torch.cuda.get_device_properties(world.device).multi_processor_count if self.is_cuda else 0
         self._trace = None          # list of (phase name, CUDA event) while tracing
         self._caps = {}             # (K, E, N) -> (rows, slots, tokens) capacities learnt from earlier calls (layout_gen)
         self.last_wait_ns = {}      # whole-layer kernel: {0: forward, 1: backward} -> int64[8] wait counters (csrc/layer.h LayerStat)
@@ -608,6 +637,73 @@ class EPEngine:
             out.copy_((land * ww[:, :, None]).sum(1).to(y.dtype))
         return out
 
+    # ------------------------------------------------------------------ layer on one rank (csrc/local_layer.cu)
+    def use_local_layer(self, T: int, K: int, E: int, H: int, I: int, opts: dict) -> bool:
+        """One real rank, sizes that the kernels take, and no switch that asks for other kernels."""
+        w = self.world
+        return (self.is_cuda and w.size == 1 and w.virtual_peers is None and USE_CTA_PAIRS and not USE_TMA_GATHER
+                and "0" not in (_LOCAL_LAYER_MODE, _LAYER_KERNEL_MODE, _FUSED_DISPATCH_MODE, _FUSED_MODE)
+                and (opts.get("wire") or LAYER_WIRE) == "entry" and 1 <= K and E <= LOCAL_LAYER_MAX_EXPERTS
+                and (T * K + 128 * min(E, T * K)) * H * 2 <= FUSED_DISPATCH_MAX_BYTES)
+
+    def _local_schedule(self, opts: dict, kind: int) -> list:
+        """[units per batch, lag percent, least lag in items, dispatch pairs, SMs], see layer_kernel_gen."""
+        num_sms = self._grid_sms(opts)
+        sms = num_sms or self._num_sms
+        return [max(1, int(opts.get("compute_batch_size", 2048)) // UNIT_ROWS), int(opts.get("combine_start_head_percent", 70)),
+                int(LAYER_MIN_LAG_PER_PAIR * (sms // 2)), dispatch_pairs(kind, int(opts.get("num_dispatch_sms", 0))), num_sms]
+
+    def _local_arena(self, T: int, K: int, E: int, H: int):
+        w = self.world
+        need = self.ext.local_layer_arena_bytes(T, K, E, H)
+        if need > w.data_bytes:
+            w.ensure_data(need)
+        w.arena_user = "tables"
+        return w.data.local_ptr(), w.data_bytes
+
+    def local_forward(self, x, topk_idx, topk_weights, W_gateup, W_down, keep_for_backward, opts):
+        """-> (out [T,H], SavedForBackward | None).  Two routing launches and one kernel; the host waits for nothing."""
+        w = self.world
+        w.poll_status()
+        T, H = x.shape
+        K, E, I = topk_idx.shape[1], W_gateup.shape[0], W_gateup.shape[1] // 2
+        self._mark("fwd:start")
+        schedule = self._local_schedule(opts, 0)
+        arena, arena_bytes = self._local_arena(T, K, E, H)
+        out, ws, preact, saved_x = self.ext.local_layer_forward(x, topk_idx, topk_weights, W_gateup, W_down, schedule, keep_for_backward, arena,
+                                                                arena_bytes, w.status)
+        self._mark("fwd:layer (routing, dispatch, gate_up, down, sum)")
+        w.note_status()
+        self.last_paths = {"fused_dispatch_gemm": True, "cta_pairs": True, "fused_combine_fwd": True, "fused_combine_bwd": True,
+                           "layer_kernel": True}
+        h = LocalLayerHandle(T, K, E, H, I, ws, schedule)
+        self.last_wait_ns[0] = (h, keep_for_backward)
+        if not keep_for_backward:
+            return out, None
+        return out, SavedForBackward(h, saved_x, preact, stats=_LazyStats(lambda: self._local_stats(h)))
+
+    def local_backward(self, saved: "SavedForBackward", grad_out, W_gateup, W_down):
+        """-> (dx, d(topk_weights), dW_gateup, dW_down)."""
+        w, h = self.world, saved.handle
+        w.poll_status()
+        self._mark("bwd:start")
+        arena, arena_bytes = self._local_arena(h.T, h.K, h.E, h.H)
+        schedule = h.schedule[:3] + [dispatch_pairs(1, 2 * h.schedule[3] if _pairs_env is None else 0)] + h.schedule[4:]
+        res = self.ext.local_layer_backward(grad_out, h.ws, saved.preact, saved.saved_x, W_gateup, W_down, h.K, schedule, arena, arena_bytes, w.status)
+        self._mark("bwd:layer (dispatch, grad_act, dX, weight gradients, sum)")
+        w.note_status()
+        self.last_wait_ns[1] = (h, True)
+        return res
+
+    def _local_words(self, h: "LocalLayerHandle", keep: bool) -> dict:
+        return self.ext.local_layer_words(h.T, h.K, h.E, h.H, h.I, keep)
+
+    def _local_stats(self, h: "LocalLayerHandle") -> dict:
+        at = self._local_words(h, True)
+        per_expert = h.ws[at["totals"]: at["totals"] + h.E].clone()
+        return {"tokens": h.T, "rows_received": h.T, "slots": int(h.ws[at["meta"] + 1]), "per_expert_rows": per_expert, "paths": dict(self.last_paths),
+                "dispatch_bytes": int(h.ws[at["meta"] + 1]) * h.H * 2, "combine_bytes": h.T * h.K * h.H * 2}
+
     # ------------------------------------------------------------------ layer forward / backward
     def forward_gen(self, x, topk_idx, topk_weights, W_gateup, W_down, num_experts, keep_for_backward=True, impl=None, num_sms=0):
         w = self.world
@@ -710,6 +806,9 @@ class EPEngine:
         rep = {}
         pairs = max(1, torch.cuda.get_device_properties(self.world.device).multi_processor_count // 2) if self.is_cuda else 1
         for kind, t in self.last_wait_ns.items():
+            if isinstance(t, tuple):                # one-rank layer: the counters sit in the call's workspace
+                at = self._local_words(*t)["stats"][kind]
+                t = t[0].ws[at: at + 48].view(torch.int64)
             v = t.tolist()
             d = {n: round(v[i] / 1e6 / (pairs if i < 3 else pairs * 2), 4) for i, n in enumerate(names)}
             # when the epilogues took the first / finished the last item of every kind, relative to the first item at all
@@ -737,7 +836,7 @@ class EPEngine:
         total = int((impl or {}).get("total_sms", 0))
         if not self.is_cuda or total <= 0:
             return 0
-        have = torch.cuda.get_device_properties(self.world.device).multi_processor_count
+        have = self._num_sms
         return 0 if total >= have else max(4, total & ~1)
 
     def fused_dispatch_gemm_gen(self, h: LayerHandle, rows_in, topk_weights, weights, kind: int, preact=None, num_sms=0,

@@ -28,7 +28,6 @@ from typing import Dict, Generator, List, Optional
 import torch
 import torch.distributed as dist
 
-STATUS_RING = 64                 # status snapshots in flight before the oldest is waited for
 STRICT_STATUS = os.environ.get("TERAMOE_STRICT_STATUS", "0") == "1"
 CONTROL_ROW_INTS = 8192          # capacity of one metadata row (E + ranks + 2 ints must fit)
 MAX_BLOCKS = 65536               # per-block arrival counters of the fused dispatch (8.4 M slot rows)
@@ -73,9 +72,10 @@ class EPWorld:
             # status block (csrc/ptx.cuh): words 0-3 error record, words 4-5 the limit (ns) of waits on other ranks
             self.status = torch.zeros(8, dtype=torch.int32, device=self.device)
             self.sizes_host = torch.zeros(12, dtype=torch.int32).pin_memory()
-            self._status_ring = torch.zeros(STATUS_RING, 4, dtype=torch.int32).pin_memory()
-            self._status_pending: list = []          # (ring row, event) of status snapshots not looked at yet
-            self._status_next = 0
+            # pinned copy of words 0-3 that kernels write themselves (words 6-7 hold its address): looking at it is one host read
+            self._status_pinned = torch.zeros(4, dtype=torch.int32).pin_memory()
+            self._status_host = self._status_pinned.numpy()
+            self.status[6:8].view(torch.int64).fill_(self._status_pinned.data_ptr())
             ms = int(os.environ.get("TERAMOE_PEER_WAIT_LIMIT_MS", "0"))
             if ms > 0:
                 self.set_wait_limit_ms(ms)
@@ -177,7 +177,7 @@ class EPWorld:
 
     def _raise_status(self, s) -> None:
         self.status[:4].zero_()
-        self._status_pending.clear()
+        self._status_host[:] = 0
         names = {1: "mbarrier wait", 2: "flag wait", 3: "barrier", 4: "bad argument"}
         raise RuntimeError(f"teramoe_b200: a device-side wait ran out on rank {self.rank}: {names.get(s[0], s[0])} "
                            f"(site {s[1]}, block {s[2]}, detail {s[3]})")
@@ -187,40 +187,22 @@ class EPWorld:
         if not self.is_cuda:
             return
         s = self.status[:4].tolist()
-        self._status_pending.clear()
         if s[0] != 0:
             self._raise_status(s)
 
     def note_status(self, strict: Optional[bool] = None) -> None:
-        """End of a call: snapshot the status block into pinned memory behind the call's kernels (16 bytes, no host
-        wait).  Snapshots are looked at by poll_status (every later call does that first) and by check_status; with
-        `strict` (or TERAMOE_STRICT_STATUS=1) the host waits for this snapshot, so the call whose wait ran out is the one
-        that raises, at the price of one stream wait per call."""
+        """End of a call.  With `strict` (or TERAMOE_STRICT_STATUS=1) the host waits for the call's kernels, so the call whose
+        wait ran out is the one that raises; otherwise a later call does (poll_status)."""
         if not self.is_cuda:
             return
-        if len(self._status_pending) >= STATUS_RING:
-            row, ev = self._status_pending.pop(0)
-            ev.synchronize()
-            if int(self._status_ring[row, 0]) != 0:
-                self._raise_status(self._status_ring[row].tolist())
-        row = self._status_next
-        self._status_next = (row + 1) % STATUS_RING
-        self._status_ring[row].copy_(self.status[:4], non_blocking=True)
-        ev = torch.cuda.Event()
-        ev.record()
-        self._status_pending.append((row, ev))
         if self.strict_status if strict is None else strict:
-            ev.synchronize()
+            torch.cuda.current_stream(self.device).synchronize()
         self.poll_status()
 
     def poll_status(self) -> None:
-        """Look at the snapshots whose copies have completed; never waits."""
-        if not self.is_cuda:
-            return
-        while self._status_pending and self._status_pending[0][1].query():
-            row, _ = self._status_pending.pop(0)
-            if int(self._status_ring[row, 0]) != 0:
-                self._raise_status(self._status_ring[row].tolist())
+        """Raise if a kernel has reported a wait that ran out; never waits."""
+        if self.is_cuda and self._status_host[0] != 0:
+            self._raise_status(self._status_host.tolist())
 
     # ------------------------------------------------------------------ arena reuse between calls
     # Peers store into this rank's data arena and every call reuses it.  The rule that makes this safe: a rank

@@ -1,0 +1,62 @@
+"""The one-rank layer (csrc/local_layer.cu) against the kernels that several ranks use, bit for bit (same slots, tiles and order
+of every sum), and against the fp32 oracle."""
+import pytest
+import torch
+
+import teramoe_b200 as tm
+from teramoe_b200.utils.numerics import assert_close_bf16
+from helpers import make_problem, oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def _run(buf, prob, idx, E, **kw):
+    r = prob["ranks"][0]
+    x = r["x"].clone().requires_grad_(True)
+    w = r["w"].clone().requires_grad_(True)
+    Wg = prob["W_gateup"].clone().requires_grad_(True)
+    Wd = prob["W_down"].clone().requires_grad_(True)
+    out = buf.teramoe_autograd(x, idx, w, Wg, Wd, E, **kw)
+    out.backward(r["go"])
+    fwd = buf.teramoe_forward(r["x"], idx, r["w"], prob["W_gateup"], prob["W_down"], E, **kw)
+    torch.cuda.synchronize()
+    return {"out": out.detach(), "dx": x.grad, "dw": w.grad, "dWg": Wg.grad, "dWd": Wd.grad, "forward only": fwd}
+
+
+@pytest.mark.parametrize("T,H,I,E,K,skew,kw", [
+    (1, 64, 64, 1, 1, False, {}),                        # the smallest sizes: one tile, mostly outside
+    (3, 256, 128, 300, 8, False, {}),                    # far more experts than entries
+    (128, 512, 192, 2, 2, False, {}),                    # exactly one full block per expert, half a column block
+    (129, 320, 320, 2, 2, False, {}),                    # one row more
+    (257, 1088, 704, 5, 3, True, {"stage": 2}),          # three chunks' worth of ragged segments, columns past every tile edge
+    (1000, 768, 640, 40, 32, False, {"compute_batch_size": 1024, "combine_start_head_percent": 0}),
+    (2100, 512, 256, 8, 4, True, {"compute_batch_size": 4096, "combine_start_head_percent": 100, "total_sms": 64, "num_dispatch_sms": 8}),
+])
+def test_one_rank_layer_matches_general_kernels_and_oracle(T, H, I, E, K, skew, kw, monkeypatch):
+    from teramoe_b200 import engine
+    prob = make_problem(1, T, H, I, E, K, seed=T, dtype=torch.bfloat16, device="cuda", x_scale=0.1, w_scale=0.02, drop_some=T > 3)
+    idx = prob["ranks"][0]["idx"]
+    if skew:                                             # most tokens take expert 0 first; some go nowhere
+        idx = idx.clone()
+        idx[::2, 0] = 0
+        idx[5::7] = -1
+        dup = (idx[:, 1:] == 0) & (idx[:, :1] == 0)
+        idx[:, 1:][dup] = -1
+        prob["ranks"][0]["idx"] = idx
+    if T == 1000:
+        idx = idx.to(torch.int32)
+    buf = tm.Buffer(None, int(64e6), explicitly_destroy=True)
+    res = {}
+    for mode in ("0", "auto"):
+        monkeypatch.setattr(engine, "_LOCAL_LAYER_MODE", mode)
+        for name in ("_FUSED_DISPATCH_MODE", "_FUSED_MODE", "_LAYER_KERNEL_MODE"):
+            monkeypatch.setattr(engine, name, "1" if mode == "0" else "auto")
+        res[mode] = [_run(buf, prob, idx, E, **kw) for _ in range(2)]
+    ref = oracle(prob)[0]
+    for name in ("out", "dx", "dw", "dWg", "dWd"):
+        assert_close_bf16(res["auto"][0][name].float(), ref[name].cuda().float(), name)
+    for name, got in res["auto"][0].items():
+        assert torch.equal(got, res["auto"][1][name]), f"{name}: two runs differ"
+        assert torch.equal(got, res["0"][0][name]), f"{name}: differs from the general kernels"
+    buf.check_status()
+    buf.destroy()
