@@ -58,13 +58,9 @@ class _TeraMoEFunction(torch.autograd.Function):
     @staticmethod
     def forward(ctx, buffer, x, topk_idx, topk_weights, W_gateup, W_down, num_experts, grad_topk_weights, opts):
         needs_bwd = any(t.requires_grad for t in (x, topk_weights, W_gateup, W_down))
-        ctx.local = buffer._layer_is_local(x, topk_idx, W_gateup, W_down, num_experts, opts)
-        if ctx.local:
-            out, saved = buffer._engine.local_forward(x, topk_idx, topk_weights, W_gateup, W_down, needs_bwd, opts)
-        else:
-            out, saved = buffer._drive(buffer._engine.forward_gen(x, topk_idx, topk_weights, W_gateup, W_down, num_experts,
-                                                                  keep_for_backward=needs_bwd, impl=opts))
-            buffer._release()
+        out, saved = buffer._drive(buffer._engine.forward_gen(x, topk_idx, topk_weights, W_gateup, W_down, num_experts,
+                                                              keep_for_backward=needs_bwd, impl=opts))
+        buffer._release()
         ctx.buffer = buffer
         ctx.saved = saved
         ctx.grad_topk_weights = grad_topk_weights
@@ -77,13 +73,9 @@ class _TeraMoEFunction(torch.autograd.Function):
     def backward(ctx, grad_out):
         W_gateup, W_down = ctx.saved_tensors
         buffer = ctx.buffer
-        if ctx.local:
-            buffer._check_open()
-            dx, gtw, dWgu, dWd = buffer._engine.local_backward(ctx.saved, grad_out.contiguous(), W_gateup, W_down)
-        else:
-            dx, gtw, dWgu, dWd = buffer._drive(buffer._engine.backward_gen(ctx.saved, grad_out.contiguous(), W_gateup, W_down,
-                                                                          impl=ctx.opts))
-            buffer._release()
+        dx, gtw, dWgu, dWd = buffer._drive(buffer._engine.backward_gen(ctx.saved, grad_out.contiguous(), W_gateup, W_down,
+                                                                      impl=ctx.opts))
+        buffer._release()
         ctx.saved = None
         if ctx.grad_topk_weights is not None:
             ctx.grad_topk_weights.copy_(gtw)
@@ -172,6 +164,8 @@ class Buffer(LowLatencyMixin):
     def _destroy(self) -> None:
         if not self._destroyed:
             self._destroyed = True
+            if self._engine.native is not None:
+                self._engine.native.close()
             self._world.close()
 
     def __del__(self):
@@ -539,13 +533,6 @@ class Buffer(LowLatencyMixin):
             if W_gateup.dtype != torch.bfloat16 or W_down.dtype != torch.bfloat16:
                 raise ValueError("weights must be bf16 on CUDA")
 
-    def _layer_is_local(self, x, topk_idx, W_gateup, W_down, num_experts, opts) -> bool:
-        """Whether this layer call runs as the one-rank kernels (a wrong number of local experts goes to the general path, which says so)."""
-        self._check_open()
-        H, I = x.shape[1], W_gateup.shape[1] // 2
-        return (self._local is not None and x.is_cuda and W_gateup.shape == (num_experts, 2 * I, H) and W_down.shape == (num_experts, H, I)
-                and self._engine.use_local_layer(x.shape[0], topk_idx.shape[1], num_experts, H, I, opts))
-
     def teramoe_autograd(self, x: torch.Tensor, topk_idx: torch.Tensor, topk_weights: torch.Tensor, W_gateup: torch.Tensor,
                          W_down: torch.Tensor, num_experts: int, num_dispatch_sms: int = 24, num_combine_sms: int = 24,
                          total_sms: int = 148, stage: int = 1, dispatch_config: Optional[Config] = None,
@@ -576,8 +563,14 @@ class Buffer(LowLatencyMixin):
         opts = {"num_dispatch_sms": num_dispatch_sms, "num_combine_sms": num_combine_sms, "total_sms": total_sms, "stage": stage,
                 "compute_batch_size": compute_batch_size, "combine_start_head_percent": combine_start_head_percent}
         tw = topk_weights if topk_weights.dtype == torch.float32 else topk_weights.float()
-        return _TeraMoEFunction.apply(self, x.contiguous(), topk_idx.contiguous(), tw.contiguous(), W_gateup, W_down, num_experts,
-                                      grad_topk_weights, opts)
+        x, topk_idx, tw = x.contiguous(), topk_idx.contiguous(), tw.contiguous()
+        if self._local is not None:
+            self._check_open()
+            out = self._engine.local_layer(x, topk_idx, tw, W_gateup, W_down, num_experts,
+                                           (num_dispatch_sms, total_sms, compute_batch_size, combine_start_head_percent), self, True, grad_topk_weights)
+            if out is not None:
+                return out
+        return _TeraMoEFunction.apply(self, x, topk_idx, tw, W_gateup, W_down, num_experts, grad_topk_weights, opts)
 
     def teramoe_forward(self, x, topk_idx, topk_weights, W_gateup, W_down, num_experts, num_dispatch_sms: int = 24,
                         num_combine_sms: int = 24, total_sms: int = 148, stage: int = 1, dispatch_config: Optional[Config] = None,
@@ -590,8 +583,12 @@ class Buffer(LowLatencyMixin):
                 "compute_batch_size": compute_batch_size, "combine_start_head_percent": combine_start_head_percent}
         with torch.no_grad():
             x, topk_idx, topk_weights = x.contiguous(), topk_idx.contiguous(), topk_weights.float().contiguous()
-            if self._layer_is_local(x, topk_idx, W_gateup, W_down, num_experts, opts):
-                return self._engine.local_forward(x, topk_idx, topk_weights, W_gateup, W_down, False, opts)[0]
+            if self._local is not None:
+                self._check_open()
+                out = self._engine.local_layer(x, topk_idx, topk_weights, W_gateup, W_down, num_experts,
+                                               (num_dispatch_sms, total_sms, compute_batch_size, combine_start_head_percent), self, False)
+                if out is not None:
+                    return out
             out, _ = self._drive(self._engine.forward_gen(x, topk_idx, topk_weights, W_gateup, W_down, num_experts, keep_for_backward=False,
                                                           impl=opts))
             self._release()

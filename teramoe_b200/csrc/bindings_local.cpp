@@ -3,9 +3,13 @@
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <pybind11/stl.h>
+#include <torch/csrc/autograd/functions/basic_ops.h>
+#include <torch/custom_class.h>
 #include <torch/extension.h>
 
 #include <array>
+#include <atomic>
+#include <memory>
 #include <mutex>
 
 #include "launch_count.h"
@@ -258,98 +262,238 @@ void check_layer_weights(const torch::Tensor& wg, const torch::Tensor& wd, int64
                 wd.size(1) == H && wd.size(2) == I, "W_down must be a contiguous bf16 [E, H, I] CUDA tensor");
 }
 
-void set_arena(tmoe::LocalLayerParams& p, int64_t rows, int64_t arena, int64_t arena_bytes) {
-    const int64_t half = rows * p.plan.H * 2;
-    TORCH_CHECK(2 * half <= arena_bytes, "the arena is too small for this call");
-    p.out_rows = (int)rows;
-    p.slot_x = reinterpret_cast<void*>(arena);
-    p.y = reinterpret_cast<void*>(arena + half);
-}
+// What the calls of one buffer share: the arena (rows in slot order and expert outputs), the status block and its copy in pinned
+// memory, and the workspaces of the last forward and backward for whoever asks for their statistics.
+class LocalLayer : public std::enable_shared_from_this<LocalLayer> {
+  public:
+    using Schedule = std::array<int64_t, 5>;      // units per batch, lag percent, least lag in items, dispatch pairs, SMs
 
-// schedule: [group_units, lag_percent, min_lag_items, dispatch_pairs, num_sms]
-// -> (out [T,H], workspace, preact [rows,2I] or None, saved_x [T,H] or None)
-std::tuple<torch::Tensor, torch::Tensor, c10::optional<torch::Tensor>, c10::optional<torch::Tensor>>
-local_layer_forward(torch::Tensor x, torch::Tensor topk_idx, torch::Tensor topk_w, torch::Tensor w_gateup, torch::Tensor w_down,
-                    std::array<int64_t, 5> schedule, bool keep, int64_t arena, int64_t arena_bytes, torch::Tensor status) {
-    c10::cuda::CUDAGuard guard(x.device());
-    const TopK tk = topk_of(topk_idx);
-    const int64_t E = w_gateup.size(0), H = x.size(1), I = w_gateup.size(1) / 2;
-    TORCH_CHECK(x.is_cuda() && x.scalar_type() == torch::kBFloat16 && x.is_contiguous() && x.dim() == 2 && x.size(0) == tk.T, "x must be a contiguous bf16 [T, H] CUDA tensor");
-    TORCH_CHECK(topk_w.is_cuda() && topk_w.scalar_type() == torch::kFloat32 && topk_w.is_contiguous() && topk_w.numel() == (int64_t)tk.T * tk.K,
-                "topk_weights must be a contiguous fp32 [T, K] CUDA tensor");
-    check_layer_weights(w_gateup, w_down, E, H, I);
-    tmoe::LocalLayerParams p{};
-    p.plan = tmoe::local_layer_plan(tk.T, tk.K, (int)E, (int)H, (int)I, keep ? 1 : 0);
-    const int64_t rows = layer_rows(p.plan);
-    set_arena(p, rows, arena, arena_bytes);
-    auto ws = torch::empty({p.plan.words}, on(x, torch::kInt32));
-    auto out = torch::empty({tk.T, H}, x.options());
-    auto act = torch::empty({rows, I}, x.options());
-    c10::optional<torch::Tensor> preact, saved_x;
-    if (keep) {
-        preact = torch::empty({rows, 2 * I}, x.options());
-        saved_x = torch::empty({tk.T, H}, x.options());
-        p.aux = preact->data_ptr();
-        p.saved_x = saved_x->data_ptr();
+    LocalLayer(torch::Tensor status, torch::Tensor status_host) : status_(status), host_(status_host) {}
+
+    void set_arena(int64_t ptr, int64_t bytes) {
+        arena_ = ptr;
+        arena_bytes_ = bytes;
     }
-    p.ws = ws.data_ptr<int>();
-    p.topk_idx = tk.ptr; p.idx_is64 = tk.is64; p.topk_w = topk_w.data_ptr<float>();
-    p.group_units = (int)schedule[0]; p.lag_percent = (int)schedule[1]; p.min_lag_items = (int)schedule[2];
-    p.dispatch_pairs = (int)schedule[3]; p.num_sms = (int)schedule[4];
-    p.x = x.data_ptr(); p.w_gateup = w_gateup.data_ptr(); p.w_down = w_down.data_ptr();
-    p.act = act.data_ptr(); p.out = out.data_ptr();
-    p.status = status.data_ptr<int>();
-    const cudaStream_t stream = cur_stream();
-    tmoe::count_launch();
-    TM_CHECK_CUDA(tmoe::local_layer_route(p, stream));
-    TM_CHECK_CUDA(tmoe::local_layer_launch(p, stream));
-    return {out, ws, preact, saved_x};
-}
+    void close() { open_ = false; }
 
-// -> (dx [T,H], d(topk_weights) [T,K], dW_gateup, dW_down)
-std::tuple<torch::Tensor, torch::Tensor, torch::Tensor, torch::Tensor>
-local_layer_backward(torch::Tensor grad_out, torch::Tensor ws, torch::Tensor preact, torch::Tensor saved_x, torch::Tensor w_gateup,
-                     torch::Tensor w_down, int64_t K, std::array<int64_t, 5> schedule, int64_t arena, int64_t arena_bytes, torch::Tensor status) {
-    c10::cuda::CUDAGuard guard(grad_out.device());
-    const int64_t E = w_gateup.size(0), T = saved_x.size(0), H = saved_x.size(1), I = w_gateup.size(1) / 2;
-    TORCH_CHECK(grad_out.is_cuda() && grad_out.scalar_type() == torch::kBFloat16 && grad_out.is_contiguous() && grad_out.dim() == 2 &&
-                grad_out.size(0) == T && grad_out.size(1) == H, "grad_out must be a contiguous bf16 [T, H] CUDA tensor");
-    check_layer_weights(w_gateup, w_down, E, H, I);
-    tmoe::LocalLayerParams p{};
-    p.plan = tmoe::local_layer_plan((int)T, (int)K, (int)E, (int)H, (int)I, 1);
-    const int64_t rows = layer_rows(p.plan);
-    TORCH_CHECK(ws.numel() == p.plan.words && preact.size(0) == rows && preact.size(1) == 2 * I, "saved tensors of another call");
-    set_arena(p, rows, arena, arena_bytes);
-    auto act_w = torch::empty({rows, I}, grad_out.options());
-    auto dgu = torch::empty({rows, 2 * I}, grad_out.options());
-    auto xperm = torch::empty({rows, H}, grad_out.options());
-    auto parts = torch::empty({rows, 2 * ((I + 255) / 256)}, on(grad_out, torch::kFloat32));
-    auto dx = torch::empty({T, H}, grad_out.options());
-    auto dw = torch::empty({T, K}, on(grad_out, torch::kFloat32));
-    auto dwg = torch::empty({E, 2 * I, H}, grad_out.options());
-    auto dwd = torch::empty({E, H, I}, grad_out.options());
-    p.ws = ws.data_ptr<int>();
-    p.group_units = (int)schedule[0]; p.lag_percent = (int)schedule[1]; p.min_lag_items = (int)schedule[2];
-    p.dispatch_pairs = (int)schedule[3]; p.num_sms = (int)schedule[4];
-    p.bwd = 1;
-    p.x = grad_out.data_ptr(); p.w_gateup = w_gateup.data_ptr(); p.w_down = w_down.data_ptr();
-    p.act = act_w.data_ptr(); p.aux = dgu.data_ptr(); p.saved_x = saved_x.data_ptr(); p.out = dx.data_ptr();
-    p.preact = preact.data_ptr(); p.droute_part = parts.data_ptr<float>(); p.xperm = xperm.data_ptr();
-    p.dw_topk = dw.data_ptr<float>(); p.dw_gateup = dwg.data_ptr(); p.dw_down = dwd.data_ptr();
-    p.status = status.data_ptr<int>();
-    TM_CHECK_CUDA(tmoe::local_layer_launch(p, cur_stream()));
-    return {dx, dw, dwg, dwd};
-}
+    // The conditions under which the kernels take a call; anything else is for the caller's slow path, which also names what is wrong.
+    bool takes(const torch::Tensor& x, const torch::Tensor& idx, const torch::Tensor& w, const torch::Tensor& wg, const torch::Tensor& wd,
+               int64_t num_experts) const {
+        if (!(x.is_cuda() && idx.is_cuda() && w.is_cuda() && wg.is_cuda() && wd.is_cuda())) return false;
+        if (x.dim() != 2 || idx.dim() != 2 || wg.dim() != 3 || wd.dim() != 3 || w.sizes() != idx.sizes() || idx.size(0) != x.size(0)) return false;
+        if (x.scalar_type() != torch::kBFloat16 || wg.scalar_type() != torch::kBFloat16 || wd.scalar_type() != torch::kBFloat16 ||
+            w.scalar_type() != torch::kFloat32 || (idx.scalar_type() != torch::kInt64 && idx.scalar_type() != torch::kInt32))
+            return false;
+        if (!(x.is_contiguous() && idx.is_contiguous() && w.is_contiguous() && wg.is_contiguous() && wd.is_contiguous())) return false;
+        const int64_t E = wg.size(0), H = x.size(1), I = wd.size(2);
+        return E == num_experts && E >= 1 && E <= tmoe::kLocalMaxExperts && wg.size(1) == 2 * I && wg.size(2) == H && wd.size(0) == E && wd.size(1) == H &&
+               H % 64 == 0 && I % 64 == 0 && idx.size(1) >= 1 && idx.size(1) <= 32;
+    }
+    // bytes of the arena that a call needs, 0 if it has them
+    int64_t wants(int64_t T, int64_t K, int64_t E, int64_t H) const {
+        const int64_t need = local_layer_arena_bytes(T, K, E, H);
+        return need > arena_bytes_ ? need : 0;
+    }
 
-// word offsets inside the workspace that the host may read: statistics of the two directions, entries per expert, slots in use
-py::dict local_layer_words(int64_t T, int64_t K, int64_t E, int64_t H, int64_t I, bool keep) {
-    const auto p = tmoe::local_layer_plan((int)T, (int)K, (int)E, (int)H, (int)I, keep ? 1 : 0);
-    py::dict d;
-    d["stats"] = py::make_tuple(p.stats[0], keep ? p.stats[1] : -1);
-    d["totals"] = p.totals;
-    d["meta"] = p.meta;
-    d["slots_cap"] = p.slots_cap;
-    return d;
+    // strict: wait for the call's kernels, so that the call whose wait ran out is the one that raises
+    void settle(bool strict) {
+        if (!strict) return;
+        const cudaError_t e = cudaStreamSynchronize(cur_stream());
+        TORCH_CHECK(e == cudaSuccess, "teramoe_b200: ", cudaGetErrorString(e));
+        check();
+    }
+    void check() {
+        TORCH_CHECK(open_, "Buffer was destroyed");
+        volatile int* h = host_.data_ptr<int>();
+        if (h[0] == 0) return;
+        static const char* names[] = {"", "mbarrier wait", "flag wait", "barrier", "bad argument"};
+        const int code = h[0], site = h[1], block = h[2], detail = h[3];
+        status_.narrow(0, 0, 4).zero_();
+        h[0] = 0;
+        TORCH_CHECK(false, "teramoe_b200: a device-side wait ran out on rank 0: ", code >= 1 && code <= 4 ? names[code] : "?", " (site ", site,
+                    ", block ", block, ", detail ", detail, ")");
+    }
+
+    struct Kept {
+        torch::Tensor ws, preact, saved_x;
+    };
+
+    torch::Tensor forward(const torch::Tensor& x, const torch::Tensor& topk_idx, const torch::Tensor& topk_w, const torch::Tensor& w_gateup,
+                          const torch::Tensor& w_down, const Schedule& schedule, Kept* kept) {
+        check();
+        c10::cuda::CUDAGuard guard(x.device());
+        const TopK tk = topk_of(topk_idx);
+        const int64_t E = w_gateup.size(0), H = x.size(1), I = w_gateup.size(1) / 2;
+        TORCH_CHECK(x.is_cuda() && x.scalar_type() == torch::kBFloat16 && x.is_contiguous() && x.dim() == 2 && x.size(0) == tk.T, "x must be a contiguous bf16 [T, H] CUDA tensor");
+        TORCH_CHECK(topk_w.is_cuda() && topk_w.scalar_type() == torch::kFloat32 && topk_w.is_contiguous() && topk_w.numel() == (int64_t)tk.T * tk.K,
+                    "topk_weights must be a contiguous fp32 [T, K] CUDA tensor");
+        check_layer_weights(w_gateup, w_down, E, H, I);
+        tmoe::LocalLayerParams p{};
+        p.plan = tmoe::local_layer_plan(tk.T, tk.K, (int)E, (int)H, (int)I, kept != nullptr ? 1 : 0);
+        const int64_t rows = set_common(p, schedule);
+        auto ws = torch::empty({p.plan.words}, on(x, torch::kInt32));
+        auto out = torch::empty({tk.T, H}, x.options());
+        auto act = torch::empty({rows, I}, x.options());
+        if (kept != nullptr) {
+            kept->ws = ws;
+            kept->preact = torch::empty({rows, 2 * I}, x.options());
+            kept->saved_x = torch::empty({tk.T, H}, x.options());
+            p.aux = kept->preact.data_ptr();
+            p.saved_x = kept->saved_x.data_ptr();
+        }
+        p.ws = ws.data_ptr<int>();
+        p.topk_idx = tk.ptr; p.idx_is64 = tk.is64; p.topk_w = topk_w.data_ptr<float>();
+        p.x = x.data_ptr(); p.w_gateup = w_gateup.data_ptr(); p.w_down = w_down.data_ptr();
+        p.act = act.data_ptr(); p.out = out.data_ptr();
+        const cudaStream_t stream = cur_stream();
+        tmoe::count_launch();
+        TM_CHECK_CUDA(tmoe::local_layer_route(p, stream));
+        TM_CHECK_CUDA(tmoe::local_layer_launch(p, stream));
+        note(0, ws, p.plan);
+        return out;
+    }
+
+    // -> dx [T,H], d(topk_weights) [T,K], dW_gateup, dW_down
+    std::array<torch::Tensor, 4> backward(const torch::Tensor& grad_out, const Kept& kept, const torch::Tensor& w_gateup, const torch::Tensor& w_down,
+                                          int64_t K, const Schedule& schedule) {
+        check();
+        c10::cuda::CUDAGuard guard(grad_out.device());
+        const int64_t E = w_gateup.size(0), T = kept.saved_x.size(0), H = kept.saved_x.size(1), I = w_gateup.size(1) / 2;
+        TORCH_CHECK(grad_out.is_cuda() && grad_out.scalar_type() == torch::kBFloat16 && grad_out.is_contiguous() && grad_out.dim() == 2 &&
+                    grad_out.size(0) == T && grad_out.size(1) == H, "grad_out must be a contiguous bf16 [T, H] CUDA tensor");
+        check_layer_weights(w_gateup, w_down, E, H, I);
+        tmoe::LocalLayerParams p{};
+        p.plan = tmoe::local_layer_plan((int)T, (int)K, (int)E, (int)H, (int)I, 1);
+        const int64_t rows = set_common(p, schedule);
+        TORCH_CHECK(kept.ws.numel() == p.plan.words && kept.preact.size(0) == rows && kept.preact.size(1) == 2 * I, "saved tensors of another call");
+        auto act_w = torch::empty({rows, I}, grad_out.options());
+        auto dgu = torch::empty({rows, 2 * I}, grad_out.options());
+        auto xperm = torch::empty({rows, H}, grad_out.options());
+        auto parts = torch::empty({rows, 2 * ((I + 255) / 256)}, on(grad_out, torch::kFloat32));
+        auto dx = torch::empty({T, H}, grad_out.options());
+        auto dw = torch::empty({T, K}, on(grad_out, torch::kFloat32));
+        auto dwg = torch::empty({E, 2 * I, H}, grad_out.options());
+        auto dwd = torch::empty({E, H, I}, grad_out.options());
+        p.ws = kept.ws.data_ptr<int>();
+        p.bwd = 1;
+        p.x = grad_out.data_ptr(); p.w_gateup = w_gateup.data_ptr(); p.w_down = w_down.data_ptr();
+        p.act = act_w.data_ptr(); p.aux = dgu.data_ptr(); p.saved_x = kept.saved_x.data_ptr(); p.out = dx.data_ptr();
+        p.preact = kept.preact.data_ptr(); p.droute_part = parts.data_ptr<float>(); p.xperm = xperm.data_ptr();
+        p.dw_topk = dw.data_ptr<float>(); p.dw_gateup = dwg.data_ptr(); p.dw_down = dwd.data_ptr();
+        TM_CHECK_CUDA(tmoe::local_layer_launch(p, cur_stream()));
+        note(1, kept.ws, p.plan);
+        return {dx, dw, dwg, dwd};
+    }
+
+    // statistics words of the last forward (0) / backward (1), None before the first
+    c10::optional<torch::Tensor> stats(int64_t dir) {
+        std::lock_guard<std::mutex> lock(mutex_);
+        if (!last_[dir].defined()) return c10::nullopt;
+        return last_[dir].narrow(0, last_at_[dir], 48).view(torch::kInt64);
+    }
+
+  private:
+    int64_t set_common(tmoe::LocalLayerParams& p, const Schedule& s) {
+        const int64_t rows = layer_rows(p.plan), half = rows * p.plan.H * 2;
+        TORCH_CHECK(2 * half <= arena_bytes_, "the arena is too small for this call");
+        p.out_rows = (int)rows;
+        p.slot_x = reinterpret_cast<void*>(arena_);
+        p.y = reinterpret_cast<void*>(arena_ + half);
+        p.group_units = (int)s[0]; p.lag_percent = (int)s[1]; p.min_lag_items = (int)s[2];
+        p.dispatch_pairs = (int)s[3]; p.num_sms = (int)s[4];
+        p.status = status_.data_ptr<int>();
+        return rows;
+    }
+    void note(int dir, const torch::Tensor& ws, const tmoe::LocalLayerPlan& plan) {
+        std::lock_guard<std::mutex> lock(mutex_);
+        last_[dir] = ws;
+        last_at_[dir] = plan.stats[dir];
+    }
+    torch::Tensor status_, host_;
+    int64_t arena_ = 0, arena_bytes_ = 0;
+    std::atomic<bool> open_{true};
+    std::mutex mutex_;
+    torch::Tensor last_[2];
+    int64_t last_at_[2] = {0, 0};
+};
+
+// The layer as a native autograd node: a backward pass runs on autograd's worker thread without the interpreter.
+class LocalLayerFunction : public torch::autograd::Function<LocalLayerFunction> {
+  public:
+    static torch::Tensor forward(torch::autograd::AutogradContext* ctx, const torch::Tensor& x, const torch::Tensor& topk_w, const torch::Tensor& w_gateup,
+                                 const torch::Tensor& w_down, const torch::Tensor& topk_idx, const c10::optional<torch::Tensor>& grad_topk_w,
+                                 std::shared_ptr<LocalLayer> layer, LocalLayer::Schedule schedule, bool strict, std::shared_ptr<PyObject> owner) {
+        LocalLayer::Kept kept;
+        auto out = layer->forward(x, topk_idx, topk_w, w_gateup, w_down, schedule, &kept);
+        // x itself is not kept
+        ctx->save_for_backward({w_gateup, w_down, kept.ws, kept.preact, kept.saved_x});
+        auto holder = c10::make_intrusive<Holder>();
+        holder->layer = std::move(layer);
+        holder->schedule = schedule;
+        holder->K = topk_idx.size(1);
+        holder->strict = strict;
+        holder->owner = std::move(owner);
+        holder->grad_topk_w = grad_topk_w;
+        ctx->saved_data["h"] = c10::IValue::make_capsule(std::move(holder));
+        return out;
+    }
+    static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::variable_list grads) {
+        const auto saved = ctx->get_saved_variables();
+        auto capsule = ctx->saved_data["h"].toCapsule();
+        auto* h = static_cast<Holder*>(capsule.get());
+        torch::autograd::variable_list res;
+        {
+            at::AutoGradMode no_grad(false);
+            auto r = h->layer->backward(grads[0].contiguous(), LocalLayer::Kept{saved[2], saved[3], saved[4]}, saved[0], saved[1], h->K, h->schedule);
+            if (h->grad_topk_w.has_value()) {
+                h->grad_topk_w->copy_(r[1]);
+                r[1] = *h->grad_topk_w;
+            }
+            h->layer->settle(h->strict);
+            res = {r[0], r[1], r[2], r[3]};
+        }
+        if (at::GradMode::is_enabled()) {
+            // a graph of this backward pass was asked for: using it raises, as there is no second derivative
+            auto err = std::make_shared<torch::autograd::DelayedError>("trying to differentiate twice a function that was marked with @once_differentiable",
+                                                                       (int64_t)res.size());
+            for (auto& r : res) r = r.detach().requires_grad_(true);
+            res = (*err)(std::move(res));
+        }
+        res.resize(10);
+        return res;
+    }
+
+  private:
+    struct Holder : torch::CustomClassHolder {
+        std::shared_ptr<LocalLayer> layer;
+        LocalLayer::Schedule schedule;
+        int64_t K;
+        bool strict;
+        c10::optional<torch::Tensor> grad_topk_w;
+        std::shared_ptr<PyObject> owner;      // the buffer lives at least as long as a graph that needs its arena
+    };
+};
+
+// -> the layer's output; None: not a call for these kernels; int: the arena has to hold that many bytes first
+py::object local_layer_call(std::shared_ptr<LocalLayer> layer, const torch::Tensor& x, const torch::Tensor& topk_idx, const torch::Tensor& topk_w,
+                            const torch::Tensor& w_gateup, const torch::Tensor& w_down, int64_t num_experts, LocalLayer::Schedule schedule,
+                            bool autograd, const c10::optional<torch::Tensor>& grad_topk_w, bool strict, py::object owner) {
+    if (!layer->takes(x, topk_idx, topk_w, w_gateup, w_down, num_experts)) return py::none();
+    if (const int64_t need = layer->wants(x.size(0), topk_idx.size(1), num_experts, x.size(1))) return py::int_(need);
+    torch::Tensor out;
+    if (autograd && at::GradMode::is_enabled() && (x.requires_grad() || topk_w.requires_grad() || w_gateup.requires_grad() || w_down.requires_grad())) {
+        std::shared_ptr<PyObject> keep(owner.release().ptr(), [](PyObject* p) {
+            if (p == nullptr || !Py_IsInitialized()) return;
+            py::gil_scoped_acquire gil;
+            Py_DECREF(p);
+        });
+        out = LocalLayerFunction::apply(x, topk_w, w_gateup, w_down, topk_idx, grad_topk_w, layer, schedule, strict, std::move(keep));
+    } else {
+        at::AutoGradMode no_grad(false);
+        out = layer->forward(x, topk_idx, topk_w, w_gateup, w_down, schedule, nullptr);
+    }
+    layer->settle(strict);
+    return py::cast(out);
 }
 
 }  // namespace
@@ -357,10 +501,12 @@ py::dict local_layer_words(int64_t T, int64_t K, int64_t E, int64_t H, int64_t I
 void register_local(pybind11::module_& m) {
     m.def("ll_local_dispatch", &ll_local_dispatch);
     m.def("ll_local_combine", &ll_local_combine);
-    m.def("local_layer_arena_bytes", &local_layer_arena_bytes);
-    m.def("local_layer_forward", &local_layer_forward);
-    m.def("local_layer_backward", &local_layer_backward);
-    m.def("local_layer_words", &local_layer_words);
+    py::class_<LocalLayer, std::shared_ptr<LocalLayer>>(m, "LocalLayer")
+        .def(py::init<torch::Tensor, torch::Tensor>())
+        .def("set_arena", &LocalLayer::set_arena)
+        .def("close", &LocalLayer::close)
+        .def("stats", &LocalLayer::stats)
+        .def("call", &local_layer_call);
     m.def("local_counts", &local_counts);
     m.def("local_scatter", &local_scatter);
     m.def("local_combine", &local_combine);

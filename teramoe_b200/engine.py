@@ -130,7 +130,7 @@ if LAYER_WIRE not in ("entry", "rank"):
 # One rank: the routing kernels and the layer kernel of csrc/local_layer.cu, launched by one native call per direction
 # ("0": the kernels that several ranks use).
 _LOCAL_LAYER_MODE = os.environ.get("TERAMOE_LOCAL_LAYER", "auto")
-LOCAL_LAYER_MAX_EXPERTS = 512    # csrc/local_layer.h kLocalMaxExperts
+_LOCAL_PATHS = {"fused_dispatch_gemm": True, "cta_pairs": True, "fused_combine_fwd": True, "fused_combine_bwd": True, "layer_kernel": True}
 LAYER_REDUCE_CHUNK = 64          # tokens per reduce item
 LAYER_MIN_LAG_PER_PAIR = float(os.environ.get("TERAMOE_LAYER_MIN_LAG", "2"))
 
@@ -209,30 +209,6 @@ class LocalHandle:
 
 
 @dataclass
-class LocalLayerHandle:
-    """What backward needs of a one-rank layer call: its int32 workspace (csrc/local_layer.h) and its sizes."""
-    T: int
-    K: int
-    E: int
-    H: int
-    I: int
-    ws: torch.Tensor
-    schedule: list
-
-
-class _LazyStats(dict):
-    """Per-call numbers that are read back from the device when somebody asks for them."""
-
-    def __init__(self, read):
-        super().__init__()
-        self._read = read
-
-    def __missing__(self, key):
-        self.update(self._read())
-        return dict.__getitem__(self, key)
-
-
-@dataclass
 class SavedForBackward:
     handle: LayerHandle
     saved_x: torch.Tensor        # [rows, H]
@@ -262,6 +238,20 @@ def _arena_geometry(maxima, H: int, K: int, fused_dispatch: bool = False):
     return offs, off, (rmax, smax, lmax, tmax)
 
 
+class _TraceMark(torch.autograd.Function):
+    """Identity that records a phase boundary when the backward pass comes by (only while tracing)."""
+
+    @staticmethod
+    def forward(ctx, t, engine, name):
+        ctx.engine, ctx.name = engine, name
+        return t.view_as(t)
+
+    @staticmethod
+    def backward(ctx, g):
+        ctx.engine._mark(ctx.name)
+        return g, None, None
+
+
 class EPEngine:
     def __init__(self, world: EPWorld):
         self.world = world
@@ -272,6 +262,12 @@ class EPEngine:
         self._caps = {}             # (K, E, N) -> (rows, slots, tokens) capacities learnt from earlier calls (layout_gen)
         self.last_wait_ns = {}      # whole-layer kernel: {0: forward, 1: backward} -> int64[8] wait counters (csrc/layer.h LayerStat)
         self.last_paths = {}
+        # one real rank: the native layer (csrc/bindings_local.cpp), its schedules by call options
+        self.native = None
+        self._schedules = {}
+        if self.is_cuda and world.size == 1 and world.virtual_peers is None and USE_CTA_PAIRS and not USE_TMA_GATHER:
+            self.native = self.ext.LocalLayer(world.status, world._status_pinned)
+            world.on_arena_change = self.native.set_arena
 
     # ------------------------------------------------------------------ phase tracing
     def enable_trace(self, on: bool = True) -> None:
@@ -638,71 +634,41 @@ class EPEngine:
         return out
 
     # ------------------------------------------------------------------ layer on one rank (csrc/local_layer.cu)
-    def use_local_layer(self, T: int, K: int, E: int, H: int, I: int, opts: dict) -> bool:
-        """One real rank, sizes that the kernels take, and no switch that asks for other kernels."""
+    def local_layer(self, x, topk_idx, topk_weights, W_gateup, W_down, num_experts: int, opts: tuple, owner, autograd: bool,
+                    grad_topk_weights=None):
+        """The layer as one native call per direction, or None where another path has to take it: several ranks, sizes or types that
+        the kernels do not take, or a switch that asks for other kernels.  opts: (num_dispatch_sms, total_sms, compute_batch_size,
+        combine_start_head_percent); owner: what has to stay alive until a backward pass is done."""
+        if self.native is None or LAYER_WIRE != "entry" or "0" in (_LOCAL_LAYER_MODE, _LAYER_KERNEL_MODE, _FUSED_DISPATCH_MODE, _FUSED_MODE):
+            return None
+        T, K = topk_idx.shape
+        if (T * K + 128 * min(num_experts, T * K)) * x.shape[1] * 2 > FUSED_DISPATCH_MAX_BYTES:
+            return None
+        schedule = self._schedules.get(opts)
+        if schedule is None:
+            # units per batch, lag percent, least lag in items, dispatch pairs, SMs (see layer_kernel_gen)
+            sms = self._grid_sms({"total_sms": opts[1]})
+            schedule = [max(1, opts[2] // UNIT_ROWS), opts[3], int(LAYER_MIN_LAG_PER_PAIR * ((sms or self._num_sms) // 2)),
+                        dispatch_pairs(0, opts[0]), sms]
+            self._schedules[opts] = schedule
+        traced = self._trace is not None or NVTX_MARKS
+        if traced:
+            self._mark("fwd:start")
+            x = _TraceMark.apply(x, self, "bwd:layer (dispatch, grad_act, dX, weight gradients, sum)")
         w = self.world
-        return (self.is_cuda and w.size == 1 and w.virtual_peers is None and USE_CTA_PAIRS and not USE_TMA_GATHER
-                and "0" not in (_LOCAL_LAYER_MODE, _LAYER_KERNEL_MODE, _FUSED_DISPATCH_MODE, _FUSED_MODE)
-                and (opts.get("wire") or LAYER_WIRE) == "entry" and 1 <= K and E <= LOCAL_LAYER_MAX_EXPERTS
-                and (T * K + 128 * min(E, T * K)) * H * 2 <= FUSED_DISPATCH_MAX_BYTES)
-
-    def _local_schedule(self, opts: dict, kind: int) -> list:
-        """[units per batch, lag percent, least lag in items, dispatch pairs, SMs], see layer_kernel_gen."""
-        num_sms = self._grid_sms(opts)
-        sms = num_sms or self._num_sms
-        return [max(1, int(opts.get("compute_batch_size", 2048)) // UNIT_ROWS), int(opts.get("combine_start_head_percent", 70)),
-                int(LAYER_MIN_LAG_PER_PAIR * (sms // 2)), dispatch_pairs(kind, int(opts.get("num_dispatch_sms", 0))), num_sms]
-
-    def _local_arena(self, T: int, K: int, E: int, H: int):
-        w = self.world
-        need = self.ext.local_layer_arena_bytes(T, K, E, H)
-        if need > w.data_bytes:
-            w.ensure_data(need)
+        args = (x, topk_idx, topk_weights, W_gateup, W_down, num_experts, schedule, autograd, grad_topk_weights, w.strict_status, owner)
+        res = self.native.call(*args)
+        if type(res) is int:                            # bytes the arena has to hold
+            w.ensure_data(res)
+            res = self.native.call(*args)
+        if res is None:
+            return None
         w.arena_user = "tables"
-        return w.data.local_ptr(), w.data_bytes
-
-    def local_forward(self, x, topk_idx, topk_weights, W_gateup, W_down, keep_for_backward, opts):
-        """-> (out [T,H], SavedForBackward | None).  Two routing launches and one kernel; the host waits for nothing."""
-        w = self.world
-        w.poll_status()
-        T, H = x.shape
-        K, E, I = topk_idx.shape[1], W_gateup.shape[0], W_gateup.shape[1] // 2
-        self._mark("fwd:start")
-        schedule = self._local_schedule(opts, 0)
-        arena, arena_bytes = self._local_arena(T, K, E, H)
-        out, ws, preact, saved_x = self.ext.local_layer_forward(x, topk_idx, topk_weights, W_gateup, W_down, schedule, keep_for_backward, arena,
-                                                                arena_bytes, w.status)
-        self._mark("fwd:layer (routing, dispatch, gate_up, down, sum)")
-        w.note_status()
-        self.last_paths = {"fused_dispatch_gemm": True, "cta_pairs": True, "fused_combine_fwd": True, "fused_combine_bwd": True,
-                           "layer_kernel": True}
-        h = LocalLayerHandle(T, K, E, H, I, ws, schedule)
-        self.last_wait_ns[0] = (h, keep_for_backward)
-        if not keep_for_backward:
-            return out, None
-        return out, SavedForBackward(h, saved_x, preact, stats=_LazyStats(lambda: self._local_stats(h)))
-
-    def local_backward(self, saved: "SavedForBackward", grad_out, W_gateup, W_down):
-        """-> (dx, d(topk_weights), dW_gateup, dW_down)."""
-        w, h = self.world, saved.handle
-        w.poll_status()
-        self._mark("bwd:start")
-        arena, arena_bytes = self._local_arena(h.T, h.K, h.E, h.H)
-        schedule = h.schedule[:3] + [dispatch_pairs(1, 2 * h.schedule[3] if _pairs_env is None else 0)] + h.schedule[4:]
-        res = self.ext.local_layer_backward(grad_out, h.ws, saved.preact, saved.saved_x, W_gateup, W_down, h.K, schedule, arena, arena_bytes, w.status)
-        self._mark("bwd:layer (dispatch, grad_act, dX, weight gradients, sum)")
-        w.note_status()
-        self.last_wait_ns[1] = (h, True)
+        self.last_paths = _LOCAL_PATHS
+        if traced:
+            self._mark("fwd:layer (routing, dispatch, gate_up, down, sum)")
+            res = _TraceMark.apply(res, self, "bwd:start")
         return res
-
-    def _local_words(self, h: "LocalLayerHandle", keep: bool) -> dict:
-        return self.ext.local_layer_words(h.T, h.K, h.E, h.H, h.I, keep)
-
-    def _local_stats(self, h: "LocalLayerHandle") -> dict:
-        at = self._local_words(h, True)
-        per_expert = h.ws[at["totals"]: at["totals"] + h.E].clone()
-        return {"tokens": h.T, "rows_received": h.T, "slots": int(h.ws[at["meta"] + 1]), "per_expert_rows": per_expert, "paths": dict(self.last_paths),
-                "dispatch_bytes": int(h.ws[at["meta"] + 1]) * h.H * 2, "combine_bytes": h.T * h.K * h.H * 2}
 
     # ------------------------------------------------------------------ layer forward / backward
     def forward_gen(self, x, topk_idx, topk_weights, W_gateup, W_down, num_experts, keep_for_backward=True, impl=None, num_sms=0):
@@ -805,10 +771,12 @@ class EPEngine:
         names = ("wait_arrival", "wait_first_gemm", "wait_wgrad", "wait_landed")
         rep = {}
         pairs = max(1, torch.cuda.get_device_properties(self.world.device).multi_processor_count // 2) if self.is_cuda else 1
-        for kind, t in self.last_wait_ns.items():
-            if isinstance(t, tuple):                # one-rank layer: the counters sit in the call's workspace
-                at = self._local_words(*t)["stats"][kind]
-                t = t[0].ws[at: at + 48].view(torch.int64)
+        counters = dict(self.last_wait_ns)
+        for kind in (0, 1):
+            local = self.native.stats(kind) if self.native is not None and self.last_paths is _LOCAL_PATHS else None
+            if local is not None:
+                counters[kind] = local
+        for kind, t in counters.items():
             v = t.tolist()
             d = {n: round(v[i] / 1e6 / (pairs if i < 3 else pairs * 2), 4) for i, n in enumerate(names)}
             # when the epilogues took the first / finished the last item of every kind, relative to the first item at all

@@ -57,6 +57,7 @@ class EPWorld:
         self.control = None
         self.data = None
         self.data_bytes = 0
+        self.on_arena_change = None                 # called with (address, bytes) of the data arena whenever it was replaced
         self._ptr_cache: Dict[str, torch.Tensor] = {}
         self.cpu_tables: Dict[str, torch.Tensor] = {}
         self.closed = False
@@ -155,6 +156,8 @@ class EPWorld:
             old.close()
         self.data_bytes = new_bytes
         self._ptr_cache = {k: v for k, v in self._ptr_cache.items() if k.startswith("control")}
+        if self.on_arena_change is not None:
+            self.on_arena_change(self.data.local_ptr(), new_bytes)
 
     def side_stream(self):
         """High-priority stream for communication kernels that overlap compute."""
@@ -309,6 +312,8 @@ class EPWorld:
                     dist.barrier(group=self.group)
                 except Exception:
                     pass
+            if self.on_arena_change is not None:
+                self.on_arena_change(0, 0)
             if self.data is not None:
                 self.data.close()
             self.control.close()

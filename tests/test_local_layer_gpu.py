@@ -60,3 +60,32 @@ def test_one_rank_layer_matches_general_kernels_and_oracle(T, H, I, E, K, skew, 
         assert torch.equal(got, res["0"][0][name]), f"{name}: differs from the general kernels"
     buf.check_status()
     buf.destroy()
+
+
+def test_native_autograd_node_keeps_its_buffer_and_fills_the_given_gradient():
+    """The buffer may go out of scope before the backward pass; d(topk_weights) goes to the caller's tensor; a second derivative
+    raises; a destroyed buffer raises."""
+    prob = make_problem(1, 200, 512, 256, 8, 2, seed=4, dtype=torch.bfloat16, device="cuda", x_scale=0.1, w_scale=0.02)
+    r = prob["ranks"][0]
+    Wg, Wd = prob["W_gateup"].requires_grad_(True), prob["W_down"].requires_grad_(True)
+    grads = []
+    for given in (None, torch.full((200, 2), 7.0, device="cuda")):
+        x, w = r["x"].clone().requires_grad_(True), r["w"].clone().requires_grad_(True)
+        out = tm.Buffer(None, 0).teramoe_autograd(x, r["idx"], w, Wg, Wd, 8, grad_topk_weights=given)
+        out.backward(r["go"])
+        grads.append((x.grad, w.grad))
+        if given is not None:
+            assert torch.equal(given, w.grad)
+    assert torch.equal(grads[0][0], grads[1][0]) and torch.equal(grads[0][1], grads[1][1])
+    buf = tm.Buffer(None, 0, explicitly_destroy=True)
+    x = r["x"].clone().requires_grad_(True)
+    out = buf.teramoe_autograd(x, r["idx"], r["w"], Wg, Wd, 8)
+    (dx,) = torch.autograd.grad(out, x, r["go"].clone().requires_grad_(True), create_graph=True)
+    assert torch.equal(dx, grads[0][0])
+    with pytest.raises(RuntimeError, match="once_differentiable"):
+        dx.float().sum().backward()
+    out = buf.teramoe_autograd(x, r["idx"], r["w"], Wg, Wd, 8)
+    buf.destroy()
+    with pytest.raises(RuntimeError, match="destroyed"):
+        out.backward(r["go"])
+
