@@ -33,9 +33,12 @@ using namespace detail;
 
 namespace {
 
-constexpr int kStagesP = 6;
+// A stage holds 64 columns of K of a tile: this CTA's 128 rows of A and, for each 256 columns of the tile, its 128 rows of B.
+// Tiles are 256 rows by 512 columns where a layer is large enough (local_layer_plan), else 256 by 256: the wide tile reads a
+// quarter fewer operand bytes from L2 per FLOP, and moving operands is what the power cap leaves least for.
+constexpr int kStagesP = 4;
 constexpr int kBHalfBytesP = (BN / 2) * BK * 2;
-constexpr int kStageBytesP = kAStageBytes + kBHalfBytesP;                 // 32 KB
+constexpr int kStageBytesP = kAStageBytes + 2 * kBHalfBytesP;             // 48 KB
 constexpr int kPipeBytesP = kStagesP * kStageBytesP;                      // 192 KB
 constexpr int kBoxBytes = 32 * 128;                                       // 32 rows x 64 bf16 columns
 constexpr int kEpiBytes = kEpiWarps * kBoxBytes;                          // 32 KB: one box per epilogue warp
@@ -44,6 +47,7 @@ constexpr int kSmemBytesP = kBarOffsetP + 512 + 1024;
 constexpr int kCopyChunk = 8192;                                          // dispatch: two buffers per warp
 constexpr int kPublishBatch = 4;
 constexpr int kRingDepth = 4;
+constexpr int kOwed = 4;                                                  // finished tiles an epilogue warp counts at once
 constexpr int kGatherTasks = 16384;                                       // least number of (token, columns) tasks of the gather role
 constexpr uint32_t kOffTmem = 496, kOffCopyBar = 128, kOffRingFull = 320, kOffRingEmpty = 352, kOffItems = 384;
 constexpr uint32_t kRingConsumers = 2 * kEpiWarps + 2;
@@ -55,6 +59,10 @@ static_assert(kSmemBytesP <= 232448, "shared memory");
 enum { kSyncItem = 0, kSyncUnits = 1, kSyncToken = 2, kSyncCopy = 3, kSyncExpand = 4, kSyncExpanded = 5, kSyncWords = 16 };
 // words of the meta block
 enum { kMetaUnits = 0, kMetaSlots = 1, kMetaWork = 2 };
+
+constexpr int kWideTiles = 74 * 4;                                        // least number of wide tiles of a GEMM
+
+constexpr int column_blocks(int n, int cols) { return (n + cols - 1) / cols; }
 
 constexpr int kRouteThreads = 256;
 constexpr int kRouteWarps = kRouteThreads / 32;
@@ -76,7 +84,7 @@ struct RouteArgs {
     const void* topk_idx;
     int is64;
     const float* topk_w;
-    int nb1[2], nb2, mu_wd, nb_wd, mu_wg, nb_wg;
+    int nb1[2], nb2[2], mu_wd, nb_wd, mu_wg, nb_wg;
     int group_units, lag_percent, min_lag_items;
 };
 
@@ -193,7 +201,7 @@ __global__ void __launch_bounds__(kRouteThreads) local_route_assign_kernel(const
     const int SG = max(1, a.group_units), NG = (U + SG - 1) / SG;
     for (int dir = 0; dir < (a.p.keep ? 2 : 1); ++dir) {
         int4* work = reinterpret_cast<int4*>(a.ws + a.p.work[dir]);
-        const int cap = a.p.work_cap[dir], nb1 = a.nb1[dir], nb2 = a.nb2;
+        const int cap = a.p.work_cap[dir], nb1 = a.nb1[dir], nb2 = a.nb2[dir];
         auto gsize = [&](int g) { return min(SG, U - g * SG); };
         auto emit = [&](int pos, int kind, int g, int r) {
             const int s = gsize(g), n_blk = r / s, u = g * SG + (r - n_blk * s);
@@ -300,12 +308,12 @@ __global__ void __launch_bounds__(kRouteThreads) local_route_assign_kernel(const
 struct Phase {
     alignas(64) CUtensorMap map_a;
     alignas(64) CUtensorMap map_b;
-    int nk, b_group_rows, num_n_blocks, n_total, m_total;
+    int nk, b_group_rows, cols, num_n_blocks, n_total, m_total;
 };
 
 struct LayerArgsP {
     Phase ph[4];
-    alignas(64) CUtensorMap st_act;      // stores: [out_rows, I] (backward: boxes of 32 columns), [out_rows, 2I], [out_rows, H] and
+    alignas(64) CUtensorMap st_act;      // stores: [out_rows, I], [out_rows, 2I] (backward: boxes of 32 columns), [out_rows, H] and
     alignas(64) CUtensorMap st_aux;      // [E, rows, cols] of the weight gradients, in boxes of 32 rows x 64 columns
     alignas(64) CUtensorMap st_y;
     alignas(64) CUtensorMap st_dwd;
@@ -361,6 +369,9 @@ __device__ __forceinline__ void tma_store_3d(const CUtensorMap* map, uint32_t sr
 __device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
     asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
 }
+__device__ __forceinline__ void ld_shared_v4(uint32_t addr, uint32_t (&v)[4]) {
+    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(addr) : "memory");
+}
 // Bounded wait until *flag >= target (counters that other SMs bump).
 __device__ __forceinline__ bool wait_count(const int* flag, int target, int* status, int site, uint32_t pause_ns) {
     if (ld_acquire_gpu(flag) >= target) return true;
@@ -394,7 +405,7 @@ __device__ __forceinline__ void copy_row_deep(int4* dst, const int4* src, int nv
 }
 
 struct Item {
-    int kind, n_blk, group, k0, nk, m0, unit, need;
+    int kind, n0, halves, group, k0, nk, m0, unit, need;      // columns n0 .. n0 + 256 * halves
     bool live;          // this CTA's 128 rows are real
     int m_in_group;     // weight gradients: first row of dW inside the expert
 };
@@ -402,14 +413,16 @@ struct Item {
 __device__ __forceinline__ void decode_item(const LayerArgsP& L, const int4& it, uint32_t rank, Item& q) {
     q.kind = it.x & 15;
     q.group = (it.x >> 8) & 0xfffff;
-    q.n_blk = it.z & 0xffff;
+    const Phase& P = L.ph[q.kind];
+    q.n0 = (it.z & 0xffff) * P.cols;
+    q.halves = (P.cols > BN && q.n0 + BN < P.n_total) ? 2 : 1;
     if (q.kind <= kWorkGemm2) {
         q.unit = it.y;
         q.need = rank == 0 ? ((it.z >> 16) & 0xff) : ((it.z >> 24) & 0xff);
         q.live = (rank == 0) || ((it.x >> 4) & 1);
         q.m0 = (it.w + (int)rank) * BM;
         q.k0 = 0;
-        q.nk = L.ph[q.kind].nk;
+        q.nk = P.nk;
         q.m_in_group = 0;
     } else {
         q.unit = -1;
@@ -440,13 +453,26 @@ struct Staging {
                 pack_bf16x2(__uint_as_float(p[4]), __uint_as_float(p[5])), pack_bf16x2(__uint_as_float(p[6]), __uint_as_float(p[7])));
         }
     }
-    // the same in a box of 32 rows x 64 bytes (64-byte swizzle)
-    __device__ __forceinline__ void put_narrow(int chunk, uint32_t a, uint32_t b, uint32_t c, uint32_t d) const {
-        st_shared_v4(base + lane * 64 + ((chunk ^ ((lane >> 1) & 3)) << 4), a, b, c, d);
+    // The box as two of 32 rows x 64 bytes (64-byte swizzle) that are used in turn: 32 columns in one, its store in flight while
+    // the other is filled.  `turn` counts the stores; a store that is not wanted still closes a group, as `reuse` counts groups.
+    __device__ __forceinline__ uint32_t narrow_at(int turn, int row, int chunk) const {
+        return base + (turn & 1) * (kBoxBytes / 2) + row * 64 + ((chunk ^ ((row >> 1) & 3)) << 4);
     }
-    // wait until this warp's last store has been read out of shared memory
+    __device__ __forceinline__ void put_narrow(int turn, int chunk, uint32_t a, uint32_t b, uint32_t c, uint32_t d) const {
+        st_shared_v4(narrow_at(turn, lane, chunk), a, b, c, d);
+    }
+    __device__ __forceinline__ void store_narrow(int turn, bool wanted, const CUtensorMap* map, int c0, int c1) const {
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+            if (wanted) tma_store_2d(map, base + (turn & 1) * (kBoxBytes / 2), c0, c1);
+            tma_store_commit();
+        }
+    }
+    // wait until all but the last N stores of this warp have been read out of shared memory
+    template <int N = 0>
     __device__ __forceinline__ void reuse() const {
-        if (lane == 0) tma_store_wait_read<0>();
+        if (lane == 0) tma_store_wait_read<N>();
         __syncwarp();
     }
     __device__ __forceinline__ void store(bool wanted, const CUtensorMap* map, int c0, int c1) const {
@@ -469,7 +495,8 @@ struct Staging {
 
 // First GEMM, forward: accumulator columns (2j, 2j+1) = (gate_j, up_j).  act = silu(g) * u * w; the pre-activation is kept for
 // backward (from a second read of tensor memory, which costs less than 32 registers to hold the activation).
-__device__ __forceinline__ void epilogue_swiglu(const LayerArgsP& L, const Staging& st, uint32_t taddr, int row0, bool live, int n0) {
+template <typename R>
+__device__ __forceinline__ void epilogue_swiglu(const LayerArgsP& L, const Staging& st, uint32_t taddr, int row0, bool live, int n0, R release) {
     const float w = live ? L.slot_w[row0 + st.lane] : 0.f;
     const int n_total = 2 * L.I;
     st.reuse();
@@ -492,6 +519,7 @@ __device__ __forceinline__ void epilogue_swiglu(const LayerArgsP& L, const Stagi
         st.put(2 * c, o[0], o[1], o[2], o[3]);
         st.put(2 * c + 1, o[4], o[5], o[6], o[7]);
     }
+    if (!L.keep) release();
     st.store(live && n0 < n_total, &L.st_act, n0 >> 1, row0);
     if (!L.keep) return;
 #pragma unroll 1
@@ -500,6 +528,7 @@ __device__ __forceinline__ void epilogue_swiglu(const LayerArgsP& L, const Stagi
         tmem_ld_x32(taddr + (uint32_t)(h * 64), a0);
         tmem_ld_x32(taddr + (uint32_t)(h * 64 + 32), a1);
         tmem_ld_wait();
+        if (h == 1) release();
         st.reuse();
         st.put32(0, a0);
         st.put32(1, a1);
@@ -509,77 +538,110 @@ __device__ __forceinline__ void epilogue_swiglu(const LayerArgsP& L, const Stagi
 
 // First GEMM, backward: accumulator column j = d act_j.  Padding rows give zeros whatever the operands hold there: dGU and
 // act x route are operands of the weight gradients, which sum over whole 64-row blocks.
-__device__ __forceinline__ void epilogue_dswiglu(const LayerArgsP& L, const Staging& st, uint32_t taddr, int row0, bool live, int n0, int part) {
+//
+// The pre-activation comes in 32 rows x 64 columns at a time.  A lane needs its own row, but 32 lanes that each load their row touch
+// 32 lines per instruction: those loads alone held the tensor cores at 38 % of their rate during the first GEMM (H = 2048,
+// 54 % without them) and slowed the operand loads of the second.  So a warp loads whole 128-byte rows, one step ahead (the first
+// ones before the accumulator is ready), and turns them in the staging box, where dGU replaces them in place.  Stores
+// alternate between the two half boxes.
+struct Preact {
+    int4 v[8];      // 16 bytes of rows 4 i + lane / 8, i = 0 .. 7
+    __device__ __forceinline__ void request(const LayerArgsP& L, int row0, int col, uint32_t rows, int lane) {
+        const int4* p = reinterpret_cast<const int4*>(L.preact + (long)(row0 + (lane >> 3)) * (2l * L.I) + 2 * col) + (lane & 7);
+        const long step = (long)L.I;                     // four rows in 16-byte units: 4 * 2I * 2 / 16
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = ((rows >> (4 * i + (lane >> 3))) & 1u) ? ld_nc_v4(p + i * step) : make_int4(0, 0, 0, 0);
+    }
+};
+
+template <typename R>
+__device__ __forceinline__ void epilogue_dswiglu(const LayerArgsP& L, const Staging& st, uint32_t taddr, int row0, bool live, uint32_t rows, int n0,
+                                                 int part, Preact& pre, R release) {
     const long row = row0 + st.lane;
-    const bool real = live && L.slot_tk[row] >= 0;
+    const bool real = (rows >> st.lane) & 1u;
     const float w = real ? L.slot_w[row] : 0.f;
     float droute = 0.f;
+    int turn = 0;
+    st.reuse();                              // (the last store may be a whole box)
 #pragma unroll 1
     for (int c = 0; c < 4; ++c) {
         const int col = n0 + c * 32;
         const bool in = live && col < L.I;
-        int4 pre[8];
-#pragma unroll
-        for (int v = 0; v < 8; ++v) pre[v] = make_int4(0, 0, 0, 0);
-        if (real && in) {
-            // issued before the tensor-memory load so that their latencies overlap
-            const int4* pp = reinterpret_cast<const int4*>(L.preact + row * (2l * L.I) + 2 * col);
-#pragma unroll
-            for (int v = 0; v < 8; ++v) pre[v] = ld_nc_v4(pp + v);
-        }
         uint32_t acc[32];
         tmem_ld_x32(taddr + (uint32_t)(c * 32), acc);
+        Preact next;
+        next.request(L, row0, col + 32, c < 3 && col + 32 < L.I ? rows : 0u, st.lane);
         tmem_ld_wait();
-        st.reuse();
+        if (c == 3) release();
         uint32_t act[16];
 #pragma unroll
-        for (int v = 0; v < 8; ++v) {
-            const uint32_t pr[4] = {(uint32_t)pre[v].x, (uint32_t)pre[v].y, (uint32_t)pre[v].z, (uint32_t)pre[v].w};
-            uint32_t dgu[4];
-            float av[4];
+        for (int h = 0; h < 2; ++h) {
+            st.reuse<1>();
+            if (((st.lane >> 2) & 1) == h) {
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const float2 gu = unpack_bf16x2(pr[e]);
-                const float ga = real ? __uint_as_float(acc[4 * v + e]) : 0.f;
-                const float sig = __fdividef(1.f, 1.f + __expf(-gu.x));
-                const float s = gu.x * sig;
-                const float a = s * gu.y;
-                const float gaw = ga * w;
-                const float d_up = s * gaw;
-                const float d_gate = (sig - s * sig + s) * gaw * gu.y;
-                dgu[e] = pack_bf16x2(d_gate, d_up);
-                av[e] = a * w;
-                droute += ga * a;
+                for (int i = 0; i < 8; ++i)
+                    st_shared_v4(st.narrow_at(turn, 4 * i + (st.lane >> 3), st.lane & 3), (uint32_t)pre.v[i].x, (uint32_t)pre.v[i].y,
+                                 (uint32_t)pre.v[i].z, (uint32_t)pre.v[i].w);
             }
-            st.put(v, dgu[0], dgu[1], dgu[2], dgu[3]);
-            act[2 * v] = pack_bf16x2(av[0], av[1]);
-            act[2 * v + 1] = pack_bf16x2(av[2], av[3]);
-        }
-        st.store(in, &L.st_aux, 2 * col, row0);
-        st.reuse();
+            __syncwarp();
 #pragma unroll
-        for (int v = 0; v < 4; ++v) st.put_narrow(v, act[4 * v], act[4 * v + 1], act[4 * v + 2], act[4 * v + 3]);
-        st.store(in, &L.st_act, col, row0);
+            for (int i = 0; i < 4; ++i) {
+                const int v = 4 * h + i;
+                uint32_t pr[4], dgu[4];
+                ld_shared_v4(st.narrow_at(turn, st.lane, i), pr);
+                float av[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const float2 gu = unpack_bf16x2(pr[e]);
+                    const float ga = real ? __uint_as_float(acc[4 * v + e]) : 0.f;
+                    const float sig = __fdividef(1.f, 1.f + __expf(-gu.x));
+                    const float s = gu.x * sig;
+                    const float a = s * gu.y;
+                    const float gaw = ga * w;
+                    const float d_up = s * gaw;
+                    const float d_gate = (sig - s * sig + s) * gaw * gu.y;
+                    dgu[e] = pack_bf16x2(d_gate, d_up);
+                    av[e] = a * w;
+                    droute += ga * a;
+                }
+                st.put_narrow(turn, i, dgu[0], dgu[1], dgu[2], dgu[3]);
+                act[2 * v] = pack_bf16x2(av[0], av[1]);
+                act[2 * v + 1] = pack_bf16x2(av[2], av[3]);
+            }
+            st.store_narrow(turn++, in, &L.st_aux, 2 * col + 32 * h, row0);
+        }
+        st.reuse<1>();
+#pragma unroll
+        for (int i = 0; i < 4; ++i) st.put_narrow(turn, i, act[4 * i], act[4 * i + 1], act[4 * i + 2], act[4 * i + 3]);
+        st.store_narrow(turn++, in, &L.st_act, col, row0);
+        pre = next;
     }
     if (live) L.droute_part[row * L.n_parts + part] = droute;
 }
 
-// 128 accumulator columns as two boxes; store_box(first column)
-template <typename F>
-__device__ __forceinline__ void epilogue_plain(const Staging& st, uint32_t taddr, bool zero, F store_box) {
-#pragma unroll 1
+// 128 accumulator columns as two boxes; store_box(first column).  The accumulator is given back before anything is stored: what a
+// wide tile exposes is the time until then.
+template <typename R, typename F>
+__device__ __forceinline__ void epilogue_plain(const Staging& st, uint32_t taddr, bool zero, R release, F store_box) {
+    uint32_t packed[2][32];
+#pragma unroll
     for (int h = 0; h < 2; ++h) {
         uint32_t a0[32], a1[32];
         tmem_ld_x32(taddr + (uint32_t)(h * 64), a0);
         tmem_ld_x32(taddr + (uint32_t)(h * 64 + 32), a1);
         tmem_ld_wait();
-        if (zero) {
 #pragma unroll
-            for (int i = 0; i < 32; ++i) a0[i] = a1[i] = 0u;
+        for (int i = 0; i < 16; ++i) {
+            packed[h][i] = zero ? 0u : pack_bf16x2(__uint_as_float(a0[2 * i]), __uint_as_float(a0[2 * i + 1]));
+            packed[h][16 + i] = zero ? 0u : pack_bf16x2(__uint_as_float(a1[2 * i]), __uint_as_float(a1[2 * i + 1]));
         }
+    }
+    release();
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
         st.reuse();
-        st.put32(0, a0);
-        st.put32(1, a1);
+#pragma unroll
+        for (int c = 0; c < 8; ++c) st.put(c, packed[h][4 * c], packed[h][4 * c + 1], packed[h][4 * c + 2], packed[h][4 * c + 3]);
         store_box(h * 64);
     }
 }
@@ -819,17 +881,24 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
             const int part = next_i % parts, t = next_t, slot = next_slot;
             claim();
             const uint32_t valid = __ballot_sync(0xffffffffu, slot >= 0);
-            bool ready = true;
-            if (slot >= 0) {
-                const int* flag = L.done2 + (slot >> 7);
-                if (ld_acquire_gpu(flag) < target2) {
-                    const uint64_t w0 = globaltimer_ns();
-                    ready = wait_count(flag, target2, L.status, 660, 500);
-                    waited += globaltimer_ns() - w0;
+            // all lanes look together, so that the entries of a token are waited for once and not one after the other
+            const int* flag = L.done2 + (slot >= 0 ? slot >> 7 : 0);
+            if (!__all_sync(0xffffffffu, slot < 0 || ld_acquire_gpu(flag) >= target2)) {
+                const uint64_t w0 = globaltimer_ns(), limit_ns = peer_wait_limit_ns(L.status);
+                while (!__all_sync(0xffffffffu, slot < 0 || ld_acquire_gpu(flag) >= target2)) {
+                    __nanosleep(250);
+                    int gone = 0;
+                    if (lane == 0) {
+                        if (ld_relaxed_sys(L.status) != 0) gone = 1;
+                        else if (globaltimer_ns() - w0 > limit_ns) gone = 2;
+                    }
+                    gone = __shfl_sync(0xffffffffu, gone, 0);
+                    if (gone == 2 && slot >= 0 && ld_acquire_gpu(flag) < target2) report_status(L.status, kStatusFlagTimeout, 660, target2);
+                    if (gone != 0) return;                                    // reported: unwind
                 }
+                waited += globaltimer_ns() - w0;
             }
-            if (!__all_sync(0xffffffffu, ready)) return;                  // reported: unwind
-            __syncwarp();                                                 // every lane reads behind the other lanes' acquires
+            __syncwarp();                                                     // every lane reads behind the other lanes' acquires
             if (stamps && !stamped) {
                 stamped = true;
                 atomicMax(L.stats + kStatKindFirst + kWorkReduce, ~globaltimer_ns());
@@ -974,30 +1043,32 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                     // stores of other SMs -> async-proxy reads; the weight gradients acquire once, so they need the fence once
                     if (q.kind <= kWorkGemm2 || !wgrad_fenced) fence_proxy_async_all();
                     if (q.kind > kWorkGemm2) wgrad_fenced = true;
-                    const int n0 = q.n_blk * BN + (int)rank * (BN / 2);
+                    const int n0 = q.n0 + (int)rank * (BN / 2);
                     const int look_kb = min(kStagesP - 1, q.nk - 1);   // all stages are in flight: a pause of this thread costs nothing
                     for (int kb = 0; kb < q.nk; ++kb) {
                         if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag, L.status, 610)) { ok = false; break; }
                         const uint32_t a_dst = smem_base + stage * kStageBytesP;
                         const uint32_t b_dst = a_dst + kAStageBytes;
                         const uint32_t bar = mapa_shared(full_bar(stage), 0);
-                        if (rank == 0) mbar_arrive_expect_tx(full_bar(stage), 2 * kStageBytesP);
+                        if (rank == 0) mbar_arrive_expect_tx(full_bar(stage), 2u * (uint32_t)(kAStageBytes + q.halves * kBHalfBytesP));
                         else mbar_arrive_cluster(bar);
                         const int k = q.k0 + kb * BK;
                         if (q.kind <= kWorkGemm2) {
                             tma_load_2d_2cta(a_dst, &P.map_a, bar, k, q.live ? q.m0 : L.out_rows);     // no rows: past the end reads zeros
-                            if constexpr (!BWD) {
-                                tma_load_2d_2cta(b_dst, &P.map_b, bar, k, q.group * P.b_group_rows + n0);
-                            } else {
-                                const int krow = q.group * P.b_group_rows + k;
-#pragma unroll
-                                for (int a = 0; a < BN / 128; ++a) tma_load_2d_2cta(b_dst + a * kAtomBytes, &P.map_b, bar, n0 + 64 * a, krow);
-                            }
                         } else {
 #pragma unroll
                             for (int a = 0; a < BM / 64; ++a) tma_load_2d_2cta(a_dst + a * kAtomBytes, &P.map_a, bar, q.m0 + 64 * a, k);
+                        }
+                        for (int h = 0; h < q.halves; ++h) {
+                            const uint32_t dst = b_dst + h * kBHalfBytesP;
+                            const int col = n0 + h * BN;
+                            if (!BWD) {
+                                tma_load_2d_2cta(dst, &P.map_b, bar, k, q.group * P.b_group_rows + col);
+                            } else {
+                                const int krow = q.kind <= kWorkGemm2 ? q.group * P.b_group_rows + k : k;
 #pragma unroll
-                            for (int a = 0; a < BN / 128; ++a) tma_load_2d_2cta(b_dst + a * kAtomBytes, &P.map_b, bar, n0 + 64 * a, k);
+                                for (int a = 0; a < BN / 128; ++a) tma_load_2d_2cta(dst + a * kAtomBytes, &P.map_b, bar, col + 64 * a, krow);
+                            }
                         }
                         if (++stage == kStagesP) { stage = 0; phase ^= 1u; }
                         // (the second CTA keeps looking until the first one has published the item)
@@ -1017,7 +1088,7 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
             bool ok = true;
             int ss = 0;
             uint32_t sph = 0;
-            int iter = 0;
+            int acc = 0;                                     // accumulators (256 columns) used so far
             while (ok) {
                 int4 it;
                 if (!next_item(ss, sph, 652, it) || it.x < 0) break;
@@ -1026,34 +1097,75 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                 const bool a_mn = q.kind >= kWorkWgradDown;
                 const uint32_t idesc = BWD ? (a_mn ? make_idesc_bf16(2 * BM, BN, true, true) : make_idesc_bf16(2 * BM, BN, false, true))
                                            : make_idesc_bf16(2 * BM, BN, false, false);
-                const int as = iter & 1;
-                const uint32_t aphase = (iter >> 1) & 1;
-                ++iter;
-                if (!mbar_wait(tempty_bar(as), aphase ^ 1u, abort_flag, L.status, 620)) { ok = false; break; }
+                const int slot0 = acc & 1, slot1 = slot0 ^ 1;
+                const uint32_t parity0 = ((acc >> 1) & 1) ^ 1u, parity1 = (((acc + 1) >> 1) & 1) ^ 1u;
+                acc += q.halves;
+                // 64 columns of K of one half of the tile
+                auto multiply = [&](int s, int h, int slot, bool first) {
+                    const uint32_t a_addr = smem_base + s * kStageBytesP;
+                    const uint32_t b_addr = a_addr + kAStageBytes + h * kBHalfBytesP;
+                    const uint32_t d_tmem = tmem_base + (uint32_t)(slot * BN);
+#pragma unroll
+                    for (int k = 0; k < BK / UK; ++k) {
+                        const uint64_t a_desc = a_mn ? make_smem_desc_sw128(a_addr + k * (UK * 128), kAtomBytes, 1024)
+                                                     : make_smem_desc_sw128(a_addr + k * (UK * 2), 0, 1024);
+                        const uint64_t b_desc = BWD ? make_smem_desc_sw128(b_addr + k * (UK * 128), kAtomBytes, 1024)
+                                                    : make_smem_desc_sw128(b_addr + k * (UK * 2), 0, 1024);
+                        umma_bf16_ss_2cta(d_tmem, a_desc, b_desc, idesc, (!first || k > 0) ? 1u : 0u);
+                    }
+                };
+                if (!mbar_wait(tempty_bar(slot0), parity0, abort_flag, L.status, 620)) { ok = false; break; }
                 tcgen05_fence_after();
-                const uint32_t d_tmem = tmem_base + (uint32_t)(as * BN);
-                for (int kb = 0; kb < q.nk; ++kb) {
+                int kb = 0;
+                if (q.halves == 2) {
+                    // The second accumulator is still being read out when a wide tile starts: the first half runs ahead over the stages
+                    // that are there, the second half follows and frees them.
+                    const int lead = min(q.nk, kStagesP);
+                    int s = stage;
+                    uint32_t ph = phase;
+                    for (int i = 0; i < lead; ++i) {
+                        if (!mbar_wait(full_bar(s), ph, abort_flag, L.status, 621)) { ok = false; break; }
+                        tcgen05_fence_after();
+                        if (elect_one()) {
+                            multiply(s, 0, slot0, i == 0);
+                            if (i == q.nk - 1) umma_commit_2cta(tfull_bar(slot0), 3u);
+                        }
+                        __syncwarp();
+                        if (++s == kStagesP) { s = 0; ph ^= 1u; }
+                    }
+                    if (!ok || !mbar_wait(tempty_bar(slot1), parity1, abort_flag, L.status, 622)) { ok = false; break; }
+                    tcgen05_fence_after();
+                    for (; kb < lead; ++kb) {
+                        if (elect_one()) {
+                            multiply(stage, 1, slot1, kb == 0);
+                            umma_commit_2cta(empty_bar(stage), 3u);
+                            if (kb == q.nk - 1) umma_commit_2cta(tfull_bar(slot1), 3u);
+                        }
+                        __syncwarp();
+                        if (++stage == kStagesP) { stage = 0; phase ^= 1u; }
+                    }
+                }
+                for (; kb < q.nk; ++kb) {
                     if (!mbar_wait(full_bar(stage), phase, abort_flag, L.status, 621)) { ok = false; break; }
                     tcgen05_fence_after();
                     if (elect_one()) {
-                        const uint32_t a_addr = smem_base + stage * kStageBytesP;
-                        const uint32_t b_addr = a_addr + kAStageBytes;
-#pragma unroll
-                        for (int k = 0; k < BK / UK; ++k) {
-                            const uint64_t a_desc = a_mn ? make_smem_desc_sw128(a_addr + k * (UK * 128), kAtomBytes, 1024)
-                                                         : make_smem_desc_sw128(a_addr + k * (UK * 2), 0, 1024);
-                            const uint64_t b_desc = BWD ? make_smem_desc_sw128(b_addr + k * (UK * 128), kAtomBytes, 1024)
-                                                        : make_smem_desc_sw128(b_addr + k * (UK * 2), 0, 1024);
-                            umma_bf16_ss_2cta(d_tmem, a_desc, b_desc, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+                        const bool last = kb == q.nk - 1;
+                        multiply(stage, 0, slot0, kb == 0);
+                        if (q.halves == 2) {
+                            if (last) umma_commit_2cta(tfull_bar(slot0), 3u);
+                            multiply(stage, 1, slot1, false);
                         }
                         umma_commit_2cta(empty_bar(stage), 3u);
-                        if (kb == q.nk - 1) umma_commit_2cta(tfull_bar(as), 3u);
+                        if (last) umma_commit_2cta(tfull_bar(q.halves == 2 ? slot1 : slot0), 3u);
                     }
                     __syncwarp();
                     if (++stage == kStagesP) { stage = 0; phase ^= 1u; }
                 }
                 if (ok && q.nk == 0) {                       // an expert without rows: the epilogue stores zeros
-                    if (elect_one()) umma_commit_2cta(tfull_bar(as), 3u);
+                    if (elect_one()) {
+                        umma_commit_2cta(tfull_bar(slot0), 3u);
+                        if (q.halves == 2) umma_commit_2cta(tfull_bar(slot1), 3u);
+                    }
                     __syncwarp();
                 }
             }
@@ -1065,77 +1177,106 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
             bool ok = true;
             int ss = 0;
             uint32_t sph = 0;
-            int iter = 0;
-            int owed_kind = -1, owed_at = 0;        // tile whose stores are not yet counted as complete
-            // Count the tile of the previous item: done right before this warp would wait for the next accumulator, when its stores
-            // have normally completed.  (Never behind that wait: the next item may be the one that waits for this count.)
+            int acc = 0;
+            // Tiles whose stores are not yet counted as complete (bit 31: first GEMM).  They are counted in one go when this warp would
+            // have to wait for its next item or accumulator, or when the list is full: narrow tiles (K of a few hundred) follow
+            // each other faster than a store, a fence and an atomic complete.  Never behind such a wait: the next item may be
+            // one that waits for this count.
+            uint32_t owed[kOwed];
+            int n_owed = 0;
+            bool owed_first = false;          // a first GEMM's tile is among them: second GEMMs may be waiting for it, so it goes out with the next item
             auto flush = [&]() {
-                if (owed_kind < 0) return;
+                if (n_owed == 0) return;
                 __syncwarp();
                 if (lane == 0) {
                     tma_store_wait<0>();
                     fence_proxy_async_all();
                     fence_acq_rel_gpu();
-                    if (owed_kind == kWorkGemm1) {
-                        if (atom_add_acq_rel(L.done1 + owed_at, 1) == target1 - 1) red_add_release_gpu(L.sync + kSyncUnits, 1);
-                    } else {
-                        red_add_release_gpu(L.done2 + owed_at, 1);
+#pragma unroll
+                    for (int i = 0; i < kOwed; ++i) {
+                        if (i >= n_owed) break;
+                        const int at = (int)(owed[i] & 0x7fffffffu);
+                        if (owed[i] >> 31) {
+                            if (atom_add_acq_rel(L.done1 + at, 1) == target1 - 1) red_add_release_gpu(L.sync + kSyncUnits, 1);
+                        } else {
+                            red_add_release_gpu(L.done2 + at, 1);
+                        }
                     }
                 }
-                owed_kind = -1;
+                n_owed = 0;
+                owed_first = false;
             };
             while (ok) {
                 int4 it;
-                flush();
+                if (n_owed != 0 && !__all_sync(0xffffffffu, mbar_try_wait(ring_full(ss), sph))) flush();
                 if (!next_item(ss, sph, 653, it) || it.x < 0) break;
                 const bool stamps = L.stats != nullptr && warp == 4 && lane == 0 && rank == 0;
                 Item q;
                 decode_item(L, it, rank, q);
                 if (stamps) atomicMax(L.stats + kStatKindFirst + q.kind, ~globaltimer_ns());
-                const int as = iter & 1;
-                const uint32_t aphase = (iter >> 1) & 1;
-                ++iter;
-                if (!mbar_wait(tfull_bar(as), aphase, abort_flag, L.status, 630)) { ok = false; break; }
-                tcgen05_fence_after();
-                const uint32_t taddr = tmem_base + ((uint32_t)(qd * 32) << 16) + (uint32_t)(as * BN + hh * (BN / 2));
-                const int n0 = q.n_blk * BN + hh * (BN / 2);
                 const int row0 = q.m0 + qd * 32;
-                if (q.kind == kWorkGemm1) {
-                    if constexpr (BWD) epilogue_dswiglu(L, st, taddr, row0, q.live, n0, q.n_blk * 2 + hh);
-                    else epilogue_swiglu(L, st, taddr, row0, q.live, n0);
-                } else if (q.kind == kWorkGemm2) {
-                    epilogue_plain(st, taddr, false, [&](int c) {
-                        st.store(q.live && n0 + c < L.H, &L.st_y, n0 + c, row0);
-                    });
+                uint32_t rows = 0;                 // backward, first GEMM: which of this warp's 32 rows are real
+                if constexpr (BWD) {
+                    if (q.kind == kWorkGemm1) rows = __ballot_sync(0xffffffffu, q.live && L.slot_tk[row0 + lane] >= 0);
+                }
+                for (int h = 0; h < q.halves; ++h) {
+                    const int slot = acc & 1;
+                    const uint32_t parity = (acc >> 1) & 1;
+                    ++acc;
+                    const int n0 = q.n0 + h * BN + hh * (BN / 2);
+                    Preact pre;
                     if constexpr (BWD) {
-                        if (q.live && q.n_blk == 0 && hh == 0) {
-                            // this row's d(route weight): the sum of the first GEMM's partials
-                            const long row = row0 + lane;
-                            const int tk = L.slot_tk[row];
-                            if (tk >= 0) {
-                                float v = 0.f;
-                                for (int p = 0; p < L.n_parts; ++p) v += __ldcg(L.droute_part + row * L.n_parts + p);
-                                L.dw_topk[tk] = v;
+                        if (q.kind == kWorkGemm1) pre.request(L, row0, n0, n0 < L.I ? rows : 0u, lane);
+                    }
+                    if (n_owed != 0 && (n_owed == kOwed || owed_first || !__all_sync(0xffffffffu, mbar_try_wait(tfull_bar(slot), parity)))) flush();
+                    if (!mbar_wait(tfull_bar(slot), parity, abort_flag, L.status, 630)) { ok = false; break; }
+                    tcgen05_fence_after();
+                    const uint32_t taddr = tmem_base + ((uint32_t)(qd * 32) << 16) + (uint32_t)(slot * BN + hh * (BN / 2));
+                    // this warp has read its part of the accumulator: the issuer may overwrite it
+                    auto release = [&]() {
+                        tcgen05_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive_cluster(mapa_shared(tempty_bar(slot), 0));
+                    };
+                    if (q.kind == kWorkGemm1) {
+                        if constexpr (BWD) epilogue_dswiglu(L, st, taddr, row0, q.live, rows, n0, n0 / (BN / 2), pre, release);
+                        else epilogue_swiglu(L, st, taddr, row0, q.live, n0, release);
+                    } else if (q.kind == kWorkGemm2) {
+                        epilogue_plain(st, taddr, false, release, [&](int c) {
+                            st.store(q.live && n0 + c < L.H, &L.st_y, n0 + c, row0);
+                        });
+                        if constexpr (BWD) {
+                            if (q.live && n0 == 0) {
+                                // this row's d(route weight): the sum of the first GEMM's partials
+                                const long row = row0 + lane;
+                                const int tk = L.slot_tk[row];
+                                if (tk >= 0) {
+                                    float v = 0.f;
+                                    for (int p = 0; p < L.n_parts; ++p) v += __ldcg(L.droute_part + row * L.n_parts + p);
+                                    L.dw_topk[tk] = v;
+                                }
                             }
                         }
-                    }
-                } else {
-                    if constexpr (BWD) {
-                        const Phase& P = L.ph[q.kind];
-                        const CUtensorMap* map = q.kind == kWorkWgradDown ? &L.st_dwd : &L.st_dwg;
-                        const int m = q.m_in_group + qd * 32;
-                        epilogue_plain(st, taddr, q.nk == 0, [&](int c) {
-                            st.store3(m < P.m_total && n0 + c < P.n_total, map, n0 + c, m, q.group);
-                        });
+                    } else {
+                        if constexpr (BWD) {
+                            const Phase& P = L.ph[q.kind];
+                            const CUtensorMap* map = q.kind == kWorkWgradDown ? &L.st_dwd : &L.st_dwg;
+                            const int m = q.m_in_group + qd * 32;
+                            epilogue_plain(st, taddr, q.nk == 0, release, [&](int c) {
+                                st.store3(m < P.m_total && n0 + c < P.n_total, map, n0 + c, m, q.group);
+                            });
+                        }
                     }
                 }
-                tcgen05_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive_cluster(mapa_shared(tempty_bar(as), 0));
+                if (!ok) break;
                 if (stamps) atomicMax(L.stats + kStatKindLast + q.kind, globaltimer_ns());
                 if (q.kind == kWorkGemm1 || (q.kind == kWorkGemm2 && q.live)) {
-                    owed_kind = q.kind;
-                    owed_at = q.kind == kWorkGemm1 ? q.unit : q.m0 / BM;
+                    const uint32_t entry = q.kind == kWorkGemm1 ? (0x80000000u | (uint32_t)q.unit) : (uint32_t)(q.m0 / BM);
+#pragma unroll
+                    for (int i = 0; i < kOwed; ++i)
+                        if (i == n_owed) owed[i] = entry;
+                    ++n_owed;
+                    owed_first |= q.kind == kWorkGemm1;
                 }
             }
             flush();
@@ -1220,9 +1361,26 @@ LocalLayerPlan local_layer_plan(int T, int K, int E, int H, int I, int keep) {
     p.blocks_cap = (int)((entries + 127 * segs) / 128);
     p.slots_cap = p.blocks_cap * 128;
     p.units_cap = (int)((p.blocks_cap + segs) / 2);
-    const int nbH = (H + BN - 1) / BN, nbI = (I + BN - 1) / BN, nb2I = (2 * I + BN - 1) / BN;
-    p.work_cap[0] = p.units_cap * (nb2I + nbH);
-    p.work_cap[1] = keep ? p.units_cap * (nbI + nbH) + E * (((H + 2 * BM - 1) / (2 * BM)) * nbI + ((2 * I + 2 * BM - 1) / (2 * BM)) * nbH) : 0;
+    // Columns per tile of every GEMM [direction][kind].  The wide tile needs columns for it, enough tiles that every CTA pair gets
+    // several, and a mainloop that is long against what it cannot hide: with both accumulators in one tile, the next tile
+    // starts when the first half has been read out (a few hundred cycles for a plain store, two to three thousand for
+    // the activations), where two 256-column tiles overlap completely.
+    const int mu_wd = (H + 2 * BM - 1) / (2 * BM), mu_wg = (2 * I + 2 * BM - 1) / (2 * BM);
+    auto columns = [&](int n, long row_units, int k, int min_k) {
+        return n >= 2 * BN && k >= min_k && row_units * column_blocks(n, 2 * BN) >= kWideTiles ? 2 * BN : BN;
+    };
+    const long units = entries / (2 * BM);
+    const int rows = (int)(entries / (segs > 0 ? segs : 1));
+    p.cols[0][0] = columns(2 * I, units, H, 2048);
+    p.cols[0][1] = columns(H, units, I, 1024);
+    p.cols[1][0] = columns(I, units, H, 4096);
+    p.cols[1][1] = columns(H, units, 2 * I, 1024);
+    p.cols[1][2] = columns(I, (long)E * mu_wd, rows, 1024);
+    p.cols[1][3] = columns(H, (long)E * mu_wg, rows, 1024);
+    p.work_cap[0] = p.units_cap * (column_blocks(2 * I, p.cols[0][0]) + column_blocks(H, p.cols[0][1]));
+    p.work_cap[1] = keep ? p.units_cap * (column_blocks(I, p.cols[1][0]) + column_blocks(H, p.cols[1][1])) +
+                               E * (mu_wd * column_blocks(I, p.cols[1][2]) + mu_wg * column_blocks(H, p.cols[1][3]))
+                         : 0;
     long at = 0;
     auto take = [&](long n) {
         const long o = at;
@@ -1260,11 +1418,10 @@ cudaError_t local_layer_route(const LocalLayerParams& q, cudaStream_t stream) {
     RouteArgs a{};
     a.p = p;
     a.ws = q.ws; a.topk_idx = q.topk_idx; a.is64 = q.idx_is64; a.topk_w = q.topk_w;
-    a.nb1[0] = (2 * p.I + BN - 1) / BN;
-    a.nb1[1] = (p.I + BN - 1) / BN;
-    a.nb2 = (p.H + BN - 1) / BN;
-    a.mu_wd = (p.H + 2 * BM - 1) / (2 * BM); a.nb_wd = (p.I + BN - 1) / BN;
-    a.mu_wg = (2 * p.I + 2 * BM - 1) / (2 * BM); a.nb_wg = (p.H + BN - 1) / BN;
+    a.nb1[0] = column_blocks(2 * p.I, p.cols[0][0]); a.nb2[0] = column_blocks(p.H, p.cols[0][1]);
+    a.nb1[1] = column_blocks(p.I, p.cols[1][0]); a.nb2[1] = column_blocks(p.H, p.cols[1][1]);
+    a.mu_wd = (p.H + 2 * BM - 1) / (2 * BM); a.nb_wd = column_blocks(p.I, p.cols[1][2]);
+    a.mu_wg = (2 * p.I + 2 * BM - 1) / (2 * BM); a.nb_wg = column_blocks(p.H, p.cols[1][3]);
     a.group_units = q.group_units; a.lag_percent = q.lag_percent; a.min_lag_items = q.min_lag_items > 0 ? q.min_lag_items : 0;
     cudaError_t e = cudaMemsetAsync(q.ws, 0, (size_t)p.zero_words * sizeof(int), stream);
     if (e != cudaSuccess) return e;
@@ -1294,8 +1451,10 @@ cudaError_t local_layer_launch(const LocalLayerParams& q, cudaStream_t stream) {
     Phase& g1 = L.ph[kWorkGemm1];
     Phase& g2 = L.ph[kWorkGemm2];
     g1.nk = H / BK;
-    g2.n_total = H; g2.num_n_blocks = (H + BN - 1) / BN;
+    g1.cols = p.cols[dir][0];
+    g2.n_total = H; g2.cols = p.cols[dir][1]; g2.num_n_blocks = column_blocks(H, g2.cols);
     if ((e = make_map(&g1.map_a, q.slot_x, R, H, BK, BM)) != cudaSuccess) return e;
+    if (q.bwd && (e = make_map_narrow(&L.st_aux, q.aux, R, 2 * I)) != cudaSuccess) return e;
     if ((e = q.bwd ? make_map_narrow(&L.st_act, q.act, R, I) : make_map(&L.st_act, q.act, R, I, 64, 32)) != cudaSuccess) return e;
     if ((e = make_map(&L.st_y, q.y, R, H, 64, 32)) != cudaSuccess) return e;
     if (!q.bwd) {
@@ -1313,7 +1472,6 @@ cudaError_t local_layer_launch(const LocalLayerParams& q, cudaStream_t stream) {
         if ((e = make_map(&g2.map_b, q.w_gateup, (uint64_t)E * 2 * I, H, 64, BK)) != cudaSuccess) return e;
         g1.n_total = I; g1.b_group_rows = H;
         g2.nk = 2 * I / BK; g2.b_group_rows = 2 * I;
-        if ((e = make_map(&L.st_aux, q.aux, R, 2 * I, 64, 32)) != cudaSuccess) return e;
         // dW_down[e] = dY[seg]^T . act_w[seg]  ([H, I]);  dW_gateup[e] = dGU[seg]^T . X[seg]  ([2I, H])
         Phase& gd = L.ph[kWorkWgradDown];
         Phase& gg = L.ph[kWorkWgradGateup];
@@ -1321,12 +1479,12 @@ cudaError_t local_layer_launch(const LocalLayerParams& q, cudaStream_t stream) {
         if ((e = make_map(&gd.map_b, q.act, R, I, 64, BK)) != cudaSuccess) return e;
         if ((e = make_map(&gg.map_a, q.aux, R, 2 * I, 64, BK)) != cudaSuccess) return e;
         if ((e = make_map(&gg.map_b, q.xperm, R, H, 64, BK)) != cudaSuccess) return e;
-        gd.m_total = H; gd.n_total = I; gd.num_n_blocks = (I + BN - 1) / BN;
-        gg.m_total = 2 * I; gg.n_total = H; gg.num_n_blocks = (H + BN - 1) / BN;
+        gd.m_total = H; gd.n_total = I; gd.cols = p.cols[1][2]; gd.num_n_blocks = column_blocks(I, gd.cols);
+        gg.m_total = 2 * I; gg.n_total = H; gg.cols = p.cols[1][3]; gg.num_n_blocks = column_blocks(H, gg.cols);
         if ((e = make_store_map3(&L.st_dwd, q.dw_down, E, H, I)) != cudaSuccess) return e;
         if ((e = make_store_map3(&L.st_dwg, q.dw_gateup, E, 2 * I, H)) != cudaSuccess) return e;
     }
-    g1.num_n_blocks = (g1.n_total + BN - 1) / BN;
+    g1.num_n_blocks = column_blocks(g1.n_total, g1.cols);
     L.T = p.T; L.K = p.K; L.H = H; L.I = I; L.E = E; L.keep = p.keep; L.out_rows = q.out_rows;
     L.x = static_cast<const uint8_t*>(q.x);
     L.slot_x = static_cast<uint8_t*>(q.slot_x);

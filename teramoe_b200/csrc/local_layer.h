@@ -16,6 +16,7 @@ struct LocalLayerPlan {
     int chunks;                          // blocks of the routing kernels
     int slots_cap, blocks_cap, units_cap;
     int work_cap[2];                     // items of the forward / backward list
+    int cols[2][4];                      // columns per tile: [direction][first GEMM, second GEMM, dW_down, dW_gateup]
     // zero-filled by local_layer_route
     long stats[2], sync[2], totals, last_hist, done1[2], done2[2], arrived[2], zero_words;
     // written by it

@@ -89,3 +89,20 @@ def test_native_autograd_node_keeps_its_buffer_and_fills_the_given_gradient():
     with pytest.raises(RuntimeError, match="destroyed"):
         out.backward(r["go"])
 
+
+def test_wide_tiles_match_general_kernels(monkeypatch):
+    """Sizes at which every GEMM takes 512-column tiles, with a last tile of one half (4160 = 8 * 512 + 64) and of one and a quarter
+    (1344 = 2 * 512 + 320)."""
+    from teramoe_b200 import engine
+    prob = make_problem(1, 6000, 4160, 1344, 8, 4, seed=9, dtype=torch.bfloat16, device="cuda", x_scale=0.1, w_scale=0.02, drop_some=True)
+    buf = tm.Buffer(None, int(64e6), explicitly_destroy=True)
+    res = {}
+    for mode in ("0", "auto"):
+        monkeypatch.setattr(engine, "_LOCAL_LAYER_MODE", mode)
+        for name in ("_FUSED_DISPATCH_MODE", "_FUSED_MODE", "_LAYER_KERNEL_MODE"):
+            monkeypatch.setattr(engine, name, "1" if mode == "0" else "auto")
+        res[mode] = _run(buf, prob, prob["ranks"][0]["idx"], 8)
+    for name, got in res["auto"].items():
+        assert torch.equal(got, res["0"][name]), f"{name}: differs from the general kernels"
+    buf.check_status()
+    buf.destroy()
