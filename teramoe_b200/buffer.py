@@ -567,7 +567,7 @@ class Buffer(LowLatencyMixin):
         if self._local is not None:
             self._check_open()
             out = self._engine.local_layer(x, topk_idx, tw, W_gateup, W_down, num_experts,
-                                           (num_dispatch_sms, total_sms, compute_batch_size, combine_start_head_percent), self, True, grad_topk_weights)
+                                           (total_sms, compute_batch_size, combine_start_head_percent), self, True, grad_topk_weights)
             if out is not None:
                 return out
         return _TeraMoEFunction.apply(self, x, topk_idx, tw, W_gateup, W_down, num_experts, grad_topk_weights, opts)
@@ -586,7 +586,7 @@ class Buffer(LowLatencyMixin):
             if self._local is not None:
                 self._check_open()
                 out = self._engine.local_layer(x, topk_idx, topk_weights, W_gateup, W_down, num_experts,
-                                               (num_dispatch_sms, total_sms, compute_batch_size, combine_start_head_percent), self, False)
+                                               (total_sms, compute_batch_size, combine_start_head_percent), self, False)
                 if out is not None:
                     return out
             out, _ = self._drive(self._engine.forward_gen(x, topk_idx, topk_weights, W_gateup, W_down, num_experts, keep_for_backward=False,

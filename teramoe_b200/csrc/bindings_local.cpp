@@ -266,7 +266,7 @@ void check_layer_weights(const torch::Tensor& wg, const torch::Tensor& wd, int64
 // memory, and the workspaces of the last forward and backward for whoever asks for their statistics.
 class LocalLayer : public std::enable_shared_from_this<LocalLayer> {
   public:
-    using Schedule = std::array<int64_t, 5>;      // units per batch, lag percent, least lag in items, dispatch pairs, SMs
+    using Schedule = std::array<int64_t, 4>;      // units per batch, lag percent, least lag in items, SMs
 
     LocalLayer(torch::Tensor status, torch::Tensor status_host) : status_(status), host_(status_host) {}
 
@@ -338,7 +338,7 @@ class LocalLayer : public std::enable_shared_from_this<LocalLayer> {
             kept->ws = ws;
             kept->preact = torch::empty({rows, 2 * I}, x.options());
             kept->saved_x = torch::empty({tk.T, H}, x.options());
-            p.aux = kept->preact.data_ptr();
+            p.preact = kept->preact.data_ptr();
             p.saved_x = kept->saved_x.data_ptr();
         }
         p.ws = ws.data_ptr<int>();
@@ -400,7 +400,7 @@ class LocalLayer : public std::enable_shared_from_this<LocalLayer> {
         p.slot_x = reinterpret_cast<void*>(arena_);
         p.y = reinterpret_cast<void*>(arena_ + half);
         p.group_units = (int)s[0]; p.lag_percent = (int)s[1]; p.min_lag_items = (int)s[2];
-        p.dispatch_pairs = (int)s[3]; p.num_sms = (int)s[4];
+        p.num_sms = (int)s[3];
         p.status = status_.data_ptr<int>();
         return rows;
     }

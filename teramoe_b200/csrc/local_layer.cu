@@ -1,25 +1,27 @@
 // The MoE layer on one rank, see local_layer.h.  Roles of the persistent kernel (74 CTA pairs, 12 warps per CTA):
 //
-//   dispatch   the first pairs copy the routed rows into slot order (bulk copies through shared memory), then join
+//   copy       every warp but the next two first copies a routed row into slot order; the gather warps copy the rest
 //   producer   claims items of the work list, hands them to the pair, loads operand tiles by TMA
-//   issuer     tcgen05 cta_group::2, 256x256 tiles, two accumulators in tensor memory
+//   issuer     tcgen05 cta_group::2, 256x256 or 256x512 tiles, two accumulators in tensor memory
 //   epilogue   8 warps: SwiGLU / dSwiGLU / store.  A warp packs 32 rows x 64 columns into shared memory (128-byte swizzle) and
-//              hands them to one TMA store.
+//              hands them to one TMA store; the pre-activation goes straight between registers and memory (preact_at).
 //   gather     warps 2 and 3, joined by the epilogue warps at the end of the list: keep a copy of x (forward), rebuild x in slot
-//              order and clear padding (backward), and sum every token's expert rows as soon as the units that hold them
-//              are finished.  Tokens are visited in the order of their last expert, which is the order in which they become ready.
+//              order (backward), and sum every token's expert rows as soon as the units that hold them are finished.
+//              Tokens are visited in the order of their last expert, which is the order in which they become ready.
 //
-// The work list, the 256x256x64 tiles and the order of every sum are those of layer.cu.  What is different because there is one
-// rank: rows are copied by slot instead of pushed by entry, expert rows stay in slot order (one TMA box per 32 rows instead
-// of 32 bulk copies to landing rows), the sum of a token waits for its own units instead of for every rank's completion
-// flag, counters have GPU scope, and no host read, table copy or padding kernel is left around the kernel.
+// The work list, the k steps and the order of every sum are those of layer.cu, except that a weight gradient's tiles are listed along
+// a row of the result: the tiles in flight at a time then write whole rows (7 % faster where the stores bound it, 57 rows per expert).
+// What is different because there is one rank: rows are copied by slot instead of pushed by entry, expert rows stay in slot
+// order (one TMA box per 32 rows instead of 32 bulk copies to landing rows), the sum of a token waits for its own units
+// instead of for every rank's completion flag, counters have GPU scope, and no host read, table copy or padding kernel is
+// left around the kernel.
 //
 // Forward + backward through the API, before (several-rank kernels, 30 to 38 launches and one host wait per step) -> after:
-//   512 tokens, H=512 I=256, 4 experts, top-2            905 ->   149 us   (was host work and launches)
-//   4096, H=2048 I=2048, 16 experts, top-8              2847 ->  2509 us
-//   8192, H=2048 I=3072, 16 experts, top-6              6047 ->  5383 us
-//   8192, H=7168 I=2048, 32 experts, top-8             16561 -> 15588 us
-//   forward only, 32 tokens of that layer                773 ->   630 us
+//   512 tokens, H=512 I=256, 4 experts, top-2            884 ->   108 us   (was host work and launches)
+//   4096, H=2048 I=2048, 16 experts, top-8              2891 ->  2484 us
+//   8192, H=2048 I=3072, 16 experts, top-6              6158 ->  5195 us
+//   8192, H=7168 I=2048, 32 experts, top-8             16905 -> 15959 us
+//   forward only, 32 tokens of that layer                815 ->   620 us
 // Large layers are bound by the power cap: the issuer counts 5.63 M cycles for the forward at 8192 tokens, of which the tiles need 5.35 M,
 // while the clock drops to 1.24 GHz.
 #include "local_layer.h"
@@ -35,30 +37,34 @@ namespace {
 
 // A stage holds 64 columns of K of a tile: this CTA's 128 rows of A and, for each 256 columns of the tile, its 128 rows of B.
 // Tiles are 256 rows by 512 columns where a layer is large enough (local_layer_plan), else 256 by 256: the wide tile reads a
-// quarter fewer operand bytes from L2 per FLOP, and moving operands is what the power cap leaves least for.
-constexpr int kStagesP = 4;
+// quarter fewer operand bytes from L2 per FLOP, and moving operands is what the power cap leaves least for.  A launch with a
+// wide GEMM has four stages of 48 KB, any other six of 32 KB: where few rows share a weight the loads come from HBM, and four
+// stages of a narrow tile (1.4 us) do not cover its latency (15 to 20 % slower).
+constexpr int kMaxStages = 6;
 constexpr int kBHalfBytesP = (BN / 2) * BK * 2;
-constexpr int kStageBytesP = kAStageBytes + 2 * kBHalfBytesP;             // 48 KB
-constexpr int kPipeBytesP = kStagesP * kStageBytesP;                      // 192 KB
+constexpr int kNarrowStageBytes = kAStageBytes + kBHalfBytesP;            // 32 KB
+constexpr int kWideStageBytes = kAStageBytes + 2 * kBHalfBytesP;          // 48 KB
+constexpr int kPipeBytesP = 6 * kNarrowStageBytes;                        // 192 KB
+static_assert(kPipeBytesP == 4 * kWideStageBytes, "both divisions use the same memory");
 constexpr int kBoxBytes = 32 * 128;                                       // 32 rows x 64 bf16 columns
 constexpr int kEpiBytes = kEpiWarps * kBoxBytes;                          // 32 KB: one box per epilogue warp
 constexpr int kBarOffsetP = kPipeBytesP + kEpiBytes;
 constexpr int kSmemBytesP = kBarOffsetP + 512 + 1024;
-constexpr int kCopyChunk = 8192;                                          // dispatch: two buffers per warp
-constexpr int kPublishBatch = 4;
+constexpr int kCopyRows = 8;                                              // slots a gather warp claims at a time (divides a block)
+constexpr int kFirstRows = 1;                                             // slots every warp copies before anything else
+constexpr int kCopyWarps = kThreads / 32 - 2;                             // warps of a CTA that copy at the start
 constexpr int kRingDepth = 4;
-constexpr int kOwed = 4;                                                  // finished tiles an epilogue warp counts at once
+constexpr int kOwed = 3;                                                  // finished tiles an epilogue warp counts at once
 constexpr int kGatherTasks = 16384;                                       // least number of (token, columns) tasks of the gather role
-constexpr uint32_t kOffTmem = 496, kOffCopyBar = 128, kOffRingFull = 320, kOffRingEmpty = 352, kOffItems = 384;
+constexpr uint32_t kOffTmem = 496, kOffRingFull = 320, kOffRingEmpty = 352, kOffItems = 384;
 constexpr uint32_t kRingConsumers = 2 * kEpiWarps + 2;
-static_assert((kThreads / 32) * 2 * kCopyChunk <= kBarOffsetP, "dispatch staging exceeds the operand stages + store staging");
-static_assert(8 * (2 * kStagesP + 4) <= (int)kOffCopyBar && kOffItems + 16 * kRingDepth <= kOffTmem && kOffTmem + 8 <= 512, "barrier block");
+static_assert(8 * (2 * kMaxStages + 4) <= (int)kOffRingFull && kOffItems + 16 * kRingDepth <= kOffTmem && kOffTmem + 8 <= 512, "barrier block");
 static_assert(kSmemBytesP <= 232448, "shared memory");
 
 // words of the sync block
-enum { kSyncItem = 0, kSyncUnits = 1, kSyncToken = 2, kSyncCopy = 3, kSyncExpand = 4, kSyncExpanded = 5, kSyncWords = 16 };
+enum { kSyncItem = 0, kSyncToken = 1, kSyncCopy = 2, kSyncKeep = 3, kSyncUnits = 4, kSyncRows = 5, kSyncWords = 8 };
 // words of the meta block
-enum { kMetaUnits = 0, kMetaSlots = 1, kMetaWork = 2 };
+enum { kMetaUnits = 0, kMetaSlots = 1, kMetaWork = 2, kMetaRows = 4, kMetaWords = 8 };
 
 constexpr int kWideTiles = 74 * 4;                                        // least number of wide tiles of a GEMM
 
@@ -139,7 +145,7 @@ __global__ void __launch_bounds__(kRouteThreads) local_route_assign_kernel(const
     int* lst = cnt + kRouteWarps * E;        // [warps][E + 1] next place in the token order
     const int* totals = a.ws + a.p.totals;
     if (warp == 0) {
-        int run_s = 0, run_u = 0;
+        int run_s = 0, run_u = 0, run_r = 0;
         for (int e0 = 0; e0 < E; e0 += 32) {
             const int e = e0 + lane;
             const int blocks = e < E ? (totals[e] + 127) / 128 : 0;
@@ -158,7 +164,9 @@ __global__ void __launch_bounds__(kRouteThreads) local_route_assign_kernel(const
             }
             run_s += __shfl_sync(0xffffffffu, s, 31);
             run_u += __shfl_sync(0xffffffffu, u, 31);
+            run_r += __reduce_add_sync(0xffffffffu, e < E ? (totals[e] + BK - 1) / BK * BK : 0);
         }
+        if (blockIdx.x == 0 && lane == 0) a.ws[a.p.meta + kMetaRows] = run_r;      // rows of whole 64-row steps
         if (lane == 0) {
             seg[E] = run_s;
             ub[E] = run_u;
@@ -199,51 +207,57 @@ __global__ void __launch_bounds__(kRouteThreads) local_route_assign_kernel(const
         }
     // ---- work lists: the order that layer.cu's scheduler writes (see there), with units in slot order
     const int SG = max(1, a.group_units), NG = (U + SG - 1) / SG;
+    const int per_wd = a.mu_wd * a.nb_wd, per_e = per_wd + a.mu_wg * a.nb_wg;
     for (int dir = 0; dir < (a.p.keep ? 2 : 1); ++dir) {
         int4* work = reinterpret_cast<int4*>(a.ws + a.p.work[dir]);
         const int cap = a.p.work_cap[dir], nb1 = a.nb1[dir], nb2 = a.nb2[dir];
+        const int items = U * (nb1 + nb2);                   // of the two GEMMs
         auto gsize = [&](int g) { return min(SG, U - g * SG); };
+        const int full1 = SG * nb1, full2 = SG * nb2;
+        const int lag_items = max((int)(((long)full1 * a.lag_percent + 99) / 100), a.min_lag_items);
+        const int lg = max(1, (lag_items + full1 - 1) / full1);
+        const int head_full = min(full1, max(0, lag_items - (lg - 1) * full1));
+        // block g of the list: the first `head` tiles of batch g's first GEMM, the second GEMM of batch g - lg, the rest of the first
+        struct Block { int g2, off, n1, n2; };
+        auto block = [&](int g) {
+            Block b;
+            b.g2 = g - lg;
+            const int c2 = min(max(b.g2, 0), NG);
+            b.off = (g < NG ? g * full1 : U * nb1) + (c2 < NG ? c2 * full2 : U * nb2);
+            b.n1 = g < NG ? gsize(g) * nb1 : 0;
+            b.n2 = (b.g2 >= 0 && b.g2 < NG) ? gsize(b.g2) * nb2 : 0;
+            return b;
+        };
         auto emit = [&](int pos, int kind, int g, int r) {
             const int s = gsize(g), n_blk = r / s, u = g * SG + (r - n_blk * s);
             const int e = find_segment(ub, E, u);
             const int blk0 = seg[e] / 128 + 2 * (u - ub[e]);
             const int two = (blk0 + 1) * 128 < seg[e + 1] ? 1 : 0;
-            const int end = seg[e] + totals[e];
+            // rows that have to be in place; backward, whole 64-row steps of K of the weight gradients
+            const int end = seg[e] + (dir == 1 ? (totals[e] + BK - 1) / BK * BK : totals[e]);
             const int need0 = max(0, min(128, end - blk0 * 128)), need1 = two ? max(0, min(128, end - (blk0 + 1) * 128)) : 0;
             if (pos < cap) work[pos] = make_int4(kind | (two << 4) | (e << 8), u, n_blk | (need0 << 16) | (need1 << 24), blk0);
         };
-        const int full1 = SG * nb1, full2 = SG * nb2;
-        const int lag_items = max((int)(((long)full1 * a.lag_percent + 99) / 100), a.min_lag_items);
-        const int lg = max(1, (lag_items + full1 - 1) / full1);
-        const int head_full = min(full1, max(0, lag_items - (lg - 1) * full1));
         for (int g = blockIdx.x; g < NG + lg && NG > 0; g += gridDim.x) {
-            const int g2 = g - lg;
-            const int c2 = min(max(g2, 0), NG);
-            const int off = (g < NG ? g * full1 : U * nb1) + (c2 < NG ? c2 * full2 : U * nb2);
-            const int n1 = g < NG ? gsize(g) * nb1 : 0;
-            const int n2 = (g2 >= 0 && g2 < NG) ? gsize(g2) * nb2 : 0;
-            const int head = min(n1, head_full);
-            for (int i = tid; i < n1 + n2; i += kRouteThreads) {
-                if (i < head) emit(off + i, kWorkGemm1, g, i);
-                else if (i < head + n2) emit(off + i, kWorkGemm2, g2, i - head);
-                else emit(off + i, kWorkGemm1, g, i - n2);
+            const Block b = block(g);
+            const int head = min(b.n1, head_full);
+            for (int i = tid; i < b.n1 + b.n2; i += kRouteThreads) {
+                if (i < head) emit(b.off + i, kWorkGemm1, g, i);
+                else if (i < head + b.n2) emit(b.off + i, kWorkGemm2, b.g2, i - head);
+                else emit(b.off + i, kWorkGemm1, g, i - b.n2);
             }
         }
-        int pos = U * (nb1 + nb2);
         if (dir == 1) {
-            const int per_wd = a.mu_wd * a.nb_wd, per_wg = a.mu_wg * a.nb_wg;
-            for (int i = gtid; i < E * (per_wd + per_wg); i += gthreads) {
+            for (int i = gtid; i < E * per_e; i += gthreads) {
                 const bool down = i < E * per_wd;
-                const int j = down ? i : i - E * per_wd;
-                const int per = down ? per_wd : per_wg, mu = down ? a.mu_wd : a.mu_wg;
-                const int e = j / per, r = j - e * per, n_blk = r / mu;
-                if (pos + i < cap)
-                    work[pos + i] = make_int4((down ? kWorkWgradDown : kWorkWgradGateup) | (e << 8), seg[e], n_blk | ((r - n_blk * mu) << 16),
-                                              (totals[e] + BK - 1) / BK);       // blocks of padding add nothing
+                const int j = down ? i : i - E * per_wd, per = down ? per_wd : per_e - per_wd, nb = down ? a.nb_wd : a.nb_wg;
+                const int e = j / per, r = j - e * per, m_blk = r / nb;
+                if (items + i < cap)
+                    work[items + i] = make_int4((down ? kWorkWgradDown : kWorkWgradGateup) | (e << 8), seg[e], (r - m_blk * nb) | (m_blk << 16),
+                                         (totals[e] + BK - 1) / BK);       // blocks of padding add nothing
             }
-            pos += E * (per_wd + per_wg);
         }
-        if (gtid == 0) meta[kMetaWork + dir] = min(pos, cap);
+        if (gtid == 0) meta[kMetaWork + dir] = min(items + (dir == 1 ? E * per_e : 0), cap);
     }
     // ---- slots of this chunk's entries, places of its tokens in the token order
     if ((int)blockIdx.x >= a.p.chunks) return;
@@ -308,6 +322,7 @@ __global__ void __launch_bounds__(kRouteThreads) local_route_assign_kernel(const
 struct Phase {
     alignas(64) CUtensorMap map_a;
     alignas(64) CUtensorMap map_b;
+    alignas(64) CUtensorMap map_a32;     // the two GEMMs: 32 rows of A
     int nk, b_group_rows, cols, num_n_blocks, n_total, m_total;
 };
 
@@ -319,20 +334,18 @@ struct LayerArgsP {
     alignas(64) CUtensorMap st_dwd;
     alignas(64) CUtensorMap st_dwg;
     int T, K, H, I, E;
-    int dispatch_pairs, keep, out_rows;
+    int stages, stage_bytes, keep, out_rows;
     const uint8_t* x;
     uint8_t* slot_x;
     const __nv_bfloat16* y;
     __nv_bfloat16* saved_x;
     __nv_bfloat16* xperm;
     __nv_bfloat16* out;
-    const __nv_bfloat16* preact;
+    __nv_bfloat16* preact;               // forward (with keep): written, backward: read; preact_at()
     float* droute_part;
     int n_parts;
     float* dw_topk;
     const int* meta;
-    const int* seg;
-    const int* totals;
     const int* slot_tk;
     const float* slot_w;
     const int* token_order;              // tokens by their last expert
@@ -347,9 +360,6 @@ struct LayerArgsP {
     int* status;
 };
 
-__device__ __forceinline__ void red_add_relaxed_gpu(int* p, int v) {
-    asm volatile("red.relaxed.gpu.global.add.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
 __device__ __forceinline__ int atom_add_acq_rel(int* p, int v) {
     int old;
     asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
@@ -493,18 +503,28 @@ struct Staging {
     }
 };
 
-// First GEMM, forward: accumulator columns (2j, 2j+1) = (gate_j, up_j).  act = silu(g) * u * w; the pre-activation is kept for
-// backward (from a second read of tensor memory, which costs less than 32 registers to hold the activation).
+// The pre-activation that forward keeps for backward lies in blocks of 32 rows x 8 columns, a block's 16-byte row pieces one after the
+// other: an epilogue lane holds one row of the accumulator, so the warp's 32 lanes write, and in backward read, 512 consecutive bytes per
+// instruction, straight between registers and memory.  In rows of 2 I columns the forward needed two more boxes and a second read of
+// the accumulator per tile, and the backward turned what it read in shared memory, half a box at a time, between the stores of
+// its results: 12 round trips and 21-24 thousand cycles per 256-column tile, three times what the tensor cores take at H = 2048.
+__device__ __forceinline__ int4* preact_at(const LayerArgsP& L, int row0, int lane, int col) {
+    return reinterpret_cast<int4*>(L.preact) + ((long)(row0 >> 5) * (L.I >> 2) + (col >> 3)) * 32 + lane;
+}
+
+// First GEMM, forward: accumulator columns (2j, 2j+1) = (gate_j, up_j).  act = silu(g) * u * w.
 template <typename R>
-__device__ __forceinline__ void epilogue_swiglu(const LayerArgsP& L, const Staging& st, uint32_t taddr, int row0, bool live, int n0, R release) {
-    const float w = live ? L.slot_w[row0 + st.lane] : 0.f;
+__device__ __forceinline__ void epilogue_swiglu(const LayerArgsP& L, const Staging& st, uint32_t taddr, int row0, int n0, R release) {
+    const float w = L.slot_w[row0 + st.lane];
     const int n_total = 2 * L.I;
+    int4* keep = preact_at(L, row0, st.lane, n0);
     st.reuse();
 #pragma unroll 1
     for (int c = 0; c < 4; ++c) {
         uint32_t acc[32];
         tmem_ld_x32(taddr + (uint32_t)(c * 32), acc);
         tmem_ld_wait();
+        if (c == 3) release();
         uint32_t o[8];
 #pragma unroll
         for (int p = 0; p < 8; ++p) {
@@ -518,47 +538,37 @@ __device__ __forceinline__ void epilogue_swiglu(const LayerArgsP& L, const Stagi
         }
         st.put(2 * c, o[0], o[1], o[2], o[3]);
         st.put(2 * c + 1, o[4], o[5], o[6], o[7]);
+        if (L.keep && n0 + c * 32 < n_total) {
+#pragma unroll
+            for (int v = 0; v < 4; ++v) {
+                const uint32_t* a = acc + 8 * v;
+                keep[(4 * c + v) * 32] = make_int4((int)pack_bf16x2(__uint_as_float(a[0]), __uint_as_float(a[1])),
+                                                   (int)pack_bf16x2(__uint_as_float(a[2]), __uint_as_float(a[3])),
+                                                   (int)pack_bf16x2(__uint_as_float(a[4]), __uint_as_float(a[5])),
+                                                   (int)pack_bf16x2(__uint_as_float(a[6]), __uint_as_float(a[7])));
+            }
+        }
     }
-    if (!L.keep) release();
-    st.store(live && n0 < n_total, &L.st_act, n0 >> 1, row0);
-    if (!L.keep) return;
-#pragma unroll 1
-    for (int h = 0; h < 2; ++h) {
-        uint32_t a0[32], a1[32];
-        tmem_ld_x32(taddr + (uint32_t)(h * 64), a0);
-        tmem_ld_x32(taddr + (uint32_t)(h * 64 + 32), a1);
-        tmem_ld_wait();
-        if (h == 1) release();
-        st.reuse();
-        st.put32(0, a0);
-        st.put32(1, a1);
-        st.store(live && n0 + h * 64 < n_total, &L.st_aux, n0 + h * 64, row0);
-    }
+    st.store(n0 < n_total, &L.st_act, n0 >> 1, row0);
 }
 
 // First GEMM, backward: accumulator column j = d act_j.  Padding rows give zeros whatever the operands hold there: dGU and
-// act x route are operands of the weight gradients, which sum over whole 64-row blocks.
-//
-// The pre-activation comes in 32 rows x 64 columns at a time.  A lane needs its own row, but 32 lanes that each load their row touch
-// 32 lines per instruction: those loads alone held the tensor cores at 38 % of their rate during the first GEMM (H = 2048,
-// 54 % without them) and slowed the operand loads of the second.  So a warp loads whole 128-byte rows, one step ahead (the first
-// ones before the accumulator is ready), and turns them in the staging box, where dGU replaces them in place.  Stores
-// alternate between the two half boxes.
+// act x route are operands of the weight gradients, which sum over whole 64-row blocks.  The pre-activation comes 32 columns ahead, the
+// first of it before the accumulator is ready.  16 columns are computed before the box is waited for and written: with one 16-byte
+// piece at a time the exponentials of four columns were all that a warp had in flight.  Stores alternate between two half boxes.
 struct Preact {
-    int4 v[8];      // 16 bytes of rows 4 i + lane / 8, i = 0 .. 7
-    __device__ __forceinline__ void request(const LayerArgsP& L, int row0, int col, uint32_t rows, int lane) {
-        const int4* p = reinterpret_cast<const int4*>(L.preact + (long)(row0 + (lane >> 3)) * (2l * L.I) + 2 * col) + (lane & 7);
-        const long step = (long)L.I;                     // four rows in 16-byte units: 4 * 2I * 2 / 16
+    int4 v[8];      // 16-byte pieces of this lane's row: columns 8 i .. 8 i + 7 of 2 I
+    __device__ __forceinline__ void request(const LayerArgsP& L, int row0, int col, bool real, int lane) {
+        const int4* p = preact_at(L, row0, lane, 2 * col);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) v[i] = ((rows >> (4 * i + (lane >> 3))) & 1u) ? ld_nc_v4(p + i * step) : make_int4(0, 0, 0, 0);
+        for (int i = 0; i < 8; ++i) v[i] = real ? ld_nc_v4(p + 32 * i) : make_int4(0, 0, 0, 0);
     }
 };
 
 template <typename R>
-__device__ __forceinline__ void epilogue_dswiglu(const LayerArgsP& L, const Staging& st, uint32_t taddr, int row0, bool live, uint32_t rows, int n0,
+__device__ __forceinline__ void epilogue_dswiglu(const LayerArgsP& L, const Staging& st, uint32_t taddr, int row0, bool real, int n0,
                                                  int part, Preact& pre, R release) {
     const long row = row0 + st.lane;
-    const bool real = (rows >> st.lane) & 1u;
     const float w = real ? L.slot_w[row] : 0.f;
     float droute = 0.f;
     int turn = 0;
@@ -566,29 +576,22 @@ __device__ __forceinline__ void epilogue_dswiglu(const LayerArgsP& L, const Stag
 #pragma unroll 1
     for (int c = 0; c < 4; ++c) {
         const int col = n0 + c * 32;
-        const bool in = live && col < L.I;
+        const bool in = col < L.I;
         uint32_t acc[32];
         tmem_ld_x32(taddr + (uint32_t)(c * 32), acc);
         Preact next;
-        next.request(L, row0, col + 32, c < 3 && col + 32 < L.I ? rows : 0u, st.lane);
+        next.request(L, row0, col + 32, real && c < 3 && col + 32 < L.I, st.lane);
         tmem_ld_wait();
         if (c == 3) release();
         uint32_t act[16];
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-            st.reuse<1>();
-            if (((st.lane >> 2) & 1) == h) {
-#pragma unroll
-                for (int i = 0; i < 8; ++i)
-                    st_shared_v4(st.narrow_at(turn, 4 * i + (st.lane >> 3), st.lane & 3), (uint32_t)pre.v[i].x, (uint32_t)pre.v[i].y,
-                                 (uint32_t)pre.v[i].z, (uint32_t)pre.v[i].w);
-            }
-            __syncwarp();
+            uint32_t dgu[16];
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 const int v = 4 * h + i;
-                uint32_t pr[4], dgu[4];
-                ld_shared_v4(st.narrow_at(turn, st.lane, i), pr);
+                const int4 g = pre.v[v];
+                const uint32_t pr[4] = {(uint32_t)g.x, (uint32_t)g.y, (uint32_t)g.z, (uint32_t)g.w};
                 float av[4];
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
@@ -600,14 +603,16 @@ __device__ __forceinline__ void epilogue_dswiglu(const LayerArgsP& L, const Stag
                     const float gaw = ga * w;
                     const float d_up = s * gaw;
                     const float d_gate = (sig - s * sig + s) * gaw * gu.y;
-                    dgu[e] = pack_bf16x2(d_gate, d_up);
+                    dgu[4 * i + e] = pack_bf16x2(d_gate, d_up);
                     av[e] = a * w;
                     droute += ga * a;
                 }
-                st.put_narrow(turn, i, dgu[0], dgu[1], dgu[2], dgu[3]);
                 act[2 * v] = pack_bf16x2(av[0], av[1]);
                 act[2 * v + 1] = pack_bf16x2(av[2], av[3]);
             }
+            st.reuse<1>();
+#pragma unroll
+            for (int i = 0; i < 4; ++i) st.put_narrow(turn, i, dgu[4 * i], dgu[4 * i + 1], dgu[4 * i + 2], dgu[4 * i + 3]);
             st.store_narrow(turn++, in, &L.st_aux, 2 * col + 32 * h, row0);
         }
         st.reuse<1>();
@@ -616,32 +621,28 @@ __device__ __forceinline__ void epilogue_dswiglu(const LayerArgsP& L, const Stag
         st.store_narrow(turn++, in, &L.st_act, col, row0);
         pre = next;
     }
-    if (live) L.droute_part[row * L.n_parts + part] = droute;
+    L.droute_part[row * L.n_parts + part] = droute;
 }
 
-// 128 accumulator columns as two boxes; store_box(first column).  The accumulator is given back before anything is stored: what a
-// wide tile exposes is the time until then.
+// 128 accumulator columns as two boxes; store_box(first column).  The second half is read while the first box is stored, and the
+// accumulator is given back before the second box waits for the first: what a wide tile exposes is the time until then.
 template <typename R, typename F>
 __device__ __forceinline__ void epilogue_plain(const Staging& st, uint32_t taddr, bool zero, R release, F store_box) {
-    uint32_t packed[2][32];
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-        uint32_t a0[32], a1[32];
+        uint32_t a0[32], a1[32], packed[32];
         tmem_ld_x32(taddr + (uint32_t)(h * 64), a0);
         tmem_ld_x32(taddr + (uint32_t)(h * 64 + 32), a1);
         tmem_ld_wait();
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
-            packed[h][i] = zero ? 0u : pack_bf16x2(__uint_as_float(a0[2 * i]), __uint_as_float(a0[2 * i + 1]));
-            packed[h][16 + i] = zero ? 0u : pack_bf16x2(__uint_as_float(a1[2 * i]), __uint_as_float(a1[2 * i + 1]));
+            packed[i] = zero ? 0u : pack_bf16x2(__uint_as_float(a0[2 * i]), __uint_as_float(a0[2 * i + 1]));
+            packed[16 + i] = zero ? 0u : pack_bf16x2(__uint_as_float(a1[2 * i]), __uint_as_float(a1[2 * i + 1]));
         }
-    }
-    release();
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
+        if (h == 1) release();
         st.reuse();
 #pragma unroll
-        for (int c = 0; c < 8; ++c) st.put(c, packed[h][4 * c], packed[h][4 * c + 1], packed[h][4 * c + 2], packed[h][4 * c + 3]);
+        for (int c = 0; c < 8; ++c) st.put(c, packed[4 * c], packed[4 * c + 1], packed[4 * c + 2], packed[4 * c + 3]);
         store_box(h * 64);
     }
 }
@@ -654,33 +655,27 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
     uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
     const uint32_t bar_base = smem_base + kBarOffsetP;
     auto full_bar = [&](int s) { return bar_base + 8u * s; };
-    auto empty_bar = [&](int s) { return bar_base + 8u * (kStagesP + s); };
-    auto tfull_bar = [&](int s) { return bar_base + 8u * (2 * kStagesP + s); };
-    auto tempty_bar = [&](int s) { return bar_base + 8u * (2 * kStagesP + 2 + s); };
+    auto empty_bar = [&](int s) { return bar_base + 8u * (kMaxStages + s); };
+    auto tfull_bar = [&](int s) { return bar_base + 8u * (2 * kMaxStages + s); };
+    auto tempty_bar = [&](int s) { return bar_base + 8u * (2 * kMaxStages + 2 + s); };
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + kBarOffsetP + kOffTmem);
     volatile uint32_t* abort_flag = tmem_slot + 1;
-    auto copy_bar = [&](int w, uint32_t b) { return bar_base + kOffCopyBar + 8u * (2u * w + b); };
     auto ring_full = [&](int e) { return bar_base + kOffRingFull + 8u * e; };
     auto ring_empty = [&](int e) { return bar_base + kOffRingEmpty + 8u * e; };
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();
-    const int pair = blockIdx.x >> 1;
 
     if (threadIdx.x == 0) {
         *abort_flag = 0u;
-        for (int s = 0; s < kStagesP; ++s) {
+        for (int s = 0; s < kMaxStages; ++s) {
             mbar_init(full_bar(s), 2);
             mbar_init(empty_bar(s), 1);
         }
         for (int s = 0; s < 2; ++s) {
             mbar_init(tfull_bar(s), 1);
             mbar_init(tempty_bar(s), 2 * kEpiWarps);
-        }
-        for (int w = 0; w < kThreads / 32; ++w) {
-            mbar_init(copy_bar(w, 0), 1);
-            mbar_init(copy_bar(w, 1), 1);
         }
         for (int e = 0; e < kRingDepth; ++e) {
             mbar_init(ring_full(e), 1);
@@ -699,132 +694,110 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
     tcgen05_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 
-    const int num_units = min(L.meta[kMetaUnits], L.max_units);
     const int num_slots = L.meta[kMetaSlots];
     const int target1 = 2 * kEpiWarps * L.ph[0].num_n_blocks;         // epilogue warps that finish a unit's first GEMM,
     const int target2 = kEpiWarps * L.ph[1].num_n_blocks;             // a block's second GEMM
 
-    if (pair < L.dispatch_pairs) {
-        // ------------------------------------------------------------------ dispatch role (all 12 warps)
-        // A warp's leader streams rows through its two 8 KB buffers (in the operand stages, which nobody uses yet): global -> shared
-        // completes on the buffer's mbarrier, shared -> slot row joins a bulk group; the load of a chunk runs while the one
-        // before it is stored.  Rows are counted into their block in batches behind one completed group and one fence.
-        if (lane == 0) {
-            const int warps_total = L.dispatch_pairs * 2 * (kThreads / 32);
-            const int wid = (pair * 2 + (int)rank) * (kThreads / 32) + warp;
-            const uint32_t buf0 = smem_base + (uint32_t)warp * (2 * kCopyChunk);
-            const uint32_t row_bytes = (uint32_t)L.H * 2u;
-            uint32_t ph0 = 0, ph1 = 0, nchunk = 0;
-            bool ok = true, pend = false, pend_last = false;
-            uint64_t pend_dst = 0;
-            uint32_t pend_bytes = 0, pend_b = 0;
-            int pend_blk = 0, pub[kPublishBatch], npub = 0;
-            auto publish = [&]() {
-                if (npub == 0) return;
-                tma_store_wait<0>();
-                fence_proxy_async_all();
-                fence_acq_rel_gpu();
-#pragma unroll
-                for (int i = 0; i < kPublishBatch; ++i)
-                    if (i < npub) red_add_relaxed_gpu(L.arrived + pub[i], 1);
-                npub = 0;
-            };
-            auto store_pending = [&]() -> bool {
-                if (!pend) return true;
-                if (!mbar_wait(copy_bar(warp, pend_b), pend_b ? ph1 : ph0, abort_flag, L.status, 640)) return false;
-                if (pend_b) ph1 ^= 1u; else ph0 ^= 1u;
-                bulk_store_1d(pend_dst, buf0 + pend_b * kCopyChunk, pend_bytes);
-                tma_store_commit();
-                pend = false;
-                if (pend_last) {
-#pragma unroll
-                    for (int i = 0; i < kPublishBatch; ++i)
-                        if (i == npub) pub[i] = pend_blk;
-                    if (++npub == kPublishBatch) publish();
-                }
-                return true;
-            };
-            int next_tk = wid < num_slots ? L.slot_tk[wid] : -1;
-            for (int s = wid; ok && s < num_slots; s += warps_total) {
-                const int tk = next_tk;
-                next_tk = s + warps_total < num_slots ? L.slot_tk[s + warps_total] : -1;
-                if (tk < 0) continue;
-                const uint8_t* src = L.x + (size_t)(tk / L.K) * row_bytes;
-                const uint64_t dst = reinterpret_cast<uint64_t>(L.slot_x) + (uint64_t)s * row_bytes;
-                for (uint32_t off = 0; off < row_bytes; off += kCopyChunk) {
-                    const uint32_t chunk = min((uint32_t)kCopyChunk, row_bytes - off);
-                    const uint32_t b = nchunk & 1u;
-                    tma_store_wait_read<0>();
-                    mbar_arrive_expect_tx(copy_bar(warp, b), chunk);
-                    bulk_load_1d(buf0 + b * kCopyChunk, src + off, chunk, copy_bar(warp, b));
-                    ++nchunk;
-                    if (!(ok = store_pending())) break;
-                    pend = true;
-                    pend_b = b;
-                    pend_dst = dst + off;
-                    pend_bytes = chunk;
-                    pend_last = off + kCopyChunk >= row_bytes;
-                    pend_blk = s >> 7;
-                }
-            }
-            if (ok) ok = store_pending();
-            if (ok) publish();
-            tma_store_wait<0>();
-        }
-        __syncwarp();
-        cluster_sync_all();                   // both CTAs of the pair are done with the staging buffers: they become operand stages
-    }
-
-    // ---------------------------------------------------------------------- gather role
+    // ---------------------------------------------------------------------- copy role
+    // Rows into slot order.  All warps but the producer's and the issuer's start with one slot each, so that the first units are in place
+    // after the latency of one row; the rest is claimed by the gather warps, eight slots at a time.  A warp has 8 KB of loads in
+    // flight: rows of 4096 columns and more one after the other, shorter ones several at once.  (Before, the first pairs of CTAs
+    // streamed rows through shared memory and joined the GEMMs afterwards; rows of 1 KB left them waiting for one row at a time:
+    // 8531 tokens, H=512, top-8 spent 240 us there.)
     const int nvec = L.H / 8;
-    auto clear_padding = [&](int s) {
-        int4* row = reinterpret_cast<int4*>(L.slot_x) + (long)s * nvec;
-        for (int i = lane; i < nvec; i += 32) row[i] = make_int4(0, 0, 0, 0);
-    };
-    auto clear_all_padding = [&]() {
-        // Forward: what stands in padding rows reaches no result, so nothing waits for this.  But the tensor cores multiply these
-        // rows too, and multiplying leftovers of earlier calls costs power, which is what limits large layers.
-        const int warps = gridDim.x * 2, gw = blockIdx.x * 2 + (warp - 2);
-        const int share = max(1, warps / L.E);
-        for (int e = gw / share; e < L.E; e += (warps + share - 1) / share)
-            for (int s = L.seg[e] + L.totals[e] + gw % share; s < L.seg[e + 1]; s += share) clear_padding(s);
-    };
-    auto copy_x_loop = [&]() {
-        // forward: backward's copy of x, eight rows per claim
-        while (true) {
-            int t0 = 0;
-            if (lane == 0) t0 = atomicAdd(L.sync + kSyncCopy, 8);
-            t0 = __shfl_sync(0xffffffffu, t0, 0);
-            if (t0 >= L.T) break;
-            for (int t = t0; t < min(t0 + 8, L.T); ++t)
-                copy_row_deep(reinterpret_cast<int4*>(L.saved_x + (long)t * L.H), reinterpret_cast<const int4*>(L.x) + (long)t * nvec, nvec, lane);
+    auto copy_slots = [&](const int4* src, int4* dst, int row, uint32_t wanted, int s0, int n) {
+        // row: source row of slot s0 + lane, -1 = zeros
+        if (nvec >= 512) {
+            for (int r = 0; r < n; ++r) {
+                if (!((wanted >> r) & 1u)) continue;
+                const int sr = __shfl_sync(0xffffffffu, row, r);
+                int4* d = dst + (long)(s0 + r) * nvec;
+                if (sr >= 0) copy_row_deep(d, src + (long)sr * nvec, nvec, lane);
+                else for (int i = lane; i < nvec; i += 32) d[i] = make_int4(0, 0, 0, 0);
+            }
+            return;
+        }
+        const int total = n * nvec;
+        for (int b = 0; b < total; b += 512) {
+            int4 v[16];
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+                const int idx = min(b + 32 * i + lane, total - 1), r = idx / nvec;
+                const int sr = __shfl_sync(0xffffffffu, row, r);
+                v[i] = ld_nc_v4(src + (long)max(sr, 0) * nvec + (idx - r * nvec));
+                if (sr < 0) v[i] = make_int4(0, 0, 0, 0);
+            }
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+                const int idx = b + 32 * i + lane;
+                if (idx < total && ((wanted >> (idx / nvec)) & 1u)) dst[(long)s0 * nvec + idx] = v[i];
+            }
         }
     };
-    auto expand_loop = [&]() {
-        // backward: x in slot order (operand of dW_gateup) and zeros in the padding rows of both slot-order operands
+    auto count_rows = [&](int* counter, int n) {
+        __syncwarp();
+        if (lane == 0 && n > 0) {
+            fence_acq_rel_gpu();
+            red_add_release_gpu(counter, n);
+        }
+    };
+    auto place = [&](int s0, int n) {
+        const int tk = lane < n ? L.slot_tk[s0 + lane] : -1;
+        const int row = tk >= 0 ? tk / L.K : -1;
+        uint32_t wanted = __ballot_sync(0xffffffffu, tk >= 0);
+        if constexpr (BWD) {
+            // both slot-order tables are operands of the weight gradients, which sum over 64 rows at a time: rows of zeros to the next 64
+            wanted = L.slot_tk[s0 & ~63] >= 0 ? (1u << n) - 1u : 0u;
+        }
+        if (wanted == 0u) return;
+        copy_slots(reinterpret_cast<const int4*>(L.x), reinterpret_cast<int4*>(L.slot_x), row, wanted, s0, n);
+        count_rows(L.arrived + (s0 >> 7), __popc(wanted));
+    };
+    auto place_x = [&](int s0, int n) {
+        const int tk = lane < n ? L.slot_tk[s0 + lane] : -1;
+        if (L.slot_tk[s0 & ~63] < 0) return;
+        copy_slots(reinterpret_cast<const int4*>(L.saved_x), reinterpret_cast<int4*>(L.xperm), tk >= 0 ? tk / L.K : -1, (1u << n) - 1u, s0, n);
+        count_rows(L.sync + kSyncRows, n);
+    };
+    // (neighbouring slots go to different SMs: a few rows in one SM would queue behind one another)
+    const int first_slots = (int)gridDim.x * kCopyWarps * kFirstRows / kCopyRows * kCopyRows;
+    if (warp >= 2) {
+        const int s0 = ((warp - 2) * (int)gridDim.x + (int)blockIdx.x) * kFirstRows;
+        if (s0 < min(num_slots, first_slots)) place(s0, kFirstRows);
+    }
+    auto copy_loop = [&]() {
         while (true) {
             int s0 = 0;
-            if (lane == 0) s0 = atomicAdd(L.sync + kSyncExpand, 8);
+            if (lane == 0) s0 = first_slots + atomicAdd(L.sync + kSyncCopy, kCopyRows);
             s0 = __shfl_sync(0xffffffffu, s0, 0);
             if (s0 >= num_slots) break;
-            const int s1 = min(s0 + 8, num_slots);
-            for (int s = s0; s < s1; ++s) {
-                const int tk = L.slot_tk[s];
-                int4* dst = reinterpret_cast<int4*>(L.xperm + (long)s * L.H);
-                if (tk >= 0) {
-                    copy_row_deep(dst, reinterpret_cast<const int4*>(L.saved_x + (long)(tk / L.K) * L.H), nvec, lane);
-                } else {
-                    for (int i = lane; i < nvec; i += 32) dst[i] = make_int4(0, 0, 0, 0);
-                    clear_padding(s);
-                }
-            }
-            __syncwarp();
-            if (lane == 0) {
-                fence_acq_rel_gpu();
-                red_add_release_gpu(L.sync + kSyncExpanded, s1 - s0);
-            }
+            place(s0, kCopyRows);
         }
     };
+    auto copy_x_loop = [&]() {
+        // backward: x in slot order, which nothing needs before the weight gradients
+        while (true) {
+            int s0 = 0;
+            if (lane == 0) s0 = atomicAdd(L.sync + kSyncKeep, kCopyRows);
+            s0 = __shfl_sync(0xffffffffu, s0, 0);
+            if (s0 >= num_slots) break;
+            place_x(s0, kCopyRows);
+        }
+    };
+    auto keep_x_loop = [&]() {
+        // forward: backward's copy of x
+        const int chunk = kCopyRows;
+        while (true) {
+            int t0 = 0;
+            if (lane == 0) t0 = atomicAdd(L.sync + kSyncKeep, chunk);
+            t0 = __shfl_sync(0xffffffffu, t0, 0);
+            if (t0 >= L.T) break;
+            const int n = min(chunk, L.T - t0);
+            copy_slots(reinterpret_cast<const int4*>(L.x), reinterpret_cast<int4*>(L.saved_x), t0 + min(lane, n - 1), (1u << n) - 1u, t0, n);
+        }
+    };
+
+    // ---------------------------------------------------------------------- gather role
     // Rows [k0, k0 + n) of a token's entries, columns v and v + 32: all loads are issued before the first is used (16 in flight
     // per lane; a load behind a lane-dependent branch would be waited for one at a time, so out-of-range columns are clamped
     // and only their stores are left out).
@@ -868,15 +841,25 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
         const bool stamps = L.stats != nullptr && lane == 0;
         // claimed one task ahead, with the token's slots, so that a task starts with the test of its counters
         int next_i = tasks, next_t = 0, next_slot = -1;
+        // Few tasks are dealt out to all warps that gather in the end: they become ready together, and an atomic per task would be
+        // half of what is left to do by then.
+        const int warps = (int)gridDim.x * kCopyWarps;
+        const bool dealt = !BWD && tasks <= 4 * warps;           // (backward they run under the weight gradients)
+        next_i = dealt ? (int)blockIdx.x * kCopyWarps + (warp - 2) - warps : 0;
         auto claim = [&]() {
-            if (lane == 0) next_i = atomicAdd(L.sync + kSyncToken, 1);
-            next_i = __shfl_sync(0xffffffffu, next_i, 0);
+            if (dealt) {
+                next_i += warps;
+            } else {
+                if (lane == 0) next_i = atomicAdd(L.sync + kSyncToken, 1);
+                next_i = __shfl_sync(0xffffffffu, next_i, 0);
+            }
             if (next_i < tasks) {
                 next_t = L.token_order[next_i / parts];
                 next_slot = lane < K ? L.order_slot[(long)(next_i / parts) * K + lane] : -1;
             }
         };
         if (L.T > 0) claim();
+        else next_i = tasks;
         while (next_i < tasks) {
             const int part = next_i % parts, t = next_t, slot = next_slot;
             claim();
@@ -984,7 +967,7 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                     } else {
                         if (blocking) {
                             if (!mbar_wait(ring_full(ss), sph, abort_flag, L.status, 651)) return -1;
-                        } else if (!mbar_try_wait(ring_full(ss), sph)) {
+                        } else if (!mbar_test_wait(ring_full(ss), sph)) {
                             return 0;
                         }
                         it = make_int4(ring[4 * ss], ring[4 * ss + 1], ring[4 * ss + 2], ring[4 * ss + 3]);
@@ -1005,10 +988,11 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                 auto operands_ready = [&](const Item& q, bool block) -> int {
                     if (q.kind == kWorkGemm1) return (!q.live || q.need == 0) ? 1 : counted(L.arrived + q.m0 / BM, q.need, block, 600, w_arrive);
                     if (q.kind == kWorkGemm2) return counted(L.done1 + q.unit, target1, block, 601, w_unit);
-                    // the weight gradients sit behind all first GEMMs in the list: one check per pair is enough
+                    // the weight gradients sit behind all first GEMMs in the list: one check per pair is enough (two loads per expert and pair
+                    // would cost as much as the smallest of these items)
                     if (wgrad_ready) return 1;
-                    const int a = counted(L.sync + kSyncExpanded, num_slots, block, 603, w_wgrad);
-                    const int b = a == 1 ? counted(L.sync + kSyncUnits, num_units, block, 602, w_wgrad) : a;
+                    const int a = counted(L.sync + kSyncRows, L.meta[kMetaRows], block, 603, w_wgrad);
+                    const int b = a == 1 ? counted(L.sync + kSyncUnits, L.meta[kMetaUnits], block, 602, w_wgrad) : a;
                     wgrad_ready = b == 1;
                     return b;
                 };
@@ -1044,17 +1028,24 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                     if (q.kind <= kWorkGemm2 || !wgrad_fenced) fence_proxy_async_all();
                     if (q.kind > kWorkGemm2) wgrad_fenced = true;
                     const int n0 = q.n0 + (int)rank * (BN / 2);
-                    const int look_kb = min(kStagesP - 1, q.nk - 1);   // all stages are in flight: a pause of this thread costs nothing
+                    const int look_kb = min(L.stages - 1, q.nk - 1);   // all stages are in flight: a pause of this thread costs nothing
                     for (int kb = 0; kb < q.nk; ++kb) {
                         if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag, L.status, 610)) { ok = false; break; }
-                        const uint32_t a_dst = smem_base + stage * kStageBytesP;
+                        const uint32_t a_dst = smem_base + stage * L.stage_bytes;
                         const uint32_t b_dst = a_dst + kAStageBytes;
                         const uint32_t bar = mapa_shared(full_bar(stage), 0);
                         if (rank == 0) mbar_arrive_expect_tx(full_bar(stage), 2u * (uint32_t)(kAStageBytes + q.halves * kBHalfBytesP));
                         else mbar_arrive_cluster(bar);
                         const int k = q.k0 + kb * BK;
                         if (q.kind <= kWorkGemm2) {
-                            tma_load_2d_2cta(a_dst, &P.map_a, bar, k, q.live ? q.m0 : L.out_rows);     // no rows: past the end reads zeros
+                            // rows that nothing waits for are not read: past the end of the table reads zeros
+                            if (q.need > 96 || q.need == 0) {
+                                tma_load_2d_2cta(a_dst, &P.map_a, bar, k, q.need > 0 ? q.m0 : L.out_rows);
+                            } else {
+#pragma unroll
+                                for (int b = 0; b < 4; ++b)
+                                    tma_load_2d_2cta(a_dst + b * (kAStageBytes / 4), &P.map_a32, bar, k, 32 * b < q.need ? q.m0 + 32 * b : L.out_rows);
+                            }
                         } else {
 #pragma unroll
                             for (int a = 0; a < BM / 64; ++a) tma_load_2d_2cta(a_dst + a * kAtomBytes, &P.map_a, bar, q.m0 + 64 * a, k);
@@ -1070,7 +1061,7 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                                 for (int a = 0; a < BN / 128; ++a) tma_load_2d_2cta(dst + a * kAtomBytes, &P.map_b, bar, col + 64 * a, krow);
                             }
                         }
-                        if (++stage == kStagesP) { stage = 0; phase ^= 1u; }
+                        if (++stage == L.stages) { stage = 0; phase ^= 1u; }
                         // (the second CTA keeps looking until the first one has published the item)
                         if (kb >= look_kb && !have && (kb == look_kb || rank != 0) && !look_ahead()) { ok = false; break; }
                     }
@@ -1100,19 +1091,18 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                 const int slot0 = acc & 1, slot1 = slot0 ^ 1;
                 const uint32_t parity0 = ((acc >> 1) & 1) ^ 1u, parity1 = (((acc + 1) >> 1) & 1) ^ 1u;
                 acc += q.halves;
+                // Operand descriptors of stage 0; a stage or a step of K further on is an addition to their address field.
+                const uint64_t a_base = make_smem_desc_sw128(smem_base, a_mn ? kAtomBytes : 0, 1024);
+                const uint64_t b_base = make_smem_desc_sw128(smem_base + kAStageBytes, BWD ? kAtomBytes : 0, 1024);
+                const uint32_t a_step = (a_mn ? UK * 128 : UK * 2) >> 4, b_step = (BWD ? UK * 128 : UK * 2) >> 4;
                 // 64 columns of K of one half of the tile
                 auto multiply = [&](int s, int h, int slot, bool first) {
-                    const uint32_t a_addr = smem_base + s * kStageBytesP;
-                    const uint32_t b_addr = a_addr + kAStageBytes + h * kBHalfBytesP;
+                    const uint32_t off = (uint32_t)(s * L.stage_bytes) >> 4;
+                    const uint64_t a_desc = a_base + off, b_desc = b_base + off + (uint32_t)(h * (kBHalfBytesP >> 4));
                     const uint32_t d_tmem = tmem_base + (uint32_t)(slot * BN);
 #pragma unroll
-                    for (int k = 0; k < BK / UK; ++k) {
-                        const uint64_t a_desc = a_mn ? make_smem_desc_sw128(a_addr + k * (UK * 128), kAtomBytes, 1024)
-                                                     : make_smem_desc_sw128(a_addr + k * (UK * 2), 0, 1024);
-                        const uint64_t b_desc = BWD ? make_smem_desc_sw128(b_addr + k * (UK * 128), kAtomBytes, 1024)
-                                                    : make_smem_desc_sw128(b_addr + k * (UK * 2), 0, 1024);
-                        umma_bf16_ss_2cta(d_tmem, a_desc, b_desc, idesc, (!first || k > 0) ? 1u : 0u);
-                    }
+                    for (int k = 0; k < BK / UK; ++k)
+                        umma_bf16_ss_2cta(d_tmem, a_desc + k * a_step, b_desc + k * b_step, idesc, (!first || k > 0) ? 1u : 0u);
                 };
                 if (!mbar_wait(tempty_bar(slot0), parity0, abort_flag, L.status, 620)) { ok = false; break; }
                 tcgen05_fence_after();
@@ -1120,7 +1110,7 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                 if (q.halves == 2) {
                     // The second accumulator is still being read out when a wide tile starts: the first half runs ahead over the stages
                     // that are there, the second half follows and frees them.
-                    const int lead = min(q.nk, kStagesP);
+                    const int lead = min(q.nk, L.stages);
                     int s = stage;
                     uint32_t ph = phase;
                     for (int i = 0; i < lead; ++i) {
@@ -1131,7 +1121,7 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                             if (i == q.nk - 1) umma_commit_2cta(tfull_bar(slot0), 3u);
                         }
                         __syncwarp();
-                        if (++s == kStagesP) { s = 0; ph ^= 1u; }
+                        if (++s == L.stages) { s = 0; ph ^= 1u; }
                     }
                     if (!ok || !mbar_wait(tempty_bar(slot1), parity1, abort_flag, L.status, 622)) { ok = false; break; }
                     tcgen05_fence_after();
@@ -1142,7 +1132,7 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                             if (kb == q.nk - 1) umma_commit_2cta(tfull_bar(slot1), 3u);
                         }
                         __syncwarp();
-                        if (++stage == kStagesP) { stage = 0; phase ^= 1u; }
+                        if (++stage == L.stages) { stage = 0; phase ^= 1u; }
                     }
                 }
                 for (; kb < q.nk; ++kb) {
@@ -1159,7 +1149,7 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                         if (last) umma_commit_2cta(tfull_bar(q.halves == 2 ? slot1 : slot0), 3u);
                     }
                     __syncwarp();
-                    if (++stage == kStagesP) { stage = 0; phase ^= 1u; }
+                    if (++stage == L.stages) { stage = 0; phase ^= 1u; }
                 }
                 if (ok && q.nk == 0) {                       // an expert without rows: the epilogue stores zeros
                     if (elect_one()) {
@@ -1184,7 +1174,6 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
             // one that waits for this count.
             uint32_t owed[kOwed];
             int n_owed = 0;
-            bool owed_first = false;          // a first GEMM's tile is among them: second GEMMs may be waiting for it, so it goes out with the next item
             auto flush = [&]() {
                 if (n_owed == 0) return;
                 __syncwarp();
@@ -1196,29 +1185,27 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                     for (int i = 0; i < kOwed; ++i) {
                         if (i >= n_owed) break;
                         const int at = (int)(owed[i] & 0x7fffffffu);
-                        if (owed[i] >> 31) {
-                            if (atom_add_acq_rel(L.done1 + at, 1) == target1 - 1) red_add_release_gpu(L.sync + kSyncUnits, 1);
-                        } else {
-                            red_add_release_gpu(L.done2 + at, 1);
-                        }
+                        if (!(owed[i] >> 31)) red_add_release_gpu(L.done2 + at, 1);
+                        else if (!BWD) red_add_release_gpu(L.done1 + at, 1);
+                        else if (atom_add_acq_rel(L.done1 + at, 1) == target1 - 1) red_add_release_gpu(L.sync + kSyncUnits, 1);
                     }
                 }
                 n_owed = 0;
-                owed_first = false;
             };
             while (ok) {
                 int4 it;
-                if (n_owed != 0 && !__all_sync(0xffffffffu, mbar_try_wait(ring_full(ss), sph))) flush();
+                if (n_owed != 0 && !__all_sync(0xffffffffu, mbar_test_wait(ring_full(ss), sph))) flush();
                 if (!next_item(ss, sph, 653, it) || it.x < 0) break;
                 const bool stamps = L.stats != nullptr && warp == 4 && lane == 0 && rank == 0;
                 Item q;
                 decode_item(L, it, rank, q);
                 if (stamps) atomicMax(L.stats + kStatKindFirst + q.kind, ~globaltimer_ns());
+                if (q.kind > kWorkGemm2) flush();  // (the weight gradients may never wait, and the sums run under them)
                 const int row0 = q.m0 + qd * 32;
-                uint32_t rows = 0;                 // backward, first GEMM: which of this warp's 32 rows are real
-                if constexpr (BWD) {
-                    if (q.kind == kWorkGemm1) rows = __ballot_sync(0xffffffffu, q.live && L.slot_tk[row0 + lane] >= 0);
-                }
+                // rows of a block beyond those that are used are neither computed on nor stored
+                const bool live = q.kind > kWorkGemm2 || (q.live && qd * 32 < q.need);
+                bool real = false;                 // backward, first GEMM: this lane's row is not padding
+                if constexpr (BWD) real = q.kind == kWorkGemm1 && live && L.slot_tk[row0 + lane] >= 0;
                 for (int h = 0; h < q.halves; ++h) {
                     const int slot = acc & 1;
                     const uint32_t parity = (acc >> 1) & 1;
@@ -1226,9 +1213,9 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                     const int n0 = q.n0 + h * BN + hh * (BN / 2);
                     Preact pre;
                     if constexpr (BWD) {
-                        if (q.kind == kWorkGemm1) pre.request(L, row0, n0, n0 < L.I ? rows : 0u, lane);
+                        if (q.kind == kWorkGemm1) pre.request(L, row0, n0, real && n0 < L.I, lane);
                     }
-                    if (n_owed != 0 && (n_owed == kOwed || owed_first || !__all_sync(0xffffffffu, mbar_try_wait(tfull_bar(slot), parity)))) flush();
+                    if (n_owed != 0 && (n_owed == kOwed || !__all_sync(0xffffffffu, mbar_test_wait(tfull_bar(slot), parity)))) flush();
                     if (!mbar_wait(tfull_bar(slot), parity, abort_flag, L.status, 630)) { ok = false; break; }
                     tcgen05_fence_after();
                     const uint32_t taddr = tmem_base + ((uint32_t)(qd * 32) << 16) + (uint32_t)(slot * BN + hh * (BN / 2));
@@ -1238,15 +1225,17 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                         __syncwarp();
                         if (lane == 0) mbar_arrive_cluster(mapa_shared(tempty_bar(slot), 0));
                     };
-                    if (q.kind == kWorkGemm1) {
-                        if constexpr (BWD) epilogue_dswiglu(L, st, taddr, row0, q.live, rows, n0, n0 / (BN / 2), pre, release);
-                        else epilogue_swiglu(L, st, taddr, row0, q.live, n0, release);
+                    if (!live) {
+                        release();
+                    } else if (q.kind == kWorkGemm1) {
+                        if constexpr (BWD) epilogue_dswiglu(L, st, taddr, row0, real, n0, n0 / (BN / 2), pre, release);
+                        else epilogue_swiglu(L, st, taddr, row0, n0, release);
                     } else if (q.kind == kWorkGemm2) {
                         epilogue_plain(st, taddr, false, release, [&](int c) {
-                            st.store(q.live && n0 + c < L.H, &L.st_y, n0 + c, row0);
+                            st.store(n0 + c < L.H, &L.st_y, n0 + c, row0);
                         });
                         if constexpr (BWD) {
-                            if (q.live && n0 == 0) {
+                            if (n0 == 0) {
                                 // this row's d(route weight): the sum of the first GEMM's partials
                                 const long row = row0 + lane;
                                 const int tk = L.slot_tk[row];
@@ -1276,7 +1265,6 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                     for (int i = 0; i < kOwed; ++i)
                         if (i == n_owed) owed[i] = entry;
                     ++n_owed;
-                    owed_first |= q.kind == kWorkGemm1;
                 }
             }
             flush();
@@ -1284,12 +1272,9 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
             __syncwarp();
             if (ok) gather_loop();            // the list is done: help with the sums
         } else if (warp >= 2) {
-            if constexpr (BWD) {
-                expand_loop();
-            } else {
-                clear_all_padding();
-                if (L.saved_x != nullptr) copy_x_loop();
-            }
+            copy_loop();
+            if (BWD) copy_x_loop();
+            else if (L.saved_x != nullptr) keep_x_loop();
             gather_loop();
         }
     }
@@ -1398,7 +1383,7 @@ LocalLayerPlan local_layer_plan(int T, int K, int E, int H, int I, int keep) {
     p.totals = take(E);
     p.last_hist = take(E + 1);
     p.zero_words = at;
-    p.meta = take(4);
+    p.meta = take(kMetaWords);
     p.seg = take(E + 1);
     p.slot_tk = take(p.slots_cap);
     p.slot_w = take(p.slots_cap);
@@ -1453,22 +1438,21 @@ cudaError_t local_layer_launch(const LocalLayerParams& q, cudaStream_t stream) {
     g1.nk = H / BK;
     g1.cols = p.cols[dir][0];
     g2.n_total = H; g2.cols = p.cols[dir][1]; g2.num_n_blocks = column_blocks(H, g2.cols);
-    if ((e = make_map(&g1.map_a, q.slot_x, R, H, BK, BM)) != cudaSuccess) return e;
+    if ((e = make_map(&g1.map_a, q.slot_x, R, H, BK, BM)) != cudaSuccess || (e = make_map(&g1.map_a32, q.slot_x, R, H, BK, 32)) != cudaSuccess) return e;
     if (q.bwd && (e = make_map_narrow(&L.st_aux, q.aux, R, 2 * I)) != cudaSuccess) return e;
     if ((e = q.bwd ? make_map_narrow(&L.st_act, q.act, R, I) : make_map(&L.st_act, q.act, R, I, 64, 32)) != cudaSuccess) return e;
     if ((e = make_map(&L.st_y, q.y, R, H, 64, 32)) != cudaSuccess) return e;
     if (!q.bwd) {
         // gate_up: A = rows in slot order, B = W_gateup [E*2I, H] K-major;  down: A = act, B = W_down [E*H, I] K-major
         if ((e = make_map(&g1.map_b, q.w_gateup, (uint64_t)E * 2 * I, H, BK, BN / 2)) != cudaSuccess) return e;
-        if ((e = make_map(&g2.map_a, q.act, R, I, BK, BM)) != cudaSuccess) return e;
+        if ((e = make_map(&g2.map_a, q.act, R, I, BK, BM)) != cudaSuccess || (e = make_map(&g2.map_a32, q.act, R, I, BK, 32)) != cudaSuccess) return e;
         if ((e = make_map(&g2.map_b, q.w_down, (uint64_t)E * H, I, BK, BN / 2)) != cudaSuccess) return e;
         g1.n_total = 2 * I; g1.b_group_rows = 2 * I;
         g2.nk = I / BK; g2.b_group_rows = H;
-        if (p.keep && (e = make_map(&L.st_aux, q.aux, R, 2 * I, 64, 32)) != cudaSuccess) return e;
     } else {
         // grad_act: A = dY, B = W_down MN-major;  dX: A = dGU, B = W_gateup MN-major
         if ((e = make_map(&g1.map_b, q.w_down, (uint64_t)E * H, I, 64, BK)) != cudaSuccess) return e;
-        if ((e = make_map(&g2.map_a, q.aux, R, 2 * I, BK, BM)) != cudaSuccess) return e;
+        if ((e = make_map(&g2.map_a, q.aux, R, 2 * I, BK, BM)) != cudaSuccess || (e = make_map(&g2.map_a32, q.aux, R, 2 * I, BK, 32)) != cudaSuccess) return e;
         if ((e = make_map(&g2.map_b, q.w_gateup, (uint64_t)E * 2 * I, H, 64, BK)) != cudaSuccess) return e;
         g1.n_total = I; g1.b_group_rows = H;
         g2.nk = 2 * I / BK; g2.b_group_rows = 2 * I;
@@ -1492,13 +1476,11 @@ cudaError_t local_layer_launch(const LocalLayerParams& q, cudaStream_t stream) {
     L.saved_x = static_cast<__nv_bfloat16*>(q.saved_x);
     L.xperm = static_cast<__nv_bfloat16*>(q.xperm);
     L.out = static_cast<__nv_bfloat16*>(q.out);
-    L.preact = static_cast<const __nv_bfloat16*>(q.preact);
+    L.preact = static_cast<__nv_bfloat16*>(q.preact);
     L.droute_part = q.droute_part;
     L.n_parts = 2 * ((I + BN - 1) / BN);
     L.dw_topk = q.dw_topk;
     L.meta = q.ws + p.meta;
-    L.seg = q.ws + p.seg;
-    L.totals = q.ws + p.totals;
     L.slot_tk = q.ws + p.slot_tk;
     L.slot_w = reinterpret_cast<const float*>(q.ws + p.slot_w);
     L.token_order = q.ws + p.token_order;
@@ -1514,7 +1496,10 @@ cudaError_t local_layer_launch(const LocalLayerParams& q, cudaStream_t stream) {
     L.status = q.status;
     const int sms = default_sms(q.num_sms) & ~1;
     if (sms < 4) return cudaErrorInvalidConfiguration;
-    L.dispatch_pairs = q.dispatch_pairs < 1 ? 1 : q.dispatch_pairs > sms / 2 - 1 ? sms / 2 - 1 : q.dispatch_pairs;
+    bool wide = false;
+    for (int k = 0; k < (q.bwd ? 4 : 2); ++k) wide |= L.ph[k].cols > BN;
+    L.stages = wide ? 4 : 6;
+    L.stage_bytes = wide ? kWideStageBytes : kNarrowStageBytes;
     return q.bwd ? launch<true>(L, sms, stream) : launch<false>(L, sms, stream);
 }
 

@@ -31,7 +31,7 @@ struct LocalLayerParams {
     int idx_is64;
     const float* topk_w;                 // forward
     // schedule
-    int group_units, lag_percent, min_lag_items, dispatch_pairs, num_sms;
+    int group_units, lag_percent, min_lag_items, num_sms;
     int bwd;
     const void* x;                       // [T, H] forward x, backward grad_out
     const void* w_gateup;
@@ -40,11 +40,11 @@ struct LocalLayerParams {
     void* y;                             // [out_rows, H] second GEMM's output in slot order
     int out_rows;                        // rows of the slot-order tensors: max(slots_cap, 128)
     void* act;                           // forward act, backward act x route [out_rows, I]
-    void* aux;                           // forward preact (may be null without keep), backward dGU [out_rows, 2I]
+    void* aux;                           // backward dGU [out_rows, 2I]
     void* saved_x;                       // [T, H] copy of x: written by forward (may be null), read by backward
     void* out;                           // [T, H]
+    void* preact;                        // written by forward (with keep), read by backward: 2I * out_rows values in 32 x 8 blocks
     // backward
-    const void* preact;
     float* droute_part;                  // [out_rows, 2 * ceil(I / 256)]
     void* xperm;                         // [out_rows, H]
     float* dw_topk;                      // [T, K]

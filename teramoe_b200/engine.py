@@ -637,7 +637,7 @@ class EPEngine:
     def local_layer(self, x, topk_idx, topk_weights, W_gateup, W_down, num_experts: int, opts: tuple, owner, autograd: bool,
                     grad_topk_weights=None):
         """The layer as one native call per direction, or None where another path has to take it: several ranks, sizes or types that
-        the kernels do not take, or a switch that asks for other kernels.  opts: (num_dispatch_sms, total_sms, compute_batch_size,
+        the kernels do not take, or a switch that asks for other kernels.  opts: (total_sms, compute_batch_size,
         combine_start_head_percent); owner: what has to stay alive until a backward pass is done."""
         if self.native is None or LAYER_WIRE != "entry" or "0" in (_LOCAL_LAYER_MODE, _LAYER_KERNEL_MODE, _FUSED_DISPATCH_MODE, _FUSED_MODE):
             return None
@@ -646,10 +646,9 @@ class EPEngine:
             return None
         schedule = self._schedules.get(opts)
         if schedule is None:
-            # units per batch, lag percent, least lag in items, dispatch pairs, SMs (see layer_kernel_gen)
-            sms = self._grid_sms({"total_sms": opts[1]})
-            schedule = [max(1, opts[2] // UNIT_ROWS), opts[3], int(LAYER_MIN_LAG_PER_PAIR * ((sms or self._num_sms) // 2)),
-                        dispatch_pairs(0, opts[0]), sms]
+            # units per batch, lag percent, least lag in items, SMs (see layer_kernel_gen)
+            sms = self._grid_sms({"total_sms": opts[0]})
+            schedule = [max(1, opts[1] // UNIT_ROWS), opts[2], int(LAYER_MIN_LAG_PER_PAIR * ((sms or self._num_sms) // 2)), sms]
             self._schedules[opts] = schedule
         traced = self._trace is not None or NVTX_MARKS
         if traced:

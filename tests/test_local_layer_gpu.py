@@ -62,6 +62,32 @@ def test_one_rank_layer_matches_general_kernels_and_oracle(T, H, I, E, K, skew, 
     buf.destroy()
 
 
+@pytest.mark.parametrize("H,I", [(192, 128), (4160, 64)])         # rows copied several at once, and one after the other
+def test_rows_per_expert_at_the_edges_of_operand_boxes(H, I, monkeypatch):
+    """An expert's rows are loaded 32 at a time up to 96 and 128 at a time above, summed 64 at a time, and stored 32 at a time."""
+    from teramoe_b200 import engine
+    counts = [1, 0, 31, 32, 33, 63, 64, 65, 95, 96, 97, 127, 128, 129, 161, 255, 256, 257]
+    E, T = len(counts), sum(counts)
+    prob = make_problem(1, T, H, I, E, 1, seed=3, dtype=torch.bfloat16, device="cuda", x_scale=0.1, w_scale=0.02)
+    order = torch.randperm(T, generator=torch.Generator().manual_seed(1))
+    idx = torch.repeat_interleave(torch.arange(E), torch.tensor(counts))[order].view(T, 1).to(prob["ranks"][0]["idx"])
+    prob["ranks"][0]["idx"] = idx
+    buf = tm.Buffer(None, int(64e6), explicitly_destroy=True)
+    res = {}
+    for mode in ("0", "auto"):
+        monkeypatch.setattr(engine, "_LOCAL_LAYER_MODE", mode)
+        for name in ("_FUSED_DISPATCH_MODE", "_FUSED_MODE", "_LAYER_KERNEL_MODE"):
+            monkeypatch.setattr(engine, name, "1" if mode == "0" else "auto")
+        res[mode] = _run(buf, prob, idx, E)
+    ref = oracle(prob)[0]
+    for name, got in res["auto"].items():
+        if name in ref:
+            assert_close_bf16(got.float(), ref[name].cuda().float(), name)
+        assert torch.equal(got, res["0"][name]), f"{name}: differs from the general kernels"
+    buf.check_status()
+    buf.destroy()
+
+
 def test_native_autograd_node_keeps_its_buffer_and_fills_the_given_gradient():
     """The buffer may go out of scope before the backward pass; d(topk_weights) goes to the caller's tensor; a second derivative
     raises; a destroyed buffer raises."""
