@@ -54,7 +54,8 @@ constexpr int kCopyRows = 8;                                              // slo
 constexpr int kFirstRows = 1;                                             // slots every warp copies before anything else
 constexpr int kCopyWarps = kThreads / 32 - 2;                             // warps of a CTA that copy at the start
 constexpr int kRingDepth = 4;
-constexpr int kOwed = 3;                                                  // finished tiles an epilogue warp counts at once
+constexpr int kSoon = 32;                                                 // looks at a barrier before its wait counts as one
+constexpr int kOwed = 4;                                                  // finished tiles an epilogue warp counts at once
 constexpr int kGatherTasks = 16384;                                       // least number of (token, columns) tasks of the gather role
 constexpr uint32_t kOffTmem = 496, kOffRingFull = 320, kOffRingEmpty = 352, kOffItems = 384;
 constexpr uint32_t kRingConsumers = 2 * kEpiWarps + 2;
@@ -62,7 +63,7 @@ static_assert(8 * (2 * kMaxStages + 4) <= (int)kOffRingFull && kOffItems + 16 * 
 static_assert(kSmemBytesP <= 232448, "shared memory");
 
 // words of the sync block
-enum { kSyncItem = 0, kSyncToken = 1, kSyncCopy = 2, kSyncKeep = 3, kSyncUnits = 4, kSyncRows = 5, kSyncWords = 8 };
+enum { kSyncItem = 0, kSyncToken = 1, kSyncCopy = 2, kSyncKeep = 3, kSyncFirsts = 4, kSyncRows = 5, kSyncWords = 8 };
 // words of the meta block
 enum { kMetaUnits = 0, kMetaSlots = 1, kMetaWork = 2, kMetaRows = 4, kMetaWords = 8 };
 
@@ -236,7 +237,9 @@ __global__ void __launch_bounds__(kRouteThreads) local_route_assign_kernel(const
             // rows that have to be in place; backward, whole 64-row steps of K of the weight gradients
             const int end = seg[e] + (dir == 1 ? (totals[e] + BK - 1) / BK * BK : totals[e]);
             const int need0 = max(0, min(128, end - blk0 * 128)), need1 = two ? max(0, min(128, end - (blk0 + 1) * 128)) : 0;
-            if (pos < cap) work[pos] = make_int4(kind | (two << 4) | (e << 8), u, n_blk | (need0 << 16) | (need1 << 24), blk0);
+            // rows of zeros among them, in the last unit of an expert
+            const int pad = (dir == 1 && (blk0 + 2) * 128 >= end) ? end - seg[e] - totals[e] : 0;
+            if (pos < cap) work[pos] = make_int4(kind | (two << 4) | (e << 8) | (pad << 24), u, n_blk | (need0 << 16) | (need1 << 24), blk0);
         };
         for (int g = blockIdx.x; g < NG + lg && NG > 0; g += gridDim.x) {
             const Block b = block(g);
@@ -360,11 +363,6 @@ struct LayerArgsP {
     int* status;
 };
 
-__device__ __forceinline__ int atom_add_acq_rel(int* p, int v) {
-    int old;
-    asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
-    return old;
-}
 __device__ __forceinline__ int4 ld_cg_v4_ordered(const void* p) {
     int4 v;
     // volatile keeps it behind the acquire loads that precede it; no memory clobber, so that many can be in flight
@@ -415,28 +413,30 @@ __device__ __forceinline__ void copy_row_deep(int4* dst, const int4* src, int nv
 }
 
 struct Item {
-    int kind, n0, halves, group, k0, nk, m0, unit, need;      // columns n0 .. n0 + 256 * halves
+    int kind, n0, halves, group, k0, nk, m0, unit, need, real;      // columns n0 .. n0 + 256 * halves; `real` of the `need` rows are not padding
     bool live;          // this CTA's 128 rows are real
     int m_in_group;     // weight gradients: first row of dW inside the expert
 };
 
 __device__ __forceinline__ void decode_item(const LayerArgsP& L, const int4& it, uint32_t rank, Item& q) {
     q.kind = it.x & 15;
-    q.group = (it.x >> 8) & 0xfffff;
+    q.group = (it.x >> 8) & 0xffff;
     const Phase& P = L.ph[q.kind];
     q.n0 = (it.z & 0xffff) * P.cols;
     q.halves = (P.cols > BN && q.n0 + BN < P.n_total) ? 2 : 1;
     if (q.kind <= kWorkGemm2) {
         q.unit = it.y;
         q.need = rank == 0 ? ((it.z >> 16) & 0xff) : ((it.z >> 24) & 0xff);
-        q.live = (rank == 0) || ((it.x >> 4) & 1);
+        const int two = (it.x >> 4) & 1;
+        q.live = rank == 0 || two;
+        q.real = q.need - ((int)rank == two ? (it.x >> 24) & 63 : 0);
         q.m0 = (it.w + (int)rank) * BM;
         q.k0 = 0;
         q.nk = P.nk;
         q.m_in_group = 0;
     } else {
         q.unit = -1;
-        q.need = 0;
+        q.need = q.real = 0;
         q.live = true;
         q.m_in_group = ((it.z >> 16) * 2 + (int)rank) * BM;
         q.m0 = q.m_in_group;
@@ -513,9 +513,17 @@ __device__ __forceinline__ int4* preact_at(const LayerArgsP& L, int row0, int la
 }
 
 // First GEMM, forward: accumulator columns (2j, 2j+1) = (gate_j, up_j).  act = silu(g) * u * w.
+// 1 / (1 + e^-x).  In the forms that flush denormals: they are lost in the 1 anyway, and the others scale their operands around every
+// one of the two instructions.
+__device__ __forceinline__ float sigmoid(float x) {
+    float t, r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(t) : "f"(x * -1.4426950408889634f));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.f + t));
+    return r;
+}
+
 template <typename R>
-__device__ __forceinline__ void epilogue_swiglu(const LayerArgsP& L, const Staging& st, uint32_t taddr, int row0, int n0, R release) {
-    const float w = L.slot_w[row0 + st.lane];
+__device__ __forceinline__ void epilogue_swiglu(const LayerArgsP& L, const Staging& st, uint32_t taddr, int row0, float w, int n0, R release) {
     const int n_total = 2 * L.I;
     int4* keep = preact_at(L, row0, st.lane, n0);
     st.reuse();
@@ -532,7 +540,7 @@ __device__ __forceinline__ void epilogue_swiglu(const LayerArgsP& L, const Stagi
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
                 const float gt = __uint_as_float(acc[4 * p + 2 * e]), up = __uint_as_float(acc[4 * p + 2 * e + 1]);
-                v[e] = __fdividef(gt, 1.f + __expf(-gt)) * up * w;
+                v[e] = gt * sigmoid(gt) * up * w;
             }
             o[p] = pack_bf16x2(v[0], v[1]);
         }
@@ -554,22 +562,22 @@ __device__ __forceinline__ void epilogue_swiglu(const LayerArgsP& L, const Stagi
 
 // First GEMM, backward: accumulator column j = d act_j.  Padding rows give zeros whatever the operands hold there: dGU and
 // act x route are operands of the weight gradients, which sum over whole 64-row blocks.  The pre-activation comes 32 columns ahead, the
-// first of it before the accumulator is ready.  16 columns are computed before the box is waited for and written: with one 16-byte
-// piece at a time the exponentials of four columns were all that a warp had in flight.  Stores alternate between two half boxes.
+// first of it before the accumulator is ready.  16 columns are computed before the half box is waited for and written: a warp is bound by
+// the latency of its instructions (about four cycles each, two epilogue warps per scheduler), and the exponentials of 16
+// columns overlap where those of one 16-byte piece did not.  15 -> 13 thousand cycles per 256-column tile.
 struct Preact {
     int4 v[8];      // 16-byte pieces of this lane's row: columns 8 i .. 8 i + 7 of 2 I
-    __device__ __forceinline__ void request(const LayerArgsP& L, int row0, int col, bool real, int lane) {
+    __device__ __forceinline__ void request(const LayerArgsP& L, int row0, int col, int half, bool real, int lane) {
         const int4* p = preact_at(L, row0, lane, 2 * col);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) v[i] = real ? ld_nc_v4(p + 32 * i) : make_int4(0, 0, 0, 0);
+        for (int i = 0; i < 4; ++i) v[4 * half + i] = real ? ld_nc_v4(p + 32 * (4 * half + i)) : make_int4(0, 0, 0, 0);
     }
 };
 
 template <typename R>
-__device__ __forceinline__ void epilogue_dswiglu(const LayerArgsP& L, const Staging& st, uint32_t taddr, int row0, bool real, int n0,
+__device__ __forceinline__ void epilogue_dswiglu(const LayerArgsP& L, const Staging& st, uint32_t taddr, int row0, bool real, float w, int n0,
                                                  int part, Preact& pre, R release) {
     const long row = row0 + st.lane;
-    const float w = real ? L.slot_w[row] : 0.f;
     float droute = 0.f;
     int turn = 0;
     st.reuse();                              // (the last store may be a whole box)
@@ -579,8 +587,6 @@ __device__ __forceinline__ void epilogue_dswiglu(const LayerArgsP& L, const Stag
         const bool in = col < L.I;
         uint32_t acc[32];
         tmem_ld_x32(taddr + (uint32_t)(c * 32), acc);
-        Preact next;
-        next.request(L, row0, col + 32, real && c < 3 && col + 32 < L.I, st.lane);
         tmem_ld_wait();
         if (c == 3) release();
         uint32_t act[16];
@@ -597,7 +603,7 @@ __device__ __forceinline__ void epilogue_dswiglu(const LayerArgsP& L, const Stag
                 for (int e = 0; e < 4; ++e) {
                     const float2 gu = unpack_bf16x2(pr[e]);
                     const float ga = real ? __uint_as_float(acc[4 * v + e]) : 0.f;
-                    const float sig = __fdividef(1.f, 1.f + __expf(-gu.x));
+                    const float sig = sigmoid(gu.x);
                     const float s = gu.x * sig;
                     const float a = s * gu.y;
                     const float gaw = ga * w;
@@ -610,6 +616,7 @@ __device__ __forceinline__ void epilogue_dswiglu(const LayerArgsP& L, const Stag
                 act[2 * v] = pack_bf16x2(av[0], av[1]);
                 act[2 * v + 1] = pack_bf16x2(av[2], av[3]);
             }
+            pre.request(L, row0, col + 32, h, real && c < 3 && col + 32 < L.I, st.lane);
             st.reuse<1>();
 #pragma unroll
             for (int i = 0; i < 4; ++i) st.put_narrow(turn, i, dgu[4 * i], dgu[4 * i + 1], dgu[4 * i + 2], dgu[4 * i + 3]);
@@ -619,7 +626,6 @@ __device__ __forceinline__ void epilogue_dswiglu(const LayerArgsP& L, const Stag
 #pragma unroll
         for (int i = 0; i < 4; ++i) st.put_narrow(turn, i, act[4 * i], act[4 * i + 1], act[4 * i + 2], act[4 * i + 3]);
         st.store_narrow(turn++, in, &L.st_act, col, row0);
-        pre = next;
     }
     L.droute_part[row * L.n_parts + part] = droute;
 }
@@ -738,7 +744,7 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
         __syncwarp();
         if (lane == 0 && n > 0) {
             fence_acq_rel_gpu();
-            red_add_release_gpu(counter, n);
+            red_add_gpu(counter, n);
         }
     };
     auto place = [&](int s0, int n) {
@@ -941,6 +947,9 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
         if (warp == 0) {
             // -------------------------------------------------------------- item fetch (first CTA) + TMA producer
             if (elect_one()) {
+                const int stages = L.stages;
+                const uint32_t stage_bytes = (uint32_t)L.stage_bytes, pair_full = mapa_shared(full_bar(0), 0);
+                auto rows_loaded = [](int need) { return need > 64 ? BM : (need + 31) & ~31; };
                 int stage = 0;
                 uint32_t phase = 0;
                 bool ok = true;
@@ -992,7 +1001,7 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                     // would cost as much as the smallest of these items)
                     if (wgrad_ready) return 1;
                     const int a = counted(L.sync + kSyncRows, L.meta[kMetaRows], block, 603, w_wgrad);
-                    const int b = a == 1 ? counted(L.sync + kSyncUnits, L.meta[kMetaUnits], block, 602, w_wgrad) : a;
+                    const int b = a == 1 ? counted(L.sync + kSyncFirsts, L.meta[kMetaUnits] * target1, block, 602, w_wgrad) : a;
                     wgrad_ready = b == 1;
                     return b;
                 };
@@ -1027,43 +1036,47 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                     // stores of other SMs -> async-proxy reads; the weight gradients acquire once, so they need the fence once
                     if (q.kind <= kWorkGemm2 || !wgrad_fenced) fence_proxy_async_all();
                     if (q.kind > kWorkGemm2) wgrad_fenced = true;
+                    const bool gemm = q.kind <= kWorkGemm2;
                     const int n0 = q.n0 + (int)rank * (BN / 2);
-                    const int look_kb = min(L.stages - 1, q.nk - 1);   // all stages are in flight: a pause of this thread costs nothing
-                    for (int kb = 0; kb < q.nk; ++kb) {
-                        if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag, L.status, 610)) { ok = false; break; }
-                        const uint32_t a_dst = smem_base + stage * L.stage_bytes;
-                        const uint32_t b_dst = a_dst + kAStageBytes;
-                        const uint32_t bar = mapa_shared(full_bar(stage), 0);
-                        if (rank == 0) mbar_arrive_expect_tx(full_bar(stage), 2u * (uint32_t)(kAStageBytes + q.halves * kBHalfBytesP));
-                        else mbar_arrive_cluster(bar);
-                        const int k = q.k0 + kb * BK;
-                        if (q.kind <= kWorkGemm2) {
-                            // rows that nothing waits for are not read: past the end of the table reads zeros
-                            if (q.need > 96 || q.need == 0) {
-                                tma_load_2d_2cta(a_dst, &P.map_a, bar, k, q.need > 0 ? q.m0 : L.out_rows);
-                            } else {
-#pragma unroll
-                                for (int b = 0; b < 4; ++b)
-                                    tma_load_2d_2cta(a_dst + b * (kAStageBytes / 4), &P.map_a32, bar, k, 32 * b < q.need ? q.m0 + 32 * b : L.out_rows);
-                            }
-                        } else {
-#pragma unroll
-                            for (int a = 0; a < BM / 64; ++a) tma_load_2d_2cta(a_dst + a * kAtomBytes, &P.map_a, bar, q.m0 + 64 * a, k);
+                    // Rows of A that a CTA loads: none that nothing is summed from, up to 64 in boxes of 32.  What a stage holds in the others
+                    // is multiplied into accumulator rows that no epilogue reads.
+                    const int a_rows = gemm ? rows_loaded(q.need) : BM;
+                    const int a_pair = gemm ? rows_loaded((cur.z >> 16) & 0xff) + rows_loaded((cur.z >> 24) & 0xff) : 2 * BM;
+                    const uint32_t tx = (uint32_t)(a_pair * (BK * 2) + 2 * q.halves * kBHalfBytesP);
+                    const int look_kb = min(stages - 1, q.nk - 1);     // all stages are in flight: a pause of this thread costs nothing
+                    auto load_steps = [&](auto&& load) {
+                        for (int kb = 0; kb < q.nk; ++kb) {
+                            if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag, L.status, 610)) return false;
+                            const uint32_t bar = pair_full + 8u * stage;
+                            if (rank == 0) mbar_arrive_expect_tx(full_bar(stage), tx);
+                            else mbar_arrive_cluster(bar);
+                            load(smem_base + (uint32_t)stage * stage_bytes, bar, kb * BK);
+                            if (++stage == stages) { stage = 0; phase ^= 1u; }
+                            // (the second CTA keeps looking until the first one has published the item)
+                            if (kb >= look_kb && !have && (kb == look_kb || rank != 0) && !look_ahead()) return false;
                         }
-                        for (int h = 0; h < q.halves; ++h) {
-                            const uint32_t dst = b_dst + h * kBHalfBytesP;
-                            const int col = n0 + h * BN;
-                            if (!BWD) {
-                                tma_load_2d_2cta(dst, &P.map_b, bar, k, q.group * P.b_group_rows + col);
-                            } else {
-                                const int krow = q.kind <= kWorkGemm2 ? q.group * P.b_group_rows + k : k;
-#pragma unroll
-                                for (int a = 0; a < BN / 128; ++a) tma_load_2d_2cta(dst + a * kAtomBytes, &P.map_b, bar, col + 64 * a, krow);
+                        return true;
+                    };
+                    const CUtensorMap* map_b = &P.map_b;
+                    if (gemm) {
+                        const CUtensorMap* map_a = a_rows == BM ? &P.map_a : &P.map_a32;
+                        const int b_row = q.group * P.b_group_rows;
+                        ok = load_steps([&](uint32_t dst, uint32_t bar, int k) {
+                            if (a_rows != 0) tma_load_2d_2cta(dst, map_a, bar, k, q.m0);
+                            if (a_rows == 64) tma_load_2d_2cta(dst + 32 * BK * 2, map_a, bar, k, q.m0 + 32);
+                            for (int h = 0; h < q.halves; ++h) {
+                                const uint32_t b_dst = dst + kAStageBytes + h * kBHalfBytesP;
+                                if (!BWD) tma_load_2d_2cta(b_dst, map_b, bar, k, b_row + n0 + h * BN);
+                                else tma_load_3d_2cta(b_dst, map_b, bar, 0, b_row + k, (n0 + h * BN) >> 6);
                             }
-                        }
-                        if (++stage == L.stages) { stage = 0; phase ^= 1u; }
-                        // (the second CTA keeps looking until the first one has published the item)
-                        if (kb >= look_kb && !have && (kb == look_kb || rank != 0) && !look_ahead()) { ok = false; break; }
+                        });
+                    } else if constexpr (BWD) {
+                        const CUtensorMap* map_a = &P.map_a;
+                        ok = load_steps([&](uint32_t dst, uint32_t bar, int k) {
+                            tma_load_3d_2cta(dst, map_a, bar, 0, q.k0 + k, q.m0 >> 6);
+                            for (int h = 0; h < q.halves; ++h)
+                                tma_load_3d_2cta(dst + kAStageBytes + h * kBHalfBytesP, map_b, bar, 0, q.k0 + k, (n0 + h * BN) >> 6);
+                        });
                     }
                 }
                 if (L.stats != nullptr) {
@@ -1169,8 +1182,8 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
             uint32_t sph = 0;
             int acc = 0;
             // Tiles whose stores are not yet counted as complete (bit 31: first GEMM).  They are counted in one go when this warp would
-            // have to wait for its next item or accumulator, or when the list is full: narrow tiles (K of a few hundred) follow
-            // each other faster than a store, a fence and an atomic complete.  Never behind such a wait: the next item may be
+            // have to wait for its next item or accumulator (for more than a moment: counting takes 3 to 6 thousand cycles), or when
+            // the list is full: narrow tiles (K of a few hundred) follow each other faster than a store, a fence and an atomic complete.  Never behind such a wait: the next item may be
             // one that waits for this count.
             uint32_t owed[kOwed];
             int n_owed = 0;
@@ -1181,20 +1194,27 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                     tma_store_wait<0>();
                     fence_proxy_async_all();
                     fence_acq_rel_gpu();
+                    int firsts = 0;
 #pragma unroll
                     for (int i = 0; i < kOwed; ++i) {
                         if (i >= n_owed) break;
                         const int at = (int)(owed[i] & 0x7fffffffu);
-                        if (!(owed[i] >> 31)) red_add_release_gpu(L.done2 + at, 1);
-                        else if (!BWD) red_add_release_gpu(L.done1 + at, 1);
-                        else if (atom_add_acq_rel(L.done1 + at, 1) == target1 - 1) red_add_release_gpu(L.sync + kSyncUnits, 1);
+                        const bool first = owed[i] >> 31;
+                        red_add_gpu((first ? L.done1 : L.done2) + at, 1);      // (ordered by the fence)
+                        firsts += first;
                     }
+                    if (BWD && firsts != 0) red_add_gpu(L.sync + kSyncFirsts, firsts);
                 }
                 n_owed = 0;
             };
+            auto soon = [&](uint32_t bar, uint32_t parity) {
+                for (int i = 0; i < kSoon; ++i)
+                    if (__all_sync(0xffffffffu, mbar_test_wait(bar, parity))) return true;
+                return false;
+            };
             while (ok) {
                 int4 it;
-                if (n_owed != 0 && !__all_sync(0xffffffffu, mbar_test_wait(ring_full(ss), sph))) flush();
+                if (n_owed != 0 && !soon(ring_full(ss), sph)) flush();
                 if (!next_item(ss, sph, 653, it) || it.x < 0) break;
                 const bool stamps = L.stats != nullptr && warp == 4 && lane == 0 && rank == 0;
                 Item q;
@@ -1205,17 +1225,21 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                 // rows of a block beyond those that are used are neither computed on nor stored
                 const bool live = q.kind > kWorkGemm2 || (q.live && qd * 32 < q.need);
                 bool real = false;                 // backward, first GEMM: this lane's row is not padding
-                if constexpr (BWD) real = q.kind == kWorkGemm1 && live && L.slot_tk[row0 + lane] >= 0;
+                if constexpr (BWD) real = q.kind == kWorkGemm1 && qd * 32 + lane < q.real;
                 for (int h = 0; h < q.halves; ++h) {
                     const int slot = acc & 1;
                     const uint32_t parity = (acc >> 1) & 1;
                     ++acc;
                     const int n0 = q.n0 + h * BN + hh * (BN / 2);
+                    const float w = (q.kind == kWorkGemm1 && live) ? L.slot_w[row0 + lane] : 0.f;       // (padding: 0)
                     Preact pre;
                     if constexpr (BWD) {
-                        if (q.kind == kWorkGemm1) pre.request(L, row0, n0, real && n0 < L.I, lane);
+                        if (q.kind == kWorkGemm1) {
+                            pre.request(L, row0, n0, 0, real && n0 < L.I, lane);
+                            pre.request(L, row0, n0, 1, real && n0 < L.I, lane);
+                        }
                     }
-                    if (n_owed != 0 && (n_owed == kOwed || !__all_sync(0xffffffffu, mbar_test_wait(tfull_bar(slot), parity)))) flush();
+                    if (n_owed != 0 && (n_owed == kOwed || !soon(tfull_bar(slot), parity))) flush();
                     if (!mbar_wait(tfull_bar(slot), parity, abort_flag, L.status, 630)) { ok = false; break; }
                     tcgen05_fence_after();
                     const uint32_t taddr = tmem_base + ((uint32_t)(qd * 32) << 16) + (uint32_t)(slot * BN + hh * (BN / 2));
@@ -1228,8 +1252,8 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                     if (!live) {
                         release();
                     } else if (q.kind == kWorkGemm1) {
-                        if constexpr (BWD) epilogue_dswiglu(L, st, taddr, row0, real, n0, n0 / (BN / 2), pre, release);
-                        else epilogue_swiglu(L, st, taddr, row0, n0, release);
+                        if constexpr (BWD) epilogue_dswiglu(L, st, taddr, row0, real, w, n0, n0 / (BN / 2), pre, release);
+                        else epilogue_swiglu(L, st, taddr, row0, w, n0, release);
                     } else if (q.kind == kWorkGemm2) {
                         epilogue_plain(st, taddr, false, release, [&](int c) {
                             st.store(n0 + c < L.H, &L.st_y, n0 + c, row0);
@@ -1302,6 +1326,22 @@ cudaError_t make_map_narrow(CUtensorMap* map, const void* base, uint64_t rows, u
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
+// [rows, cols] bf16 (cols a multiple of 64) as an operand whose rows are steps of K: boxes of 64 rows x 128 columns, laid down as two
+// swizzled atoms of 64 columns, in one copy
+cudaError_t make_map_mn(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols) {
+    EncodeTiledFn fn = get_encode_fn();
+    if (fn == nullptr) return cudaErrorNotSupported;
+    if ((reinterpret_cast<uintptr_t>(base) & 15u) != 0) return cudaErrorInvalidValue;
+    cuuint64_t dims[3] = {64, rows, cols / 64};
+    cuuint64_t strides[2] = {cols * 2, 128};
+    cuuint32_t box[3] = {64, BK, 2};
+    cuuint32_t estr[3] = {1, 1, 1};
+    const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
+                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
+}
+
 // [groups, rows, cols] bf16, boxes of 32 rows x 64 columns of one group; rows and columns outside a group are not written
 cudaError_t make_store_map3(CUtensorMap* map, const void* base, uint64_t groups, uint64_t rows, uint64_t cols) {
     EncodeTiledFn fn = get_encode_fn();
@@ -1348,8 +1388,9 @@ LocalLayerPlan local_layer_plan(int T, int K, int E, int H, int I, int keep) {
     p.units_cap = (int)((p.blocks_cap + segs) / 2);
     // Columns per tile of every GEMM [direction][kind].  The wide tile needs columns for it, enough tiles that every CTA pair gets
     // several, and a mainloop that is long against what it cannot hide: with both accumulators in one tile, the next tile
-    // starts when the first half has been read out (a few hundred cycles for a plain store, two to three thousand for
-    // the activations), where two 256-column tiles overlap completely.
+    // starts when the first half has been read out (about a thousand cycles for a plain store, three for SwiGLU, twelve for its
+    // backward), where two 256-column tiles overlap completely.  Operand copies are what the narrow tile lacks: backward's first GEMM
+    // at H = 2048 took 950 cycles per step of K, of which the tensor cores need 512 (wide: 1200 of 1024; a layer 1.5 % faster).
     const int mu_wd = (H + 2 * BM - 1) / (2 * BM), mu_wg = (2 * I + 2 * BM - 1) / (2 * BM);
     auto columns = [&](int n, long row_units, int k, int min_k) {
         return n >= 2 * BN && k >= min_k && row_units * column_blocks(n, 2 * BN) >= kWideTiles ? 2 * BN : BN;
@@ -1358,7 +1399,7 @@ LocalLayerPlan local_layer_plan(int T, int K, int E, int H, int I, int keep) {
     const int rows = (int)(entries / (segs > 0 ? segs : 1));
     p.cols[0][0] = columns(2 * I, units, H, 2048);
     p.cols[0][1] = columns(H, units, I, 1024);
-    p.cols[1][0] = columns(I, units, H, 4096);
+    p.cols[1][0] = columns(I, units, H, 2048);
     p.cols[1][1] = columns(H, units, 2 * I, 1024);
     p.cols[1][2] = columns(I, (long)E * mu_wd, rows, 1024);
     p.cols[1][3] = columns(H, (long)E * mu_wg, rows, 1024);
@@ -1451,18 +1492,18 @@ cudaError_t local_layer_launch(const LocalLayerParams& q, cudaStream_t stream) {
         g2.nk = I / BK; g2.b_group_rows = H;
     } else {
         // grad_act: A = dY, B = W_down MN-major;  dX: A = dGU, B = W_gateup MN-major
-        if ((e = make_map(&g1.map_b, q.w_down, (uint64_t)E * H, I, 64, BK)) != cudaSuccess) return e;
+        if ((e = make_map_mn(&g1.map_b, q.w_down, (uint64_t)E * H, I)) != cudaSuccess) return e;
         if ((e = make_map(&g2.map_a, q.aux, R, 2 * I, BK, BM)) != cudaSuccess || (e = make_map(&g2.map_a32, q.aux, R, 2 * I, BK, 32)) != cudaSuccess) return e;
-        if ((e = make_map(&g2.map_b, q.w_gateup, (uint64_t)E * 2 * I, H, 64, BK)) != cudaSuccess) return e;
+        if ((e = make_map_mn(&g2.map_b, q.w_gateup, (uint64_t)E * 2 * I, H)) != cudaSuccess) return e;
         g1.n_total = I; g1.b_group_rows = H;
         g2.nk = 2 * I / BK; g2.b_group_rows = 2 * I;
         // dW_down[e] = dY[seg]^T . act_w[seg]  ([H, I]);  dW_gateup[e] = dGU[seg]^T . X[seg]  ([2I, H])
         Phase& gd = L.ph[kWorkWgradDown];
         Phase& gg = L.ph[kWorkWgradGateup];
-        if ((e = make_map(&gd.map_a, q.slot_x, R, H, 64, BK)) != cudaSuccess) return e;
-        if ((e = make_map(&gd.map_b, q.act, R, I, 64, BK)) != cudaSuccess) return e;
-        if ((e = make_map(&gg.map_a, q.aux, R, 2 * I, 64, BK)) != cudaSuccess) return e;
-        if ((e = make_map(&gg.map_b, q.xperm, R, H, 64, BK)) != cudaSuccess) return e;
+        if ((e = make_map_mn(&gd.map_a, q.slot_x, R, H)) != cudaSuccess) return e;
+        if ((e = make_map_mn(&gd.map_b, q.act, R, I)) != cudaSuccess) return e;
+        if ((e = make_map_mn(&gg.map_a, q.aux, R, 2 * I)) != cudaSuccess) return e;
+        if ((e = make_map_mn(&gg.map_b, q.xperm, R, H)) != cudaSuccess) return e;
         gd.m_total = H; gd.n_total = I; gd.cols = p.cols[1][2]; gd.num_n_blocks = column_blocks(I, gd.cols);
         gg.m_total = 2 * I; gg.n_total = H; gg.cols = p.cols[1][3]; gg.num_n_blocks = column_blocks(H, gg.cols);
         if ((e = make_store_map3(&L.st_dwd, q.dw_down, E, H, I)) != cudaSuccess) return e;
