@@ -315,7 +315,7 @@ class LocalLayer : public std::enable_shared_from_this<LocalLayer> {
     }
 
     struct Kept {
-        torch::Tensor ws, preact, saved_x;
+        torch::Tensor ws, rows;       // rows: x [T, H], then the pre-activation of every slot (2I values)
     };
 
     torch::Tensor forward(const torch::Tensor& x, const torch::Tensor& topk_idx, const torch::Tensor& topk_w, const torch::Tensor& w_gateup,
@@ -336,10 +336,9 @@ class LocalLayer : public std::enable_shared_from_this<LocalLayer> {
         auto act = torch::empty({rows, I}, x.options());
         if (kept != nullptr) {
             kept->ws = ws;
-            kept->preact = torch::empty({rows, 2 * I}, x.options());
-            kept->saved_x = torch::empty({tk.T, H}, x.options());
-            p.preact = kept->preact.data_ptr();
-            p.saved_x = kept->saved_x.data_ptr();
+            kept->rows = torch::empty({tk.T * H + rows * 2 * I}, x.options());
+            p.saved_x = kept->rows.data_ptr();
+            p.preact = kept->rows.data_ptr<at::BFloat16>() + tk.T * H;
         }
         p.ws = ws.data_ptr<int>();
         p.topk_idx = tk.ptr; p.idx_is64 = tk.is64; p.topk_w = topk_w.data_ptr<float>();
@@ -358,18 +357,21 @@ class LocalLayer : public std::enable_shared_from_this<LocalLayer> {
                                           int64_t K, const Schedule& schedule) {
         check();
         c10::cuda::CUDAGuard guard(grad_out.device());
-        const int64_t E = w_gateup.size(0), T = kept.saved_x.size(0), H = kept.saved_x.size(1), I = w_gateup.size(1) / 2;
+        const int64_t E = w_gateup.size(0), T = grad_out.size(0), H = w_gateup.size(2), I = w_gateup.size(1) / 2;
         TORCH_CHECK(grad_out.is_cuda() && grad_out.scalar_type() == torch::kBFloat16 && grad_out.is_contiguous() && grad_out.dim() == 2 &&
-                    grad_out.size(0) == T && grad_out.size(1) == H, "grad_out must be a contiguous bf16 [T, H] CUDA tensor");
+                    grad_out.size(1) == H, "grad_out must be a contiguous bf16 [T, H] CUDA tensor");
         check_layer_weights(w_gateup, w_down, E, H, I);
         tmoe::LocalLayerParams p{};
         p.plan = tmoe::local_layer_plan((int)T, (int)K, (int)E, (int)H, (int)I, 1);
         const int64_t rows = set_common(p, schedule);
-        TORCH_CHECK(kept.ws.numel() == p.plan.words && kept.preact.size(0) == rows && kept.preact.size(1) == 2 * I, "saved tensors of another call");
-        auto act_w = torch::empty({rows, I}, grad_out.options());
-        auto dgu = torch::empty({rows, 2 * I}, grad_out.options());
-        auto xperm = torch::empty({rows, H}, grad_out.options());
-        auto parts = torch::empty({rows, 2 * ((I + 255) / 256)}, on(grad_out, torch::kFloat32));
+        TORCH_CHECK(kept.ws.numel() == p.plan.words && kept.rows.numel() == T * H + rows * 2 * I, "saved tensors of another call");
+        // act x route [rows, I], dGU [rows, 2I], x in slot order [rows, H], partial sums of d(route weight): one allocation (rows and I, H are
+        // multiples of 64: every part starts on a 16-byte boundary)
+        auto scratch = torch::empty({rows * (3 * I + H + 4 * ((I + 255) / 256))}, grad_out.options());
+        auto* act_w = scratch.data_ptr<at::BFloat16>();
+        auto* dgu = act_w + rows * I;
+        auto* xperm = dgu + rows * 2 * I;
+        auto* parts = xperm + rows * H;
         auto dx = torch::empty({T, H}, grad_out.options());
         auto dw = torch::empty({T, K}, on(grad_out, torch::kFloat32));
         auto dwg = torch::empty({E, 2 * I, H}, grad_out.options());
@@ -377,8 +379,8 @@ class LocalLayer : public std::enable_shared_from_this<LocalLayer> {
         p.ws = kept.ws.data_ptr<int>();
         p.bwd = 1;
         p.x = grad_out.data_ptr(); p.w_gateup = w_gateup.data_ptr(); p.w_down = w_down.data_ptr();
-        p.act = act_w.data_ptr(); p.aux = dgu.data_ptr(); p.saved_x = kept.saved_x.data_ptr(); p.out = dx.data_ptr();
-        p.preact = kept.preact.data_ptr(); p.droute_part = parts.data_ptr<float>(); p.xperm = xperm.data_ptr();
+        p.act = act_w; p.aux = dgu; p.saved_x = kept.rows.data_ptr(); p.out = dx.data_ptr();
+        p.preact = kept.rows.data_ptr<at::BFloat16>() + T * H; p.droute_part = reinterpret_cast<float*>(parts); p.xperm = xperm;
         p.dw_topk = dw.data_ptr<float>(); p.dw_gateup = dwg.data_ptr(); p.dw_down = dwd.data_ptr();
         TM_CHECK_CUDA(tmoe::local_layer_launch(p, cur_stream()));
         note(1, kept.ws, p.plan);
@@ -426,7 +428,7 @@ class LocalLayerFunction : public torch::autograd::Function<LocalLayerFunction> 
         LocalLayer::Kept kept;
         auto out = layer->forward(x, topk_idx, topk_w, w_gateup, w_down, schedule, &kept);
         // x itself is not kept
-        ctx->save_for_backward({w_gateup, w_down, kept.ws, kept.preact, kept.saved_x});
+        ctx->save_for_backward({w_gateup, w_down, kept.ws, kept.rows});
         auto holder = c10::make_intrusive<Holder>();
         holder->layer = std::move(layer);
         holder->schedule = schedule;
@@ -444,7 +446,7 @@ class LocalLayerFunction : public torch::autograd::Function<LocalLayerFunction> 
         torch::autograd::variable_list res;
         {
             at::AutoGradMode no_grad(false);
-            auto r = h->layer->backward(grads[0].contiguous(), LocalLayer::Kept{saved[2], saved[3], saved[4]}, saved[0], saved[1], h->K, h->schedule);
+            auto r = h->layer->backward(grads[0].contiguous(), LocalLayer::Kept{saved[2], saved[3]}, saved[0], saved[1], h->K, h->schedule);
             if (h->grad_topk_w.has_value()) {
                 h->grad_topk_w->copy_(r[1]);
                 r[1] = *h->grad_topk_w;

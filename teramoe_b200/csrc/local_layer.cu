@@ -73,6 +73,7 @@ constexpr int column_blocks(int n, int cols) { return (n + cols - 1) / cols; }
 
 constexpr int kRouteThreads = 256;
 constexpr int kRouteWarps = kRouteThreads / 32;
+constexpr int kDirectEntries = 4096;                                      // most entries that every block counts itself
 
 __device__ __forceinline__ int load_expert(const void* idx, int is64, long i, int E) {
     const long long e = is64 ? reinterpret_cast<const long long*>(idx)[i] : (long long) reinterpret_cast<const int*>(idx)[i];
@@ -81,9 +82,11 @@ __device__ __forceinline__ int load_expert(const void* idx, int is64, long i, in
 
 // -------------------------------------------------------------------------------------------------
 // Routing.  A chunk is 256 tokens (a warp per 32); slots are ordered by (expert, 32-token group, k, lane) as in routing.cu.
-// count: histograms of a chunk's entries over experts and of its tokens over their LAST expert, plus the totals.
-// assign: every block derives the segment table from the totals and its own bases from the chunk histograms before it, so
-// no block waits for another and no scan kernel sits in between.
+// count: histograms of a chunk's entries over experts and of its tokens over their LAST expert; clears the counters of the layer.
+// assign: every block adds up all chunk histograms, which gives it the segment table and its own bases, so no block waits for
+// another and no scan kernel sits in between.  With few entries (kDirectEntries) every block counts all of them itself and
+// clears a share of the counters: one launch instead of two and a memset.  512 tokens, top-2: 10.0 us and two gaps -> 7.4 us; 1000,
+// top-8 is past the break-even (15.0 -> 21.7 us).
 // -------------------------------------------------------------------------------------------------
 struct RouteArgs {
     LocalLayerPlan p;
@@ -94,6 +97,11 @@ struct RouteArgs {
     int nb1[2], nb2[2], mu_wd, nb_wd, mu_wg, nb_wg;
     int group_units, lag_percent, min_lag_items;
 };
+
+__device__ __forceinline__ void clear_counters(const RouteArgs& a) {
+    int4* z = reinterpret_cast<int4*>(a.ws);
+    for (long i = (long)blockIdx.x * kRouteThreads + threadIdx.x; i < a.p.zero_words / 4; i += (long)gridDim.x * kRouteThreads) z[i] = make_int4(0, 0, 0, 0);
+}
 
 __global__ void __launch_bounds__(kRouteThreads) local_route_count_kernel(const RouteArgs a) {
     extern __shared__ int sh[];
@@ -115,14 +123,9 @@ __global__ void __launch_bounds__(kRouteThreads) local_route_count_kernel(const 
     __syncthreads();
     int* ch = a.ws + a.p.chunk_hist + (long)blockIdx.x * E;
     int* cl = a.ws + a.p.chunk_last + (long)blockIdx.x * (E + 1);
-    for (int e = tid; e < E; e += kRouteThreads) {
-        ch[e] = hist[e];
-        if (hist[e] != 0) atomicAdd(a.ws + a.p.totals + e, hist[e]);
-    }
-    for (int e = tid; e <= E; e += kRouteThreads) {
-        cl[e] = last[e];
-        if (last[e] != 0) atomicAdd(a.ws + a.p.last_hist + e, last[e]);
-    }
+    for (int e = tid; e < E; e += kRouteThreads) ch[e] = hist[e];
+    for (int e = tid; e <= E; e += kRouteThreads) cl[e] = last[e];
+    clear_counters(a);
 }
 
 // largest e with base[e] <= v < base[e + 1]
@@ -136,6 +139,7 @@ __device__ __forceinline__ int find_segment(const int* base, int E, int v) {
     return lo;
 }
 
+template <bool DIRECT>
 __global__ void __launch_bounds__(kRouteThreads) local_route_assign_kernel(const RouteArgs a) {
     extern __shared__ int sh[];
     const int E = a.p.E, K = a.p.K, T = a.p.T, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -144,7 +148,48 @@ __global__ void __launch_bounds__(kRouteThreads) local_route_assign_kernel(const
     int* ob = ub + E + 1;                    // [E + 1] first place in the token order, by last expert
     int* cnt = ob + E + 1;                   // [warps][E] next slot
     int* lst = cnt + kRouteWarps * E;        // [warps][E + 1] next place in the token order
-    const int* totals = a.ws + a.p.totals;
+    int* totals = lst + kRouteWarps * (E + 1);   // [E] entries, [E + 1] tokens by their last expert: of all chunks ...
+    int* before_own = totals + 2 * E + 1;        // ... and of those before this block's
+    const int* last_hist = totals + E;
+    if (DIRECT) {
+        for (int i = tid; i < 2 * (2 * E + 1); i += kRouteThreads) totals[i] = 0;
+        clear_counters(a);
+        __syncthreads();
+        for (int g = warp; 32 * g < T; g += kRouteWarps) {
+            const int t = 32 * g + lane;
+            const bool earlier = g / kRouteWarps < (int)blockIdx.x;
+            auto count = [&](int i, bool there) {        // one more in bin i of the lanes that have one
+                const uint32_t same = __match_any_sync(0xffffffffu, there ? i : -1);
+                if (there && (same & ((1u << lane) - 1u)) == 0) {
+                    atomicAdd(&totals[i], __popc(same));
+                    if (earlier) atomicAdd(&before_own[i], __popc(same));
+                }
+            };
+            int m = -1;
+            for (int k = 0; k < K; ++k) {
+                const int e = t < T ? load_expert(a.topk_idx, a.is64, (long)t * K + k, E) : -1;
+                count(e, e >= 0);
+                m = max(m, e);
+            }
+            count(E + m + 1, t < T);
+        }
+    } else {
+        const int* ch = a.ws + a.p.chunk_hist;
+        const int* cl = a.ws + a.p.chunk_last;
+        for (int i = tid; i < 2 * E + 1; i += kRouteThreads) {
+            const int* h = i < E ? ch + i : cl + (i - E);
+            const int cols = i < E ? E : E + 1;
+            int run = 0, own = 0;
+#pragma unroll 8
+            for (int c = 0; c < a.p.chunks; ++c) {
+                if (c == (int)blockIdx.x) own = run;
+                run += h[(long)c * cols];
+            }
+            totals[i] = run;
+            before_own[i] = own;
+        }
+    }
+    __syncthreads();
     if (warp == 0) {
         int run_s = 0, run_u = 0, run_r = 0;
         for (int e0 = 0; e0 < E; e0 += 32) {
@@ -176,7 +221,7 @@ __global__ void __launch_bounds__(kRouteThreads) local_route_assign_kernel(const
     if (warp == 1) {
         int run = 0;
         for (int e0 = 0; e0 <= E; e0 += 32) {
-            const int own = e0 + lane <= E ? a.ws[a.p.last_hist + e0 + lane] : 0;
+            const int own = e0 + lane <= E ? last_hist[e0 + lane] : 0;
             int v = own;
             for (int o = 1; o < 32; o <<= 1) {
                 const int u = __shfl_up_sync(0xffffffffu, v, o);
@@ -275,15 +320,10 @@ __global__ void __launch_bounds__(kRouteThreads) local_route_assign_kernel(const
         atomicAdd(&lst[warp * (E + 1) + m + 1], 1);
     }
     __syncthreads();
-    const int* ch = a.ws + a.p.chunk_hist;
-    const int* cl = a.ws + a.p.chunk_last;
     for (int i = tid; i < 2 * E + 1; i += kRouteThreads) {
         const bool slots = i < E;
         const int e = slots ? i : i - E, cols = slots ? E : E + 1;
-        const int* h = slots ? ch : cl;
-        int run = slots ? seg[e] : ob[e];
-#pragma unroll 8
-        for (int c = 0; c < (int)blockIdx.x; ++c) run += h[(long)c * cols + e];
+        int run = (slots ? seg[e] : ob[e]) + before_own[i];
         int* w = slots ? cnt : lst;
         for (int v = 0; v < kRouteWarps; ++v) {
             const int n = w[v * cols + e];
@@ -1032,10 +1072,6 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                     Item q;
                     decode_item(L, cur, rank, q);
                     const Phase& P = L.ph[q.kind];
-                    if (!cur_ready && operands_ready(q, true) != 1) { *abort_flag = 1u; ok = false; break; }
-                    // stores of other SMs -> async-proxy reads; the weight gradients acquire once, so they need the fence once
-                    if (q.kind <= kWorkGemm2 || !wgrad_fenced) fence_proxy_async_all();
-                    if (q.kind > kWorkGemm2) wgrad_fenced = true;
                     const bool gemm = q.kind <= kWorkGemm2;
                     const int n0 = q.n0 + (int)rank * (BN / 2);
                     // Rows of A that a CTA loads: none that nothing is summed from, up to 64 in boxes of 32.  What a stage holds in the others
@@ -1044,39 +1080,64 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                     const int a_pair = gemm ? rows_loaded((cur.z >> 16) & 0xff) + rows_loaded((cur.z >> 24) & 0xff) : 2 * BM;
                     const uint32_t tx = (uint32_t)(a_pair * (BK * 2) + 2 * q.halves * kBHalfBytesP);
                     const int look_kb = min(stages - 1, q.nk - 1);     // all stages are in flight: a pause of this thread costs nothing
-                    auto load_steps = [&](auto&& load) {
+                    auto take_stage = [&](int st, uint32_t ph) {
+                        if (!mbar_wait(empty_bar(st), ph ^ 1u, abort_flag, L.status, 610)) return false;
+                        if (rank == 0) mbar_arrive_expect_tx(full_bar(st), tx);
+                        else mbar_arrive_cluster(pair_full + 8u * st);
+                        return true;
+                    };
+                    const CUtensorMap* map_b = &P.map_b;
+                    const int b_row = q.group * P.b_group_rows;
+                    auto load_b = [&](int st, int k) {
+                        const uint32_t dst = smem_base + (uint32_t)st * stage_bytes + kAStageBytes, bar = pair_full + 8u * st;
+                        for (int h = 0; h < q.halves; ++h) {
+                            if (!BWD) tma_load_2d_2cta(dst + h * kBHalfBytesP, map_b, bar, k, b_row + n0 + h * BN);
+                            else tma_load_3d_2cta(dst + h * kBHalfBytesP, map_b, bar, 0, b_row + k, (n0 + h * BN) >> 6);
+                        }
+                    };
+                    // What a GEMM waits for is its rows; the weights of its first steps come meanwhile (the first items of a call would else
+                    // wait for memory twice, one after the other).
+                    int early = 0;
+                    if (!cur_ready) {
+                        if (gemm) {
+                            int st = stage;
+                            uint32_t ph = phase;
+                            for (; early < min(stages, q.nk); ++early) {
+                                if (!(ok = take_stage(st, ph))) break;
+                                load_b(st, early * BK);
+                                if (++st == stages) { st = 0; ph ^= 1u; }
+                            }
+                        }
+                        if (!ok || operands_ready(q, true) != 1) {
+                            *abort_flag = 1u;
+                            __nanosleep(100000);                       // (the copies under way land)
+                            ok = false;
+                            break;
+                        }
+                    }
+                    // stores of other SMs -> async-proxy reads; the weight gradients acquire once, so they need the fence once
+                    if (gemm || !wgrad_fenced) fence_proxy_async_all();
+                    if (!gemm) wgrad_fenced = true;
+                    auto load_steps = [&](auto&& load_a) {
                         for (int kb = 0; kb < q.nk; ++kb) {
-                            if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag, L.status, 610)) return false;
-                            const uint32_t bar = pair_full + 8u * stage;
-                            if (rank == 0) mbar_arrive_expect_tx(full_bar(stage), tx);
-                            else mbar_arrive_cluster(bar);
-                            load(smem_base + (uint32_t)stage * stage_bytes, bar, kb * BK);
+                            if (kb >= early && !take_stage(stage, phase)) return false;
+                            load_a(smem_base + (uint32_t)stage * stage_bytes, pair_full + 8u * stage, kb * BK);
+                            if (kb >= early) load_b(stage, q.k0 + kb * BK);
                             if (++stage == stages) { stage = 0; phase ^= 1u; }
                             // (the second CTA keeps looking until the first one has published the item)
                             if (kb >= look_kb && !have && (kb == look_kb || rank != 0) && !look_ahead()) return false;
                         }
                         return true;
                     };
-                    const CUtensorMap* map_b = &P.map_b;
                     if (gemm) {
                         const CUtensorMap* map_a = a_rows == BM ? &P.map_a : &P.map_a32;
-                        const int b_row = q.group * P.b_group_rows;
                         ok = load_steps([&](uint32_t dst, uint32_t bar, int k) {
                             if (a_rows != 0) tma_load_2d_2cta(dst, map_a, bar, k, q.m0);
                             if (a_rows == 64) tma_load_2d_2cta(dst + 32 * BK * 2, map_a, bar, k, q.m0 + 32);
-                            for (int h = 0; h < q.halves; ++h) {
-                                const uint32_t b_dst = dst + kAStageBytes + h * kBHalfBytesP;
-                                if (!BWD) tma_load_2d_2cta(b_dst, map_b, bar, k, b_row + n0 + h * BN);
-                                else tma_load_3d_2cta(b_dst, map_b, bar, 0, b_row + k, (n0 + h * BN) >> 6);
-                            }
                         });
                     } else if constexpr (BWD) {
                         const CUtensorMap* map_a = &P.map_a;
-                        ok = load_steps([&](uint32_t dst, uint32_t bar, int k) {
-                            tma_load_3d_2cta(dst, map_a, bar, 0, q.k0 + k, q.m0 >> 6);
-                            for (int h = 0; h < q.halves; ++h)
-                                tma_load_3d_2cta(dst + kAStageBytes + h * kBHalfBytesP, map_b, bar, 0, q.k0 + k, (n0 + h * BN) >> 6);
-                        });
+                        ok = load_steps([&](uint32_t dst, uint32_t bar, int k) { tma_load_3d_2cta(dst, map_a, bar, 0, q.k0 + k, q.m0 >> 6); });
                     }
                 }
                 if (L.stats != nullptr) {
@@ -1421,8 +1482,6 @@ LocalLayerPlan local_layer_plan(int T, int K, int E, int H, int I, int keep) {
         p.done2[d] = take(p.blocks_cap);
         p.arrived[d] = take(p.blocks_cap);
     }
-    p.totals = take(E);
-    p.last_hist = take(E + 1);
     p.zero_words = at;
     p.meta = take(kMetaWords);
     p.seg = take(E + 1);
@@ -1449,15 +1508,17 @@ cudaError_t local_layer_route(const LocalLayerParams& q, cudaStream_t stream) {
     a.mu_wd = (p.H + 2 * BM - 1) / (2 * BM); a.nb_wd = column_blocks(p.I, p.cols[1][2]);
     a.mu_wg = (2 * p.I + 2 * BM - 1) / (2 * BM); a.nb_wg = column_blocks(p.H, p.cols[1][3]);
     a.group_units = q.group_units; a.lag_percent = q.lag_percent; a.min_lag_items = q.min_lag_items > 0 ? q.min_lag_items : 0;
-    cudaError_t e = cudaMemsetAsync(q.ws, 0, (size_t)p.zero_words * sizeof(int), stream);
-    if (e != cudaSuccess) return e;
-    if (p.chunks > 0) {
-        local_route_count_kernel<<<p.chunks, kRouteThreads, (2 * p.E + 1) * sizeof(int), stream>>>(a);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    }
     // 64 blocks at least: the lists (tens of thousands of items for a large layer) are written by all blocks
     const int grid = p.chunks > 64 ? p.chunks : 64;
-    local_route_assign_kernel<<<grid, kRouteThreads, (3 * (p.E + 1) + kRouteWarps * (2 * p.E + 1)) * sizeof(int), stream>>>(a);
+    const size_t smem = (3 * (p.E + 1) + (kRouteWarps + 2) * (2 * p.E + 1)) * sizeof(int);
+    if ((long)p.T * p.K <= kDirectEntries) {
+        local_route_assign_kernel<true><<<grid, kRouteThreads, smem, stream>>>(a);
+        return cudaGetLastError();
+    }
+    local_route_count_kernel<<<p.chunks, kRouteThreads, (2 * p.E + 1) * sizeof(int), stream>>>(a);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    local_route_assign_kernel<false><<<grid, kRouteThreads, smem, stream>>>(a);
     return cudaGetLastError();
 }
 

@@ -7,7 +7,7 @@
 
 namespace tmoe {
 
-constexpr int kLocalMaxExperts = 512;    // the routing kernels keep 19 words per expert in shared memory
+constexpr int kLocalMaxExperts = 512;    // the routing kernels keep 23 words per expert in shared memory
 
 // Word offsets of the tables of one call inside its int32 workspace.  Capacities follow from the sizes alone (T * K entries in
 // at most min(E, T * K) segments padded to 128 rows), so the host never has to read the layout back.
@@ -18,7 +18,7 @@ struct LocalLayerPlan {
     int work_cap[2];                     // items of the forward / backward list
     int cols[2][4];                      // columns per tile: [direction][first GEMM, second GEMM, dW_down, dW_gateup]
     // zero-filled by local_layer_route
-    long stats[2], sync[2], totals, last_hist, done1[2], done2[2], arrived[2], zero_words;
+    long stats[2], sync[2], done1[2], done2[2], arrived[2], zero_words;
     // written by it
     long meta, seg, slot_tk, slot_w, token_order, order_slot, chunk_hist, chunk_last, work[2], words;
 };

@@ -29,6 +29,8 @@ def _run(buf, prob, idx, E, **kw):
     (128, 512, 192, 2, 2, False, {}),                    # exactly one full block per expert, half a column block
     (129, 320, 320, 2, 2, False, {}),                    # one row more
     (257, 1088, 704, 5, 3, True, {"stage": 2}),          # three chunks' worth of ragged segments, columns past every tile edge
+    (512, 128, 64, 20, 8, False, {}),                    # the most entries that every routing block counts itself
+    (513, 128, 64, 20, 8, False, {}),                    # one token more: chunk histograms
     (1000, 768, 640, 40, 32, False, {"compute_batch_size": 1024, "combine_start_head_percent": 0}),
     (2100, 512, 256, 8, 4, True, {"compute_batch_size": 4096, "combine_start_head_percent": 100, "total_sms": 64, "num_dispatch_sms": 8}),
 ])
