@@ -9,6 +9,7 @@
 
 #include <array>
 #include <atomic>
+#include <climits>
 #include <memory>
 #include <mutex>
 
@@ -129,17 +130,13 @@ std::tuple<torch::Tensor, torch::Tensor, torch::Tensor> local_counts(torch::Tens
     const auto s = route_scratch(topk_idx, tk, E);
     auto in_rank = torch::empty({tk.T, 1}, on(topk_idx, torch::kBool));
     TM_CHECK_CUDA(tmoe::local_route(tk.ptr, tk.is64, tk.T, tk.K, (int)E, s.totals, s.row_local, s.chunk_base,
-                                    reinterpret_cast<uint8_t*>(in_rank.data_ptr<bool>()), nullptr, cur_stream()));
+                                    reinterpret_cast<uint8_t*>(in_rank.data_ptr<bool>()), nullptr, 0, cur_stream()));
     return {s.all.narrow(0, E, 1), s.all.narrow(0, 0, E), in_rank};
 }
 
-// The one piece of host state: a pinned block that local_route writes the counts into, and the event behind it.
+// The one piece of host state: a pinned block that local_route writes the counts into, each with the number of the call.
 class LocalExchange {
   public:
-    ~LocalExchange() {
-        if (event_ != nullptr) cudaEventDestroy(event_);
-    }
-
     // -> (received payloads, recv_idx, recv_w, counts per expert rounded up to `alignment` (empty with worst_rows), rows (-1: not read),
     //     send_row [T], totals: device [E+1], entries per expert and rows)
     py::tuple dispatch(std::vector<torch::Tensor> parts, torch::Tensor topk_idx, torch::Tensor topk_weights, int64_t E, int64_t worst_rows,
@@ -173,20 +170,16 @@ class LocalExchange {
             const bool wait = worst_rows <= 0;
             if (wait) host_block(E + 1);
             TM_CHECK_CUDA(tmoe::local_route(tk.ptr, tk.is64, tk.T, tk.K, (int)E, s.totals, s.row_local, s.chunk_base, nullptr,
-                                            wait ? host_.data_ptr<int>() : nullptr, stream));
-            if (wait) TORCH_CHECK(cudaEventRecord(event_, stream) == cudaSuccess, "teramoe_b200: cudaEventRecord failed");
+                                            wait ? host_words() : nullptr, seq_, stream));
             TM_CHECK_CUDA(tmoe::local_dispatch(lp.data(), (int)lp.size(), tk.ptr, tk.is64, w.data_ptr<float>(), tk.T, tk.K, (int)E, s.totals,
                                                s.row_local, s.chunk_base, send_row.data_ptr<int>(), idx_out.data_ptr(), w_out.data_ptr<float>(),
                                                (int)std::max<int64_t>(worst_rows, 0), stream));
             totals = s.all.narrow(0, 0, E + 1);
             if (wait) {
                 // the rows are being copied while the host waits for the counts
-                const cudaError_t e = cudaEventSynchronize(event_);
-                TORCH_CHECK(e == cudaSuccess, "teramoe_b200: dispatch failed: ", cudaGetErrorString(e));
-                const int* h = host_.data_ptr<int>();
-                rows = h[0];
+                rows = await_count(0, stream);
                 counts.resize(E);
-                for (int64_t e2 = 0; e2 < E; ++e2) counts[e2] = (h[1 + e2] + alignment - 1) / alignment * alignment;
+                for (int64_t e2 = 0; e2 < E; ++e2) counts[e2] = (await_count(1 + e2, stream) + alignment - 1) / alignment * alignment;
                 if (rows < cap) {
                     for (auto& r : recv) r = r.narrow(0, 0, rows);
                     idx_out = idx_out.narrow(0, 0, rows);
@@ -199,14 +192,27 @@ class LocalExchange {
 
   private:
     void host_block(int64_t n) {
-        if (event_ == nullptr)
-            TORCH_CHECK(cudaEventCreateWithFlags(&event_, cudaEventDisableTiming) == cudaSuccess, "teramoe_b200: cudaEventCreate failed");
         if (!host_.defined() || host_.numel() < n)
-            host_ = torch::empty({n}, torch::TensorOptions().dtype(torch::kInt32).pinned_memory(true));
+            host_ = torch::zeros({n}, torch::TensorOptions().dtype(torch::kInt64).pinned_memory(true));
+        seq_ = seq_ == INT_MAX ? 1 : seq_ + 1;
+    }
+    unsigned long long* host_words() const { return reinterpret_cast<unsigned long long*>(host_.data_ptr<int64_t>()); }
+    // A count, when the kernel has written it.  The stream is asked now and then, so that a failed launch raises and does not spin.
+    int64_t await_count(int64_t i, cudaStream_t stream) const {
+        const unsigned long long* word = host_words() + i;
+        for (int spins = 1;; ++spins) {
+            unsigned long long v = __atomic_load_n(word, __ATOMIC_ACQUIRE);
+            if ((v >> 32) == (unsigned long long)seq_) return (int64_t)(v & 0xffffffffull);
+            if (spins % 20000 != 0) continue;
+            const cudaError_t e = cudaStreamQuery(stream);
+            TORCH_CHECK(e == cudaSuccess || e == cudaErrorNotReady, "teramoe_b200: dispatch failed: ", cudaGetErrorString(e));
+            v = __atomic_load_n(word, __ATOMIC_ACQUIRE);
+            TORCH_CHECK(e == cudaErrorNotReady || (v >> 32) == (unsigned long long)seq_, "teramoe_b200: dispatch wrote no counts");
+        }
     }
     std::mutex mutex_;
     torch::Tensor host_;
-    cudaEvent_t event_ = nullptr;
+    int seq_ = 0;
 };
 
 // A dispatch whose layout is known: payload rows of the tokens that have a row.

@@ -1,6 +1,7 @@
 // Un-fused dispatch / combine on one rank, see local.h.
 //
-//   local_route     counts per expert and the row of every token: one launch, the last block to finish scans the chunks
+//   local_route     counts per expert and the row of every token: up to 1024 tokens one block, which needs no cleared counters; above, a
+//                   memset and one block per 128 tokens, of which the last to finish scans the chunks
 //   local_dispatch  rows, expert ids and weights of the tokens that go anywhere, in token order
 //   local_move      the repeat of a dispatch with a known layout, and the combine
 //
@@ -8,7 +9,9 @@
 // flight per lane), so that a few hundred rows already fill the SMs.  Through the symmetric arena the same dispatch took a
 // push into the arena, a copy out of it, nine table copies and two waits of the host.  Measured through the API, hidden 7168,
 // top-8, 32 experts: layout + dispatch + combine + cached dispatch + combine with weights at 4096 tokens 1175 -> 99 us (77 launches
-// before), layout + FP8 dispatch + combine at 1003 tokens 718 -> 52 us.
+// before), layout + FP8 dispatch + combine at 1003 tokens 718 -> 45 us.
+// The latter is host work: five allocations and four launches, and the wait for the counts, for which the host watches the pinned
+// words that the route kernel writes (an event behind it was seen a few microseconds later).
 #include "local.h"
 
 #include "ptx.cuh"
@@ -18,6 +21,8 @@ namespace tmoe {
 namespace {
 
 constexpr uint32_t kSegBytes = 2048;
+constexpr int kLocalOneBlock = 1024;     // most tokens that one block routes
+static_assert(kLocalOneBlock == 1024, "a warp adds up the counts of 32 warps");
 
 struct Parts {
     LocalPart p[kLocalMaxParts];
@@ -30,9 +35,15 @@ __device__ __forceinline__ long long load_entry(const void* idx, int is64, long 
     return is64 ? reinterpret_cast<const long long*>(idx)[i] : (long long) reinterpret_cast<const int*>(idx)[i];
 }
 
+// A count for the host, with the number of the call in the upper half: every word says by itself whether it is there, so the kernel
+// ends without a fence over the bus (2 us with one and a flag behind it).
+__device__ __forceinline__ void publish(volatile unsigned long long* word, int seq, int count) {
+    *word = ((unsigned long long)(uint32_t)seq << 32) | (uint32_t)count;
+}
+
 __global__ void __launch_bounds__(kLocalChunk)
 local_route_kernel(const void* topk_idx, int is64, int T, int K, int E, int* totals, int* row_local, int* chunk_base, uint8_t* in_rank,
-                   int* host_out) {
+                   unsigned long long* host_out, int host_seq) {
     extern __shared__ int hist[];
     __shared__ int warp_rows[kLocalChunk / 32];
     __shared__ int last;
@@ -88,9 +99,51 @@ local_route_kernel(const void* topk_idx, int is64, int T, int K, int E, int* tot
         }
     }
     if (host_out != nullptr) {
-        if (tid == 0) host_out[0] = __ldcg(totals + E);
-        for (int e = tid; e < E; e += kLocalChunk) host_out[1 + e] = __ldcg(totals + e);
-        __threadfence_system();
+        if (tid == 0) publish(host_out, host_seq, __ldcg(totals + E));
+        for (int e = tid; e < E; e += kLocalChunk) publish(host_out + 1 + e, host_seq, __ldcg(totals + e));
+    }
+}
+
+__global__ void __launch_bounds__(kLocalOneBlock)
+local_route_small_kernel(const void* topk_idx, int is64, int T, int K, int E, int* totals, int* row_local, int* chunk_base, uint8_t* in_rank,
+                         unsigned long long* host_out, int host_seq) {
+    extern __shared__ int hist[];
+    __shared__ int warp_rows[kLocalOneBlock / 32];
+    constexpr int kChunkWarps = kLocalChunk / 32;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5, first = warp / kChunkWarps * kChunkWarps;
+    for (int e = t; e < E; e += kLocalOneBlock) hist[e] = 0;
+    __syncthreads();
+    bool any = false;
+    if (t < T) {
+        for (int k = 0; k < K; ++k) {
+            const long long e = load_entry(topk_idx, is64, (long)t * K + k);
+            if (e >= 0 && e < E) {
+                atomicAdd(&hist[(int)e], 1);
+                any = true;
+            }
+        }
+        if (in_rank != nullptr) in_rank[t] = any ? 1 : 0;
+    }
+    const uint32_t b = __ballot_sync(0xffffffffu, any);
+    if (lane == 0) warp_rows[warp] = __popc(b);
+    __syncthreads();
+    // rows of the warps before this one: of its chunk, and of the chunks before
+    const int own = warp_rows[lane];
+    const int chunks = __reduce_add_sync(0xffffffffu, lane < first ? own : 0);
+    const int before = __reduce_add_sync(0xffffffffu, lane >= first && lane < warp ? own : 0);
+    const int rows = __reduce_add_sync(0xffffffffu, own);
+    if (t < T) {
+        row_local[t] = any ? before + __popc(b & ((1u << lane) - 1u)) : -1;
+        if (t % kLocalChunk == 0) chunk_base[t / kLocalChunk] = chunks;
+    }
+    for (int e = t; e < E; e += kLocalOneBlock) {
+        totals[e] = hist[e];
+        if (host_out != nullptr) publish(host_out + 1 + e, host_seq, hist[e]);
+    }
+    if (t == 0) {
+        totals[E] = rows;
+        if (T == 0) chunk_base[0] = 0;
+        if (host_out != nullptr) publish(host_out, host_seq, rows);
     }
 }
 
@@ -204,13 +257,17 @@ int move_grid(long rows, int segs) {
 }  // namespace
 
 cudaError_t local_route(const void* topk_idx, int is64, int T, int K, int E, int* totals, int* row_local, int* chunk_base, uint8_t* in_rank,
-                        int* host_out, cudaStream_t stream) {
+                        unsigned long long* host_out, int host_seq, cudaStream_t stream) {
     const size_t smem = (size_t)E * sizeof(int);
     if (E < 1 || smem > 40 * 1024) return cudaErrorInvalidValue;
+    if (T <= kLocalOneBlock) {
+        local_route_small_kernel<<<1, kLocalOneBlock, smem, stream>>>(topk_idx, is64, T, K, E, totals, row_local, chunk_base, in_rank, host_out, host_seq);
+        return cudaGetLastError();
+    }
     cudaError_t e = cudaMemsetAsync(totals, 0, (size_t)(E + 2) * sizeof(int), stream);
     if (e != cudaSuccess) return e;
-    const int chunks = T > 0 ? (T + kLocalChunk - 1) / kLocalChunk : 1;
-    local_route_kernel<<<chunks, kLocalChunk, smem, stream>>>(topk_idx, is64, T, K, E, totals, row_local, chunk_base, in_rank, host_out);
+    const int chunks = (T + kLocalChunk - 1) / kLocalChunk;
+    local_route_kernel<<<chunks, kLocalChunk, smem, stream>>>(topk_idx, is64, T, K, E, totals, row_local, chunk_base, in_rank, host_out, host_seq);
     return cudaGetLastError();
 }
 

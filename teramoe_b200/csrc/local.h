@@ -15,13 +15,14 @@ struct LocalPart {
     uint32_t row_bytes;                  // any size; 16-byte multiples on 16-byte aligned tensors are copied 16 bytes at a time
 };
 
-// Routing summary of topk_idx [T,K] in one launch.
-//   totals     [E + 2] zeroed: entries per expert, tokens with at least one valid entry, (scratch)
+// Routing summary of topk_idx [T,K].
+//   totals     [E + 2]: entries per expert, tokens with at least one valid entry, (scratch)
 //   row_local  [T] position of the token among its chunk's tokens that have a valid entry, -1 for tokens without
 //   chunk_base [ceil(T / kLocalChunk)] row of the chunk's first such token
-//   in_rank    optional bool [T]; host_out optional host-visible [E + 1]: number of rows, entries per expert
+//   in_rank    optional bool [T]; host_out optional host-visible [E + 1]: number of rows, entries per expert,
+//              each with host_seq in its upper half
 cudaError_t local_route(const void* topk_idx, int is64, int T, int K, int E, int* totals, int* row_local, int* chunk_base, uint8_t* in_rank,
-                        int* host_out, cudaStream_t stream);
+                        unsigned long long* host_out, int host_seq, cudaStream_t stream);
 
 // Rows of the tokens that have a valid entry, in token order, with their expert ids (-1 where invalid) and weights (0 there);
 // send_row[t] = row of token t or -1.  worst_rows > 0: rows from the received count to worst_rows read as "nothing".

@@ -59,7 +59,8 @@ def test_low_latency_local_kernels_match_window_kernels(T, H, E, K, M, wire):
 
 
 # chunks of 128 tokens: one, a full one, one more token, several; rows of 2 KB segments: a short one, several, odd byte counts (fp8 scales)
-@pytest.mark.parametrize("T,H,E,K", [(0, 256, 4, 2), (1, 128, 4, 1), (128, 1024, 8, 4), (129, 1032, 300, 8), (1003, 7168, 32, 8), (5000, 256, 40, 32)])
+@pytest.mark.parametrize("T,H,E,K", [(0, 256, 4, 2), (1, 128, 4, 1), (128, 1024, 8, 4), (129, 1032, 300, 8), (1003, 7168, 32, 8), (1024, 128, 40, 8), (1025, 128, 40, 8),
+                                      (5000, 256, 40, 32)])
 @pytest.mark.parametrize("fp8", [False, True])
 def test_unfused_exchange_matches_plain_indexing(T, H, E, K, fp8):
     idx, w = _routing(T, E, K, seed=T + H, dtype=torch.int32 if T == 1003 else torch.int64)
