@@ -547,7 +547,7 @@ class Buffer(LowLatencyMixin):
 
         What the schedule arguments do here (same names and accepted values as the reference, teramoe/buffer.py:764-790):
           num_dispatch_sms            SMs (two per CTA pair) that first stream this rank's rows to the other ranks and then
-                                      join the GEMM work
+                                      join the GEMM work (no effect with one rank: nothing is sent)
           total_sms                   grid of the layer kernel / the GEMM kernels
           compute_batch_size          rows per batch of the work list (1024 / 2048 / 4096): a batch's second GEMM follows
                                       its first GEMM batch by batch, so it sets how much activation sits between them
