@@ -31,6 +31,9 @@ CUDA_FLAGS = [
     "-Xptxas", "-v",
 ]
 CXX_FLAGS = ["-O3", "-std=c++17"]
+# The C++ runtime that torch's libraries use.  A compiler that only has the static archive would else put a second runtime into the
+# extension; the two share some symbols and not others, and formatting a number into an error message then crashed the process.
+LD_FLAGS = ["-l:libstdc++.so.6"]
 
 
 def sources() -> list[Path]:
@@ -42,7 +45,7 @@ def _source_hash() -> str:
     for p in sorted(list(_CSRC.glob("*.cu")) + list(_CSRC.glob("*.cpp")) + list(_CSRC.glob("*.h")) + list(_CSRC.glob("*.cuh"))):
         h.update(p.name.encode())
         h.update(p.read_bytes())
-    h.update(" ".join(CUDA_FLAGS + CXX_FLAGS).encode())
+    h.update(" ".join(CUDA_FLAGS + CXX_FLAGS + LD_FLAGS).encode())
     return h.hexdigest()
 
 
@@ -72,6 +75,7 @@ def build(verbose: bool = False) -> Path:
         sources=[str(p) for p in sources()],
         extra_cflags=CXX_FLAGS,
         extra_cuda_cflags=CUDA_FLAGS,
+        extra_ldflags=LD_FLAGS,
         extra_include_paths=[str(_CSRC)],
         build_directory=str(_EXT_DIR),
         with_cuda=True,

@@ -513,6 +513,7 @@ void register_local(pybind11::module_& m) {
         .def(py::init<torch::Tensor, torch::Tensor>())
         .def("set_arena", &LocalLayer::set_arena)
         .def("close", &LocalLayer::close)
+        .def("check", &LocalLayer::check)
         .def("stats", &LocalLayer::stats)
         .def("call", &local_layer_call);
     m.def("local_counts", &local_counts);
