@@ -449,10 +449,14 @@ class LocalLayerFunction : public torch::autograd::Function<LocalLayerFunction> 
         const auto saved = ctx->get_saved_variables();
         auto capsule = ctx->saved_data["h"].toCapsule();
         auto* h = static_cast<Holder*>(capsule.get());
+        // The counters of the workspace are cleared by the forward's routing kernels only, so the kernel can run on it once.  (The node's own
+        // lock covers `spent`.)
+        TORCH_CHECK(!h->spent, "teramoe_b200: a second backward pass over the same forward: its workspace is used up, also with retain_graph=True");
         torch::autograd::variable_list res;
         {
             at::AutoGradMode no_grad(false);
             auto r = h->layer->backward(grads[0].contiguous(), LocalLayer::Kept{saved[2], saved[3]}, saved[0], saved[1], h->K, h->schedule);
+            h->spent = true;
             if (h->grad_topk_w.has_value()) {
                 h->grad_topk_w->copy_(r[1]);
                 r[1] = *h->grad_topk_w;
@@ -476,7 +480,7 @@ class LocalLayerFunction : public torch::autograd::Function<LocalLayerFunction> 
         std::shared_ptr<LocalLayer> layer;
         LocalLayer::Schedule schedule;
         int64_t K;
-        bool strict;
+        bool strict, spent = false;
         c10::optional<torch::Tensor> grad_topk_w;
         std::shared_ptr<PyObject> owner;      // the buffer lives at least as long as a graph that needs its arena
     };

@@ -118,6 +118,33 @@ def test_native_autograd_node_keeps_its_buffer_and_fills_the_given_gradient():
         out.backward(r["go"])
 
 
+def test_second_backward_of_one_forward_raises():
+    """The workspace of a forward serves one backward pass: a second one raises, with and without retain_graph, on this path as on the
+    several-rank kernels, and a call that was refused before it reached the GPU does not count."""
+    prob = make_problem(1, 200, 512, 256, 8, 2, seed=4, dtype=torch.bfloat16, device="cuda", x_scale=0.1, w_scale=0.02)
+    r = prob["ranks"][0]
+    buf = tm.Buffer(None, 0, explicitly_destroy=True)
+    leaves = [r["x"].clone().requires_grad_(True), r["w"].clone().requires_grad_(True), prob["W_gateup"].requires_grad_(True),
+              prob["W_down"].requires_grad_(True)]
+
+    def forward():
+        return buf.teramoe_autograd(leaves[0], r["idx"], leaves[1], leaves[2], leaves[3], 8)
+    want = torch.autograd.grad(forward(), leaves, r["go"])
+    for keep in (False, True):
+        out = forward()
+        buf._world.status[0] = 1                        # a report of an earlier call is raised before anything is launched ...
+        buf._world._status_host[0] = 1
+        with pytest.raises(RuntimeError, match="ran out"):
+            torch.autograd.grad(out, leaves, r["go"], retain_graph=True)
+        got = torch.autograd.grad(out, leaves, r["go"], retain_graph=keep)        # ... so this is the first pass
+        for a, b in zip(got, want):
+            assert torch.equal(a, b)
+        with pytest.raises(RuntimeError, match="second"):
+            torch.autograd.grad(out, leaves, r["go"])
+    buf.check_status()
+    buf.destroy()
+
+
 def test_wide_tiles_match_general_kernels(monkeypatch):
     """Sizes at which every GEMM takes 512-column tiles, with a last tile of one half (4160 = 8 * 512 + 64) and of one and a quarter
     (1344 = 2 * 512 + 320)."""
