@@ -292,8 +292,9 @@ class Buffer(LowLatencyMixin):
         return res, self._leave(cur, async_finish, list(_leaves(res)))
 
     def _run_local(self, fn: Callable, previous_event, async_finish):
-        """A call of the one-rank paths.  It touches no arena, so it needs no order against other calls on this buffer: unless
-        the caller asks for the asynchronous protocol, it goes straight to the current stream."""
+        """A call of the one-rank paths.  It touches no arena, so all it needs to wait for on this buffer is the handle that it is
+        given, whichever stream wrote that (the native calls do): unless the caller asks for the asynchronous protocol, it goes
+        straight to the current stream."""
         self._check_open()
         self._world.poll_status()
         if async_finish or previous_event is not None:
@@ -418,7 +419,8 @@ class Buffer(LowLatencyMixin):
             raise RuntimeError("x must be a bf16 CUDA tensor (or a tuple of payload and scales)")
         if handle is not None:
             rows = handle.num_rows()
-            recv, ev = self._run_local(lambda: self._world.ext.local_scatter(parts, handle.send_row, rows), previous_event, async_finish)
+            recv, ev = self._run_local(lambda: self._world.ext.local_scatter(parts, handle.send_row, handle.written, rows), previous_event,
+                                       async_finish)
             return (tuple(recv) if isinstance(x, tuple) else recv[0]), None, None, None, handle, ev
         if topk_idx is None or topk_weights is None:
             raise ValueError("topk_idx and topk_weights are required without a cached handle")
@@ -428,16 +430,16 @@ class Buffer(LowLatencyMixin):
         if worst > 0 and parts[0].shape[0] > worst:
             raise ValueError(f"{parts[0].shape[0]} tokens exceed num_worst_tokens={worst}")
         topk_idx = topk_idx.contiguous()
-        (recv, recv_idx, recv_w, counts, rows, send_row, totals), ev = self._run_local(
+        (recv, recv_idx, recv_w, counts, rows, send_row, totals, written), ev = self._run_local(
             lambda: self._local.dispatch(parts, topk_idx, topk_weights, E, worst, expert_alignment), previous_event, async_finish)
-        h = LocalHandle(topk_idx.shape[0], topk_idx.shape[1], E, topk_idx, send_row, totals, rows)
+        h = LocalHandle(topk_idx.shape[0], topk_idx.shape[1], E, topk_idx, send_row, totals, rows, written)
         return (tuple(recv) if isinstance(x, tuple) else recv[0]), recv_idx, recv_w, counts, h, ev
 
     def _combine_local(self, x, handle, topk_weights):
         rows = handle.num_rows()
         if x.shape[0] < rows:
             raise ValueError(f"expected {rows} rows (one per received token), got {x.shape[0]}")
-        return self._world.ext.local_combine(x, handle.send_row, handle.topk_idx, handle.E, topk_weights)
+        return self._world.ext.local_combine(x, handle.send_row, handle.written, handle.topk_idx, handle.E, topk_weights)
 
     def _dispatch_fixed_shape(self, x, topk_idx, topk_weights, E, worst):
         """Dispatch with `num_worst_tokens` rows of output and NO host wait (csrc/kernels/intranode.cu:521-531 in the

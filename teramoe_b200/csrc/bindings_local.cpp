@@ -1,6 +1,8 @@
 // Bindings of the one-rank paths.  They allocate their results and launch in one call, so that a call costs the host a few
 // allocations and launches instead of a Python pipeline.
 #include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/CUDAEvent.h>
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <pybind11/stl.h>
 #include <torch/csrc/autograd/functions/basic_ops.h>
@@ -45,6 +47,40 @@ torch::Tensor weights_of(const torch::Tensor& w) {
 }
 torch::TensorOptions on(const torch::Tensor& like, torch::ScalarType t) { return torch::TensorOptions().dtype(t).device(like.device()); }
 
+// The stream that wrote the tables of a handle.  The plain form of a call runs on the caller's stream and the asynchronous one on the
+// communication stream, so a call may use tables that another stream writes: it waits for them there, and the allocator keeps their
+// memory until it is done with them, whenever the handle goes.
+class Written {
+  public:
+    Written() : stream_(c10::cuda::getCurrentCUDAStream()), capture_(capture_of(stream_)) {}
+    bool captured() const { return capture_ != 0; }
+    // Mark the place to wait for; without a mark it is whatever the stream holds when another stream asks.
+    void mark() { event_.record(stream_); }
+    void before_use(std::initializer_list<torch::Tensor> tables) {
+        const auto stream = c10::cuda::getCurrentCUDAStream();
+        for (const auto& t : tables) c10::cuda::CUDACachingAllocator::recordStream(t.storage().data_ptr(), stream);
+        // a graph does not wait for what was enqueued outside it, nor the other way round
+        if (stream == stream_ || capture_of(stream) != capture_) return;
+        if (!event_.isCreated()) {
+            if (capture_of(stream_) != capture_) return;
+            mark();
+        }
+        event_.block(stream);
+    }
+
+  private:
+    static unsigned long long capture_of(const c10::cuda::CUDAStream& s) {
+        cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+        unsigned long long id = 0;
+        const cudaError_t e = cudaStreamGetCaptureInfo(s.stream(), &status, &id);
+        TORCH_CHECK(e == cudaSuccess, "teramoe_b200: ", cudaGetErrorString(e));
+        return status == cudaStreamCaptureStatusNone ? 0 : id;
+    }
+    c10::cuda::CUDAStream stream_;
+    unsigned long long capture_;
+    at::cuda::CUDAEvent event_;
+};
+
 // ------------------------------------------------------------------------------------------------ low latency
 tmoe::LowLatLayout local_layout(int64_t E, int64_t M, int64_t H, int wire, bool logfmt) {
     tmoe::LowLatLayout l{};
@@ -55,8 +91,9 @@ tmoe::LowLatLayout local_layout(int64_t E, int64_t M, int64_t H, int wire, bool 
 }
 
 // wire: 0 bf16, 1 e4m3 + fp32 scales, 2 power-of-two scales, 3 scales packed as UE8M0 bytes
-// -> (recv_x [E,M,H], scales (transposed view of [E,groups,M]) or None, count [E], src_info [E,M], layout_range [E,1], entry_row [T,K])
-std::tuple<torch::Tensor, c10::optional<torch::Tensor>, torch::Tensor, torch::Tensor, torch::Tensor, torch::Tensor>
+// -> (recv_x [E,M,H], scales (transposed view of [E,groups,M]) or None, count [E], src_info [E,M], layout_range [E,1], entry_row [T,K],
+//     stream that writes it)
+std::tuple<torch::Tensor, c10::optional<torch::Tensor>, torch::Tensor, torch::Tensor, torch::Tensor, torch::Tensor, std::shared_ptr<Written>>
 ll_local_dispatch(torch::Tensor x, torch::Tensor topk_idx, int64_t M, int64_t E, int64_t wire, c10::optional<torch::Tensor> expert_stats) {
     c10::cuda::CUDAGuard guard(x.device());
     x = x.contiguous();
@@ -82,12 +119,13 @@ ll_local_dispatch(torch::Tensor x, torch::Tensor topk_idx, int64_t M, int64_t E,
                                           reinterpret_cast<long long*>(range.data_ptr<int64_t>()), count.data_ptr<int>(), stats,
                                           entry.data_ptr<int>(), cur_stream()));
     if (scales.has_value()) scales = scales->transpose(1, 2);
-    return {recv, scales, count, src_info, range, entry};
+    return {recv, scales, count, src_info, range, entry, std::make_shared<Written>()};
 }
 
-torch::Tensor ll_local_combine(torch::Tensor x, torch::Tensor topk_idx, torch::Tensor topk_weights, torch::Tensor entry_row, int64_t M, int64_t E,
-                               int64_t H, bool logfmt, c10::optional<torch::Tensor> out) {
+torch::Tensor ll_local_combine(torch::Tensor x, torch::Tensor topk_idx, torch::Tensor topk_weights, torch::Tensor entry_row,
+                               std::shared_ptr<Written> written, int64_t M, int64_t E, int64_t H, bool logfmt, c10::optional<torch::Tensor> out) {
     c10::cuda::CUDAGuard guard(x.device());
+    written->before_use({entry_row});
     x = x.contiguous();
     topk_idx = topk_idx.contiguous();
     const TopK tk = topk_of(topk_idx);
@@ -138,11 +176,12 @@ std::tuple<torch::Tensor, torch::Tensor, torch::Tensor> local_counts(torch::Tens
 class LocalExchange {
   public:
     // -> (received payloads, recv_idx, recv_w, counts per expert rounded up to `alignment` (empty with worst_rows), rows (-1: not read),
-    //     send_row [T], totals: device [E+1], entries per expert and rows)
+    //     send_row [T], totals: device [E+1], entries per expert and rows, stream that writes them)
     py::tuple dispatch(std::vector<torch::Tensor> parts, torch::Tensor topk_idx, torch::Tensor topk_weights, int64_t E, int64_t worst_rows,
                        int64_t alignment) {
         std::vector<torch::Tensor> recv;
         torch::Tensor idx_out, w_out, send_row, totals;
+        std::shared_ptr<Written> written;
         std::vector<int64_t> counts;
         int64_t rows = -1;
         {
@@ -175,6 +214,9 @@ class LocalExchange {
                                                s.row_local, s.chunk_base, send_row.data_ptr<int>(), idx_out.data_ptr(), w_out.data_ptr<float>(),
                                                (int)std::max<int64_t>(worst_rows, 0), stream));
             totals = s.all.narrow(0, 0, E + 1);
+            written = std::make_shared<Written>();
+            written->before_use({topk_idx});             // (the handle keeps it, possibly a copy from another stream)
+            if (!written->captured()) written->mark();
             if (wait) {
                 // the rows are being copied while the host waits for the counts
                 rows = await_count(0, stream);
@@ -187,7 +229,7 @@ class LocalExchange {
                 }
             }
         }
-        return py::make_tuple(recv, idx_out, w_out, counts, rows, send_row, totals);
+        return py::make_tuple(recv, idx_out, w_out, counts, rows, send_row, totals, written);
     }
 
   private:
@@ -216,8 +258,9 @@ class LocalExchange {
 };
 
 // A dispatch whose layout is known: payload rows of the tokens that have a row.
-std::vector<torch::Tensor> local_scatter(std::vector<torch::Tensor> parts, torch::Tensor send_row, int64_t rows) {
+std::vector<torch::Tensor> local_scatter(std::vector<torch::Tensor> parts, torch::Tensor send_row, std::shared_ptr<Written> written, int64_t rows) {
     c10::cuda::CUDAGuard guard(send_row.device());
+    written->before_use({send_row});
     std::vector<torch::Tensor> recv;
     std::vector<tmoe::LocalPart> lp;
     const int64_t T = send_row.numel();
@@ -234,9 +277,10 @@ std::vector<torch::Tensor> local_scatter(std::vector<torch::Tensor> parts, torch
 }
 
 // out[t] = row send_row[t] of x (zeros for tokens that went nowhere) and, with weights [rows, K], the entries' weights [T, K]
-std::tuple<torch::Tensor, c10::optional<torch::Tensor>> local_combine(torch::Tensor x, torch::Tensor send_row, torch::Tensor topk_idx, int64_t E,
-                                                                      c10::optional<torch::Tensor> weights) {
+std::tuple<torch::Tensor, c10::optional<torch::Tensor>> local_combine(torch::Tensor x, torch::Tensor send_row, std::shared_ptr<Written> written,
+                                                                      torch::Tensor topk_idx, int64_t E, c10::optional<torch::Tensor> weights) {
     c10::cuda::CUDAGuard guard(x.device());
+    written->before_use({send_row, topk_idx});
     x = x.contiguous();
     const TopK tk = topk_of(topk_idx);
     TORCH_CHECK(x.is_cuda() && x.scalar_type() == torch::kBFloat16 && x.dim() == 2, "x must be a bf16 [rows, H] CUDA tensor");
@@ -511,6 +555,7 @@ py::object local_layer_call(std::shared_ptr<LocalLayer> layer, const torch::Tens
 }  // namespace
 
 void register_local(pybind11::module_& m) {
+    py::class_<Written, std::shared_ptr<Written>>(m, "Written");
     m.def("ll_local_dispatch", &ll_local_dispatch);
     m.def("ll_local_combine", &ll_local_combine);
     py::class_<LocalLayer, std::shared_ptr<LocalLayer>>(m, "LocalLayer")

@@ -204,6 +204,7 @@ class LocalHandle:
     send_row: torch.Tensor       # [T] row of the token, -1 if it went nowhere
     totals: torch.Tensor         # [E+1] on the device: entries per expert, number of rows
     rows: int                    # number of rows, -1 while only the device knows it (fixed-shape dispatch)
+    written: object              # stream that wrote the tables (csrc/bindings_local.cpp): calls on other streams wait for it
 
     def num_rows(self) -> int:
         if self.rows < 0:

@@ -103,3 +103,70 @@ def test_unfused_exchange_matches_plain_indexing(T, H, E, K, fp8):
         with pytest.raises(ValueError, match="expected"):
             buf.deepep_combine(y[:-1], fixed)
     buf.destroy()
+
+
+def _stall(stream, ms=40):
+    with torch.cuda.stream(stream):
+        torch.cuda._sleep(int(ms * 1.5e6))             # cycles
+
+
+@pytest.mark.parametrize("call", ["combine", "repeat", "low latency"])
+def test_a_handle_of_the_communication_stream_is_waited_for(call):
+    """The dispatch runs on the communication stream, behind other work there; the next call on its handle runs on the caller's
+    stream and needs nothing else of the dispatch, so nobody has waited for its event."""
+    T, H, E, K, M = (8192, 7168, 32, 8, 0) if call != "low latency" else (64, 512, 8, 4, 64)
+    idx, w = _routing(T, E, K, seed=5)
+    goes = (idx >= 0).any(1)
+    buf = tm.Buffer(None, 0, low_latency_mode=True, explicitly_destroy=True)
+    x = torch.randn(T, H, device="cuda").to(torch.bfloat16)
+    if call == "low latency":
+        y = torch.randn(E, M, H, device="cuda").to(torch.bfloat16)
+        plain = buf.low_latency_dispatch(x, idx, M, E, use_fp8=False)[2]
+        want = buf.low_latency_combine(y, idx, w, plain)[0].clone()
+    torch.cuda.synchronize()
+    _stall(buf.get_comm_stream())
+    if call == "low latency":
+        handle = buf.low_latency_dispatch(x, idx, M, E, use_fp8=False, async_finish=True)[2]
+        got = buf.low_latency_combine(y, idx, w, handle)[0]
+    else:
+        handle = buf.deepep_dispatch(x, topk_idx=idx, topk_weights=w, num_experts=E, async_finish=True)[4]
+        if call == "repeat":
+            got, want = buf.deepep_dispatch(x, handle=handle)[0], x[goes]
+        else:
+            want = torch.where(goes[:, None], x, torch.zeros_like(x))
+            got = buf.deepep_combine(x[goes], handle)[0]
+    torch.cuda.synchronize()
+    assert torch.equal(got, want)
+    buf.destroy()
+
+
+@pytest.mark.parametrize("call", ["combine", "repeat", "low latency"])
+def test_the_tables_of_a_dropped_handle_outlive_the_calls_on_them(call):
+    """The handle goes while the call that uses it still waits on the communication stream.  Memory of its size is asked for at once
+    and filled with zeros, which are valid rows."""
+    T, H, E, K, M = 1000, 512, 8, 4, 1000
+    idx, w = _routing(T, E, K, seed=6)
+    goes = (idx >= 0).any(1)
+    buf = tm.Buffer(None, 0, low_latency_mode=True, explicitly_destroy=True)
+    x = torch.randn(T, H, device="cuda").to(torch.bfloat16)
+    if call == "low latency":
+        y = torch.randn(E, M, H, device="cuda").to(torch.bfloat16)
+        handle = buf.low_latency_dispatch(x, idx, M, E, use_fp8=False)[2]
+        want, n = buf.low_latency_combine(y, idx, w, handle)[0].clone(), T * K
+    else:
+        y = x[goes].contiguous()
+        handle, n = buf.deepep_dispatch(x, topk_idx=idx, topk_weights=w, num_experts=E)[4], T
+        want = y if call == "repeat" else torch.where(goes[:, None], x, torch.zeros_like(x))
+    torch.cuda.synchronize()
+    _stall(buf.get_comm_stream())
+    if call == "low latency":
+        got = buf.low_latency_combine(y, idx, w, handle, async_finish=True)[0]
+    elif call == "repeat":
+        got = buf.deepep_dispatch(x, handle=handle, async_finish=True)[0]
+    else:
+        got = buf.deepep_combine(y, handle, async_finish=True)[0]
+    del handle
+    reuse = [torch.zeros(n, dtype=torch.int32, device="cuda") for _ in range(8)]
+    torch.cuda.synchronize()
+    assert torch.equal(got, want) and len(reuse) == 8
+    buf.destroy()
