@@ -347,7 +347,8 @@ class Buffer(LowLatencyMixin):
         Rows arrive once per (token, rank), ordered by source rank then token.  `recv_topk_idx` holds
         LOCAL expert ids (-1 for experts of other ranks, weights zeroed there), like
         csrc/kernels/intranode.cu:369-378.  With `handle=` (cached mode) only the payload moves and
-        no host synchronisation happens.  `num_worst_tokens > 0` gives fixed-shape outputs (padded rows are
+        no host synchronisation happens (the first use of a fixed-shape handle on one rank waits for its number of rows, which was
+        copied behind the routing).  `num_worst_tokens > 0` gives fixed-shape outputs (padded rows are
         zero, expert id -1, empty per-expert list) without any host wait: the tables are sized for that many rows
         and the layout sizes stay on the device (`_dispatch_fixed_shape`)."""
         if self._local is not None and (x[0] if isinstance(x, tuple) else x).is_cuda:

@@ -1,5 +1,6 @@
 // Bindings of the one-rank paths.  They allocate their results and launch in one call, so that a call costs the host a few
 // allocations and launches instead of a Python pipeline.
+#include <ATen/core/CachingHostAllocator.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/CUDAEvent.h>
 #include <c10/cuda/CUDACachingAllocator.h>
@@ -49,7 +50,8 @@ torch::TensorOptions on(const torch::Tensor& like, torch::ScalarType t) { return
 
 // The stream that wrote the tables of a handle.  The plain form of a call runs on the caller's stream and the asynchronous one on the
 // communication stream, so a call may use tables that another stream writes: it waits for them there, and the allocator keeps their
-// memory until it is done with them, whenever the handle goes.
+// memory until it is done with them, whenever the handle goes.  A handle of a fixed-shape dispatch also gets the number of its rows here:
+// copied behind the routing, to be waited for by whoever asks, from any stream and without waiting for anything else.
 class Written {
   public:
     Written() : stream_(c10::cuda::getCurrentCUDAStream()), capture_(capture_of(stream_)) {}
@@ -68,6 +70,20 @@ class Written {
         event_.block(stream);
     }
 
+    void copy_rows(const int* device_rows) {
+        host_rows_ = torch::empty({1}, torch::TensorOptions().dtype(torch::kInt32).pinned_memory(true));
+        const cudaError_t e = cudaMemcpyAsync(host_rows_.data_ptr(), device_rows, sizeof(int), cudaMemcpyDeviceToHost, stream_.stream());
+        TORCH_CHECK(e == cudaSuccess, "teramoe_b200: ", cudaGetErrorString(e));
+        at::getHostAllocator(at::kCUDA)->record_event(host_rows_.data_ptr(), host_rows_.storage().data_ptr().get_context(), stream_.unwrap());
+        rows_event_.record(stream_);
+    }
+    // -1: not copied
+    int64_t rows() const {
+        if (!host_rows_.defined()) return -1;
+        rows_event_.synchronize();
+        return *host_rows_.data_ptr<int>();
+    }
+
   private:
     static unsigned long long capture_of(const c10::cuda::CUDAStream& s) {
         cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
@@ -78,7 +94,8 @@ class Written {
     }
     c10::cuda::CUDAStream stream_;
     unsigned long long capture_;
-    at::cuda::CUDAEvent event_;
+    at::cuda::CUDAEvent event_, rows_event_;
+    torch::Tensor host_rows_;
 };
 
 // ------------------------------------------------------------------------------------------------ low latency
@@ -210,11 +227,12 @@ class LocalExchange {
             if (wait) host_block(E + 1);
             TM_CHECK_CUDA(tmoe::local_route(tk.ptr, tk.is64, tk.T, tk.K, (int)E, s.totals, s.row_local, s.chunk_base, nullptr,
                                             wait ? host_words() : nullptr, seq_, stream));
+            written = std::make_shared<Written>();
+            if (!wait && !written->captured()) written->copy_rows(s.totals + E);
             TM_CHECK_CUDA(tmoe::local_dispatch(lp.data(), (int)lp.size(), tk.ptr, tk.is64, w.data_ptr<float>(), tk.T, tk.K, (int)E, s.totals,
                                                s.row_local, s.chunk_base, send_row.data_ptr<int>(), idx_out.data_ptr(), w_out.data_ptr<float>(),
                                                (int)std::max<int64_t>(worst_rows, 0), stream));
             totals = s.all.narrow(0, 0, E + 1);
-            written = std::make_shared<Written>();
             written->before_use({topk_idx});             // (the handle keeps it, possibly a copy from another stream)
             if (!written->captured()) written->mark();
             if (wait) {
@@ -555,7 +573,7 @@ py::object local_layer_call(std::shared_ptr<LocalLayer> layer, const torch::Tens
 }  // namespace
 
 void register_local(pybind11::module_& m) {
-    py::class_<Written, std::shared_ptr<Written>>(m, "Written");
+    py::class_<Written, std::shared_ptr<Written>>(m, "Written").def("rows", &Written::rows, py::call_guard<py::gil_scoped_release>());
     m.def("ll_local_dispatch", &ll_local_dispatch);
     m.def("ll_local_combine", &ll_local_combine);
     py::class_<LocalLayer, std::shared_ptr<LocalLayer>>(m, "LocalLayer")

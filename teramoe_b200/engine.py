@@ -208,8 +208,9 @@ class LocalHandle:
 
     def num_rows(self) -> int:
         if self.rows < 0:
-            self.rows = int(self.totals[self.E])
-        return self.rows
+            self.rows = self.written.rows()
+        # a dispatch inside a graph has no copy for the host, and its count may change with every replay
+        return self.rows if self.rows >= 0 else int(self.totals[self.E])
 
 
 @dataclass

@@ -170,3 +170,56 @@ def test_the_tables_of_a_dropped_handle_outlive_the_calls_on_them(call):
     torch.cuda.synchronize()
     assert torch.equal(got, want) and len(reuse) == 8
     buf.destroy()
+
+
+def test_a_fixed_shape_handle_counts_its_rows_on_the_stream_of_its_dispatch():
+    """dispatch on the stalled communication stream, then a repeat behind its event and a combine of the repeated rows"""
+    T, H, E, K = 1000, 512, 8, 4
+    idx, w = _routing(T, E, K, seed=7)
+    goes = (idx >= 0).any(1)
+    buf = tm.Buffer(None, 0, explicitly_destroy=True)
+    x = torch.randn(T, H, device="cuda").to(torch.bfloat16)
+    torch.cuda.synchronize()
+    _stall(buf.get_comm_stream())
+    *_, counts, handle, ev = buf.deepep_dispatch(x, topk_idx=idx, topk_weights=w, num_experts=E, num_worst_tokens=T + 9, async_finish=True)
+    assert counts == [] and handle.rows == -1
+    *_, ev = got = buf.deepep_dispatch(x, handle=handle, previous_event=ev, async_finish=True)
+    ev.current_stream_wait()
+    assert torch.equal(got[0], x[goes]) and handle.rows == int(goes.sum())
+    assert torch.equal(buf.deepep_combine(got[0], handle)[0], torch.where(goes[:, None], x, torch.zeros_like(x)))
+    buf.destroy()
+
+
+def test_the_rows_of_a_fixed_shape_handle_wait_for_nothing_behind_them():
+    T, H, E, K = 300, 512, 8, 4
+    idx, w = _routing(T, E, K, seed=8)
+    buf = tm.Buffer(None, 0, explicitly_destroy=True)
+    x = torch.randn(T, H, device="cuda").to(torch.bfloat16)
+    handle = buf.deepep_dispatch(x, topk_idx=idx, topk_weights=w, num_experts=E, num_worst_tokens=T)[4]
+    _stall(torch.cuda.current_stream(), 300)
+    behind = torch.cuda.Event()
+    behind.record()
+    rows = handle.num_rows()
+    assert not behind.query()
+    assert rows == int((idx >= 0).any(1).sum())
+    buf.destroy()
+
+
+def test_a_fixed_shape_dispatch_in_a_graph_counts_the_rows_of_the_last_replay():
+    T, H, E, K = 300, 512, 8, 4
+    idx, w = _routing(T, E, K, seed=9)
+    buf = tm.Buffer(None, 0, explicitly_destroy=True)
+    x = torch.randn(T, H, device="cuda").to(torch.bfloat16)
+    dispatch = lambda: buf.deepep_dispatch(x, topk_idx=idx, topk_weights=w, num_experts=E, num_worst_tokens=T)
+    dispatch()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        recv, *_, handle, _ = dispatch()
+    for _ in range(2):
+        graph.replay()
+        goes = (idx >= 0).any(1)
+        n = int(goes.sum())
+        assert handle.num_rows() == n and torch.equal(recv[:n], x[goes])
+        idx[: T // 2] = -1
+    buf.destroy()
