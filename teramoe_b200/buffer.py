@@ -440,7 +440,7 @@ class Buffer(LowLatencyMixin):
         rows = handle.num_rows()
         if x.shape[0] < rows:
             raise ValueError(f"expected {rows} rows (one per received token), got {x.shape[0]}")
-        return self._world.ext.local_combine(x, handle.send_row, handle.written, handle.topk_idx, handle.E, topk_weights)
+        return self._world.ext.local_combine(x, handle.send_row, handle.written, rows, handle.topk_idx, handle.E, topk_weights)
 
     def _dispatch_fixed_shape(self, x, topk_idx, topk_weights, E, worst):
         """Dispatch with `num_worst_tokens` rows of output and NO host wait (csrc/kernels/intranode.cu:521-531 in the

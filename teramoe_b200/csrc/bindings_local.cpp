@@ -289,29 +289,34 @@ std::vector<torch::Tensor> local_scatter(std::vector<torch::Tensor> parts, torch
         recv.push_back(torch::empty({rows, p.size(1)}, p.options()));
         lp.push_back(part(p, recv.back()));
     }
-    TM_CHECK_CUDA(tmoe::local_move(lp.data(), (int)lp.size(), send_row.data_ptr<int>(), (int)T, 1, nullptr, 0, 0, 0, nullptr, nullptr,
-                                   cur_stream()));
+    TM_CHECK_CUDA(tmoe::local_move(lp.data(), (int)lp.size(), send_row.data_ptr<int>(), (int)T, rows, 1, nullptr, 0, 0, 0, nullptr,
+                                   nullptr, cur_stream()));
     return recv;
 }
 
-// out[t] = row send_row[t] of x (zeros for tokens that went nowhere) and, with weights [rows, K], the entries' weights [T, K]
+// out[t] = row send_row[t] of x (zeros for tokens that went nowhere) and, with weights [rows, K], the entries' weights [T, K].
+// x and weights may have more rows, and weights more columns, than the dispatch sent.
 std::tuple<torch::Tensor, c10::optional<torch::Tensor>> local_combine(torch::Tensor x, torch::Tensor send_row, std::shared_ptr<Written> written,
-                                                                      torch::Tensor topk_idx, int64_t E, c10::optional<torch::Tensor> weights) {
+                                                                      int64_t rows, torch::Tensor topk_idx, int64_t E,
+                                                                      c10::optional<torch::Tensor> weights) {
     c10::cuda::CUDAGuard guard(x.device());
     written->before_use({send_row, topk_idx});
     x = x.contiguous();
     const TopK tk = topk_of(topk_idx);
-    TORCH_CHECK(x.is_cuda() && x.scalar_type() == torch::kBFloat16 && x.dim() == 2, "x must be a bf16 [rows, H] CUDA tensor");
+    TORCH_CHECK(x.is_cuda() && x.scalar_type() == torch::kBFloat16 && x.dim() == 2 && x.size(0) >= rows, "x must be a bf16 [rows, H] CUDA tensor");
+    TORCH_CHECK(send_row.numel() == tk.T, "the handle is one of another routing");
     auto out = torch::empty({tk.T, x.size(1)}, x.options());
     c10::optional<torch::Tensor> w_out;
     torch::Tensor w;
     if (weights.has_value()) {
-        w = weights_of(*weights);
+        TORCH_CHECK(weights->device() == x.device() && weights->dim() == 2 && weights->size(0) >= rows && weights->size(1) >= tk.K,
+                    "topk_weights must be a [rows, K] tensor on the device of x, as the dispatch returned it");
+        w = weights_of(weights->narrow(1, 0, tk.K));
         w_out = torch::empty({tk.T, tk.K}, w.options());
     }
     const tmoe::LocalPart p = part(x, out);
-    TM_CHECK_CUDA(tmoe::local_move(&p, 1, send_row.data_ptr<int>(), tk.T, 0, tk.ptr, tk.is64, tk.K, (int)E, w.defined() ? w.data_ptr<float>() : nullptr,
-                                   w_out.has_value() ? w_out->data_ptr<float>() : nullptr, cur_stream()));
+    TM_CHECK_CUDA(tmoe::local_move(&p, 1, send_row.data_ptr<int>(), tk.T, rows, 0, tk.ptr, tk.is64, tk.K, (int)E,
+                                   w.defined() ? w.data_ptr<float>() : nullptr, w_out.has_value() ? w_out->data_ptr<float>() : nullptr, cur_stream()));
     return {out, w_out};
 }
 

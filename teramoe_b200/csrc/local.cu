@@ -215,7 +215,7 @@ local_dispatch_kernel(const __grid_constant__ Parts ps, const void* topk_idx, in
 }
 
 __global__ void __launch_bounds__(256)
-local_move_kernel(const __grid_constant__ Parts ps, const int* send_row, int T, int to_rows, const void* topk_idx, int is64, int K, int E,
+local_move_kernel(const __grid_constant__ Parts ps, const int* send_row, int T, long rows, int to_rows, const void* topk_idx, int is64, int K, int E,
                   const float* weights, float* weights_out) {
     const int lane = threadIdx.x & 31;
     const long warps = (long)gridDim.x * (blockDim.x >> 5);
@@ -223,7 +223,8 @@ local_move_kernel(const __grid_constant__ Parts ps, const int* send_row, int T, 
     for (long i = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < work; i += warps) {
         const long t = i / ps.total_segs;
         const int seg = (int)(i - t * ps.total_segs);
-        const long row = send_row[t];
+        const int sent = send_row[t];
+        const long row = sent < rows ? sent : -1;
         if (to_rows) {
             if (row >= 0) move_row_segment(ps, seg, row, t, lane);
             continue;
@@ -283,12 +284,12 @@ cudaError_t local_dispatch(const LocalPart* parts, int num_parts, const void* to
     return cudaGetLastError();
 }
 
-cudaError_t local_move(const LocalPart* parts, int num_parts, const int* send_row, int T, int to_rows, const void* topk_idx, int is64, int K,
+cudaError_t local_move(const LocalPart* parts, int num_parts, const int* send_row, int T, long rows, int to_rows, const void* topk_idx, int is64, int K,
                        int E, const float* weights, float* weights_out, cudaStream_t stream) {
     Parts ps{};
     if (!make_parts(parts, num_parts, ps) || K > 32) return cudaErrorInvalidValue;
     if (T == 0) return cudaSuccess;
-    local_move_kernel<<<move_grid(T, ps.total_segs), 256, 0, stream>>>(ps, send_row, T, to_rows, topk_idx, is64, K, E, weights, weights_out);
+    local_move_kernel<<<move_grid(T, ps.total_segs), 256, 0, stream>>>(ps, send_row, T, rows, to_rows, topk_idx, is64, K, E, weights, weights_out);
     return cudaGetLastError();
 }
 

@@ -31,8 +31,9 @@ cudaError_t local_dispatch(const LocalPart* parts, int num_parts, const void* to
                            int worst_rows, cudaStream_t stream);
 
 // to_rows: dst row send_row[t] <- src row t; otherwise dst row t <- src row send_row[t] (zeros where that is -1), and with
-// `weights` [rows, K]: weights_out[t, k] = weights[send_row[t], k] for valid entries, else 0.
-cudaError_t local_move(const LocalPart* parts, int num_parts, const int* send_row, int T, int to_rows, const void* topk_idx, int is64, int K,
+// `weights` [rows, K]: weights_out[t, k] = weights[send_row[t], k] for valid entries, else 0.  A row past `rows` (those of the tensors
+// that send_row points into) is left alone, or reads as none.
+cudaError_t local_move(const LocalPart* parts, int num_parts, const int* send_row, int T, long rows, int to_rows, const void* topk_idx, int is64, int K,
                        int E, const float* weights, float* weights_out, cudaStream_t stream);
 
 }  // namespace tmoe

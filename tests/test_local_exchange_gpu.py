@@ -223,3 +223,26 @@ def test_a_fixed_shape_dispatch_in_a_graph_counts_the_rows_of_the_last_replay():
         assert handle.num_rows() == n and torch.equal(recv[:n], x[goes])
         idx[: T // 2] = -1
     buf.destroy()
+
+
+def test_combine_takes_weights_of_the_received_rows_only():
+    """As on the several-rank path, more rows and columns than were sent are accepted and left out; fewer, a vector or host memory are not."""
+    T, H, E, K = 300, 512, 8, 4
+    idx, w = _routing(T, E, K, seed=10)
+    valid = idx >= 0
+    buf = tm.Buffer(None, 0, explicitly_destroy=True)
+    x = torch.randn(T, H, device="cuda").to(torch.bfloat16)
+    recv, _, recv_w, _, handle, _ = buf.deepep_dispatch(x, topk_idx=idx, topk_weights=w, num_experts=E)
+    n = recv.shape[0]
+    want = torch.where(valid, w, torch.zeros_like(w))
+    wide = torch.full((n + 3, K + 2), 7.0, device="cuda")
+    wide[:n, :K] = recv_w
+    for good in (recv_w, wide, recv_w.double(), recv_w.t().contiguous().t()):
+        assert torch.equal(buf.deepep_combine(recv, handle, topk_weights=good)[1], want)
+    for bad in (recv_w[:-1], recv_w[:, :-1], recv_w.reshape(-1), recv_w.cpu()):
+        with pytest.raises(RuntimeError, match="topk_weights"):
+            buf.deepep_combine(recv, handle, topk_weights=bad)
+    for bad in (recv[:-1], recv.float(), recv.reshape(-1)):
+        with pytest.raises((ValueError, RuntimeError)):
+            buf.deepep_combine(bad, handle)
+    buf.destroy()
