@@ -343,9 +343,15 @@ class LocalLayer : public std::enable_shared_from_this<LocalLayer> {
 
     LocalLayer(torch::Tensor status, torch::Tensor status_host) : status_(status), host_(status_host) {}
 
+    // Returns when no thread is about to launch on the arena before: what is launched later uses the new one.
     void set_arena(int64_t ptr, int64_t bytes) {
+        std::lock_guard<std::mutex> lock(arena_mutex_);
         arena_ = ptr;
         arena_bytes_ = bytes;
+    }
+    int64_t arena() const {
+        std::lock_guard<std::mutex> lock(arena_mutex_);
+        return arena_;
     }
     void close() { open_ = false; }
 
@@ -365,6 +371,7 @@ class LocalLayer : public std::enable_shared_from_this<LocalLayer> {
     // bytes of the arena that a call needs, 0 if it has them
     int64_t wants(int64_t T, int64_t K, int64_t E, int64_t H) const {
         const int64_t need = local_layer_arena_bytes(T, K, E, H);
+        std::lock_guard<std::mutex> lock(arena_mutex_);
         return need > arena_bytes_ ? need : 0;
     }
 
@@ -403,7 +410,7 @@ class LocalLayer : public std::enable_shared_from_this<LocalLayer> {
         check_layer_weights(w_gateup, w_down, E, H, I);
         tmoe::LocalLayerParams p{};
         p.plan = tmoe::local_layer_plan(tk.T, tk.K, (int)E, (int)H, (int)I, kept != nullptr ? 1 : 0);
-        const int64_t rows = set_common(p, schedule);
+        const int64_t rows = layer_rows(p.plan);
         auto ws = torch::empty({p.plan.words}, on(x, torch::kInt32));
         auto out = torch::empty({tk.T, H}, x.options());
         auto act = torch::empty({rows, I}, x.options());
@@ -418,9 +425,13 @@ class LocalLayer : public std::enable_shared_from_this<LocalLayer> {
         p.x = x.data_ptr(); p.w_gateup = w_gateup.data_ptr(); p.w_down = w_down.data_ptr();
         p.act = act.data_ptr(); p.out = out.data_ptr();
         const cudaStream_t stream = cur_stream();
-        tmoe::count_launch();
-        TM_CHECK_CUDA(tmoe::local_layer_route(p, stream));
-        TM_CHECK_CUDA(tmoe::local_layer_launch(p, stream));
+        {
+            std::lock_guard<std::mutex> lock(arena_mutex_);
+            set_common(p, schedule);
+            tmoe::count_launch();
+            TM_CHECK_CUDA(tmoe::local_layer_route(p, stream));
+            TM_CHECK_CUDA(tmoe::local_layer_launch(p, stream));
+        }
         note(0, ws, p.plan);
         return out;
     }
@@ -436,7 +447,7 @@ class LocalLayer : public std::enable_shared_from_this<LocalLayer> {
         check_layer_weights(w_gateup, w_down, E, H, I);
         tmoe::LocalLayerParams p{};
         p.plan = tmoe::local_layer_plan((int)T, (int)K, (int)E, (int)H, (int)I, 1);
-        const int64_t rows = set_common(p, schedule);
+        const int64_t rows = layer_rows(p.plan);
         TORCH_CHECK(kept.ws.numel() == p.plan.words && kept.rows.numel() == T * H + rows * 2 * I, "saved tensors of another call");
         // act x route [rows, I], dGU [rows, 2I], x in slot order [rows, H], partial sums of d(route weight): one allocation (rows and I, H are
         // multiples of 64: every part starts on a 16-byte boundary)
@@ -455,7 +466,11 @@ class LocalLayer : public std::enable_shared_from_this<LocalLayer> {
         p.act = act_w; p.aux = dgu; p.saved_x = kept.rows.data_ptr(); p.out = dx.data_ptr();
         p.preact = kept.rows.data_ptr<at::BFloat16>() + T * H; p.droute_part = reinterpret_cast<float*>(parts); p.xperm = xperm;
         p.dw_topk = dw.data_ptr<float>(); p.dw_gateup = dwg.data_ptr(); p.dw_down = dwd.data_ptr();
-        TM_CHECK_CUDA(tmoe::local_layer_launch(p, cur_stream()));
+        {
+            std::lock_guard<std::mutex> lock(arena_mutex_);
+            set_common(p, schedule);
+            TM_CHECK_CUDA(tmoe::local_layer_launch(p, cur_stream()));
+        }
         note(1, kept.ws, p.plan);
         return {dx, dw, dwg, dwd};
     }
@@ -468,7 +483,8 @@ class LocalLayer : public std::enable_shared_from_this<LocalLayer> {
     }
 
   private:
-    int64_t set_common(tmoe::LocalLayerParams& p, const Schedule& s) {
+    // (with arena_mutex_ held, until the launch)
+    void set_common(tmoe::LocalLayerParams& p, const Schedule& s) const {
         const int64_t rows = layer_rows(p.plan), half = rows * p.plan.H * 2;
         TORCH_CHECK(2 * half <= arena_bytes_, "the arena is too small for this call");
         p.out_rows = (int)rows;
@@ -477,14 +493,16 @@ class LocalLayer : public std::enable_shared_from_this<LocalLayer> {
         p.group_units = (int)s[0]; p.lag_percent = (int)s[1]; p.min_lag_items = (int)s[2];
         p.num_sms = (int)s[3];
         p.status = status_.data_ptr<int>();
-        return rows;
     }
     void note(int dir, const torch::Tensor& ws, const tmoe::LocalLayerPlan& plan) {
+        torch::Tensor before = ws;            // (the one that goes may have to wait for the interpreter: not under the lock)
         std::lock_guard<std::mutex> lock(mutex_);
-        last_[dir] = ws;
+        std::swap(last_[dir], before);
         last_at_[dir] = plan.stats[dir];
     }
     torch::Tensor status_, host_;
+    // A backward pass runs without the interpreter's lock, next to a call that replaces the arena.
+    mutable std::mutex arena_mutex_;
     int64_t arena_ = 0, arena_bytes_ = 0;
     std::atomic<bool> open_{true};
     std::mutex mutex_;
@@ -583,7 +601,8 @@ void register_local(pybind11::module_& m) {
     m.def("ll_local_combine", &ll_local_combine);
     py::class_<LocalLayer, std::shared_ptr<LocalLayer>>(m, "LocalLayer")
         .def(py::init<torch::Tensor, torch::Tensor>())
-        .def("set_arena", &LocalLayer::set_arena)
+        .def("set_arena", &LocalLayer::set_arena, py::call_guard<py::gil_scoped_release>())
+        .def("arena", &LocalLayer::arena)
         .def("close", &LocalLayer::close)
         .def("check", &LocalLayer::check)
         .def("stats", &LocalLayer::stats)

@@ -23,6 +23,7 @@ The pipeline is written as a generator that yields where it needs something from
 from __future__ import annotations
 
 import os
+import threading
 from typing import Dict, Generator, List, Optional
 
 import torch
@@ -57,7 +58,8 @@ class EPWorld:
         self.control = None
         self.data = None
         self.data_bytes = 0
-        self.on_arena_change = None                 # called with (address, bytes) of the data arena whenever it was replaced
+        self.on_arena_change = None                 # called with (address, bytes) of the data arena before the one it replaces goes
+        self._arena_lock = threading.RLock()        # one thread at a time replaces the arena
         self._ptr_cache: Dict[str, torch.Tensor] = {}
         self.cpu_tables: Dict[str, torch.Tensor] = {}
         self.closed = False
@@ -140,24 +142,28 @@ class EPWorld:
 
     def ensure_data(self, nbytes: int) -> None:
         """Real-mode growth of the data arena (collective over the group)."""
-        if nbytes <= self.data_bytes:
-            return
-        assert self.virtual_peers is None, "virtual clusters grow through VirtualCluster.grow"
-        new_bytes = _round_up(int(nbytes * 1.25))
-        torch.cuda.synchronize(self.device)
-        if self.group is not None and self.size > 1:
-            dist.barrier(group=self.group)
-        old = self.data
-        self.data = self._new_arena(new_bytes)
-        self._open_ipc(self.data)
-        if old is not None:
+        with self._arena_lock:
+            if nbytes <= self.data_bytes:
+                return
+            assert self.virtual_peers is None, "virtual clusters grow through VirtualCluster.grow"
+            new_bytes = _round_up(int(nbytes * 1.25))
+            torch.cuda.synchronize(self.device)
             if self.group is not None and self.size > 1:
                 dist.barrier(group=self.group)
-            old.close()
-        self.data_bytes = new_bytes
-        self._ptr_cache = {k: v for k, v in self._ptr_cache.items() if k.startswith("control")}
-        if self.on_arena_change is not None:
-            self.on_arena_change(self.data.local_ptr(), new_bytes)
+            old = self.data
+            self.data = self._new_arena(new_bytes)
+            self._open_ipc(self.data)
+            self.data_bytes = new_bytes
+            self._ptr_cache = {k: v for k, v in self._ptr_cache.items() if k.startswith("control")}
+            if self.on_arena_change is not None:
+                # a native backward pass needs no interpreter lock: it launches on the new arena from here on, and what it has
+                # launched on the old one since the wait above is waited for
+                self.on_arena_change(self.data.local_ptr(), new_bytes)
+                torch.cuda.synchronize(self.device)
+            if old is not None:
+                if self.group is not None and self.size > 1:
+                    dist.barrier(group=self.group)
+                old.close()
 
     def side_stream(self):
         """High-priority stream for communication kernels that overlap compute."""
@@ -301,6 +307,8 @@ class EPWorld:
             return
         self.closed = True
         if self.is_cuda:
+            if self.on_arena_change is not None:
+                self.on_arena_change(0, 0)           # nothing is launched on the arena behind the wait
             torch.cuda.synchronize(self.device)
             pending_error = None
             try:
@@ -312,8 +320,6 @@ class EPWorld:
                     dist.barrier(group=self.group)
                 except Exception:
                     pass
-            if self.on_arena_change is not None:
-                self.on_arena_change(0, 0)
             if self.data is not None:
                 self.data.close()
             self.control.close()

@@ -3,6 +3,11 @@ import os
 import subprocess
 import sys
 
+import torch
+
+from teramoe_b200.parallel import world as world_module
+from teramoe_b200.parallel.world import EPWorld
+
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
@@ -28,3 +33,53 @@ layer.check()
 print(status.tolist(), int(host[0]))
 """)
     assert "flag wait (site 601, block 5, detail 128)" in out and "[0, 0, 0, 0, 0, 0, 0, 0] 0" in out
+
+
+class _Arena:
+    def __init__(self, log, name):
+        self.log, self.name = log, name
+
+    def local_ptr(self):
+        return 4096 * self.name
+
+    def close(self):
+        self.log.append(("free", self.name))
+
+
+def _logged_world(monkeypatch):
+    log, names = [], iter(range(1, 9))
+    w = EPWorld.single("cpu")
+    monkeypatch.setattr(world_module.torch.cuda, "synchronize", lambda device=None: log.append(("wait",)))
+    monkeypatch.setattr(w, "_new_arena", lambda n: _Arena(log, next(names)))
+    monkeypatch.setattr(w, "_open_ipc", lambda arena: None)
+    w.on_arena_change = lambda ptr, n: log.append(("use", ptr // 4096))
+    return w, log
+
+
+def test_an_arena_is_freed_behind_a_wait_for_its_last_user(monkeypatch):
+    """A backward pass in another thread may launch on the old arena until it is told of the new one: the wait that the old one is
+    freed behind comes after that."""
+    w, log = _logged_world(monkeypatch)
+    w.ensure_data(1000)
+    w.ensure_data(5000)
+    w.ensure_data(10)
+    assert [e for e in log if e[0] != "wait"] == [("use", 1), ("use", 2), ("free", 1)]
+    told, freed = log.index(("use", 2)), log.index(("free", 1))
+    assert ("wait",) in log[told:freed]
+
+
+def test_closing_a_world_takes_the_arena_away_before_it_waits(monkeypatch):
+    w, log = _logged_world(monkeypatch)
+    w.ensure_data(1000)
+    w.is_cuda, w.control = True, _Arena(log, 8)
+    monkeypatch.setattr(w, "check_status", lambda: None)
+    w.close()
+    taken = log.index(("use", 0))
+    assert ("wait",) in log[taken:log.index(("free", 1))]
+
+
+def test_the_native_layer_follows_the_arena():
+    from teramoe_b200._build import load_ext
+    layer = load_ext().LocalLayer(torch.zeros(8, dtype=torch.int32), torch.zeros(4, dtype=torch.int32))
+    layer.set_arena(4096, 100)
+    assert layer.arena() == 4096

@@ -145,6 +145,29 @@ def test_second_backward_of_one_forward_raises():
     buf.destroy()
 
 
+def test_backward_next_to_a_growing_arena():
+    """One thread runs backward passes, which need no interpreter lock, while this one replaces the arena under them."""
+    import threading
+    prob = make_problem(1, 300, 512, 256, 8, 2, seed=6, dtype=torch.bfloat16, device="cuda", x_scale=0.1, w_scale=0.02)
+    r = prob["ranks"][0]
+    buf = tm.Buffer(None, 0, explicitly_destroy=True)
+    leaves = [r["x"].clone().requires_grad_(True), prob["W_gateup"].requires_grad_(True), prob["W_down"].requires_grad_(True)]
+    outs = [buf.teramoe_autograd(leaves[0], r["idx"], r["w"], leaves[1], leaves[2], 8) for _ in range(40)]
+    torch.cuda.synchronize()
+    got = []
+    thread = threading.Thread(target=lambda: got.extend(torch.autograd.grad(o, leaves, r["go"]) for o in outs))
+    thread.start()
+    for _ in range(6):
+        buf._world.ensure_data(buf._world.data_bytes + (1 << 20))
+    thread.join()
+    torch.cuda.synchronize()
+    assert len(got) == len(outs)
+    for g in got[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(g, got[0]))
+    buf.check_status()
+    buf.destroy()
+
+
 def test_wide_tiles_match_general_kernels(monkeypatch):
     """Sizes at which every GEMM takes 512-column tiles, with a last tile of one half (4160 = 8 * 512 + 64) and of one and a quarter
     (1344 = 2 * 512 + 320)."""
