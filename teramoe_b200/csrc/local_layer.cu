@@ -420,10 +420,12 @@ __device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t a, uint32_t
 __device__ __forceinline__ void ld_shared_v4(uint32_t addr, uint32_t (&v)[4]) {
     asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(addr) : "memory");
 }
-// Bounded wait until *flag >= target (counters that other SMs bump).
+// Bounded wait until *flag >= target (counters that other SMs of this GPU bump, so a second is long).  It runs out before the waits
+// inside the CTA pair do (2 s): while the producer waits here, the issuer and the epilogue wait for its operands.
+constexpr uint64_t kCountLimitNs = 1000000000ull;
 __device__ __forceinline__ bool wait_count(const int* flag, int target, int* status, int site, uint32_t pause_ns) {
     if (ld_acquire_gpu(flag) >= target) return true;
-    const uint64_t limit_ns = peer_wait_limit_ns(status);
+    const uint64_t limit_ns = min(peer_wait_limit_ns(status), kCountLimitNs);
     const uint64_t t0 = globaltimer_ns();
 #pragma unroll 1
     while (true) {
@@ -1118,12 +1120,11 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                                 if (++st == stages) { st = 0; ph ^= 1u; }
                             }
                         }
-                        if (!ok || operands_ready(q, true) != 1) {
-                            *abort_flag = 1u;
-                            __nanosleep(100000);                       // (the copies under way land)
-                            ok = false;
-                            break;
-                        }
+                        if (!ok) break;
+                        // A wait that runs out has been reported.  This item is carried through all the same, on whatever its operands
+                        // hold: loads and stores under way end in order, as do the other roles, and no copy outlives its block.  The pair
+                        // takes no further item when the first CTA sees it, and no CTA waits for long once the report is there.
+                        if (operands_ready(q, true) != 1 && rank == 0) claim = total_items;
                     }
                     // stores of other SMs -> async-proxy reads; the weight gradients acquire once, so they need the fence once
                     if (gemm || !wgrad_fenced) fence_proxy_async_all();
@@ -1149,6 +1150,11 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                         const CUtensorMap* map_a = &P.map_a;
                         ok = load_steps([&](uint32_t dst, uint32_t bar, int k) { tma_load_3d_2cta(dst, map_a, bar, 0, q.k0 + k, q.m0 >> 6); });
                     }
+                }
+                if (!ok) {
+                    // A wait inside the pair ran out: no barrier says when the copies under way have landed (those of both CTAs count on the
+                    // first one's, which may never complete).  They take microseconds; no block of the pair ends before this one.
+                    for (const uint64_t t0 = globaltimer_ns(); globaltimer_ns() - t0 < 10000000ull;) __nanosleep(1000);
                 }
                 if (L.stats != nullptr) {
                     if (w_arrive) atomicAdd(L.stats + kStatWaitArrival, w_arrive);

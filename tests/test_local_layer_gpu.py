@@ -145,6 +145,38 @@ def test_second_backward_of_one_forward_raises():
     buf.destroy()
 
 
+def test_a_wait_that_runs_out_is_reported_and_the_next_call_works():
+    """A slot table that says less than the work list lets a block's rows never arrive: the wait for them runs out behind the early
+    loads of weights, the kernel ends in order, the report is raised, and the buffer can be used again."""
+    T, H, E = 128, 512, 2
+    prob = make_problem(1, T, H, 256, E, 1, seed=7, dtype=torch.bfloat16, device="cuda", x_scale=0.1, w_scale=0.02)
+    r = prob["ranks"][0]
+    idx = (torch.arange(T, device="cuda") // 64).view(T, 1)
+    leaves = [r["x"].clone().requires_grad_(True), prob["W_gateup"].requires_grad_(True), prob["W_down"].requires_grad_(True)]
+    buf = tm.Buffer(None, 0, explicitly_destroy=True)
+
+    def forward():
+        return buf.teramoe_autograd(leaves[0], idx, r["w"], leaves[1], leaves[2], E)
+    want = torch.autograd.grad(forward(), leaves, r["go"])
+    out = forward()
+    torch.cuda.synchronize()
+    ws = torch.empty(0, dtype=torch.int32, device="cuda").set_(buf._engine.native.stats(0).untyped_storage())      # tables of that forward
+    slots = list(range(64)) + [-1] * 64 + list(range(64, 128)) + [-1] * 64
+    words = ws.tolist()
+    at = [i for i in range(len(words) - 256) if words[i] == 0 and words[i:i + 256] == slots]
+    assert len(at) == 1
+    ws[at[0]] = -1                                    # the first 64 rows are not copied
+    buf.set_wait_limit_ms(20)
+    torch.autograd.grad(out, leaves, r["go"])
+    with pytest.raises(RuntimeError, match="flag wait"):
+        buf.check_status()
+    buf.set_wait_limit_ms(0)
+    got = torch.autograd.grad(forward(), leaves, r["go"])
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+    buf.check_status()
+    buf.destroy()
+
+
 def test_backward_next_to_a_growing_arena():
     """One thread runs backward passes, which need no interpreter lock, while this one replaces the arena under them."""
     import threading
