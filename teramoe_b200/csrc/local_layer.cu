@@ -554,16 +554,7 @@ __device__ __forceinline__ int4* preact_at(const LayerArgsP& L, int row0, int la
     return reinterpret_cast<int4*>(L.preact) + ((long)(row0 >> 5) * (L.I >> 2) + (col >> 3)) * 32 + lane;
 }
 
-// First GEMM, forward: accumulator columns (2j, 2j+1) = (gate_j, up_j).  act = silu(g) * u * w.
-// 1 / (1 + e^-x).  In the forms that flush denormals: they are lost in the 1 anyway, and the others scale their operands around every
-// one of the two instructions.
-__device__ __forceinline__ float sigmoid(float x) {
-    float t, r;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(t) : "f"(x * -1.4426950408889634f));
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.f + t));
-    return r;
-}
-
+// First GEMM, forward: accumulator columns (2j, 2j+1) = (gate_j, up_j).  act = silu(g) * u * w, as in gemm_common.cuh.
 template <typename R>
 __device__ __forceinline__ void epilogue_swiglu(const LayerArgsP& L, const Staging& st, uint32_t taddr, int row0, float w, int n0, R release) {
     const int n_total = 2 * L.I;
@@ -582,7 +573,7 @@ __device__ __forceinline__ void epilogue_swiglu(const LayerArgsP& L, const Stagi
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
                 const float gt = __uint_as_float(acc[4 * p + 2 * e]), up = __uint_as_float(acc[4 * p + 2 * e + 1]);
-                v[e] = gt * sigmoid(gt) * up * w;
+                v[e] = __fdividef(gt, 1.f + __expf(-gt)) * up * w;
             }
             o[p] = pack_bf16x2(v[0], v[1]);
         }
@@ -645,7 +636,7 @@ __device__ __forceinline__ void epilogue_dswiglu(const LayerArgsP& L, const Stag
                 for (int e = 0; e < 4; ++e) {
                     const float2 gu = unpack_bf16x2(pr[e]);
                     const float ga = real ? __uint_as_float(acc[4 * v + e]) : 0.f;
-                    const float sig = sigmoid(gu.x);
+                    const float sig = __fdividef(1.f, 1.f + __expf(-gu.x));
                     const float s = gu.x * sig;
                     const float a = s * gu.y;
                     const float gaw = ga * w;

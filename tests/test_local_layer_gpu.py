@@ -145,6 +145,47 @@ def test_second_backward_of_one_forward_raises():
     buf.destroy()
 
 
+def test_activation_and_its_gradient_over_the_range_of_the_gate(monkeypatch):
+    """One expert with W_down = identity and gate = x[0], up = x[1] for every column: `out` is the activation itself and dx its two
+    derivatives (64 equal terms).  Against the formulas in 64 bits; silu(g) and its derivative, computed by CUDA's functions, are within
+    their documented errors (a few ulp of 32 bits) far below bf16, whose rounding (2^-9 each of preact, act and result) bounds the rest."""
+    from teramoe_b200 import engine
+    g = torch.cat([s * torch.logspace(-38, 4, 300, dtype=torch.float64) for s in (1.0, -1.0)] + [torch.linspace(-100, 100, 401, dtype=torch.float64),
+                  torch.zeros(1, dtype=torch.float64), torch.linspace(-89, -85, 33, dtype=torch.float64)])
+    T, H, I = g.numel(), 64, 64
+    u = torch.tensor([1.0, -0.75, 3.0], dtype=torch.float64).repeat(T)[:T]
+    x = torch.zeros(T, H)
+    x[:, 0], x[:, 1] = g, u
+    x = x.to(torch.bfloat16).cuda()
+    g, u = x[:, 0].double(), x[:, 1].double()
+    Wg = torch.zeros(1, 2 * I, H, device="cuda", dtype=torch.bfloat16)
+    Wg[0, 0::2, 0] = 1.0
+    Wg[0, 1::2, 1] = 1.0
+    Wd = torch.eye(I, device="cuda", dtype=torch.bfloat16).view(1, H, I).contiguous()
+    idx, w = torch.zeros(T, 1, dtype=torch.int64, device="cuda"), torch.full((T, 1), 0.5, device="cuda")
+    buf = tm.Buffer(None, 0, explicitly_destroy=True)
+    res = []
+    for mode in ("0", "auto"):
+        monkeypatch.setattr(engine, "_LOCAL_LAYER_MODE", mode)
+        leaf = x.clone().requires_grad_(True)
+        out = buf.teramoe_autograd(leaf, idx, w, Wg, Wd, 1)
+        out.backward(torch.ones_like(out))
+        res.append((out.detach(), leaf.grad))
+    assert torch.equal(res[0][0], res[1][0]) and torch.equal(res[0][1], res[1][1])
+    out, dx = res[1]
+    sig = torch.sigmoid(g)
+    s = g * sig
+    tiny = 1e-35                                      # where 1 + e^-g leaves the range of the fast division, and below the normal numbers
+    want = 0.5 * s * u
+    assert bool(((out[:, 0].double() - want).abs() <= 2.0 ** -8 * want.abs() + tiny).all())
+    assert torch.equal(out, out[:, :1].expand_as(out))
+    d_gate, d_up = (sig - s * sig + s) * 0.5 * u, 0.5 * s
+    size = (sig + (s * sig).abs() + s.abs()) * 0.5 * u.abs()      # terms of the derivative, which cancel around g = -1.28
+    assert bool(((dx[:, 0].double() / I - d_gate).abs() <= 2.0 ** -8 * d_gate.abs() + 2.0 ** -20 * size + tiny).all())
+    assert bool(((dx[:, 1].double() / I - d_up).abs() <= 2.0 ** -8 * d_up.abs() + tiny).all())
+    buf.destroy()
+
+
 def test_a_wait_that_runs_out_is_reported_and_the_next_call_works():
     """A slot table that says less than the work list lets a block's rows never arrive: the wait for them runs out behind the early
     loads of weights, the kernel ends in order, the report is raised, and the buffer can be used again."""
