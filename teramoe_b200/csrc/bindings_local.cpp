@@ -60,16 +60,18 @@ class Written {
     void mark() { event_.record(stream_); }
     void before_use(std::initializer_list<torch::Tensor> tables) {
         const auto stream = c10::cuda::getCurrentCUDAStream();
+        if (stream == stream_) return;
         for (const auto& t : tables) c10::cuda::CUDACachingAllocator::recordStream(t.storage().data_ptr(), stream);
         // a graph does not wait for what was enqueued outside it, nor the other way round
-        if (stream == stream_ || capture_of(stream) != capture_) return;
+        if (capture_of(stream) != capture_) return;
         if (!event_.isCreated()) {
             if (capture_of(stream_) != capture_) return;
             mark();
         }
         event_.block(stream);
     }
-
+    // a table that another stream may have made, for as long as this one uses it
+    void keep(const torch::Tensor& table) const { c10::cuda::CUDACachingAllocator::recordStream(table.storage().data_ptr(), stream_); }
     void copy_rows(const int* device_rows) {
         host_rows_ = torch::empty({1}, torch::TensorOptions().dtype(torch::kInt32).pinned_memory(true));
         const cudaError_t e = cudaMemcpyAsync(host_rows_.data_ptr(), device_rows, sizeof(int), cudaMemcpyDeviceToHost, stream_.stream());
@@ -233,7 +235,7 @@ class LocalExchange {
                                                s.row_local, s.chunk_base, send_row.data_ptr<int>(), idx_out.data_ptr(), w_out.data_ptr<float>(),
                                                (int)std::max<int64_t>(worst_rows, 0), stream));
             totals = s.all.narrow(0, 0, E + 1);
-            written->before_use({topk_idx});             // (the handle keeps it, possibly a copy from another stream)
+            written->keep(topk_idx);
             if (!written->captured()) written->mark();
             if (wait) {
                 // the rows are being copied while the host waits for the counts
@@ -311,7 +313,7 @@ std::tuple<torch::Tensor, c10::optional<torch::Tensor>> local_combine(torch::Ten
     if (weights.has_value()) {
         TORCH_CHECK(weights->device() == x.device() && weights->dim() == 2 && weights->size(0) >= rows && weights->size(1) >= tk.K,
                     "topk_weights must be a [rows, K] tensor on the device of x, as the dispatch returned it");
-        w = weights_of(weights->narrow(1, 0, tk.K));
+        w = weights_of(weights->size(1) == tk.K ? *weights : weights->narrow(1, 0, tk.K));
         w_out = torch::empty({tk.T, tk.K}, w.options());
     }
     const tmoe::LocalPart p = part(x, out);
