@@ -450,7 +450,9 @@ class LocalLayer : public std::enable_shared_from_this<LocalLayer> {
         tmoe::LocalLayerParams p{};
         p.plan = tmoe::local_layer_plan((int)T, (int)K, (int)E, (int)H, (int)I, 1);
         const int64_t rows = layer_rows(p.plan);
-        TORCH_CHECK(kept.ws.numel() == p.plan.words && kept.rows.numel() == T * H + rows * 2 * I, "saved tensors of another call");
+        TORCH_CHECK(kept.ws.numel() == p.plan.words && kept.rows.numel() == T * H + rows * 2 * I && kept.rows.device() == grad_out.device() &&
+                    kept.rows.scalar_type() == torch::kBFloat16 && kept.rows.is_contiguous() && reinterpret_cast<uintptr_t>(kept.rows.data_ptr()) % 16 == 0,
+                    "saved tensors of another call");
         // act x route [rows, I], dGU [rows, 2I], x in slot order [rows, H], partial sums of d(route weight): one allocation (rows and I, H are
         // multiples of 64: every part starts on a 16-byte boundary)
         auto scratch = torch::empty({rows * (3 * I + H + 4 * ((I + 255) / 256))}, grad_out.options());
@@ -520,9 +522,11 @@ class LocalLayerFunction : public torch::autograd::Function<LocalLayerFunction> 
                                  std::shared_ptr<LocalLayer> layer, LocalLayer::Schedule schedule, bool strict, std::shared_ptr<PyObject> owner) {
         LocalLayer::Kept kept;
         auto out = layer->forward(x, topk_idx, topk_w, w_gateup, w_down, schedule, &kept);
-        // x itself is not kept
-        ctx->save_for_backward({w_gateup, w_down, kept.ws, kept.rows});
+        // x itself is not kept.  Hooks on saved tensors may move or recompute the rows, or store them in another form; they are not
+        // given the workspace, whose words are places in memory.
+        ctx->save_for_backward({w_gateup, w_down, kept.rows});
         auto holder = c10::make_intrusive<Holder>();
+        holder->ws = kept.ws;
         holder->layer = std::move(layer);
         holder->schedule = schedule;
         holder->K = topk_idx.size(1);
@@ -542,8 +546,9 @@ class LocalLayerFunction : public torch::autograd::Function<LocalLayerFunction> 
         torch::autograd::variable_list res;
         {
             at::AutoGradMode no_grad(false);
-            auto r = h->layer->backward(grads[0].contiguous(), LocalLayer::Kept{saved[2], saved[3]}, saved[0], saved[1], h->K, h->schedule);
+            auto r = h->layer->backward(grads[0].contiguous(), LocalLayer::Kept{h->ws, saved[2]}, saved[0], saved[1], h->K, h->schedule);
             h->spent = true;
+            h->ws = torch::Tensor();
             if (h->grad_topk_w.has_value()) {
                 h->grad_topk_w->copy_(r[1]);
                 r[1] = *h->grad_topk_w;
@@ -568,6 +573,7 @@ class LocalLayerFunction : public torch::autograd::Function<LocalLayerFunction> 
         LocalLayer::Schedule schedule;
         int64_t K;
         bool strict, spent = false;
+        torch::Tensor ws;
         c10::optional<torch::Tensor> grad_topk_w;
         std::shared_ptr<PyObject> owner;      // the buffer lives at least as long as a graph that needs its arena
     };

@@ -186,6 +186,52 @@ def test_activation_and_its_gradient_over_the_range_of_the_gate(monkeypatch):
     buf.destroy()
 
 
+def test_hooks_on_saved_tensors_see_no_workspace():
+    """Hooks get the weights and the kept rows, which they may store elsewhere, recompute (activation checkpointing) or round; a hook that
+    cannot take integers still works, and one that returns something else than it was given raises."""
+    from torch.utils.checkpoint import checkpoint
+    prob = make_problem(1, 200, 512, 256, 8, 2, seed=4, dtype=torch.bfloat16, device="cuda", x_scale=0.1, w_scale=0.02)
+    r = prob["ranks"][0]
+    buf = tm.Buffer(None, 0, explicitly_destroy=True)
+    leaves = [r["x"].clone().requires_grad_(True), r["w"].clone().requires_grad_(True), prob["W_gateup"].requires_grad_(True),
+              prob["W_down"].requires_grad_(True)]
+
+    def forward(*a):
+        return buf.teramoe_autograd(a[0], r["idx"], a[1], a[2], a[3], 8)
+    want = torch.autograd.grad(forward(*leaves), leaves, r["go"])
+    seen = []
+
+    def pack(t):
+        seen.append(t.dtype)
+        return (t.float() * 2).cpu()
+    hooks = torch.autograd.graph.saved_tensors_hooks
+    with hooks(pack, lambda t: (t / 2).to(torch.bfloat16).cuda()):
+        out = forward(*leaves)
+    got = [torch.autograd.grad(out, leaves, r["go"])]
+    assert seen == [torch.bfloat16] * 3
+    got.append(torch.autograd.grad(checkpoint(forward, *leaves, use_reentrant=False), leaves, r["go"]))
+    with torch.autograd.graph.save_on_cpu(pin_memory=True):
+        out = forward(*leaves)
+    got.append(torch.autograd.grad(out, leaves, r["go"]))
+    for g in got:
+        assert all(torch.equal(a, b) for a, b in zip(g, want))
+    for wrong in (lambda t: t.float(), lambda t: t.cpu(), lambda t: t[..., :-1]):
+        with hooks(lambda t: t, wrong):
+            out = forward(*leaves)
+        with pytest.raises(RuntimeError):
+            torch.autograd.grad(out, leaves, r["go"])
+    # only the rows are returned in another form
+    rows = lambda t: t.dim() == 1
+    for wrong in (lambda t: t.float(), lambda t: t.cpu(), lambda t: t[:-1], lambda t: t.repeat_interleave(2)[::2],
+                  lambda t: torch.cat([t[:1], t])[1:]):
+        with hooks(lambda t: t, lambda t, wrong=wrong: wrong(t) if rows(t) else t):
+            out = forward(*leaves)
+        with pytest.raises(RuntimeError, match="saved tensors"):
+            torch.autograd.grad(out, leaves, r["go"])
+    buf.check_status()
+    buf.destroy()
+
+
 def test_a_wait_that_runs_out_is_reported_and_the_next_call_works():
     """A slot table that says less than the work list lets a block's rows never arrive: the wait for them runs out behind the early
     loads of weights, the kernel ends in order, the report is raised, and the buffer can be used again."""
