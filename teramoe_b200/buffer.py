@@ -431,8 +431,11 @@ class Buffer(LowLatencyMixin):
         if worst > 0 and parts[0].shape[0] > worst:
             raise ValueError(f"{parts[0].shape[0]} tokens exceed num_worst_tokens={worst}")
         topk_idx = topk_idx.contiguous()
+        usual = type(expert_alignment) is int and expert_alignment > 0
         (recv, recv_idx, recv_w, counts, rows, send_row, totals, written), ev = self._run_local(
-            lambda: self._local.dispatch(parts, topk_idx, topk_weights, E, worst, expert_alignment), previous_event, async_finish)
+            lambda: self._local.dispatch(parts, topk_idx, topk_weights, E, worst, expert_alignment if usual else 1), previous_event, async_finish)
+        if not usual:                                # as on the several-rank path: zero raises
+            counts = [(c + expert_alignment - 1) // expert_alignment * expert_alignment for c in counts]
         h = LocalHandle(topk_idx.shape[0], topk_idx.shape[1], E, topk_idx, send_row, totals, rows, written)
         return (tuple(recv) if isinstance(x, tuple) else recv[0]), recv_idx, recv_w, counts, h, ev
 

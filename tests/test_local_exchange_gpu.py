@@ -246,3 +246,19 @@ def test_combine_takes_weights_of_the_received_rows_only():
         with pytest.raises((ValueError, RuntimeError)):
             buf.deepep_combine(bad, handle)
     buf.destroy()
+
+
+def test_expert_alignment_of_any_value():
+    """What Python's integer arithmetic gives, on which the several-rank path relies: zero raises."""
+    T, H, E, K = 100, 256, 8, 4
+    idx, w = _routing(T, E, K, seed=11)
+    buf = tm.Buffer(None, 0, explicitly_destroy=True)
+    x = torch.randn(T, H, device="cuda").to(torch.bfloat16)
+    sent = torch.bincount(idx[idx >= 0], minlength=E).tolist()
+    dispatch = lambda a, **kw: buf.deepep_dispatch(x, topk_idx=idx, topk_weights=w, num_experts=E, expert_alignment=a, **kw)[3]
+    for a in (1, 7, 128, -4):
+        assert dispatch(a) == [(c + a - 1) // a * a for c in sent]
+    with pytest.raises(ZeroDivisionError):
+        dispatch(0)
+    assert dispatch(0, num_worst_tokens=T) == []
+    buf.destroy()
