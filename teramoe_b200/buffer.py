@@ -23,7 +23,7 @@ import torch.distributed as dist
 from .config import COMPUTE_BATCH_SIZES, Config, topk_idx_t
 from .engine import EPEngine, LayerHandle, LocalHandle
 from .low_latency import LowLatencyMixin
-from .parallel.world import EPWorld
+from .parallel.world import CONTROL_ROW_INTS, EPWorld
 from .utils.events import EventHandle, EventOverlap
 from .utils.nvlink import check_nvlink_connections
 
@@ -416,6 +416,8 @@ class Buffer(LowLatencyMixin):
         """`deepep_dispatch` on one rank (csrc/local.cu): the rows of the tokens that go anywhere, straight from the caller's
         tensors into the results.  Both parts of an FP8 payload move in the same launch."""
         parts = list(x) if isinstance(x, tuple) else [x]
+        if isinstance(x, tuple) and len(parts) != 2:
+            raise ValueError(f"expected a tuple of payload and scales, got {len(parts)} tensors")
         if not isinstance(x, tuple) and x.dtype != torch.bfloat16:
             raise RuntimeError("x must be a bf16 CUDA tensor (or a tuple of payload and scales)")
         if handle is not None:
@@ -428,6 +430,8 @@ class Buffer(LowLatencyMixin):
         E = num_experts if num_experts is not None else (int(num_tokens_per_expert.numel()) if num_tokens_per_expert is not None else None)
         if E is None:
             raise ValueError("pass num_tokens_per_expert (from get_dispatch_layout) or num_experts")
+        if E + 3 > CONTROL_ROW_INTS:                 # as on the several-rank path: counts of the experts, ranks and tokens
+            raise ValueError("too many experts for the metadata row")
         if worst > 0 and parts[0].shape[0] > worst:
             raise ValueError(f"{parts[0].shape[0]} tokens exceed num_worst_tokens={worst}")
         topk_idx = topk_idx.contiguous()

@@ -262,3 +262,19 @@ def test_expert_alignment_of_any_value():
         dispatch(0)
     assert dispatch(0, num_worst_tokens=T) == []
     buf.destroy()
+
+
+def test_dispatch_refuses_what_the_several_rank_path_refuses():
+    T, H, E, K = 20, 256, 8, 2
+    idx, w = _routing(T, E, K, seed=12)
+    buf = tm.Buffer(None, 0, explicitly_destroy=True)
+    x = torch.randn(T, H, device="cuda").to(torch.bfloat16)
+    handle = buf.deepep_dispatch(x, topk_idx=idx, topk_weights=w, num_experts=8189)[4]
+    for payload in ((x,), (x, x, x)):
+        with pytest.raises(ValueError):
+            buf.deepep_dispatch(payload, topk_idx=idx, topk_weights=w, num_experts=E)
+        with pytest.raises(ValueError):
+            buf.deepep_dispatch(payload, handle=handle)
+    with pytest.raises(ValueError, match="too many experts"):
+        buf.deepep_dispatch(x, topk_idx=idx, topk_weights=w, num_experts=8190)
+    buf.destroy()
