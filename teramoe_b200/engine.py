@@ -653,7 +653,7 @@ class EPEngine:
         if schedule is None:
             # units per batch, lag percent, least lag in items, SMs (see layer_kernel_gen)
             sms = self._grid_sms({"total_sms": opts[0]})
-            schedule = [max(1, opts[1] // UNIT_ROWS), opts[2], int(LOCAL_LAYER_MIN_LAG_PER_PAIR * ((sms or self._num_sms) // 2)), sms]
+            schedule = [max(1, int(opts[1]) // UNIT_ROWS), int(opts[2]), int(LOCAL_LAYER_MIN_LAG_PER_PAIR * ((sms or self._num_sms) // 2)), sms]
             self._schedules[opts] = schedule
         traced = self._trace is not None or NVTX_MARKS
         if traced:

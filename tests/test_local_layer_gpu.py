@@ -186,6 +186,18 @@ def test_activation_and_its_gradient_over_the_range_of_the_gate(monkeypatch):
     buf.destroy()
 
 
+def test_schedule_arguments_may_be_floats():
+    prob = make_problem(1, 200, 512, 256, 8, 2, seed=4, dtype=torch.bfloat16, device="cuda", x_scale=0.1, w_scale=0.02)
+    r = prob["ranks"][0]
+    buf = tm.Buffer(None, 0, explicitly_destroy=True)
+    call = lambda **kw: buf.teramoe_forward(r["x"], r["idx"], r["w"], prob["W_gateup"], prob["W_down"], 8, **kw)
+    want = call()
+    for kw in ({"combine_start_head_percent": 55.5}, {"compute_batch_size": 1024.0, "combine_start_head_percent": 41}, {"total_sms": 100.0}):
+        assert torch.equal(call(**kw), want)
+    assert buf._engine.last_paths.get("layer_kernel", False)
+    buf.destroy()
+
+
 def test_hooks_on_saved_tensors_see_no_workspace():
     """Hooks get the weights and the kept rows, which they may store elsewhere, recompute (activation checkpointing) or round; a hook that
     cannot take integers still works, and one that returns something else than it was given raises."""
