@@ -584,6 +584,10 @@ py::object local_layer_call(std::shared_ptr<LocalLayer> layer, const torch::Tens
                             const torch::Tensor& w_gateup, const torch::Tensor& w_down, int64_t num_experts, LocalLayer::Schedule schedule,
                             bool autograd, const c10::optional<torch::Tensor>& grad_topk_w, bool strict, py::object owner) {
     if (!layer->takes(x, topk_idx, topk_w, w_gateup, w_down, num_experts)) return py::none();
+    // Forward-mode derivatives do not exist.  The Python node says so, also for tensors that require no gradient; this node is not asked then.
+    if (autograd)
+        for (const torch::Tensor* t : {&x, &topk_w, &w_gateup, &w_down})
+            if (t->_fw_grad(0).defined()) return py::none();
     if (const int64_t need = layer->wants(x.size(0), topk_idx.size(1), num_experts, x.size(1))) return py::int_(need);
     torch::Tensor out;
     if (autograd && at::GradMode::is_enabled() && (x.requires_grad() || topk_w.requires_grad() || w_gateup.requires_grad() || w_down.requires_grad())) {

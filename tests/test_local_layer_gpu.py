@@ -198,6 +198,29 @@ def test_schedule_arguments_may_be_floats():
     buf.destroy()
 
 
+def test_forward_mode_and_function_transforms_raise():
+    """There is no forward-mode derivative and no batching rule: both raise, with and without tensors that require a gradient."""
+    import torch.autograd.forward_ad as fwad
+    prob = make_problem(1, 64, 256, 128, 4, 2, seed=4, dtype=torch.bfloat16, device="cuda", x_scale=0.1, w_scale=0.02)
+    r = prob["ranks"][0]
+    buf = tm.Buffer(None, 0, explicitly_destroy=True)
+    tensors = [r["x"], r["w"], prob["W_gateup"], prob["W_down"]]
+    call = lambda x, w, wg, wd: buf.teramoe_autograd(x, r["idx"], w, wg, wd, 4)
+    for i in range(4):
+        for leaf in (False, True):
+            with fwad.dual_level(), pytest.raises(NotImplementedError):
+                args = [t.clone().requires_grad_(leaf and j == i) for j, t in enumerate(tensors)]
+                args[i] = fwad.make_dual(args[i], torch.ones_like(args[i]))
+                call(*args)
+    for transform in (lambda f: torch.func.grad(f)(tensors[0]), lambda f: torch.func.vmap(f)(tensors[0][None]),
+                      lambda f: torch.func.jvp(f, (tensors[0],), (tensors[0],))):
+        with pytest.raises(RuntimeError):
+            transform(lambda x: call(x, *tensors[1:]).float().sum())
+    assert torch.equal(call(*tensors), buf.teramoe_forward(tensors[0], r["idx"], *tensors[1:], 4))
+    buf.check_status()
+    buf.destroy()
+
+
 def test_hooks_on_saved_tensors_see_no_workspace():
     """Hooks get the weights and the kept rows, which they may store elsewhere, recompute (activation checkpointing) or round; a hook that
     cannot take integers still works, and one that returns something else than it was given raises."""
