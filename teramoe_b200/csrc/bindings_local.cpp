@@ -101,6 +101,12 @@ class Written {
 };
 
 // ------------------------------------------------------------------------------------------------ low latency
+// The statistics of waits are accepted as the window kernels accept them and left as they are: nothing is waited for here.
+void check_wait_stats(const c10::optional<torch::Tensor>& t) {
+    TORCH_CHECK(!t.has_value() || (t->is_cuda() && t->scalar_type() == torch::kInt64 && t->is_contiguous()),
+                "wait_stats must be a contiguous int64 CUDA tensor");
+}
+
 tmoe::LowLatLayout local_layout(int64_t E, int64_t M, int64_t H, int wire, bool logfmt) {
     tmoe::LowLatLayout l{};
     l.num_ranks = 1; l.num_experts = (int)E; l.max_tokens = (int)M; l.hidden = (int)H;
@@ -113,8 +119,10 @@ tmoe::LowLatLayout local_layout(int64_t E, int64_t M, int64_t H, int wire, bool 
 // -> (recv_x [E,M,H], scales (transposed view of [E,groups,M]) or None, count [E], src_info [E,M], layout_range [E,1], entry_row [T,K],
 //     stream that writes it)
 std::tuple<torch::Tensor, c10::optional<torch::Tensor>, torch::Tensor, torch::Tensor, torch::Tensor, torch::Tensor, std::shared_ptr<Written>>
-ll_local_dispatch(torch::Tensor x, torch::Tensor topk_idx, int64_t M, int64_t E, int64_t wire, c10::optional<torch::Tensor> expert_stats) {
+ll_local_dispatch(torch::Tensor x, torch::Tensor topk_idx, int64_t M, int64_t E, int64_t wire, c10::optional<torch::Tensor> expert_stats,
+                  c10::optional<torch::Tensor> wait_stats) {
     c10::cuda::CUDAGuard guard(x.device());
+    check_wait_stats(wait_stats);
     x = x.contiguous();
     topk_idx = topk_idx.contiguous();
     const TopK tk = topk_of(topk_idx);
@@ -142,8 +150,10 @@ ll_local_dispatch(torch::Tensor x, torch::Tensor topk_idx, int64_t M, int64_t E,
 }
 
 torch::Tensor ll_local_combine(torch::Tensor x, torch::Tensor topk_idx, torch::Tensor topk_weights, torch::Tensor entry_row,
-                               std::shared_ptr<Written> written, int64_t M, int64_t E, int64_t H, bool logfmt, c10::optional<torch::Tensor> out) {
+                               std::shared_ptr<Written> written, int64_t M, int64_t E, int64_t H, bool logfmt, c10::optional<torch::Tensor> out,
+                               c10::optional<torch::Tensor> wait_stats) {
     c10::cuda::CUDAGuard guard(x.device());
+    check_wait_stats(wait_stats);
     written->before_use({entry_row});
     x = x.contiguous();
     topk_idx = topk_idx.contiguous();

@@ -189,8 +189,8 @@ class LowLatencyMixin:
             raise ValueError(f"{T} tokens exceed num_max_dispatch_tokens_per_rank={M}")
         El = num_experts // N
         if x.is_cuda and self._local is not None and not self.enable_shrink:
-            return self._ll_dispatch_local(x, topk_idx, M, num_experts, cumulative_local_expert_recv_stats, use_fp8, round_scale, use_ue8m0,
-                                           async_finish, return_recv_hook)
+            return self._ll_dispatch_local(x, topk_idx, M, num_experts, cumulative_local_expert_recv_stats, dispatch_wait_recv_cost_stats,
+                                           use_fp8, round_scale, use_ue8m0, async_finish, return_recv_hook)
         if x.is_cuda:
             return self._ll_dispatch_cuda(x, topk_idx, M, num_experts, cumulative_local_expert_recv_stats, dispatch_wait_recv_cost_stats,
                                           use_fp8, round_scale, use_ue8m0, async_finish, return_recv_hook)
@@ -236,7 +236,8 @@ class LowLatencyMixin:
 
     # ------------------------------------------------------------------ one rank (csrc/lowlat.cu, ll_local_*)
     # Nothing crosses a link: the call is one kernel on the caller's stream, into tensors of its own.  Nothing is awaited
-    # either, so with `return_recv_hook` the work is done when the call returns and the hook has nothing left to do.
+    # either, so with `return_recv_hook` the work is done when the call returns and the hook has nothing left to do, and the
+    # statistics of waits stay as they are.
     @staticmethod
     def _ll_check(H, use_fp8, round_scale, use_ue8m0):
         if H % 256 != 0:
@@ -244,22 +245,24 @@ class LowLatencyMixin:
         if use_ue8m0 and not (use_fp8 and round_scale and H % 512 == 0):
             raise ValueError("UE8M0 scales need use_fp8, round_scale and hidden % 512 == 0")
 
-    def _ll_dispatch_local(self, x, topk_idx, M, num_experts, expert_stats, use_fp8, round_scale, use_ue8m0, async_finish, return_recv_hook):
+    def _ll_dispatch_local(self, x, topk_idx, M, num_experts, expert_stats, wait_stats, use_fp8, round_scale, use_ue8m0, async_finish,
+                           return_recv_hook):
         H = x.shape[1]
         self._ll_check(H, use_fp8, round_scale, use_ue8m0)
         wire = 0 if not use_fp8 else 3 if use_ue8m0 else 2 if round_scale else 1
         (recv, scales, count, src_info, layout_range, entry_row, written), ev = self._run_local(
-            lambda: self._world.ext.ll_local_dispatch(x, topk_idx, M, num_experts, wire, expert_stats), None, async_finish and not return_recv_hook)
+            lambda: self._world.ext.ll_local_dispatch(x, topk_idx, M, num_experts, wire, expert_stats, wait_stats), None,
+            async_finish and not return_recv_hook)
         handle = LowLatencyHandle(None, M, H, num_experts, src_info=src_info, layout_range=layout_range, entry_row=entry_row,
                                   written=written)
         return ((recv, scales) if use_fp8 else recv), count, handle, ev, (_nothing if return_recv_hook else None)
 
-    def _ll_combine_local(self, x, topk_idx, topk_weights, handle, use_logfmt, async_finish, return_recv_hook, out):
+    def _ll_combine_local(self, x, topk_idx, topk_weights, handle, use_logfmt, async_finish, return_recv_hook, out, wait_stats):
         if topk_idx.shape[0] > handle.max_tokens:
             raise ValueError(f"{topk_idx.shape[0]} tokens exceed num_max_dispatch_tokens_per_rank={handle.max_tokens}")
         res, ev = self._run_local(
             lambda: self._world.ext.ll_local_combine(x, topk_idx, topk_weights, handle.entry_row, handle.written, handle.max_tokens,
-                                                     handle.num_experts, handle.hidden, use_logfmt, out), None, async_finish and not return_recv_hook)
+                                                     handle.num_experts, handle.hidden, use_logfmt, out, wait_stats), None, async_finish and not return_recv_hook)
         return res, ev, (_nothing if return_recv_hook else None)
 
     # ------------------------------------------------------------------ kernel path (csrc/lowlat.cu)
@@ -395,7 +398,8 @@ class LowLatencyMixin:
         -> (combined_x [T,H], event, hook)."""
         src = self.get_next_low_latency_combine_buffer(handle) if zero_copy else x
         if handle.entry_row is not None:
-            return self._ll_combine_local(src, topk_idx, topk_weights, handle, use_logfmt, async_finish, return_recv_hook, out)
+            return self._ll_combine_local(src, topk_idx, topk_weights, handle, use_logfmt, async_finish, return_recv_hook, out,
+                                          combine_wait_recv_cost_stats)
         if handle.src_info is not None:
             return self._ll_combine_cuda(src, topk_idx, topk_weights, handle, use_logfmt, async_finish, return_recv_hook, out,
                                          combine_wait_recv_cost_stats)

@@ -278,3 +278,21 @@ def test_dispatch_refuses_what_the_several_rank_path_refuses():
     with pytest.raises(ValueError, match="too many experts"):
         buf.deepep_dispatch(x, topk_idx=idx, topk_weights=w, num_experts=8190)
     buf.destroy()
+
+
+def test_wait_statistics_are_checked_and_nothing_is_added():
+    T, H, E, K = 20, 256, 8, 2
+    idx, w = _routing(T, E, K, seed=13)
+    buf = tm.Buffer(None, 0, low_latency_mode=True, explicitly_destroy=True)
+    x, y = torch.randn(T, H, device="cuda").to(torch.bfloat16), torch.randn(E, T, H, device="cuda").to(torch.bfloat16)
+    stats = torch.full((1,), 5, dtype=torch.int64, device="cuda")
+    dispatch = lambda t: buf.low_latency_dispatch(x, idx, T, E, dispatch_wait_recv_cost_stats=t)[2]
+    handle = dispatch(stats)
+    combine = lambda t: buf.low_latency_combine(y, idx, w, handle, combine_wait_recv_cost_stats=t)
+    combine(stats)
+    assert stats.tolist() == [5]
+    for bad in (stats.cpu(), stats.int(), torch.zeros(4, dtype=torch.int64, device="cuda")[::2]):
+        for call in (dispatch, combine):
+            with pytest.raises(RuntimeError, match="wait_stats"):
+                call(bad)
+    buf.destroy()
