@@ -387,6 +387,12 @@ class LocalLayer : public std::enable_shared_from_this<LocalLayer> {
         return need > arena_bytes_ ? need : 0;
     }
 
+    // Forward and backward passes so far: each writes over the arena, a backward pass without anybody in Python being told.
+    int64_t launches() const {
+        std::lock_guard<std::mutex> lock(arena_mutex_);
+        return launches_;
+    }
+
     // strict: wait for the call's kernels, so that the call whose wait ran out is the one that raises
     void settle(bool strict) {
         if (!strict) return;
@@ -498,7 +504,7 @@ class LocalLayer : public std::enable_shared_from_this<LocalLayer> {
 
   private:
     // (with arena_mutex_ held, until the launch)
-    void set_common(tmoe::LocalLayerParams& p, const Schedule& s) const {
+    void set_common(tmoe::LocalLayerParams& p, const Schedule& s) {
         const int64_t rows = layer_rows(p.plan), half = rows * p.plan.H * 2;
         TORCH_CHECK(2 * half <= arena_bytes_, "the arena is too small for this call");
         p.out_rows = (int)rows;
@@ -507,6 +513,7 @@ class LocalLayer : public std::enable_shared_from_this<LocalLayer> {
         p.group_units = (int)s[0]; p.lag_percent = (int)s[1]; p.min_lag_items = (int)s[2];
         p.num_sms = (int)s[3];
         p.status = status_.data_ptr<int>();
+        ++launches_;
     }
     void note(int dir, const torch::Tensor& ws, const tmoe::LocalLayerPlan& plan) {
         torch::Tensor before = ws;            // (the one that goes may have to wait for the interpreter: not under the lock)
@@ -517,7 +524,7 @@ class LocalLayer : public std::enable_shared_from_this<LocalLayer> {
     torch::Tensor status_, host_;
     // A backward pass runs without the interpreter's lock, next to a call that replaces the arena.
     mutable std::mutex arena_mutex_;
-    int64_t arena_ = 0, arena_bytes_ = 0;
+    int64_t arena_ = 0, arena_bytes_ = 0, launches_ = 0;
     std::atomic<bool> open_{true};
     std::mutex mutex_;
     torch::Tensor last_[2];
@@ -625,6 +632,7 @@ void register_local(pybind11::module_& m) {
         .def(py::init<torch::Tensor, torch::Tensor>())
         .def("set_arena", &LocalLayer::set_arena, py::call_guard<py::gil_scoped_release>())
         .def("arena", &LocalLayer::arena)
+        .def("launches", &LocalLayer::launches)
         .def("close", &LocalLayer::close)
         .def("check", &LocalLayer::check)
         .def("stats", &LocalLayer::stats)

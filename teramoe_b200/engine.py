@@ -667,7 +667,6 @@ class EPEngine:
             res = self.native.call(*args)
         if res is None:
             return None
-        w.arena_user = "tables"
         self.last_paths = _LOCAL_PATHS
         if traced:
             self._mark("fwd:layer (routing, dispatch, gate_up, down, sum)")

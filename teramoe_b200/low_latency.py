@@ -271,7 +271,8 @@ class LowLatencyMixin:
         cleared and the ranks cross a barrier, so that no stale bytes can pass for a flag of this call."""
         w = self._world
         geom, total, flag_ranges = _ll_geometry(self.group_size, self.rank, E, M, H, use_fp8, use_ue8m0, round_scale, use_logfmt)
-        key = ("ll", M, H, E, geom[13], geom[14])
+        native = self._engine.native
+        key = ("ll", M, H, E, geom[13], geom[14], native.launches() if native is not None else 0)
 
         def gen():
             yield ("grow", total)

@@ -296,3 +296,24 @@ def test_wait_statistics_are_checked_and_nothing_is_added():
             with pytest.raises(RuntimeError, match="wait_stats"):
                 call(bad)
     buf.destroy()
+
+
+def test_a_backward_pass_of_the_layer_leaves_the_low_latency_windows_to_be_laid_out_again():
+    """The windows of a buffer with a rank mask share the arena with the layer: their flags are cleared behind a backward pass too."""
+    T, H, E, K, M = 256, 512, 4, 2, 8
+    idx, w = _routing(T, E, K, seed=14, drop=0.0)
+    buf = tm.Buffer(None, 0, low_latency_mode=True, explicitly_destroy=True, enable_shrink=True)
+    x = torch.randn(T, H, device="cuda").to(torch.bfloat16).requires_grad_(True)
+    Wg, Wd = (torch.randn(E, n, k, device="cuda").to(torch.bfloat16) * 0.02 for n, k in ((256, H), (H, 128)))
+    out = buf.teramoe_autograd(x, idx, w, Wg, Wd, E)
+    low = lambda: buf.low_latency_dispatch(x.detach()[:M, :256].contiguous(), idx[:M].contiguous(), M, E, use_fp8=False)
+    low()
+    out.backward(torch.ones_like(out))
+    geom = buf._ll_prepare(M, 256, E, False, False, False, False)
+    for off, n in ((geom[10], E * 8), (geom[12], E * 8)):
+        assert not bool(buf._world.data.view(off, [n // 8], torch.int64).any())
+    _, count, *_ = low()
+    sent = idx[:M].flatten().long()
+    assert torch.equal(count.long(), torch.bincount(sent[sent >= 0], minlength=E))
+    buf.check_status()
+    buf.destroy()
