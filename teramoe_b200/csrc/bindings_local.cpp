@@ -446,7 +446,6 @@ class LocalLayer : public std::enable_shared_from_this<LocalLayer> {
         {
             std::lock_guard<std::mutex> lock(arena_mutex_);
             set_common(p, schedule);
-            tmoe::count_launch();
             TM_CHECK_CUDA(tmoe::local_layer_route(p, stream));
             TM_CHECK_CUDA(tmoe::local_layer_launch(p, stream));
         }

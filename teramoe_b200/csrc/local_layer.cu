@@ -27,6 +27,7 @@
 #include "local_layer.h"
 
 #include "gemm_common.cuh"
+#include "launch_count.h"
 #include "layer.h"
 
 namespace tmoe {
@@ -1522,6 +1523,7 @@ cudaError_t local_layer_route(const LocalLayerParams& q, cudaStream_t stream) {
         local_route_assign_kernel<true><<<grid, kRouteThreads, smem, stream>>>(a);
         return cudaGetLastError();
     }
+    count_launch();                                       // (callers count one launch)
     local_route_count_kernel<<<p.chunks, kRouteThreads, (2 * p.E + 1) * sizeof(int), stream>>>(a);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;

@@ -1,4 +1,4 @@
-// The MoE layer on one rank (local_layer.cu): routing preparation in two launches, then ONE cooperative persistent kernel per
+// The MoE layer on one rank (local_layer.cu): routing preparation in one launch or two (by the number of entries), then ONE cooperative persistent kernel per
 // direction.  Same work list, tiles and summation orders as the kernel for several ranks (layer.h), so both give the same
 // bits; what differs is everything that only a second rank needs (peer tables, completion flags, landing rows).
 #pragma once

@@ -221,6 +221,24 @@ def test_forward_mode_and_function_transforms_raise():
     buf.destroy()
 
 
+def test_launches_of_a_call():
+    """Routing is one kernel up to 4096 entries and two above, each direction of the layer one."""
+    from teramoe_b200._build import load_ext
+    buf = tm.Buffer(None, 0, explicitly_destroy=True)
+    for T, forward in ((2048, 2), (2049, 3)):
+        prob = make_problem(1, T, 128, 64, 4, 2, seed=4, dtype=torch.bfloat16, device="cuda", x_scale=0.1, w_scale=0.02)
+        r = prob["ranks"][0]
+        x = r["x"].clone().requires_grad_(True)
+        n = [load_ext().launch_count()]
+        out = buf.teramoe_autograd(x, r["idx"], r["w"], prob["W_gateup"], prob["W_down"], 4)
+        n.append(load_ext().launch_count())
+        out.backward(r["go"])
+        n.append(load_ext().launch_count())
+        assert [b - a for a, b in zip(n, n[1:])] == [forward, 1]
+    buf.check_status()
+    buf.destroy()
+
+
 def test_hooks_on_saved_tensors_see_no_workspace():
     """Hooks get the weights and the kept rows, which they may store elsewhere, recompute (activation checkpointing) or round; a hook that
     cannot take integers still works, and one that returns something else than it was given raises."""
