@@ -367,7 +367,7 @@ struct Phase {
     alignas(64) CUtensorMap map_a;
     alignas(64) CUtensorMap map_b;
     alignas(64) CUtensorMap map_a32;     // the two GEMMs: 32 rows of A
-    int nk, b_group_rows, cols, num_n_blocks, n_total, m_total;
+    int nk, b_group_rows, cols, num_n_blocks, n_total, m_total;      // num_n_blocks: of the two GEMMs
 };
 
 struct LayerArgsP {
@@ -378,7 +378,7 @@ struct LayerArgsP {
     alignas(64) CUtensorMap st_dwd;
     alignas(64) CUtensorMap st_dwg;
     int T, K, H, I, E;
-    int stages, stage_bytes, keep, out_rows;
+    int stages, stage_bytes, keep;
     const uint8_t* x;
     uint8_t* slot_x;
     const __nv_bfloat16* y;
@@ -395,7 +395,7 @@ struct LayerArgsP {
     const int* token_order;              // tokens by their last expert
     const int* order_slot;               // [T, K] slots of the tokens in that order
     const int4* work;
-    int max_work, max_units;
+    int max_work;
     int* sync;
     int* done1;                          // per unit: epilogue warps that finished a tile of the first GEMM
     int* done2;                          // per 128-row block: the same for the second GEMM
@@ -1574,13 +1574,13 @@ cudaError_t local_layer_launch(const LocalLayerParams& q, cudaStream_t stream) {
         if ((e = make_map_mn(&gd.map_b, q.act, R, I)) != cudaSuccess) return e;
         if ((e = make_map_mn(&gg.map_a, q.aux, R, 2 * I)) != cudaSuccess) return e;
         if ((e = make_map_mn(&gg.map_b, q.xperm, R, H)) != cudaSuccess) return e;
-        gd.m_total = H; gd.n_total = I; gd.cols = p.cols[1][2]; gd.num_n_blocks = column_blocks(I, gd.cols);
-        gg.m_total = 2 * I; gg.n_total = H; gg.cols = p.cols[1][3]; gg.num_n_blocks = column_blocks(H, gg.cols);
+        gd.m_total = H; gd.n_total = I; gd.cols = p.cols[1][2];
+        gg.m_total = 2 * I; gg.n_total = H; gg.cols = p.cols[1][3];
         if ((e = make_store_map3(&L.st_dwd, q.dw_down, E, H, I)) != cudaSuccess) return e;
         if ((e = make_store_map3(&L.st_dwg, q.dw_gateup, E, 2 * I, H)) != cudaSuccess) return e;
     }
     g1.num_n_blocks = column_blocks(g1.n_total, g1.cols);
-    L.T = p.T; L.K = p.K; L.H = H; L.I = I; L.E = E; L.keep = p.keep; L.out_rows = q.out_rows;
+    L.T = p.T; L.K = p.K; L.H = H; L.I = I; L.E = E; L.keep = p.keep;
     L.x = static_cast<const uint8_t*>(q.x);
     L.slot_x = static_cast<uint8_t*>(q.slot_x);
     L.y = static_cast<const __nv_bfloat16*>(q.y);
@@ -1598,7 +1598,6 @@ cudaError_t local_layer_launch(const LocalLayerParams& q, cudaStream_t stream) {
     L.order_slot = q.ws + p.order_slot;
     L.work = reinterpret_cast<const int4*>(q.ws + p.work[dir]);
     L.max_work = p.work_cap[dir];
-    L.max_units = p.units_cap;
     L.sync = q.ws + p.sync[dir];
     L.done1 = q.ws + p.done1[dir];
     L.done2 = q.ws + p.done2[dir];
