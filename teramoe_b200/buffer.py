@@ -347,8 +347,8 @@ class Buffer(LowLatencyMixin):
         Rows arrive once per (token, rank), ordered by source rank then token.  `recv_topk_idx` holds
         LOCAL expert ids (-1 for experts of other ranks, weights zeroed there), like
         csrc/kernels/intranode.cu:369-378.  With `handle=` (cached mode) only the payload moves and
-        no host synchronisation happens (the first use of a fixed-shape handle on one rank waits for its number of rows, which was
-        copied behind the routing).  `num_worst_tokens > 0` gives fixed-shape outputs (padded rows are
+        no host synchronisation happens (the first use of a fixed-shape handle on one rank waits for its dispatch, to learn its number
+        of rows).  `num_worst_tokens > 0` gives fixed-shape outputs (padded rows are
         zero, expert id -1, empty per-expert list) without any host wait: the tables are sized for that many rows
         and the layout sizes stay on the device (`_dispatch_fixed_shape`)."""
         if self._local is not None and (x[0] if isinstance(x, tuple) else x).is_cuda:
@@ -422,8 +422,7 @@ class Buffer(LowLatencyMixin):
             raise RuntimeError("x must be a bf16 CUDA tensor (or a tuple of payload and scales)")
         if handle is not None:
             rows = handle.num_rows()
-            recv, ev = self._run_local(lambda: self._world.ext.local_scatter(parts, handle.send_row, handle.written, rows), previous_event,
-                                       async_finish)
+            recv, ev = self._run_local(lambda: self._world.ext.local_scatter(parts, handle.layout, rows), previous_event, async_finish)
             return (tuple(recv) if isinstance(x, tuple) else recv[0]), None, None, None, handle, ev
         if topk_idx is None or topk_weights is None:
             raise ValueError("topk_idx and topk_weights are required without a cached handle")
@@ -436,18 +435,19 @@ class Buffer(LowLatencyMixin):
             raise ValueError(f"{parts[0].shape[0]} tokens exceed num_worst_tokens={worst}")
         topk_idx = topk_idx.contiguous()
         usual = type(expert_alignment) is int and expert_alignment > 0
-        (recv, recv_idx, recv_w, counts, rows, send_row, totals, written), ev = self._run_local(
-            lambda: self._local.dispatch(parts, topk_idx, topk_weights, E, worst, expert_alignment if usual else 1), previous_event, async_finish)
+        (recv, recv_idx, recv_w, counts, rows, layout), ev = self._run_local(
+            lambda: self._local.dispatch(parts, topk_idx, topk_weights, E, worst, expert_alignment if usual else 1,
+                                         async_finish or previous_event is not None), previous_event, async_finish)
         if not usual:                                # as on the several-rank path: zero raises
             counts = [(c + expert_alignment - 1) // expert_alignment * expert_alignment for c in counts]
-        h = LocalHandle(topk_idx.shape[0], topk_idx.shape[1], E, topk_idx, send_row, totals, rows, written)
+        h = LocalHandle(topk_idx.shape[0], topk_idx.shape[1], E, topk_idx, layout, rows)
         return (tuple(recv) if isinstance(x, tuple) else recv[0]), recv_idx, recv_w, counts, h, ev
 
     def _combine_local(self, x, handle, topk_weights):
         rows = handle.num_rows()
         if x.shape[0] < rows:
             raise ValueError(f"expected {rows} rows (one per received token), got {x.shape[0]}")
-        return self._world.ext.local_combine(x, handle.send_row, handle.written, rows, handle.topk_idx, handle.E, topk_weights)
+        return self._world.ext.local_combine(x, handle.layout, rows, handle.topk_idx, handle.E, topk_weights)
 
     def _dispatch_fixed_shape(self, x, topk_idx, topk_weights, E, worst):
         """Dispatch with `num_worst_tokens` rows of output and NO host wait (csrc/kernels/intranode.cu:521-531 in the

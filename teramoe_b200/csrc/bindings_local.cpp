@@ -1,6 +1,5 @@
 // Bindings of the one-rank paths.  They allocate their results and launch in one call, so that a call costs the host a few
 // allocations and launches instead of a Python pipeline.
-#include <ATen/core/CachingHostAllocator.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/CUDAEvent.h>
 #include <c10/cuda/CUDACachingAllocator.h>
@@ -48,57 +47,28 @@ torch::Tensor weights_of(const torch::Tensor& w) {
 }
 torch::TensorOptions on(const torch::Tensor& like, torch::ScalarType t) { return torch::TensorOptions().dtype(t).device(like.device()); }
 
-// The stream that wrote the tables of a handle.  The plain form of a call runs on the caller's stream and the asynchronous one on the
-// communication stream, so a call may use tables that another stream writes: it waits for them there, and the allocator keeps their
-// memory until it is done with them, whenever the handle goes.  A handle of a fixed-shape dispatch also gets the number of its rows here:
-// copied behind the routing, to be waited for by whoever asks, from any stream and without waiting for anything else.
-class Written {
-  public:
-    Written() : stream_(c10::cuda::getCurrentCUDAStream()), capture_(capture_of(stream_)) {}
-    bool captured() const { return capture_ != 0; }
-    // Mark the place to wait for; without a mark it is whatever the stream holds when another stream asks.
-    void mark() { event_.record(stream_); }
-    void before_use(std::initializer_list<torch::Tensor> tables) {
-        const auto stream = c10::cuda::getCurrentCUDAStream();
-        if (stream == stream_) return;
-        for (const auto& t : tables) c10::cuda::CUDACachingAllocator::recordStream(t.storage().data_ptr(), stream);
-        // a graph does not wait for what was enqueued outside it, nor the other way round
-        if (capture_of(stream) != capture_) return;
-        if (!event_.isCreated()) {
-            if (capture_of(stream_) != capture_) return;
-            mark();
-        }
-        event_.block(stream);
-    }
-    // a table that another stream may have made, for as long as this one uses it
-    void keep(const torch::Tensor& table) const { c10::cuda::CUDACachingAllocator::recordStream(table.storage().data_ptr(), stream_); }
-    void copy_rows(const int* device_rows) {
-        host_rows_ = torch::empty({1}, torch::TensorOptions().dtype(torch::kInt32).pinned_memory(true));
-        const cudaError_t e = cudaMemcpyAsync(host_rows_.data_ptr(), device_rows, sizeof(int), cudaMemcpyDeviceToHost, stream_.stream());
-        TORCH_CHECK(e == cudaSuccess, "teramoe_b200: ", cudaGetErrorString(e));
-        at::getHostAllocator(at::kCUDA)->record_event(host_rows_.data_ptr(), host_rows_.storage().data_ptr().get_context(), stream_.unwrap());
-        rows_event_.record(stream_);
-    }
-    // -1: not copied
-    int64_t rows() const {
-        if (!host_rows_.defined()) return -1;
-        rows_event_.synchronize();
-        return *host_rows_.data_ptr<int>();
-    }
-
-  private:
-    static unsigned long long capture_of(const c10::cuda::CUDAStream& s) {
-        cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
-        unsigned long long id = 0;
-        const cudaError_t e = cudaStreamGetCaptureInfo(s.stream(), &status, &id);
-        TORCH_CHECK(e == cudaSuccess, "teramoe_b200: ", cudaGetErrorString(e));
-        return status == cudaStreamCaptureStatusNone ? 0 : id;
-    }
-    c10::cuda::CUDAStream stream_;
-    unsigned long long capture_;
-    at::cuda::CUDAEvent event_, rows_event_;
-    torch::Tensor host_rows_;
-};
+// The plain form of a call runs on the caller's stream and the asynchronous one on the communication stream, so a call may use tables of a
+// handle that another stream writes.  It waits for them there (for `mark`, or else for whatever that stream holds by then), and the
+// allocator keeps their memory until it is done with them, whenever the handle goes.
+unsigned long long capture_of(const c10::cuda::CUDAStream& s) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    unsigned long long id = 0;
+    const cudaError_t e = cudaStreamGetCaptureInfo(s.stream(), &status, &id);
+    TORCH_CHECK(e == cudaSuccess, "teramoe_b200: ", cudaGetErrorString(e));
+    return status == cudaStreamCaptureStatusNone ? 0 : id;
+}
+void use_tables(const c10::cuda::CUDAStream& writer, unsigned long long capture, at::cuda::CUDAEvent* mark, std::initializer_list<torch::Tensor> tables) {
+    const auto stream = c10::cuda::getCurrentCUDAStream();
+    if (stream == writer) return;
+    for (const auto& t : tables) c10::cuda::CUDACachingAllocator::recordStream(t.storage().data_ptr(), stream);
+    // a graph does not wait for what was enqueued outside it, nor the other way round
+    if (capture_of(stream) != capture) return;
+    if (mark != nullptr) return mark->block(stream);
+    if (capture_of(writer) != capture) return;
+    at::cuda::CUDAEvent now;
+    now.record(writer);
+    now.block(stream);
+}
 
 // ------------------------------------------------------------------------------------------------ low latency
 // The statistics of waits are accepted as the window kernels accept them and left as they are: nothing is waited for here.
@@ -117,8 +87,8 @@ tmoe::LowLatLayout local_layout(int64_t E, int64_t M, int64_t H, int wire, bool 
 
 // wire: 0 bf16, 1 e4m3 + fp32 scales, 2 power-of-two scales, 3 scales packed as UE8M0 bytes
 // -> (recv_x [E,M,H], scales (transposed view of [E,groups,M]) or None, count [E], src_info [E,M], layout_range [E,1], entry_row [T,K],
-//     stream that writes it)
-std::tuple<torch::Tensor, c10::optional<torch::Tensor>, torch::Tensor, torch::Tensor, torch::Tensor, torch::Tensor, std::shared_ptr<Written>>
+//     id of the stream that writes it)
+std::tuple<torch::Tensor, c10::optional<torch::Tensor>, torch::Tensor, torch::Tensor, torch::Tensor, torch::Tensor, int64_t>
 ll_local_dispatch(torch::Tensor x, torch::Tensor topk_idx, int64_t M, int64_t E, int64_t wire, c10::optional<torch::Tensor> expert_stats,
                   c10::optional<torch::Tensor> wait_stats) {
     c10::cuda::CUDAGuard guard(x.device());
@@ -146,15 +116,16 @@ ll_local_dispatch(torch::Tensor x, torch::Tensor topk_idx, int64_t M, int64_t E,
                                           reinterpret_cast<long long*>(range.data_ptr<int64_t>()), count.data_ptr<int>(), stats,
                                           entry.data_ptr<int>(), cur_stream()));
     if (scales.has_value()) scales = scales->transpose(1, 2);
-    return {recv, scales, count, src_info, range, entry, std::make_shared<Written>()};
+    return {recv, scales, count, src_info, range, entry, c10::cuda::getCurrentCUDAStream().id()};
 }
 
 torch::Tensor ll_local_combine(torch::Tensor x, torch::Tensor topk_idx, torch::Tensor topk_weights, torch::Tensor entry_row,
-                               std::shared_ptr<Written> written, int64_t M, int64_t E, int64_t H, bool logfmt, c10::optional<torch::Tensor> out,
+                               int64_t writer, int64_t M, int64_t E, int64_t H, bool logfmt, c10::optional<torch::Tensor> out,
                                c10::optional<torch::Tensor> wait_stats) {
     c10::cuda::CUDAGuard guard(x.device());
     check_wait_stats(wait_stats);
-    written->before_use({entry_row});
+    const auto w_stream = c10::cuda::CUDAStream::unpack3(writer, x.device().index(), c10::DeviceType::CUDA);
+    if (w_stream != c10::cuda::getCurrentCUDAStream()) use_tables(w_stream, capture_of(w_stream), nullptr, {entry_row});
     x = x.contiguous();
     topk_idx = topk_idx.contiguous();
     const TopK tk = topk_of(topk_idx);
@@ -201,16 +172,70 @@ std::tuple<torch::Tensor, torch::Tensor, torch::Tensor> local_counts(torch::Tens
     return {s.all.narrow(0, E, 1), s.all.narrow(0, 0, E), in_rank};
 }
 
+// Events of dropped layouts, for the next ones: creating and destroying one costs about as much as recording it.
+struct Marks {
+    static constexpr size_t kMost = 16;
+    std::mutex mutex;
+    std::vector<at::cuda::CUDAEvent> spare;
+    at::cuda::CUDAEvent take() {
+        std::lock_guard<std::mutex> lock(mutex);
+        if (spare.empty()) return at::cuda::CUDAEvent();
+        at::cuda::CUDAEvent e = std::move(spare.back());
+        spare.pop_back();
+        return e;
+    }
+    void give(at::cuda::CUDAEvent&& e) {
+        std::lock_guard<std::mutex> lock(mutex);
+        if (e.isCreated() && spare.size() < kMost) spare.push_back(std::move(e));
+    }
+};
+
+// What a dispatch leaves for the calls on its handle: where the tokens' rows are, the totals, and the stream that writes both.
+struct LocalLayout {
+    LocalLayout() = default;
+    LocalLayout(const LocalLayout&) = delete;
+    ~LocalLayout() {
+        if (marks != nullptr) marks->give(std::move(written));
+    }
+
+    torch::Tensor send_row, scratch;         // [T]; [E + 1] and more: entries per expert, rows
+    int64_t E = 0;
+    c10::cuda::CUDAStream writer = c10::cuda::getCurrentCUDAStream();
+    unsigned long long capture = capture_of(writer);
+    std::shared_ptr<Marks> marks;
+    at::cuda::CUDAEvent written;             // recorded where `mark` was called
+
+    // Not called in a graph, nor for a plain call of known size: that one is on the caller's stream, which those who go on with its handle on
+    // another one usually wait for anyway.
+    void mark(std::shared_ptr<Marks> m) {
+        marks = std::move(m);
+        written = marks->take();
+        written.record(writer);
+    }
+    void use(std::initializer_list<torch::Tensor> tables) { use_tables(writer, capture, marks != nullptr ? &written : nullptr, tables); }
+    // The number of rows, for whoever asks, from any stream and without waiting for what was enqueued since.  Of a dispatch inside a graph,
+    // that of the last replay.
+    int64_t rows() {
+        c10::cuda::CUDAGuard guard(scratch.device());
+        const torch::Tensor n = scratch.narrow(0, E, 1);
+        if (marks == nullptr) return n.item<int>();
+        const auto side = c10::cuda::getStreamFromPool();
+        c10::cuda::CUDAStreamGuard on_side(side);
+        written.block(side);
+        return n.item<int>();
+    }
+};
+
 // The one piece of host state: a pinned block that local_route writes the counts into, each with the number of the call.
 class LocalExchange {
   public:
     // -> (received payloads, recv_idx, recv_w, counts per expert rounded up to `alignment` (empty with worst_rows), rows (-1: not read),
-    //     send_row [T], totals: device [E+1], entries per expert and rows, stream that writes them)
+    //     layout)
     py::tuple dispatch(std::vector<torch::Tensor> parts, torch::Tensor topk_idx, torch::Tensor topk_weights, int64_t E, int64_t worst_rows,
-                       int64_t alignment) {
+                       int64_t alignment, bool mark) {
         std::vector<torch::Tensor> recv;
-        torch::Tensor idx_out, w_out, send_row, totals;
-        std::shared_ptr<Written> written;
+        torch::Tensor idx_out, w_out;
+        std::shared_ptr<LocalLayout> layout;
         std::vector<int64_t> counts;
         int64_t rows = -1;
         {
@@ -234,19 +259,21 @@ class LocalExchange {
             }
             idx_out = torch::empty({cap, tk.K}, topk_idx.options());
             w_out = torch::empty({cap, tk.K}, w.options());
-            send_row = torch::empty({tk.T}, on(topk_idx, torch::kInt32));
+            const auto send_row = torch::empty({tk.T}, on(topk_idx, torch::kInt32));
             const bool wait = worst_rows <= 0;
             if (wait) host_block(E + 1);
             TM_CHECK_CUDA(tmoe::local_route(tk.ptr, tk.is64, tk.T, tk.K, (int)E, s.totals, s.row_local, s.chunk_base, nullptr,
                                             wait ? host_words() : nullptr, seq_, stream));
-            written = std::make_shared<Written>();
-            if (!wait && !written->captured()) written->copy_rows(s.totals + E);
             TM_CHECK_CUDA(tmoe::local_dispatch(lp.data(), (int)lp.size(), tk.ptr, tk.is64, w.data_ptr<float>(), tk.T, tk.K, (int)E, s.totals,
                                                s.row_local, s.chunk_base, send_row.data_ptr<int>(), idx_out.data_ptr(), w_out.data_ptr<float>(),
                                                (int)std::max<int64_t>(worst_rows, 0), stream));
-            totals = s.all.narrow(0, 0, E + 1);
-            written->keep(topk_idx);
-            if (!written->captured()) written->mark();
+            layout = std::make_shared<LocalLayout>();
+            layout->send_row = send_row;
+            layout->scratch = s.all;
+            layout->E = E;
+            // the handle keeps the indices, which another stream may have made
+            c10::cuda::CUDACachingAllocator::recordStream(topk_idx.storage().data_ptr(), layout->writer);
+            if ((mark || !wait) && layout->capture == 0) layout->mark(marks_);
             if (wait) {
                 // the rows are being copied while the host waits for the counts
                 rows = await_count(0, stream);
@@ -259,7 +286,7 @@ class LocalExchange {
                 }
             }
         }
-        return py::make_tuple(recv, idx_out, w_out, counts, rows, send_row, totals, written);
+        return py::make_tuple(recv, idx_out, w_out, counts, rows, layout);
     }
 
   private:
@@ -283,14 +310,16 @@ class LocalExchange {
         }
     }
     std::mutex mutex_;
+    std::shared_ptr<Marks> marks_ = std::make_shared<Marks>();
     torch::Tensor host_;
     int seq_ = 0;
 };
 
 // A dispatch whose layout is known: payload rows of the tokens that have a row.
-std::vector<torch::Tensor> local_scatter(std::vector<torch::Tensor> parts, torch::Tensor send_row, std::shared_ptr<Written> written, int64_t rows) {
+std::vector<torch::Tensor> local_scatter(std::vector<torch::Tensor> parts, const std::shared_ptr<LocalLayout>& layout, int64_t rows) {
+    const torch::Tensor& send_row = layout->send_row;
     c10::cuda::CUDAGuard guard(send_row.device());
-    written->before_use({send_row});
+    layout->use({send_row});
     std::vector<torch::Tensor> recv;
     std::vector<tmoe::LocalPart> lp;
     const int64_t T = send_row.numel();
@@ -308,11 +337,11 @@ std::vector<torch::Tensor> local_scatter(std::vector<torch::Tensor> parts, torch
 
 // out[t] = row send_row[t] of x (zeros for tokens that went nowhere) and, with weights [rows, K], the entries' weights [T, K].
 // x and weights may have more rows, and weights more columns, than the dispatch sent.
-std::tuple<torch::Tensor, c10::optional<torch::Tensor>> local_combine(torch::Tensor x, torch::Tensor send_row, std::shared_ptr<Written> written,
-                                                                      int64_t rows, torch::Tensor topk_idx, int64_t E,
-                                                                      c10::optional<torch::Tensor> weights) {
+std::tuple<torch::Tensor, c10::optional<torch::Tensor>> local_combine(torch::Tensor x, const std::shared_ptr<LocalLayout>& layout, int64_t rows,
+                                                                      torch::Tensor topk_idx, int64_t E, c10::optional<torch::Tensor> weights) {
+    const torch::Tensor& send_row = layout->send_row;
     c10::cuda::CUDAGuard guard(x.device());
-    written->before_use({send_row, topk_idx});
+    layout->use({send_row, topk_idx});
     x = x.contiguous();
     const TopK tk = topk_of(topk_idx);
     TORCH_CHECK(x.is_cuda() && x.scalar_type() == torch::kBFloat16 && x.dim() == 2 && x.size(0) >= rows, "x must be a bf16 [rows, H] CUDA tensor");
@@ -624,7 +653,11 @@ py::object local_layer_call(std::shared_ptr<LocalLayer> layer, const torch::Tens
 }  // namespace
 
 void register_local(pybind11::module_& m) {
-    py::class_<Written, std::shared_ptr<Written>>(m, "Written").def("rows", &Written::rows, py::call_guard<py::gil_scoped_release>());
+    py::class_<LocalLayout, std::shared_ptr<LocalLayout>>(m, "LocalLayout")
+        .def_readonly("send_row", &LocalLayout::send_row)
+        .def("totals", [](const LocalLayout& l) { return l.scratch.narrow(0, 0, l.E + 1); })
+        .def("captured", [](const LocalLayout& l) { return l.capture != 0; })
+        .def("rows", &LocalLayout::rows, py::call_guard<py::gil_scoped_release>());
     m.def("ll_local_dispatch", &ll_local_dispatch);
     m.def("ll_local_combine", &ll_local_combine);
     py::class_<LocalLayer, std::shared_ptr<LocalLayer>>(m, "LocalLayer")

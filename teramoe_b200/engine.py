@@ -201,16 +201,26 @@ class LocalHandle:
     K: int
     E: int
     topk_idx: torch.Tensor
-    send_row: torch.Tensor       # [T] row of the token, -1 if it went nowhere
-    totals: torch.Tensor         # [E+1] on the device: entries per expert, number of rows
+    layout: object               # native (csrc/bindings_local.cpp): the tables and the stream that writes them, for which calls on others wait
     rows: int                    # number of rows, -1 while only the device knows it (fixed-shape dispatch)
-    written: object              # stream that wrote the tables (csrc/bindings_local.cpp): calls on other streams wait for it
+
+    @property
+    def send_row(self) -> torch.Tensor:
+        """[T] row of the token, -1 if it went nowhere"""
+        return self.layout.send_row
+
+    @property
+    def totals(self) -> torch.Tensor:
+        """[E+1] on the device: entries per expert, number of rows"""
+        return self.layout.totals()
 
     def num_rows(self) -> int:
-        if self.rows < 0:
-            self.rows = self.written.rows()
-        # a dispatch inside a graph has no copy for the host, and its count may change with every replay
-        return self.rows if self.rows >= 0 else int(self.totals[self.E])
+        if self.rows >= 0:
+            return self.rows
+        rows = self.layout.rows()
+        if not self.layout.captured():               # (inside a graph the count may change with every replay)
+            self.rows = rows
+        return rows
 
 
 @dataclass

@@ -38,7 +38,7 @@ class LowLatencyHandle:
     layout_range: Optional[torch.Tensor] = None   # [E_local, ranks] int64: rows << 32 | first row
     seq: int = 0                                  # call number the flags of this dispatch / its combine carry
     entry_row: Optional[torch.Tensor] = None      # one rank: [T,K] packed row of every entry (-1: none)
-    written: Optional[object] = None              # one rank: stream that wrote entry_row (csrc/bindings_local.cpp)
+    writer: int = 0                               # one rank: id of the stream that writes entry_row; a call on another one waits for it
 
 
 def _ll_geometry(N: int, rank: int, E: int, M: int, H: int, use_fp8: bool, use_ue8m0: bool, round_scale: bool, use_logfmt: bool):
@@ -250,18 +250,18 @@ class LowLatencyMixin:
         H = x.shape[1]
         self._ll_check(H, use_fp8, round_scale, use_ue8m0)
         wire = 0 if not use_fp8 else 3 if use_ue8m0 else 2 if round_scale else 1
-        (recv, scales, count, src_info, layout_range, entry_row, written), ev = self._run_local(
+        (recv, scales, count, src_info, layout_range, entry_row, writer), ev = self._run_local(
             lambda: self._world.ext.ll_local_dispatch(x, topk_idx, M, num_experts, wire, expert_stats, wait_stats), None,
             async_finish and not return_recv_hook)
         handle = LowLatencyHandle(None, M, H, num_experts, src_info=src_info, layout_range=layout_range, entry_row=entry_row,
-                                  written=written)
+                                  writer=writer)
         return ((recv, scales) if use_fp8 else recv), count, handle, ev, (_nothing if return_recv_hook else None)
 
     def _ll_combine_local(self, x, topk_idx, topk_weights, handle, use_logfmt, async_finish, return_recv_hook, out, wait_stats):
         if topk_idx.shape[0] > handle.max_tokens:
             raise ValueError(f"{topk_idx.shape[0]} tokens exceed num_max_dispatch_tokens_per_rank={handle.max_tokens}")
         res, ev = self._run_local(
-            lambda: self._world.ext.ll_local_combine(x, topk_idx, topk_weights, handle.entry_row, handle.written, handle.max_tokens,
+            lambda: self._world.ext.ll_local_combine(x, topk_idx, topk_weights, handle.entry_row, handle.writer, handle.max_tokens,
                                                      handle.num_experts, handle.hidden, use_logfmt, out, wait_stats), None, async_finish and not return_recv_hook)
         return res, ev, (_nothing if return_recv_hook else None)
 

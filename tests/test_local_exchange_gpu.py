@@ -140,6 +140,25 @@ def test_a_handle_of_the_communication_stream_is_waited_for(call):
     buf.destroy()
 
 
+@pytest.mark.parametrize("worst", [0, 1009])
+def test_a_handle_of_the_callers_stream_is_waited_for(worst):
+    """The other way round: a plain dispatch on a stalled stream, then asynchronous calls behind an event that says nothing of it."""
+    T, H, E, K = 1000, 512, 8, 4
+    idx, w = _routing(T, E, K, seed=15)
+    goes = (idx >= 0).any(1)
+    buf = tm.Buffer(None, 0, explicitly_destroy=True)
+    x = torch.randn(T, H, device="cuda").to(torch.bfloat16)
+    rows, before = x[goes].contiguous(), buf.capture()
+    torch.cuda.synchronize()
+    _stall(torch.cuda.current_stream())
+    handle = buf.deepep_dispatch(x, topk_idx=idx, topk_weights=w, num_experts=E, num_worst_tokens=worst)[4]
+    again = buf.deepep_dispatch(x, handle=handle, previous_event=before, async_finish=True)[0]
+    out = buf.deepep_combine(rows, handle, previous_event=before, async_finish=True)[0]
+    torch.cuda.synchronize()
+    assert torch.equal(again, rows) and torch.equal(out, torch.where(goes[:, None], x, torch.zeros_like(x)))
+    buf.destroy()
+
+
 @pytest.mark.parametrize("call", ["combine", "repeat", "low latency"])
 def test_the_tables_of_a_dropped_handle_outlive_the_calls_on_them(call):
     """The handle goes while the call that uses it still waits on the communication stream.  Memory of its size is asked for at once
