@@ -8,8 +8,8 @@
 // All are bound by memory traffic: every row is read once and written once.  A warp moves 2 KB of a row (four 16-byte loads in
 // flight per lane), so that a few hundred rows already fill the SMs.  Through the symmetric arena the same dispatch took a
 // push into the arena, a copy out of it, nine table copies and two waits of the host.  Measured through the API, hidden 7168,
-// top-8, 32 experts: layout + dispatch + combine + cached dispatch + combine with weights at 4096 tokens 1175 -> 99 us (77 launches
-// before), layout + FP8 dispatch + combine at 1003 tokens 718 -> 45 us.
+// top-8, 32 experts: layout + dispatch + combine + cached dispatch + combine with weights at 4096 tokens 1216 -> 99 us (77 launches
+// before), layout + FP8 dispatch + combine at 1003 tokens 736 -> 47 us.
 // The latter is host work: five allocations and four launches, and the wait for the counts, for which the host watches the pinned
 // words that the route kernel writes (an event behind it was seen a few microseconds later).
 #include "local.h"
@@ -250,6 +250,8 @@ bool make_parts(const LocalPart* parts, int n, Parts& ps) {
     return true;
 }
 
+// A block per eight segments, up to 16 blocks for each of a B200's 148 SMs; warps stride over the rest.  16384 rows of 14 KB, repeat of a dispatch:
+// 2 blocks per SM 78.6 us, 4 76.2, 8 79.0, 16 76.8, 64 71.9; combine with weights at 4096 rows: 23.1, 16.7, 16.4, 15.4, 16.5.
 int move_grid(long rows, int segs) {
     const long blocks = (rows * segs + 7) / 8;
     return (int)(blocks < 1 ? 1 : blocks > 148 * 16 ? 148 * 16 : blocks);

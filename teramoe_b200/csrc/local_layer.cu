@@ -16,14 +16,14 @@
 // instead of for every rank's completion flag, counters have GPU scope, and no host read, table copy or padding kernel is
 // left around the kernel.
 //
-// Forward + backward through the API, before (several-rank kernels, 30 to 38 launches and one host wait per step) -> after:
-//   512 tokens, H=512 I=256, 4 experts, top-2            884 ->   108 us   (was host work and launches)
-//   4096, H=2048 I=2048, 16 experts, top-8              2891 ->  2484 us
-//   8192, H=2048 I=3072, 16 experts, top-6              6158 ->  5195 us
-//   8192, H=7168 I=2048, 32 experts, top-8             16905 -> 15959 us
-//   forward only, 32 tokens of that layer                815 ->   620 us
-// Large layers are bound by the power cap: the issuer counts 5.63 M cycles for the forward at 8192 tokens, of which the tiles need 5.35 M,
-// while the clock drops to 1.24 GHz.
+// Forward + backward through the API, several-rank kernels (30 to 38 launches and one host wait per step) -> these:
+//   512 tokens, H=512 I=256, 4 experts, top-2            873 ->    99 us   (was host work and launches)
+//   4096, H=2048 I=2048, 16 experts, top-8              2914 ->  2331 us
+//   8192, H=2048 I=3072, 16 experts, top-6              6192 ->  5002 us
+//   8192, H=7168 I=2048, 32 experts, top-8             16737 -> 15088 us
+//   forward only, 32 tokens of that layer                830 ->   573 us
+// Large layers are bound by the power cap: at H=7168 a step of K of the forward takes 1042 to 1045 cycles of which the tensor cores need 1024,
+// while the clock drops to 1.1 to 1.3 GHz.
 #include "local_layer.h"
 
 #include "gemm_common.cuh"
@@ -68,7 +68,7 @@ enum { kSyncItem = 0, kSyncToken = 1, kSyncCopy = 2, kSyncKeep = 3, kSyncFirsts 
 // words of the meta block
 enum { kMetaUnits = 0, kMetaSlots = 1, kMetaWork = 2, kMetaRows = 4, kMetaWords = 8 };
 
-constexpr int kWideTiles = 74 * 4;                                        // least number of wide tiles of a GEMM
+constexpr int kWideTiles = 74 * 4;                                        // least number of wide tiles of a GEMM (local_layer_plan)
 
 constexpr int column_blocks(int n, int cols) { return (n + cols - 1) / cols; }
 
@@ -86,8 +86,9 @@ __device__ __forceinline__ int load_expert(const void* idx, int is64, long i, in
 // count: histograms of a chunk's entries over experts and of its tokens over their LAST expert; clears the counters of the layer.
 // assign: every block adds up all chunk histograms, which gives it the segment table and its own bases, so no block waits for
 // another and no scan kernel sits in between.  With few entries (kDirectEntries) every block counts all of them itself and
-// clears a share of the counters: one launch instead of two and a memset.  512 tokens, top-2: 10.0 us and two gaps -> 7.4 us; 1000,
-// top-8 is past the break-even (15.0 -> 21.7 us).
+// clears a share of the counters: one launch instead of two.  A forward call by itself, one launch / two, by entries (32 experts, top-8):
+// 512 51.3 / 53.5 us, 2048 54.6 / 55.6, 3072 57.8 / 56.8, 4096 59.8 / 59.1, 6144 66.9 / 64.2; with 4 experts, top-2, 3072 is still
+// ahead (56.1 / 56.9) and 4096 is not (60.2 / 59.1).  On the GPU alone the two are even at 2048.
 // -------------------------------------------------------------------------------------------------
 struct RouteArgs {
     LocalLayerPlan p;
@@ -548,9 +549,9 @@ struct Staging {
 
 // The pre-activation that forward keeps for backward lies in blocks of 32 rows x 8 columns, a block's 16-byte row pieces one after the
 // other: an epilogue lane holds one row of the accumulator, so the warp's 32 lanes write, and in backward read, 512 consecutive bytes per
-// instruction, straight between registers and memory.  In rows of 2 I columns the forward needed two more boxes and a second read of
-// the accumulator per tile, and the backward turned what it read in shared memory, half a box at a time, between the stores of
-// its results: 12 round trips and 21-24 thousand cycles per 256-column tile, three times what the tensor cores take at H = 2048.
+// instruction, straight between registers and memory.  In rows of 2 I columns the forward would need two more boxes and a second read of
+// the accumulator per tile, and the backward would have to turn what it reads in shared memory, half a box at a time, between the
+// stores of its results.
 __device__ __forceinline__ int4* preact_at(const LayerArgsP& L, int row0, int lane, int col) {
     return reinterpret_cast<int4*>(L.preact) + ((long)(row0 >> 5) * (L.I >> 2) + (col >> 3)) * 32 + lane;
 }
@@ -596,9 +597,9 @@ __device__ __forceinline__ void epilogue_swiglu(const LayerArgsP& L, const Stagi
 
 // First GEMM, backward: accumulator column j = d act_j.  Padding rows give zeros whatever the operands hold there: dGU and
 // act x route are operands of the weight gradients, which sum over whole 64-row blocks.  The pre-activation comes 32 columns ahead, the
-// first of it before the accumulator is ready.  16 columns are computed before the half box is waited for and written: a warp is bound by
-// the latency of its instructions (about four cycles each, two epilogue warps per scheduler), and the exponentials of 16
-// columns overlap where those of one 16-byte piece did not.  15 -> 13 thousand cycles per 256-column tile.
+// first of it before the accumulator is ready.  16 columns are computed before the half box is waited for and written, so that the
+// exponentials of 16 columns overlap: a warp is bound by the latency of its instructions (two epilogue warps per scheduler).  A
+// 256-column accumulator takes 13.3 to 13.8 thousand cycles, the forward's 3.6 to 3.9, a plain store 1.5 to 2.6 (profiles/).
 struct Preact {
     int4 v[8];      // 16-byte pieces of this lane's row: columns 8 i .. 8 i + 7 of 2 I
     __device__ __forceinline__ void request(const LayerArgsP& L, int row0, int col, int half, bool real, int lane) {
@@ -729,8 +730,9 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
         }
     }
     // With few rows per expert most rows of A are never loaded.  Zeros there cost the tensor cores least power; what an earlier kernel left in
-    // shared memory would be multiplied for the whole call (32 tokens, H=7168, back to back: 1.05 GHz and 682 us, with zeros
-    // 1.3 GHz and 580 us).
+    // shared memory would be multiplied for the whole call.  H=7168, I=2048, 32 experts, back to back behind a large call, without / with zeros:
+    // 8 rows per expert 623 / 547 us, 32 641 / 573, 64 661 / 616.  Above, an expert's rows begin to be loaded 128 at a time; zeros would
+    // still gain there (96 684 / 637, 128 702 / 662).
     if ((long)L.T * L.K <= 64l * L.E) {
         for (int i = threadIdx.x; i < L.stages * (kAStageBytes / 16); i += kThreads) {
             const int st = i / (kAStageBytes / 16);
@@ -1251,9 +1253,9 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
             uint32_t sph = 0;
             int acc = 0;
             // Tiles whose stores are not yet counted as complete (bit 31: first GEMM).  They are counted in one go when this warp would
-            // have to wait for its next item or accumulator (for more than a moment: counting takes 3 to 6 thousand cycles), or when
-            // the list is full: narrow tiles (K of a few hundred) follow each other faster than a store, a fence and an atomic complete.  Never behind such a wait: the next item may be
-            // one that waits for this count.
+            // have to wait for its next item or accumulator (for more than a moment: counting waits for the stores), or when the
+            // list is full: narrow tiles (K of a few hundred) follow each other faster than a store, a fence and an atomic complete.  Never
+            // behind such a wait: the next item may be one that waits for this count.
             uint32_t owed[kOwed];
             int n_owed = 0;
             auto flush = [&]() {
@@ -1436,7 +1438,7 @@ cudaError_t launch(const LayerArgsP& L, int num_sms, cudaStream_t stream) {
     cfg.blockDim = dim3(kThreads);
     cfg.dynamicSmemBytes = kSmemBytesP;
     cfg.stream = stream;
-    // workers wait for rows that the dispatch pairs copy and for tiles of other pairs: all of them have to be resident
+    // every pair waits for rows that warps of all blocks copy and for tiles of other pairs: all of them have to be resident
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeCooperative;
     at[0].val.cooperative = 1;
@@ -1457,9 +1459,17 @@ LocalLayerPlan local_layer_plan(int T, int K, int E, int H, int I, int keep) {
     p.units_cap = (int)((p.blocks_cap + segs) / 2);
     // Columns per tile of every GEMM [direction][kind].  The wide tile needs columns for it, enough tiles that every CTA pair gets
     // several, and a mainloop that is long against what it cannot hide: with both accumulators in one tile, the next tile
-    // starts when the first half has been read out (about a thousand cycles for a plain store, three for SwiGLU, twelve for its
-    // backward), where two 256-column tiles overlap completely.  Operand copies are what the narrow tile lacks: backward's first GEMM
-    // at H = 2048 took 950 cycles per step of K, of which the tensor cores need 512 (wide: 1200 of 1024; a layer 1.5 % faster).
+    // starts when the first half has been read out (in cycles: 2 thousand for a plain store, 3.6 for SwiGLU, 13.5 for its backward), where
+    // two 256-column tiles overlap completely.  What the narrow tile lacks is operand bandwidth.  us, wide / narrow (8192 tokens, 16
+    // experts, top-8; a forward, or a step in which only this GEMM of the backward changes):
+    //   forward's first, by H     512 399 / 455    1024 726 / 791    1536 1070 / 1137   2048 1393 / 1476   4096 2756 / 2992
+    //   forward's second, by I    256 728 / 780     512 941 / 1014   1024 1542 / 1646   2048 2823 / 2945
+    //   backward's first, by H   1024 2573 / 2512  1536 3489 / 3401  2048 4472 / 4419   3072 6426 / 6373   4096 8257 / 8284
+    //   backward's second, by 2I  512 2063 / 2077  1024 2777 / 2873  2048 4405 / 4588   4096 8361 / 8506
+    //   weight gradients, by rows per expert   512 1368 / 1346   1024 2303 / 2363   2048 4302 / 4360   4096 8370 / 8368
+    // The lines of the forward are on the safe side (wide tiles gain down to H = 512 and I = 256), backward's first is within 1.2 % either way.
+    // Number of wide tiles, H=4096 I=2048, 8 experts, top-4, forward: 128 263 / 241, 192 352 / 346, 256 431 / 439, 384 592 / 608.  The number
+    // is counted against the whole chip also where total_sms asks for less.
     const int mu_wd = (H + 2 * BM - 1) / (2 * BM), mu_wg = (2 * I + 2 * BM - 1) / (2 * BM);
     auto columns = [&](int n, long row_units, int k, int min_k) {
         return n >= 2 * BN && k >= min_k && row_units * column_blocks(n, 2 * BN) >= kWideTiles ? 2 * BN : BN;
