@@ -45,6 +45,7 @@ torch::Tensor weights_of(const torch::Tensor& w) {
     auto f = w.scalar_type() == torch::kFloat32 ? w : w.to(torch::kFloat32);
     return f.contiguous();
 }
+bool aligned16(const torch::Tensor& t) { return reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0; }
 torch::TensorOptions on(const torch::Tensor& like, torch::ScalarType t) { return torch::TensorOptions().dtype(t).device(like.device()); }
 
 // The plain form of a call runs on the caller's stream and the asynchronous one on the communication stream, so a call may use tables of a
@@ -97,6 +98,7 @@ ll_local_dispatch(torch::Tensor x, torch::Tensor topk_idx, int64_t M, int64_t E,
     topk_idx = topk_idx.contiguous();
     const TopK tk = topk_of(topk_idx);
     TORCH_CHECK(x.is_cuda() && x.scalar_type() == torch::kBFloat16 && x.dim() == 2 && x.size(0) == tk.T, "x must be a bf16 [T, hidden] CUDA tensor");
+    TORCH_CHECK(aligned16(x), "x must start on a 16-byte boundary");          // (rows are read 16 bytes at a time)
     int* stats = nullptr;
     if (expert_stats.has_value()) {
         TORCH_CHECK(expert_stats->is_cuda() && expert_stats->scalar_type() == torch::kInt32 && expert_stats->is_contiguous() &&
@@ -135,6 +137,7 @@ torch::Tensor ll_local_combine(torch::Tensor x, torch::Tensor topk_idx, torch::T
     if (!out.has_value()) out = torch::empty({tk.T, H}, on(x, torch::kBFloat16));
     TORCH_CHECK(out->is_cuda() && out->scalar_type() == torch::kBFloat16 && out->is_contiguous() && out->dim() == 2 && out->size(0) == tk.T &&
                 out->size(1) == H, "out must be a contiguous bf16 [T, hidden] CUDA tensor");
+    TORCH_CHECK(aligned16(x) && aligned16(*out), "x and out must start on a 16-byte boundary");
     TM_CHECK_CUDA(tmoe::ll_local_combine(local_layout(E, M, H, 0, logfmt), x.data_ptr(), tk.ptr, tk.is64, w.data_ptr<float>(),
                                          entry_row.data_ptr<int>(), tk.T, tk.K, (int)entry_row.size(0), (int)entry_row.size(1), out->data_ptr(),
                                          cur_stream()));
@@ -495,7 +498,7 @@ class LocalLayer : public std::enable_shared_from_this<LocalLayer> {
         p.plan = tmoe::local_layer_plan((int)T, (int)K, (int)E, (int)H, (int)I, 1);
         const int64_t rows = layer_rows(p.plan);
         TORCH_CHECK(kept.ws.numel() == p.plan.words && kept.rows.numel() == T * H + rows * 2 * I && kept.rows.device() == grad_out.device() &&
-                    kept.rows.scalar_type() == torch::kBFloat16 && kept.rows.is_contiguous() && reinterpret_cast<uintptr_t>(kept.rows.data_ptr()) % 16 == 0,
+                    kept.rows.scalar_type() == torch::kBFloat16 && kept.rows.is_contiguous() && aligned16(kept.rows),
                     "saved tensors of another call");
         // act x route [rows, I], dGU [rows, 2I], x in slot order [rows, H], partial sums of d(route weight): one allocation (rows and I, H are
         // multiples of 64: every part starts on a 16-byte boundary)

@@ -336,3 +336,26 @@ def test_a_backward_pass_of_the_layer_leaves_the_low_latency_windows_to_be_laid_
     assert torch.equal(count.long(), torch.bincount(sent[sent >= 0], minlength=E))
     buf.check_status()
     buf.destroy()
+
+
+def test_rows_off_a_16_byte_boundary():
+    """Contiguous tensors may start anywhere: the un-fused calls copy them byte by byte, the low-latency calls refuse them."""
+    T, H, E, K = 20, 256, 8, 2
+    idx, w = _routing(T, E, K, seed=16)
+    goes = (idx >= 0).any(1)
+    buf = tm.Buffer(None, 0, low_latency_mode=True, explicitly_destroy=True)
+
+    def shifted(*shape):
+        n = torch.Size(shape).numel()
+        return torch.randn(n + 1, device="cuda").to(torch.bfloat16)[1:].view(shape)
+    x, y, out = shifted(T, H), shifted(E, T, H), shifted(T, H)
+    recv, *_, handle, _ = buf.deepep_dispatch(x, topk_idx=idx, topk_weights=w, num_experts=E)
+    assert torch.equal(recv, x[goes]) and torch.equal(buf.deepep_combine(x[: recv.shape[0]], handle)[0][goes], x[: recv.shape[0]])
+    with pytest.raises(RuntimeError, match="16-byte"):
+        buf.low_latency_dispatch(x, idx, T, E, use_fp8=False)
+    low = buf.low_latency_dispatch(x.clone(), idx, T, E, use_fp8=False)[2]
+    with pytest.raises(RuntimeError, match="16-byte"):
+        buf.low_latency_combine(y, idx, w, low)
+    with pytest.raises(RuntimeError, match="16-byte"):
+        buf.low_latency_combine(y.clone(), idx, w, low, out=out)
+    buf.destroy()
