@@ -73,9 +73,10 @@ def build(verbose: bool = False) -> Path:
     cpp_extension.load(
         name=_NAME,
         sources=[str(p) for p in sources()],
-        extra_cflags=CXX_FLAGS,
-        extra_cuda_cflags=CUDA_FLAGS,
-        extra_ldflags=LD_FLAGS,
+        # copies: the linker flags are completed in place, which would change the recorded hash
+        extra_cflags=list(CXX_FLAGS),
+        extra_cuda_cflags=list(CUDA_FLAGS),
+        extra_ldflags=list(LD_FLAGS),
         extra_include_paths=[str(_CSRC)],
         build_directory=str(_EXT_DIR),
         with_cuda=True,

@@ -83,3 +83,15 @@ def test_the_native_layer_follows_the_arena():
     layer = load_ext().LocalLayer(torch.zeros(8, dtype=torch.int32), torch.zeros(4, dtype=torch.int32))
     layer.set_arena(4096, 100)
     assert layer.arena() == 4096
+
+
+def test_a_build_is_recognised_by_the_next_process(monkeypatch, tmp_path):
+    """The stamp of a build is the hash that another process computes from the same sources and flags, whatever the build does with them."""
+    from torch.utils import cpp_extension
+
+    from teramoe_b200 import _build
+    monkeypatch.setattr(_build, "_EXT_DIR", tmp_path)
+    monkeypatch.setattr(cpp_extension, "load", lambda **kw: [kw[k].append("-more") for k in ("extra_cflags", "extra_cuda_cflags", "extra_ldflags")])
+    before = _build._source_hash()
+    _build.build()
+    assert _build._stamp_path().read_text() == before == _build._source_hash()
