@@ -90,6 +90,29 @@ def test_rows_per_expert_at_the_edges_of_operand_boxes(H, I, monkeypatch):
     buf.destroy()
 
 
+@pytest.mark.parametrize("batch", [1024, 2048, 4096])
+def test_batches_end_where_experts_do(batch, monkeypatch):
+    """Experts of 9, 4, 1, 0, 2, 8, 3, 5 and 1 units of 256 rows in nominal batches of 4, 8 and 16: ends that move to an expert's, that stay inside
+    one, and a tie."""
+    from teramoe_b200 import engine
+    counts = [9 * 256 - 100, 1024, 1, 0, 500, 2048, 513, 1200, 200]
+    E, T = len(counts), sum(counts)
+    prob = make_problem(1, T, 128, 64, E, 1, seed=5, dtype=torch.bfloat16, device="cuda", x_scale=0.1, w_scale=0.02)
+    order = torch.randperm(T, generator=torch.Generator().manual_seed(2))
+    idx = torch.repeat_interleave(torch.arange(E), torch.tensor(counts))[order].view(T, 1).to(prob["ranks"][0]["idx"])
+    buf = tm.Buffer(None, int(64e6), explicitly_destroy=True)
+    res = {}
+    for mode in ("0", "auto"):
+        monkeypatch.setattr(engine, "_LOCAL_LAYER_MODE", mode)
+        for name in ("_FUSED_DISPATCH_MODE", "_FUSED_MODE", "_LAYER_KERNEL_MODE"):
+            monkeypatch.setattr(engine, name, "1" if mode == "0" else "auto")
+        res[mode] = _run(buf, prob, idx, E, compute_batch_size=batch)
+    for name, got in res["auto"].items():
+        assert torch.equal(got, res["0"][name]), f"{name}: differs from the general kernels"
+    buf.check_status()
+    buf.destroy()
+
+
 def test_native_autograd_node_keeps_its_buffer_and_fills_the_given_gradient():
     """The buffer may go out of scope before the backward pass; d(topk_weights) goes to the caller's tensor; a second derivative
     raises; a destroyed buffer raises."""
