@@ -367,9 +367,9 @@ std::tuple<torch::Tensor, c10::optional<torch::Tensor>> local_combine(torch::Ten
 // ------------------------------------------------------------------------------------------------ layer
 int64_t layer_rows(const tmoe::LocalLayerPlan& plan) { return std::max(plan.slots_cap, 128); }
 
-// bytes of the arena that a call with these sizes uses: rows in slot order and expert outputs in slot order
+// bytes of the arena that a call with these sizes uses: expert outputs in slot order
 int64_t local_layer_arena_bytes(int64_t T, int64_t K, int64_t E, int64_t H) {
-    return 2 * layer_rows(tmoe::local_layer_plan((int)T, (int)K, (int)E, (int)H, 64, 0)) * H * 2;
+    return layer_rows(tmoe::local_layer_plan((int)T, (int)K, (int)E, (int)H, 64, 0)) * H * 2;
 }
 
 void check_layer_weights(const torch::Tensor& wg, const torch::Tensor& wd, int64_t E, int64_t H, int64_t I) {
@@ -379,7 +379,7 @@ void check_layer_weights(const torch::Tensor& wg, const torch::Tensor& wd, int64
                 wd.size(1) == H && wd.size(2) == I, "W_down must be a contiguous bf16 [E, H, I] CUDA tensor");
 }
 
-// What the calls of one buffer share: the arena (rows in slot order and expert outputs), the status block and its copy in pinned
+// What the calls of one buffer share: the arena (expert outputs in slot order), the status block and its copy in pinned
 // memory, and the workspaces of the last forward and backward for whoever asks for their statistics.
 class LocalLayer : public std::enable_shared_from_this<LocalLayer> {
   public:
@@ -500,13 +500,12 @@ class LocalLayer : public std::enable_shared_from_this<LocalLayer> {
         TORCH_CHECK(kept.ws.numel() == p.plan.words && kept.rows.numel() == T * H + rows * 2 * I && kept.rows.device() == grad_out.device() &&
                     kept.rows.scalar_type() == torch::kBFloat16 && kept.rows.is_contiguous() && aligned16(kept.rows),
                     "saved tensors of another call");
-        // act x route [rows, I], dGU [rows, 2I], x in slot order [rows, H], partial sums of d(route weight): one allocation (rows and I, H are
-        // multiples of 64: every part starts on a 16-byte boundary)
-        auto scratch = torch::empty({rows * (3 * I + H + 4 * ((I + 255) / 256))}, grad_out.options());
+        // act x route [rows, I], dGU [rows, 2I], partial sums of d(route weight): one allocation (rows and I are multiples of 64: every part
+        // starts on a 16-byte boundary)
+        auto scratch = torch::empty({rows * (3 * I + 4 * ((I + 255) / 256))}, grad_out.options());
         auto* act_w = scratch.data_ptr<at::BFloat16>();
         auto* dgu = act_w + rows * I;
-        auto* xperm = dgu + rows * 2 * I;
-        auto* parts = xperm + rows * H;
+        auto* parts = dgu + rows * 2 * I;
         auto dx = torch::empty({T, H}, grad_out.options());
         auto dw = torch::empty({T, K}, on(grad_out, torch::kFloat32));
         auto dwg = torch::empty({E, 2 * I, H}, grad_out.options());
@@ -515,7 +514,7 @@ class LocalLayer : public std::enable_shared_from_this<LocalLayer> {
         p.bwd = 1;
         p.x = grad_out.data_ptr(); p.w_gateup = w_gateup.data_ptr(); p.w_down = w_down.data_ptr();
         p.act = act_w; p.aux = dgu; p.saved_x = kept.rows.data_ptr(); p.out = dx.data_ptr();
-        p.preact = kept.rows.data_ptr<at::BFloat16>() + T * H; p.droute_part = reinterpret_cast<float*>(parts); p.xperm = xperm;
+        p.preact = kept.rows.data_ptr<at::BFloat16>() + T * H; p.droute_part = reinterpret_cast<float*>(parts);
         p.dw_topk = dw.data_ptr<float>(); p.dw_gateup = dwg.data_ptr(); p.dw_down = dwd.data_ptr();
         {
             std::lock_guard<std::mutex> lock(arena_mutex_);
@@ -536,11 +535,10 @@ class LocalLayer : public std::enable_shared_from_this<LocalLayer> {
   private:
     // (with arena_mutex_ held, until the launch)
     void set_common(tmoe::LocalLayerParams& p, const Schedule& s) {
-        const int64_t rows = layer_rows(p.plan), half = rows * p.plan.H * 2;
-        TORCH_CHECK(2 * half <= arena_bytes_, "the arena is too small for this call");
+        const int64_t rows = layer_rows(p.plan);
+        TORCH_CHECK(rows * p.plan.H * 2 <= arena_bytes_, "the arena is too small for this call");
         p.out_rows = (int)rows;
-        p.slot_x = reinterpret_cast<void*>(arena_);
-        p.y = reinterpret_cast<void*>(arena_ + half);
+        p.y = reinterpret_cast<void*>(arena_);
         p.group_units = (int)s[0]; p.lag_percent = (int)s[1]; p.min_lag_items = (int)s[2];
         p.num_sms = (int)s[3];
         p.status = status_.data_ptr<int>();

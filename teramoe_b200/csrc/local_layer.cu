@@ -1,17 +1,17 @@
-// The MoE layer on one rank, see local_layer.h.  Roles of the persistent kernel (74 CTA pairs, 12 warps per CTA):
+// The MoE layer on one rank, see local_layer.h.  Roles of the persistent kernel (74 CTA pairs, 16 warps per CTA):
 //
-//   copy       every warp but the next two first copies a routed row into slot order; the gather warps copy the rest
 //   producer   claims items of the work list, hands them to the pair, loads operand tiles by TMA
 //   issuer     tcgen05 cta_group::2, 256x256 or 256x512 tiles, two accumulators in tensor memory
+//   loaders    4 warps: bring the operands that are made of token rows from the caller's tensor (load_rows)
 //   epilogue   8 warps: SwiGLU / dSwiGLU / store.  A warp packs 32 rows x 64 columns into shared memory (128-byte swizzle) and
 //              hands them to one TMA store; the pre-activation goes straight between registers and memory (preact_at).
-//   gather     warps 2 and 3, joined by the epilogue warps at the end of the list: keep a copy of x (forward), rebuild x in slot
-//              order (backward), and sum every token's expert rows as soon as the units that hold them are finished.
+//   gather     warps 2 and 3, joined by the epilogue warps at the end of the list: keep a copy of x (forward), and sum every
+//              token's expert rows as soon as the units that hold them are finished.
 //              Tokens are visited in the order of their last expert, which is the order in which they become ready.
 //
 // The work list, the k steps and the order of every sum are those of layer.cu, except that a weight gradient's tiles are listed along
 // a row of the result: the tiles in flight at a time then write whole rows (7 % faster where the stores bound it, 57 rows per expert).
-// What is different because there is one rank: rows are copied by slot instead of pushed by entry, expert rows stay in slot
+// What is different because there is one rank: token rows are loaded by slot instead of pushed by entry, expert rows stay in slot
 // order (one TMA box per 32 rows instead of 32 bulk copies to landing rows), the sum of a token waits for its own units
 // instead of for every rank's completion flag, counters have GPU scope, and no host read, table copy or padding kernel is
 // left around the kernel.
@@ -25,6 +25,8 @@
 // Large layers are bound by the power cap: at H=7168 a step of K of the forward takes 1042 to 1045 cycles of which the tensor cores need 1024,
 // while the clock drops to 1.1 to 1.3 GHz.
 #include "local_layer.h"
+
+#include <type_traits>
 
 #include "gemm_common.cuh"
 #include "launch_count.h"
@@ -51,22 +53,26 @@ constexpr int kBoxBytes = 32 * 128;                                       // 32 
 constexpr int kEpiBytes = kEpiWarps * kBoxBytes;                          // 32 KB: one box per epilogue warp
 constexpr int kBarOffsetP = kPipeBytesP + kEpiBytes;
 constexpr int kSmemBytesP = kBarOffsetP + 512 + 1024;
-constexpr int kCopyRows = 8;                                              // slots a gather warp claims at a time (divides a block)
-constexpr int kFirstRows = 1;                                             // slots every warp copies before anything else
-constexpr int kCopyWarps = kThreads / 32 - 2;                             // warps of a CTA that copy at the start
+constexpr int kKeepRows = 8;                                              // rows of x a gather warp claims at a time
+constexpr int kGatherWarps = 2 + kEpiWarps;                               // warps of a CTA that sum in the end
+constexpr int kLoadWarps = 4;
+constexpr int kLayerThreads = kThreads + 32 * kLoadWarps;
+// Registers per thread: 128 at launch (512 threads), then by warpgroup
+constexpr int kRegsControl = 120, kRegsEpilogue = 168, kRegsLoad = 56;
+static_assert(128 * kRegsControl + 256 * kRegsEpilogue + 128 * kRegsLoad <= 65536 && kThreads == 384 && kLayerThreads == 512, "register file");
 constexpr int kRingDepth = 4;
 constexpr int kSoon = 32;                                                 // looks at a barrier before its wait counts as one
 constexpr int kOwed = 4;                                                  // finished tiles an epilogue warp counts at once
 constexpr int kGatherTasks = 16384;                                       // least number of (token, columns) tasks of the gather role
-constexpr uint32_t kOffTmem = 496, kOffRingFull = 320, kOffRingEmpty = 352, kOffItems = 384;
-constexpr uint32_t kRingConsumers = 2 * kEpiWarps + 2;
-static_assert(8 * (2 * kMaxStages + 4) <= (int)kOffRingFull && kOffItems + 16 * kRingDepth <= kOffTmem && kOffTmem + 8 <= 512, "barrier block");
+constexpr uint32_t kOffTmem = 496, kOffRows = 192, kOffRingFull = 320, kOffRingEmpty = 352, kOffItems = 384;
+constexpr uint32_t kRingConsumers = 2 * (kEpiWarps + kLoadWarps) + 2;
+static_assert(8 * (2 * kMaxStages + 4) <= (int)kOffRows && kOffRows + 8 * kMaxStages <= kOffRingFull && kOffItems + 16 * kRingDepth <= kOffTmem && kOffTmem + 8 <= 512, "barrier block");
 static_assert(kSmemBytesP <= 232448, "shared memory");
 
 // words of the sync block
-enum { kSyncItem = 0, kSyncToken = 1, kSyncCopy = 2, kSyncKeep = 3, kSyncFirsts = 4, kSyncRows = 5, kSyncWords = 8 };
+enum { kSyncItem = 0, kSyncToken = 1, kSyncKeep = 2, kSyncFirsts = 3, kSyncWords = 8 };
 // words of the meta block
-enum { kMetaUnits = 0, kMetaSlots = 1, kMetaWork = 2, kMetaRows = 4, kMetaWords = 8 };
+enum { kMetaUnits = 0, kMetaWork = 2, kMetaWords = 8 };
 
 constexpr int kWideTiles = 74 * 4;                                        // least number of wide tiles of a GEMM (local_layer_plan)
 
@@ -193,7 +199,7 @@ __global__ void __launch_bounds__(kRouteThreads) local_route_assign_kernel(const
     }
     __syncthreads();
     if (warp == 0) {
-        int run_s = 0, run_u = 0, run_r = 0;
+        int run_s = 0, run_u = 0;
         for (int e0 = 0; e0 < E; e0 += 32) {
             const int e = e0 + lane;
             const int blocks = e < E ? (totals[e] + 127) / 128 : 0;
@@ -212,9 +218,7 @@ __global__ void __launch_bounds__(kRouteThreads) local_route_assign_kernel(const
             }
             run_s += __shfl_sync(0xffffffffu, s, 31);
             run_u += __shfl_sync(0xffffffffu, u, 31);
-            run_r += __reduce_add_sync(0xffffffffu, e < E ? (totals[e] + BK - 1) / BK * BK : 0);
         }
-        if (blockIdx.x == 0 && lane == 0) a.ws[a.p.meta + kMetaRows] = run_r;      // rows of whole 64-row steps
         if (lane == 0) {
             seg[E] = run_s;
             ub[E] = run_u;
@@ -235,7 +239,7 @@ __global__ void __launch_bounds__(kRouteThreads) local_route_assign_kernel(const
     }
     for (int i = tid; i < kRouteWarps * (2 * E + 1); i += kRouteThreads) cnt[i] = 0;
     __syncthreads();
-    const int U = ub[E], S = seg[E];
+    const int U = ub[E];
     const int gtid = blockIdx.x * kRouteThreads + tid, gthreads = gridDim.x * kRouteThreads;
     // ---- tables
     int* meta = a.ws + a.p.meta;
@@ -243,10 +247,7 @@ __global__ void __launch_bounds__(kRouteThreads) local_route_assign_kernel(const
     float* slot_w = reinterpret_cast<float*>(a.ws + a.p.slot_w);
     if (blockIdx.x == 0) {
         for (int e = tid; e <= E; e += kRouteThreads) a.ws[a.p.seg + e] = seg[e];
-        if (tid == 0) {
-            meta[kMetaUnits] = U;
-            meta[kMetaSlots] = S;
-        }
+        if (tid == 0) meta[kMetaUnits] = U;
     }
     for (int e = blockIdx.x; e < E; e += gridDim.x)
         for (int s = seg[e] + totals[e] + tid; s < seg[e + 1]; s += kRouteThreads) {
@@ -372,7 +373,7 @@ __global__ void __launch_bounds__(kRouteThreads) local_route_assign_kernel(const
 struct Phase {
     alignas(64) CUtensorMap map_a;
     alignas(64) CUtensorMap map_b;
-    alignas(64) CUtensorMap map_a32;     // the two GEMMs: 32 rows of A
+    alignas(64) CUtensorMap map_a32;     // second GEMM: 32 rows of A
     int nk, b_group_rows, cols, num_n_blocks, n_total, m_total;      // num_n_blocks: of the two GEMMs
 };
 
@@ -385,11 +386,9 @@ struct LayerArgsP {
     alignas(64) CUtensorMap st_dwg;
     int T, K, H, I, E;
     int stages, stage_bytes, keep;
-    const uint8_t* x;
-    uint8_t* slot_x;
+    const uint8_t* x;                    // [T, H]: forward x, backward grad_out
     const __nv_bfloat16* y;
-    __nv_bfloat16* saved_x;
-    __nv_bfloat16* xperm;
+    __nv_bfloat16* saved_x;              // [T, H]: written by forward (may be null), read by backward
     __nv_bfloat16* out;
     __nv_bfloat16* preact;               // forward (with keep): written, backward: read; preact_at()
     float* droute_part;
@@ -405,7 +404,6 @@ struct LayerArgsP {
     int* sync;
     int* done1;                          // per unit: epilogue warps that finished a tile of the first GEMM
     int* done2;                          // per 128-row block: the same for the second GEMM
-    int* arrived;                        // per 128-row block: rows in place
     unsigned long long* stats;
     int* status;
 };
@@ -449,16 +447,21 @@ __device__ __forceinline__ bool wait_count(const int* flag, int target, int* sta
     }
 }
 
-// Warp-wide row copy with 16 loads in flight per lane (8 KB per warp): two warps per SM have to keep HBM busy.
-__device__ __forceinline__ void copy_row_deep(int4* dst, const int4* src, int nvec, int lane) {
-    for (int b = 0; b < nvec; b += 512) {
-        int4 v[16];
-#pragma unroll
-        for (int i = 0; i < 16; ++i) v[i] = ld_nc_v4(src + min(b + 32 * i + lane, nvec - 1));
-#pragma unroll
-        for (int i = 0; i < 16; ++i)
-            if (b + 32 * i + lane < nvec) dst[b + 32 * i + lane] = v[i];
-    }
+// 16 bytes from memory into shared memory, or zeros
+__device__ __forceinline__ void cp_async_16(uint32_t dst_smem, const void* src) {
+    asm volatile("cp.async.cg.shared.global.L2::256B [%0], [%1], 16;" ::"r"(dst_smem), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_16_or_zeros(uint32_t dst_smem, const void* src, bool wanted) {
+    asm volatile("cp.async.cg.shared.global.L2::256B [%0], [%1], 16, %2;" ::"r"(dst_smem), "l"(src), "r"(wanted ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+template <int R>
+__device__ __forceinline__ void registers_inc() {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(R));
+}
+template <int R>
+__device__ __forceinline__ void registers_dec() {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(R));
 }
 
 struct Item {
@@ -694,7 +697,7 @@ __device__ __forceinline__ void epilogue_plain(const Staging& st, uint32_t taddr
 }
 
 template <bool BWD>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kLayerThreads, 1)
 local_layer_kernel(const __grid_constant__ LayerArgsP L) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -706,6 +709,7 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
     auto tempty_bar = [&](int s) { return bar_base + 8u * (2 * kMaxStages + 2 + s); };
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + kBarOffsetP + kOffTmem);
     volatile uint32_t* abort_flag = tmem_slot + 1;
+    auto rows_bar = [&](int s) { return bar_base + kOffRows + 8u * s; };
     auto ring_full = [&](int e) { return bar_base + kOffRingFull + 8u * e; };
     auto ring_empty = [&](int e) { return bar_base + kOffRingEmpty + 8u * e; };
 
@@ -718,6 +722,7 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
         for (int s = 0; s < kMaxStages; ++s) {
             mbar_init(full_bar(s), 2);
             mbar_init(empty_bar(s), 1);
+            mbar_init(rows_bar(s), 2);
         }
         for (int s = 0; s < 2; ++s) {
             mbar_init(tfull_bar(s), 1);
@@ -730,8 +735,8 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
         fence_mbar_init();
 #pragma unroll
         for (int p = 0; p < (BWD ? 4 : 2); ++p) {
-            tma_prefetch_desc(&L.ph[p].map_a);
-            tma_prefetch_desc(&L.ph[p].map_b);
+            if (p != kWorkGemm1 && p != kWorkWgradDown) tma_prefetch_desc(&L.ph[p].map_a);
+            if (p != kWorkWgradGateup) tma_prefetch_desc(&L.ph[p].map_b);
         }
     }
     // With few rows per expert most rows of A are never loaded.  Zeros there cost the tensor cores least power; what an earlier kernel left in
@@ -739,7 +744,7 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
     // 8 rows per expert 623 / 547 us, 32 641 / 573, 64 661 / 616.  Above, an expert's rows begin to be loaded 128 at a time; zeros would
     // still gain there (96 684 / 637, 128 702 / 662).
     if ((long)L.T * L.K <= 64l * L.E) {
-        for (int i = threadIdx.x; i < L.stages * (kAStageBytes / 16); i += kThreads) {
+        for (int i = threadIdx.x; i < L.stages * (kAStageBytes / 16); i += kLayerThreads) {
             const int st = i / (kAStageBytes / 16);
             *reinterpret_cast<int4*>(smem_gen + st * L.stage_bytes + (i - st * (kAStageBytes / 16)) * 16) = make_int4(0, 0, 0, 0);
         }
@@ -751,106 +756,29 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
     tcgen05_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 
-    const int num_slots = L.meta[kMetaSlots];
     const int target1 = 2 * kEpiWarps * L.ph[0].num_n_blocks;         // epilogue warps that finish a unit's first GEMM,
     const int target2 = kEpiWarps * L.ph[1].num_n_blocks;             // a block's second GEMM
 
-    // ---------------------------------------------------------------------- copy role
-    // Rows into slot order.  All warps but the producer's and the issuer's start with one slot each, so that the first units are in place
-    // after the latency of one row; the rest is claimed by the gather warps, eight slots at a time.  A warp has 8 KB of loads in
-    // flight: rows of 4096 columns and more one after the other, shorter ones several at once.  (Before, the first pairs of CTAs
-    // streamed rows through shared memory and joined the GEMMs afterwards; rows of 1 KB left them waiting for one row at a time:
-    // 8531 tokens, H=512, top-8 spent 240 us there.)
+    // ---------------------------------------------------------------------- backward's copy of x
     const int nvec = L.H / 8;
-    auto copy_slots = [&](const int4* src, int4* dst, int row, uint32_t wanted, int s0, int n) {
-        // row: source row of slot s0 + lane, -1 = zeros
-        if (nvec >= 512) {
-            for (int r = 0; r < n; ++r) {
-                if (!((wanted >> r) & 1u)) continue;
-                const int sr = __shfl_sync(0xffffffffu, row, r);
-                int4* d = dst + (long)(s0 + r) * nvec;
-                if (sr >= 0) copy_row_deep(d, src + (long)sr * nvec, nvec, lane);
-                else for (int i = lane; i < nvec; i += 32) d[i] = make_int4(0, 0, 0, 0);
-            }
-            return;
-        }
-        const int total = n * nvec;
-        for (int b = 0; b < total; b += 512) {
-            int4 v[16];
-#pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                const int idx = min(b + 32 * i + lane, total - 1), r = idx / nvec;
-                const int sr = __shfl_sync(0xffffffffu, row, r);
-                v[i] = ld_nc_v4(src + (long)max(sr, 0) * nvec + (idx - r * nvec));
-                if (sr < 0) v[i] = make_int4(0, 0, 0, 0);
-            }
-#pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                const int idx = b + 32 * i + lane;
-                if (idx < total && ((wanted >> (idx / nvec)) & 1u)) dst[(long)s0 * nvec + idx] = v[i];
-            }
-        }
-    };
-    auto count_rows = [&](int* counter, int n) {
-        __syncwarp();
-        if (lane == 0 && n > 0) {
-            fence_acq_rel_gpu();
-            red_add_gpu(counter, n);
-        }
-    };
-    auto place = [&](int s0, int n) {
-        const int tk = lane < n ? L.slot_tk[s0 + lane] : -1;
-        const int row = tk >= 0 ? tk / L.K : -1;
-        uint32_t wanted = __ballot_sync(0xffffffffu, tk >= 0);
-        if constexpr (BWD) {
-            // both slot-order tables are operands of the weight gradients, which sum over 64 rows at a time: rows of zeros to the next 64
-            wanted = L.slot_tk[s0 & ~63] >= 0 ? (1u << n) - 1u : 0u;
-        }
-        if (wanted == 0u) return;
-        copy_slots(reinterpret_cast<const int4*>(L.x), reinterpret_cast<int4*>(L.slot_x), row, wanted, s0, n);
-        count_rows(L.arrived + (s0 >> 7), __popc(wanted));
-    };
-    auto place_x = [&](int s0, int n) {
-        const int tk = lane < n ? L.slot_tk[s0 + lane] : -1;
-        if (L.slot_tk[s0 & ~63] < 0) return;
-        copy_slots(reinterpret_cast<const int4*>(L.saved_x), reinterpret_cast<int4*>(L.xperm), tk >= 0 ? tk / L.K : -1, (1u << n) - 1u, s0, n);
-        count_rows(L.sync + kSyncRows, n);
-    };
-    // (neighbouring slots go to different SMs: a few rows in one SM would queue behind one another)
-    const int first_slots = (int)gridDim.x * kCopyWarps * kFirstRows / kCopyRows * kCopyRows;
-    if (warp >= 2) {
-        const int s0 = ((warp - 2) * (int)gridDim.x + (int)blockIdx.x) * kFirstRows;
-        if (s0 < min(num_slots, first_slots)) place(s0, kFirstRows);
-    }
-    auto copy_loop = [&]() {
-        while (true) {
-            int s0 = 0;
-            if (lane == 0) s0 = first_slots + atomicAdd(L.sync + kSyncCopy, kCopyRows);
-            s0 = __shfl_sync(0xffffffffu, s0, 0);
-            if (s0 >= num_slots) break;
-            place(s0, kCopyRows);
-        }
-    };
-    auto copy_x_loop = [&]() {
-        // backward: x in slot order, which nothing needs before the weight gradients
-        while (true) {
-            int s0 = 0;
-            if (lane == 0) s0 = atomicAdd(L.sync + kSyncKeep, kCopyRows);
-            s0 = __shfl_sync(0xffffffffu, s0, 0);
-            if (s0 >= num_slots) break;
-            place_x(s0, kCopyRows);
-        }
-    };
     auto keep_x_loop = [&]() {
-        // forward: backward's copy of x
-        const int chunk = kCopyRows;
+        // 4 KB of loads in flight per warp
         while (true) {
             int t0 = 0;
-            if (lane == 0) t0 = atomicAdd(L.sync + kSyncKeep, chunk);
+            if (lane == 0) t0 = atomicAdd(L.sync + kSyncKeep, kKeepRows);
             t0 = __shfl_sync(0xffffffffu, t0, 0);
             if (t0 >= L.T) break;
-            const int n = min(chunk, L.T - t0);
-            copy_slots(reinterpret_cast<const int4*>(L.x), reinterpret_cast<int4*>(L.saved_x), t0 + min(lane, n - 1), (1u << n) - 1u, t0, n);
+            const long first = (long)t0 * nvec, total = (long)min(kKeepRows, L.T - t0) * nvec;
+            const int4* src = reinterpret_cast<const int4*>(L.x) + first;
+            int4* dst = reinterpret_cast<int4*>(L.saved_x) + first;
+            for (long b = lane; b < total; b += 256) {
+                int4 v[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) v[i] = ld_nc_v4(src + min(b + 32 * i, total - 1));
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    if (b + 32 * i < total) dst[b + 32 * i] = v[i];
+            }
         }
     };
 
@@ -900,9 +828,9 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
         int next_i = tasks, next_t = 0, next_slot = -1;
         // Few tasks are dealt out to all warps that gather in the end: they become ready together, and an atomic per task would be
         // half of what is left to do by then.
-        const int warps = (int)gridDim.x * kCopyWarps;
+        const int warps = (int)gridDim.x * kGatherWarps;
         const bool dealt = !BWD && tasks <= 4 * warps;           // (backward they run under the weight gradients)
-        next_i = dealt ? (int)blockIdx.x * kCopyWarps + (warp - 2) - warps : 0;
+        next_i = dealt ? (int)blockIdx.x * kGatherWarps + (warp - 2) - warps : 0;
         auto claim = [&]() {
             if (dealt) {
                 next_i += warps;
@@ -995,6 +923,108 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
             return true;
         };
 
+        // -------------------------------------------------------------- token rows
+        // Operands that are made of token rows come straight from the caller's [T, H] tensor, row by row of the slot table: A of the first GEMM
+        // (128 rows x 64 columns of K per step), A of dW_down and B of dW_gateup (64 rows of K x 128 or more columns).  Four warps of each CTA
+        // copy them, eight lanes to 128 bytes, in the layout that TMA gives the other operands.  Before, other warps copied every
+        // row into slot order first, and TMA loaded it from there: K times the tensor written and read once more (0.94 GB of each per
+        // copy and three copies in a step of 8192 tokens, H=7168, top-8).  TMA's own row gather moves 512 bytes in 70 cycles, a third of what
+        // a mainloop needs.  Forward + backward, ms: 16384 tokens, H=7168 I=512, top-8 9.55 -> 8.77 (backward's first GEMM no longer waits
+        // for rows: 2283 -> 1280 cycles per step); 4096, H=2048 I=2048, top-8 2.342 -> 2.299; 8192, H=7168 I=2048 14.93 -> 14.92;
+        // forward of 3001 tokens 1.897 -> 1.871, of 32 tokens 0.582 -> 0.592.  (With TMA loads of as many consecutive rows instead the
+        // large forward would take 3 % less: what these copies cost.)
+        //
+        // A warp takes every fourth step: it waits for the stage, copies, sees its copies through and hands the step over, so that four
+        // steps' copies are under way at a time.  All four warps on every step, two steps under way, were 4 % slower; an address
+        // computed per column block instead of per row made dW_gateup 25 % slower.
+        auto load_rows = [&]() {
+            const int sub = lane >> 3, chunk = lane & 7;
+            const uint32_t pair_rows = mapa_shared(rows_bar(0), 0);
+            const uint32_t at[2] = {(uint32_t)(sub * 128 + ((chunk ^ sub) << 4)), (uint32_t)(sub * 128 + ((chunk ^ (sub + 4)) << 4))};      // rows 8i + sub, 8i + 4 + sub
+            const uint64_t inverse = ~0ull / (uint32_t)L.K;   // entry / K = (entry + 1) * floor((2^64 - 1) / K) / 2^64, exact for 32-bit entries
+            auto token = [&](int tk) { return tk < 0 ? -1 : (int)__umul64hi((uint64_t)(uint32_t)tk + 1u, inverse); };
+            const long pitch = L.H * 2l;
+            int step = warp - 12, stage = step, ss = 0;      // this warp's next step, counted from the start of the item; its stage
+            uint32_t phase = 0, sph = 0;
+            while (true) {
+                int4 it;
+                if (!next_item(ss, sph, 654, it) || it.x < 0) break;
+                Item q;
+                decode_item(L, it, rank, q);
+                int row[4] = {-1, -1, -1, -1};               // first GEMM: tokens of rows lane + 32 i; gradients: entries of K rows lane + 32 i of this step
+                const bool down = q.kind == kWorkWgradDown;
+                if (q.kind == kWorkGemm1) {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const int r = lane + 32 * i;
+                        if (r >= q.real) continue;
+                        row[i] = token(L.slot_tk[q.m0 + r]);
+                        // a table that says less than the list: a row that never arrives
+                        if (row[i] < 0) report_status(L.status, kStatusFlagTimeout, 600, q.m0 + r);
+                    }
+                } else if (BWD && q.kind != kWorkGemm2) {
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) row[i] = step < q.nk ? L.slot_tk[q.k0 + step * BK + lane + 32 * i] : -1;
+                }
+                bool ok = true;
+                for (; step < q.nk; step += kLoadWarps) {
+                    // (a step of the second GEMM is waited for as well: a phase is told from the next but one by its parity alone)
+                    if (!(ok = mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag, L.status, 611))) break;
+                    const uint32_t dst = smem_base + (uint32_t)(stage * L.stage_bytes);
+                    if (q.kind == kWorkGemm1) {
+                        const uint8_t* src = L.x + step * 128 + 16 * chunk;
+                        // (unrolled, with no branch between them, the loads follow each other; a loop that ends with the rows is a third slower)
+                        auto copy = [&](auto quads) {
+#pragma unroll
+                            for (int j = 0; j < decltype(quads)::value; ++j) {
+                                const int t = __shfl_sync(0xffffffffu, row[j >> 3], (4 * j + sub) & 31);
+                                if (t >= 0) cp_async_16(dst + j * 512 + at[j & 1], src + t * pitch);
+                            }
+                        };
+                        if (q.real > 32) copy(std::integral_constant<int, 32>());
+                        else copy(std::integral_constant<int, 8>());
+                    } else if (BWD && q.kind != kWorkGemm2) {
+                        const uint8_t* src = (down ? L.x : reinterpret_cast<const uint8_t*>(L.saved_x)) + 16 * chunk;
+                        const int tok[2] = {token(row[0]), token(row[1])};
+#pragma unroll
+                        for (int i = 0; i < 2; ++i)
+                            row[i] = step + kLoadWarps < q.nk ? L.slot_tk[q.k0 + (step + kLoadWarps) * BK + lane + 32 * i] : -1;
+                        // (columns past the last are not loaded: they are rows or columns of the result that are not stored)
+                        const int c0 = down ? q.m0 : q.n0 + (int)rank * (BN / 2);
+                        auto copy = [&](auto atoms) {
+#pragma unroll
+                            for (int j = 0; j < 16; ++j) {
+                                const int t = __shfl_sync(0xffffffffu, tok[j >> 3], (4 * j + sub) & 31);
+                                const uint8_t* from = src + max(t, 0) * pitch + c0 * 2;
+                                const uint32_t to = dst + (down ? 0 : kAStageBytes) + j * 512 + at[j & 1];
+#pragma unroll
+                                for (int a = 0; a < decltype(atoms)::value; ++a)
+                                    if (c0 + (a >> 1) * BN + (a & 1) * 64 < L.H)
+                                        cp_async_16_or_zeros(to + a * kAtomBytes, from + ((a >> 1) * BN + (a & 1) * 64) * 2, t >= 0);
+                            }
+                        };
+                        if (down || q.halves == 1) copy(std::integral_constant<int, 2>());
+                        else copy(std::integral_constant<int, 4>());
+                    }
+                    if (q.kind != kWorkGemm2) {
+                        cp_async_wait_all();
+                        fence_proxy_async_smem();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive_cluster(pair_rows + 8u * stage);
+                    }
+                    stage += kLoadWarps;
+                    if (stage >= L.stages) { stage -= L.stages; phase ^= 1u; }
+                }
+                if (!ok) break;
+                step -= q.nk;
+            }
+        };
+
+        if (warp >= 12) {
+            registers_dec<kRegsLoad>();
+            load_rows();
+        } else if (warp < 4) {
+        registers_dec<kRegsControl>();
         if (warp == 0) {
             // -------------------------------------------------------------- item fetch (first CTA) + TMA producer
             if (elect_one()) {
@@ -1009,7 +1039,7 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                 // Both producers look at the NEXT item while the loads of the current one are in flight: they fetch it and test what
                 // its operands wait for, so that between two items there is normally nothing to wait for.
                 int claim = (rank == 0) ? atomicAdd(L.sync + kSyncItem, 1) : 0;
-                unsigned long long w_arrive = 0, w_unit = 0, w_wgrad = 0;
+                unsigned long long w_unit = 0, w_wgrad = 0;
                 bool wgrad_ready = false, wgrad_fenced = false;
                 int4 cur = make_int4(-1, 0, 0, 0), nxt = cur;
                 bool have = false, nxt_ready = false;
@@ -1046,15 +1076,14 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                 };
                 // what the operands of an item wait for; `block`: wait (bounded) instead of only looking
                 auto operands_ready = [&](const Item& q, bool block) -> int {
-                    if (q.kind == kWorkGemm1) return (!q.live || q.need == 0) ? 1 : counted(L.arrived + q.m0 / BM, q.need, block, 600, w_arrive);
+                    if (q.kind == kWorkGemm1) return 1;
                     if (q.kind == kWorkGemm2) return counted(L.done1 + q.unit, target1, block, 601, w_unit);
                     // the weight gradients sit behind all first GEMMs in the list: one check per pair is enough (two loads per expert and pair
                     // would cost as much as the smallest of these items)
                     if (wgrad_ready) return 1;
-                    const int a = counted(L.sync + kSyncRows, L.meta[kMetaRows], block, 603, w_wgrad);
-                    const int b = a == 1 ? counted(L.sync + kSyncFirsts, L.meta[kMetaUnits] * target1, block, 602, w_wgrad) : a;
-                    wgrad_ready = b == 1;
-                    return b;
+                    const int r = counted(L.sync + kSyncFirsts, L.meta[kMetaUnits] * target1, block, 602, w_wgrad);
+                    wgrad_ready = r == 1;
+                    return r;
                 };
                 auto look_ahead = [&]() -> bool {            // false: a wait ran out
                     const int r = get_item(nxt, false);
@@ -1085,11 +1114,13 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                     const Phase& P = L.ph[q.kind];
                     const bool gemm = q.kind <= kWorkGemm2;
                     const int n0 = q.n0 + (int)rank * (BN / 2);
-                    // Rows of A that a CTA loads: none that nothing is summed from, up to 64 in boxes of 32.  What a stage holds in the others
-                    // is multiplied into accumulator rows that no epilogue reads.
-                    const int a_rows = gemm ? rows_loaded(q.need) : BM;
-                    const int a_pair = gemm ? rows_loaded((cur.z >> 16) & 0xff) + rows_loaded((cur.z >> 24) & 0xff) : 2 * BM;
-                    const uint32_t tx = (uint32_t)(a_pair * (BK * 2) + 2 * q.halves * kBHalfBytesP);
+                    // Second GEMM, rows of A that a CTA loads: none that nothing is summed from, up to 64 in boxes of 32.  What a stage holds in
+                    // the others is multiplied into accumulator rows that no epilogue reads.  What is made of token rows comes from the
+                    // loading warps: A of the first GEMM and of dW_down, B of dW_gateup.
+                    const int a_rows = rows_loaded(q.need);
+                    const int a_pair = q.kind == kWorkGemm2 ? rows_loaded((cur.z >> 16) & 0xff) + rows_loaded((cur.z >> 24) & 0xff)
+                                                            : (q.kind == kWorkWgradGateup ? 2 * BM : 0);
+                    const uint32_t tx = (uint32_t)(a_pair * (BK * 2) + (q.kind == kWorkWgradGateup ? 0 : 2 * q.halves * kBHalfBytesP));
                     const int look_kb = min(stages - 1, q.nk - 1);     // all stages are in flight: a pause of this thread costs nothing
                     auto take_stage = [&](int st, uint32_t ph) {
                         if (!mbar_wait(empty_bar(st), ph ^ 1u, abort_flag, L.status, 610)) return false;
@@ -1100,14 +1131,14 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                     const CUtensorMap* map_b = &P.map_b;
                     const int b_row = q.group * P.b_group_rows;
                     auto load_b = [&](int st, int k) {
+                        if (q.kind == kWorkWgradGateup) return;
                         const uint32_t dst = smem_base + (uint32_t)st * stage_bytes + kAStageBytes, bar = pair_full + 8u * st;
                         for (int h = 0; h < q.halves; ++h) {
                             if (!BWD) tma_load_2d_2cta(dst + h * kBHalfBytesP, map_b, bar, k, b_row + n0 + h * BN);
                             else tma_load_3d_2cta(dst + h * kBHalfBytesP, map_b, bar, 0, b_row + k, (n0 + h * BN) >> 6);
                         }
                     };
-                    // What a GEMM waits for is its rows; the weights of its first steps come meanwhile (the first items of a call would else
-                    // wait for memory twice, one after the other).
+                    // What a GEMM waits for is its rows; the weights of its first steps come meanwhile.
                     int early = 0;
                     if (!cur_ready) {
                         if (gemm) {
@@ -1139,7 +1170,9 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                         }
                         return true;
                     };
-                    if (gemm) {
+                    if (q.kind == kWorkGemm1 || q.kind == kWorkWgradDown) {
+                        ok = load_steps([](uint32_t, uint32_t, int) {});
+                    } else if (gemm) {
                         const CUtensorMap* map_a = a_rows == BM ? &P.map_a : &P.map_a32;
                         ok = load_steps([&](uint32_t dst, uint32_t bar, int k) {
                             if (a_rows != 0) tma_load_2d_2cta(dst, map_a, bar, k, q.m0);
@@ -1156,7 +1189,6 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                     for (const uint64_t t0 = globaltimer_ns(); globaltimer_ns() - t0 < 10000000ull;) __nanosleep(1000);
                 }
                 if (L.stats != nullptr) {
-                    if (w_arrive) atomicAdd(L.stats + kStatWaitArrival, w_arrive);
                     if (w_unit) atomicAdd(L.stats + kStatWaitFirstGemm, w_unit);
                     if (w_wgrad) atomicAdd(L.stats + kStatWaitWgrad, w_wgrad);
                 }
@@ -1169,12 +1201,23 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
             int ss = 0;
             uint32_t sph = 0;
             int acc = 0;                                     // accumulators (256 columns) used so far
+            uint32_t rows_phase = 0;                         // per stage: the phase of its rows_bar
             while (ok) {
                 int4 it;
                 if (!next_item(ss, sph, 652, it) || it.x < 0) break;
                 Item q;
                 decode_item(L, it, rank, q);
                 const bool a_mn = q.kind >= kWorkWgradDown;
+                // operands of a step are there: what TMA brings and what the loading warps do
+                auto loaded = [&](int s, uint32_t ph) {
+                    if (!mbar_wait(full_bar(s), ph, abort_flag, L.status, 621)) return false;
+                    if (q.kind != kWorkGemm2) {
+                        if (!mbar_wait(rows_bar(s), (rows_phase >> s) & 1u, abort_flag, L.status, 623)) return false;
+                        rows_phase ^= 1u << s;
+                    }
+                    tcgen05_fence_after();
+                    return true;
+                };
                 const uint32_t idesc = BWD ? (a_mn ? make_idesc_bf16(2 * BM, BN, true, true) : make_idesc_bf16(2 * BM, BN, false, true))
                                            : make_idesc_bf16(2 * BM, BN, false, false);
                 const int slot0 = acc & 1, slot1 = slot0 ^ 1;
@@ -1203,8 +1246,7 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                     int s = stage;
                     uint32_t ph = phase;
                     for (int i = 0; i < lead; ++i) {
-                        if (!mbar_wait(full_bar(s), ph, abort_flag, L.status, 621)) { ok = false; break; }
-                        tcgen05_fence_after();
+                        if (!(ok = loaded(s, ph))) break;
                         if (elect_one()) {
                             multiply(s, 0, slot0, i == 0);
                             if (i == q.nk - 1) umma_commit_2cta(tfull_bar(slot0), 3u);
@@ -1225,8 +1267,7 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                     }
                 }
                 for (; kb < q.nk; ++kb) {
-                    if (!mbar_wait(full_bar(stage), phase, abort_flag, L.status, 621)) { ok = false; break; }
-                    tcgen05_fence_after();
+                    if (!(ok = loaded(stage, phase))) break;
                     if (elect_one()) {
                         const bool last = kb == q.nk - 1;
                         multiply(stage, 0, slot0, kb == 0);
@@ -1248,8 +1289,13 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                     __syncwarp();
                 }
             }
-        } else if (warp >= 4) {
+        } else if (warp >= 2) {
+            if (!BWD && L.saved_x != nullptr) keep_x_loop();
+            gather_loop();
+        }
+        } else {
             // -------------------------------------------------------------- epilogue, then gather
+            registers_inc<kRegsEpilogue>();
             const int qd = warp & 3;
             const int hh = (warp - 4) >> 2;
             const Staging st{smem_base + kPipeBytesP + (uint32_t)(warp - 4) * kBoxBytes, lane};
@@ -1371,11 +1417,6 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
             if (lane == 0) tma_store_wait<0>();
             __syncwarp();
             if (ok) gather_loop();            // the list is done: help with the sums
-        } else if (warp >= 2) {
-            copy_loop();
-            if (BWD) copy_x_loop();
-            else if (L.saved_x != nullptr) keep_x_loop();
-            gather_loop();
         }
     }
 
@@ -1440,7 +1481,7 @@ cudaError_t launch(const LayerArgsP& L, int num_sms, cudaStream_t stream) {
     if (cudaError_t e = ensure_smem_limit(kern, kSmemBytesP, configured); e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(num_sms & ~1);
-    cfg.blockDim = dim3(kThreads);
+    cfg.blockDim = dim3(kLayerThreads);
     cfg.dynamicSmemBytes = kSmemBytesP;
     cfg.stream = stream;
     // every pair waits for rows that warps of all blocks copy and for tiles of other pairs: all of them have to be resident
@@ -1503,7 +1544,6 @@ LocalLayerPlan local_layer_plan(int T, int K, int E, int H, int I, int keep) {
         p.sync[d] = take(kSyncWords);
         p.done1[d] = take(p.units_cap);
         p.done2[d] = take(p.blocks_cap);
-        p.arrived[d] = take(p.blocks_cap);
     }
     p.zero_words = at;
     p.meta = take(kMetaWords);
@@ -1551,7 +1591,7 @@ cudaError_t local_layer_launch(const LocalLayerParams& q, cudaStream_t stream) {
     const int H = p.H, I = p.I, E = p.E, dir = q.bwd ? 1 : 0;
     if (H % BK != 0 || I % BK != 0 || q.out_rows % BM != 0 || q.out_rows < BM || q.out_rows < p.slots_cap || p.K < 1 || p.K > 32 || (q.bwd && !p.keep))
         return cudaErrorInvalidValue;
-    if (reinterpret_cast<uintptr_t>(q.x) % 16 != 0 || reinterpret_cast<uintptr_t>(q.slot_x) % 16 != 0) return cudaErrorInvalidValue;
+    if (reinterpret_cast<uintptr_t>(q.x) % 16 != 0 || reinterpret_cast<uintptr_t>(q.saved_x) % 16 != 0) return cudaErrorInvalidValue;
     const uint64_t R = (uint64_t)q.out_rows;
     LayerArgsP L{};
     cudaError_t e;
@@ -1564,7 +1604,6 @@ cudaError_t local_layer_launch(const LocalLayerParams& q, cudaStream_t stream) {
     g1.nk = H / BK;
     g1.cols = p.cols[dir][0];
     g2.n_total = H; g2.cols = p.cols[dir][1]; g2.num_n_blocks = column_blocks(H, g2.cols);
-    if ((e = make_map(&g1.map_a, q.slot_x, R, H, BK, BM)) != cudaSuccess || (e = make_map(&g1.map_a32, q.slot_x, R, H, BK, 32)) != cudaSuccess) return e;
     if (q.bwd && (e = make_map_narrow(&L.st_aux, q.aux, R, 2 * I)) != cudaSuccess) return e;
     if ((e = q.bwd ? make_map_narrow(&L.st_act, q.act, R, I) : make_map(&L.st_act, q.act, R, I, 64, 32)) != cudaSuccess) return e;
     if ((e = make_map(&L.st_y, q.y, R, H, 64, 32)) != cudaSuccess) return e;
@@ -1585,10 +1624,8 @@ cudaError_t local_layer_launch(const LocalLayerParams& q, cudaStream_t stream) {
         // dW_down[e] = dY[seg]^T . act_w[seg]  ([H, I]);  dW_gateup[e] = dGU[seg]^T . X[seg]  ([2I, H])
         Phase& gd = L.ph[kWorkWgradDown];
         Phase& gg = L.ph[kWorkWgradGateup];
-        if ((e = make_map_mn(&gd.map_a, q.slot_x, R, H)) != cudaSuccess) return e;
         if ((e = make_map_mn(&gd.map_b, q.act, R, I)) != cudaSuccess) return e;
         if ((e = make_map_mn(&gg.map_a, q.aux, R, 2 * I)) != cudaSuccess) return e;
-        if ((e = make_map_mn(&gg.map_b, q.xperm, R, H)) != cudaSuccess) return e;
         gd.m_total = H; gd.n_total = I; gd.cols = p.cols[1][2];
         gg.m_total = 2 * I; gg.n_total = H; gg.cols = p.cols[1][3];
         if ((e = make_store_map3(&L.st_dwd, q.dw_down, E, H, I)) != cudaSuccess) return e;
@@ -1597,10 +1634,8 @@ cudaError_t local_layer_launch(const LocalLayerParams& q, cudaStream_t stream) {
     g1.num_n_blocks = column_blocks(g1.n_total, g1.cols);
     L.T = p.T; L.K = p.K; L.H = H; L.I = I; L.E = E; L.keep = p.keep;
     L.x = static_cast<const uint8_t*>(q.x);
-    L.slot_x = static_cast<uint8_t*>(q.slot_x);
     L.y = static_cast<const __nv_bfloat16*>(q.y);
     L.saved_x = static_cast<__nv_bfloat16*>(q.saved_x);
-    L.xperm = static_cast<__nv_bfloat16*>(q.xperm);
     L.out = static_cast<__nv_bfloat16*>(q.out);
     L.preact = static_cast<__nv_bfloat16*>(q.preact);
     L.droute_part = q.droute_part;
@@ -1616,7 +1651,6 @@ cudaError_t local_layer_launch(const LocalLayerParams& q, cudaStream_t stream) {
     L.sync = q.ws + p.sync[dir];
     L.done1 = q.ws + p.done1[dir];
     L.done2 = q.ws + p.done2[dir];
-    L.arrived = q.ws + p.arrived[dir];
     L.stats = reinterpret_cast<unsigned long long*>(q.ws + p.stats[dir]);
     L.status = q.status;
     const int sms = default_sms(q.num_sms) & ~1;

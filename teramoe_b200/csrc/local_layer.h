@@ -18,7 +18,7 @@ struct LocalLayerPlan {
     int work_cap[2];                     // items of the forward / backward list
     int cols[2][4];                      // columns per tile: [direction][first GEMM, second GEMM, dW_down, dW_gateup]
     // zero-filled by local_layer_route
-    long stats[2], sync[2], done1[2], done2[2], arrived[2], zero_words;
+    long stats[2], sync[2], done1[2], done2[2], zero_words;
     // written by it
     long meta, seg, slot_tk, slot_w, token_order, order_slot, chunk_hist, chunk_last, work[2], words;
 };
@@ -36,7 +36,6 @@ struct LocalLayerParams {
     const void* x;                       // [T, H] forward x, backward grad_out
     const void* w_gateup;
     const void* w_down;
-    void* slot_x;                        // [out_rows, H] rows in slot order
     void* y;                             // [out_rows, H] second GEMM's output in slot order
     int out_rows;                        // rows of the slot-order tensors: max(slots_cap, 128)
     void* act;                           // forward act, backward act x route [out_rows, I]
@@ -46,7 +45,6 @@ struct LocalLayerParams {
     void* preact;                        // written by forward (with keep), read by backward: 2I * out_rows values in 32 x 8 blocks
     // backward
     float* droute_part;                  // [out_rows, 2 * ceil(I / 256)]
-    void* xperm;                         // [out_rows, H]
     float* dw_topk;                      // [T, K]
     void* dw_gateup;
     void* dw_down;
