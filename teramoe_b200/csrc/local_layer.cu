@@ -57,16 +57,16 @@ constexpr int kKeepRows = 8;                                              // row
 constexpr int kGatherWarps = 2 + kEpiWarps;                               // warps of a CTA that sum in the end
 constexpr int kLoadWarps = 4;
 constexpr int kLayerThreads = kThreads + 32 * kLoadWarps;
-// Registers per thread: 128 at launch (512 threads), then by warpgroup
-constexpr int kRegsControl = 120, kRegsEpilogue = 168, kRegsLoad = 56;
-static_assert(128 * kRegsControl + 256 * kRegsEpilogue + 128 * kRegsLoad <= 65536 && kThreads == 384 && kLayerThreads == 512, "register file");
+// Registers per thread: 128 at launch (512 threads), which the first warpgroup keeps
+constexpr int kRegsEpilogue = 144, kRegsLoad = 96;
+static_assert(128 * 128 + 256 * kRegsEpilogue + 128 * kRegsLoad <= 65536 && kThreads == 384 && kLayerThreads == 512, "register file");
 constexpr int kRingDepth = 4;
 constexpr int kSoon = 32;                                                 // looks at a barrier before its wait counts as one
 constexpr int kOwed = 4;                                                  // finished tiles an epilogue warp counts at once
 constexpr int kGatherTasks = 16384;                                       // least number of (token, columns) tasks of the gather role
-constexpr uint32_t kOffTmem = 496, kOffRows = 192, kOffRingFull = 320, kOffRingEmpty = 352, kOffItems = 384;
+constexpr uint32_t kOffTmem = 496, kOffRingFull = 320, kOffRingEmpty = 352, kOffItems = 384;
 constexpr uint32_t kRingConsumers = 2 * (kEpiWarps + kLoadWarps) + 2;
-static_assert(8 * (2 * kMaxStages + 4) <= (int)kOffRows && kOffRows + 8 * kMaxStages <= kOffRingFull && kOffItems + 16 * kRingDepth <= kOffTmem && kOffTmem + 8 <= 512, "barrier block");
+static_assert(8 * (2 * kMaxStages + 4) <= (int)kOffRingFull && kOffItems + 16 * kRingDepth <= kOffTmem && kOffTmem + 8 <= 512, "barrier block");
 static_assert(kSmemBytesP <= 232448, "shared memory");
 
 // words of the sync block
@@ -448,13 +448,14 @@ __device__ __forceinline__ bool wait_count(const int* flag, int target, int* sta
 }
 
 // 16 bytes from memory into shared memory, or zeros
-__device__ __forceinline__ void cp_async_16(uint32_t dst_smem, const void* src) {
-    asm volatile("cp.async.cg.shared.global.L2::256B [%0], [%1], 16;" ::"r"(dst_smem), "l"(src) : "memory");
-}
 __device__ __forceinline__ void cp_async_16_or_zeros(uint32_t dst_smem, const void* src, bool wanted) {
     asm volatile("cp.async.cg.shared.global.L2::256B [%0], [%1], 16, %2;" ::"r"(dst_smem), "l"(src), "r"(wanted ? 16 : 0) : "memory");
 }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
 template <int R>
 __device__ __forceinline__ void registers_inc() {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(R));
@@ -709,7 +710,6 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
     auto tempty_bar = [&](int s) { return bar_base + 8u * (2 * kMaxStages + 2 + s); };
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + kBarOffsetP + kOffTmem);
     volatile uint32_t* abort_flag = tmem_slot + 1;
-    auto rows_bar = [&](int s) { return bar_base + kOffRows + 8u * s; };
     auto ring_full = [&](int e) { return bar_base + kOffRingFull + 8u * e; };
     auto ring_empty = [&](int e) { return bar_base + kOffRingEmpty + 8u * e; };
 
@@ -720,9 +720,8 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
     if (threadIdx.x == 0) {
         *abort_flag = 0u;
         for (int s = 0; s < kMaxStages; ++s) {
-            mbar_init(full_bar(s), 2);
+            mbar_init(full_bar(s), 4);                       // of each CTA the producer and a loading warp
             mbar_init(empty_bar(s), 1);
-            mbar_init(rows_bar(s), 2);
         }
         for (int s = 0; s < 2; ++s) {
             mbar_init(tfull_bar(s), 1);
@@ -875,21 +874,17 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                 if (part == 0 && lane < K && slot < 0) L.dw_topk[(long)t * K + lane] = 0.f;
             }
             int4* dst = reinterpret_cast<int4*>(L.out + (long)t * L.H);
-            int sl[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) sl[j] = max(0, __shfl_sync(0xffffffffu, slot, j));
             const int step1 = min(steps, (part + 1) * part_steps);
             for (int step = part * part_steps; step < step1; ++step) {
                 const int c0 = step * 64 + lane, c1 = c0 + 32;
                 const int v0 = min(c0, nvec - 1), v1 = min(c1, nvec - 1);
                 float a0[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
                 float a1[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-                add_rows(sl, min(K, 8), valid, v0, v1, a0, a1);
-                for (int k0 = 8; k0 < K; k0 += 8) {
-                    int more[8];
+                for (int k0 = 0; k0 < K; k0 += 8) {
+                    int sl[8];
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) more[j] = max(0, __shfl_sync(0xffffffffu, slot, (k0 + j) & 31));
-                    add_rows(more, min(K - k0, 8), valid >> k0, v0, v1, a0, a1);
+                    for (int j = 0; j < 8; ++j) sl[j] = max(0, __shfl_sync(0xffffffffu, slot, (k0 + j) & 31));
+                    add_rows(sl, min(K - k0, 8), valid >> k0, v0, v1, a0, a1);
                 }
                 if (c0 < nvec)
                     dst[c0] = make_int4((int)pack_bf16x2(a0[0], a0[1]), (int)pack_bf16x2(a0[2], a0[3]), (int)pack_bf16x2(a0[4], a0[5]),
@@ -934,20 +929,34 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
         // forward of 3001 tokens 1.897 -> 1.871, of 32 tokens 0.582 -> 0.592.  (With TMA loads of as many consecutive rows instead the
         // large forward would take 3 % less: what these copies cost.)
         //
-        // A warp takes every fourth step: it waits for the stage, copies, sees its copies through and hands the step over, so that four
-        // steps' copies are under way at a time.  All four warps on every step, two steps under way, were 4 % slower; an address
-        // computed per column block instead of per row made dW_gateup 25 % slower.
+        // A warp takes every fourth step: it waits for the stage, copies, and hands the step over when its copies have landed, which it sees to
+        // behind the copies of its next step if that one's stage is free, so that copies into all stages are under way at a time.
+        // All four warps on every step, two steps under way, were 4 % slower; an address computed per column block instead of per
+        // row made dW_gateup 25 % slower; registers for fewer addresses (56 instead of 96 per thread, some spilled) cost 5 %.
         auto load_rows = [&]() {
             const int sub = lane >> 3, chunk = lane & 7;
-            const uint32_t pair_rows = mapa_shared(rows_bar(0), 0);
+            const uint32_t pair_full = mapa_shared(full_bar(0), 0);
             const uint32_t at[2] = {(uint32_t)(sub * 128 + ((chunk ^ sub) << 4)), (uint32_t)(sub * 128 + ((chunk ^ (sub + 4)) << 4))};      // rows 8i + sub, 8i + 4 + sub
             const uint64_t inverse = ~0ull / (uint32_t)L.K;   // entry / K = (entry + 1) * floor((2^64 - 1) / K) / 2^64, exact for 32-bit entries
             auto token = [&](int tk) { return tk < 0 ? -1 : (int)__umul64hi((uint64_t)(uint32_t)tk + 1u, inverse); };
             const long pitch = L.H * 2l;
             int step = warp - 12, stage = step, ss = 0;      // this warp's next step, counted from the start of the item; its stage
             uint32_t phase = 0, sph = 0;
+            int under_way = -1;                              // stage of the step before, if its copies are not yet seen through
+            auto hand_over = [&](int s) {
+                fence_proxy_async_smem();
+                __syncwarp();
+                if (lane == 0) mbar_arrive_cluster(pair_full + 8u * s);
+            };
+            auto settle = [&]() {
+                if (under_way < 0) return;
+                cp_async_wait<0>();
+                hand_over(under_way);
+                under_way = -1;
+            };
             while (true) {
                 int4 it;
+                if (!__all_sync(0xffffffffu, mbar_test_wait(ring_full(ss), sph))) settle();
                 if (!next_item(ss, sph, 654, it) || it.x < 0) break;
                 Item q;
                 decode_item(L, it, rank, q);
@@ -968,7 +977,8 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                 }
                 bool ok = true;
                 for (; step < q.nk; step += kLoadWarps) {
-                    // (a step of the second GEMM is waited for as well: a phase is told from the next but one by its parity alone)
+                    // (never behind a wait: the stage may be waiting for the step before)
+                    if (q.kind == kWorkGemm2 || !__all_sync(0xffffffffu, mbar_test_wait(empty_bar(stage), phase ^ 1u))) settle();
                     if (!(ok = mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag, L.status, 611))) break;
                     const uint32_t dst = smem_base + (uint32_t)(stage * L.stage_bytes);
                     if (q.kind == kWorkGemm1) {
@@ -978,7 +988,7 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
 #pragma unroll
                             for (int j = 0; j < decltype(quads)::value; ++j) {
                                 const int t = __shfl_sync(0xffffffffu, row[j >> 3], (4 * j + sub) & 31);
-                                if (t >= 0) cp_async_16(dst + j * 512 + at[j & 1], src + t * pitch);
+                                cp_async_16_or_zeros(dst + j * 512 + at[j & 1], src + max(t, 0) * pitch, t >= 0);
                             }
                         };
                         if (q.real > 32) copy(std::integral_constant<int, 32>());
@@ -989,28 +999,41 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
 #pragma unroll
                         for (int i = 0; i < 2; ++i)
                             row[i] = step + kLoadWarps < q.nk ? L.slot_tk[q.k0 + (step + kLoadWarps) * BK + lane + 32 * i] : -1;
-                        // (columns past the last are not loaded: they are rows or columns of the result that are not stored)
+                        // (no branch between the copies: columns past the last are zeros)
                         const int c0 = down ? q.m0 : q.n0 + (int)rank * (BN / 2);
                         auto copy = [&](auto atoms) {
+                            constexpr int kAtoms = decltype(atoms)::value;
+                            bool in[kAtoms];
+                            int at_col[kAtoms];
+#pragma unroll
+                            for (int a = 0; a < kAtoms; ++a) {
+                                const int col = c0 + (a >> 1) * BN + (a & 1) * 64;
+                                in[a] = col < L.H;
+                                at_col[a] = in[a] ? col * 2 : 0;
+                            }
 #pragma unroll
                             for (int j = 0; j < 16; ++j) {
                                 const int t = __shfl_sync(0xffffffffu, tok[j >> 3], (4 * j + sub) & 31);
-                                const uint8_t* from = src + max(t, 0) * pitch + c0 * 2;
+                                const uint8_t* from = src + max(t, 0) * pitch;
                                 const uint32_t to = dst + (down ? 0 : kAStageBytes) + j * 512 + at[j & 1];
 #pragma unroll
-                                for (int a = 0; a < decltype(atoms)::value; ++a)
-                                    if (c0 + (a >> 1) * BN + (a & 1) * 64 < L.H)
-                                        cp_async_16_or_zeros(to + a * kAtomBytes, from + ((a >> 1) * BN + (a & 1) * 64) * 2, t >= 0);
+                                for (int a = 0; a < kAtoms; ++a) cp_async_16_or_zeros(to + a * kAtomBytes, from + at_col[a], in[a] && t >= 0);
                             }
                         };
                         if (down || q.halves == 1) copy(std::integral_constant<int, 2>());
                         else copy(std::integral_constant<int, 4>());
                     }
-                    if (q.kind != kWorkGemm2) {
-                        cp_async_wait_all();
-                        fence_proxy_async_smem();
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive_cluster(pair_rows + 8u * stage);
+                    if (q.kind == kWorkGemm2) {
+                        // no rows; the warp takes part all the same, so that it is never a whole turn through the stages behind or ahead of the
+                        // others, which the parity of a phase would not show
+                        hand_over(stage);
+                    } else {
+                        cp_async_commit();
+                        if (under_way >= 0) {
+                            cp_async_wait<1>();
+                            hand_over(under_way);
+                        }
+                        under_way = stage;
                     }
                     stage += kLoadWarps;
                     if (stage >= L.stages) { stage -= L.stages; phase ^= 1u; }
@@ -1018,13 +1041,13 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                 if (!ok) break;
                 step -= q.nk;
             }
+            settle();
         };
 
         if (warp >= 12) {
             registers_dec<kRegsLoad>();
             load_rows();
         } else if (warp < 4) {
-        registers_dec<kRegsControl>();
         if (warp == 0) {
             // -------------------------------------------------------------- item fetch (first CTA) + TMA producer
             if (elect_one()) {
@@ -1201,23 +1224,12 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
             int ss = 0;
             uint32_t sph = 0;
             int acc = 0;                                     // accumulators (256 columns) used so far
-            uint32_t rows_phase = 0;                         // per stage: the phase of its rows_bar
             while (ok) {
                 int4 it;
                 if (!next_item(ss, sph, 652, it) || it.x < 0) break;
                 Item q;
                 decode_item(L, it, rank, q);
                 const bool a_mn = q.kind >= kWorkWgradDown;
-                // operands of a step are there: what TMA brings and what the loading warps do
-                auto loaded = [&](int s, uint32_t ph) {
-                    if (!mbar_wait(full_bar(s), ph, abort_flag, L.status, 621)) return false;
-                    if (q.kind != kWorkGemm2) {
-                        if (!mbar_wait(rows_bar(s), (rows_phase >> s) & 1u, abort_flag, L.status, 623)) return false;
-                        rows_phase ^= 1u << s;
-                    }
-                    tcgen05_fence_after();
-                    return true;
-                };
                 const uint32_t idesc = BWD ? (a_mn ? make_idesc_bf16(2 * BM, BN, true, true) : make_idesc_bf16(2 * BM, BN, false, true))
                                            : make_idesc_bf16(2 * BM, BN, false, false);
                 const int slot0 = acc & 1, slot1 = slot0 ^ 1;
@@ -1246,7 +1258,8 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                     int s = stage;
                     uint32_t ph = phase;
                     for (int i = 0; i < lead; ++i) {
-                        if (!(ok = loaded(s, ph))) break;
+                        if (!mbar_wait(full_bar(s), ph, abort_flag, L.status, 621)) { ok = false; break; }
+                        tcgen05_fence_after();
                         if (elect_one()) {
                             multiply(s, 0, slot0, i == 0);
                             if (i == q.nk - 1) umma_commit_2cta(tfull_bar(slot0), 3u);
@@ -1267,7 +1280,8 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                     }
                 }
                 for (; kb < q.nk; ++kb) {
-                    if (!(ok = loaded(stage, phase))) break;
+                    if (!mbar_wait(full_bar(stage), phase, abort_flag, L.status, 621)) { ok = false; break; }
+                    tcgen05_fence_after();
                     if (elect_one()) {
                         const bool last = kb == q.nk - 1;
                         multiply(stage, 0, slot0, kb == 0);

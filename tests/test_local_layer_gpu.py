@@ -113,6 +113,20 @@ def test_batches_end_where_experts_do(batch, monkeypatch):
     buf.destroy()
 
 
+@pytest.mark.parametrize("H,I", [(512, 64), (64, 512), (1024, 128)])
+def test_loading_warps_keep_up_with_short_items(H, I):
+    """Items of one to a few steps of K, in which the loading warps have rows to bring and in which they have none, many times over: no
+    step is left behind (its wait would run out) and every run gives the same bits."""
+    prob = make_problem(1, 3000, H, I, 24, 4, seed=H, dtype=torch.bfloat16, device="cuda", x_scale=0.1, w_scale=0.02)
+    buf = tm.Buffer(None, int(64e6), explicitly_destroy=True)
+    want = _run(buf, prob, prob["ranks"][0]["idx"], 24)
+    for _ in range(30):
+        got = _run(buf, prob, prob["ranks"][0]["idx"], 24)
+        assert all(torch.equal(got[name], want[name]) for name in want)
+    buf.check_status()
+    buf.destroy()
+
+
 def test_native_autograd_node_keeps_its_buffer_and_fills_the_given_gradient():
     """The buffer may go out of scope before the backward pass; d(topk_weights) goes to the caller's tensor; a second derivative
     raises; a destroyed buffer raises."""
