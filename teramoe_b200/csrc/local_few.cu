@@ -1,0 +1,365 @@
+// The layer's forward on one rank when experts have few rows (local_layer_plan decides), as in decoding: the time is that of reading the
+// weights once.  The weights are the M operand here, 128 rows of a tile, and an expert's tokens the N operand, 16 to 64 columns.  With the
+// roles of local_layer.cu eight tokens were multiplied as 256 rows; under the power cap, which such a call reaches too, the tensor
+// cores' share is bandwidth lost.  Forward of 32 tokens, H=7168 I=2048, 32 experts, top-8: 577 -> 441 us, 6.4 TB/s, which is what a plain
+// copy reaches; of 16 tokens, H=2048 I=2048, 16 experts 110 -> 85; of 16 tokens, H=512 I=256, 4 experts, top-2 31 -> 22.
+//
+// One persistent block per SM, no clusters.  Items: first the tiles of the first GEMM (128 rows of W_gateup of an expert x a unit of up to
+// 64 of its tokens), then those of the second, dealt out in turn: they all cost the same.  Units of one expert are neighbours, so that
+// they share the tile of weights in L2.
+//   warp 0     loads: weights by TMA boxes, token rows by TMA row gather (16 copies of 4 rows in a step at most; what made it too slow
+//              for the large tiles of local_layer.cu hides here behind the weights), the second GEMM's rows by boxes of 16
+//   warp 1     issues tcgen05.mma, 128 x N x 16, into one of four accumulators
+//   warps 4-7  epilogue: a lane holds one row of weights, so gate and up of a token sit in neighbouring lanes
+//   warps 2-7  at the end: sums of the tokens' expert rows, in the order of their entries
+// Nine stages of 24 KB keep 144 KB of weights per SM on their way.
+#include "local_layer.h"
+
+#include "gemm_common.cuh"
+
+namespace tmoe {
+
+using namespace detail;
+
+namespace {
+
+constexpr int kUnit = kFewUnitRows;
+constexpr int kFewStages = 9;
+constexpr int kFewStageBytes = kAStageBytes + kUnit * BK * 2;             // 24 KB
+constexpr int kFewAccs = 4;
+constexpr int kFewThreads = 256;
+constexpr int kFewEpiWarps = 4;
+constexpr int kFewSumWarps = 6;
+constexpr int kFewBarOffset = kFewStages * kFewStageBytes;
+constexpr int kFewUnitsOffset = kFewBarOffset + 256;                      // [experts + 1] first unit, [experts] rows, [experts] first slot
+constexpr int kFewSmemBytes = kFewUnitsOffset + (3 * kLocalMaxExperts + 1) * 4 + 1024;
+static_assert(8 * (2 * kFewStages + 2 * kFewAccs) <= 248 && kFewSmemBytes <= 232448, "shared memory");
+
+struct FewArgs {
+    alignas(64) CUtensorMap map_wg, map_wd, map_x, map_act;
+    int T, K, H, I, E;
+    __nv_bfloat16* act;
+    __nv_bfloat16* y;
+    __nv_bfloat16* out;
+    const int* seg;
+    const int* counts;
+    const int* slot_tk;
+    const float* slot_w;
+    const int* token_order;
+    const int* order_slot;
+    int* done1;                          // per 64 slots: epilogue warps that finished a tile of the first GEMM
+    int* done2;                          // the same for the second
+    int* status;
+};
+
+struct FewItem {
+    int second, expert, tile, slot0, rows, n;      // n: columns of the accumulator that are computed
+};
+
+__global__ void __launch_bounds__(kFewThreads, 1) local_few_kernel(const __grid_constant__ FewArgs L) {
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
+    const uint32_t bar_base = smem_base + kFewBarOffset;
+    auto full_bar = [&](int s) { return bar_base + 8u * s; };
+    auto empty_bar = [&](int s) { return bar_base + 8u * (kFewStages + s); };
+    auto tfull_bar = [&](int a) { return bar_base + 8u * (2 * kFewStages + a); };
+    auto tempty_bar = [&](int a) { return bar_base + 8u * (2 * kFewStages + kFewAccs + a); };
+    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + kFewBarOffset + 248);
+    volatile uint32_t* abort_flag = tmem_slot + 1;
+    int* units = reinterpret_cast<int*>(smem_gen + kFewUnitsOffset);
+    int* counts = units + L.E + 1;
+    int* seg = counts + L.E;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, E = L.E;
+
+    if (threadIdx.x == 0) {
+        *abort_flag = 0u;
+        for (int s = 0; s < kFewStages; ++s) {
+            mbar_init(full_bar(s), 1);
+            mbar_init(empty_bar(s), 1);
+        }
+        for (int a = 0; a < kFewAccs; ++a) {
+            mbar_init(tfull_bar(a), 1);
+            mbar_init(tempty_bar(a), kFewEpiWarps);
+        }
+        fence_mbar_init();
+        tma_prefetch_desc(&L.map_wg);
+        tma_prefetch_desc(&L.map_wd);
+        tma_prefetch_desc(&L.map_x);
+        tma_prefetch_desc(&L.map_act);
+    }
+    if (warp == 2) tmem_alloc(smem_u32((const void*)tmem_slot), kFewAccs * kUnit);
+    if (warp == 1) {
+        int run = 0;
+        for (int e0 = 0; e0 < E; e0 += 32) {
+            const int e = e0 + lane, c = e < E ? L.counts[e] : 0, own = (c + kUnit - 1) / kUnit;
+            int v = own;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int u = __shfl_up_sync(0xffffffffu, v, o);
+                if (lane >= o) v += u;
+            }
+            if (e < E) {
+                units[e] = run + v - own;
+                counts[e] = c;
+                seg[e] = L.seg[e];
+            }
+            run += __shfl_sync(0xffffffffu, v, 31);
+        }
+        if (lane == 0) units[E] = run;
+    }
+    tcgen05_fence_before();
+    __syncthreads();
+    tcgen05_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+
+    const int n1 = 2 * L.I / BM, n2 = (L.H + BM - 1) / BM, U = units[E], items = U * (n1 + n2);
+    auto decode = [&](int i) {
+        FewItem q;
+        q.second = i >= U * n1;
+        const int n = q.second ? n2 : n1, j = q.second ? i - U * n1 : i;
+        int lo = 0, hi = E;                          // the expert: units[lo] * n <= j < units[lo + 1] * n
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if (units[mid] * n <= j) lo = mid;
+            else hi = mid;
+        }
+        const int of_expert = units[lo + 1] - units[lo], r = j - units[lo] * n;
+        q.expert = lo;
+        q.tile = r / of_expert;
+        const int row0 = (r - q.tile * of_expert) * kUnit;
+        q.slot0 = seg[lo] + row0;
+        q.rows = min(kUnit, counts[lo] - row0);
+        q.n = (q.rows + 15) & ~15;
+        return q;
+    };
+    const int nk1 = L.H / BK, nk2 = L.I / BK;
+
+    if (warp == 0) {
+        int stage = 0;
+        uint32_t phase = 0;
+        bool ok = true;
+        for (int i = blockIdx.x; i < items && ok; i += gridDim.x) {
+            const FewItem q = decode(i);
+            const int nk = q.second ? nk2 : nk1, quads = (q.rows + 3) / 4, boxes = q.n / 16;
+            const int w_row = q.second ? q.expert * L.H + q.tile * BM : q.expert * 2 * L.I + q.tile * BM;
+            const CUtensorMap* map_w = q.second ? &L.map_wd : &L.map_wg;
+            const uint32_t tx = (uint32_t)(kAStageBytes + (q.second ? boxes * 16 : quads * 4) * BK * 2);
+            int4 tokens = make_int4(L.T, L.T, L.T, L.T);         // (past the end: zeros)
+            if (!q.second && lane < quads) {
+                int t[4];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) t[c] = 4 * lane + c < q.rows ? L.slot_tk[q.slot0 + 4 * lane + c] / L.K : L.T;
+                tokens = make_int4(t[0], t[1], t[2], t[3]);
+            }
+            auto weights = [&](int s, uint32_t ph, int kb) {
+                if (!mbar_wait(empty_bar(s), ph ^ 1u, abort_flag, L.status, 680)) return false;
+                if (lane == 0) {
+                    mbar_arrive_expect_tx(full_bar(s), tx);
+                    tma_load_2d(smem_base + s * kFewStageBytes, map_w, full_bar(s), kb * BK, w_row);
+                }
+                __syncwarp();
+                return true;
+            };
+            // the weights of a second GEMM's first steps come while its rows are waited for
+            int early = 0;
+            if (q.second) {
+                const int* flag = L.done1 + q.slot0 / kUnit;
+                int ready = lane == 0 ? ld_acquire_gpu(flag) >= kFewEpiWarps * n1 : 0;
+                ready = __shfl_sync(0xffffffffu, ready, 0);
+                if (!ready) {
+                    int s = stage;
+                    uint32_t ph = phase;
+                    for (; early < min(kFewStages, nk); ++early) {
+                        if (!(ok = weights(s, ph, early))) break;
+                        if (++s == kFewStages) { s = 0; ph ^= 1u; }
+                    }
+                    if (!ok) break;
+                    // (a wait that runs out is reported, and the item carried through on whatever its rows hold)
+                    if (lane == 0) wait_count_gpu(flag, kFewEpiWarps * n1, L.status, 681, 64);
+                }
+                __syncwarp();
+                fence_proxy_async_all();                         // stores of other SMs -> async-proxy reads
+            }
+            for (int kb = 0; kb < nk; ++kb) {
+                if (kb >= early && !(ok = weights(stage, phase, kb))) break;
+                const uint32_t dst = smem_base + stage * kFewStageBytes + kAStageBytes;
+                if (q.second) {
+                    if (lane < boxes) tma_load_2d(dst + lane * 16 * BK * 2, &L.map_act, full_bar(stage), kb * BK, q.slot0 + 16 * lane);
+                } else if (lane < quads) {
+                    tma_gather4(dst + lane * 4 * BK * 2, &L.map_x, full_bar(stage), kb * BK, tokens);
+                }
+                if (++stage == kFewStages) { stage = 0; phase ^= 1u; }
+            }
+        }
+        if (!ok)                                                 // (no barrier says when the copies under way have landed: microseconds)
+            for (const uint64_t t0 = globaltimer_ns(); globaltimer_ns() - t0 < 10000000ull;) __nanosleep(1000);
+    } else if (warp == 1) {
+        int stage = 0, acc = 0;
+        uint32_t phase = 0, acc_phase = 0;
+        bool ok = true;
+        for (int i = blockIdx.x; i < items && ok; i += gridDim.x) {
+            const FewItem q = decode(i);
+            const int nk = q.second ? nk2 : nk1;
+            const uint32_t idesc = make_idesc_bf16(BM, q.n, false, false);
+            if (!(ok = mbar_wait(tempty_bar(acc), acc_phase ^ 1u, abort_flag, L.status, 682))) break;
+            tcgen05_fence_after();
+            for (int kb = 0; kb < nk; ++kb) {
+                if (!(ok = mbar_wait(full_bar(stage), phase, abort_flag, L.status, 683))) break;
+                tcgen05_fence_after();
+                if (elect_one()) {
+                    const uint32_t at = smem_base + stage * kFewStageBytes;
+                    const uint64_t a = make_smem_desc_sw128(at, 0, 1024), b = make_smem_desc_sw128(at + kAStageBytes, 0, 1024);
+#pragma unroll
+                    for (int k = 0; k < BK / UK; ++k)
+                        umma_bf16_ss(tmem_base + acc * kUnit, a + k * (UK * 2 >> 4), b + k * (UK * 2 >> 4), idesc, (kb | k) != 0 ? 1u : 0u);
+                    umma_commit(empty_bar(stage));
+                    if (kb == nk - 1) umma_commit(tfull_bar(acc));
+                }
+                __syncwarp();
+                if (++stage == kFewStages) { stage = 0; phase ^= 1u; }
+            }
+            if (++acc == kFewAccs) { acc = 0; acc_phase ^= 1u; }
+        }
+    } else if (warp >= 4) {
+        const int quarter = warp & 3;
+        int acc = 0;
+        uint32_t acc_phase = 0;
+        for (int i = blockIdx.x; i < items; i += gridDim.x) {
+            const FewItem q = decode(i);
+            const float w[2] = {!q.second && lane < q.rows ? L.slot_w[q.slot0 + lane] : 0.f, !q.second && lane + 32 < q.rows ? L.slot_w[q.slot0 + lane + 32] : 0.f};
+            if (!mbar_wait(tfull_bar(acc), acc_phase, abort_flag, L.status, 684)) break;
+            tcgen05_fence_after();
+            const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * kUnit);
+#pragma unroll
+            for (int c = 0; c < kUnit / 32; ++c) {
+                if (c * 32 >= q.rows) break;
+                uint32_t v[32];
+                tmem_ld_x32(taddr + c * 32, v);
+                tmem_ld_wait();
+                if (q.second) {
+                    const int h = q.tile * BM + quarter * 32 + lane;
+                    __nv_bfloat16* y = L.y + (long)(q.slot0 + c * 32) * L.H + h;
+#pragma unroll
+                    for (int r = 0; r < 32; ++r)
+                        if (c * 32 + r < q.rows && h < L.H) y[(long)r * L.H] = __float2bfloat16_rn(__uint_as_float(v[r]));
+                } else {
+                    // lanes 2j and 2j + 1 hold gate and up of column j: of two tokens each lane takes one
+                    const int odd = lane & 1;
+                    __nv_bfloat16* act = L.act + (long)(q.slot0 + c * 32 + odd) * L.I + q.tile * (BM / 2) + quarter * 16 + (lane >> 1);
+#pragma unroll
+                    for (int r = 0; r < 32; r += 2) {
+                        const float mine = __uint_as_float(odd ? v[r + 1] : v[r]);
+                        const float other = __shfl_xor_sync(0xffffffffu, __uint_as_float(odd ? v[r] : v[r + 1]), 1);
+                        const float route = __shfl_sync(0xffffffffu, w[c], r + odd);
+                        const float gt = odd ? other : mine, up = odd ? mine : other;
+                        const float a = __fdividef(gt, 1.f + __expf(-gt)) * up * route;
+                        if (c * 32 + r + odd < q.rows) act[(long)r * L.I] = __float2bfloat16_rn(a);
+                    }
+                }
+            }
+            tcgen05_fence_before();
+            __syncwarp();
+            if (lane == 0) {
+                mbar_arrive(tempty_bar(acc));
+                fence_acq_rel_gpu();
+                red_add_gpu((q.second ? L.done2 : L.done1) + q.slot0 / kUnit, 1);
+            }
+            if (++acc == kFewAccs) { acc = 0; acc_phase ^= 1u; }
+        }
+    }
+    __syncwarp();
+
+    if (warp >= 2) {
+        // sums: (token, 256 columns) per task
+        const int nvec = L.H / 8, parts = (nvec + 31) / 32, tasks = L.T * parts, K = L.K;
+        for (int task = (warp - 2) * (int)gridDim.x + (int)blockIdx.x; task < tasks; task += kFewSumWarps * (int)gridDim.x) {
+            const int place = task / parts, col = (task - place * parts) * 32 + lane, at = min(col, nvec - 1);
+            const int t = L.token_order[place], slot = lane < K ? L.order_slot[(long)place * K + lane] : -1;
+            const uint32_t valid = __ballot_sync(0xffffffffu, slot >= 0);
+            bool there = true;
+            if (slot >= 0) there = wait_count_gpu(L.done2 + slot / kUnit, kFewEpiWarps * n2, L.status, 685, 64);
+            if (!__all_sync(0xffffffffu, there)) break;          // reported: unwind
+            __syncwarp();                                        // every lane reads behind the other lanes' acquires
+            float sum[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+            for (int k0 = 0; k0 < K; k0 += 8) {
+                int4 v[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const int s = max(0, __shfl_sync(0xffffffffu, slot, (k0 + j) & 31));
+                    // (volatile keeps the load behind the acquire loads above)
+                    if (k0 + j < K)
+                        asm volatile("ld.global.cg.v4.s32 {%0, %1, %2, %3}, [%4];" : "=r"(v[j].x), "=r"(v[j].y), "=r"(v[j].z), "=r"(v[j].w)
+                                     : "l"(reinterpret_cast<const int4*>(L.y) + (long)s * nvec + at));
+                }
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    if (k0 + j >= K || !((valid >> (k0 + j)) & 1u)) continue;
+                    const uint32_t p[4] = {(uint32_t)v[j].x, (uint32_t)v[j].y, (uint32_t)v[j].z, (uint32_t)v[j].w};
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const float2 f = unpack_bf16x2(p[i]);
+                        sum[2 * i] += f.x;
+                        sum[2 * i + 1] += f.y;
+                    }
+                }
+            }
+            if (col < nvec)
+                reinterpret_cast<int4*>(L.out + (long)t * L.H)[col] = make_int4((int)pack_bf16x2(sum[0], sum[1]), (int)pack_bf16x2(sum[2], sum[3]),
+                                                                                (int)pack_bf16x2(sum[4], sum[5]), (int)pack_bf16x2(sum[6], sum[7]));
+        }
+    }
+    tcgen05_fence_before();
+    __syncthreads();
+    if (warp == 2) {
+        tcgen05_fence_after();
+        tmem_dealloc(tmem_base, kFewAccs * kUnit);
+    }
+}
+
+}  // namespace
+
+cudaError_t local_few_launch(const LocalLayerParams& q, cudaStream_t stream) {
+    const LocalLayerPlan& p = q.plan;
+    const int H = p.H, I = p.I, E = p.E;
+    if (!p.few || q.bwd || H % BK != 0 || I % BK != 0 || q.out_rows < p.slots_cap || p.K < 1 || p.K > 32 || E < 1 || E > kLocalMaxExperts)
+        return cudaErrorInvalidValue;
+    int dev = 0;
+    cudaError_t e;
+    if ((e = cudaGetDevice(&dev)) != cudaSuccess || (e = cudaSetDevice(dev)) != cudaSuccess) return e;      // (the tensor-map encoder wants a current context)
+    FewArgs L{};
+    if ((e = make_map(&L.map_wg, q.w_gateup, (uint64_t)E * 2 * I, H, BK, BM)) != cudaSuccess) return e;
+    if ((e = make_map(&L.map_wd, q.w_down, (uint64_t)E * H, I, BK, BM)) != cudaSuccess) return e;
+    if ((e = make_map(&L.map_x, q.x, p.T, H, BK, 1)) != cudaSuccess) return e;
+    if ((e = make_map(&L.map_act, q.act, q.out_rows, I, BK, 16)) != cudaSuccess) return e;
+    L.T = p.T; L.K = p.K; L.H = H; L.I = I; L.E = E;
+    L.act = static_cast<__nv_bfloat16*>(q.act);
+    L.y = static_cast<__nv_bfloat16*>(q.y);
+    L.out = static_cast<__nv_bfloat16*>(q.out);
+    L.seg = q.ws + p.seg;
+    L.counts = q.ws + p.counts;
+    L.slot_tk = q.ws + p.slot_tk;
+    L.slot_w = reinterpret_cast<const float*>(q.ws + p.slot_w);
+    L.token_order = q.ws + p.token_order;
+    L.order_slot = q.ws + p.order_slot;
+    L.done1 = q.ws + p.done1[0];
+    L.done2 = q.ws + p.done2[0];
+    L.status = q.status;
+    static bool configured[64] = {};
+    if ((e = ensure_smem_limit(local_few_kernel, kFewSmemBytes, configured)) != cudaSuccess) return e;
+    const int sms = default_sms(q.num_sms) & ~1;
+    if (sms < 4) return cudaErrorInvalidConfiguration;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(sms);
+    cfg.blockDim = dim3(kFewThreads);
+    cfg.dynamicSmemBytes = kFewSmemBytes;
+    cfg.stream = stream;
+    // blocks wait for tiles of other blocks: all of them have to be resident
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, local_few_kernel, L);
+}
+
+}  // namespace tmoe

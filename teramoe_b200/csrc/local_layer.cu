@@ -76,6 +76,8 @@ enum { kMetaUnits = 0, kMetaWork = 2, kMetaWords = 8 };
 
 constexpr int kWideTiles = 74 * 4;                                        // least number of wide tiles of a GEMM (local_layer_plan)
 
+constexpr int kFewRows = 16;                                              // most rows per expert of a forward in local_few.cu (local_layer_plan)
+
 constexpr int column_blocks(int n, int cols) { return (n + cols - 1) / cols; }
 
 constexpr int kRouteThreads = 256;
@@ -247,6 +249,7 @@ __global__ void __launch_bounds__(kRouteThreads) local_route_assign_kernel(const
     float* slot_w = reinterpret_cast<float*>(a.ws + a.p.slot_w);
     if (blockIdx.x == 0) {
         for (int e = tid; e <= E; e += kRouteThreads) a.ws[a.p.seg + e] = seg[e];
+        for (int e = tid; e < E; e += kRouteThreads) a.ws[a.p.counts + e] = totals[e];
         if (tid == 0) meta[kMetaUnits] = U;
     }
     for (int e = blockIdx.x; e < E; e += gridDim.x)
@@ -268,7 +271,7 @@ __global__ void __launch_bounds__(kRouteThreads) local_route_assign_kernel(const
         return 2 * behind < SG ? ub[e + 1] : (int)v;
     };
     const int per_wd = a.mu_wd * a.nb_wd, per_e = per_wd + a.mu_wg * a.nb_wg;
-    for (int dir = 0; dir < (a.p.keep ? 2 : 1); ++dir) {
+    for (int dir = 0; dir < (a.p.few ? 0 : a.p.keep ? 2 : 1); ++dir) {
         int4* work = reinterpret_cast<int4*>(a.ws + a.p.work[dir]);
         const int cap = a.p.work_cap[dir], nb1 = a.nb1[dir], nb2 = a.nb2[dir];
         const int items = U * (nb1 + nb2);                   // of the two GEMMs
@@ -425,28 +428,6 @@ __device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t a, uint32_t
 __device__ __forceinline__ void ld_shared_v4(uint32_t addr, uint32_t (&v)[4]) {
     asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(addr) : "memory");
 }
-// Bounded wait until *flag >= target (counters that other SMs of this GPU bump, so a second is long).  It runs out before the waits
-// inside the CTA pair do (2 s): while the producer waits here, the issuer and the epilogue wait for its operands.
-constexpr uint64_t kCountLimitNs = 1000000000ull;
-__device__ __forceinline__ bool wait_count(const int* flag, int target, int* status, int site, uint32_t pause_ns) {
-    if (ld_acquire_gpu(flag) >= target) return true;
-    const uint64_t limit_ns = min(peer_wait_limit_ns(status), kCountLimitNs);
-    const uint64_t t0 = globaltimer_ns();
-#pragma unroll 1
-    while (true) {
-#pragma unroll 1
-        for (int i = 0; i < 32; ++i) {
-            if (ld_acquire_gpu(flag) >= target) return true;
-            __nanosleep(pause_ns);
-        }
-        if (status != nullptr && ld_relaxed_sys(status) != 0) return false;
-        if (globaltimer_ns() - t0 > limit_ns) {
-            report_status(status, kStatusFlagTimeout, site, target);
-            return false;
-        }
-    }
-}
-
 // 16 bytes from memory into shared memory, or zeros
 __device__ __forceinline__ void cp_async_16_or_zeros(uint32_t dst_smem, const void* src, bool wanted) {
     asm volatile("cp.async.cg.shared.global.L2::256B [%0], [%1], 16, %2;" ::"r"(dst_smem), "l"(src), "r"(wanted ? 16 : 0) : "memory");
@@ -1093,7 +1074,7 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                     if (ld_acquire_gpu(flag) >= target) return 1;
                     if (!block) return 0;
                     const uint64_t t0 = globaltimer_ns();
-                    const bool got = wait_count(flag, target, L.status, site, 64);
+                    const bool got = wait_count_gpu(flag, target, L.status, site, 64);
                     waited += globaltimer_ns() - t0;
                     return got ? 1 : -1;
                 };
@@ -1517,6 +1498,11 @@ LocalLayerPlan local_layer_plan(int T, int K, int E, int H, int I, int keep) {
     p.blocks_cap = (int)((entries + 127 * segs) / 128);
     p.slots_cap = p.blocks_cap * 128;
     p.units_cap = (int)((p.blocks_cap + segs) / 2);
+    // Few rows per expert, forward only: weights as the M operand (local_few.cu).  us, here / there (32 experts, top-8, H=7168 I=2048; I=512), by
+    // rows per expert: 1 368 / 279, 8 577 / 441, 16 589 / 471; 184 / 151, 24 600 / 522; 191 / 172, 32 615 / 566; 200 / 194.  Skewed routing
+    // (hottest expert 2.5 times the mean) at 20: 603 / 528; 189 / 186, and with the hottest 5 times the mean 606 / 538; 189 / 221 (at 16:
+    // 185 / 185), as experts of more than 64 rows take their weights twice: the line is where that still costs nothing.
+    p.few = !keep && T > 0 && entries <= (long)kFewRows * E;
     // Columns per tile of every GEMM [direction][kind].  The wide tile needs columns for it, enough tiles that every CTA pair gets
     // several, and a mainloop that is long against what it cannot hide: with both accumulators in one tile, the next tile
     // starts when the first half has been read out (in cycles: 2 thousand for a plain store, 3.6 for SwiGLU, 13.5 for its backward), where
@@ -1542,7 +1528,7 @@ LocalLayerPlan local_layer_plan(int T, int K, int E, int H, int I, int keep) {
     p.cols[1][1] = columns(H, units, 2 * I, 1024);
     p.cols[1][2] = columns(I, (long)E * mu_wd, rows, 1024);
     p.cols[1][3] = columns(H, (long)E * mu_wg, rows, 1024);
-    p.work_cap[0] = p.units_cap * (column_blocks(2 * I, p.cols[0][0]) + column_blocks(H, p.cols[0][1]));
+    p.work_cap[0] = p.few ? 0 : p.units_cap * (column_blocks(2 * I, p.cols[0][0]) + column_blocks(H, p.cols[0][1]));
     p.work_cap[1] = keep ? p.units_cap * (column_blocks(I, p.cols[1][0]) + column_blocks(H, p.cols[1][1])) +
                                E * (mu_wd * column_blocks(I, p.cols[1][2]) + mu_wg * column_blocks(H, p.cols[1][3]))
                          : 0;
@@ -1556,12 +1542,13 @@ LocalLayerPlan local_layer_plan(int T, int K, int E, int H, int I, int keep) {
     for (int d = 0; d < dirs; ++d) {
         p.stats[d] = take(2 * kLayerStatWords);
         p.sync[d] = take(kSyncWords);
-        p.done1[d] = take(p.units_cap);
-        p.done2[d] = take(p.blocks_cap);
+        p.done1[d] = take(p.few ? 128 / kFewUnitRows * p.blocks_cap : p.units_cap);
+        p.done2[d] = take(p.few ? 128 / kFewUnitRows * p.blocks_cap : p.blocks_cap);
     }
     p.zero_words = at;
     p.meta = take(kMetaWords);
     p.seg = take(E + 1);
+    p.counts = take(E);
     p.slot_tk = take(p.slots_cap);
     p.slot_w = take(p.slots_cap);
     p.token_order = take(T);
@@ -1602,6 +1589,7 @@ cudaError_t local_layer_route(const LocalLayerParams& q, cudaStream_t stream) {
 
 cudaError_t local_layer_launch(const LocalLayerParams& q, cudaStream_t stream) {
     const LocalLayerPlan& p = q.plan;
+    if (p.few) return local_few_launch(q, stream);
     const int H = p.H, I = p.I, E = p.E, dir = q.bwd ? 1 : 0;
     if (H % BK != 0 || I % BK != 0 || q.out_rows % BM != 0 || q.out_rows < BM || q.out_rows < p.slots_cap || p.K < 1 || p.K > 32 || (q.bwd && !p.keep))
         return cudaErrorInvalidValue;

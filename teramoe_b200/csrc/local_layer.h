@@ -7,12 +7,14 @@
 
 namespace tmoe {
 
+constexpr int kFewUnitRows = 64;         // rows of an expert that local_few.cu multiplies at a time
 constexpr int kLocalMaxExperts = 512;    // the routing kernels keep 23 words per expert in shared memory
 
 // Word offsets of the tables of one call inside its int32 workspace.  Capacities follow from the sizes alone (T * K entries in
 // at most min(E, T * K) segments padded to 128 rows), so the host never has to read the layout back.
 struct LocalLayerPlan {
     int T, K, E, H, I, keep;             // keep: tables of the backward pass too
+    int few;                             // a forward with few rows per expert: local_few.cu
     int chunks;                          // blocks of the routing kernels
     int slots_cap, blocks_cap, units_cap;
     int work_cap[2];                     // items of the forward / backward list
@@ -20,7 +22,7 @@ struct LocalLayerPlan {
     // zero-filled by local_layer_route
     long stats[2], sync[2], done1[2], done2[2], zero_words;
     // written by it
-    long meta, seg, slot_tk, slot_w, token_order, order_slot, chunk_hist, chunk_last, work[2], words;
+    long meta, seg, counts, slot_tk, slot_w, token_order, order_slot, chunk_hist, chunk_last, work[2], words;
 };
 LocalLayerPlan local_layer_plan(int T, int K, int E, int H, int I, int keep);
 
@@ -54,5 +56,7 @@ struct LocalLayerParams {
 // Routing tables and both work lists (p: plan, ws, topk_*, schedule).
 cudaError_t local_layer_route(const LocalLayerParams& p, cudaStream_t stream);
 cudaError_t local_layer_launch(const LocalLayerParams& p, cudaStream_t stream);
+// The same for plans with `few` (local_few.cu).
+cudaError_t local_few_launch(const LocalLayerParams& p, cudaStream_t stream);
 
 }  // namespace tmoe

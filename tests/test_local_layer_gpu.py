@@ -127,6 +127,36 @@ def test_loading_warps_keep_up_with_short_items(H, I):
     buf.destroy()
 
 
+@pytest.mark.parametrize("H,I", [(192, 64), (1088, 320)])         # a last tile of weights that is half outside
+def test_forward_with_few_rows_per_expert(H, I, monkeypatch):
+    """Rows per expert around the multiples of 4 (row gather), 16 (columns of the accumulator) and 64 (units); tokens without an expert;
+    more blocks than tiles and the other way round."""
+    from teramoe_b200 import engine
+    counts = [1, 3, 4, 5, 15, 16, 17, 31, 33, 47, 63, 64, 65, 127, 128, 129, 2] + [0] * 100
+    E, T = len(counts), sum(counts) + 3
+    gen = torch.Generator().manual_seed(1)
+    experts = torch.repeat_interleave(torch.arange(E), torch.tensor(counts))
+    idx = torch.full((T, 2), -1, dtype=torch.int64)
+    idx[torch.randperm(T, generator=gen)[: len(experts)], 1] = experts[torch.randperm(len(experts), generator=gen)]
+    assert idx.numel() <= 16 * E
+    prob = make_problem(1, T, H, I, E, 2, seed=8, dtype=torch.bfloat16, device="cuda", x_scale=0.1, w_scale=0.02)
+    r = prob["ranks"][0]
+    idx = idx.cuda()
+    buf = tm.Buffer(None, int(64e6), explicitly_destroy=True)
+    res = {}
+    for mode in ("0", "auto"):
+        monkeypatch.setattr(engine, "_LOCAL_LAYER_MODE", mode)
+        for name in ("_FUSED_DISPATCH_MODE", "_FUSED_MODE", "_LAYER_KERNEL_MODE"):
+            monkeypatch.setattr(engine, name, "1" if mode == "0" else "auto")
+        call = lambda i, **kw: buf.teramoe_forward(r["x"], i, r["w"], prob["W_gateup"], prob["W_down"], E, **kw)
+        res[mode] = [call(idx), call(idx, total_sms=16, num_dispatch_sms=4, num_combine_sms=4), call(idx[:, :1].expand(T, 2).contiguous())]
+    for got, want in zip(res["auto"], res["0"]):
+        assert torch.equal(got, want)
+    assert not bool(res["auto"][2].any())
+    buf.check_status()
+    buf.destroy()
+
+
 def test_native_autograd_node_keeps_its_buffer_and_fills_the_given_gradient():
     """The buffer may go out of scope before the backward pass; d(topk_weights) goes to the caller's tensor; a second derivative
     raises; a destroyed buffer raises."""
