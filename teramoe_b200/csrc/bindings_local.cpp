@@ -463,7 +463,8 @@ class LocalLayer : public std::enable_shared_from_this<LocalLayer> {
         const int64_t rows = layer_rows(p.plan);
         auto ws = torch::empty({p.plan.words}, on(x, torch::kInt32));
         auto out = torch::empty({tk.T, H}, x.options());
-        auto act = torch::empty({rows, I}, x.options());
+        // act [rows, I] and, with copies, x in slot order [rows, H]
+        auto act = torch::empty({rows * (I + (p.plan.copies[0] ? H : 0))}, x.options());
         if (kept != nullptr) {
             kept->ws = ws;
             kept->rows = torch::empty({tk.T * H + rows * 2 * I}, x.options());
@@ -474,6 +475,7 @@ class LocalLayer : public std::enable_shared_from_this<LocalLayer> {
         p.topk_idx = tk.ptr; p.idx_is64 = tk.is64; p.topk_w = topk_w.data_ptr<float>();
         p.x = x.data_ptr(); p.w_gateup = w_gateup.data_ptr(); p.w_down = w_down.data_ptr();
         p.act = act.data_ptr(); p.out = out.data_ptr();
+        if (p.plan.copies[0]) p.slot_rows = act.data_ptr<at::BFloat16>() + rows * I;
         const cudaStream_t stream = cur_stream();
         {
             std::lock_guard<std::mutex> lock(arena_mutex_);
@@ -500,12 +502,18 @@ class LocalLayer : public std::enable_shared_from_this<LocalLayer> {
         TORCH_CHECK(kept.ws.numel() == p.plan.words && kept.rows.numel() == T * H + rows * 2 * I && kept.rows.device() == grad_out.device() &&
                     kept.rows.scalar_type() == torch::kBFloat16 && kept.rows.is_contiguous() && aligned16(kept.rows),
                     "saved tensors of another call");
-        // act x route [rows, I], dGU [rows, 2I], partial sums of d(route weight): one allocation (rows and I are multiples of 64: every part
-        // starts on a 16-byte boundary)
-        auto scratch = torch::empty({rows * (3 * I + 4 * ((I + 255) / 256))}, grad_out.options());
+        // act x route [rows, I], dGU [rows, 2I], grad_out and x in slot order [rows, H] (with copies), partial sums of d(route weight): one
+        // allocation (rows and I, H are multiples of 64: every part starts on a 16-byte boundary)
+        const int64_t copied = p.plan.copies[1] ? 2 * H : 0;
+        auto scratch = torch::empty({rows * (3 * I + copied + 4 * ((I + 255) / 256))}, grad_out.options());
         auto* act_w = scratch.data_ptr<at::BFloat16>();
         auto* dgu = act_w + rows * I;
-        auto* parts = dgu + rows * 2 * I;
+        auto* slot_rows = dgu + rows * 2 * I;
+        auto* parts = slot_rows + rows * copied;
+        if (copied != 0) {
+            p.slot_rows = slot_rows;
+            p.slot_x = slot_rows + rows * H;
+        }
         auto dx = torch::empty({T, H}, grad_out.options());
         auto dw = torch::empty({T, K}, on(grad_out, torch::kFloat32));
         auto dwg = torch::empty({E, 2 * I, H}, grad_out.options());

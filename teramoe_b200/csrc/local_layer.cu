@@ -53,12 +53,13 @@ constexpr int kBoxBytes = 32 * 128;                                       // 32 
 constexpr int kEpiBytes = kEpiWarps * kBoxBytes;                          // 32 KB: one box per epilogue warp
 constexpr int kBarOffsetP = kPipeBytesP + kEpiBytes;
 constexpr int kSmemBytesP = kBarOffsetP + 512 + 1024;
-constexpr int kKeepRows = 8;                                              // rows of x a gather warp claims at a time
+constexpr int kCopyRows = 8;                                              // rows a gather warp claims at a time (divides a block)
+constexpr int kFirstRows = 1;                                             // with copies: slots every warp copies before anything else
 constexpr int kGatherWarps = 2 + kEpiWarps;                               // warps of a CTA that sum in the end
 constexpr int kLoadWarps = 4;
 constexpr int kLayerThreads = kThreads + 32 * kLoadWarps;
 // Registers per thread: 128 at launch (512 threads), which the first warpgroup keeps
-constexpr int kRegsEpilogue = 144, kRegsLoad = 96;
+constexpr int kRegsEpilogue = 136, kRegsLoad = 112;
 static_assert(128 * 128 + 256 * kRegsEpilogue + 128 * kRegsLoad <= 65536 && kThreads == 384 && kLayerThreads == 512, "register file");
 constexpr int kRingDepth = 4;
 constexpr int kSoon = 32;                                                 // looks at a barrier before its wait counts as one
@@ -70,9 +71,9 @@ static_assert(8 * (2 * kMaxStages + 4) <= (int)kOffRingFull && kOffItems + 16 * 
 static_assert(kSmemBytesP <= 232448, "shared memory");
 
 // words of the sync block
-enum { kSyncItem = 0, kSyncToken = 1, kSyncKeep = 2, kSyncFirsts = 3, kSyncWords = 8 };
+enum { kSyncItem = 0, kSyncToken = 1, kSyncCopy = 2, kSyncKeep = 3, kSyncFirsts = 4, kSyncRows = 5, kSyncWords = 8 };
 // words of the meta block
-enum { kMetaUnits = 0, kMetaWork = 2, kMetaWords = 8 };
+enum { kMetaUnits = 0, kMetaSlots = 1, kMetaWork = 2, kMetaRows = 4, kMetaWords = 8 };
 
 constexpr int kWideTiles = 74 * 4;                                        // least number of wide tiles of a GEMM (local_layer_plan)
 
@@ -201,7 +202,7 @@ __global__ void __launch_bounds__(kRouteThreads) local_route_assign_kernel(const
     }
     __syncthreads();
     if (warp == 0) {
-        int run_s = 0, run_u = 0;
+        int run_s = 0, run_u = 0, run_r = 0;
         for (int e0 = 0; e0 < E; e0 += 32) {
             const int e = e0 + lane;
             const int blocks = e < E ? (totals[e] + 127) / 128 : 0;
@@ -220,7 +221,9 @@ __global__ void __launch_bounds__(kRouteThreads) local_route_assign_kernel(const
             }
             run_s += __shfl_sync(0xffffffffu, s, 31);
             run_u += __shfl_sync(0xffffffffu, u, 31);
+            run_r += __reduce_add_sync(0xffffffffu, e < E ? (totals[e] + BK - 1) / BK * BK : 0);
         }
+        if (blockIdx.x == 0 && lane == 0) a.ws[a.p.meta + kMetaRows] = run_r;      // rows of whole 64-row steps
         if (lane == 0) {
             seg[E] = run_s;
             ub[E] = run_u;
@@ -250,7 +253,10 @@ __global__ void __launch_bounds__(kRouteThreads) local_route_assign_kernel(const
     if (blockIdx.x == 0) {
         for (int e = tid; e <= E; e += kRouteThreads) a.ws[a.p.seg + e] = seg[e];
         for (int e = tid; e < E; e += kRouteThreads) a.ws[a.p.counts + e] = totals[e];
-        if (tid == 0) meta[kMetaUnits] = U;
+        if (tid == 0) {
+            meta[kMetaUnits] = U;
+            meta[kMetaSlots] = seg[E];
+        }
     }
     for (int e = blockIdx.x; e < E; e += gridDim.x)
         for (int s = seg[e] + totals[e] + tid; s < seg[e + 1]; s += kRouteThreads) {
@@ -313,7 +319,7 @@ __global__ void __launch_bounds__(kRouteThreads) local_route_assign_kernel(const
                 const int e = j / per, r = j - e * per, m_blk = r / nb;
                 if (items + i < cap)
                     work[items + i] = make_int4((down ? kWorkWgradDown : kWorkWgradGateup) | (e << 8), seg[e], (r - m_blk * nb) | (m_blk << 16),
-                                         (totals[e] + BK - 1) / BK);       // blocks of padding add nothing
+                                         (totals[e] + UK - 1) / UK);       // (in 16 rows: padding adds nothing)
             }
         }
         if (gtid == 0) meta[kMetaWork + dir] = min(items + (dir == 1 ? E * per_e : 0), cap);
@@ -376,7 +382,7 @@ __global__ void __launch_bounds__(kRouteThreads) local_route_assign_kernel(const
 struct Phase {
     alignas(64) CUtensorMap map_a;
     alignas(64) CUtensorMap map_b;
-    alignas(64) CUtensorMap map_a32;     // second GEMM: 32 rows of A
+    alignas(64) CUtensorMap map_a32;     // the two GEMMs: 32 rows of A
     int nk, b_group_rows, cols, num_n_blocks, n_total, m_total;      // num_n_blocks: of the two GEMMs
 };
 
@@ -392,6 +398,8 @@ struct LayerArgsP {
     const uint8_t* x;                    // [T, H]: forward x, backward grad_out
     const __nv_bfloat16* y;
     __nv_bfloat16* saved_x;              // [T, H]: written by forward (may be null), read by backward
+    uint8_t* slot_rows;                  // without loading warps: x in slot order
+    uint8_t* slot_x;                     // the same, backward: saved_x in slot order
     __nv_bfloat16* out;
     __nv_bfloat16* preact;               // forward (with keep): written, backward: read; preact_at()
     float* droute_part;
@@ -407,6 +415,7 @@ struct LayerArgsP {
     int* sync;
     int* done1;                          // per unit: epilogue warps that finished a tile of the first GEMM
     int* done2;                          // per 128-row block: the same for the second GEMM
+    int* arrived;                        // without loading warps, per 128-row block: rows of slot_rows in place
     unsigned long long* stats;
     int* status;
 };
@@ -428,6 +437,18 @@ __device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t a, uint32_t
 __device__ __forceinline__ void ld_shared_v4(uint32_t addr, uint32_t (&v)[4]) {
     asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(addr) : "memory");
 }
+// Warp-wide row copy with 16 loads in flight per lane (8 KB per warp): two warps per SM have to keep HBM busy.
+__device__ __forceinline__ void copy_row_deep(int4* dst, const int4* src, int nvec, int lane) {
+    for (int b = 0; b < nvec; b += 512) {
+        int4 v[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = ld_nc_v4(src + min(b + 32 * i + lane, nvec - 1));
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+            if (b + 32 * i + lane < nvec) dst[b + 32 * i + lane] = v[i];
+    }
+}
+
 // 16 bytes from memory into shared memory, or zeros
 __device__ __forceinline__ void cp_async_16_or_zeros(uint32_t dst_smem, const void* src, bool wanted) {
     asm volatile("cp.async.cg.shared.global.L2::256B [%0], [%1], 16, %2;" ::"r"(dst_smem), "l"(src), "r"(wanted ? 16 : 0) : "memory");
@@ -447,7 +468,7 @@ __device__ __forceinline__ void registers_dec() {
 }
 
 struct Item {
-    int kind, n0, halves, group, k0, nk, m0, unit, need, real;      // columns n0 .. n0 + 256 * halves; `real` of the `need` rows are not padding
+    int kind, n0, halves, group, k0, nk, tail, m0, unit, need, real;      // columns n0 .. n0 + 256 * halves; `real` of the `need` rows are not padding; tail: 16-row slices of the last step
     bool live;          // this CTA's 128 rows are real
     int m_in_group;     // weight gradients: first row of dW inside the expert
 };
@@ -467,6 +488,7 @@ __device__ __forceinline__ void decode_item(const LayerArgsP& L, const int4& it,
         q.m0 = (it.w + (int)rank) * BM;
         q.k0 = 0;
         q.nk = P.nk;
+        q.tail = BK / UK;
         q.m_in_group = 0;
     } else {
         q.unit = -1;
@@ -475,7 +497,8 @@ __device__ __forceinline__ void decode_item(const LayerArgsP& L, const int4& it,
         q.m_in_group = ((it.z >> 16) * 2 + (int)rank) * BM;
         q.m0 = q.m_in_group;
         q.k0 = it.y;
-        q.nk = it.w;
+        q.nk = (it.w + BK / UK - 1) / (BK / UK);
+        q.tail = it.w - (q.nk - 1) * (BK / UK);
     }
 }
 
@@ -678,8 +701,10 @@ __device__ __forceinline__ void epilogue_plain(const Staging& st, uint32_t taddr
     }
 }
 
-template <bool BWD>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kLayerThreads, 1)
+// ROWS: the loading warps bring what is made of token rows.  Without them (where local_layer_plan says so) rows are copied into slot order by
+// the other warps first, and TMA loads them from there.
+template <bool BWD, bool ROWS>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(ROWS ? kLayerThreads : kThreads, 1)
 local_layer_kernel(const __grid_constant__ LayerArgsP L) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -701,7 +726,7 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
     if (threadIdx.x == 0) {
         *abort_flag = 0u;
         for (int s = 0; s < kMaxStages; ++s) {
-            mbar_init(full_bar(s), 4);                       // of each CTA the producer and a loading warp
+            mbar_init(full_bar(s), ROWS ? 4 : 2);            // of each CTA the producer and a loading warp
             mbar_init(empty_bar(s), 1);
         }
         for (int s = 0; s < 2; ++s) {
@@ -710,13 +735,13 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
         }
         for (int e = 0; e < kRingDepth; ++e) {
             mbar_init(ring_full(e), 1);
-            mbar_init(ring_empty(e), kRingConsumers);
+            mbar_init(ring_empty(e), ROWS ? kRingConsumers : kRingConsumers - 2 * kLoadWarps);
         }
         fence_mbar_init();
 #pragma unroll
         for (int p = 0; p < (BWD ? 4 : 2); ++p) {
-            if (p != kWorkGemm1 && p != kWorkWgradDown) tma_prefetch_desc(&L.ph[p].map_a);
-            if (p != kWorkWgradGateup) tma_prefetch_desc(&L.ph[p].map_b);
+            if (!ROWS || (p != kWorkGemm1 && p != kWorkWgradDown)) tma_prefetch_desc(&L.ph[p].map_a);
+            if (!ROWS || p != kWorkWgradGateup) tma_prefetch_desc(&L.ph[p].map_b);
         }
     }
     // With few rows per expert most rows of A are never loaded.  Zeros there cost the tensor cores least power; what an earlier kernel left in
@@ -724,7 +749,7 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
     // 8 rows per expert 623 / 547 us, 32 641 / 573, 64 661 / 616.  Above, an expert's rows begin to be loaded 128 at a time; zeros would
     // still gain there (96 684 / 637, 128 702 / 662).
     if ((long)L.T * L.K <= 64l * L.E) {
-        for (int i = threadIdx.x; i < L.stages * (kAStageBytes / 16); i += kLayerThreads) {
+        for (int i = threadIdx.x; i < L.stages * (kAStageBytes / 16); i += (int)blockDim.x) {
             const int st = i / (kAStageBytes / 16);
             *reinterpret_cast<int4*>(smem_gen + st * L.stage_bytes + (i - st * (kAStageBytes / 16)) * 16) = make_int4(0, 0, 0, 0);
         }
@@ -739,16 +764,102 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
     const int target1 = 2 * kEpiWarps * L.ph[0].num_n_blocks;         // epilogue warps that finish a unit's first GEMM,
     const int target2 = kEpiWarps * L.ph[1].num_n_blocks;             // a block's second GEMM
 
-    // ---------------------------------------------------------------------- backward's copy of x
     const int nvec = L.H / 8;
+    // ---------------------------------------------------------------------- copy role (without loading warps)
+    // Rows into slot order.  All warps but the producer's and the issuer's start with one slot each, so that the first units are in place
+    // after the latency of one row; the rest is claimed by the gather warps, eight slots at a time.  A warp has 8 KB of loads in
+    // flight: rows of 4096 columns and more one after the other, shorter ones several at once.  (Before, the first pairs of CTAs
+    // streamed rows through shared memory and joined the GEMMs afterwards; rows of 1 KB left them waiting for one row at a time:
+    // 8531 tokens, H=512, top-8 spent 240 us there.)
+    auto copy_slots = [&](const int4* src, int4* dst, int row, uint32_t wanted, int s0, int n) {
+        // row: source row of slot s0 + lane, -1 = zeros
+        if (nvec >= 512) {
+            for (int r = 0; r < n; ++r) {
+                if (!((wanted >> r) & 1u)) continue;
+                const int sr = __shfl_sync(0xffffffffu, row, r);
+                int4* d = dst + (long)(s0 + r) * nvec;
+                if (sr >= 0) copy_row_deep(d, src + (long)sr * nvec, nvec, lane);
+                else for (int i = lane; i < nvec; i += 32) d[i] = make_int4(0, 0, 0, 0);
+            }
+            return;
+        }
+        const int total = n * nvec;
+        for (int b = 0; b < total; b += 512) {
+            int4 v[16];
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+                const int idx = min(b + 32 * i + lane, total - 1), r = idx / nvec;
+                const int sr = __shfl_sync(0xffffffffu, row, r);
+                v[i] = ld_nc_v4(src + (long)max(sr, 0) * nvec + (idx - r * nvec));
+                if (sr < 0) v[i] = make_int4(0, 0, 0, 0);
+            }
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+                const int idx = b + 32 * i + lane;
+                if (idx < total && ((wanted >> (idx / nvec)) & 1u)) dst[(long)s0 * nvec + idx] = v[i];
+            }
+        }
+    };
+    auto count_rows = [&](int* counter, int n) {
+        __syncwarp();
+        if (lane == 0 && n > 0) {
+            fence_acq_rel_gpu();
+            red_add_gpu(counter, n);
+        }
+    };
+    auto place = [&](int s0, int n) {
+        const int tk = lane < n ? L.slot_tk[s0 + lane] : -1;
+        const int row = tk >= 0 ? tk / L.K : -1;
+        uint32_t wanted = __ballot_sync(0xffffffffu, tk >= 0);
+        if constexpr (BWD) {
+            // both slot-order tables are operands of the weight gradients, which sum over 64 rows at a time: rows of zeros to the next 64
+            wanted = L.slot_tk[s0 & ~63] >= 0 ? (1u << n) - 1u : 0u;
+        }
+        if (wanted == 0u) return;
+        copy_slots(reinterpret_cast<const int4*>(L.x), reinterpret_cast<int4*>(L.slot_rows), row, wanted, s0, n);
+        count_rows(L.arrived + (s0 >> 7), __popc(wanted));
+    };
+    auto place_x = [&](int s0, int n) {
+        const int tk = lane < n ? L.slot_tk[s0 + lane] : -1;
+        if (L.slot_tk[s0 & ~63] < 0) return;
+        copy_slots(reinterpret_cast<const int4*>(L.saved_x), reinterpret_cast<int4*>(L.slot_x), tk >= 0 ? tk / L.K : -1, (1u << n) - 1u, s0, n);
+        count_rows(L.sync + kSyncRows, n);
+    };
+    const int num_slots = L.meta[kMetaSlots];
+    // (neighbouring slots go to different SMs: a few rows in one SM would queue behind one another)
+    const int first_slots = (int)gridDim.x * kGatherWarps * kFirstRows / kCopyRows * kCopyRows;
+    if (!ROWS && warp >= 2) {
+        const int s0 = ((warp - 2) * (int)gridDim.x + (int)blockIdx.x) * kFirstRows;
+        if (s0 < min(num_slots, first_slots)) place(s0, kFirstRows);
+    }
+    auto copy_loop = [&]() {
+        while (true) {
+            int s0 = 0;
+            if (lane == 0) s0 = first_slots + atomicAdd(L.sync + kSyncCopy, kCopyRows);
+            s0 = __shfl_sync(0xffffffffu, s0, 0);
+            if (s0 >= num_slots) break;
+            place(s0, kCopyRows);
+        }
+    };
+    auto copy_x_loop = [&]() {
+        // backward: x in slot order, which nothing needs before the weight gradients
+        while (true) {
+            int s0 = 0;
+            if (lane == 0) s0 = atomicAdd(L.sync + kSyncKeep, kCopyRows);
+            s0 = __shfl_sync(0xffffffffu, s0, 0);
+            if (s0 >= num_slots) break;
+            place_x(s0, kCopyRows);
+        }
+    };
+    // ---------------------------------------------------------------------- forward: backward's copy of x
     auto keep_x_loop = [&]() {
         // 4 KB of loads in flight per warp
         while (true) {
             int t0 = 0;
-            if (lane == 0) t0 = atomicAdd(L.sync + kSyncKeep, kKeepRows);
+            if (lane == 0) t0 = atomicAdd(L.sync + kSyncKeep, kCopyRows);
             t0 = __shfl_sync(0xffffffffu, t0, 0);
             if (t0 >= L.T) break;
-            const long first = (long)t0 * nvec, total = (long)min(kKeepRows, L.T - t0) * nvec;
+            const long first = (long)t0 * nvec, total = (long)min(kCopyRows, L.T - t0) * nvec;
             const int4* src = reinterpret_cast<const int4*>(L.x) + first;
             int4* dst = reinterpret_cast<int4*>(L.saved_x) + first;
             for (long b = lane; b < total; b += 256) {
@@ -763,31 +874,33 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
     };
 
     // ---------------------------------------------------------------------- gather role
-    // Rows [k0, k0 + n) of a token's entries, columns v and v + 32: all loads are issued before the first is used (16 in flight
-    // per lane; a load behind a lane-dependent branch would be waited for one at a time, so out-of-range columns are clamped
-    // and only their stores are left out).
-    auto add_rows = [&](const int (&slots)[8], int n, uint32_t valid, int v0, int v1, float (&a0)[8], float (&a1)[8]) {
-        int4 r0[8], r1[8];
+    // Rows [k0, k0 + n) of a token's entries, kVecs pieces of 16 bytes of each per lane, 32 pieces apart: all loads are issued before the
+    // first is used (8 kVecs in flight per lane; a load behind a lane-dependent branch would be waited for one at a time, so
+    // out-of-range columns are clamped and only their stores are left out).  Backward with loading warps, where the sums run under the weight
+    // gradients, one piece: with two the registers do not suffice, and what is spilled then costs 5 %.
+    constexpr int kVecs = BWD && ROWS ? 1 : 2;
+    auto add_rows = [&](const int (&slots)[8], int n, uint32_t valid, const int (&at)[kVecs], float (&sum)[kVecs][8]) {
+        int4 r[kVecs][8];
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             if (j < n) {
                 const int4* row = reinterpret_cast<const int4*>(L.y) + (long)slots[j] * nvec;
-                r0[j] = ld_cg_v4_ordered(row + v0);
-                r1[j] = ld_cg_v4_ordered(row + v1);
+#pragma unroll
+                for (int v = 0; v < kVecs; ++v) r[v][j] = ld_cg_v4_ordered(row + at[v]);
             }
         }
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             if (j < n && ((valid >> j) & 1u)) {
-                const uint32_t p0[4] = {(uint32_t)r0[j].x, (uint32_t)r0[j].y, (uint32_t)r0[j].z, (uint32_t)r0[j].w};
-                const uint32_t p1[4] = {(uint32_t)r1[j].x, (uint32_t)r1[j].y, (uint32_t)r1[j].z, (uint32_t)r1[j].w};
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const float2 f0 = unpack_bf16x2(p0[i]), f1 = unpack_bf16x2(p1[i]);
-                    a0[2 * i] += f0.x;
-                    a0[2 * i + 1] += f0.y;
-                    a1[2 * i] += f1.x;
-                    a1[2 * i + 1] += f1.y;
+                for (int v = 0; v < kVecs; ++v) {
+                    const uint32_t p[4] = {(uint32_t)r[v][j].x, (uint32_t)r[v][j].y, (uint32_t)r[v][j].z, (uint32_t)r[v][j].w};
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const float2 f = unpack_bf16x2(p[i]);
+                        sum[v][2 * i] += f.x;
+                        sum[v][2 * i + 1] += f.y;
+                    }
                 }
             }
         }
@@ -797,7 +910,7 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
         // is as long as the last tasks: about eleven for each of the 1480 warps that take part by then, down to 512 columns.
         // The order of a sum (k ascending) does not depend on it.
         const int K = L.K;
-        const int steps = (nvec + 63) / 64;
+        const int steps = (nvec + 32 * kVecs - 1) / (32 * kVecs);
         const int parts = max(1, min(steps, kGatherTasks / max(L.T, 1)));
         const int part_steps = (steps + parts - 1) / parts;
         const int tasks = L.T * parts;
@@ -857,22 +970,25 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
             int4* dst = reinterpret_cast<int4*>(L.out + (long)t * L.H);
             const int step1 = min(steps, (part + 1) * part_steps);
             for (int step = part * part_steps; step < step1; ++step) {
-                const int c0 = step * 64 + lane, c1 = c0 + 32;
-                const int v0 = min(c0, nvec - 1), v1 = min(c1, nvec - 1);
-                float a0[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-                float a1[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+                int at[kVecs];
+                float sum[kVecs][8];
+#pragma unroll
+                for (int v = 0; v < kVecs; ++v) {
+                    at[v] = min((step * kVecs + v) * 32 + lane, nvec - 1);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) sum[v][i] = 0.f;
+                }
                 for (int k0 = 0; k0 < K; k0 += 8) {
                     int sl[8];
 #pragma unroll
                     for (int j = 0; j < 8; ++j) sl[j] = max(0, __shfl_sync(0xffffffffu, slot, (k0 + j) & 31));
-                    add_rows(sl, min(K - k0, 8), valid >> k0, v0, v1, a0, a1);
+                    add_rows(sl, min(K - k0, 8), valid >> k0, at, sum);
                 }
-                if (c0 < nvec)
-                    dst[c0] = make_int4((int)pack_bf16x2(a0[0], a0[1]), (int)pack_bf16x2(a0[2], a0[3]), (int)pack_bf16x2(a0[4], a0[5]),
-                                        (int)pack_bf16x2(a0[6], a0[7]));
-                if (c1 < nvec)
-                    dst[c1] = make_int4((int)pack_bf16x2(a1[0], a1[1]), (int)pack_bf16x2(a1[2], a1[3]), (int)pack_bf16x2(a1[4], a1[5]),
-                                        (int)pack_bf16x2(a1[6], a1[7]));
+#pragma unroll
+                for (int v = 0; v < kVecs; ++v)
+                    if ((step * kVecs + v) * 32 + lane < nvec)
+                        dst[at[v]] = make_int4((int)pack_bf16x2(sum[v][0], sum[v][1]), (int)pack_bf16x2(sum[v][2], sum[v][3]),
+                                               (int)pack_bf16x2(sum[v][4], sum[v][5]), (int)pack_bf16x2(sum[v][6], sum[v][7]));
             }
         }
         if (stamps) {
@@ -913,7 +1029,7 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
         // A warp takes every fourth step: it waits for the stage, copies, and hands the step over when its copies have landed, which it sees to
         // behind the copies of its next step if that one's stage is free, so that copies into all stages are under way at a time.
         // All four warps on every step, two steps under way, were 4 % slower; an address computed per column block instead of per
-        // row made dW_gateup 25 % slower; registers for fewer addresses (56 instead of 96 per thread, some spilled) cost 5 %.
+        // row made dW_gateup 25 % slower; registers for fewer addresses (56 instead of 112 per thread, some spilled) cost 5 %.
         auto load_rows = [&]() {
             const int sub = lane >> 3, chunk = lane & 7;
             const uint32_t pair_full = mapa_shared(full_bar(0), 0);
@@ -992,13 +1108,18 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                                 in[a] = col < L.H;
                                 at_col[a] = in[a] ? col * 2 : 0;
                             }
+                            const int slices = step == q.nk - 1 ? q.tail : BK / UK;
+#pragma unroll 1
+                            for (int k = 0; k < slices; ++k) {       // 16 rows
+                                const int rows = k < 2 ? tok[0] : tok[1];
 #pragma unroll
-                            for (int j = 0; j < 16; ++j) {
-                                const int t = __shfl_sync(0xffffffffu, tok[j >> 3], (4 * j + sub) & 31);
-                                const uint8_t* from = src + max(t, 0) * pitch;
-                                const uint32_t to = dst + (down ? 0 : kAStageBytes) + j * 512 + at[j & 1];
+                                for (int j = 0; j < 4; ++j) {
+                                    const int t = __shfl_sync(0xffffffffu, rows, (16 * k + 4 * j + sub) & 31);
+                                    const uint8_t* from = src + max(t, 0) * pitch;
+                                    const uint32_t to = dst + (down ? 0 : kAStageBytes) + (4 * k + j) * 512 + at[j & 1];
 #pragma unroll
-                                for (int a = 0; a < kAtoms; ++a) cp_async_16_or_zeros(to + a * kAtomBytes, from + at_col[a], in[a] && t >= 0);
+                                    for (int a = 0; a < kAtoms; ++a) cp_async_16_or_zeros(to + a * kAtomBytes, from + at_col[a], in[a] && t >= 0);
+                                }
                             }
                         };
                         if (down || q.halves == 1) copy(std::integral_constant<int, 2>());
@@ -1025,7 +1146,7 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
             settle();
         };
 
-        if (warp >= 12) {
+        if (ROWS && warp >= 12) {
             registers_dec<kRegsLoad>();
             load_rows();
         } else if (warp < 4) {
@@ -1043,7 +1164,7 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                 // Both producers look at the NEXT item while the loads of the current one are in flight: they fetch it and test what
                 // its operands wait for, so that between two items there is normally nothing to wait for.
                 int claim = (rank == 0) ? atomicAdd(L.sync + kSyncItem, 1) : 0;
-                unsigned long long w_unit = 0, w_wgrad = 0;
+                unsigned long long w_arrive = 0, w_unit = 0, w_wgrad = 0;
                 bool wgrad_ready = false, wgrad_fenced = false;
                 int4 cur = make_int4(-1, 0, 0, 0), nxt = cur;
                 bool have = false, nxt_ready = false;
@@ -1080,12 +1201,13 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                 };
                 // what the operands of an item wait for; `block`: wait (bounded) instead of only looking
                 auto operands_ready = [&](const Item& q, bool block) -> int {
-                    if (q.kind == kWorkGemm1) return 1;
+                    if (q.kind == kWorkGemm1) return (ROWS || !q.live || q.need == 0) ? 1 : counted(L.arrived + q.m0 / BM, q.need, block, 600, w_arrive);
                     if (q.kind == kWorkGemm2) return counted(L.done1 + q.unit, target1, block, 601, w_unit);
                     // the weight gradients sit behind all first GEMMs in the list: one check per pair is enough (two loads per expert and pair
                     // would cost as much as the smallest of these items)
                     if (wgrad_ready) return 1;
-                    const int r = counted(L.sync + kSyncFirsts, L.meta[kMetaUnits] * target1, block, 602, w_wgrad);
+                    int r = counted(L.sync + kSyncFirsts, L.meta[kMetaUnits] * target1, block, 602, w_wgrad);
+                    if (!ROWS && r == 1) r = counted(L.sync + kSyncRows, L.meta[kMetaRows], block, 603, w_wgrad);
                     wgrad_ready = r == 1;
                     return r;
                 };
@@ -1118,13 +1240,13 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                     const Phase& P = L.ph[q.kind];
                     const bool gemm = q.kind <= kWorkGemm2;
                     const int n0 = q.n0 + (int)rank * (BN / 2);
-                    // Second GEMM, rows of A that a CTA loads: none that nothing is summed from, up to 64 in boxes of 32.  What a stage holds in
-                    // the others is multiplied into accumulator rows that no epilogue reads.  What is made of token rows comes from the
-                    // loading warps: A of the first GEMM and of dW_down, B of dW_gateup.
+                    // The two GEMMs, rows of A that a CTA loads: none that nothing is summed from, up to 64 in boxes of 32.  What a stage holds in
+                    // the others is multiplied into accumulator rows that no epilogue reads.  What is made of token rows may come from
+                    // the loading warps: A of the first GEMM and of dW_down, B of dW_gateup.
                     const int a_rows = rows_loaded(q.need);
-                    const int a_pair = q.kind == kWorkGemm2 ? rows_loaded((cur.z >> 16) & 0xff) + rows_loaded((cur.z >> 24) & 0xff)
-                                                            : (q.kind == kWorkWgradGateup ? 2 * BM : 0);
-                    const uint32_t tx = (uint32_t)(a_pair * (BK * 2) + (q.kind == kWorkWgradGateup ? 0 : 2 * q.halves * kBHalfBytesP));
+                    const bool rows_a = ROWS && (q.kind == kWorkGemm1 || q.kind == kWorkWgradDown), rows_b = ROWS && q.kind == kWorkWgradGateup;
+                    const int a_pair = rows_a ? 0 : (gemm ? rows_loaded((cur.z >> 16) & 0xff) + rows_loaded((cur.z >> 24) & 0xff) : 2 * BM);
+                    const uint32_t tx = (uint32_t)(a_pair * (BK * 2) + (rows_b ? 0 : 2 * q.halves * kBHalfBytesP));
                     const int look_kb = min(stages - 1, q.nk - 1);     // all stages are in flight: a pause of this thread costs nothing
                     auto take_stage = [&](int st, uint32_t ph) {
                         if (!mbar_wait(empty_bar(st), ph ^ 1u, abort_flag, L.status, 610)) return false;
@@ -1135,7 +1257,7 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                     const CUtensorMap* map_b = &P.map_b;
                     const int b_row = q.group * P.b_group_rows;
                     auto load_b = [&](int st, int k) {
-                        if (q.kind == kWorkWgradGateup) return;
+                        if (rows_b) return;
                         const uint32_t dst = smem_base + (uint32_t)st * stage_bytes + kAStageBytes, bar = pair_full + 8u * st;
                         for (int h = 0; h < q.halves; ++h) {
                             if (!BWD) tma_load_2d_2cta(dst + h * kBHalfBytesP, map_b, bar, k, b_row + n0 + h * BN);
@@ -1174,7 +1296,7 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                         }
                         return true;
                     };
-                    if (q.kind == kWorkGemm1 || q.kind == kWorkWgradDown) {
+                    if (rows_a) {
                         ok = load_steps([](uint32_t, uint32_t, int) {});
                     } else if (gemm) {
                         const CUtensorMap* map_a = a_rows == BM ? &P.map_a : &P.map_a32;
@@ -1193,6 +1315,7 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                     for (const uint64_t t0 = globaltimer_ns(); globaltimer_ns() - t0 < 10000000ull;) __nanosleep(1000);
                 }
                 if (L.stats != nullptr) {
+                    if (w_arrive) atomicAdd(L.stats + kStatWaitArrival, w_arrive);
                     if (w_unit) atomicAdd(L.stats + kStatWaitFirstGemm, w_unit);
                     if (w_wgrad) atomicAdd(L.stats + kStatWaitWgrad, w_wgrad);
                 }
@@ -1221,13 +1344,14 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                 const uint64_t b_base = make_smem_desc_sw128(smem_base + kAStageBytes, BWD ? kAtomBytes : 0, 1024);
                 const uint32_t a_step = (a_mn ? UK * 128 : UK * 2) >> 4, b_step = (BWD ? UK * 128 : UK * 2) >> 4;
                 // 64 columns of K of one half of the tile
-                auto multiply = [&](int s, int h, int slot, bool first) {
+                auto multiply = [&](int s, int h, int slot, int kb) {
                     const uint32_t off = (uint32_t)(s * L.stage_bytes) >> 4;
                     const uint64_t a_desc = a_base + off, b_desc = b_base + off + (uint32_t)(h * (kBHalfBytesP >> 4));
                     const uint32_t d_tmem = tmem_base + (uint32_t)(slot * BN);
+                    const int slices = BWD && kb == q.nk - 1 ? q.tail : BK / UK;
 #pragma unroll
                     for (int k = 0; k < BK / UK; ++k)
-                        umma_bf16_ss_2cta(d_tmem, a_desc + k * a_step, b_desc + k * b_step, idesc, (!first || k > 0) ? 1u : 0u);
+                        if (k < slices) umma_bf16_ss_2cta(d_tmem, a_desc + k * a_step, b_desc + k * b_step, idesc, (kb | k) != 0 ? 1u : 0u);
                 };
                 if (!mbar_wait(tempty_bar(slot0), parity0, abort_flag, L.status, 620)) { ok = false; break; }
                 tcgen05_fence_after();
@@ -1242,7 +1366,7 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                         if (!mbar_wait(full_bar(s), ph, abort_flag, L.status, 621)) { ok = false; break; }
                         tcgen05_fence_after();
                         if (elect_one()) {
-                            multiply(s, 0, slot0, i == 0);
+                            multiply(s, 0, slot0, i);
                             if (i == q.nk - 1) umma_commit_2cta(tfull_bar(slot0), 3u);
                         }
                         __syncwarp();
@@ -1252,7 +1376,7 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                     tcgen05_fence_after();
                     for (; kb < lead; ++kb) {
                         if (elect_one()) {
-                            multiply(stage, 1, slot1, kb == 0);
+                            multiply(stage, 1, slot1, kb);
                             umma_commit_2cta(empty_bar(stage), 3u);
                             if (kb == q.nk - 1) umma_commit_2cta(tfull_bar(slot1), 3u);
                         }
@@ -1265,10 +1389,10 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                     tcgen05_fence_after();
                     if (elect_one()) {
                         const bool last = kb == q.nk - 1;
-                        multiply(stage, 0, slot0, kb == 0);
+                        multiply(stage, 0, slot0, kb);
                         if (q.halves == 2) {
                             if (last) umma_commit_2cta(tfull_bar(slot0), 3u);
-                            multiply(stage, 1, slot1, false);
+                            multiply(stage, 1, slot1, kb);
                         }
                         umma_commit_2cta(empty_bar(stage), 3u);
                         if (last) umma_commit_2cta(tfull_bar(q.halves == 2 ? slot1 : slot0), 3u);
@@ -1285,12 +1409,14 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                 }
             }
         } else if (warp >= 2) {
+            if constexpr (!ROWS) copy_loop();
+            if constexpr (BWD && !ROWS) copy_x_loop();
             if (!BWD && L.saved_x != nullptr) keep_x_loop();
             gather_loop();
         }
         } else {
             // -------------------------------------------------------------- epilogue, then gather
-            registers_inc<kRegsEpilogue>();
+            if constexpr (ROWS) registers_inc<kRegsEpilogue>();
             const int qd = warp & 3;
             const int hh = (warp - 4) >> 2;
             const Staging st{smem_base + kPipeBytesP + (uint32_t)(warp - 4) * kBoxBytes, lane};
@@ -1469,14 +1595,14 @@ cudaError_t make_store_map3(CUtensorMap* map, const void* base, uint64_t groups,
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
-template <bool BWD>
+template <bool BWD, bool ROWS>
 cudaError_t launch(const LayerArgsP& L, int num_sms, cudaStream_t stream) {
-    auto kern = local_layer_kernel<BWD>;
+    auto kern = local_layer_kernel<BWD, ROWS>;
     static bool configured[64] = {};
     if (cudaError_t e = ensure_smem_limit(kern, kSmemBytesP, configured); e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(num_sms & ~1);
-    cfg.blockDim = dim3(kLayerThreads);
+    cfg.blockDim = dim3(ROWS ? kLayerThreads : kThreads);
     cfg.dynamicSmemBytes = kSmemBytesP;
     cfg.stream = stream;
     // every pair waits for rows that warps of all blocks copy and for tiles of other pairs: all of them have to be resident
@@ -1498,6 +1624,17 @@ LocalLayerPlan local_layer_plan(int T, int K, int E, int H, int I, int keep) {
     p.blocks_cap = (int)((entries + 127 * segs) / 128);
     p.slots_cap = p.blocks_cap * 128;
     p.units_cap = (int)((p.blocks_cap + segs) / 2);
+    const int rows = (int)(entries / (segs > 0 ? segs : 1));
+    // Token rows through the loading warps, or copied into slot order first.  The loading warps load a row again for every tile of the other
+    // operand, with more energy per byte than TMA; a copy is written and read once.  ms of a step, backward by loaders / by copies: 2048
+    // tokens, H=7168 I=512, 32 experts, top-8 (512 rows per expert) 1.41 / 1.73; 2048, H=2048 I=256, 32, top-6 (384 rows) 0.263 / 0.322;
+    // 8192, H=2048 I=3072, 16, top-6 (3072) 4.89 / 4.97; 8192, H=7168 I=2048 (2048) 14.66 to 14.95 / 14.83 to 14.86; 4096, H=5120 I=1536,
+    // 16, top-2 (512) 1.412 / 1.392; 2048, H=4096 I=768, 32, top-4 (256) 0.840 / 0.817; 512, H=7168 I=2048 (128) 2.416 / 2.204; 64 of them
+    // (16) 1.969 / 1.757.  I = 14336 (H=4096, 8 experts, 4096 tokens, top-2), loaders in both directions, in the forward alone, in none:
+    // 7.85, 7.94, 7.68.
+    const bool large_i = I >= 4096;
+    p.copies[0] = large_i;
+    p.copies[1] = keep && (large_i || 2 * rows < I);
     // Few rows per expert, forward only: weights as the M operand (local_few.cu).  us, here / there (32 experts, top-8, H=7168 I=2048; I=512), by
     // rows per expert: 1 368 / 279, 8 577 / 441, 16 589 / 471; 184 / 151, 24 600 / 522; 191 / 172, 32 615 / 566; 200 / 194.  Skewed routing
     // (hottest expert 2.5 times the mean) at 20: 603 / 528; 189 / 186, and with the hottest 5 times the mean 606 / 538; 189 / 221 (at 16:
@@ -1521,7 +1658,6 @@ LocalLayerPlan local_layer_plan(int T, int K, int E, int H, int I, int keep) {
         return n >= 2 * BN && k >= min_k && row_units * column_blocks(n, 2 * BN) >= kWideTiles ? 2 * BN : BN;
     };
     const long units = entries / (2 * BM);
-    const int rows = (int)(entries / (segs > 0 ? segs : 1));
     p.cols[0][0] = columns(2 * I, units, H, 2048);
     p.cols[0][1] = columns(H, units, I, 1024);
     p.cols[1][0] = columns(I, units, H, 2048);
@@ -1543,6 +1679,7 @@ LocalLayerPlan local_layer_plan(int T, int K, int E, int H, int I, int keep) {
         p.stats[d] = take(2 * kLayerStatWords);
         p.sync[d] = take(kSyncWords);
         p.done1[d] = take(p.few ? 128 / kFewUnitRows * p.blocks_cap : p.units_cap);
+        p.arrived[d] = take(p.copies[d] ? p.blocks_cap : 0);
         p.done2[d] = take(p.few ? 128 / kFewUnitRows * p.blocks_cap : p.blocks_cap);
     }
     p.zero_words = at;
@@ -1606,6 +1743,8 @@ cudaError_t local_layer_launch(const LocalLayerParams& q, cudaStream_t stream) {
     g1.nk = H / BK;
     g1.cols = p.cols[dir][0];
     g2.n_total = H; g2.cols = p.cols[dir][1]; g2.num_n_blocks = column_blocks(H, g2.cols);
+    const bool copies = p.copies[dir] != 0;
+    if (copies && ((e = make_map(&g1.map_a, q.slot_rows, R, H, BK, BM)) != cudaSuccess || (e = make_map(&g1.map_a32, q.slot_rows, R, H, BK, 32)) != cudaSuccess)) return e;
     if (q.bwd && (e = make_map_narrow(&L.st_aux, q.aux, R, 2 * I)) != cudaSuccess) return e;
     if ((e = q.bwd ? make_map_narrow(&L.st_act, q.act, R, I) : make_map(&L.st_act, q.act, R, I, 64, 32)) != cudaSuccess) return e;
     if ((e = make_map(&L.st_y, q.y, R, H, 64, 32)) != cudaSuccess) return e;
@@ -1626,8 +1765,10 @@ cudaError_t local_layer_launch(const LocalLayerParams& q, cudaStream_t stream) {
         // dW_down[e] = dY[seg]^T . act_w[seg]  ([H, I]);  dW_gateup[e] = dGU[seg]^T . X[seg]  ([2I, H])
         Phase& gd = L.ph[kWorkWgradDown];
         Phase& gg = L.ph[kWorkWgradGateup];
+        if (copies && (e = make_map_mn(&gd.map_a, q.slot_rows, R, H)) != cudaSuccess) return e;
         if ((e = make_map_mn(&gd.map_b, q.act, R, I)) != cudaSuccess) return e;
         if ((e = make_map_mn(&gg.map_a, q.aux, R, 2 * I)) != cudaSuccess) return e;
+        if (copies && (e = make_map_mn(&gg.map_b, q.slot_x, R, H)) != cudaSuccess) return e;
         gd.m_total = H; gd.n_total = I; gd.cols = p.cols[1][2];
         gg.m_total = 2 * I; gg.n_total = H; gg.cols = p.cols[1][3];
         if ((e = make_store_map3(&L.st_dwd, q.dw_down, E, H, I)) != cudaSuccess) return e;
@@ -1638,6 +1779,9 @@ cudaError_t local_layer_launch(const LocalLayerParams& q, cudaStream_t stream) {
     L.x = static_cast<const uint8_t*>(q.x);
     L.y = static_cast<const __nv_bfloat16*>(q.y);
     L.saved_x = static_cast<__nv_bfloat16*>(q.saved_x);
+    L.slot_rows = static_cast<uint8_t*>(q.slot_rows);
+    L.slot_x = static_cast<uint8_t*>(q.slot_x);
+    L.arrived = q.ws + p.arrived[dir];
     L.out = static_cast<__nv_bfloat16*>(q.out);
     L.preact = static_cast<__nv_bfloat16*>(q.preact);
     L.droute_part = q.droute_part;
@@ -1661,7 +1805,8 @@ cudaError_t local_layer_launch(const LocalLayerParams& q, cudaStream_t stream) {
     for (int k = 0; k < (q.bwd ? 4 : 2); ++k) wide |= L.ph[k].cols > BN;
     L.stages = wide ? 4 : 6;
     L.stage_bytes = wide ? kWideStageBytes : kNarrowStageBytes;
-    return q.bwd ? launch<true>(L, sms, stream) : launch<false>(L, sms, stream);
+    if (q.bwd) return copies ? launch<true, false>(L, sms, stream) : launch<true, true>(L, sms, stream);
+    return copies ? launch<false, false>(L, sms, stream) : launch<false, true>(L, sms, stream);
 }
 
 }  // namespace tmoe

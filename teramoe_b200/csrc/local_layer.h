@@ -14,13 +14,14 @@ constexpr int kLocalMaxExperts = 512;    // the routing kernels keep 23 words pe
 // at most min(E, T * K) segments padded to 128 rows), so the host never has to read the layout back.
 struct LocalLayerPlan {
     int T, K, E, H, I, keep;             // keep: tables of the backward pass too
+    int copies[2];                       // per direction: token rows are copied into slot order, not loaded by the slot table
     int few;                             // a forward with few rows per expert: local_few.cu
     int chunks;                          // blocks of the routing kernels
     int slots_cap, blocks_cap, units_cap;
     int work_cap[2];                     // items of the forward / backward list
     int cols[2][4];                      // columns per tile: [direction][first GEMM, second GEMM, dW_down, dW_gateup]
     // zero-filled by local_layer_route
-    long stats[2], sync[2], done1[2], done2[2], zero_words;
+    long stats[2], sync[2], done1[2], done2[2], arrived[2], zero_words;
     // written by it
     long meta, seg, counts, slot_tk, slot_w, token_order, order_slot, chunk_hist, chunk_last, work[2], words;
 };
@@ -45,6 +46,8 @@ struct LocalLayerParams {
     void* saved_x;                       // [T, H] copy of x: written by forward (may be null), read by backward
     void* out;                           // [T, H]
     void* preact;                        // written by forward (with keep), read by backward: 2I * out_rows values in 32 x 8 blocks
+    void* slot_rows;                     // with plan.copies: rows of x in slot order [out_rows, H], backward also of saved_x
+    void* slot_x;
     // backward
     float* droute_part;                  // [out_rows, 2 * ceil(I / 256)]
     float* dw_topk;                      // [T, K]

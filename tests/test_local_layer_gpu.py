@@ -157,6 +157,28 @@ def test_forward_with_few_rows_per_expert(H, I, monkeypatch):
     buf.destroy()
 
 
+@pytest.mark.parametrize("T,H,I,E,K", [
+    (511, 192, 512, 4, 2),                               # 255 rows per expert on average, below half of I: copies in backward
+    (512, 192, 512, 4, 2),                               # at half of it: loading warps
+    (700, 320, 4096, 3, 2),                              # I so large that rows are copied in both directions
+])
+def test_rows_by_copies_and_by_loading_warps(T, H, I, E, K, monkeypatch):
+    """Both sides of the rule that says how token rows become operands."""
+    from teramoe_b200 import engine
+    prob = make_problem(1, T, H, I, E, K, seed=T, dtype=torch.bfloat16, device="cuda", x_scale=0.1, w_scale=0.02, drop_some=False)
+    buf = tm.Buffer(None, int(64e6), explicitly_destroy=True)
+    res = {}
+    for mode in ("0", "auto"):
+        monkeypatch.setattr(engine, "_LOCAL_LAYER_MODE", mode)
+        for name in ("_FUSED_DISPATCH_MODE", "_FUSED_MODE", "_LAYER_KERNEL_MODE"):
+            monkeypatch.setattr(engine, name, "1" if mode == "0" else "auto")
+        res[mode] = _run(buf, prob, prob["ranks"][0]["idx"], E)
+    for name, got in res["auto"].items():
+        assert torch.equal(got, res["0"][name]), f"{name}: differs from the general kernels"
+    buf.check_status()
+    buf.destroy()
+
+
 def test_native_autograd_node_keeps_its_buffer_and_fills_the_given_gradient():
     """The buffer may go out of scope before the backward pass; d(topk_weights) goes to the caller's tensor; a second derivative
     raises; a destroyed buffer raises."""
