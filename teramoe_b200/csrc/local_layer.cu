@@ -17,13 +17,13 @@
 // left around the kernel.
 //
 // Forward + backward through the API, several-rank kernels (30 to 38 launches and one host wait per step) -> these:
-//   512 tokens, H=512 I=256, 4 experts, top-2            873 ->    99 us   (was host work and launches)
-//   4096, H=2048 I=2048, 16 experts, top-8              2914 ->  2331 us
-//   8192, H=2048 I=3072, 16 experts, top-6              6192 ->  5002 us
-//   8192, H=7168 I=2048, 32 experts, top-8             16737 -> 15088 us
-//   forward only, 32 tokens of that layer                830 ->   573 us
-// Large layers are bound by the power cap: at H=7168 a step of K of the forward takes 1042 to 1045 cycles of which the tensor cores need 1024,
-// while the clock drops to 1.1 to 1.3 GHz.
+//   512 tokens, H=512 I=256, 4 experts, top-2            873 ->    97 us   (was host work and launches)
+//   4096, H=2048 I=2048, 16 experts, top-8              2914 ->  2321 us
+//   8192, H=2048 I=3072, 16 experts, top-6              6192 ->  5030 us
+//   8192, H=7168 I=2048, 32 experts, top-8             16737 -> 15056 us
+//   16384, H=7168 I=512, 32 experts, top-8             10388 ->  8429 us
+// Large layers are bound by the power cap: the SM clock drops to 1.0 to 1.3 GHz, and time is energy (0.86 pJ per FLOP at H=7168 I=2048, of
+// which cuBLAS alone takes 0.74).
 #include "local_layer.h"
 
 #include <type_traits>
