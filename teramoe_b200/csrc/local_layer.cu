@@ -1040,10 +1040,13 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
             int step = warp - 12, stage = step, ss = 0;      // this warp's next step, counted from the start of the item; its stage
             uint32_t phase = 0, sph = 0;
             int under_way = -1;                              // stage of the step before, if its copies are not yet seen through
+            // The arrive is all that orders the rows before the products that the first CTA issues: no byte count covers them.
             auto hand_over = [&](int s) {
                 fence_proxy_async_smem();
                 __syncwarp();
-                if (lane == 0) mbar_arrive_cluster(pair_full + 8u * s);
+                if (lane != 0) return;
+                if (rank == 0) mbar_arrive(full_bar(s));
+                else mbar_arrive_cluster_release_smem(pair_full + 8u * s);
             };
             auto settle = [&]() {
                 if (under_way < 0) return;
@@ -1353,6 +1356,10 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                     for (int k = 0; k < BK / UK; ++k)
                         if (k < slices) umma_bf16_ss_2cta(d_tmem, a_desc + k * a_step, b_desc + k * b_step, idesc, (kb | k) != 0 ? 1u : 0u);
                 };
+                // (the second CTA's loading warps hand over rows that lie there)
+                auto wait_full = [&](int s, uint32_t ph) {
+                    return ROWS ? mbar_wait_cluster_acquire_smem(full_bar(s), ph, abort_flag, L.status, 621) : mbar_wait(full_bar(s), ph, abort_flag, L.status, 621);
+                };
                 if (!mbar_wait(tempty_bar(slot0), parity0, abort_flag, L.status, 620)) { ok = false; break; }
                 tcgen05_fence_after();
                 int kb = 0;
@@ -1363,7 +1370,7 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                     int s = stage;
                     uint32_t ph = phase;
                     for (int i = 0; i < lead; ++i) {
-                        if (!mbar_wait(full_bar(s), ph, abort_flag, L.status, 621)) { ok = false; break; }
+                        if (!wait_full(s, ph)) { ok = false; break; }
                         tcgen05_fence_after();
                         if (elect_one()) {
                             multiply(s, 0, slot0, i);
@@ -1385,7 +1392,7 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                     }
                 }
                 for (; kb < q.nk; ++kb) {
-                    if (!mbar_wait(full_bar(stage), phase, abort_flag, L.status, 621)) { ok = false; break; }
+                    if (!wait_full(stage, phase)) { ok = false; break; }
                     tcgen05_fence_after();
                     if (elect_one()) {
                         const bool last = kb == q.nk - 1;

@@ -95,3 +95,17 @@ def test_a_build_is_recognised_by_the_next_process(monkeypatch, tmp_path):
     before = _build._source_hash()
     _build.build()
     assert _build._stamp_path().read_text() == before == _build._source_hash()
+
+
+def test_rows_of_the_second_cta_are_published_at_cluster_scope():
+    """The loading warps' arrive is all that orders the second CTA's rows before the products that the first one issues.  A missing order
+    shows on the GPU rarely or never, so what is looked at is the source: the arrive from the second CTA and every wait of the issuer for a
+    stage that such rows may fill are a release and an acquire at cluster scope."""
+    src = open(os.path.join(ROOT, "teramoe_b200", "csrc", "local_layer.cu")).read()
+    hand_over = src[src.index("auto hand_over = "):]
+    hand_over = hand_over[: hand_over.index("};")]
+    assert "mbar_arrive_cluster_release" in hand_over and "mbar_arrive_cluster(" not in hand_over
+    issuer = src[src.index("// ----", src.index("TMA producer")):]
+    issuer = issuer[issuer.index("UMMA issuer"): issuer.index("epilogue, then gather")]
+    waits = [line for line in issuer.splitlines() if "mbar_wait" in line and "full_bar" in line and "tfull_bar" not in line]
+    assert waits and all("mbar_wait_cluster_acquire" in line for line in waits)

@@ -127,6 +127,31 @@ def test_loading_warps_keep_up_with_short_items(H, I):
     buf.destroy()
 
 
+@pytest.mark.parametrize("H,I", [(128, 64), (1024, 128)])         # one step of K after the other, and two turns through the stages
+def test_rows_of_both_ctas_are_those_of_this_call(H, I, monkeypatch):
+    """Units of 256 rows, half of them loaded by the second CTA, with other values in every call: an operand that is multiplied before it is
+    there holds rows of another step or another call."""
+    from teramoe_b200 import engine
+    prob = make_problem(1, 2048, H, I, 8, 1, seed=H, dtype=torch.bfloat16, device="cuda", x_scale=0.1, w_scale=0.02)
+    r = prob["ranks"][0]
+    r["idx"] = (torch.arange(2048, device="cuda") % 8).view(2048, 1)
+    buf = tm.Buffer(None, int(64e6), explicitly_destroy=True)
+    gen = torch.Generator(device="cuda").manual_seed(7)
+    for _ in range(10):
+        r["x"].normal_(0, 0.1, generator=gen)
+        r["go"].normal_(0, 1.0, generator=gen)
+        res = {}
+        for mode in ("0", "auto"):
+            monkeypatch.setattr(engine, "_LOCAL_LAYER_MODE", mode)
+            for name in ("_FUSED_DISPATCH_MODE", "_FUSED_MODE", "_LAYER_KERNEL_MODE"):
+                monkeypatch.setattr(engine, name, "1" if mode == "0" else "auto")
+            res[mode] = _run(buf, prob, r["idx"], 8)
+        for name, got in res["auto"].items():
+            assert torch.equal(got, res["0"][name]), f"{name}: differs from the general kernels"
+    buf.check_status()
+    buf.destroy()
+
+
 @pytest.mark.parametrize("H,I", [(192, 64), (1088, 320)])         # a last tile of weights that is half outside
 def test_forward_with_few_rows_per_expert(H, I, monkeypatch):
     """Rows per expert around the multiples of 4 (row gather), 16 (columns of the accumulator) and 64 (units); tokens without an expert;
