@@ -372,6 +372,16 @@ int64_t local_layer_arena_bytes(int64_t T, int64_t K, int64_t E, int64_t H) {
     return layer_rows(tmoe::local_layer_plan((int)T, (int)K, (int)E, (int)H, 64, 0)) * H * 2;
 }
 
+// which kernels a call with these sizes runs, for tests that are about one of them
+py::dict local_layer_variant(int64_t T, int64_t K, int64_t E, int64_t H, int64_t I, bool keep) {
+    const tmoe::LocalLayerPlan p = tmoe::local_layer_plan((int)T, (int)K, (int)E, (int)H, (int)I, keep ? 1 : 0);
+    py::dict d;
+    d["few"] = p.few;
+    d["copies_forward"] = p.copies[0] != 0;
+    d["copies_backward"] = p.copies[1] != 0;
+    return d;
+}
+
 void check_layer_weights(const torch::Tensor& wg, const torch::Tensor& wd, int64_t E, int64_t H, int64_t I) {
     TORCH_CHECK(wg.is_cuda() && wg.scalar_type() == torch::kBFloat16 && wg.is_contiguous() && wg.dim() == 3 && wg.size(0) == E &&
                 wg.size(1) == 2 * I && wg.size(2) == H, "W_gateup must be a contiguous bf16 [E, 2I, H] CUDA tensor");
@@ -678,6 +688,7 @@ void register_local(pybind11::module_& m) {
         .def("check", &LocalLayer::check)
         .def("stats", &LocalLayer::stats)
         .def("call", &local_layer_call);
+    m.def("local_layer_variant", &local_layer_variant);
     m.def("local_counts", &local_counts);
     m.def("local_scatter", &local_scatter);
     m.def("local_combine", &local_combine);

@@ -1632,6 +1632,11 @@ LocalLayerPlan local_layer_plan(int T, int K, int E, int H, int I, int keep) {
     p.slots_cap = p.blocks_cap * 128;
     p.units_cap = (int)((p.blocks_cap + segs) / 2);
     const int rows = (int)(entries / (segs > 0 ? segs : 1));
+    // Few rows per expert, forward only: weights as the M operand (local_few.cu).  us, here / there (32 experts, top-8, H=7168 I=2048; I=512), by
+    // rows per expert: 1 368 / 279, 8 577 / 441, 16 589 / 471; 184 / 151, 24 600 / 522; 191 / 172, 32 615 / 566; 200 / 194.  Skewed routing
+    // (hottest expert 2.5 times the mean) at 20: 603 / 528; 189 / 186, and with the hottest 5 times the mean 606 / 538; 189 / 221 (at 16:
+    // 185 / 185), as experts of more than 64 rows take their weights twice: the line is where that still costs nothing.
+    p.few = !keep && T > 0 && entries <= (long)kFewRows * E;
     // Token rows through the loading warps, or copied into slot order first.  The loading warps load a row again for every tile of the other
     // operand, with more energy per byte than TMA; a copy is written and read once.  ms of a step, backward by loaders / by copies: 2048
     // tokens, H=7168 I=512, 32 experts, top-8 (512 rows per expert) 1.41 / 1.73; 2048, H=2048 I=256, 32, top-6 (384 rows) 0.263 / 0.322;
@@ -1640,13 +1645,8 @@ LocalLayerPlan local_layer_plan(int T, int K, int E, int H, int I, int keep) {
     // (16) 1.969 / 1.757.  I = 14336 (H=4096, 8 experts, 4096 tokens, top-2), loaders in both directions, in the forward alone, in none:
     // 7.85, 7.94, 7.68.
     const bool large_i = I >= 4096;
-    p.copies[0] = large_i;
+    p.copies[0] = large_i && !p.few;          // (local_few.cu gathers rows from x itself)
     p.copies[1] = keep && (large_i || 2 * rows < I);
-    // Few rows per expert, forward only: weights as the M operand (local_few.cu).  us, here / there (32 experts, top-8, H=7168 I=2048; I=512), by
-    // rows per expert: 1 368 / 279, 8 577 / 441, 16 589 / 471; 184 / 151, 24 600 / 522; 191 / 172, 32 615 / 566; 200 / 194.  Skewed routing
-    // (hottest expert 2.5 times the mean) at 20: 603 / 528; 189 / 186, and with the hottest 5 times the mean 606 / 538; 189 / 221 (at 16:
-    // 185 / 185), as experts of more than 64 rows take their weights twice: the line is where that still costs nothing.
-    p.few = !keep && T > 0 && entries <= (long)kFewRows * E;
     // Columns per tile of every GEMM [direction][kind].  The wide tile needs columns for it, enough tiles that every CTA pair gets
     // several, and a mainloop that is long against what it cannot hide: with both accumulators in one tile, the next tile
     // starts when the first half has been read out (in cycles: 2 thousand for a plain store, 3.6 for SwiGLU, 13.5 for its backward), where

@@ -109,3 +109,16 @@ def test_rows_of_the_second_cta_are_published_at_cluster_scope():
     issuer = issuer[issuer.index("UMMA issuer"): issuer.index("epilogue, then gather")]
     waits = [line for line in issuer.splitlines() if "mbar_wait" in line and "full_bar" in line and "tfull_bar" not in line]
     assert waits and all("mbar_wait_cluster_acquire" in line for line in waits)
+
+
+def test_kernels_of_a_call_by_its_sizes():
+    """A forward with few rows per expert gathers its rows from x: no memory for copies of them, whatever I is."""
+    from teramoe_b200._build import load_ext
+    variant = lambda T, K, E, I, keep: tuple(bool(v) for v in load_ext().local_layer_variant(T, K, E, 4096, I, keep).values())
+    assert variant(8, 2, 8, 4096, False) == (True, False, False)
+    assert variant(8, 2, 8, 14336, False) == (True, False, False)
+    assert variant(512, 2, 8, 4096, False) == (False, True, False)
+    assert variant(512, 2, 8, 4032, False) == (False, False, False)
+    assert variant(8, 2, 8, 14336, True) == (False, True, True)
+    assert variant(511, 2, 4, 512, True) == (False, False, True)
+    assert variant(512, 2, 4, 512, True) == (False, False, False)
