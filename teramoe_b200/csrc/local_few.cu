@@ -1,14 +1,14 @@
 // The layer's forward on one rank when experts have few rows (local_layer_plan decides), as in decoding: the time is that of reading the
 // weights once.  The weights are the M operand here, 128 rows of a tile, and an expert's tokens the N operand, 16 to 64 columns.  With the
 // roles of local_layer.cu eight tokens were multiplied as 256 rows; under the power cap, which such a call reaches too, the tensor
-// cores' share is bandwidth lost.  Forward of 32 tokens, H=7168 I=2048, 32 experts, top-8: 577 -> 441 us, 6.4 TB/s, which is what a plain
-// copy reaches; of 16 tokens, H=2048 I=2048, 16 experts 110 -> 85; of 16 tokens, H=512 I=256, 4 experts, top-2 31 -> 22.
+// cores' share is bandwidth lost.  Forward of 32 tokens, H=7168 I=2048, 32 experts, top-8: 585 -> 430 us, 6.6 TB/s, which is what a plain
+// copy reaches; of 64 tokens 588 -> 437; with I=512 179 -> 132 and 185 -> 134.
 //
 // One persistent block per SM, no clusters.  Items: first the tiles of the first GEMM (128 rows of W_gateup of an expert x a unit of up to
 // 64 of its tokens), then those of the second, dealt out in turn: they all cost the same.  Units of one expert are neighbours, so that
 // they share the tile of weights in L2.
-//   warp 0     loads: weights by TMA boxes, token rows by TMA row gather (16 copies of 4 rows in a step at most; what made it too slow
-//              for the large tiles of local_layer.cu hides here behind the weights), the second GEMM's rows by boxes of 16
+//   warp 0     loads: weights by TMA boxes, the second GEMM's rows by boxes of 16
+//   warps 2, 3 load the first GEMM's token rows, every other step each, by cp.async
 //   warp 1     issues tcgen05.mma, 128 x N x 16, into one of four accumulators
 //   warps 4-7  epilogue: a lane holds one row of weights, so gate and up of a token sit in neighbouring lanes
 //   warps 2-7  at the end: sums of the tokens' expert rows, in the order of their entries
@@ -36,7 +36,8 @@ constexpr int kFewSmemBytes = kFewUnitsOffset + (3 * kLocalMaxExperts + 1) * 4 +
 static_assert(8 * (2 * kFewStages + 2 * kFewAccs) <= 248 && kFewSmemBytes <= 232448, "shared memory");
 
 struct FewArgs {
-    alignas(64) CUtensorMap map_wg, map_wd, map_x, map_act;
+    alignas(64) CUtensorMap map_wg, map_wd, map_act;
+    const uint8_t* x;
     int T, K, H, I, E;
     __nv_bfloat16* act;
     __nv_bfloat16* y;
@@ -75,7 +76,7 @@ __global__ void __launch_bounds__(kFewThreads, 1) local_few_kernel(const __grid_
     if (threadIdx.x == 0) {
         *abort_flag = 0u;
         for (int s = 0; s < kFewStages; ++s) {
-            mbar_init(full_bar(s), 1);
+            mbar_init(full_bar(s), 1 + 32);                  // the producer, and every lane of a loading warp
             mbar_init(empty_bar(s), 1);
         }
         for (int a = 0; a < kFewAccs; ++a) {
@@ -85,7 +86,6 @@ __global__ void __launch_bounds__(kFewThreads, 1) local_few_kernel(const __grid_
         fence_mbar_init();
         tma_prefetch_desc(&L.map_wg);
         tma_prefetch_desc(&L.map_wd);
-        tma_prefetch_desc(&L.map_x);
         tma_prefetch_desc(&L.map_act);
     }
     if (warp == 2) tmem_alloc(smem_u32((const void*)tmem_slot), kFewAccs * kUnit);
@@ -140,17 +140,10 @@ __global__ void __launch_bounds__(kFewThreads, 1) local_few_kernel(const __grid_
         bool ok = true;
         for (int i = blockIdx.x; i < items && ok; i += gridDim.x) {
             const FewItem q = decode(i);
-            const int nk = q.second ? nk2 : nk1, quads = (q.rows + 3) / 4, boxes = q.n / 16;
+            const int nk = q.second ? nk2 : nk1, boxes = q.n / 16;
             const int w_row = q.second ? q.expert * L.H + q.tile * BM : q.expert * 2 * L.I + q.tile * BM;
             const CUtensorMap* map_w = q.second ? &L.map_wd : &L.map_wg;
-            const uint32_t tx = (uint32_t)(kAStageBytes + (q.second ? boxes * 16 : quads * 4) * BK * 2);
-            int4 tokens = make_int4(L.T, L.T, L.T, L.T);         // (past the end: zeros)
-            if (!q.second && lane < quads) {
-                int t[4];
-#pragma unroll
-                for (int c = 0; c < 4; ++c) t[c] = 4 * lane + c < q.rows ? L.slot_tk[q.slot0 + 4 * lane + c] / L.K : L.T;
-                tokens = make_int4(t[0], t[1], t[2], t[3]);
-            }
+            const uint32_t tx = (uint32_t)(kAStageBytes + (q.second ? boxes * 16 * BK * 2 : 0));
             auto weights = [&](int s, uint32_t ph, int kb) {
                 if (!mbar_wait(empty_bar(s), ph ^ 1u, abort_flag, L.status, 680)) return false;
                 if (lane == 0) {
@@ -183,11 +176,7 @@ __global__ void __launch_bounds__(kFewThreads, 1) local_few_kernel(const __grid_
             for (int kb = 0; kb < nk; ++kb) {
                 if (kb >= early && !(ok = weights(stage, phase, kb))) break;
                 const uint32_t dst = smem_base + stage * kFewStageBytes + kAStageBytes;
-                if (q.second) {
-                    if (lane < boxes) tma_load_2d(dst + lane * 16 * BK * 2, &L.map_act, full_bar(stage), kb * BK, q.slot0 + 16 * lane);
-                } else if (lane < quads) {
-                    tma_gather4(dst + lane * 4 * BK * 2, &L.map_x, full_bar(stage), kb * BK, tokens);
-                }
+                if (q.second && lane < boxes) tma_load_2d(dst + lane * 16 * BK * 2, &L.map_act, full_bar(stage), kb * BK, q.slot0 + 16 * lane);
                 if (++stage == kFewStages) { stage = 0; phase ^= 1u; }
             }
         }
@@ -205,6 +194,7 @@ __global__ void __launch_bounds__(kFewThreads, 1) local_few_kernel(const __grid_
             tcgen05_fence_after();
             for (int kb = 0; kb < nk; ++kb) {
                 if (!(ok = mbar_wait(full_bar(stage), phase, abort_flag, L.status, 683))) break;
+                if (!q.second) fence_proxy_async_smem();         // rows that the loading warps' copies wrote -> async-proxy reads
                 tcgen05_fence_after();
                 if (elect_one()) {
                     const uint32_t at = smem_base + stage * kFewStageBytes;
@@ -220,7 +210,47 @@ __global__ void __launch_bounds__(kFewThreads, 1) local_few_kernel(const __grid_
             }
             if (++acc == kFewAccs) { acc = 0; acc_phase ^= 1u; }
         }
-    } else if (warp >= 4) {
+    } else if (warp < 4) {
+        // Token rows.  Eight lanes copy 128 bytes of a row, in the layout that TMA gives the weights; a warp's arrive follows its copies by itself.
+        // It takes part in every step, also where it has no rows to bring, so that it is never a whole turn through the stages ahead.
+        // TMA's row gather takes 70 cycles for four rows, 1120 for a unit of 64, where a step's weights take 720: with experts of unequal
+        // load the few SMs that had the tiles of a large one came last.  us, general kernel / row gather / this: 64 tokens, H=7168 I=512, 32
+        // experts, top-8, hottest expert 20 rows 185 / 150 / 134, 43 rows 185 / 173 / 134, 63 rows 185 / 195 / 136, all on 8 experts 91 / 124 / 85;
+        // with total_sms = 32, 16 tokens 517 / 429 / 395, 64 tokens 535 / 529 / 412.
+        const int sub = lane >> 3, chunk = lane & 7;
+        const uint32_t at[2] = {(uint32_t)(sub * 128 + ((chunk ^ sub) << 4)), (uint32_t)(sub * 128 + ((chunk ^ (sub + 4)) << 4))};      // rows 8j + sub, 8j + 4 + sub
+        int step = warp - 2, stage = step;                       // this warp's next step, counted from the start of the item; its stage
+        uint32_t phase = 0;
+        bool ok = true;
+        for (int i = blockIdx.x; i < items && ok; i += gridDim.x) {
+            const FewItem q = decode(i);
+            const int nk = q.second ? nk2 : nk1, quads = (q.rows + 3) / 4;
+            int token[2] = {0, 0};                               // of rows lane, lane + 32
+            if (!q.second) {
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+                    if (lane + 32 * h < q.rows) token[h] = L.slot_tk[q.slot0 + lane + 32 * h] / L.K;
+            }
+            for (; step < nk; step += 2) {
+                if (!(ok = mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag, L.status, 686))) break;
+                if (!q.second) {
+                    const uint32_t dst = smem_base + stage * kFewStageBytes + kAStageBytes;
+                    const uint8_t* src = L.x + step * (BK * 2) + 16 * chunk;
+#pragma unroll
+                    for (int j = 0; j < kUnit / 4; ++j) {        // (rows of the last four that are not there: any row, its column is not read)
+                        if (j >= quads) break;
+                        const int t = __shfl_sync(0xffffffffu, token[j >> 3], (4 * j + sub) & 31);
+                        cp_async_16(dst + j * 512 + at[j & 1], src + (long)t * (L.H * 2l));
+                    }
+                }
+                cp_async_arrive(full_bar(stage));
+                stage += 2;
+                if (stage >= kFewStages) { stage -= kFewStages; phase ^= 1u; }
+            }
+            step -= nk;
+        }
+        cp_async_wait_all();
+    } else {
         const int quarter = warp & 3;
         int acc = 0;
         uint32_t acc_phase = 0;
@@ -323,15 +353,16 @@ cudaError_t local_few_launch(const LocalLayerParams& q, cudaStream_t stream) {
     const int H = p.H, I = p.I, E = p.E;
     if (!p.few || q.bwd || H % BK != 0 || I % BK != 0 || q.out_rows < p.slots_cap || p.K < 1 || p.K > 32 || E < 1 || E > kLocalMaxExperts)
         return cudaErrorInvalidValue;
+    if (reinterpret_cast<uintptr_t>(q.x) % 16 != 0) return cudaErrorInvalidValue;
     int dev = 0;
     cudaError_t e;
     if ((e = cudaGetDevice(&dev)) != cudaSuccess || (e = cudaSetDevice(dev)) != cudaSuccess) return e;      // (the tensor-map encoder wants a current context)
     FewArgs L{};
     if ((e = make_map(&L.map_wg, q.w_gateup, (uint64_t)E * 2 * I, H, BK, BM)) != cudaSuccess) return e;
     if ((e = make_map(&L.map_wd, q.w_down, (uint64_t)E * H, I, BK, BM)) != cudaSuccess) return e;
-    if ((e = make_map(&L.map_x, q.x, p.T, H, BK, 1)) != cudaSuccess) return e;
     if ((e = make_map(&L.map_act, q.act, q.out_rows, I, BK, 16)) != cudaSuccess) return e;
     L.T = p.T; L.K = p.K; L.H = H; L.I = I; L.E = E;
+    L.x = static_cast<const uint8_t*>(q.x);
     L.act = static_cast<__nv_bfloat16*>(q.act);
     L.y = static_cast<__nv_bfloat16*>(q.y);
     L.out = static_cast<__nv_bfloat16*>(q.out);

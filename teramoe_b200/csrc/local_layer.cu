@@ -449,15 +449,6 @@ __device__ __forceinline__ void copy_row_deep(int4* dst, const int4* src, int nv
     }
 }
 
-// 16 bytes from memory into shared memory, or zeros
-__device__ __forceinline__ void cp_async_16_or_zeros(uint32_t dst_smem, const void* src, bool wanted) {
-    asm volatile("cp.async.cg.shared.global.L2::256B [%0], [%1], 16, %2;" ::"r"(dst_smem), "l"(src), "r"(wanted ? 16 : 0) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
 template <int R>
 __device__ __forceinline__ void registers_inc() {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(R));
@@ -1632,10 +1623,8 @@ LocalLayerPlan local_layer_plan(int T, int K, int E, int H, int I, int keep) {
     p.slots_cap = p.blocks_cap * 128;
     p.units_cap = (int)((p.blocks_cap + segs) / 2);
     const int rows = (int)(entries / (segs > 0 ? segs : 1));
-    // Few rows per expert, forward only: weights as the M operand (local_few.cu).  us, here / there (32 experts, top-8, H=7168 I=2048; I=512), by
-    // rows per expert: 1 368 / 279, 8 577 / 441, 16 589 / 471; 184 / 151, 24 600 / 522; 191 / 172, 32 615 / 566; 200 / 194.  Skewed routing
-    // (hottest expert 2.5 times the mean) at 20: 603 / 528; 189 / 186, and with the hottest 5 times the mean 606 / 538; 189 / 221 (at 16:
-    // 185 / 185), as experts of more than 64 rows take their weights twice: the line is where that still costs nothing.
+    // Few rows per expert, forward only: weights as the M operand (local_few.cu).  us, here / there, by rows per expert: 16 (32 experts, top-8,
+    // H=7168 I=2048) 588 / 437, (I=512) 185 / 134, (64 experts, top-4, H=4096 I=768) 286 / 216, (64 experts, top-2, H=2048 I=512) 121 / 90.
     p.few = !keep && T > 0 && entries <= (long)kFewRows * E;
     // Token rows through the loading warps, or copied into slot order first.  The loading warps load a row again for every tile of the other
     // operand, with more energy per byte than TMA; a copy is written and read once.  ms of a step, backward by loaders / by copies: 2048

@@ -152,19 +152,28 @@ def test_rows_of_both_ctas_are_those_of_this_call(H, I, monkeypatch):
     buf.destroy()
 
 
-@pytest.mark.parametrize("H,I", [(192, 64), (1088, 320)])         # a last tile of weights that is half outside
-def test_forward_with_few_rows_per_expert(H, I, monkeypatch):
-    """Rows per expert around the multiples of 4 (row gather), 16 (columns of the accumulator) and 64 (units); tokens without an expert;
-    more blocks than tiles and the other way round."""
+@pytest.mark.parametrize("counts,empty,H,I,K", [
+    # rows around the multiples of 4 (row copies), 16 (columns of the accumulator) and 64 (units); a last tile of weights that is half outside
+    ([1, 3, 4, 5, 15, 16, 17, 31, 33, 47, 63, 64, 65, 127, 128, 129, 2], 100, 192, 64, 2),
+    ([1, 3, 4, 5, 15, 16, 17, 31, 33, 47, 63, 64, 65, 127, 128, 129, 2], 100, 1088, 320, 2),
+    ([300], 60, 1088, 320, 2),                           # all rows on one expert, far more than the average
+    ([64, 64, 1], 40, 512, 4096, 3),                     # I so large that other forwards copy rows
+    ([70, 20, 9], 100, 320, 128, 9),                     # sums of more than eight entries, one at the end
+    ([40, 33, 2], 200, 320, 128, 32),
+])
+def test_forward_with_few_rows_per_expert(counts, empty, H, I, K, monkeypatch):
+    """Also: tokens without an expert; more blocks than tiles and the other way round."""
     from teramoe_b200 import engine
-    counts = [1, 3, 4, 5, 15, 16, 17, 31, 33, 47, 63, 64, 65, 127, 128, 129, 2] + [0] * 100
-    E, T = len(counts), sum(counts) + 3
+    from teramoe_b200._build import load_ext
+    E, T = len(counts) + empty, sum(counts) + 3
+    assert load_ext().local_layer_variant(T, K, E, H, I, False)["few"]
     gen = torch.Generator().manual_seed(1)
-    experts = torch.repeat_interleave(torch.arange(E), torch.tensor(counts))
-    idx = torch.full((T, 2), -1, dtype=torch.int64)
-    idx[torch.randperm(T, generator=gen)[: len(experts)], 1] = experts[torch.randperm(len(experts), generator=gen)]
-    assert idx.numel() <= 16 * E
-    prob = make_problem(1, T, H, I, E, 2, seed=8, dtype=torch.bfloat16, device="cuda", x_scale=0.1, w_scale=0.02)
+    experts = torch.repeat_interleave(torch.arange(len(counts)), torch.tensor(counts))
+    idx = torch.full((T, K), -1, dtype=torch.int64)
+    idx[torch.randperm(T, generator=gen)[: len(experts)], K - 1] = experts[torch.randperm(len(experts), generator=gen)]
+    if K > 8:                                            # and for some tokens all entries
+        idx[:2] = torch.randperm(E - len(counts), generator=gen)[:K] + len(counts)
+    prob = make_problem(1, T, H, I, E, K, seed=8, dtype=torch.bfloat16, device="cuda", x_scale=0.1, w_scale=0.02)
     r = prob["ranks"][0]
     idx = idx.cuda()
     buf = tm.Buffer(None, int(64e6), explicitly_destroy=True)
@@ -174,10 +183,10 @@ def test_forward_with_few_rows_per_expert(H, I, monkeypatch):
         for name in ("_FUSED_DISPATCH_MODE", "_FUSED_MODE", "_LAYER_KERNEL_MODE"):
             monkeypatch.setattr(engine, name, "1" if mode == "0" else "auto")
         call = lambda i, **kw: buf.teramoe_forward(r["x"], i, r["w"], prob["W_gateup"], prob["W_down"], E, **kw)
-        res[mode] = [call(idx), call(idx, total_sms=16, num_dispatch_sms=4, num_combine_sms=4), call(idx[:, :1].expand(T, 2).contiguous())]
+        res[mode] = [call(idx), call(idx, total_sms=16, num_dispatch_sms=4, num_combine_sms=4), call(torch.full_like(idx, -1))]
     for got, want in zip(res["auto"], res["0"]):
         assert torch.equal(got, want)
-    assert not bool(res["auto"][2].any())
+    assert bool(res["auto"][0].any()) and not bool(res["auto"][2].any())
     buf.check_status()
     buf.destroy()
 
