@@ -549,6 +549,11 @@ class LocalLayer : public std::enable_shared_from_this<LocalLayer> {
         if (!last_[dir].defined()) return c10::nullopt;
         return last_[dir].narrow(0, last_at_[dir], 48).view(torch::kInt64);
     }
+    // whether the last forward ran in local_few.cu (reads the routing's word back)
+    bool ran_few() {
+        std::lock_guard<std::mutex> lock(mutex_);
+        return last_[0].defined() && last_[0][last_few_].item<int>() != 0;
+    }
 
   private:
     // (with arena_mutex_ held, until the launch)
@@ -567,6 +572,7 @@ class LocalLayer : public std::enable_shared_from_this<LocalLayer> {
         std::lock_guard<std::mutex> lock(mutex_);
         std::swap(last_[dir], before);
         last_at_[dir] = plan.stats[dir];
+        if (dir == 0) last_few_ = plan.meta + tmoe::kMetaFew;
     }
     torch::Tensor status_, host_;
     // A backward pass runs without the interpreter's lock, next to a call that replaces the arena.
@@ -575,7 +581,7 @@ class LocalLayer : public std::enable_shared_from_this<LocalLayer> {
     std::atomic<bool> open_{true};
     std::mutex mutex_;
     torch::Tensor last_[2];
-    int64_t last_at_[2] = {0, 0};
+    int64_t last_at_[2] = {0, 0}, last_few_ = 0;
 };
 
 // The layer as a native autograd node: a backward pass runs on autograd's worker thread without the interpreter.
@@ -687,6 +693,7 @@ void register_local(pybind11::module_& m) {
         .def("close", &LocalLayer::close)
         .def("check", &LocalLayer::check)
         .def("stats", &LocalLayer::stats)
+        .def("ran_few", &LocalLayer::ran_few, py::call_guard<py::gil_scoped_release>())
         .def("call", &local_layer_call);
     m.def("local_layer_variant", &local_layer_variant);
     m.def("local_counts", &local_counts);

@@ -51,6 +51,7 @@ struct FewArgs {
     int* done1;                          // per 64 slots: epilogue warps that finished a tile of the first GEMM
     int* done2;                          // the same for the second
     int* status;
+    const int* wanted;                   // the routing's word for this kernel; null: it takes the call
 };
 
 struct FewItem {
@@ -58,6 +59,7 @@ struct FewItem {
 };
 
 __global__ void __launch_bounds__(kFewThreads, 1) local_few_kernel(const __grid_constant__ FewArgs L) {
+    if (L.wanted != nullptr && *L.wanted == 0) return;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
@@ -215,8 +217,7 @@ __global__ void __launch_bounds__(kFewThreads, 1) local_few_kernel(const __grid_
         // It takes part in every step, also where it has no rows to bring, so that it is never a whole turn through the stages ahead.
         // TMA's row gather takes 70 cycles for four rows, 1120 for a unit of 64, where a step's weights take 720: with experts of unequal
         // load the few SMs that had the tiles of a large one came last.  us, general kernel / row gather / this: 64 tokens, H=7168 I=512, 32
-        // experts, top-8, hottest expert 20 rows 185 / 150 / 134, 43 rows 185 / 173 / 134, 63 rows 185 / 195 / 136, all on 8 experts 91 / 124 / 85;
-        // with total_sms = 32, 16 tokens 517 / 429 / 395, 64 tokens 535 / 529 / 412.
+        // experts, top-8, hottest expert 20 rows 179 / 151 / 134, 63 rows 179 / 195 / 132, all on 8 experts 90 / 122 / 70.
         const int sub = lane >> 3, chunk = lane & 7;
         const uint32_t at[2] = {(uint32_t)(sub * 128 + ((chunk ^ sub) << 4)), (uint32_t)(sub * 128 + ((chunk ^ (sub + 4)) << 4))};      // rows 8j + sub, 8j + 4 + sub
         int step = warp - 2, stage = step;                       // this warp's next step, counted from the start of the item; its stage
@@ -237,8 +238,10 @@ __global__ void __launch_bounds__(kFewThreads, 1) local_few_kernel(const __grid_
                     const uint32_t dst = smem_base + stage * kFewStageBytes + kAStageBytes;
                     const uint8_t* src = L.x + step * (BK * 2) + 16 * chunk;
 #pragma unroll
-                    for (int j = 0; j < kUnit / 4; ++j) {        // (rows of the last four that are not there: any row, its column is not read)
-                        if (j >= quads) break;
+                    for (int j = 0; j < kUnit / 4; ++j) {
+                        // 16 rows with no branch between the copies, so that they follow each other (the last example 85 -> 70 us); for
+                        // rows that are not there any row, as nobody reads its column
+                        if ((j & 3) == 0 && j >= quads) break;
                         const int t = __shfl_sync(0xffffffffu, token[j >> 3], (4 * j + sub) & 31);
                         cp_async_16(dst + j * 512 + at[j & 1], src + (long)t * (L.H * 2l));
                     }
@@ -375,6 +378,7 @@ cudaError_t local_few_launch(const LocalLayerParams& q, cudaStream_t stream) {
     L.done1 = q.ws + p.done1[0];
     L.done2 = q.ws + p.done2[0];
     L.status = q.status;
+    L.wanted = p.few == 2 ? q.ws + p.meta + kMetaFew : nullptr;
     static bool configured[64] = {};
     if ((e = ensure_smem_limit(local_few_kernel, kFewSmemBytes, configured)) != cudaSuccess) return e;
     const int sms = default_sms(q.num_sms) & ~1;

@@ -72,8 +72,6 @@ static_assert(kSmemBytesP <= 232448, "shared memory");
 
 // words of the sync block
 enum { kSyncItem = 0, kSyncToken = 1, kSyncCopy = 2, kSyncKeep = 3, kSyncFirsts = 4, kSyncRows = 5, kSyncWords = 8 };
-// words of the meta block
-enum { kMetaUnits = 0, kMetaSlots = 1, kMetaWork = 2, kMetaRows = 4, kMetaWords = 8 };
 
 constexpr int kWideTiles = 74 * 4;                                        // least number of wide tiles of a GEMM (local_layer_plan)
 
@@ -162,6 +160,7 @@ __global__ void __launch_bounds__(kRouteThreads) local_route_assign_kernel(const
     int* totals = lst + kRouteWarps * (E + 1);   // [E] entries, [E + 1] tokens by their last expert: of all chunks ...
     int* before_own = totals + 2 * E + 1;        // ... and of those before this block's
     const int* last_hist = totals + E;
+    int* few_word = before_own + 2 * E + 1;      // local_few.cu takes the call
     if (DIRECT) {
         for (int i = tid; i < 2 * (2 * E + 1); i += kRouteThreads) totals[i] = 0;
         clear_counters(a);
@@ -202,10 +201,12 @@ __global__ void __launch_bounds__(kRouteThreads) local_route_assign_kernel(const
     }
     __syncthreads();
     if (warp == 0) {
-        int run_s = 0, run_u = 0, run_r = 0;
+        int run_s = 0, run_u = 0, run_r = 0, hit = 0, few_units = 0;
         for (int e0 = 0; e0 < E; e0 += 32) {
             const int e = e0 + lane;
             const int blocks = e < E ? (totals[e] + 127) / 128 : 0;
+            hit += __popc(__ballot_sync(0xffffffffu, blocks != 0));
+            few_units += __reduce_add_sync(0xffffffffu, e < E ? (totals[e] + kFewUnitRows - 1) / kFewUnitRows : 0);
             int s = blocks * 128, u = (blocks + 1) / 2;
             const int s_own = s, u_own = u;
             for (int o = 1; o < 32; o <<= 1) {
@@ -227,6 +228,10 @@ __global__ void __launch_bounds__(kRouteThreads) local_route_assign_kernel(const
         if (lane == 0) {
             seg[E] = run_s;
             ub[E] = run_u;
+            // Units beyond an expert's first, each of which takes its weights again, from L2: as many as experts with rows at most.  us, general
+            // kernel / local_few.cu (64 experts, top-4, H=7168 I=768, all tokens on four experts): 128 tokens, one such unit per expert, 88 / 76,
+            // 256 tokens, three, 95 / 115.
+            *few_word = a.p.few == 1 || (a.p.few == 2 && few_units - hit <= hit);
         }
     }
     if (warp == 1) {
@@ -256,6 +261,7 @@ __global__ void __launch_bounds__(kRouteThreads) local_route_assign_kernel(const
         if (tid == 0) {
             meta[kMetaUnits] = U;
             meta[kMetaSlots] = seg[E];
+            meta[kMetaFew] = *few_word;
         }
     }
     for (int e = blockIdx.x; e < E; e += gridDim.x)
@@ -277,7 +283,7 @@ __global__ void __launch_bounds__(kRouteThreads) local_route_assign_kernel(const
         return 2 * behind < SG ? ub[e + 1] : (int)v;
     };
     const int per_wd = a.mu_wd * a.nb_wd, per_e = per_wd + a.mu_wg * a.nb_wg;
-    for (int dir = 0; dir < (a.p.few ? 0 : a.p.keep ? 2 : 1); ++dir) {
+    for (int dir = 0; dir < (*few_word ? 0 : a.p.keep ? 2 : 1); ++dir) {
         int4* work = reinterpret_cast<int4*>(a.ws + a.p.work[dir]);
         const int cap = a.p.work_cap[dir], nb1 = a.nb1[dir], nb2 = a.nb2[dir];
         const int items = U * (nb1 + nb2);                   // of the two GEMMs
@@ -418,6 +424,7 @@ struct LayerArgsP {
     int* arrived;                        // without loading warps, per 128-row block: rows of slot_rows in place
     unsigned long long* stats;
     int* status;
+    int unless_few;                      // the call is local_few.cu's, whose kernel ran before, if the routing says so
 };
 
 __device__ __forceinline__ int4 ld_cg_v4_ordered(const void* p) {
@@ -697,6 +704,9 @@ __device__ __forceinline__ void epilogue_plain(const Staging& st, uint32_t taddr
 template <bool BWD, bool ROWS>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(ROWS ? kLayerThreads : kThreads, 1)
 local_layer_kernel(const __grid_constant__ LayerArgsP L) {
+    if constexpr (!BWD) {
+        if (L.unless_few && L.meta[kMetaFew] != 0) return;
+    }
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
@@ -1625,7 +1635,12 @@ LocalLayerPlan local_layer_plan(int T, int K, int E, int H, int I, int keep) {
     const int rows = (int)(entries / (segs > 0 ? segs : 1));
     // Few rows per expert, forward only: weights as the M operand (local_few.cu).  us, here / there, by rows per expert: 16 (32 experts, top-8,
     // H=7168 I=2048) 588 / 437, (I=512) 185 / 134, (64 experts, top-4, H=4096 I=768) 286 / 216, (64 experts, top-2, H=2048 I=512) 121 / 90.
-    p.few = !keep && T > 0 && entries <= (long)kFewRows * E;
+    // An expert of more than 64 rows takes its weights again for every 64.  The host cannot see one, but that it matters takes tokens and a large layer:
+    // if all T tokens chose the same K experts, K * (T / 64 - 1) units would read 6 H I bytes each.  Up to 128 tokens, or 96 MB, the kernel is
+    // ahead on any routing (512 tokens on two experts, H=2048 I=512, 84 MB 47 / 43).  Beyond, the routing decides on the GPU: both kernels are
+    // launched, and one returns at once, for 5 us (256 tokens, H=4096 I=768, 64 experts, top-4 268 / 215; all on two experts, H=7168 I=2048 95 / 102).
+    const long again = (long)K * ((T + kFewUnitRows - 1) / kFewUnitRows - 1) * 6 * H * I;
+    p.few = keep || T <= 0 || entries > (long)kFewRows * E ? 0 : T <= 2 * kFewUnitRows || again <= 96l << 20 ? 1 : 2;
     // Token rows through the loading warps, or copied into slot order first.  The loading warps load a row again for every tile of the other
     // operand, with more energy per byte than TMA; a copy is written and read once.  ms of a step, backward by loaders / by copies: 2048
     // tokens, H=7168 I=512, 32 experts, top-8 (512 rows per expert) 1.41 / 1.73; 2048, H=2048 I=256, 32, top-6 (384 rows) 0.263 / 0.322;
@@ -1634,7 +1649,7 @@ LocalLayerPlan local_layer_plan(int T, int K, int E, int H, int I, int keep) {
     // (16) 1.969 / 1.757.  I = 14336 (H=4096, 8 experts, 4096 tokens, top-2), loaders in both directions, in the forward alone, in none:
     // 7.85, 7.94, 7.68.
     const bool large_i = I >= 4096;
-    p.copies[0] = large_i && !p.few;          // (local_few.cu gathers rows from x itself)
+    p.copies[0] = large_i && p.few != 1;          // (local_few.cu gathers rows from x itself)
     p.copies[1] = keep && (large_i || 2 * rows < I);
     // Columns per tile of every GEMM [direction][kind].  The wide tile needs columns for it, enough tiles that every CTA pair gets
     // several, and a mainloop that is long against what it cannot hide: with both accumulators in one tile, the next tile
@@ -1660,7 +1675,7 @@ LocalLayerPlan local_layer_plan(int T, int K, int E, int H, int I, int keep) {
     p.cols[1][1] = columns(H, units, 2 * I, 1024);
     p.cols[1][2] = columns(I, (long)E * mu_wd, rows, 1024);
     p.cols[1][3] = columns(H, (long)E * mu_wg, rows, 1024);
-    p.work_cap[0] = p.few ? 0 : p.units_cap * (column_blocks(2 * I, p.cols[0][0]) + column_blocks(H, p.cols[0][1]));
+    p.work_cap[0] = p.few == 1 ? 0 : p.units_cap * (column_blocks(2 * I, p.cols[0][0]) + column_blocks(H, p.cols[0][1]));
     p.work_cap[1] = keep ? p.units_cap * (column_blocks(I, p.cols[1][0]) + column_blocks(H, p.cols[1][1])) +
                                E * (mu_wd * column_blocks(I, p.cols[1][2]) + mu_wg * column_blocks(H, p.cols[1][3]))
                          : 0;
@@ -1707,7 +1722,7 @@ cudaError_t local_layer_route(const LocalLayerParams& q, cudaStream_t stream) {
     a.group_units = q.group_units; a.lag_percent = q.lag_percent; a.min_lag_items = q.min_lag_items > 0 ? q.min_lag_items : 0;
     // 64 blocks at least: the lists (tens of thousands of items for a large layer) are written by all blocks
     const int grid = p.chunks > 64 ? p.chunks : 64;
-    const size_t smem = (3 * (p.E + 1) + (kRouteWarps + 2) * (2 * p.E + 1)) * sizeof(int);
+    const size_t smem = (3 * (p.E + 1) + (kRouteWarps + 2) * (2 * p.E + 1) + 1) * sizeof(int);
     if ((long)p.T * p.K <= kDirectEntries) {
         local_route_assign_kernel<true><<<grid, kRouteThreads, smem, stream>>>(a);
         return cudaGetLastError();
@@ -1722,7 +1737,11 @@ cudaError_t local_layer_route(const LocalLayerParams& q, cudaStream_t stream) {
 
 cudaError_t local_layer_launch(const LocalLayerParams& q, cudaStream_t stream) {
     const LocalLayerPlan& p = q.plan;
-    if (p.few) return local_few_launch(q, stream);
+    if (p.few) {
+        const cudaError_t e = local_few_launch(q, stream);
+        if (p.few == 1 || e != cudaSuccess) return e;
+        count_launch();                                   // (callers count one launch)
+    }
     const int H = p.H, I = p.I, E = p.E, dir = q.bwd ? 1 : 0;
     if (H % BK != 0 || I % BK != 0 || q.out_rows % BM != 0 || q.out_rows < BM || q.out_rows < p.slots_cap || p.K < 1 || p.K > 32 || (q.bwd && !p.keep))
         return cudaErrorInvalidValue;
@@ -1795,6 +1814,7 @@ cudaError_t local_layer_launch(const LocalLayerParams& q, cudaStream_t stream) {
     L.done2 = q.ws + p.done2[dir];
     L.stats = reinterpret_cast<unsigned long long*>(q.ws + p.stats[dir]);
     L.status = q.status;
+    L.unless_few = p.few == 2;
     const int sms = default_sms(q.num_sms) & ~1;
     if (sms < 4) return cudaErrorInvalidConfiguration;
     bool wide = false;

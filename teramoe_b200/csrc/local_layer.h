@@ -10,12 +10,15 @@ namespace tmoe {
 constexpr int kFewUnitRows = 64;         // rows of an expert that local_few.cu multiplies at a time
 constexpr int kLocalMaxExperts = 512;    // the routing kernels keep 23 words per expert in shared memory
 
+// words of the meta block
+enum { kMetaUnits = 0, kMetaSlots = 1, kMetaWork = 2, kMetaRows = 4, kMetaFew = 5, kMetaWords = 8 };
+
 // Word offsets of the tables of one call inside its int32 workspace.  Capacities follow from the sizes alone (T * K entries in
 // at most min(E, T * K) segments padded to 128 rows), so the host never has to read the layout back.
 struct LocalLayerPlan {
     int T, K, E, H, I, keep;             // keep: tables of the backward pass too
     int copies[2];                       // per direction: token rows are copied into slot order, not loaded by the slot table
-    int few;                             // a forward with few rows per expert: local_few.cu
+    int few;                             // a forward with few rows per expert: 1 local_few.cu, 2 local_few.cu if the routing says so (kMetaFew)
     int chunks;                          // blocks of the routing kernels
     int slots_cap, blocks_cap, units_cap;
     int work_cap[2];                     // items of the forward / backward list

@@ -114,11 +114,17 @@ def test_rows_of_the_second_cta_are_published_at_cluster_scope():
 def test_kernels_of_a_call_by_its_sizes():
     """A forward with few rows per expert gathers its rows from x: no memory for copies of them, whatever I is."""
     from teramoe_b200._build import load_ext
-    variant = lambda T, K, E, I, keep: tuple(bool(v) for v in load_ext().local_layer_variant(T, K, E, 4096, I, keep).values())
-    assert variant(8, 2, 8, 4096, False) == (True, False, False)
-    assert variant(8, 2, 8, 14336, False) == (True, False, False)
-    assert variant(512, 2, 8, 4096, False) == (False, True, False)
-    assert variant(512, 2, 8, 4032, False) == (False, False, False)
-    assert variant(8, 2, 8, 14336, True) == (False, True, True)
-    assert variant(511, 2, 4, 512, True) == (False, False, True)
-    assert variant(512, 2, 4, 512, True) == (False, False, False)
+    variant = lambda T, K, E, I, keep: tuple(int(v) for v in load_ext().local_layer_variant(T, K, E, 4096, I, keep).values())
+    assert variant(8, 2, 8, 4096, False) == (1, 0, 0)
+    assert variant(64, 2, 8, 14336, False) == (1, 0, 0)
+    assert variant(65, 2, 8, 14336, False) == (0, 1, 0)
+    assert variant(64, 2, 9, 14336, False) == (1, 0, 0)
+    assert variant(128, 2, 16, 14336, False) == (1, 0, 0)
+    assert variant(129, 2, 17, 14336, False) == (2, 1, 0)       # (the routing decides: both kernels are launched)
+    assert variant(192, 2, 24, 1024, False) == (1, 0, 0)        # (four units read again, 96 MB)
+    assert variant(193, 2, 25, 1024, False) == (2, 0, 0)
+    assert variant(512, 2, 8, 4032, False) == (0, 0, 0)
+    assert variant(8, 2, 8, 14336, True) == (0, 1, 1)
+    assert variant(511, 2, 4, 512, True) == (0, 0, 1)
+    assert variant(512, 2, 4, 512, True) == (0, 0, 0)
+    assert variant(0, 2, 4, 512, False) == (0, 0, 0)

@@ -191,6 +191,48 @@ def test_forward_with_few_rows_per_expert(counts, empty, H, I, K, monkeypatch):
     buf.destroy()
 
 
+@pytest.mark.parametrize("counts,H,I,few", [
+    ([64] * 20 + [8] * 10, 4096, 1024, True),            # no second unit
+    ([129] * 6 + [64] * 6, 4096, 1024, True),            # as many as experts with rows
+    ([129] * 7 + [64] * 5 + [8], 4096, 1024, False),     # one more
+    ([700], 4096, 1024, False),                          # all rows on one expert
+    ([700], 512, 256, True),                             # so small a layer that it does not matter
+])
+def test_forward_with_few_rows_on_average_by_their_spread(counts, H, I, few, monkeypatch):
+    """Which kernel takes a call is decided by the routing, on the GPU: also when a captured call is replayed with other indices."""
+    from teramoe_b200 import engine
+    from teramoe_b200._build import load_ext
+    T = sum(counts) + 3
+    E = max(-(-2 * T // 16), len(counts))
+    assert load_ext().local_layer_variant(T, 2, E, H, I, False)["few"] == (2 if H > 512 else 1)
+    idx = torch.full((T, 2), -1, dtype=torch.int64)
+    idx[: sum(counts), 0] = torch.repeat_interleave(torch.arange(len(counts)), torch.tensor(counts))
+    idx = idx[torch.randperm(T, generator=torch.Generator().manual_seed(1))].cuda()
+    even = (torch.arange(2 * T, device="cuda") % E).view(T, 2)
+    prob = make_problem(1, T, H, I, E, 2, seed=8, dtype=torch.bfloat16, device="cuda", x_scale=0.1, w_scale=0.02)
+    r = prob["ranks"][0]
+    buf = tm.Buffer(None, int(64e6), explicitly_destroy=True)
+    call = lambda i: buf.teramoe_forward(r["x"], i, r["w"], prob["W_gateup"], prob["W_down"], E)
+    with monkeypatch.context() as m:
+        m.setattr(engine, "_LOCAL_LAYER_MODE", "0")
+        for name in ("_FUSED_DISPATCH_MODE", "_FUSED_MODE", "_LAYER_KERNEL_MODE"):
+            m.setattr(engine, name, "1")
+        want, want_even = call(idx), call(even)
+    ran_few = buf._engine.native.ran_few
+    for i, ref, kernel in ((idx, want, few), (even, want_even, True)):
+        assert torch.equal(call(i), ref) and ran_few() == kernel
+    static = even.clone()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = call(static)
+    for i, ref, kernel in ((idx, want, few), (even, want_even, True), (idx, want, few)):
+        static.copy_(i)
+        graph.replay()
+        assert torch.equal(out, ref) and ran_few() == kernel
+    buf.check_status()
+    buf.destroy()
+
+
 @pytest.mark.parametrize("T,H,I,E,K", [
     (511, 192, 512, 4, 2),                               # 255 rows per expert on average, below half of I: copies in backward
     (512, 192, 512, 4, 2),                               # at half of it: loading warps
