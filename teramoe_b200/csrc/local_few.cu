@@ -16,6 +16,7 @@
 #include "local_layer.h"
 
 #include "gemm_common.cuh"
+#include "layer.h"
 
 namespace tmoe {
 
@@ -50,6 +51,7 @@ struct FewArgs {
     const int* order_slot;
     int* done1;                          // per 64 slots: epilogue warps that finished a tile of the first GEMM
     int* done2;                          // the same for the second
+    unsigned long long* stats;
     int* status;
     const int* wanted;                   // the routing's word for this kernel; null: it takes the call
 };
@@ -140,6 +142,7 @@ __global__ void __launch_bounds__(kFewThreads, 1) local_few_kernel(const __grid_
         int stage = 0;
         uint32_t phase = 0;
         bool ok = true;
+        uint64_t waited = 0;
         for (int i = blockIdx.x; i < items && ok; i += gridDim.x) {
             const FewItem q = decode(i);
             const int nk = q.second ? nk2 : nk1, boxes = q.n / 16;
@@ -170,7 +173,11 @@ __global__ void __launch_bounds__(kFewThreads, 1) local_few_kernel(const __grid_
                     }
                     if (!ok) break;
                     // (a wait that runs out is reported, and the item carried through on whatever its rows hold)
-                    if (lane == 0) wait_count_gpu(flag, kFewEpiWarps * n1, L.status, 681, 64);
+                    if (lane == 0) {
+                        const uint64_t t0 = globaltimer_ns();
+                        wait_count_gpu(flag, kFewEpiWarps * n1, L.status, 681, 64);
+                        waited += globaltimer_ns() - t0;
+                    }
                 }
                 __syncwarp();
                 fence_proxy_async_all();                         // stores of other SMs -> async-proxy reads
@@ -182,6 +189,7 @@ __global__ void __launch_bounds__(kFewThreads, 1) local_few_kernel(const __grid_
                 if (++stage == kFewStages) { stage = 0; phase ^= 1u; }
             }
         }
+        if (waited != 0) atomicAdd(L.stats + kStatWaitFirstGemm, (unsigned long long)waited);
         if (!ok)                                                 // (no barrier says when the copies under way have landed: microseconds)
             for (const uint64_t t0 = globaltimer_ns(); globaltimer_ns() - t0 < 10000000ull;) __nanosleep(1000);
     } else if (warp == 1) {
@@ -257,8 +265,15 @@ __global__ void __launch_bounds__(kFewThreads, 1) local_few_kernel(const __grid_
         const int quarter = warp & 3;
         int acc = 0;
         uint32_t acc_phase = 0;
+        const bool stamps = warp == 4 && lane == 0;
+        uint64_t first[2] = {0, 0}, last[2] = {0, 0};            // when items of the two GEMMs were taken, finished
         for (int i = blockIdx.x; i < items; i += gridDim.x) {
             const FewItem q = decode(i);
+            if (stamps) {
+                const uint64_t now = globaltimer_ns();
+                if (first[0] == 0 && !q.second) first[0] = now;
+                if (first[1] == 0 && q.second) first[1] = now;
+            }
             const float w[2] = {!q.second && lane < q.rows ? L.slot_w[q.slot0 + lane] : 0.f, !q.second && lane + 32 < q.rows ? L.slot_w[q.slot0 + lane + 32] : 0.f};
             if (!mbar_wait(tfull_bar(acc), acc_phase, abort_flag, L.status, 684)) break;
             tcgen05_fence_after();
@@ -297,7 +312,16 @@ __global__ void __launch_bounds__(kFewThreads, 1) local_few_kernel(const __grid_
                 fence_acq_rel_gpu();
                 red_add_gpu((q.second ? L.done2 : L.done1) + q.slot0 / kUnit, 1);
             }
+            if (stamps) (q.second ? last[1] : last[0]) = globaltimer_ns();
             if (++acc == kFewAccs) { acc = 0; acc_phase ^= 1u; }
+        }
+        if (stamps) {
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                if (first[k] == 0) continue;
+                atomicMax(L.stats + kStatKindFirst + (k == 0 ? kWorkGemm1 : kWorkGemm2), ~first[k]);
+                atomicMax(L.stats + kStatKindLast + (k == 0 ? kWorkGemm1 : kWorkGemm2), last[k]);
+            }
         }
     }
     __syncwarp();
@@ -305,13 +329,13 @@ __global__ void __launch_bounds__(kFewThreads, 1) local_few_kernel(const __grid_
     if (warp >= 2) {
         // sums: (token, 256 columns) per task
         const int nvec = L.H / 8, parts = (nvec + 31) / 32, tasks = L.T * parts, K = L.K;
+        uint64_t waited = 0, first = 0;
         for (int task = (warp - 2) * (int)gridDim.x + (int)blockIdx.x; task < tasks; task += kFewSumWarps * (int)gridDim.x) {
             const int place = task / parts, col = (task - place * parts) * 32 + lane, at = min(col, nvec - 1);
             const int t = L.token_order[place], slot = lane < K ? L.order_slot[(long)place * K + lane] : -1;
             const uint32_t valid = __ballot_sync(0xffffffffu, slot >= 0);
-            bool there = true;
-            if (slot >= 0) there = wait_count_gpu(L.done2 + slot / kUnit, kFewEpiWarps * n2, L.status, 685, 64);
-            if (!__all_sync(0xffffffffu, there)) break;          // reported: unwind
+            if (!wait_counts_warp(L.done2 + max(slot, 0) / kUnit, slot >= 0, kFewEpiWarps * n2, L.status, 685, waited)) break;      // reported: unwind
+            if (first == 0) first = globaltimer_ns();
             __syncwarp();                                        // every lane reads behind the other lanes' acquires
             float sum[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
             for (int k0 = 0; k0 < K; k0 += 8) {
@@ -339,6 +363,11 @@ __global__ void __launch_bounds__(kFewThreads, 1) local_few_kernel(const __grid_
             if (col < nvec)
                 reinterpret_cast<int4*>(L.out + (long)t * L.H)[col] = make_int4((int)pack_bf16x2(sum[0], sum[1]), (int)pack_bf16x2(sum[2], sum[3]),
                                                                                 (int)pack_bf16x2(sum[4], sum[5]), (int)pack_bf16x2(sum[6], sum[7]));
+        }
+        if (lane == 0 && first != 0) {
+            atomicMax(L.stats + kStatKindFirst + kWorkReduce, ~first);
+            atomicMax(L.stats + kStatKindLast + kWorkReduce, globaltimer_ns());
+            if (waited != 0) atomicAdd(L.stats + kStatWaitLanded, (unsigned long long)waited);
         }
     }
     tcgen05_fence_before();
@@ -377,6 +406,7 @@ cudaError_t local_few_launch(const LocalLayerParams& q, cudaStream_t stream) {
     L.order_slot = q.ws + p.order_slot;
     L.done1 = q.ws + p.done1[0];
     L.done2 = q.ws + p.done2[0];
+    L.stats = reinterpret_cast<unsigned long long*>(q.ws + p.stats[0]);
     L.status = q.status;
     L.wanted = p.few == 2 ? q.ws + p.meta + kMetaFew : nullptr;
     static bool configured[64] = {};

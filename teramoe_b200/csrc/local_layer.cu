@@ -943,23 +943,7 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
             const int part = next_i % parts, t = next_t, slot = next_slot;
             claim();
             const uint32_t valid = __ballot_sync(0xffffffffu, slot >= 0);
-            // all lanes look together, so that the entries of a token are waited for once and not one after the other
-            const int* flag = L.done2 + (slot >= 0 ? slot >> 7 : 0);
-            if (!__all_sync(0xffffffffu, slot < 0 || ld_acquire_gpu(flag) >= target2)) {
-                const uint64_t w0 = globaltimer_ns(), limit_ns = peer_wait_limit_ns(L.status);
-                while (!__all_sync(0xffffffffu, slot < 0 || ld_acquire_gpu(flag) >= target2)) {
-                    __nanosleep(250);
-                    int gone = 0;
-                    if (lane == 0) {
-                        if (ld_relaxed_sys(L.status) != 0) gone = 1;
-                        else if (globaltimer_ns() - w0 > limit_ns) gone = 2;
-                    }
-                    gone = __shfl_sync(0xffffffffu, gone, 0);
-                    if (gone == 2 && slot >= 0 && ld_acquire_gpu(flag) < target2) report_status(L.status, kStatusFlagTimeout, 660, target2);
-                    if (gone != 0) return;                                    // reported: unwind
-                }
-                waited += globaltimer_ns() - w0;
-            }
+            if (!wait_counts_warp(L.done2 + (slot >= 0 ? slot >> 7 : 0), slot >= 0, target2, L.status, 660, waited)) return;      // reported: unwind
             __syncwarp();                                                     // every lane reads behind the other lanes' acquires
             if (stamps && !stamped) {
                 stamped = true;
@@ -1638,7 +1622,7 @@ LocalLayerPlan local_layer_plan(int T, int K, int E, int H, int I, int keep) {
     // An expert of more than 64 rows takes its weights again for every 64.  The host cannot see one, but that it matters takes tokens and a large layer:
     // if all T tokens chose the same K experts, K * (T / 64 - 1) units would read 6 H I bytes each.  Up to 128 tokens, or 96 MB, the kernel is
     // ahead on any routing (512 tokens on two experts, H=2048 I=512, 84 MB 47 / 43).  Beyond, the routing decides on the GPU: both kernels are
-    // launched, and one returns at once, for 5 us (256 tokens, H=4096 I=768, 64 experts, top-4 268 / 215; all on two experts, H=7168 I=2048 95 / 102).
+    // launched, and one returns at once, for 5 us (256 tokens, H=4096 I=768, 64 experts, top-4 268 / 215; all on two experts, H=7168 I=2048 95 / 98).
     const long again = (long)K * ((T + kFewUnitRows - 1) / kFewUnitRows - 1) * 6 * H * I;
     p.few = keep || T <= 0 || entries > (long)kFewRows * E ? 0 : T <= 2 * kFewUnitRows || again <= 96l << 20 ? 1 : 2;
     // Token rows through the loading warps, or copied into slot order first.  The loading warps load a row again for every tile of the other

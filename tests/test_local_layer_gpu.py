@@ -450,6 +450,47 @@ def test_hooks_on_saved_tensors_see_no_workspace():
     buf.destroy()
 
 
+@pytest.mark.parametrize("T,E,few", [(32, 16, True), (512, 16, False)])
+def test_a_forward_reports_its_spans_and_waits(T, E, few):
+    """Every forward replaces the report of the one before, and its time stamps lie in the order of the work."""
+    from teramoe_b200._build import load_ext
+    assert bool(load_ext().local_layer_variant(T, 8, E, 4096, 1024, False)["few"]) == few
+    prob = make_problem(1, T, 4096, 1024, E, 8, seed=7, dtype=torch.bfloat16, device="cuda", x_scale=0.1, w_scale=0.02)
+    r = prob["ranks"][0]
+    buf = tm.Buffer(None, 0, explicitly_destroy=True)
+    call = lambda i: buf.teramoe_forward(r["x"], i, r["w"], prob["W_gateup"], prob["W_down"], E)
+    call(r["idx"])
+    rep = buf._engine.wait_report()["fwd"]
+    spans = rep["spans_ms"]
+    assert set(spans) == {"gemm1", "gemm2", "reduce"}
+    assert all(0 <= a <= b < 100 for a, b in spans.values())
+    assert spans["gemm1"][0] == 0 and spans["gemm1"][0] < spans["gemm2"][0] < spans["reduce"][1]
+    assert spans["gemm1"][1] < spans["gemm2"][1] < spans["reduce"][1] and spans["gemm2"][1] > 0
+    assert rep["wait_first_gemm"] > 0 and rep["wait_landed"] > 0 and rep["wait_arrival"] == rep["wait_wgrad"] == 0
+    call(torch.full_like(r["idx"], -1))
+    assert set(buf._engine.wait_report()["fwd"]["spans_ms"]) == {"reduce"}
+    buf.destroy()
+
+
+def test_waits_of_a_forward_with_few_rows_that_run_out_are_reported():
+    """With a limit of a nanosecond every wait for another block's tiles runs out: the kernel ends in order, the report is raised, and the buffer
+    can be used again."""
+    prob = make_problem(1, 32, 4096, 1024, 16, 8, seed=7, dtype=torch.bfloat16, device="cuda", x_scale=0.1, w_scale=0.02)
+    r = prob["ranks"][0]
+    buf = tm.Buffer(None, 0, explicitly_destroy=True)
+    call = lambda: buf.teramoe_forward(r["x"], r["idx"], r["w"], prob["W_gateup"], prob["W_down"], 16)
+    want = call()
+    limit = buf._world.status[4:6]
+    limit[0] = 1
+    call()
+    with pytest.raises(RuntimeError, match="flag wait"):
+        buf.check_status()
+    limit[0] = 0
+    assert torch.equal(call(), want)
+    buf.check_status()
+    buf.destroy()
+
+
 def test_a_wait_that_runs_out_is_reported_and_the_next_call_works():
     """A slot table that says less than the work list lets a block's rows never arrive: the wait for them runs out behind the early
     loads of weights, the kernel ends in order, the report is raised, and the buffer can be used again."""
