@@ -64,12 +64,23 @@ def test_one_rank_layer_matches_general_kernels_and_oracle(T, H, I, E, K, skew, 
     buf.destroy()
 
 
-@pytest.mark.parametrize("H,I", [(192, 128), (4160, 64)])         # rows copied several at once, and one after the other
-def test_rows_per_expert_at_the_edges_of_operand_boxes(H, I, monkeypatch):
-    """An expert's rows are loaded 32 at a time up to 96 and 128 at a time above, summed 64 at a time, and stored 32 at a time."""
+@pytest.mark.parametrize("H,I,copies", [
+    (192, 128, (False, False)),                          # loading warps, two slices of columns and a half, and many
+    (4160, 64, (False, False)),
+    (192, 256, (False, True)),                           # rows copied several at once, and one after the other
+    (4160, 256, (False, True)),
+    (192, 4096, (True, True)),
+    (4160, 4096, (True, True)),
+])
+def test_rows_per_expert_at_the_edges_of_operand_boxes(H, I, copies, monkeypatch):
+    """An expert's rows are copied 8 at a time, loaded 32 at a time up to 64 and 128 at a time above (by loading warps 32 or 128), summed 16
+    at a time, and stored 32 at a time."""
     from teramoe_b200 import engine
+    from teramoe_b200._build import load_ext
     counts = [1, 0, 31, 32, 33, 63, 64, 65, 95, 96, 97, 127, 128, 129, 161, 255, 256, 257]
     E, T = len(counts), sum(counts)
+    train, forward = (load_ext().local_layer_variant(T, 1, E, H, I, keep) for keep in (True, False))
+    assert (train["copies_forward"], train["copies_backward"], forward["copies_forward"], forward["few"]) == (*copies, copies[0], 0)
     prob = make_problem(1, T, H, I, E, 1, seed=3, dtype=torch.bfloat16, device="cuda", x_scale=0.1, w_scale=0.02)
     order = torch.randperm(T, generator=torch.Generator().manual_seed(1))
     idx = torch.repeat_interleave(torch.arange(E), torch.tensor(counts))[order].view(T, 1).to(prob["ranks"][0]["idx"])
@@ -233,14 +244,18 @@ def test_forward_with_few_rows_on_average_by_their_spread(counts, H, I, few, mon
     buf.destroy()
 
 
-@pytest.mark.parametrize("T,H,I,E,K", [
-    (511, 192, 512, 4, 2),                               # 255 rows per expert on average, below half of I: copies in backward
-    (512, 192, 512, 4, 2),                               # at half of it: loading warps
-    (700, 320, 4096, 3, 2),                              # I so large that rows are copied in both directions
+@pytest.mark.parametrize("T,H,I,E,K,copies", [
+    (511, 192, 512, 4, 2, (False, True)),                # 255 rows per expert on average, below half of I: copies in backward
+    (512, 192, 512, 4, 2, (False, False)),               # at half of it: loading warps
+    (700, 320, 4032, 3, 2, (False, True)),
+    (700, 320, 4096, 3, 2, (True, True)),                # I so large that rows are copied in both directions
 ])
-def test_rows_by_copies_and_by_loading_warps(T, H, I, E, K, monkeypatch):
+def test_rows_by_copies_and_by_loading_warps(T, H, I, E, K, copies, monkeypatch):
     """Both sides of the rule that says how token rows become operands."""
     from teramoe_b200 import engine
+    from teramoe_b200._build import load_ext
+    variant = load_ext().local_layer_variant(T, K, E, H, I, True)
+    assert (variant["copies_forward"], variant["copies_backward"]) == copies
     prob = make_problem(1, T, H, I, E, K, seed=T, dtype=torch.bfloat16, device="cuda", x_scale=0.1, w_scale=0.02, drop_some=False)
     buf = tm.Buffer(None, int(64e6), explicitly_destroy=True)
     res = {}
@@ -491,11 +506,14 @@ def test_waits_of_a_forward_with_few_rows_that_run_out_are_reported():
     buf.destroy()
 
 
-def test_a_wait_that_runs_out_is_reported_and_the_next_call_works():
-    """A slot table that says less than the work list lets a block's rows never arrive: the wait for them runs out behind the early
-    loads of weights, the kernel ends in order, the report is raised, and the buffer can be used again."""
+@pytest.mark.parametrize("I,copies", [(256, True), (128, False)])
+def test_a_wait_that_runs_out_is_reported_and_the_next_call_works(I, copies):
+    """A slot table that says less than the work list lets a block's rows never arrive: the wait for their copies runs out behind the early
+    loads of weights, or the loading warps see it at once; the kernel ends in order, the report is raised, and the buffer can be used again."""
+    from teramoe_b200._build import load_ext
     T, H, E = 128, 512, 2
-    prob = make_problem(1, T, H, 256, E, 1, seed=7, dtype=torch.bfloat16, device="cuda", x_scale=0.1, w_scale=0.02)
+    assert load_ext().local_layer_variant(T, 1, E, H, I, True)["copies_backward"] == copies
+    prob = make_problem(1, T, H, I, E, 1, seed=7, dtype=torch.bfloat16, device="cuda", x_scale=0.1, w_scale=0.02)
     r = prob["ranks"][0]
     idx = (torch.arange(T, device="cuda") // 64).view(T, 1)
     leaves = [r["x"].clone().requires_grad_(True), prob["W_gateup"].requires_grad_(True), prob["W_down"].requires_grad_(True)]
@@ -511,7 +529,7 @@ def test_a_wait_that_runs_out_is_reported_and_the_next_call_works():
     words = ws.tolist()
     at = [i for i in range(len(words) - 256) if words[i] == 0 and words[i:i + 256] == slots]
     assert len(at) == 1
-    ws[at[0]] = -1                                    # the first 64 rows are not copied
+    ws[at[0]] = -1                                    # the first 64 rows are not copied (or the first is not there)
     buf.set_wait_limit_ms(20)
     torch.autograd.grad(out, leaves, r["go"])
     with pytest.raises(RuntimeError, match="flag wait"):
