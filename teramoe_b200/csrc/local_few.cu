@@ -5,13 +5,13 @@
 // copy reaches; of 64 tokens 588 -> 437; with I=512 179 -> 132 and 185 -> 134.
 //
 // One persistent block per SM, no clusters.  Items: first the tiles of the first GEMM (128 rows of W_gateup of an expert x a unit of up to
-// 64 of its tokens), then those of the second, dealt out in turn: they all cost the same.  Units of one expert are neighbours, so that
+// 64 of its tokens), then those of the second, dealt out in turn: they nearly cost the same.  Units of one expert are neighbours, so that
 // they share the tile of weights in L2.
 //   warp 0     loads: weights by TMA boxes, the second GEMM's rows by boxes of 16
 //   warps 2, 3 load the first GEMM's token rows, every other step each, by cp.async
 //   warp 1     issues tcgen05.mma, 128 x N x 16, into one of four accumulators
 //   warps 4-7  epilogue: a lane holds one row of weights, so gate and up of a token sit in neighbouring lanes
-//   warps 2-7  at the end: sums of the tokens' expert rows, in the order of their entries
+//   warps 2-7  at the end of their items: sums of the tokens' expert rows, in the order of their entries
 // Nine stages of 24 KB keep 144 KB of weights per SM on their way.
 #include "local_layer.h"
 

@@ -2,16 +2,19 @@
 //
 //   producer   claims items of the work list, hands them to the pair, loads operand tiles by TMA
 //   issuer     tcgen05 cta_group::2, 256x256 or 256x512 tiles, two accumulators in tensor memory
-//   loaders    4 warps: bring the operands that are made of token rows from the caller's tensor (load_rows)
+//   loaders    4 warps: bring the operands that are made of token rows from the caller's tensor (load_rows).  An instance of the kernel
+//              has none: there all warps but the first two copy rows into slot order (copy role), and the producer loads them
 //   epilogue   8 warps: SwiGLU / dSwiGLU / store.  A warp packs 32 rows x 64 columns into shared memory (128-byte swizzle) and
 //              hands them to one TMA store; the pre-activation goes straight between registers and memory (preact_at).
 //   gather     warps 2 and 3, joined by the epilogue warps at the end of the list: keep a copy of x (forward), and sum every
 //              token's expert rows as soon as the units that hold them are finished.
 //              Tokens are visited in the order of their last expert, which is the order in which they become ready.
 //
-// The work list, the k steps and the order of every sum are those of layer.cu, except that a weight gradient's tiles are listed along
-// a row of the result: the tiles in flight at a time then write whole rows (7 % faster where the stores bound it, 57 rows per expert).
-// What is different because there is one rank: token rows are loaded by slot instead of pushed by entry, expert rows stay in slot
+// The work list and the order of every sum are those of layer.cu, with three exceptions, none of which changes a result: batches of the list
+// end where experts do (see there); K of a weight gradient ends after the 16 rows that hold the last one, as what layer.cu adds beyond is
+// zeros; and a weight gradient's tiles are listed along a row of the result: the tiles in flight at a time then write whole rows (7 %
+// faster where the stores bound it, 57 rows per expert).
+// What is different because there is one rank: token rows are loaded or copied by slot instead of pushed by entry, expert rows stay in slot
 // order (one TMA box per 32 rows instead of 32 bulk copies to landing rows), the sum of a token waits for its own units
 // instead of for every rank's completion flag, counters have GPU scope, and no host read, table copy or padding kernel is
 // left around the kernel.
@@ -510,14 +513,6 @@ struct Staging {
     __device__ __forceinline__ void put(int chunk, uint32_t a, uint32_t b, uint32_t c, uint32_t d) const {
         st_shared_v4(base + lane * 128 + ((chunk ^ (lane & 7)) << 4), a, b, c, d);
     }
-    __device__ __forceinline__ void put32(int half, const uint32_t (&acc)[32]) const {
-#pragma unroll
-        for (int v = 0; v < 4; ++v) {
-            const uint32_t* p = acc + 8 * v;
-            put(4 * half + v, pack_bf16x2(__uint_as_float(p[0]), __uint_as_float(p[1])), pack_bf16x2(__uint_as_float(p[2]), __uint_as_float(p[3])),
-                pack_bf16x2(__uint_as_float(p[4]), __uint_as_float(p[5])), pack_bf16x2(__uint_as_float(p[6]), __uint_as_float(p[7])));
-        }
-    }
     // The box as two of 32 rows x 64 bytes (64-byte swizzle) that are used in turn: 32 columns in one, its store in flight while
     // the other is filled.  `turn` counts the stores; a store that is not wanted still closes a group, as `reuse` counts groups.
     __device__ __forceinline__ uint32_t narrow_at(int turn, int row, int chunk) const {
@@ -746,9 +741,9 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
         }
     }
     // With few rows per expert most rows of A are never loaded.  Zeros there cost the tensor cores least power; what an earlier kernel left in
-    // shared memory would be multiplied for the whole call.  H=7168, I=2048, 32 experts, back to back behind a large call, without / with zeros:
-    // 8 rows per expert 623 / 547 us, 32 641 / 573, 64 661 / 616.  Above, an expert's rows begin to be loaded 128 at a time; zeros would
-    // still gain there (96 684 / 637, 128 702 / 662).
+    // shared memory would be multiplied for the whole call.  us of a step, back to back, zeros / none: 256 tokens, H=7168 I=2048, 32 experts, top-8
+    // 1938 / 1985, I=512 588 / 600, H=4096 I=14336, 8 experts, top-2 1940 / 2011, with 8 rows per expert 1761 / 1770.  Forwards of 17 to 64
+    // rows per expert 0 (behind other kernels not measured), steps of 128 rows 0 to 2 %.
     if ((long)L.T * L.K <= 64l * L.E) {
         for (int i = threadIdx.x; i < L.stages * (kAStageBytes / 16); i += (int)blockDim.x) {
             const int st = i / (kAStageBytes / 16);
@@ -1597,7 +1592,7 @@ cudaError_t launch(const LayerArgsP& L, int num_sms, cudaStream_t stream) {
     cfg.blockDim = dim3(ROWS ? kLayerThreads : kThreads);
     cfg.dynamicSmemBytes = kSmemBytesP;
     cfg.stream = stream;
-    // every pair waits for rows that warps of all blocks copy and for tiles of other pairs: all of them have to be resident
+    // every pair waits for tiles of other pairs, and without loading warps for rows that warps of all blocks copy: all have to be resident
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeCooperative;
     at[0].val.cooperative = 1;
@@ -1626,12 +1621,20 @@ LocalLayerPlan local_layer_plan(int T, int K, int E, int H, int I, int keep) {
     const long again = (long)K * ((T + kFewUnitRows - 1) / kFewUnitRows - 1) * 6 * H * I;
     p.few = keep || T <= 0 || entries > (long)kFewRows * E ? 0 : T <= 2 * kFewUnitRows || again <= 96l << 20 ? 1 : 2;
     // Token rows through the loading warps, or copied into slot order first.  The loading warps load a row again for every tile of the other
-    // operand, with more energy per byte than TMA; a copy is written and read once.  ms of a step, backward by loaders / by copies: 2048
-    // tokens, H=7168 I=512, 32 experts, top-8 (512 rows per expert) 1.41 / 1.73; 2048, H=2048 I=256, 32, top-6 (384 rows) 0.263 / 0.322;
-    // 8192, H=2048 I=3072, 16, top-6 (3072) 4.89 / 4.97; 8192, H=7168 I=2048 (2048) 14.66 to 14.95 / 14.83 to 14.86; 4096, H=5120 I=1536,
-    // 16, top-2 (512) 1.412 / 1.392; 2048, H=4096 I=768, 32, top-4 (256) 0.840 / 0.817; 512, H=7168 I=2048 (128) 2.416 / 2.204; 64 of them
-    // (16) 1.969 / 1.757.  I = 14336 (H=4096, 8 experts, 4096 tokens, top-2), loaders in both directions, in the forward alone, in none:
-    // 7.85, 7.94, 7.68.
+    // operand, with more energy per byte than TMA; a copy is written and read once.  us of a step, backward by loaders / by copies, by rows per
+    // expert:
+    //   H=7168 I=2048, 32 experts, top-8   16 1918 / 1748   128 2344 / 2150   256 3144 / 2992   512 4682 / 4567   1024 7629 / 7642
+    //   H=7168 I=512, 32, top-8            16 549 / 518     128 701 / 661     256 926 / 919     512 1392 / 1448
+    //   H=4096 I=3072, 16, top-2           32 902 / 808     128 1074 / 964    512 2162 / 2035   1024 3308 / 3243
+    //   H=4096 I=4096, 16, top-2           32 1172 / 1048   128 1394 / 1248   512 2846 / 2670
+    //   H=2048 I=768, 32, top-4            32 279 / 250     128 333 / 309     512 648 / 671
+    //   H=4096 I=14336, 8, top-2           128 2385 / 2120  1024 8002 / 7722
+    // A forward, by loaders / by copies:
+    //   H=7168 I=2048                      17 563 / 561     64 612 / 611      256 994 / 1019    512 1471 / 1507
+    //   H=7168 I=512                       17 175 / 177     64 196 / 203      256 308 / 346
+    //   H=4096 I=3072                      20 254 / 254     64 279 / 275      256 435 / 434     512 683 / 684
+    //   H=4096 I=4096                      20 332 / 333     64 363 / 360      256 571 / 564     512 883 / 884
+    //   H=4096 I=14336                     20 583 / 579     128 671 / 655     1024 2614 / 2583
     const bool large_i = I >= 4096;
     p.copies[0] = large_i && p.few != 1;          // (local_few.cu gathers rows from x itself)
     p.copies[1] = keep && (large_i || 2 * rows < I);
@@ -1748,7 +1751,7 @@ cudaError_t local_layer_launch(const LocalLayerParams& q, cudaStream_t stream) {
     if ((e = q.bwd ? make_map_narrow(&L.st_act, q.act, R, I) : make_map(&L.st_act, q.act, R, I, 64, 32)) != cudaSuccess) return e;
     if ((e = make_map(&L.st_y, q.y, R, H, 64, 32)) != cudaSuccess) return e;
     if (!q.bwd) {
-        // gate_up: A = rows in slot order, B = W_gateup [E*2I, H] K-major;  down: A = act, B = W_down [E*H, I] K-major
+        // gate_up: A = token rows, B = W_gateup [E*2I, H] K-major;  down: A = act, B = W_down [E*H, I] K-major
         if ((e = make_map(&g1.map_b, q.w_gateup, (uint64_t)E * 2 * I, H, BK, BN / 2)) != cudaSuccess) return e;
         if ((e = make_map(&g2.map_a, q.act, R, I, BK, BM)) != cudaSuccess || (e = make_map(&g2.map_a32, q.act, R, I, BK, 32)) != cudaSuccess) return e;
         if ((e = make_map(&g2.map_b, q.w_down, (uint64_t)E * H, I, BK, BN / 2)) != cudaSuccess) return e;

@@ -1,6 +1,7 @@
 // The MoE layer on one rank (local_layer.cu): routing preparation in one launch or two (by the number of entries), then ONE cooperative persistent kernel per
-// direction.  Same work list, tiles and summation orders as the kernel for several ranks (layer.h), so both give the same
-// bits; what differs is everything that only a second rank needs (peer tables, completion flags, landing rows).
+// direction; a forward with few rows per expert has its own (local_few.cu).  Every sum has the terms and the order that it has in the kernel
+// for several ranks (layer.h), so both give the same bits; what differs is where batches of the work list end, slices of K that are
+// all padding, and everything that only a second rank needs (peer tables, completion flags, landing rows).
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -62,7 +63,7 @@ struct LocalLayerParams {
 // Routing tables and both work lists (p: plan, ws, topk_*, schedule).
 cudaError_t local_layer_route(const LocalLayerParams& p, cudaStream_t stream);
 cudaError_t local_layer_launch(const LocalLayerParams& p, cudaStream_t stream);
-// The same for plans with `few` (local_few.cu).
+// The forward of plans with `few` (local_few.cu); local_layer_launch calls it.
 cudaError_t local_few_launch(const LocalLayerParams& p, cudaStream_t stream);
 
 }  // namespace tmoe
