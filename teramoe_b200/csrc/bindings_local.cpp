@@ -551,8 +551,14 @@ class LocalLayer : public std::enable_shared_from_this<LocalLayer> {
     }
     // whether the last forward ran in local_few.cu (reads the routing's word back)
     bool ran_few() {
-        std::lock_guard<std::mutex> lock(mutex_);
-        return last_[0].defined() && last_[0][last_few_].item<int>() != 0;
+        torch::Tensor ws;
+        int64_t at;
+        {
+            std::lock_guard<std::mutex> lock(mutex_);
+            ws = last_[0];
+            at = last_few_;
+        }
+        return ws.defined() && ws[at].item<int>() != 0;
     }
 
   private:

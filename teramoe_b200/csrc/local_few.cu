@@ -152,6 +152,7 @@ __global__ void __launch_bounds__(kFewThreads, 1) local_few_kernel(const __grid_
             auto weights = [&](int s, uint32_t ph, int kb) {
                 if (!mbar_wait(empty_bar(s), ph ^ 1u, abort_flag, L.status, 680)) return false;
                 if (lane == 0) {
+                    if (q.second) mbar_arrive_n(full_bar(s), 32);            // for the loading warp
                     mbar_arrive_expect_tx(full_bar(s), tx);
                     tma_load_2d(smem_base + s * kFewStageBytes, map_w, full_bar(s), kb * BK, w_row);
                 }
@@ -204,9 +205,9 @@ __global__ void __launch_bounds__(kFewThreads, 1) local_few_kernel(const __grid_
             tcgen05_fence_after();
             for (int kb = 0; kb < nk; ++kb) {
                 if (!(ok = mbar_wait(full_bar(stage), phase, abort_flag, L.status, 683))) break;
-                if (!q.second) fence_proxy_async_smem();         // rows that the loading warps' copies wrote -> async-proxy reads
                 tcgen05_fence_after();
                 if (elect_one()) {
+                    if (!q.second) fence_proxy_async_smem();     // rows that the loading warps' copies wrote -> async-proxy reads
                     const uint32_t at = smem_base + stage * kFewStageBytes;
                     const uint64_t a = make_smem_desc_sw128(at, 0, 1024), b = make_smem_desc_sw128(at + kAStageBytes, 0, 1024);
 #pragma unroll
@@ -222,43 +223,48 @@ __global__ void __launch_bounds__(kFewThreads, 1) local_few_kernel(const __grid_
         }
     } else if (warp < 4) {
         // Token rows.  Eight lanes copy 128 bytes of a row, in the layout that TMA gives the weights; a warp's arrive follows its copies by itself.
-        // It takes part in every step, also where it has no rows to bring, so that it is never a whole turn through the stages ahead.
+        // (Handed over behind the copies of the next step, as in local_layer.cu, fewer would be under way: us, so / here, 32 tokens, H=7168 I=2048,
+        // 32 experts, top-8 449 / 433; where items have few steps it is the other way round, 21 tokens, H=512 I=4096, 16 experts 66 / 69.)
+        // The second GEMM's items are all behind the first's; there the producer arrives for it.
         // TMA's row gather takes 70 cycles for four rows, 1120 for a unit of 64, where a step's weights take 720: with experts of unequal
         // load the few SMs that had the tiles of a large one came last.  us, general kernel / row gather / this: 64 tokens, H=7168 I=512, 32
-        // experts, top-8, hottest expert 20 rows 179 / 151 / 134, 63 rows 179 / 195 / 132, all on 8 experts 90 / 122 / 70.
+        // experts, top-8, hottest expert 20 rows 179 / 149 / 137, 63 rows 179 / 195 / 137, all on 8 experts 90 / 122 / 70.
         const int sub = lane >> 3, chunk = lane & 7;
         const uint32_t at[2] = {(uint32_t)(sub * 128 + ((chunk ^ sub) << 4)), (uint32_t)(sub * 128 + ((chunk ^ (sub + 4)) << 4))};      // rows 8j + sub, 8j + 4 + sub
         int step = warp - 2, stage = step;                       // this warp's next step, counted from the start of the item; its stage
         uint32_t phase = 0;
         bool ok = true;
-        for (int i = blockIdx.x; i < items && ok; i += gridDim.x) {
+        for (int i = blockIdx.x; i < U * n1 && ok; i += gridDim.x) {
             const FewItem q = decode(i);
-            const int nk = q.second ? nk2 : nk1, quads = (q.rows + 3) / 4;
-            int token[2] = {0, 0};                               // of rows lane, lane + 32
-            if (!q.second) {
-#pragma unroll
-                for (int h = 0; h < 2; ++h)
-                    if (lane + 32 * h < q.rows) token[h] = L.slot_tk[q.slot0 + lane + 32 * h] / L.K;
-            }
-            for (; step < nk; step += 2) {
+            const int quads = (q.rows + 3) / 4;
+            // of rows lane, lane + 32; past the last row that one again, whose copies nobody reads (of all SMs the same row would be one hot line of L2)
+            const int token[2] = {L.slot_tk[q.slot0 + min(lane, q.rows - 1)] / L.K, L.slot_tk[q.slot0 + min(lane + 32, q.rows - 1)] / L.K};
+            for (; step < nk1; step += 2) {
                 if (!(ok = mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag, L.status, 686))) break;
-                if (!q.second) {
-                    const uint32_t dst = smem_base + stage * kFewStageBytes + kAStageBytes;
-                    const uint8_t* src = L.x + step * (BK * 2) + 16 * chunk;
+                const uint32_t dst = smem_base + stage * kFewStageBytes + kAStageBytes;
+                const uint8_t* src = L.x + step * (BK * 2) + 16 * chunk;
+                auto copy = [&](int j) {
+                    const int t = __shfl_sync(0xffffffffu, token[j >> 3], (4 * j + sub) & 31);
+                    cp_async_16(dst + j * 512 + at[j & 1], src + (long)t * (L.H * 2l));
+                };
+                if (quads <= 4) {
 #pragma unroll
-                    for (int j = 0; j < kUnit / 4; ++j) {
-                        // 16 rows with no branch between the copies, so that they follow each other (the last example 85 -> 70 us); for
-                        // rows that are not there any row, as nobody reads its column
-                        if ((j & 3) == 0 && j >= quads) break;
-                        const int t = __shfl_sync(0xffffffffu, token[j >> 3], (4 * j + sub) & 31);
-                        cp_async_16(dst + j * 512 + at[j & 1], src + (long)t * (L.H * 2l));
+                    for (int j = 0; j < 4; ++j)
+                        if (j < quads) copy(j);
+                } else {
+                    // 16 rows with no branch between the copies, so that they follow each other (the last example 85 -> 70 us)
+#pragma unroll
+                    for (int g = 0; g < kUnit / 16; ++g) {
+                        if (4 * g >= quads) break;
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) copy(4 * g + j);
                     }
                 }
                 cp_async_arrive(full_bar(stage));
                 stage += 2;
                 if (stage >= kFewStages) { stage -= kFewStages; phase ^= 1u; }
             }
-            step -= nk;
+            step -= nk1;
         }
         cp_async_wait_all();
     } else {
@@ -266,14 +272,12 @@ __global__ void __launch_bounds__(kFewThreads, 1) local_few_kernel(const __grid_
         int acc = 0;
         uint32_t acc_phase = 0;
         const bool stamps = warp == 4 && lane == 0;
-        uint64_t first[2] = {0, 0}, last[2] = {0, 0};            // when items of the two GEMMs were taken, finished
         for (int i = blockIdx.x; i < items; i += gridDim.x) {
             const FewItem q = decode(i);
-            if (stamps) {
-                const uint64_t now = globaltimer_ns();
-                if (first[0] == 0 && !q.second) first[0] = now;
-                if (first[1] == 0 && q.second) first[1] = now;
-            }
+            // (the clock is read for the first and the last item of a kind only)
+            const bool ends = i + (int)gridDim.x >= (q.second ? items : U * n1);
+            if (stamps && i - (int)gridDim.x < (q.second ? U * n1 : 0))
+                atomicMax(L.stats + kStatKindFirst + (q.second ? kWorkGemm2 : kWorkGemm1), ~globaltimer_ns());
             const float w[2] = {!q.second && lane < q.rows ? L.slot_w[q.slot0 + lane] : 0.f, !q.second && lane + 32 < q.rows ? L.slot_w[q.slot0 + lane + 32] : 0.f};
             if (!mbar_wait(tfull_bar(acc), acc_phase, abort_flag, L.status, 684)) break;
             tcgen05_fence_after();
@@ -312,30 +316,24 @@ __global__ void __launch_bounds__(kFewThreads, 1) local_few_kernel(const __grid_
                 fence_acq_rel_gpu();
                 red_add_gpu((q.second ? L.done2 : L.done1) + q.slot0 / kUnit, 1);
             }
-            if (stamps) (q.second ? last[1] : last[0]) = globaltimer_ns();
+            if (stamps && ends) atomicMax(L.stats + kStatKindLast + (q.second ? kWorkGemm2 : kWorkGemm1), globaltimer_ns());
             if (++acc == kFewAccs) { acc = 0; acc_phase ^= 1u; }
-        }
-        if (stamps) {
-#pragma unroll
-            for (int k = 0; k < 2; ++k) {
-                if (first[k] == 0) continue;
-                atomicMax(L.stats + kStatKindFirst + (k == 0 ? kWorkGemm1 : kWorkGemm2), ~first[k]);
-                atomicMax(L.stats + kStatKindLast + (k == 0 ? kWorkGemm1 : kWorkGemm2), last[k]);
-            }
         }
     }
     __syncwarp();
 
     if (warp >= 2) {
-        // sums: (token, 256 columns) per task
+        // sums: (token, 256 columns) per task.  The loading warps wait for the epilogue: looking at counters during the second GEMM would slow it down
+        // (64 tokens, H=7168 I=512, 32 experts, top-8 137 -> 150 us).
+        asm volatile("bar.sync 1, %0;" ::"n"(32 * kFewSumWarps) : "memory");
         const int nvec = L.H / 8, parts = (nvec + 31) / 32, tasks = L.T * parts, K = L.K;
-        uint64_t waited = 0, first = 0;
+        const bool stamps = warp == 2 && lane == 0;              // (one warp's clock: atomics of all of them would be a microsecond of a small call)
+        uint64_t waited = 0, counted = 0;
         for (int task = (warp - 2) * (int)gridDim.x + (int)blockIdx.x; task < tasks; task += kFewSumWarps * (int)gridDim.x) {
             const int place = task / parts, col = (task - place * parts) * 32 + lane, at = min(col, nvec - 1);
             const int t = L.token_order[place], slot = lane < K ? L.order_slot[(long)place * K + lane] : -1;
             const uint32_t valid = __ballot_sync(0xffffffffu, slot >= 0);
             if (!wait_counts_warp(L.done2 + max(slot, 0) / kUnit, slot >= 0, kFewEpiWarps * n2, L.status, 685, waited)) break;      // reported: unwind
-            if (first == 0) first = globaltimer_ns();
             __syncwarp();                                        // every lane reads behind the other lanes' acquires
             float sum[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
             for (int k0 = 0; k0 < K; k0 += 8) {
@@ -347,6 +345,13 @@ __global__ void __launch_bounds__(kFewThreads, 1) local_few_kernel(const __grid_
                     if (k0 + j < K)
                         asm volatile("ld.global.cg.v4.s32 {%0, %1, %2, %3}, [%4];" : "=r"(v[j].x), "=r"(v[j].y), "=r"(v[j].z), "=r"(v[j].w)
                                      : "l"(reinterpret_cast<const int4*>(L.y) + (long)s * nvec + at));
+                }
+                if (stamps && k0 == 0) {                         // while the loads are under way: reading the clock takes long, and this may be the end
+                    const uint64_t now = globaltimer_ns();
+                    atomicMax(L.stats + kStatKindFirst + kWorkReduce, ~now);
+                    atomicMax(L.stats + kStatKindLast + kWorkReduce, now);
+                    if (waited != counted) atomicAdd(L.stats + kStatWaitLanded, (unsigned long long)(waited - counted));
+                    counted = waited;
                 }
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
@@ -363,11 +368,6 @@ __global__ void __launch_bounds__(kFewThreads, 1) local_few_kernel(const __grid_
             if (col < nvec)
                 reinterpret_cast<int4*>(L.out + (long)t * L.H)[col] = make_int4((int)pack_bf16x2(sum[0], sum[1]), (int)pack_bf16x2(sum[2], sum[3]),
                                                                                 (int)pack_bf16x2(sum[4], sum[5]), (int)pack_bf16x2(sum[6], sum[7]));
-        }
-        if (lane == 0 && first != 0) {
-            atomicMax(L.stats + kStatKindFirst + kWorkReduce, ~first);
-            atomicMax(L.stats + kStatKindLast + kWorkReduce, globaltimer_ns());
-            if (waited != 0) atomicAdd(L.stats + kStatWaitLanded, (unsigned long long)waited);
         }
     }
     tcgen05_fence_before();

@@ -1616,8 +1616,10 @@ LocalLayerPlan local_layer_plan(int T, int K, int E, int H, int I, int keep) {
     // H=7168 I=2048) 588 / 437, (I=512) 185 / 134, (64 experts, top-4, H=4096 I=768) 286 / 216, (64 experts, top-2, H=2048 I=512) 121 / 90.
     // An expert of more than 64 rows takes its weights again for every 64.  The host cannot see one, but that it matters takes tokens and a large layer:
     // if all T tokens chose the same K experts, K * (T / 64 - 1) units would read 6 H I bytes each.  Up to 128 tokens, or 96 MB, the kernel is
-    // ahead on any routing (512 tokens on two experts, H=2048 I=512, 84 MB 47 / 43).  Beyond, the routing decides on the GPU: both kernels are
-    // launched, and one returns at once, for 5 us (256 tokens, H=4096 I=768, 64 experts, top-4 268 / 215; all on two experts, H=7168 I=2048 95 / 98).
+    // ahead on any routing or close to it; us, general kernel / local_few.cu: 512 tokens on two experts, H=2048 I=512, 84 MB 49 / 41; H=7168,
+    // 128 tokens on two experts, I=2048 92 / 77, on eight, I=1024 130 / 123, 96 tokens on eight, I=768 103 / 110 (the worst that was
+    // found).  Beyond, the routing decides on the GPU: both kernels are launched, and one returns at once, for 5 us (256 tokens, H=4096 I=768, 64
+    // experts, top-4 268 / 215; all on two experts, H=7168 I=2048 95 / 98).
     const long again = (long)K * ((T + kFewUnitRows - 1) / kFewUnitRows - 1) * 6 * H * I;
     p.few = keep || T <= 0 || entries > (long)kFewRows * E ? 0 : T <= 2 * kFewUnitRows || again <= 96l << 20 ? 1 : 2;
     // Token rows through the loading warps, or copied into slot order first.  The loading warps load a row again for every tile of the other

@@ -465,7 +465,7 @@ def test_hooks_on_saved_tensors_see_no_workspace():
     buf.destroy()
 
 
-@pytest.mark.parametrize("T,E,few", [(32, 16, True), (512, 16, False)])
+@pytest.mark.parametrize("T,E,few", [(1, 16, True), (32, 16, True), (512, 16, False)])
 def test_a_forward_reports_its_spans_and_waits(T, E, few):
     """Every forward replaces the report of the one before, and its time stamps lie in the order of the work."""
     from teramoe_b200._build import load_ext
@@ -479,9 +479,10 @@ def test_a_forward_reports_its_spans_and_waits(T, E, few):
     spans = rep["spans_ms"]
     assert set(spans) == {"gemm1", "gemm2", "reduce"}
     assert all(0 <= a <= b < 100 for a, b in spans.values())
-    assert spans["gemm1"][0] == 0 and spans["gemm1"][0] < spans["gemm2"][0] < spans["reduce"][1]
-    assert spans["gemm1"][1] < spans["gemm2"][1] < spans["reduce"][1] and spans["gemm2"][1] > 0
-    assert rep["wait_first_gemm"] > 0 and rep["wait_landed"] > 0 and rep["wait_arrival"] == rep["wait_wgrad"] == 0
+    # (the clock ticks once in a microsecond or so)
+    assert spans["gemm1"][0] == 0 <= spans["gemm2"][0] < spans["reduce"][0] and 0 < spans["gemm1"][1] < spans["gemm2"][1] <= spans["reduce"][1]
+    assert rep["wait_arrival"] == rep["wait_wgrad"] == 0 and min(rep["wait_first_gemm"], rep["wait_landed"]) >= 0
+    assert T == 1 or (rep["wait_first_gemm"] > 0 and rep["wait_landed"] > 0)
     call(torch.full_like(r["idx"], -1))
     assert set(buf._engine.wait_report()["fwd"]["spans_ms"]) == {"reduce"}
     buf.destroy()
