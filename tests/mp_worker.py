@@ -359,8 +359,8 @@ def main():
             assert len(fds) == world and fds[rank] == fd
             for r, f in enumerate(fds):
                 assert f >= 0
-                os.lseek(f, 0, os.SEEK_SET)
-                assert os.read(f, 64).decode() == f"rank {r} round {rnd}", (r, rnd)
+                # (a descriptor that was passed on shares its position with the other ranks')
+                assert os.pread(f, 64, 0).decode() == f"rank {r} round {rnd}", (r, rnd)
             dist.barrier()
             for f in fds:
                 os.close(f)
