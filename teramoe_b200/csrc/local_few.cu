@@ -1,18 +1,20 @@
 // The layer's forward on one rank when experts have few rows (local_layer_plan decides), as in decoding: the time is that of reading the
-// weights once.  The weights are the M operand here, 128 rows of a tile, and an expert's tokens the N operand, 16 to 64 columns.  With the
+// weights once.  The weights are the M operand here, 128 rows of a tile, and an expert's tokens the N operand, 16 to 64 or 128 columns.  With the
 // roles of local_layer.cu eight tokens were multiplied as 256 rows; under the power cap, which such a call reaches too, the tensor
 // cores' share is bandwidth lost.  Forward of 32 tokens, H=7168 I=2048, 32 experts, top-8: 585 -> 430 us, 6.6 TB/s, which is what a plain
-// copy reaches; of 64 tokens 588 -> 437; with I=512 179 -> 132 and 185 -> 134.
+// copy reaches; of 64 tokens 588 -> 437; with I=512 179 -> 132 and 185 -> 134; of 128 and 256 tokens (32 and 64 rows per expert) 620 -> 467 and
+// 654 -> 548: every step brings a unit's rows from L2 next to the weights, half as many bytes again at 64 rows, which is what the time grows by.
 //
 // One persistent block per SM, no clusters.  Items: first the tiles of the first GEMM (128 rows of W_gateup of an expert x a unit of up to
-// 64 of its tokens), then those of the second, dealt out in turn: they nearly cost the same.  Units of one expert are neighbours, so that
+// 64 or 128 of its tokens), then those of the second, dealt out in turn: they nearly cost the same.  Units of one expert are neighbours, so that
 // they share the tile of weights in L2.
 //   warp 0     loads: weights by TMA boxes, the second GEMM's rows by boxes of 16
 //   warps 2, 3 load the first GEMM's token rows, every other step each, by cp.async
 //   warp 1     issues tcgen05.mma, 128 x N x 16, into one of four accumulators
 //   warps 4-7  epilogue: a lane holds one row of weights, so gate and up of a token sit in neighbouring lanes
 //   warps 2-7  at the end of their items: sums of the tokens' expert rows, in the order of their entries
-// Nine stages of 24 KB keep 144 KB of weights per SM on their way.
+// Nine stages of 24 KB keep 144 KB of weights per SM on their way; with units of 128 rows, six of 32 KB keep 96 KB, which costs 2 to 4 % where experts
+// have few rows (32 tokens as above 430 / 449) and saves reading weights again where many have more than 64 (256 tokens 651 / 539).
 #include "local_layer.h"
 
 #include "gemm_common.cuh"
@@ -24,17 +26,22 @@ using namespace detail;
 
 namespace {
 
-constexpr int kUnit = kFewUnitRows;
-constexpr int kFewStages = 9;
-constexpr int kFewStageBytes = kAStageBytes + kUnit * BK * 2;             // 24 KB
 constexpr int kFewAccs = 4;
 constexpr int kFewThreads = 256;
 constexpr int kFewEpiWarps = 4;
 constexpr int kFewSumWarps = 6;
-constexpr int kFewBarOffset = kFewStages * kFewStageBytes;
-constexpr int kFewUnitsOffset = kFewBarOffset + 256;                      // [experts + 1] first unit, [experts] rows, [experts] first slot
-constexpr int kFewSmemBytes = kFewUnitsOffset + (3 * kLocalMaxExperts + 1) * 4 + 1024;
-static_assert(8 * (2 * kFewStages + 2 * kFewAccs) <= 248 && kFewSmemBytes <= 232448, "shared memory");
+
+// What follows from the rows of a unit
+template <int UNIT>
+struct Few {
+    static constexpr int kStageBytes = kAStageBytes + UNIT * BK * 2;      // 24 KB, 32 KB
+    static constexpr int kStages = UNIT == 64 ? 9 : 6;
+    static constexpr int kBarOffset = kStages * kStageBytes;
+    static constexpr int kUnitsOffset = kBarOffset + 256;                 // [experts + 1] first unit, [experts] rows, [experts] first slot
+    static constexpr int kSmemBytes = kUnitsOffset + (3 * kLocalMaxExperts + 1) * 4 + 1024;
+    static_assert(8 * (2 * kStages + 2 * kFewAccs) <= 248 && kSmemBytes <= 232448, "shared memory");
+    static_assert(UNIT % 64 == 0 && 128 % UNIT == 0 && kFewAccs * UNIT <= 512, "units");
+};
 
 struct FewArgs {
     alignas(64) CUtensorMap map_wg, map_wd, map_act;
@@ -60,19 +67,21 @@ struct FewItem {
     int second, expert, tile, slot0, rows, n;      // n: columns of the accumulator that are computed
 };
 
+template <int UNIT>
 __global__ void __launch_bounds__(kFewThreads, 1) local_few_kernel(const __grid_constant__ FewArgs L) {
     if (L.wanted != nullptr && *L.wanted == 0) return;
+    constexpr int kUnit = UNIT, kFewStages = Few<UNIT>::kStages, kFewStageBytes = Few<UNIT>::kStageBytes;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
-    const uint32_t bar_base = smem_base + kFewBarOffset;
+    const uint32_t bar_base = smem_base + Few<UNIT>::kBarOffset;
     auto full_bar = [&](int s) { return bar_base + 8u * s; };
     auto empty_bar = [&](int s) { return bar_base + 8u * (kFewStages + s); };
     auto tfull_bar = [&](int a) { return bar_base + 8u * (2 * kFewStages + a); };
     auto tempty_bar = [&](int a) { return bar_base + 8u * (2 * kFewStages + kFewAccs + a); };
-    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + kFewBarOffset + 248);
+    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + Few<UNIT>::kBarOffset + 248);
     volatile uint32_t* abort_flag = tmem_slot + 1;
-    int* units = reinterpret_cast<int*>(smem_gen + kFewUnitsOffset);
+    int* units = reinterpret_cast<int*>(smem_gen + Few<UNIT>::kUnitsOffset);
     int* counts = units + L.E + 1;
     int* seg = counts + L.E;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, E = L.E;
@@ -237,8 +246,10 @@ __global__ void __launch_bounds__(kFewThreads, 1) local_few_kernel(const __grid_
         for (int i = blockIdx.x; i < U * n1 && ok; i += gridDim.x) {
             const FewItem q = decode(i);
             const int quads = (q.rows + 3) / 4;
-            // of rows lane, lane + 32; past the last row that one again, whose copies nobody reads (of all SMs the same row would be one hot line of L2)
-            const int token[2] = {L.slot_tk[q.slot0 + min(lane, q.rows - 1)] / L.K, L.slot_tk[q.slot0 + min(lane + 32, q.rows - 1)] / L.K};
+            // of rows lane + 32 c; past the last row that one again, whose copies nobody reads (of all SMs the same row would be one hot line of L2)
+            int token[kUnit / 32];
+#pragma unroll
+            for (int c = 0; c < kUnit / 32; ++c) token[c] = L.slot_tk[q.slot0 + min(lane + 32 * c, q.rows - 1)] / L.K;
             for (; step < nk1; step += 2) {
                 if (!(ok = mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag, L.status, 686))) break;
                 const uint32_t dst = smem_base + stage * kFewStageBytes + kAStageBytes;
@@ -278,7 +289,9 @@ __global__ void __launch_bounds__(kFewThreads, 1) local_few_kernel(const __grid_
             const bool ends = i + (int)gridDim.x >= (q.second ? items : U * n1);
             if (stamps && i - (int)gridDim.x < (q.second ? U * n1 : 0))
                 atomicMax(L.stats + kStatKindFirst + (q.second ? kWorkGemm2 : kWorkGemm1), ~globaltimer_ns());
-            const float w[2] = {!q.second && lane < q.rows ? L.slot_w[q.slot0 + lane] : 0.f, !q.second && lane + 32 < q.rows ? L.slot_w[q.slot0 + lane + 32] : 0.f};
+            float w[kUnit / 32];
+#pragma unroll
+            for (int c = 0; c < kUnit / 32; ++c) w[c] = !q.second && lane + 32 * c < q.rows ? L.slot_w[q.slot0 + lane + 32 * c] : 0.f;
             if (!mbar_wait(tfull_bar(acc), acc_phase, abort_flag, L.status, 684)) break;
             tcgen05_fence_after();
             const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * kUnit);
@@ -378,6 +391,26 @@ __global__ void __launch_bounds__(kFewThreads, 1) local_few_kernel(const __grid_
     }
 }
 
+template <int UNIT>
+cudaError_t launch(const FewArgs& L, int num_sms, cudaStream_t stream) {
+    static bool configured[64] = {};
+    if (cudaError_t e = ensure_smem_limit(local_few_kernel<UNIT>, Few<UNIT>::kSmemBytes, configured); e != cudaSuccess) return e;
+    const int sms = default_sms(num_sms) & ~1;
+    if (sms < 4) return cudaErrorInvalidConfiguration;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(sms);
+    cfg.blockDim = dim3(kFewThreads);
+    cfg.dynamicSmemBytes = Few<UNIT>::kSmemBytes;
+    cfg.stream = stream;
+    // blocks wait for tiles of other blocks: all of them have to be resident
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, local_few_kernel<UNIT>, L);
+}
+
 }  // namespace
 
 cudaError_t local_few_launch(const LocalLayerParams& q, cudaStream_t stream) {
@@ -409,22 +442,7 @@ cudaError_t local_few_launch(const LocalLayerParams& q, cudaStream_t stream) {
     L.stats = reinterpret_cast<unsigned long long*>(q.ws + p.stats[0]);
     L.status = q.status;
     L.wanted = p.few == 2 ? q.ws + p.meta + kMetaFew : nullptr;
-    static bool configured[64] = {};
-    if ((e = ensure_smem_limit(local_few_kernel, kFewSmemBytes, configured)) != cudaSuccess) return e;
-    const int sms = default_sms(q.num_sms) & ~1;
-    if (sms < 4) return cudaErrorInvalidConfiguration;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(sms);
-    cfg.blockDim = dim3(kFewThreads);
-    cfg.dynamicSmemBytes = kFewSmemBytes;
-    cfg.stream = stream;
-    // blocks wait for tiles of other blocks: all of them have to be resident
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeCooperative;
-    at[0].val.cooperative = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, local_few_kernel, L);
+    return p.few_unit == 64 ? launch<64>(L, q.num_sms, stream) : launch<128>(L, q.num_sms, stream);
 }
 
 }  // namespace tmoe

@@ -78,8 +78,6 @@ enum { kSyncItem = 0, kSyncToken = 1, kSyncCopy = 2, kSyncKeep = 3, kSyncFirsts 
 
 constexpr int kWideTiles = 74 * 4;                                        // least number of wide tiles of a GEMM (local_layer_plan)
 
-constexpr int kFewRows = 16;                                              // most rows per expert of a forward in local_few.cu (local_layer_plan)
-
 constexpr int column_blocks(int n, int cols) { return (n + cols - 1) / cols; }
 
 constexpr int kRouteThreads = 256;
@@ -209,7 +207,7 @@ __global__ void __launch_bounds__(kRouteThreads) local_route_assign_kernel(const
             const int e = e0 + lane;
             const int blocks = e < E ? (totals[e] + 127) / 128 : 0;
             hit += __popc(__ballot_sync(0xffffffffu, blocks != 0));
-            few_units += __reduce_add_sync(0xffffffffu, e < E ? (totals[e] + kFewUnitRows - 1) / kFewUnitRows : 0);
+            few_units += __reduce_add_sync(0xffffffffu, e < E ? (totals[e] + a.p.few_unit - 1) / a.p.few_unit : 0);
             int s = blocks * 128, u = (blocks + 1) / 2;
             const int s_own = s, u_own = u;
             for (int o = 1; o < 32; o <<= 1) {
@@ -234,7 +232,7 @@ __global__ void __launch_bounds__(kRouteThreads) local_route_assign_kernel(const
             // Units beyond an expert's first, each of which takes its weights again, from L2: as many as experts with rows at most.  us, general
             // kernel / local_few.cu (64 experts, top-4, H=7168 I=768, all tokens on four experts): 128 tokens, one such unit per expert, 88 / 76,
             // 256 tokens, three, 95 / 115.
-            *few_word = a.p.few == 1 || (a.p.few == 2 && few_units - hit <= hit);
+            *few_word = a.p.few == 1 || (a.p.few == 2 && (few_units - hit) * a.p.few_again <= hit);
         }
     }
     if (warp == 1) {
@@ -1612,16 +1610,29 @@ LocalLayerPlan local_layer_plan(int T, int K, int E, int H, int I, int keep) {
     p.slots_cap = p.blocks_cap * 128;
     p.units_cap = (int)((p.blocks_cap + segs) / 2);
     const int rows = (int)(entries / (segs > 0 ? segs : 1));
-    // Few rows per expert, forward only: weights as the M operand (local_few.cu).  us, here / there, by rows per expert: 16 (32 experts, top-8,
-    // H=7168 I=2048) 588 / 437, (I=512) 185 / 134, (64 experts, top-4, H=4096 I=768) 286 / 216, (64 experts, top-2, H=2048 I=512) 121 / 90.
-    // An expert of more than 64 rows takes its weights again for every 64.  The host cannot see one, but that it matters takes tokens and a large layer:
-    // if all T tokens chose the same K experts, K * (T / 64 - 1) units would read 6 H I bytes each.  Up to 128 tokens, or 96 MB, the kernel is
-    // ahead on any routing or close to it; us, general kernel / local_few.cu: 512 tokens on two experts, H=2048 I=512, 84 MB 49 / 41; H=7168,
-    // 128 tokens on two experts, I=2048 92 / 77, on eight, I=1024 130 / 123, 96 tokens on eight, I=768 103 / 110 (the worst that was
-    // found).  Beyond, the routing decides on the GPU: both kernels are launched, and one returns at once, for 5 us (256 tokens, H=4096 I=768, 64
-    // experts, top-4 268 / 215; all on two experts, H=7168 I=2048 95 / 98).
-    const long again = (long)K * ((T + kFewUnitRows - 1) / kFewUnitRows - 1) * 6 * H * I;
-    p.few = keep || T <= 0 || entries > (long)kFewRows * E ? 0 : T <= 2 * kFewUnitRows || again <= 96l << 20 ? 1 : 2;
+    // Few rows per expert, forward only: weights as the M operand (local_few.cu), 64 rows of an expert at a time, from 41 on average 128.  us, general
+    // kernel / 64 / 128, by rows per expert (even routing):
+    //   H=7168 I=2048, 32 experts, top-8   16 588 / 440 / 455   32 598 / 463 / 475   40 610 / 484 / 491   64 630 / 651 / 539    80 652 / 860 / 567
+    //   (as above)                         96 667 / 856 / 613   112 674 / 852 / 679  128 685 / 944 / 873
+    //   H=2048 I=512, 64, top-4            16 121 / 89 / 91     32 119 / 96 / 99     48 123 / 106 / 107   64 127 / 130 / 119    96 132 / 158 / 136
+    //   H=4096 I=1536, 16, top-2           16 153 / 116 / 120   32 150 / 123 / 129   48 157 / 130 / 135   64 162 / 152 / 143    96 165 / 197 / 161
+    // What an item of the second GEMM stores grows with the rows, what it reads with I: H=4096 I=256, 32 experts, top-2, 37 rows 89 / 85, 62 rows 94 / 102;
+    // hence the line at I / 10 rows, but for calls so small that latencies decide (H=2048 I=256, 8 experts, top-4, 50 rows 42 / 31).  With I >= 4096
+    // it stays at 16 rows: the rows of act that a tile reads are long there (H=1024 I=14336, 4 experts, 48 rows 138 / 131, 64 rows 139 / 149).
+    // An expert of more rows than a unit takes its weights again for every unit.  The host cannot see one, but that it matters takes tokens and a
+    // large layer: if all T tokens chose the same K experts, K * (T / 64 - 1) units would read 6 H I bytes each.  Up to 128 tokens, or with up to 16 rows
+    // on average 96 MB, the kernel is ahead on any routing or close to it; us, general kernel / local_few.cu: 512 tokens on two experts, H=2048 I=512,
+    // 84 MB 49 / 41; H=7168, 128 tokens on two experts, I=2048 92 / 77, on four 122 / 114, on eight, I=1024 130 / 123, I=768 114 / 114, 96 tokens on
+    // eight, I=768 103 / 110, 128 tokens with 32 rows on average on eight of 32, I=768 102 / 112 (the worst that was found).  Beyond, the routing decides on the GPU: both kernels are launched, and one returns at once,
+    // for 5 us (256 tokens, H=4096 I=768, 64 experts, top-4 268 / 215; all on two experts, H=7168 I=2048 95 / 98).  Kept to 1 / few_again of the
+    // experts with rows, such units cost less than the kernel gains: 192 tokens, H=7168 I=512, hottest expert three times the mean 195 / 167; 320, I=2048
+    // 619 / 612.
+    const bool sixteen = entries <= 16l * E;
+    p.few_unit = entries <= 40l * E || T <= 64 ? 64 : 128;
+    p.few_again = sixteen ? 1 : p.few_unit == 64 ? 2 : 3;
+    const long again = (long)K * ((T + 63) / 64 - 1) * 6 * H * I;
+    const bool few = sixteen || (I < 4096 && entries <= 80l * E && (T <= 128 || 10 * entries <= (long)I * E));
+    p.few = keep || T <= 0 || !few ? 0 : T <= 128 || (sixteen && again <= 96l << 20) ? 1 : 2;
     // Token rows through the loading warps, or copied into slot order first.  The loading warps load a row again for every tile of the other
     // operand, with more energy per byte than TMA; a copy is written and read once.  us of a step, backward by loaders / by copies, by rows per
     // expert:
@@ -1678,9 +1689,9 @@ LocalLayerPlan local_layer_plan(int T, int K, int E, int H, int I, int keep) {
     for (int d = 0; d < dirs; ++d) {
         p.stats[d] = take(2 * kLayerStatWords);
         p.sync[d] = take(kSyncWords);
-        p.done1[d] = take(p.few ? 128 / kFewUnitRows * p.blocks_cap : p.units_cap);
+        p.done1[d] = take(p.few ? 2 * p.blocks_cap : p.units_cap);
         p.arrived[d] = take(p.copies[d] ? p.blocks_cap : 0);
-        p.done2[d] = take(p.few ? 128 / kFewUnitRows * p.blocks_cap : p.blocks_cap);
+        p.done2[d] = take(p.few ? 2 * p.blocks_cap : p.blocks_cap);
     }
     p.zero_words = at;
     p.meta = take(kMetaWords);

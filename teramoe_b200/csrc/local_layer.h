@@ -8,7 +8,6 @@
 
 namespace tmoe {
 
-constexpr int kFewUnitRows = 64;         // rows of an expert that local_few.cu multiplies at a time
 constexpr int kLocalMaxExperts = 512;    // the routing kernels keep 23 words per expert in shared memory
 
 // words of the meta block
@@ -20,6 +19,8 @@ struct LocalLayerPlan {
     int T, K, E, H, I, keep;             // keep: tables of the backward pass too
     int copies[2];                       // per direction: token rows are copied into slot order, not loaded by the slot table
     int few;                             // a forward with few rows per expert: 1 local_few.cu, 2 local_few.cu if the routing says so (kMetaFew)
+    int few_unit;                        // rows of an expert that it multiplies at a time: 64 or 128
+    int few_again;                       // with few = 2: most units beyond an expert's first, as a share of the experts with rows: 1 / few_again
     int chunks;                          // blocks of the routing kernels
     int slots_cap, blocks_cap, units_cap;
     int work_cap[2];                     // items of the forward / backward list

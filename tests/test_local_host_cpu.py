@@ -128,3 +128,15 @@ def test_kernels_of_a_call_by_its_sizes():
     assert variant(511, 2, 4, 512, True) == (0, 0, 1)
     assert variant(512, 2, 4, 512, True) == (0, 0, 0)
     assert variant(0, 2, 4, 512, False) == (0, 0, 0)
+
+
+def test_which_forwards_have_few_rows_per_expert():
+    """Up to 16 rows on average, up to 80 where I is below 4096 and either at least ten times that or there are 128 tokens at most."""
+    from teramoe_b200._build import load_ext
+    few = lambda T, K, E, I: load_ext().local_layer_variant(T, K, E, 4096, I, False)["few"]
+    assert [few(T, 2, 8, 256) for T in (64, 65, 128)] == [1, 1, 1]
+    assert [few(T, 2, 16, 256) for T in (128, 129, 204, 205)] == [1, 2, 2, 0]
+    assert [few(T, 2, 8, 4032) for T in (128, 129, 320, 321)] == [1, 2, 2, 0]
+    assert [few(T, 2, 8, 4096) for T in (64, 65)] == [1, 0]
+    assert few(128, 8, 8, 4032) == 0
+    assert load_ext().local_layer_variant(128, 2, 8, 4096, 4032, True)["few"] == 0

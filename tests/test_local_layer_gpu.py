@@ -202,6 +202,40 @@ def test_forward_with_few_rows_per_expert(counts, empty, H, I, K, monkeypatch):
     buf.destroy()
 
 
+@pytest.mark.parametrize("counts,E,T,H,I,few,ran", [
+    ([70, 33, 15, 5], 8, 128, 320, 64, 1, True),         # units of 64 rows
+    ([65, 64, 63, 33, 31, 17, 16, 15], 25, 307, 192, 256, 2, True),
+    ([200, 50, 50], 25, 307, 1088, 320, 2, False),       # three units beyond the first ones of three experts
+    ([100, 20, 5], 4, 128, 320, 64, 1, True),            # units of 128 rows
+    ([60, 1], 3, 64, 320, 64, 1, True),                  # (not where there are no more tokens than 64)
+    ([1, 15, 17, 33, 64, 65, 95, 96, 97, 127, 128, 129], 30, 870, 192, 640, 2, True),      # a last tile of weights that is half outside
+    ([1, 15, 17, 33, 64, 65, 95, 96, 97, 127, 128, 129], 30, 870, 1088, 1024, 2, True),
+    ([257, 129, 128], 24, 520, 1088, 448, 2, False),     # as many units beyond the first as experts
+])
+def test_forward_with_up_to_eighty_rows_per_expert(counts, E, T, H, I, few, ran, monkeypatch):
+    """Rows at the edges of row copies (4), accumulator columns (16), reads of the accumulator (32) and units (64, 128); which kernel takes the
+    call; twice, and on fewer SMs: the bits of the several-rank kernels each time."""
+    from teramoe_b200 import engine
+    from teramoe_b200._build import load_ext
+    assert 16 * E < 2 * T <= 80 * E and load_ext().local_layer_variant(T, 2, E, H, I, False)["few"] == few
+    idx = torch.full((T, 2), -1, dtype=torch.int64)
+    idx[: sum(counts), 1] = torch.repeat_interleave(torch.arange(len(counts)), torch.tensor(counts))
+    idx = idx[torch.randperm(T, generator=torch.Generator().manual_seed(1))].cuda()
+    prob = make_problem(1, T, H, I, E, 2, seed=8, dtype=torch.bfloat16, device="cuda", x_scale=0.1, w_scale=0.02)
+    r = prob["ranks"][0]
+    buf = tm.Buffer(None, int(64e6), explicitly_destroy=True)
+    call = lambda **kw: buf.teramoe_forward(r["x"], idx, r["w"], prob["W_gateup"], prob["W_down"], E, **kw)
+    with monkeypatch.context() as m:
+        m.setattr(engine, "_LOCAL_LAYER_MODE", "0")
+        for name in ("_FUSED_DISPATCH_MODE", "_FUSED_MODE", "_LAYER_KERNEL_MODE"):
+            m.setattr(engine, name, "1")
+        want = call()
+    for kw in ({}, {}, dict(total_sms=16, num_dispatch_sms=4, num_combine_sms=4)):
+        assert torch.equal(call(**kw), want) and buf._engine.native.ran_few() == ran
+    buf.check_status()
+    buf.destroy()
+
+
 @pytest.mark.parametrize("counts,H,I,few", [
     ([64] * 20 + [8] * 10, 4096, 1024, True),            # no second unit
     ([129] * 6 + [64] * 6, 4096, 1024, True),            # as many as experts with rows
