@@ -490,7 +490,7 @@ class LocalLayer : public std::enable_shared_from_this<LocalLayer> {
         {
             std::lock_guard<std::mutex> lock(arena_mutex_);
             set_common(p, schedule);
-            TM_CHECK_CUDA(tmoe::local_layer_route(p, stream));
+            if (!p.plan.routes) TM_CHECK_CUDA(tmoe::local_layer_route(p, stream));
             TM_CHECK_CUDA(tmoe::local_layer_launch(p, stream));
         }
         note(0, ws, p.plan);

@@ -15,10 +15,18 @@
 //   warps 2-7  at the end of their items: sums of the tokens' expert rows, in the order of their entries
 // Nine stages of 24 KB keep 144 KB of weights per SM on their way; with units of 128 rows, six of 32 KB keep 96 KB, which costs 2 to 4 % where experts
 // have few rows (32 tokens as above 430 / 449) and saves reading weights again where many have more than 64 (256 tokens 651 / 539).
+//
+// Where the host can tell that this kernel takes the call (LocalLayerPlan::routes) it makes the routing tables too, in front of a barrier of the whole grid:
+// a kernel of their own costs 5 us, and a boundary between two kernels of a stream up to 2 us more.  us of a forward, routing kernel / here / here with the
+// first weights on their way meanwhile: one token, H=2048 I=768, 16 experts, top-4 28.7 / 26.7 / 26.7, 30, H=1024 I=512, 8, top-2 24.6 / 22.6 / 22.6,
+// 64, H=7168 I=512, 32, top-8 138 / 136 / 133, 400, H=1024 I=256, 64, top-2 37.0 / 35.7 / 34.9.
 #include "local_layer.h"
+
+#include <cooperative_groups.h>
 
 #include "gemm_common.cuh"
 #include "layer.h"
+#include "local_route.cuh"
 
 namespace tmoe {
 
@@ -40,6 +48,7 @@ struct Few {
     static constexpr int kUnitsOffset = kBarOffset + 256;                 // [experts + 1] first unit, [experts] rows, [experts] first slot
     static constexpr int kSmemBytes = kUnitsOffset + (3 * kLocalMaxExperts + 1) * 4 + 1024;
     static_assert(8 * (2 * kStages + 2 * kFewAccs) <= 248 && kSmemBytes <= 232448, "shared memory");
+    static_assert(kFewThreads == kRouteThreads, "routing");
     static_assert(UNIT % 64 == 0 && 128 % UNIT == 0 && kFewAccs * UNIT <= 512, "units");
 };
 
@@ -50,7 +59,6 @@ struct FewArgs {
     __nv_bfloat16* act;
     __nv_bfloat16* y;
     __nv_bfloat16* out;
-    const int* seg;
     const int* counts;
     const int* slot_tk;
     const float* slot_w;
@@ -67,8 +75,8 @@ struct FewItem {
     int second, expert, tile, slot0, rows, n;      // n: columns of the accumulator that are computed
 };
 
-template <int UNIT>
-__global__ void __launch_bounds__(kFewThreads, 1) local_few_kernel(const __grid_constant__ FewArgs L) {
+template <int UNIT, bool ROUTES>
+__global__ void __launch_bounds__(kFewThreads, 1) local_few_kernel(const __grid_constant__ FewArgs L, const __grid_constant__ RouteArgs R) {
     if (L.wanted != nullptr && *L.wanted == 0) return;
     constexpr int kUnit = UNIT, kFewStages = Few<UNIT>::kStages, kFewStageBytes = Few<UNIT>::kStageBytes;
     extern __shared__ uint8_t smem_raw[];
@@ -102,21 +110,47 @@ __global__ void __launch_bounds__(kFewThreads, 1) local_few_kernel(const __grid_
         tma_prefetch_desc(&L.map_act);
     }
     if (warp == 2) tmem_alloc(smem_u32((const void*)tmem_slot), kFewAccs * kUnit);
+    // Routing in the same launch: a few blocks write the tables, the others only count.  All know the units then, and those others have the weights
+    // of their first item on their way while they wait for the tables.  (The stages that the routing works in, the last ones, are left out.)
+    constexpr int kRouteStages = 2;
+    static_assert(route_words(kLocalMaxExperts) * 4 <= kRouteStages * kFewStageBytes, "routing");
+    int* route = reinterpret_cast<int*>(smem_gen + (kFewStages - kRouteStages) * kFewStageBytes);
+    bool counts_only = false;
+    if constexpr (ROUTES) {
+        __shared__ int bound[4];
+        clear_counters(R);
+        const int blocks = R.p.chunks + kRouteTableBlocks;
+        counts_only = (int)blockIdx.x >= blocks;
+        if (counts_only) {
+            for (int i = threadIdx.x; i < 2 * E + 1; i += kFewThreads) route[route_totals(E) + i] = 0;
+            __syncthreads();
+            count_entries(R, route + route_totals(E), nullptr, 0);
+        }
+        for (int b = blockIdx.x; b < blocks; b += gridDim.x) {
+            __syncthreads();
+            route_assign<true>(R, route, bound, b, blocks);
+        }
+        __syncthreads();
+    }
     if (warp == 1) {
-        int run = 0;
+        int run = 0, run_s = 0;
         for (int e0 = 0; e0 < E; e0 += 32) {
-            const int e = e0 + lane, c = e < E ? L.counts[e] : 0, own = (c + kUnit - 1) / kUnit;
-            int v = own;
+            const int e = e0 + lane, c = e < E ? (ROUTES ? route[route_totals(E) + e] : L.counts[e]) : 0, own = (c + kUnit - 1) / kUnit, own_s = (c + 127) & ~127;
+            int v = own, s = own_s;
             for (int o = 1; o < 32; o <<= 1) {
-                const int u = __shfl_up_sync(0xffffffffu, v, o);
-                if (lane >= o) v += u;
+                const int u = __shfl_up_sync(0xffffffffu, v, o), us = __shfl_up_sync(0xffffffffu, s, o);
+                if (lane >= o) {
+                    v += u;
+                    s += us;
+                }
             }
             if (e < E) {
                 units[e] = run + v - own;
                 counts[e] = c;
-                seg[e] = L.seg[e];
+                seg[e] = run_s + s - own_s;
             }
             run += __shfl_sync(0xffffffffu, v, 31);
+            run_s += __shfl_sync(0xffffffffu, s, 31);
         }
         if (lane == 0) units[E] = run;
     }
@@ -146,6 +180,22 @@ __global__ void __launch_bounds__(kFewThreads, 1) local_few_kernel(const __grid_
         return q;
     };
     const int nk1 = L.H / BK, nk2 = L.I / BK;
+    int primed = 0;                                              // steps of this block's first item whose weights are on their way
+    if constexpr (ROUTES) {
+        fence_proxy_async_smem();                                // what the routing wrote is written over by copies
+        if (counts_only && (int)blockIdx.x < U * n1) {
+            primed = min(nk1, kFewStages - kRouteStages);
+            if (warp == 0 && lane == 0) {
+                const FewItem q = decode(blockIdx.x);
+                for (int s = 0; s < primed; ++s) {
+                    mbar_arrive_expect_tx(full_bar(s), kAStageBytes);
+                    tma_load_2d(smem_base + s * kFewStageBytes, &L.map_wg, full_bar(s), s * BK, q.expert * 2 * L.I + q.tile * BM);
+                }
+            }
+            __syncwarp();
+        }
+        cooperative_groups::this_grid().sync();
+    }
 
     if (warp == 0) {
         int stage = 0;
@@ -169,7 +219,7 @@ __global__ void __launch_bounds__(kFewThreads, 1) local_few_kernel(const __grid_
                 return true;
             };
             // the weights of a second GEMM's first steps come while its rows are waited for
-            int early = 0;
+            int early = i == (int)blockIdx.x ? primed : 0;
             if (q.second) {
                 const int* flag = L.done1 + q.slot0 / kUnit;
                 int ready = lane == 0 ? ld_acquire_gpu(flag) >= kFewEpiWarps * n1 : 0;
@@ -391,10 +441,10 @@ __global__ void __launch_bounds__(kFewThreads, 1) local_few_kernel(const __grid_
     }
 }
 
-template <int UNIT>
-cudaError_t launch(const FewArgs& L, int num_sms, cudaStream_t stream) {
+template <int UNIT, bool ROUTES>
+cudaError_t launch(const FewArgs& L, const RouteArgs& R, int num_sms, cudaStream_t stream) {
     static bool configured[64] = {};
-    if (cudaError_t e = ensure_smem_limit(local_few_kernel<UNIT>, Few<UNIT>::kSmemBytes, configured); e != cudaSuccess) return e;
+    if (cudaError_t e = ensure_smem_limit(local_few_kernel<UNIT, ROUTES>, Few<UNIT>::kSmemBytes, configured); e != cudaSuccess) return e;
     const int sms = default_sms(num_sms) & ~1;
     if (sms < 4) return cudaErrorInvalidConfiguration;
     cudaLaunchConfig_t cfg = {};
@@ -408,7 +458,7 @@ cudaError_t launch(const FewArgs& L, int num_sms, cudaStream_t stream) {
     at[0].val.cooperative = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, local_few_kernel<UNIT>, L);
+    return cudaLaunchKernelEx(&cfg, local_few_kernel<UNIT, ROUTES>, L, R);
 }
 
 }  // namespace
@@ -416,6 +466,7 @@ cudaError_t launch(const FewArgs& L, int num_sms, cudaStream_t stream) {
 cudaError_t local_few_launch(const LocalLayerParams& q, cudaStream_t stream) {
     const LocalLayerPlan& p = q.plan;
     const int H = p.H, I = p.I, E = p.E;
+    if (q.group_units <= 0 || q.lag_percent < 0 || q.lag_percent > 100) return cudaErrorInvalidValue;
     if (!p.few || q.bwd || H % BK != 0 || I % BK != 0 || q.out_rows < p.slots_cap || p.K < 1 || p.K > 32 || E < 1 || E > kLocalMaxExperts)
         return cudaErrorInvalidValue;
     if (reinterpret_cast<uintptr_t>(q.x) % 16 != 0) return cudaErrorInvalidValue;
@@ -431,7 +482,6 @@ cudaError_t local_few_launch(const LocalLayerParams& q, cudaStream_t stream) {
     L.act = static_cast<__nv_bfloat16*>(q.act);
     L.y = static_cast<__nv_bfloat16*>(q.y);
     L.out = static_cast<__nv_bfloat16*>(q.out);
-    L.seg = q.ws + p.seg;
     L.counts = q.ws + p.counts;
     L.slot_tk = q.ws + p.slot_tk;
     L.slot_w = reinterpret_cast<const float*>(q.ws + p.slot_w);
@@ -442,7 +492,9 @@ cudaError_t local_few_launch(const LocalLayerParams& q, cudaStream_t stream) {
     L.stats = reinterpret_cast<unsigned long long*>(q.ws + p.stats[0]);
     L.status = q.status;
     L.wanted = p.few == 2 ? q.ws + p.meta + kMetaFew : nullptr;
-    return p.few_unit == 64 ? launch<64>(L, q.num_sms, stream) : launch<128>(L, q.num_sms, stream);
+    if (!p.routes) return p.few_unit == 64 ? launch<64, false>(L, {}, q.num_sms, stream) : launch<128, false>(L, {}, q.num_sms, stream);
+    const RouteArgs R = local_route_args(q);
+    return p.few_unit == 64 ? launch<64, true>(L, R, q.num_sms, stream) : launch<128, true>(L, R, q.num_sms, stream);
 }
 
 }  // namespace tmoe

@@ -21,6 +21,7 @@ struct LocalLayerPlan {
     int few;                             // a forward with few rows per expert: 1 local_few.cu, 2 local_few.cu if the routing says so (kMetaFew)
     int few_unit;                        // rows of an expert that it multiplies at a time: 64 or 128
     int few_again;                       // with few = 2: most units beyond an expert's first, as a share of the experts with rows: 1 / few_again
+    int routes;                          // local_few.cu makes the routing tables itself: there is no routing kernel
     int chunks;                          // blocks of the routing kernels
     int slots_cap, blocks_cap, units_cap;
     int work_cap[2];                     // items of the forward / backward list
@@ -61,7 +62,7 @@ struct LocalLayerParams {
     int* status;
 };
 
-// Routing tables and both work lists (p: plan, ws, topk_*, schedule).
+// Routing tables and both work lists (p: plan, ws, topk_*, schedule).  Not called with plan.routes.
 cudaError_t local_layer_route(const LocalLayerParams& p, cudaStream_t stream);
 cudaError_t local_layer_launch(const LocalLayerParams& p, cudaStream_t stream);
 // The forward of plans with `few` (local_few.cu); local_layer_launch calls it.
