@@ -260,11 +260,16 @@ __device__ __forceinline__ void logfmt_roundtrip_group(float (&v)[8]) {
     logfmt_range(v, amax, amin);
     logfmt_params(amax, amin, log_amin, step, use);
     if (!use) return;
+    // logfmt_value(logfmt_code(a)) without the way through an integer: the conversions and floorf run at an eighth of the other instructions' rate.
+    // The codes are below 2^23, so that adding 2^23, rounded down, leaves the floor of what is not negative; what is becomes code 1 either way.
     const float inv_step = 1.f / fmaxf(step, 1e-30f);
 #pragma unroll
     for (int c = 0; c < 8; ++c) {
-        const float a = logfmt_value(logfmt_code(fabsf(v[c]), log_amin, inv_step), log_amin, step);
-        v[c] = v[c] < 0.f ? -a : a;
+        const float a = fabsf(v[c]);
+        const float at = (log2f(fmaxf(a, 1e-38f)) - log_amin) * inv_step + 0.5f;
+        const float code = fminf(fmaxf(__fadd_rd(at, 8388608.f) - 8388608.f + 1.f, 1.f), 511.f);
+        const float r = a > 0.f ? exp2f((code - 1.f) * step + log_amin) : 0.f;
+        v[c] = v[c] < 0.f ? -r : r;
     }
 }
 
@@ -429,6 +434,9 @@ ll_combine_recv_kernel(LowLatLayout lay, const uint8_t* arena, const void* topk_
 // Measured as dispatch + combine through the API, hidden 7168, top-8, 32 experts: 128 tokens, FP8 out and bf16 back 392 -> 52 us
 // (the window kernels alone took 301 us: a block per expert found its tokens and cast every row once per expert, and the
 // combine waited for one load after the other); 77 tokens, UE8M0 out and LogFMT-10 back with hooks 580 -> 51 us.
+// The kernels themselves, us, with 64 experts at 512 tokens: dispatch with FP8 of 16 tokens 3.8, 128 5.9, 512 13.7 (before, with a division per row for the
+// place of its scale, indices of earlier tokens one at a time and a match.any: 4.8, 8.5, 19.7); combine of LogFMT rows of 1 token 3.4, 77 15.1,
+// 512 84 (13.4, 18.0, 99), of bf16 rows 2.7, 3.6, 12.2.
 // ---------------------------------------------------------------------------------------------------------------
 constexpr int kLocalThreads = 256;
 constexpr int kLocalWarps = kLocalThreads / 32;
@@ -442,6 +450,7 @@ ll_local_dispatch_kernel(LowLatLayout lay, const __nv_bfloat16* x, const void* t
                          uint8_t* recv_scales, int* src_info, long long* layout_range, int* recv_count, int* expert_stats, int* entry_row) {
     extern __shared__ int table[];                 // [experts]: slot of the expert among this token's entries / row count
     __shared__ int first_of[kMaxTopK], count[kMaxTopK], row_of[kMaxTopK];
+    __shared__ long long scale_of[kMaxTopK];       // where the row's first scale is, in floats (UE8M0: in words of four)
     const int E = lay.num_experts, M = lay.max_tokens, H = lay.hidden, G = H / 128;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if ((int)blockIdx.x == T * splits) {
@@ -461,6 +470,10 @@ ll_local_dispatch_kernel(LowLatLayout lay, const __nv_bfloat16* x, const void* t
         return;
     }
     const int t = blockIdx.x / splits, part = blockIdx.x - t * splits;
+    // this warp's first 256 channels are requested before the rows are known
+    const int c_first = part * kLocalWarps + warp;
+    uint4 raw_first = make_uint4(0u, 0u, 0u, 0u);
+    if (c_first < H / 256) raw_first = *reinterpret_cast<const uint4*>(x + (size_t)t * H + c_first * 256 + lane * 8);
     for (int e = tid; e < E; e += kLocalThreads) table[e] = -1;
     if (tid < kMaxTopK) count[tid] = 0;
     __syncthreads();
@@ -470,16 +483,27 @@ ll_local_dispatch_kernel(LowLatLayout lay, const __nv_bfloat16* x, const void* t
             const long long v = load_idx(topk_idx, is64, (long)t * K + lane);
             if (v >= 0 && v < E) e = (int)v;
         }
-        const uint32_t same = __match_any_sync(0xffffffffu, e);
+        // lanes with the same expert, by votes on the bits of its number (match.any takes a step per different number)
+        uint32_t same = 0xffffffffu;
+        const int id = e < 0 ? E : e;
+        for (int bit = 0; (E >> bit) != 0; ++bit) {
+            const bool one = (id >> bit) & 1;
+            const uint32_t ones = __ballot_sync(0xffffffffu, one);
+            same &= one ? ones : ~ones;
+        }
         first_of[lane] = __ffs(same) - 1;
         row_of[lane] = e < 0 ? -1 : __popc(same & ((1u << lane) - 1u));      // rank among this token's own entries for the expert
         if (e >= 0 && first_of[lane] == lane) table[e] = lane;
     }
     __syncthreads();
-    for (int i = tid; i < t * K; i += kLocalThreads) {
-        const long long e = load_idx(topk_idx, is64, i);
-        if (e >= 0 && e < E) {
-            const int k = table[(int)e];
+    for (int i0 = tid; i0 < t * K; i0 += 4 * kLocalThreads) {
+        long long e[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) e[j] = i0 + j * kLocalThreads < t * K ? load_idx(topk_idx, is64, i0 + j * kLocalThreads) : -1;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            if (e[j] < 0 || e[j] >= E) continue;
+            const int k = table[(int)e[j]];
             if (k >= 0) atomicAdd(&count[k], 1);
         }
     }
@@ -492,6 +516,8 @@ ll_local_dispatch_kernel(LowLatLayout lay, const __nv_bfloat16* x, const void* t
         }
         __syncwarp();
         row_of[lane] = row;
+        const int re = max(row, 0) / M;
+        scale_of[lane] = (long long)re * (lay.use_ue8m0 ? G / 4 : G) * M + (max(row, 0) - re * M);
         if (part == 0) {
             if (lane < K) entry_row[(long)t * K + lane] = row;
             if (row >= 0) src_info[row] = t;
@@ -499,8 +525,8 @@ ll_local_dispatch_kernel(LowLatLayout lay, const __nv_bfloat16* x, const void* t
     }
     __syncthreads();
     const int half = lane >> 4, j = lane & 15;
-    for (int c = part * kLocalWarps + warp; c < H / 256; c += splits * kLocalWarps) {
-        const uint4 raw = *reinterpret_cast<const uint4*>(x + (size_t)t * H + c * 256 + lane * 8);
+    for (int c = c_first; c < H / 256; c += splits * kLocalWarps) {
+        const uint4 raw = c == c_first ? raw_first : *reinterpret_cast<const uint4*>(x + (size_t)t * H + c * 256 + lane * 8);
         if (!lay.use_fp8) {
             for (int k = 0; k < K; ++k) {
                 const int row = row_of[k];
@@ -516,61 +542,68 @@ ll_local_dispatch_kernel(LowLatLayout lay, const __nv_bfloat16* x, const void* t
 #pragma unroll
         for (int o = 8; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
         amax = fmaxf(amax, kFp8Margin);
-        const float s = fp8_scale(amax, lay.round_scale);
+        const float s = fp8_scale(amax, lay.round_scale), inverse = 1.f / s;
         uint32_t word[2] = {0u, 0u};
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-            const float q = fminf(fmaxf(__fdiv_rn(v[i], s), -kFp8Max), kFp8Max);
+            // (dividing by a power of two is multiplying by another; the scales are 2^-22 and more)
+            const float scaled = lay.round_scale ? v[i] * inverse : __fdiv_rn(v[i], s);
+            const float q = fminf(fmaxf(scaled, -kFp8Max), kFp8Max);
             word[i >> 2] |= (uint32_t)__nv_cvt_float_to_fp8(q, __NV_SATFINITE, __NV_E4M3) << (8 * (i & 3));
         }
         const int g = 2 * c + half;
+        // scales of an expert are column-major: [G (UE8M0: G/4 words of four bytes), M]
+        const size_t scale_col = lay.use_ue8m0 ? (size_t)(g >> 2) * M : (size_t)g * M;
         for (int k = 0; k < K; ++k) {
             const int row = row_of[k];
             if (row < 0) continue;
             *reinterpret_cast<uint2*>(recv_x + (size_t)row * H + c * 256 + lane * 8) = make_uint2(word[0], word[1]);
             if (j == 0) {
-                // scales of an expert are column-major: [G (UE8M0: G/4 words of four bytes), M]
-                const int e = row / M, r = row - e * M;
-                if (lay.use_ue8m0) recv_scales[(((size_t)e * (G / 4) + (g >> 2)) * M + r) * 4 + (g & 3)] = (uint8_t)(__float_as_uint(s) >> 23);
-                else reinterpret_cast<float*>(recv_scales)[((size_t)e * G + g) * M + r] = s;
+                const size_t at = (size_t)scale_of[k] + scale_col;
+                if (lay.use_ue8m0) recv_scales[at * 4 + (g & 3)] = (uint8_t)(__float_as_uint(s) >> 23);
+                else reinterpret_cast<float*>(recv_scales)[at] = s;
             }
         }
     }
 }
 
-// out[t] = sum over k of w[t,k] * x[row of (t,k)], k ascending.  `entry_row` is where the dispatch put the token's entries; an
-// entry is looked up by its expert, so the routing may come with entries removed or reordered.  With LogFMT the row's
-// groups go through the same encoder and decoder as on the wire.  A warp owns 256 channels; all rows are requested
+// Row in x and weight of entry `lane` of token t.  `entry_row` is where the dispatch put the token's entries; an entry is looked up by its expert,
+// so the routing may come with entries removed or reordered.
+__device__ __forceinline__ void combine_entry(const LowLatLayout& lay, const void* topk_idx, int is64, const float* topk_w, const int* entry_row, int t, int K,
+                                              int entry_t, int entry_k, int lane, int& row, float& w) {
+    int e = -1, at = -1;
+    row = -1;
+    w = 0.f;
+    if (lane < K) {
+        const long long v = load_idx(topk_idx, is64, (long)t * K + lane);
+        if (v >= 0 && v < lay.num_experts) {
+            e = (int)v;
+            w = topk_w[(long)t * K + lane];
+        }
+    }
+    if (lane < entry_k && t < entry_t) at = entry_row[(long)t * entry_k + lane];
+    const int at_e = at < 0 ? -2 : at / lay.max_tokens;
+    if (e == at_e) row = at;
+    if (__any_sync(0xffffffffu, e >= 0 && row < 0)) {
+        for (int k = 0; k < entry_k; ++k) {
+            const int e2 = __shfl_sync(0xffffffffu, at_e, k), r2 = __shfl_sync(0xffffffffu, at, k);
+            if (e >= 0 && row < 0 && e2 == e) row = r2;
+        }
+    }
+}
+
+// out[t] = sum over k of w[t,k] * x[row of (t,k)], k ascending.  A warp owns 256 channels; all rows are requested
 // before the first is used (eight loads in flight per lane).
-template <bool LOGFMT>
 __global__ void __launch_bounds__(128)
 ll_local_combine_kernel(LowLatLayout lay, const __nv_bfloat16* x, const void* topk_idx, int is64, const float* topk_w, const int* entry_row, int T,
                         int K, int entry_t, int entry_k, __nv_bfloat16* out) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int t = blockIdx.x, c = blockIdx.y * 4 + warp;
-    const int M = lay.max_tokens, H = lay.hidden;
+    const int H = lay.hidden;
     if (c >= H / 256) return;
-    int row = -1;
-    float w = 0.f;
-    {
-        int e = -1, at = -1;
-        if (lane < K) {
-            const long long v = load_idx(topk_idx, is64, (long)t * K + lane);
-            if (v >= 0 && v < lay.num_experts) {
-                e = (int)v;
-                w = topk_w[(long)t * K + lane];
-            }
-        }
-        if (lane < entry_k && t < entry_t) at = entry_row[(long)t * entry_k + lane];
-        const int at_e = at < 0 ? -2 : at / M;
-        if (e == at_e) row = at;
-        if (__any_sync(0xffffffffu, e >= 0 && row < 0)) {
-            for (int k = 0; k < entry_k; ++k) {
-                const int e2 = __shfl_sync(0xffffffffu, at_e, k), r2 = __shfl_sync(0xffffffffu, at, k);
-                if (e >= 0 && row < 0 && e2 == e) row = r2;
-            }
-        }
-    }
+    int row;
+    float w;
+    combine_entry(lay, topk_idx, is64, topk_w, entry_row, t, K, entry_t, entry_k, lane, row, w);
     const size_t col = (size_t)c * 256 + lane * 8;
     float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     for (int k0 = 0; k0 < K; k0 += 8) {
@@ -587,8 +620,7 @@ ll_local_combine_kernel(LowLatLayout lay, const __nv_bfloat16* x, const void* to
             const float wk = __shfl_sync(0xffffffffu, w, (k0 + i) & 31);
             if (k0 + i >= K || r < 0) continue;
             const float2 a = unpack_bf16x2(raw[i].x), b = unpack_bf16x2(raw[i].y), d = unpack_bf16x2(raw[i].z), f = unpack_bf16x2(raw[i].w);
-            float v[8] = {a.x, a.y, b.x, b.y, d.x, d.y, f.x, f.y};
-            if constexpr (LOGFMT) logfmt_roundtrip_group(v);
+            const float v[8] = {a.x, a.y, b.x, b.y, d.x, d.y, f.x, f.y};
 #pragma unroll
             for (int n = 0; n < 8; ++n) acc[n] += wk * v[n];
         }
@@ -596,6 +628,49 @@ ll_local_combine_kernel(LowLatLayout lay, const __nv_bfloat16* x, const void* to
     uint4 o;
     o.x = pack_bf16x2(acc[0], acc[1]); o.y = pack_bf16x2(acc[2], acc[3]); o.z = pack_bf16x2(acc[4], acc[5]); o.w = pack_bf16x2(acc[6], acc[7]);
     *reinterpret_cast<uint4*>(out + (size_t)t * H + col) = o;
+}
+
+// The same with rows in LogFMT: their groups go through the same encoder and decoder as on the wire, a logarithm and an exponential per value,
+// which is what bounds it.  Eight warps take a row each of 256 channels (with ROWS below eight of several 256 channels), and then all add up the rows in
+// the order of k.  (A warp for all rows of its channels, one after the other, left a scheduler with four warps and one chain each.)
+template <int ROWS>
+__global__ void __launch_bounds__(256)
+ll_local_combine_logfmt_kernel(LowLatLayout lay, const __nv_bfloat16* x, const void* topk_idx, int is64, const float* topk_w, const int* entry_row, int T,
+                               int K, int entry_t, int entry_k, __nv_bfloat16* out) {
+    constexpr int kChunks = 8 / ROWS;
+    __shared__ float4 value[8][64];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int t = blockIdx.x, c0 = blockIdx.y * kChunks, H = lay.hidden, chunks = min(kChunks, H / 256 - c0);
+    int row;
+    float w;
+    combine_entry(lay, topk_idx, is64, topk_w, entry_row, t, K, entry_t, entry_k, lane, row, w);
+    float acc[kChunks] = {};
+    for (int k0 = 0; k0 < K; k0 += ROWS) {
+        const int k = k0 + warp % ROWS, c = warp / ROWS;
+        const int r = __shfl_sync(0xffffffffu, row, k & 31);
+        if (k < K && r >= 0 && c < chunks) {
+            const uint4 raw = *reinterpret_cast<const uint4*>(x + (size_t)r * H + (size_t)(c0 + c) * 256 + lane * 8);
+            const float2 a = unpack_bf16x2(raw.x), b = unpack_bf16x2(raw.y), d = unpack_bf16x2(raw.z), f = unpack_bf16x2(raw.w);
+            float v[8] = {a.x, a.y, b.x, b.y, d.x, d.y, f.x, f.y};
+            logfmt_roundtrip_group(v);
+            value[warp][2 * lane] = make_float4(v[0], v[1], v[2], v[3]);
+            value[warp][2 * lane + 1] = make_float4(v[4], v[5], v[6], v[7]);
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < ROWS; ++i) {
+            const int ri = __shfl_sync(0xffffffffu, row, (k0 + i) & 31);
+            const float wk = __shfl_sync(0xffffffffu, w, (k0 + i) & 31);
+            if (k0 + i >= K || ri < 0) continue;
+#pragma unroll
+            for (int j = 0; j < kChunks; ++j)
+                if (j < chunks) acc[j] += wk * reinterpret_cast<const float*>(value[j * ROWS + i])[threadIdx.x];
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int j = 0; j < kChunks; ++j)
+        if (j < chunks) out[(size_t)t * H + (size_t)(c0 + j) * 256 + threadIdx.x] = __float2bfloat16_rn(acc[j]);
 }
 
 __global__ void ll_mask_update_kernel(int* mask, int num_ranks, int rank, int value) {
@@ -674,10 +749,18 @@ cudaError_t ll_local_combine(const LowLatLayout& lay, const void* x, const void*
                              const int* entry_row, int T, int K, int entry_t, int entry_k, void* out, cudaStream_t stream) {
     if (!layout_ok(lay) || lay.num_ranks != 1 || T > lay.max_tokens || K > kMaxTopK || entry_k > kMaxTopK) return cudaErrorInvalidValue;
     if (T == 0) return cudaSuccess;
-    const dim3 grid(T, (lay.hidden / 256 + 3) / 4);
-    auto kern = lay.use_logfmt ? ll_local_combine_kernel<true> : ll_local_combine_kernel<false>;
-    kern<<<grid, 128, 0, stream>>>(lay, static_cast<const __nv_bfloat16*>(x), topk_idx, idx_is64, topk_weights, entry_row, T, K, entry_t, entry_k,
-                                   static_cast<__nv_bfloat16*>(out));
+    const int chunks = lay.hidden / 256;
+    if (lay.use_logfmt) {
+        const int rows = K > 4 ? 8 : K > 2 ? 4 : K;
+        auto kern = rows == 8 ? ll_local_combine_logfmt_kernel<8> : rows == 4 ? ll_local_combine_logfmt_kernel<4> : rows == 2 ? ll_local_combine_logfmt_kernel<2>
+                                                                                                                   : ll_local_combine_logfmt_kernel<1>;
+        const int per_block = rows == 0 ? 8 : 8 / rows;
+        kern<<<dim3(T, (chunks + per_block - 1) / per_block), 256, 0, stream>>>(lay, static_cast<const __nv_bfloat16*>(x), topk_idx, idx_is64, topk_weights,
+                                                                               entry_row, T, K, entry_t, entry_k, static_cast<__nv_bfloat16*>(out));
+        return cudaGetLastError();
+    }
+    ll_local_combine_kernel<<<dim3(T, (chunks + 3) / 4), 128, 0, stream>>>(lay, static_cast<const __nv_bfloat16*>(x), topk_idx, idx_is64, topk_weights, entry_row, T,
+                                                                          K, entry_t, entry_k, static_cast<__nv_bfloat16*>(out));
     return cudaGetLastError();
 }
 
