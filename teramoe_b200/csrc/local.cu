@@ -1,18 +1,21 @@
 // Un-fused dispatch / combine on one rank, see local.h.
 //
-//   local_route     counts per expert and the row of every token: up to 1024 tokens one block, which needs no cleared counters; above, a
-//                   memset and one block per 128 tokens, of which the last to finish scans the chunks
+//   local_route     counts per expert and the row of every token: up to 1024 tokens one block, up to 128 K entries a cluster of eight that add up
+//                   each other's counts, neither of which needs cleared counters; above, a memset and one block per 128 tokens, of which the
+//                   last to finish scans the chunks
 //   local_dispatch  rows, expert ids and weights of the tokens that go anywhere, in token order
 //   local_move      the repeat of a dispatch with a known layout, and the combine
 //
 // All are bound by memory traffic: every row is read once and written once.  A warp moves 2 KB of a row (four 16-byte loads in
 // flight per lane), so that a few hundred rows already fill the SMs.  Through the symmetric arena the same dispatch took a
 // push into the arena, a copy out of it, nine table copies and two waits of the host.  Measured through the API, hidden 7168,
-// top-8, 32 experts: layout + dispatch + combine + cached dispatch + combine with weights at 4096 tokens 1216 -> 99 us (77 launches
+// top-8, 32 experts: layout + dispatch + combine + cached dispatch + combine with weights at 4096 tokens 1216 -> 96 us (77 launches
 // before), layout + FP8 dispatch + combine at 1003 tokens 736 -> 47 us.
 // The latter is host work: five allocations and four launches, and the wait for the counts, for which the host watches the pinned
 // words that the route kernel writes (an event behind it was seen a few microseconds later).
 #include "local.h"
+
+#include <cooperative_groups.h>
 
 #include "ptx.cuh"
 
@@ -22,6 +25,8 @@ namespace {
 
 constexpr uint32_t kSegBytes = 2048;
 constexpr int kLocalOneBlock = 1024;     // most tokens that one block routes
+constexpr int kLocalCluster = 8;         // blocks that route more,
+constexpr long kLocalClusterEntries = 128 * 1024;   // and most entries that they do
 static_assert(kLocalOneBlock == 1024, "a warp adds up the counts of 32 warps");
 
 struct Parts {
@@ -41,9 +46,86 @@ __device__ __forceinline__ void publish(volatile unsigned long long* word, int s
     *word = ((unsigned long long)(uint32_t)seq << 32) | (uint32_t)count;
 }
 
-__global__ void __launch_bounds__(kLocalChunk)
+// counts a token's valid entries; true if there are any.  (Eight indices are on their way at a time.)
+__device__ __forceinline__ bool count_token(const void* topk_idx, int is64, long t, int K, int E, int* hist) {
+    bool any = false;
+    for (int k0 = 0; k0 < K; k0 += 8) {
+        long long e[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) e[j] = k0 + j < K ? load_entry(topk_idx, is64, t * K + k0 + j) : -1;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            if (e[j] < 0 || e[j] >= E) continue;
+            atomicAdd(&hist[(int)e[j]], 1);
+            any = true;
+        }
+    }
+    return any;
+}
+
+// Every block of the cluster takes a run of chunks, eight at a time, and keeps its counts; then each reads what the others have.  With more
+// entries (local_route_many_kernel) counters in memory are cleared by a memset and added to by a block per chunk: two more steps of the stream, each
+// of which takes 2 us and more however little is done in it.  us of layout + dispatch through the API, so / here: 2000 tokens, top-8, 32 experts 50.5 / 41.0,
+// 4096 49.8 / 41.5, 16384, 256 experts 52.3 / 50.1 (the kernel 8.5 / 11.6, an atomic per entry in few SMs); 100000, 32 experts 73 / 126.
+__global__ void __cluster_dims__(kLocalCluster, 1, 1) __launch_bounds__(kLocalOneBlock)
 local_route_kernel(const void* topk_idx, int is64, int T, int K, int E, int* totals, int* row_local, int* chunk_base, uint8_t* in_rank,
                    unsigned long long* host_out, int host_seq) {
+    extern __shared__ int hist[];
+    __shared__ int warp_rows[kLocalOneBlock / 32];
+    __shared__ int rows_here;
+    constexpr int kChunkWarps = kLocalChunk / 32, kAtATime = kLocalOneBlock / kLocalChunk;
+    const auto cluster = cooperative_groups::this_cluster();
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, first = warp / kChunkWarps * kChunkWarps, rank = (int)cluster.block_rank();
+    const int chunks = (T + kLocalChunk - 1) / kLocalChunk, share = (chunks + kLocalCluster - 1) / kLocalCluster;
+    const int begin = min(rank * share, chunks), end = min(begin + share, chunks);
+    for (int e = tid; e < E; e += kLocalOneBlock) hist[e] = 0;
+    __syncthreads();
+    int run = 0;
+    for (int c0 = begin; c0 < end; c0 += kAtATime) {
+        const int chunk = c0 + warp / kChunkWarps, t = chunk * kLocalChunk + (tid & (kLocalChunk - 1));
+        const bool live = chunk < end && t < T;
+        const bool any = live && count_token(topk_idx, is64, t, K, E, hist);
+        if (live && in_rank != nullptr) in_rank[t] = any ? 1 : 0;
+        const uint32_t b = __ballot_sync(0xffffffffu, any);
+        if (lane == 0) warp_rows[warp] = __popc(b);
+        __syncthreads();
+        const int own = warp_rows[lane];
+        const int earlier = __reduce_add_sync(0xffffffffu, lane < first ? own : 0);
+        const int before = __reduce_add_sync(0xffffffffu, lane >= first && lane < warp ? own : 0);
+        const int rows = __reduce_add_sync(0xffffffffu, own);
+        if (live) row_local[t] = any ? before + __popc(b & ((1u << lane) - 1u)) : -1;
+        if (chunk < end && warp == first && lane == 0) chunk_base[chunk] = run + earlier;
+        run += rows;
+        __syncthreads();
+    }
+    if (tid == 0) rows_here = run;
+    cluster.sync();
+    int base = 0, all = 0;
+#pragma unroll
+    for (int j = 0; j < kLocalCluster; ++j) {
+        const int n = *cluster.map_shared_rank(&rows_here, j);
+        if (j < rank) base += n;
+        all += n;
+    }
+    if (base != 0)
+        for (int c = begin + tid; c < end; c += kLocalOneBlock) chunk_base[c] += base;
+    for (int e = rank * kLocalOneBlock + tid; e < E; e += kLocalCluster * kLocalOneBlock) {
+        int n = 0;
+#pragma unroll
+        for (int j = 0; j < kLocalCluster; ++j) n += cluster.map_shared_rank(hist, j)[e];
+        totals[e] = n;
+        if (host_out != nullptr) publish(host_out + 1 + e, host_seq, n);
+    }
+    if (rank == 0 && tid == 0) {
+        totals[E] = all;
+        if (host_out != nullptr) publish(host_out, host_seq, all);
+    }
+    cluster.sync();                          // (no block may end while another reads its counts)
+}
+
+__global__ void __launch_bounds__(kLocalChunk)
+local_route_many_kernel(const void* topk_idx, int is64, int T, int K, int E, int* totals, int* row_local, int* chunk_base, uint8_t* in_rank,
+                        unsigned long long* host_out, int host_seq) {
     extern __shared__ int hist[];
     __shared__ int warp_rows[kLocalChunk / 32];
     __shared__ int last;
@@ -51,17 +133,8 @@ local_route_kernel(const void* topk_idx, int is64, int T, int K, int E, int* tot
     for (int e = tid; e < E; e += kLocalChunk) hist[e] = 0;
     __syncthreads();
     const int t = blockIdx.x * kLocalChunk + tid;
-    bool any = false;
-    if (t < T) {
-        for (int k = 0; k < K; ++k) {
-            const long long e = load_entry(topk_idx, is64, (long)t * K + k);
-            if (e >= 0 && e < E) {
-                atomicAdd(&hist[(int)e], 1);
-                any = true;
-            }
-        }
-        if (in_rank != nullptr) in_rank[t] = any ? 1 : 0;
-    }
+    const bool any = t < T && count_token(topk_idx, is64, t, K, E, hist);
+    if (t < T && in_rank != nullptr) in_rank[t] = any ? 1 : 0;
     const uint32_t b = __ballot_sync(0xffffffffu, any);
     if (lane == 0) warp_rows[warp] = __popc(b);
     __syncthreads();
@@ -113,17 +186,8 @@ local_route_small_kernel(const void* topk_idx, int is64, int T, int K, int E, in
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5, first = warp / kChunkWarps * kChunkWarps;
     for (int e = t; e < E; e += kLocalOneBlock) hist[e] = 0;
     __syncthreads();
-    bool any = false;
-    if (t < T) {
-        for (int k = 0; k < K; ++k) {
-            const long long e = load_entry(topk_idx, is64, (long)t * K + k);
-            if (e >= 0 && e < E) {
-                atomicAdd(&hist[(int)e], 1);
-                any = true;
-            }
-        }
-        if (in_rank != nullptr) in_rank[t] = any ? 1 : 0;
-    }
+    const bool any = t < T && count_token(topk_idx, is64, t, K, E, hist);
+    if (t < T && in_rank != nullptr) in_rank[t] = any ? 1 : 0;
     const uint32_t b = __ballot_sync(0xffffffffu, any);
     if (lane == 0) warp_rows[warp] = __popc(b);
     __syncthreads();
@@ -267,10 +331,14 @@ cudaError_t local_route(const void* topk_idx, int is64, int T, int K, int E, int
         local_route_small_kernel<<<1, kLocalOneBlock, smem, stream>>>(topk_idx, is64, T, K, E, totals, row_local, chunk_base, in_rank, host_out, host_seq);
         return cudaGetLastError();
     }
+    if ((long)T * K <= kLocalClusterEntries) {
+        local_route_kernel<<<kLocalCluster, kLocalOneBlock, smem, stream>>>(topk_idx, is64, T, K, E, totals, row_local, chunk_base, in_rank, host_out, host_seq);
+        return cudaGetLastError();
+    }
     cudaError_t e = cudaMemsetAsync(totals, 0, (size_t)(E + 2) * sizeof(int), stream);
     if (e != cudaSuccess) return e;
     const int chunks = (T + kLocalChunk - 1) / kLocalChunk;
-    local_route_kernel<<<chunks, kLocalChunk, smem, stream>>>(topk_idx, is64, T, K, E, totals, row_local, chunk_base, in_rank, host_out, host_seq);
+    local_route_many_kernel<<<chunks, kLocalChunk, smem, stream>>>(topk_idx, is64, T, K, E, totals, row_local, chunk_base, in_rank, host_out, host_seq);
     return cudaGetLastError();
 }
 

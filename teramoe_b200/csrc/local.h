@@ -6,7 +6,7 @@
 
 namespace tmoe {
 
-constexpr int kLocalChunk = 128;         // tokens per block of local_route
+constexpr int kLocalChunk = 128;         // tokens that local_route numbers the rows of together
 constexpr int kLocalMaxParts = 2;        // payloads that travel together (FP8 rows and their scales)
 
 struct LocalPart {

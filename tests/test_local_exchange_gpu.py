@@ -105,6 +105,25 @@ def test_unfused_exchange_matches_plain_indexing(T, H, E, K, fp8):
     buf.destroy()
 
 
+# one block | a cluster of eight, of which the last have nothing, a chunk each, several at a time and a short last one, all that they take | one block per chunk
+@pytest.mark.parametrize("T,E,K", [(1024, 5, 2), (1025, 5, 2), (1153, 300, 8), (9001, 2500, 2), (16384, 33, 8), (16385, 33, 8)])
+def test_layout_of_many_tokens(T, E, K):
+    """Counts, ranks and the rows' order, on the device and as the host reads them; tokens without an expert in every chunk, and a chunk of them."""
+    idx, w = _routing(T, E, K, seed=T, dtype=torch.int32 if T % 2 else torch.int64)
+    idx[130:300] = -1
+    valid = idx >= 0
+    goes = valid.any(1)
+    buf = tm.Buffer(None, 0, explicitly_destroy=True)
+    x = torch.arange(T, device="cuda").view(T, 1).expand(T, 4).to(torch.int16).contiguous().view(torch.bfloat16)
+    for _ in range(2):
+        per_rank, _, per_expert, in_rank, _ = buf.get_dispatch_layout(idx, E)
+        want = torch.bincount(idx[valid].long(), minlength=E)
+        assert per_rank.tolist() == [int(goes.sum())] and torch.equal(per_expert.long(), want) and torch.equal(in_rank[:, 0], goes)
+        recv, recv_idx, _, counts, _, _ = buf.deepep_dispatch(x, topk_idx=idx, topk_weights=w, num_tokens_per_expert=per_expert)
+        assert counts == want.tolist() and torch.equal(recv.view(torch.int16), x[goes].view(torch.int16)) and torch.equal(recv_idx, idx[goes])
+    buf.destroy()
+
+
 def _stall(stream, ms=40):
     with torch.cuda.stream(stream):
         torch.cuda._sleep(int(ms * 1.5e6))             # cycles
