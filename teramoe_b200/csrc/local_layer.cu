@@ -137,7 +137,7 @@ struct LayerArgsP {
     alignas(64) CUtensorMap st_dwd;
     alignas(64) CUtensorMap st_dwg;
     int T, K, H, I, E;
-    int stages, stage_bytes, keep;
+    int stages, stage_bytes, keep, clean;
     const uint8_t* x;                    // [T, H]: forward x, backward grad_out
     const __nv_bfloat16* y;
     __nv_bfloat16* saved_x;              // [T, H]: written by forward (may be null), read by backward
@@ -236,6 +236,26 @@ __device__ __forceinline__ void decode_item(const LayerArgsP& L, const int4& it,
         q.tail = it.w - (q.nk - 1) * (BK / UK);
     }
 }
+
+// Rows of A that do not exist are multiplied all the same, into rows of the accumulator that nobody reads, and what earlier items left there draws as much
+// power as what counts.  So an item whose rows are fewer than those that may be left has zeros put behind them, in its first steps: as many as there are
+// stages, which then stay clean.  Up to 32 rows are left as they are, so that experts of about the same size do not clean all the time.  The producers
+// and the loading warps follow, each for itself, how many rows of a CTA's stages may hold something.
+// Only where experts have more than 224 rows on average (LayerArgsP::clean): up to there nearly all have one unit, whose second half, if it is there at
+// all, mostly takes all rows.  us, without / with, by rows per expert, forward (H=7168 I=2048, 32 experts, top-8): 100 660 / 667, 140 697 / 700, 180 743 /
+// 743, 275 1251 / 1200, 525 1669 / 1614, 750 1919 / 1909; steps: 64 1960 / 1968, 140 2278 / 2237, 180 2341 / 2386, 275 3556 / 3458, H=4096 I=1536, 525
+// 2192 / 2156, of 2048 rows and more 0 to 0.9 %.
+struct Leftover {
+    bool on;
+    int rows;                                // multiple of 32
+    // takes an item that loads `loaded` rows (0 .. 128, a multiple of 32) in nk steps; up to which row its first steps have to write
+    __device__ __forceinline__ int clean(int loaded, int nk, int stages) {
+        const bool need = on && rows > loaded + 32;
+        const int to = need ? rows : loaded;
+        rows = need && nk >= stages ? loaded : max(rows, loaded);
+        return to;
+    }
+};
 
 // Store staging of one epilogue warp: a box of 32 rows x 128 bytes, swizzled as the tensor maps expect.  One box per warp, because the
 // 32 KB that a second one would take are worth more as a sixth operand stage; the wait until the store has read the box
@@ -729,6 +749,8 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
             return true;
         };
 
+        // rows of A that TMA loads for an item of which `need` are wanted, in boxes of 32 or of all
+        auto rows_loaded = [](int need) { return need > 64 ? BM : (need + 31) & ~31; };
         // -------------------------------------------------------------- token rows
         // Operands that are made of token rows come straight from the caller's [T, H] tensor, row by row of the slot table: A of the first GEMM
         // (128 rows x 64 columns of K per step), A of dW_down and B of dW_gateup (64 rows of K x 128 or more columns).  Four warps of each CTA
@@ -754,6 +776,7 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
             int step = warp - 12, stage = step, ss = 0;      // this warp's next step, counted from the start of the item; its stage
             uint32_t phase = 0, sph = 0;
             int under_way = -1;                              // stage of the step before, if its copies are not yet seen through
+            Leftover left{L.clean != 0, BM};
             // The arrive is all that orders the rows before the products that the first CTA issues: no byte count covers them.
             auto hand_over = [&](int s) {
                 fence_proxy_async_smem();
@@ -776,7 +799,10 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                 decode_item(L, it, rank, q);
                 int row[4] = {-1, -1, -1, -1};               // first GEMM: tokens of rows lane + 32 i; gradients: entries of K rows lane + 32 i of this step
                 const bool down = q.kind == kWorkWgradDown;
+                int all_rows = 0;                            // first GEMM: steps whose 128 rows are all written
                 if (q.kind == kWorkGemm1) {
+                    all_rows = q.real > 32 ? q.nk : left.clean(32, q.nk, L.stages) > 32 ? L.stages : 0;
+                    if (q.real > 32) left.rows = q.nk >= L.stages ? (q.real + 31) & ~31 : BM;
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
                         const int r = lane + 32 * i;
@@ -785,7 +811,10 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                         // a table that says less than the list: a row that never arrives
                         if (row[i] < 0) report_status(L.status, kStatusFlagTimeout, 600, q.m0 + r);
                     }
-                } else if (BWD && q.kind != kWorkGemm2) {
+                } else if (q.kind == kWorkGemm2) {
+                    left.clean(rows_loaded(q.need), q.nk, L.stages);
+                } else if (BWD) {
+                    left.rows = BM;
 #pragma unroll
                     for (int i = 0; i < 2; ++i) row[i] = step < q.nk ? L.slot_tk[q.k0 + step * BK + lane + 32 * i] : -1;
                 }
@@ -805,7 +834,7 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                                 cp_async_16_or_zeros(dst + j * 512 + at[j & 1], src + max(t, 0) * pitch, t >= 0);
                             }
                         };
-                        if (q.real > 32) copy(std::integral_constant<int, 32>());
+                        if (step < all_rows) copy(std::integral_constant<int, 32>());
                         else copy(std::integral_constant<int, 8>());
                     } else if (BWD && q.kind != kWorkGemm2) {
                         const uint8_t* src = (down ? L.x : reinterpret_cast<const uint8_t*>(L.saved_x)) + 16 * chunk;
@@ -872,7 +901,7 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
             if (elect_one()) {
                 const int stages = L.stages;
                 const uint32_t stage_bytes = (uint32_t)L.stage_bytes, pair_full = mapa_shared(full_bar(0), 0);
-                auto rows_loaded = [](int need) { return need > 64 ? BM : (need + 31) & ~31; };
+                Leftover left[2] = {{L.clean != 0, BM}, {L.clean != 0, BM}};         // of both CTAs: the first one's producer counts the bytes of both
                 int stage = 0;
                 uint32_t phase = 0;
                 bool ok = true;
@@ -957,13 +986,32 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                     const Phase& P = L.ph[q.kind];
                     const bool gemm = q.kind <= kWorkGemm2;
                     const int n0 = q.n0 + (int)rank * (BN / 2);
-                    // The two GEMMs, rows of A that a CTA loads: none that nothing is summed from, up to 64 in boxes of 32.  What a stage holds in
-                    // the others is multiplied into accumulator rows that no epilogue reads.  What is made of token rows may come from
+                    // The two GEMMs, rows of A that a CTA loads: none that nothing is summed from, up to 64 in boxes of 32; behind them zeros in the
+                    // first steps, where something else may be left.  What is made of token rows may come from
                     // the loading warps: A of the first GEMM and of dW_down, B of dW_gateup.
-                    const int a_rows = rows_loaded(q.need);
+                    const int a_rows = rows_loaded(q.need), needs[2] = {(cur.z >> 16) & 0xff, (cur.z >> 24) & 0xff};
                     const bool rows_a = ROWS && (q.kind == kWorkGemm1 || q.kind == kWorkWgradDown), rows_b = ROWS && q.kind == kWorkWgradGateup;
-                    const int a_pair = rows_a ? 0 : (gemm ? rows_loaded((cur.z >> 16) & 0xff) + rows_loaded((cur.z >> 24) & 0xff) : 2 * BM);
-                    const uint32_t tx = (uint32_t)(a_pair * (BK * 2) + (rows_b ? 0 : 2 * q.halves * kBHalfBytesP));
+                    const int a_pair = rows_a ? 0 : (gemm ? rows_loaded(needs[0]) + rows_loaded(needs[1]) : 2 * BM);
+                    uint32_t tx = (uint32_t)(a_pair * (BK * 2) + (rows_b ? 0 : 2 * q.halves * kBHalfBytesP));
+                    int zeros_to = 0;                                          // up to which row the first steps write zeros, in this CTA,
+                    uint32_t tx_zeros = 0;                                     // and their bytes in both
+                    if (L.clean) {
+#pragma unroll
+                        for (int r = 0; r < 2; ++r) {
+                            if (!gemm) {
+                                left[r].rows = BM;
+                            } else if (rows_a) {                               // (as the loading warps do it)
+                                const int real = needs[r] - (r == ((cur.x >> 4) & 1) ? (cur.x >> 24) & 63 : 0);
+                                if (real > 32) left[r].rows = q.nk >= stages ? (real + 31) & ~31 : BM;
+                                else left[r].clean(32, q.nk, stages);
+                            } else {
+                                const int loaded = rows_loaded(needs[r]), to = left[r].clean(loaded, q.nk, stages);
+                                tx_zeros += (uint32_t)((to - loaded) * (BK * 2));
+                                if (r == (int)rank) zeros_to = to;
+                            }
+                        }
+                    }
+                    tx += tx_zeros;                                            // (taken off again behind those steps)
                     const int look_kb = min(stages - 1, q.nk - 1);     // all stages are in flight: a pause of this thread costs nothing
                     auto take_stage = [&](int st, uint32_t ph) {
                         if (!mbar_wait(empty_bar(st), ph ^ 1u, abort_flag, L.status, 610)) return false;
@@ -1002,8 +1050,9 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                     // stores of other SMs -> async-proxy reads; the weight gradients acquire once, so they need the fence once
                     if (gemm || !wgrad_fenced) fence_proxy_async_all();
                     if (!gemm) wgrad_fenced = true;
-                    auto load_steps = [&](auto&& load_a) {
-                        for (int kb = 0; kb < q.nk; ++kb) {
+                    int kb = 0;
+                    auto load_steps = [&](int end, auto&& load_a) {
+                        for (; kb < end; ++kb) {
                             if (kb >= early && !take_stage(stage, phase)) return false;
                             load_a(smem_base + (uint32_t)stage * stage_bytes, pair_full + 8u * stage, kb * BK);
                             if (kb >= early) load_b(stage, q.k0 + kb * BK);
@@ -1014,16 +1063,25 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                         return true;
                     };
                     if (rows_a) {
-                        ok = load_steps([](uint32_t, uint32_t, int) {});
+                        ok = load_steps(q.nk, [](uint32_t, uint32_t, int) {});
                     } else if (gemm) {
                         const CUtensorMap* map_a = a_rows == BM ? &P.map_a : &P.map_a32;
-                        ok = load_steps([&](uint32_t dst, uint32_t bar, int k) {
+                        auto load_a = [&](uint32_t dst, uint32_t bar, int k) {
                             if (a_rows != 0) tma_load_2d_2cta(dst, map_a, bar, k, q.m0);
                             if (a_rows == 64) tma_load_2d_2cta(dst + 32 * BK * 2, map_a, bar, k, q.m0 + 32);
-                        });
+                        };
+                        if (tx_zeros != 0) {
+                            // (rows past the last one of the map are zeros)
+                            ok = load_steps(min(stages, q.nk), [&](uint32_t dst, uint32_t bar, int k) {
+                                load_a(dst, bar, k);
+                                for (int r = a_rows; r < zeros_to; r += 32) tma_load_2d_2cta(dst + r * BK * 2, &P.map_a32, bar, k, P.m_total);
+                            });
+                            tx -= tx_zeros;
+                        }
+                        ok = ok && load_steps(q.nk, load_a);
                     } else if constexpr (BWD) {
                         const CUtensorMap* map_a = &P.map_a;
-                        ok = load_steps([&](uint32_t dst, uint32_t bar, int k) { tma_load_3d_2cta(dst, map_a, bar, 0, q.k0 + k, q.m0 >> 6); });
+                        ok = load_steps(q.nk, [&](uint32_t dst, uint32_t bar, int k) { tma_load_3d_2cta(dst, map_a, bar, 0, q.k0 + k, q.m0 >> 6); });
                     }
                 }
                 if (!ok) {
@@ -1541,6 +1599,7 @@ cudaError_t local_layer_launch(const LocalLayerParams& q, cudaStream_t stream) {
         if ((e = make_store_map3(&L.st_dwg, q.dw_gateup, E, 2 * I, H)) != cudaSuccess) return e;
     }
     g1.num_n_blocks = column_blocks(g1.n_total, g1.cols);
+    g1.m_total = g2.m_total = q.out_rows;
     L.T = p.T; L.K = p.K; L.H = H; L.I = I; L.E = E; L.keep = p.keep;
     L.x = static_cast<const uint8_t*>(q.x);
     L.y = static_cast<const __nv_bfloat16*>(q.y);
@@ -1571,6 +1630,7 @@ cudaError_t local_layer_launch(const LocalLayerParams& q, cudaStream_t stream) {
     bool wide = false;
     for (int k = 0; k < (q.bwd ? 4 : 2); ++k) wide |= L.ph[k].cols > BN;
     L.stages = wide ? 4 : 6;
+    L.clean = (long)p.T * p.K > 224l * E;
     L.stage_bytes = wide ? kWideStageBytes : kNarrowStageBytes;
     if (q.bwd) return copies ? launch<true, false>(L, sms, stream) : launch<true, true>(L, sms, stream);
     return copies ? launch<false, false>(L, sms, stream) : launch<false, true>(L, sms, stream);
