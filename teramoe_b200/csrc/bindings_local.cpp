@@ -382,6 +382,11 @@ py::dict local_layer_variant(int64_t T, int64_t K, int64_t E, int64_t H, int64_t
     return d;
 }
 
+// whether units of one 128-row block are multiplied as 128 rows
+bool local_layer_halves(int64_t T, int64_t K, int64_t E, int64_t H, int64_t I) {
+    return tmoe::local_layer_plan((int)T, (int)K, (int)E, (int)H, (int)I, 0).halves != 0;
+}
+
 void check_layer_weights(const torch::Tensor& wg, const torch::Tensor& wd, int64_t E, int64_t H, int64_t I) {
     TORCH_CHECK(wg.is_cuda() && wg.scalar_type() == torch::kBFloat16 && wg.is_contiguous() && wg.dim() == 3 && wg.size(0) == E &&
                 wg.size(1) == 2 * I && wg.size(2) == H, "W_gateup must be a contiguous bf16 [E, 2I, H] CUDA tensor");
@@ -702,6 +707,7 @@ void register_local(pybind11::module_& m) {
         .def("ran_few", &LocalLayer::ran_few, py::call_guard<py::gil_scoped_release>())
         .def("call", &local_layer_call);
     m.def("local_layer_variant", &local_layer_variant);
+    m.def("local_layer_halves", &local_layer_halves);
     m.def("local_counts", &local_counts);
     m.def("local_scatter", &local_scatter);
     m.def("local_combine", &local_combine);

@@ -137,7 +137,7 @@ struct LayerArgsP {
     alignas(64) CUtensorMap st_dwd;
     alignas(64) CUtensorMap st_dwg;
     int T, K, H, I, E;
-    int stages, stage_bytes, keep, clean;
+    int stages, stage_bytes, keep, clean, halves;
     const uint8_t* x;                    // [T, H]: forward x, backward grad_out
     const __nv_bfloat16* y;
     __nv_bfloat16* saved_x;              // [T, H]: written by forward (may be null), read by backward
@@ -204,9 +204,17 @@ __device__ __forceinline__ void registers_dec() {
 
 struct Item {
     int kind, n0, halves, group, k0, nk, tail, m0, unit, need, real;      // columns n0 .. n0 + 256 * halves; `real` of the `need` rows are not padding; tail: 16-row slices of the last step
-    bool live;          // this CTA's 128 rows are real
+    bool half;          // a unit of one 128-row block, 64 of whose rows each CTA has
+    int wait;           // rows of the block that have to be there
     int m_in_group;     // weight gradients: first row of dW inside the expert
 };
+
+// rows that a CTA of the pair has of an item of the two GEMMs; `real`: without those that are padding (backward, in the last block of an expert)
+__device__ __forceinline__ int unit_rows(const int4& it, uint32_t rank, bool half, bool real) {
+    const int two = (it.x >> 4) & 1, pad = real ? (it.x >> 24) & 63 : 0;
+    if (half) return max(0, min(BM / 2, ((it.z >> 16) & 0xff) - pad - (int)rank * (BM / 2)));
+    return ((it.z >> (rank == 0 ? 16 : 24)) & 0xff) - ((int)rank == two ? pad : 0);
+}
 
 __device__ __forceinline__ void decode_item(const LayerArgsP& L, const int4& it, uint32_t rank, Item& q) {
     q.kind = it.x & 15;
@@ -214,21 +222,21 @@ __device__ __forceinline__ void decode_item(const LayerArgsP& L, const int4& it,
     const Phase& P = L.ph[q.kind];
     q.n0 = (it.z & 0xffff) * P.cols;
     q.halves = (P.cols > BN && q.n0 + BN < P.n_total) ? 2 : 1;
+    q.half = false;
     if (q.kind <= kWorkGemm2) {
         q.unit = it.y;
-        q.need = rank == 0 ? ((it.z >> 16) & 0xff) : ((it.z >> 24) & 0xff);
-        const int two = (it.x >> 4) & 1;
-        q.live = rank == 0 || two;
-        q.real = q.need - ((int)rank == two ? (it.x >> 24) & 63 : 0);
-        q.m0 = (it.w + (int)rank) * BM;
+        q.half = L.halves != 0 && ((it.x >> 4) & 1) == 0;
+        q.wait = (it.z >> (rank == 0 || q.half ? 16 : 24)) & 0xff;
+        q.need = unit_rows(it, rank, q.half, false);
+        q.real = unit_rows(it, rank, q.half, true);
+        q.m0 = it.w * BM + (int)rank * (q.half ? BM / 2 : BM);
         q.k0 = 0;
         q.nk = P.nk;
         q.tail = BK / UK;
         q.m_in_group = 0;
     } else {
         q.unit = -1;
-        q.need = q.real = 0;
-        q.live = true;
+        q.need = q.real = q.wait = 0;
         q.m_in_group = ((it.z >> 16) * 2 + (int)rank) * BM;
         q.m0 = q.m_in_group;
         q.k0 = it.y;
@@ -248,12 +256,24 @@ __device__ __forceinline__ void decode_item(const LayerArgsP& L, const int4& it,
 struct Leftover {
     bool on;
     int rows;                                // multiple of 32
-    // takes an item that loads `loaded` rows (0 .. 128, a multiple of 32) in nk steps; up to which row its first steps have to write
-    __device__ __forceinline__ int clean(int loaded, int nk, int stages) {
-        const bool need = on && rows > loaded + 32;
-        const int to = need ? rows : loaded;
-        rows = need && nk >= stages ? loaded : max(rows, loaded);
+    // An item whose A is loaded in boxes, `loaded` rows (0 .. 128, a multiple of 32) in nk steps: up to which row its first steps have to write.  (Of a half
+    // unit 64 rows are multiplied.)
+    __device__ __forceinline__ int take_boxes(bool half, int loaded, int nk, int stages) {
+        const int most = half ? min(rows, BM / 2) : rows;
+        const bool need = on && most > loaded + (half ? 0 : 32);
+        const int to = need ? most : loaded;
+        rows = need && nk >= stages && most == rows ? loaded : max(rows, loaded);
         return to;
+    }
+    // An item whose A the loading warps bring, 32 rows or all, with zeros behind the `real` ones: how many steps have to write all.
+    __device__ __forceinline__ int take_rows(bool half, int real, int nk, int stages) {
+        if (real <= 32) {
+            if (take_boxes(half, 32, nk, stages) == 32) return 0;
+            if (nk >= stages) rows = 32;                     // (all 128 are written)
+            return stages;
+        }
+        rows = nk >= stages ? (real + 31) & ~31 : BM;
+        return nk;
     }
 };
 
@@ -801,8 +821,7 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                 const bool down = q.kind == kWorkWgradDown;
                 int all_rows = 0;                            // first GEMM: steps whose 128 rows are all written
                 if (q.kind == kWorkGemm1) {
-                    all_rows = q.real > 32 ? q.nk : left.clean(32, q.nk, L.stages) > 32 ? L.stages : 0;
-                    if (q.real > 32) left.rows = q.nk >= L.stages ? (q.real + 31) & ~31 : BM;
+                    all_rows = left.take_rows(q.half, q.real, q.nk, L.stages);
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
                         const int r = lane + 32 * i;
@@ -812,7 +831,7 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                         if (row[i] < 0) report_status(L.status, kStatusFlagTimeout, 600, q.m0 + r);
                     }
                 } else if (q.kind == kWorkGemm2) {
-                    left.clean(rows_loaded(q.need), q.nk, L.stages);
+                    left.take_boxes(q.half, rows_loaded(q.need), q.nk, L.stages);
                 } else if (BWD) {
                     left.rows = BM;
 #pragma unroll
@@ -947,7 +966,7 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                 };
                 // what the operands of an item wait for; `block`: wait (bounded) instead of only looking
                 auto operands_ready = [&](const Item& q, bool block) -> int {
-                    if (q.kind == kWorkGemm1) return (ROWS || !q.live || q.need == 0) ? 1 : counted(L.arrived + q.m0 / BM, q.need, block, 600, w_arrive);
+                    if (q.kind == kWorkGemm1) return (ROWS || q.need == 0) ? 1 : counted(L.arrived + q.m0 / BM, q.wait, block, 600, w_arrive);
                     if (q.kind == kWorkGemm2) return counted(L.done1 + q.unit, target1, block, 601, w_unit);
                     // the weight gradients sit behind all first GEMMs in the list: one check per pair is enough (two loads per expert and pair
                     // would cost as much as the smallest of these items)
@@ -989,7 +1008,7 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                     // The two GEMMs, rows of A that a CTA loads: none that nothing is summed from, up to 64 in boxes of 32; behind them zeros in the
                     // first steps, where something else may be left.  What is made of token rows may come from
                     // the loading warps: A of the first GEMM and of dW_down, B of dW_gateup.
-                    const int a_rows = rows_loaded(q.need), needs[2] = {(cur.z >> 16) & 0xff, (cur.z >> 24) & 0xff};
+                    const int a_rows = rows_loaded(q.need), needs[2] = {unit_rows(cur, 0, q.half, false), unit_rows(cur, 1, q.half, false)};
                     const bool rows_a = ROWS && (q.kind == kWorkGemm1 || q.kind == kWorkWgradDown), rows_b = ROWS && q.kind == kWorkWgradGateup;
                     const int a_pair = rows_a ? 0 : (gemm ? rows_loaded(needs[0]) + rows_loaded(needs[1]) : 2 * BM);
                     uint32_t tx = (uint32_t)(a_pair * (BK * 2) + (rows_b ? 0 : 2 * q.halves * kBHalfBytesP));
@@ -1001,11 +1020,9 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                             if (!gemm) {
                                 left[r].rows = BM;
                             } else if (rows_a) {                               // (as the loading warps do it)
-                                const int real = needs[r] - (r == ((cur.x >> 4) & 1) ? (cur.x >> 24) & 63 : 0);
-                                if (real > 32) left[r].rows = q.nk >= stages ? (real + 31) & ~31 : BM;
-                                else left[r].clean(32, q.nk, stages);
+                                left[r].take_rows(q.half, unit_rows(cur, r, q.half, true), q.nk, stages);
                             } else {
-                                const int loaded = rows_loaded(needs[r]), to = left[r].clean(loaded, q.nk, stages);
+                                const int loaded = rows_loaded(needs[r]), to = left[r].take_boxes(q.half, loaded, q.nk, stages);
                                 tx_zeros += (uint32_t)((to - loaded) * (BK * 2));
                                 if (r == (int)rank) zeros_to = to;
                             }
@@ -1108,77 +1125,85 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                 if (!next_item(ss, sph, 652, it) || it.x < 0) break;
                 Item q;
                 decode_item(L, it, rank, q);
-                const bool a_mn = q.kind >= kWorkWgradDown;
-                const uint32_t idesc = BWD ? (a_mn ? make_idesc_bf16(2 * BM, BN, true, true) : make_idesc_bf16(2 * BM, BN, false, true))
-                                           : make_idesc_bf16(2 * BM, BN, false, false);
                 const int slot0 = acc & 1, slot1 = slot0 ^ 1;
                 const uint32_t parity0 = ((acc >> 1) & 1) ^ 1u, parity1 = (((acc + 1) >> 1) & 1) ^ 1u;
                 acc += q.halves;
-                // Operand descriptors of stage 0; a stage or a step of K further on is an addition to their address field.
-                const uint64_t a_base = make_smem_desc_sw128(smem_base, a_mn ? kAtomBytes : 0, 1024);
-                const uint64_t b_base = make_smem_desc_sw128(smem_base + kAStageBytes, BWD ? kAtomBytes : 0, 1024);
-                const uint32_t a_step = (a_mn ? UK * 128 : UK * 2) >> 4, b_step = (BWD ? UK * 128 : UK * 2) >> 4;
-                // 64 columns of K of one half of the tile
-                auto multiply = [&](int s, int h, int slot, int kb) {
-                    const uint32_t off = (uint32_t)(s * L.stage_bytes) >> 4;
-                    const uint64_t a_desc = a_base + off, b_desc = b_base + off + (uint32_t)(h * (kBHalfBytesP >> 4));
-                    const uint32_t d_tmem = tmem_base + (uint32_t)(slot * BN);
-                    const int slices = BWD && kb == q.nk - 1 ? q.tail : BK / UK;
+                // ROWS_M rows of A, A_MN: K runs along its rows.  (An instance of the loop for each: the instruction descriptor is a constant in it.)
+                auto mainloop = [&](auto rows_m, auto a_mn_) -> bool {
+                    constexpr bool a_mn = decltype(a_mn_)::value;
+                    constexpr uint32_t idesc = make_idesc_bf16(decltype(rows_m)::value, BN, a_mn, BWD);
+                    // Operand descriptors of stage 0; a stage or a step of K further on is an addition to their address field.
+                    const uint64_t a_base = make_smem_desc_sw128(smem_base, a_mn ? kAtomBytes : 0, 1024);
+                    const uint64_t b_base = make_smem_desc_sw128(smem_base + kAStageBytes, BWD ? kAtomBytes : 0, 1024);
+                    constexpr uint32_t a_step = (a_mn ? UK * 128 : UK * 2) >> 4, b_step = (BWD ? UK * 128 : UK * 2) >> 4;
+                    // 64 columns of K of one half of the tile
+                    auto multiply = [&](int s, int h, int slot, int kb) {
+                        const uint32_t off = (uint32_t)(s * L.stage_bytes) >> 4;
+                        const uint64_t a_desc = a_base + off, b_desc = b_base + off + (uint32_t)(h * (kBHalfBytesP >> 4));
+                        const uint32_t d_tmem = tmem_base + (uint32_t)(slot * BN);
+                        const int slices = BWD && kb == q.nk - 1 ? q.tail : BK / UK;
 #pragma unroll
-                    for (int k = 0; k < BK / UK; ++k)
-                        if (k < slices) umma_bf16_ss_2cta(d_tmem, a_desc + k * a_step, b_desc + k * b_step, idesc, (kb | k) != 0 ? 1u : 0u);
-                };
-                // (the second CTA's loading warps hand over rows that lie there)
-                auto wait_full = [&](int s, uint32_t ph) {
-                    return ROWS ? mbar_wait_cluster_acquire_smem(full_bar(s), ph, abort_flag, L.status, 621) : mbar_wait(full_bar(s), ph, abort_flag, L.status, 621);
-                };
-                if (!mbar_wait(tempty_bar(slot0), parity0, abort_flag, L.status, 620)) { ok = false; break; }
-                tcgen05_fence_after();
-                int kb = 0;
-                if (q.halves == 2) {
-                    // The second accumulator is still being read out when a wide tile starts: the first half runs ahead over the stages
-                    // that are there, the second half follows and frees them.
-                    const int lead = min(q.nk, L.stages);
-                    int s = stage;
-                    uint32_t ph = phase;
-                    for (int i = 0; i < lead; ++i) {
-                        if (!wait_full(s, ph)) { ok = false; break; }
+                        for (int k = 0; k < BK / UK; ++k)
+                            if (k < slices) umma_bf16_ss_2cta(d_tmem, a_desc + k * a_step, b_desc + k * b_step, idesc, (kb | k) != 0 ? 1u : 0u);
+                    };
+                    // (the second CTA's loading warps hand over rows that lie there)
+                    auto wait_full = [&](int s, uint32_t ph) {
+                        return ROWS ? mbar_wait_cluster_acquire_smem(full_bar(s), ph, abort_flag, L.status, 621) : mbar_wait(full_bar(s), ph, abort_flag, L.status, 621);
+                    };
+                    if (!mbar_wait(tempty_bar(slot0), parity0, abort_flag, L.status, 620)) return false;
+                    tcgen05_fence_after();
+                    int kb = 0;
+                    if (q.halves == 2) {
+                        // The second accumulator is still being read out when a wide tile starts: the first half runs ahead over the stages
+                        // that are there, the second half follows and frees them.
+                        const int lead = min(q.nk, L.stages);
+                        int s = stage;
+                        uint32_t ph = phase;
+                        for (int i = 0; i < lead; ++i) {
+                            if (!wait_full(s, ph)) return false;
+                            tcgen05_fence_after();
+                            if (elect_one()) {
+                                multiply(s, 0, slot0, i);
+                                if (i == q.nk - 1) umma_commit_2cta(tfull_bar(slot0), 3u);
+                            }
+                            __syncwarp();
+                            if (++s == L.stages) { s = 0; ph ^= 1u; }
+                        }
+                        if (!mbar_wait(tempty_bar(slot1), parity1, abort_flag, L.status, 622)) return false;
+                        tcgen05_fence_after();
+                        for (; kb < lead; ++kb) {
+                            if (elect_one()) {
+                                multiply(stage, 1, slot1, kb);
+                                umma_commit_2cta(empty_bar(stage), 3u);
+                                if (kb == q.nk - 1) umma_commit_2cta(tfull_bar(slot1), 3u);
+                            }
+                            __syncwarp();
+                            if (++stage == L.stages) { stage = 0; phase ^= 1u; }
+                        }
+                    }
+                    for (; kb < q.nk; ++kb) {
+                        if (!wait_full(stage, phase)) return false;
                         tcgen05_fence_after();
                         if (elect_one()) {
-                            multiply(s, 0, slot0, i);
-                            if (i == q.nk - 1) umma_commit_2cta(tfull_bar(slot0), 3u);
-                        }
-                        __syncwarp();
-                        if (++s == L.stages) { s = 0; ph ^= 1u; }
-                    }
-                    if (!ok || !mbar_wait(tempty_bar(slot1), parity1, abort_flag, L.status, 622)) { ok = false; break; }
-                    tcgen05_fence_after();
-                    for (; kb < lead; ++kb) {
-                        if (elect_one()) {
-                            multiply(stage, 1, slot1, kb);
+                            const bool last = kb == q.nk - 1;
+                            multiply(stage, 0, slot0, kb);
+                            if (q.halves == 2) {
+                                if (last) umma_commit_2cta(tfull_bar(slot0), 3u);
+                                multiply(stage, 1, slot1, kb);
+                            }
                             umma_commit_2cta(empty_bar(stage), 3u);
-                            if (kb == q.nk - 1) umma_commit_2cta(tfull_bar(slot1), 3u);
+                            if (last) umma_commit_2cta(tfull_bar(q.halves == 2 ? slot1 : slot0), 3u);
                         }
                         __syncwarp();
                         if (++stage == L.stages) { stage = 0; phase ^= 1u; }
                     }
-                }
-                for (; kb < q.nk; ++kb) {
-                    if (!wait_full(stage, phase)) { ok = false; break; }
-                    tcgen05_fence_after();
-                    if (elect_one()) {
-                        const bool last = kb == q.nk - 1;
-                        multiply(stage, 0, slot0, kb);
-                        if (q.halves == 2) {
-                            if (last) umma_commit_2cta(tfull_bar(slot0), 3u);
-                            multiply(stage, 1, slot1, kb);
-                        }
-                        umma_commit_2cta(empty_bar(stage), 3u);
-                        if (last) umma_commit_2cta(tfull_bar(q.halves == 2 ? slot1 : slot0), 3u);
-                    }
-                    __syncwarp();
-                    if (++stage == L.stages) { stage = 0; phase ^= 1u; }
-                }
+                    return true;
+                };
+                using Rows = std::integral_constant<uint32_t, 2 * BM>;
+                using HalfRows = std::integral_constant<uint32_t, BM>;
+                if (BWD && q.kind >= kWorkWgradDown) ok = mainloop(Rows(), std::integral_constant<bool, BWD>());
+                else if (q.half) ok = mainloop(HalfRows(), std::false_type());
+                else ok = mainloop(Rows(), std::false_type());
                 if (ok && q.nk == 0) {                       // an expert without rows: the epilogue stores zeros
                     if (elect_one()) {
                         umma_commit_2cta(tfull_bar(slot0), 3u);
@@ -1243,16 +1268,19 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                 decode_item(L, it, rank, q);
                 if (stamps) atomicMax(L.stats + kStatKindFirst + q.kind, ~globaltimer_ns());
                 if (q.kind > kWorkGemm2) flush();  // (the weight gradients may never wait, and the sums run under them)
-                const int row0 = q.m0 + qd * 32;
+                // The accumulator of a half unit: its 64 rows are twice in tensor memory, lanes 0 to 63 with the first 128 columns of the tile and
+                // lanes 64 to 127 with the others, so that one of the two warps of a quarter has nothing to do.
+                const int row_in = (q.half ? qd & 1 : qd) * 32, col_in = (q.half ? qd >> 1 : hh) * (BN / 2), tmem_col = q.half ? 0 : hh * (BN / 2);
+                const int row0 = q.m0 + row_in;
                 // rows of a block beyond those that are used are neither computed on nor stored
-                const bool live = q.kind > kWorkGemm2 || (q.live && qd * 32 < q.need);
+                const bool live = q.kind > kWorkGemm2 || (row_in < q.need && !(q.half && hh != 0));
                 bool real = false;                 // backward, first GEMM: this lane's row is not padding
-                if constexpr (BWD) real = q.kind == kWorkGemm1 && qd * 32 + lane < q.real;
+                if constexpr (BWD) real = q.kind == kWorkGemm1 && live && row_in + lane < q.real;
                 for (int h = 0; h < q.halves; ++h) {
                     const int slot = acc & 1;
                     const uint32_t parity = (acc >> 1) & 1;
                     ++acc;
-                    const int n0 = q.n0 + h * BN + hh * (BN / 2);
+                    const int n0 = q.n0 + h * BN + col_in;
                     const float w = (q.kind == kWorkGemm1 && live) ? L.slot_w[row0 + lane] : 0.f;       // (padding: 0)
                     Preact pre;
                     if constexpr (BWD) {
@@ -1264,7 +1292,7 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                     if (n_owed != 0 && (n_owed == kOwed || !soon(tfull_bar(slot), parity))) flush();
                     if (!mbar_wait(tfull_bar(slot), parity, abort_flag, L.status, 630)) { ok = false; break; }
                     tcgen05_fence_after();
-                    const uint32_t taddr = tmem_base + ((uint32_t)(qd * 32) << 16) + (uint32_t)(slot * BN + hh * (BN / 2));
+                    const uint32_t taddr = tmem_base + ((uint32_t)(qd * 32) << 16) + (uint32_t)(slot * BN + tmem_col);
                     // this warp has read its part of the accumulator: the issuer may overwrite it
                     auto release = [&]() {
                         tcgen05_fence_before();
@@ -1305,7 +1333,8 @@ local_layer_kernel(const __grid_constant__ LayerArgsP L) {
                 }
                 if (!ok) break;
                 if (stamps) atomicMax(L.stats + kStatKindLast + q.kind, globaltimer_ns());
-                if (q.kind == kWorkGemm1 || (q.kind == kWorkGemm2 && q.live)) {
+                // (of a half unit both CTAs count for the one block)
+                if (q.kind == kWorkGemm1 || (q.kind == kWorkGemm2 && (q.half ? hh == 0 : rank == 0 || ((it.x >> 4) & 1) != 0))) {
                     const uint32_t entry = q.kind == kWorkGemm1 ? (0x80000000u | (uint32_t)q.unit) : (uint32_t)(q.m0 / BM);
 #pragma unroll
                     for (int i = 0; i < kOwed; ++i)
@@ -1443,6 +1472,13 @@ LocalLayerPlan local_layer_plan(int T, int K, int E, int H, int I, int keep) {
     //   H=4096 I=3072                      20 254 / 254     64 279 / 275      256 435 / 434     512 683 / 684
     //   H=4096 I=4096                      20 332 / 333     64 363 / 360      256 571 / 564     512 883 / 884
     //   H=4096 I=14336                     20 583 / 579     128 671 / 655     1024 2614 / 2583
+    // Units of a single 128-row block as products of 128 rows, 64 from each CTA, which take half the time of those of 256 (64 and 128 cycles for 256 columns and
+    // 16 of K, measured), or with zeros for a second block.  us, zeros / half, by rows per expert: forward (H=7168 I=2048, 32 experts, top-8) 90 670 / 589, 125
+    // 736 / 680, 275 1209 / 1129, 325 1187 / 1222, 525 1645 / 1754, 750 1973 / 2026, H=4096 I=1536, 16, top-2 312 307 / 289; steps: 16 1829 / 1715, 64 1972 /
+    // 1834, 275 3466 / 3367, 2048 14940 / 15192, H=4096 I=14336, 8, top-2 375 3762 / 3925, H=2048 I=768, 16, top-4 325 284 / 277, H=2048 I=2048, 16, top-8 2048
+    // 2277 / 2262, H=2048 I=3072, 16, top-6 3072 5169 / 5136.  Where an expert has whole units besides, a half one runs ahead of them through the weights that
+    // they share, and on a long K what it has fetched is gone from L2 before they come: hence only few rows, or short tiles.
+    p.halves = entries <= 300l * E || (H <= 2048 && I <= 3072);
     const bool large_i = I >= 4096;
     p.copies[0] = large_i && p.few != 1;          // (local_few.cu gathers rows from x itself)
     p.copies[1] = keep && (large_i || 2 * rows < I);
@@ -1631,6 +1667,7 @@ cudaError_t local_layer_launch(const LocalLayerParams& q, cudaStream_t stream) {
     for (int k = 0; k < (q.bwd ? 4 : 2); ++k) wide |= L.ph[k].cols > BN;
     L.stages = wide ? 4 : 6;
     L.clean = (long)p.T * p.K > 224l * E;
+    L.halves = p.halves;
     L.stage_bytes = wide ? kWideStageBytes : kNarrowStageBytes;
     if (q.bwd) return copies ? launch<true, false>(L, sms, stream) : launch<true, true>(L, sms, stream);
     return copies ? launch<false, false>(L, sms, stream) : launch<false, true>(L, sms, stream);

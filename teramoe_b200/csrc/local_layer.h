@@ -22,6 +22,7 @@ struct LocalLayerPlan {
     int few_unit;                        // rows of an expert that it multiplies at a time: 64 or 128
     int few_again;                       // with few = 2: most units beyond an expert's first, as a share of the experts with rows: 1 / few_again
     int routes;                          // local_few.cu makes the routing tables itself: there is no routing kernel
+    int halves;                          // units of one 128-row block are multiplied as 128 rows
     int chunks;                          // blocks of the routing kernels
     int slots_cap, blocks_cap, units_cap;
     int work_cap[2];                     // items of the forward / backward list

@@ -101,6 +101,35 @@ def test_rows_per_expert_at_the_edges_of_operand_boxes(H, I, copies, monkeypatch
     buf.destroy()
 
 
+@pytest.mark.parametrize("counts,H,I,halves", [
+    ([257, 300, 320, 321, 383, 384, 385, 641, 0], 192, 128, 1),      # half units behind whole ones: 1, 44, 64, 65, 127 and 128 rows of the last block
+    ([257, 300, 320, 321, 383, 384, 385, 641, 0], 192, 1024, 1),     # (rows by copies in backward)
+    ([257, 300, 320, 321, 383, 384, 385, 641, 0], 2112, 128, 0),     # the same with zeros for a second block
+    ([257, 300, 320, 321, 383, 384, 385, 641, 0], 2112, 1024, 0),
+    ([1, 31, 32, 33, 63, 64, 65, 96, 97, 127, 128, 500], 2112, 4096, 1),
+])
+def test_last_units_of_experts(counts, H, I, halves, monkeypatch):
+    from teramoe_b200 import engine
+    from teramoe_b200._build import load_ext
+    E, T = len(counts), sum(counts)
+    assert load_ext().local_layer_halves(T, 1, E, H, I) == halves
+    prob = make_problem(1, T, H, I, E, 1, seed=3, dtype=torch.bfloat16, device="cuda", x_scale=0.1, w_scale=0.02)
+    order = torch.randperm(T, generator=torch.Generator().manual_seed(1))
+    idx = torch.repeat_interleave(torch.arange(E), torch.tensor(counts))[order].view(T, 1).to(prob["ranks"][0]["idx"])
+    buf = tm.Buffer(None, int(64e6), explicitly_destroy=True)
+    res = {}
+    for mode in ("0", "auto"):
+        monkeypatch.setattr(engine, "_LOCAL_LAYER_MODE", mode)
+        for name in ("_FUSED_DISPATCH_MODE", "_FUSED_MODE", "_LAYER_KERNEL_MODE"):
+            monkeypatch.setattr(engine, name, "1" if mode == "0" else "auto")
+        res[mode] = [_run(buf, prob, idx, E) for _ in range(2)]
+    for runs in zip(*res.values()):
+        for name, got in runs[1].items():
+            assert torch.equal(got, runs[0][name]), f"{name}: differs from the general kernels"
+    buf.check_status()
+    buf.destroy()
+
+
 @pytest.mark.parametrize("batch", [1024, 2048, 4096])
 def test_batches_end_where_experts_do(batch, monkeypatch):
     """Experts of 9, 4, 1, 0, 2, 8, 3, 5 and 1 units of 256 rows in nominal batches of 4, 8 and 16: ends that move to an expert's, that stay inside
