@@ -2,8 +2,8 @@
 // weights once.  The weights are the M operand here, 128 rows of a tile, and an expert's tokens the N operand, 16 to 64 or 128 columns.  With the
 // roles of local_layer.cu eight tokens were multiplied as 256 rows; under the power cap, which such a call reaches too, the tensor
 // cores' share is bandwidth lost.  Forward of 32 tokens, H=7168 I=2048, 32 experts, top-8: 585 -> 430 us, 6.6 TB/s, which is what a plain
-// copy reaches; of 64 tokens 588 -> 437; with I=512 179 -> 132 and 185 -> 134; of 128 and 256 tokens (32 and 64 rows per expert) 620 -> 467 and
-// 654 -> 548: every step brings a unit's rows from L2 next to the weights, half as many bytes again at 64 rows, which is what the time grows by.
+// copy reaches; of 64 tokens 588 -> 437; with I=512 179 -> 132 and 185 -> 134; of 128 and 256 tokens (32 and 64 rows per expert) 507 -> 438 and
+// 534 -> 515: every step brings a unit's rows from L2 next to the weights, half as many bytes again at 64 rows, which is what the time grows by.
 //
 // One persistent block per SM, no clusters.  Items: first the tiles of the first GEMM (128 rows of W_gateup of an expert x a unit of up to
 // 64 or 128 of its tokens), then those of the second, dealt out in turn: they nearly cost the same.  Units of one expert are neighbours, so that

@@ -1434,27 +1434,28 @@ LocalLayerPlan local_layer_plan(int T, int K, int E, int H, int I, int keep) {
     p.units_cap = (int)((p.blocks_cap + segs) / 2);
     const int rows = (int)(entries / (segs > 0 ? segs : 1));
     // Few rows per expert, forward only: weights as the M operand (local_few.cu), 64 rows of an expert at a time, from 41 on average 128.  us, general
-    // kernel / 64 / 128, by rows per expert (even routing):
-    //   H=7168 I=2048, 32 experts, top-8   16 588 / 440 / 455   32 598 / 463 / 475   40 610 / 484 / 491   64 630 / 651 / 539    80 652 / 860 / 567
-    //   (as above)                         96 667 / 856 / 613   112 674 / 852 / 679  128 685 / 944 / 873
-    //   H=2048 I=512, 64, top-4            16 121 / 89 / 91     32 119 / 96 / 99     48 123 / 106 / 107   64 127 / 130 / 119    96 132 / 158 / 136
-    //   H=4096 I=1536, 16, top-2           16 153 / 116 / 120   32 150 / 123 / 129   48 157 / 130 / 135   64 162 / 152 / 143    96 165 / 197 / 161
-    // What an item of the second GEMM stores grows with the rows, what it reads with I: H=4096 I=256, 32 experts, top-2, 37 rows 89 / 85, 62 rows 94 / 102;
-    // hence the line at I / 10 rows, but for calls so small that latencies decide (H=2048 I=256, 8 experts, top-4, 50 rows 42 / 31).  With I >= 4096
-    // it stays at 16 rows: the rows of act that a tile reads are long there (H=1024 I=14336, 4 experts, 48 rows 138 / 131, 64 rows 139 / 149).
+    // kernel / local_few.cu, by rows per expert (even routing; in brackets units of 64 and of 128 rows, measured on another box):
+    //   H=7168 I=2048, 32 experts, top-8   20 489 / 425   32 507 / 438 (463, 475)   48 523 / 484 (496, 506)   64 534 / 515 (651, 539)   80 545 / 543
+    //   H=2048 I=512, 64, top-4            32 103 / 98    48 107 / 108 (106, 107)   51 110 / 113
+    //   H=4096 I=1536, 16, top-2           24 129 / 119   48 139 / 139              64 144 / 147   80 147 / 154
+    //   H=5120 I=3072, 8, top-2            32 166 / 132   64 178 / 156
+    // What an item of the second GEMM stores grows with the rows, what it reads with I (H=4096 I=256, 32 experts, top-2, 37 rows 89 / 85, 62 rows 94 / 102): hence
+    // the lines at I / 10 rows up to 40 and at I / 32 up to 64.  Calls of up to 128 tokens are so small that latencies decide: up to 80 rows (H=2048
+    // I=256, 8 experts, top-4, 50 rows 39 / 29, H=1024 I=3072, 4, top-2, 32 rows 51 / 37, H=7168 I=768, 16, top-8, 64 rows 139 / 131).  With I >= 4096 it
+    // stays at 16 rows: the rows of act that a tile reads are long there (H=1024 I=14336, 4 experts, 48 rows 138 / 131, 64 rows 139 / 149).
     // An expert of more rows than a unit takes its weights again for every unit.  The host cannot see one, but that it matters takes tokens and a
     // large layer: if all T tokens chose the same K experts, K * (T / 64 - 1) units would read 6 H I bytes each.  Up to 128 tokens, or with up to 16 rows
     // on average 96 MB, the kernel is ahead on any routing or close to it; us, general kernel / local_few.cu: 512 tokens on two experts, H=2048 I=512,
     // 84 MB 49 / 41; H=7168, 128 tokens on two experts, I=2048 92 / 77, on four 122 / 114, on eight, I=1024 130 / 123, I=768 114 / 114, 96 tokens on
-    // eight, I=768 103 / 110, 128 tokens with 32 rows on average on eight of 32, I=768 102 / 112 (the worst that was found).  Beyond, the routing decides on the GPU: both kernels are launched, and one returns at once,
-    // for 5 us (256 tokens, H=4096 I=768, 64 experts, top-4 268 / 215; all on two experts, H=7168 I=2048 95 / 98).  Kept to 1 / few_again of the
-    // experts with rows, such units cost less than the kernel gains: 192 tokens, H=7168 I=512, hottest expert three times the mean 195 / 167; 320, I=2048
-    // 619 / 612.
+    // eight, I=768 103 / 110, 128 tokens with 32 rows on average on eight of 32, I=768 102 / 112 (the worst that was found).  Beyond, the routing decides on
+    // the GPU: both kernels are launched, and one returns at once, for 5 us (256 tokens, H=4096 I=768, 64 experts, top-4 268 / 215; all on two experts,
+    // H=7168 I=2048 95 / 98).  Units beyond an expert's first may be 1 / few_again of the experts with rows: with 48 rows on average, hottest expert three
+    // times the mean, H=7168 I=2048 524 / 512, with 64 543 / 560.
     const bool sixteen = entries <= 16l * E;
     p.few_unit = entries <= 40l * E || T <= 64 ? 64 : 128;
-    p.few_again = sixteen ? 1 : p.few_unit == 64 ? 2 : 3;
-    const long again = (long)K * ((T + 63) / 64 - 1) * 6 * H * I;
-    const bool few = sixteen || (I < 4096 && entries <= 80l * E && (T <= 128 || 10 * entries <= (long)I * E));
+    p.few_again = sixteen ? 1 : p.few_unit == 64 ? 3 : 8;
+    const long again = (long)K * ((T + 63) / 64 - 1) * 6 * H * I, area = (long)I * E;
+    const bool few = sixteen || (I < 4096 && (T <= 128 ? entries <= 80l * E : (entries <= 40l * E && 10 * entries <= area) || (entries <= 64l * E && 32 * entries <= area)));
     p.few = keep || T <= 0 || !few ? 0 : T <= 128 || (sixteen && again <= 96l << 20) ? 1 : 2;
     p.routes = p.few == 1 && entries <= kDirectEntries;
     // Token rows through the loading warps, or copied into slot order first.  The loading warps load a row again for every tile of the other

@@ -131,12 +131,14 @@ def test_kernels_of_a_call_by_its_sizes():
 
 
 def test_which_forwards_have_few_rows_per_expert():
-    """Up to 16 rows on average, up to 80 where I is below 4096 and either at least ten times that or there are 128 tokens at most."""
+    """Up to 16 rows on average; where I is below 4096 up to 40 and I / 10, up to 64 and I / 32, and with 128 tokens at most up to 80."""
     from teramoe_b200._build import load_ext
     few = lambda T, K, E, I: load_ext().local_layer_variant(T, K, E, 4096, I, False)["few"]
     assert [few(T, 2, 8, 256) for T in (64, 65, 128)] == [1, 1, 1]
     assert [few(T, 2, 16, 256) for T in (128, 129, 204, 205)] == [1, 2, 2, 0]
-    assert [few(T, 2, 8, 4032) for T in (128, 129, 320, 321)] == [1, 2, 2, 0]
+    assert [few(T, 2, 8, 4032) for T in (128, 129, 256, 257)] == [1, 2, 2, 0]
+    assert [few(T, 2, 8, 1536) for T in (160, 161, 192, 193)] == [2, 2, 2, 0]
+    assert [few(T, 6, 8, 64) for T in (106, 107)] == [1, 0]
     assert [few(T, 2, 8, 4096) for T in (64, 65)] == [1, 0]
     assert few(128, 8, 8, 4032) == 0
     assert load_ext().local_layer_variant(128, 2, 8, 4096, 4032, True)["few"] == 0

@@ -237,9 +237,9 @@ def test_forward_with_few_rows_per_expert(counts, empty, H, I, K, monkeypatch):
     ([200, 50, 50], 25, 307, 1088, 320, 2, False),       # three units beyond the first ones of three experts
     ([100, 20, 5], 4, 128, 320, 64, 1, True),            # units of 128 rows
     ([60, 1], 3, 64, 320, 64, 1, True),                  # (not where there are no more tokens than 64)
-    ([1, 15, 17, 33, 64, 65, 95, 96, 97, 127, 128, 129], 30, 870, 192, 640, 2, True),      # a last tile of weights that is half outside
-    ([1, 15, 17, 33, 64, 65, 95, 96, 97, 127, 128, 129], 30, 870, 1088, 1024, 2, True),
-    ([257, 129, 128], 24, 520, 1088, 448, 2, False),     # as many units beyond the first as experts
+    ([1, 15, 17, 33, 64, 65, 95, 96, 97, 127, 128, 129], 30, 870, 192, 1920, 2, True),      # a last tile of weights that is half outside
+    ([1, 15, 17, 33, 64, 65, 95, 96, 97, 127, 128, 129], 30, 870, 1088, 1920, 2, True),
+    ([257, 129, 128], 24, 520, 1088, 1408, 2, False),     # as many units beyond the first as experts
 ])
 def test_forward_with_up_to_eighty_rows_per_expert(counts, E, T, H, I, few, ran, monkeypatch):
     """Rows at the edges of row copies (4), accumulator columns (16), reads of the accumulator (32) and units (64, 128); which kernel takes the
