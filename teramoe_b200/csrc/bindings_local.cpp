@@ -71,6 +71,16 @@ void use_tables(const c10::cuda::CUDAStream& writer, unsigned long long capture,
     now.block(stream);
 }
 
+// A tensor of its own over part of another one's memory, from byte `at` on.  An allocation costs the host about a microsecond, this a tenth of it: small
+// results and tables of one call lie in one block.
+torch::Tensor piece(const torch::Tensor& block, int64_t at, at::IntArrayRef sizes, at::ScalarType type) {
+    auto t = at::detail::make_tensor<c10::TensorImpl>(c10::Storage(block.storage()), c10::DispatchKeySet(c10::DispatchKey::CUDA),
+                                                      c10::scalarTypeToTypeMeta(type));
+    t.unsafeGetTensorImpl()->set_sizes_contiguous(sizes);
+    t.unsafeGetTensorImpl()->set_storage_offset(at / (int64_t)c10::elementSize(type));
+    return t;
+}
+
 // ------------------------------------------------------------------------------------------------ low latency
 // The statistics of waits are accepted as the window kernels accept them and left as they are: nothing is waited for here.
 void check_wait_stats(const c10::optional<torch::Tensor>& t) {
@@ -109,15 +119,18 @@ ll_local_dispatch(torch::Tensor x, torch::Tensor topk_idx, int64_t M, int64_t E,
     auto recv = torch::empty({E, M, H}, on(x, wire > 0 ? torch::kFloat8_e4m3fn : torch::kBFloat16));
     c10::optional<torch::Tensor> scales;
     if (wire > 0) scales = wire == 3 ? torch::empty({E, G / 4, M}, on(x, torch::kInt32)) : torch::empty({E, G, M}, on(x, torch::kFloat32));
-    auto count = torch::empty({E}, on(x, torch::kInt32));
-    auto src_info = torch::empty({E, M}, on(x, torch::kInt32));
-    auto range = torch::empty({E, 1}, on(x, torch::kInt64));
-    auto entry = torch::empty({tk.T, tk.K}, on(x, torch::kInt32));
+    const auto block = torch::empty({8 * E + 4 * (E + E * M + (int64_t)tk.T * tk.K)}, on(x, torch::kUInt8));
+    const auto range = piece(block, 0, {E, 1}, torch::kInt64), count = piece(block, 8 * E, {E}, torch::kInt32);
+    const auto src_info = piece(block, 12 * E, {E, M}, torch::kInt32), entry = piece(block, 12 * E + 4 * E * M, {tk.T, tk.K}, torch::kInt32);
     TM_CHECK_CUDA(tmoe::ll_local_dispatch(local_layout(E, M, H, (int)wire, false), x.data_ptr(), tk.ptr, tk.is64, tk.T, tk.K, recv.data_ptr(),
                                           scales.has_value() ? scales->data_ptr() : nullptr, src_info.data_ptr<int>(),
                                           reinterpret_cast<long long*>(range.data_ptr<int64_t>()), count.data_ptr<int>(), stats,
                                           entry.data_ptr<int>(), cur_stream()));
-    if (scales.has_value()) scales = scales->transpose(1, 2);
+    if (scales.has_value()) {
+        // [E, M, groups] over column-major memory
+        const int64_t groups = scales->size(1), sizes[3] = {E, M, groups}, strides[3] = {groups * M, 1, M};
+        scales->unsafeGetTensorImpl()->set_sizes_and_strides(sizes, strides);
+    }
     return {recv, scales, count, src_info, range, entry, c10::cuda::getCurrentCUDAStream().id()};
 }
 
@@ -146,16 +159,18 @@ torch::Tensor ll_local_combine(torch::Tensor x, torch::Tensor topk_idx, torch::T
 
 // ------------------------------------------------------------------------------------------------ un-fused exchange
 struct Scratch {
-    torch::Tensor all;
+    torch::Tensor all;                       // int32: totals [E + 2], row_local [T], chunk_base, and [T] for whoever asks
     int *totals, *row_local, *chunk_base;
+    int64_t extra;                           // byte of the last part
 };
 Scratch route_scratch(const torch::Tensor& idx, const TopK& tk, int64_t E) {
     const int64_t chunks = std::max<int64_t>(1, (tk.T + tmoe::kLocalChunk - 1) / tmoe::kLocalChunk);
     Scratch s;
-    s.all = torch::empty({E + 2 + tk.T + chunks}, on(idx, torch::kInt32));
+    s.all = torch::empty({E + 2 + 2 * (int64_t)tk.T + chunks}, on(idx, torch::kInt32));
     s.totals = s.all.data_ptr<int>();
     s.row_local = s.totals + E + 2;
     s.chunk_base = s.row_local + tk.T;
+    s.extra = (E + 2 + tk.T + chunks) * 4;
     return s;
 }
 
@@ -169,10 +184,10 @@ std::tuple<torch::Tensor, torch::Tensor, torch::Tensor> local_counts(torch::Tens
     topk_idx = topk_idx.contiguous();
     const TopK tk = topk_of(topk_idx);
     const auto s = route_scratch(topk_idx, tk, E);
-    auto in_rank = torch::empty({tk.T, 1}, on(topk_idx, torch::kBool));
+    const auto in_rank = piece(s.all, s.extra, {tk.T, 1}, torch::kBool);
     TM_CHECK_CUDA(tmoe::local_route(tk.ptr, tk.is64, tk.T, tk.K, (int)E, s.totals, s.row_local, s.chunk_base,
                                     reinterpret_cast<uint8_t*>(in_rank.data_ptr<bool>()), nullptr, 0, cur_stream()));
-    return {s.all.narrow(0, E, 1), s.all.narrow(0, 0, E), in_rank};
+    return {piece(s.all, 4 * E, {1}, torch::kInt32), piece(s.all, 0, {E}, torch::kInt32), in_rank};
 }
 
 // Events of dropped layouts, for the next ones: creating and destroying one costs about as much as recording it.
@@ -262,7 +277,7 @@ class LocalExchange {
             }
             idx_out = torch::empty({cap, tk.K}, topk_idx.options());
             w_out = torch::empty({cap, tk.K}, w.options());
-            const auto send_row = torch::empty({tk.T}, on(topk_idx, torch::kInt32));
+            const auto send_row = piece(s.all, s.extra, {tk.T}, torch::kInt32);
             const bool wait = worst_rows <= 0;
             if (wait) host_block(E + 1);
             TM_CHECK_CUDA(tmoe::local_route(tk.ptr, tk.is64, tk.T, tk.K, (int)E, s.totals, s.row_local, s.chunk_base, nullptr,
