@@ -314,11 +314,13 @@ bool make_parts(const LocalPart* parts, int n, Parts& ps) {
     return true;
 }
 
-// A block per eight segments, up to 16 blocks for each of a B200's 148 SMs; warps stride over the rest.  16384 rows of 14 KB, repeat of a dispatch:
-// 2 blocks per SM 78.6 us, 4 76.2, 8 79.0, 16 76.8, 64 71.9; combine with weights at 4096 rows: 23.1, 16.7, 16.4, 15.4, 16.5.
-int move_grid(long rows, int segs) {
-    const long blocks = (rows * segs + 7) / 8;
-    return (int)(blocks < 1 ? 1 : blocks > 148 * 16 ? 148 * 16 : blocks);
+// A block per eight segments, up to 16 blocks for each of a B200's 148 SMs, with more than `many` segments 64; warps stride over the rest.  us by blocks per
+// SM: 16384 rows of 14 KB (115 K segments), repeat of a dispatch 2 78.6, 4 76.2, 8 79.0, 16 77.7, 32 74.0, 64 72.6, dispatch 16 74.1, 64 72.5, with FP8 rows and
+// scales (82 K) 16 40.3, 64 41.6; 10000 rows (70 K), repeat 16 47.4, 64 45.2; combine with weights at 4096 rows (29 K) 2 23.1, 4 16.7, 8 16.4, 16 15.4, 64
+// 16.5.  Segments of 1 and 4 KB, or 32 bytes per lane and load, are slower (dispatch + repeat at 4096 rows 38.5; 1 KB 40.0, 4 KB 45.4, 32 bytes 40.6).
+int move_grid(long rows, int segs, long many) {
+    const long most = 148 * (rows * segs > many ? 64 : 16), blocks = (rows * segs + 7) / 8;
+    return (int)(blocks < 1 ? 1 : blocks > most ? most : blocks);
 }
 
 }  // namespace
@@ -349,7 +351,7 @@ cudaError_t local_dispatch(const LocalPart* parts, int num_parts, const void* to
     if (!make_parts(parts, num_parts, ps) || K > 32) return cudaErrorInvalidValue;
     const long rows = T > worst_rows ? T : worst_rows;
     if (rows == 0) return cudaSuccess;
-    local_dispatch_kernel<<<move_grid(rows, ps.total_segs), 256, 0, stream>>>(ps, topk_idx, is64, topk_w, T, K, E, totals, row_local, chunk_base,
+    local_dispatch_kernel<<<move_grid(rows, ps.total_segs, 96 * 1024), 256, 0, stream>>>(ps, topk_idx, is64, topk_w, T, K, E, totals, row_local, chunk_base,
                                                                              send_row, recv_idx, recv_w, worst_rows);
     return cudaGetLastError();
 }
@@ -359,7 +361,7 @@ cudaError_t local_move(const LocalPart* parts, int num_parts, const int* send_ro
     Parts ps{};
     if (!make_parts(parts, num_parts, ps) || K > 32) return cudaErrorInvalidValue;
     if (T == 0) return cudaSuccess;
-    local_move_kernel<<<move_grid(T, ps.total_segs), 256, 0, stream>>>(ps, send_row, T, rows, to_rows, topk_idx, is64, K, E, weights, weights_out);
+    local_move_kernel<<<move_grid(T, ps.total_segs, 64 * 1024), 256, 0, stream>>>(ps, send_row, T, rows, to_rows, topk_idx, is64, K, E, weights, weights_out);
     return cudaGetLastError();
 }
 
