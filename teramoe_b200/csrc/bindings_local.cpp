@@ -81,6 +81,9 @@ torch::Tensor piece(const torch::Tensor& block, int64_t at, at::IntArrayRef size
     return t;
 }
 
+// Where the next part of a block starts: on a boundary as an allocation has it.
+int64_t behind(int64_t at, int64_t bytes) { return (at + bytes + 511) / 512 * 512; }
+
 // ------------------------------------------------------------------------------------------------ low latency
 // The statistics of waits are accepted as the window kernels accept them and left as they are: nothing is waited for here.
 void check_wait_stats(const c10::optional<torch::Tensor>& t) {
@@ -119,9 +122,10 @@ ll_local_dispatch(torch::Tensor x, torch::Tensor topk_idx, int64_t M, int64_t E,
     auto recv = torch::empty({E, M, H}, on(x, wire > 0 ? torch::kFloat8_e4m3fn : torch::kBFloat16));
     c10::optional<torch::Tensor> scales;
     if (wire > 0) scales = wire == 3 ? torch::empty({E, G / 4, M}, on(x, torch::kInt32)) : torch::empty({E, G, M}, on(x, torch::kFloat32));
-    const auto block = torch::empty({8 * E + 4 * (E + E * M + (int64_t)tk.T * tk.K)}, on(x, torch::kUInt8));
-    const auto range = piece(block, 0, {E, 1}, torch::kInt64), count = piece(block, 8 * E, {E}, torch::kInt32);
-    const auto src_info = piece(block, 12 * E, {E, M}, torch::kInt32), entry = piece(block, 12 * E + 4 * E * M, {tk.T, tk.K}, torch::kInt32);
+    const int64_t at_count = behind(0, 8 * E), at_src = behind(at_count, 4 * E), at_entry = behind(at_src, 4 * E * M);
+    const auto block = torch::empty({at_entry + 4 * (int64_t)tk.T * tk.K}, on(x, torch::kUInt8));
+    const auto range = piece(block, 0, {E, 1}, torch::kInt64), count = piece(block, at_count, {E}, torch::kInt32);
+    const auto src_info = piece(block, at_src, {E, M}, torch::kInt32), entry = piece(block, at_entry, {tk.T, tk.K}, torch::kInt32);
     TM_CHECK_CUDA(tmoe::ll_local_dispatch(local_layout(E, M, H, (int)wire, false), x.data_ptr(), tk.ptr, tk.is64, tk.T, tk.K, recv.data_ptr(),
                                           scales.has_value() ? scales->data_ptr() : nullptr, src_info.data_ptr<int>(),
                                           reinterpret_cast<long long*>(range.data_ptr<int64_t>()), count.data_ptr<int>(), stats,
@@ -166,11 +170,11 @@ struct Scratch {
 Scratch route_scratch(const torch::Tensor& idx, const TopK& tk, int64_t E) {
     const int64_t chunks = std::max<int64_t>(1, (tk.T + tmoe::kLocalChunk - 1) / tmoe::kLocalChunk);
     Scratch s;
-    s.all = torch::empty({E + 2 + 2 * (int64_t)tk.T + chunks}, on(idx, torch::kInt32));
+    s.extra = behind(0, 4 * (E + 2 + tk.T + chunks));
+    s.all = torch::empty({s.extra / 4 + tk.T}, on(idx, torch::kInt32));
     s.totals = s.all.data_ptr<int>();
     s.row_local = s.totals + E + 2;
     s.chunk_base = s.row_local + tk.T;
-    s.extra = (E + 2 + tk.T + chunks) * 4;
     return s;
 }
 

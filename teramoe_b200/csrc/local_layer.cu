@@ -1434,7 +1434,7 @@ LocalLayerPlan local_layer_plan(int T, int K, int E, int H, int I, int keep) {
     p.units_cap = (int)((p.blocks_cap + segs) / 2);
     const int rows = (int)(entries / (segs > 0 ? segs : 1));
     // Few rows per expert, forward only: weights as the M operand (local_few.cu), 64 rows of an expert at a time, from 41 on average 128.  us, general
-    // kernel / local_few.cu, by rows per expert (even routing; in brackets units of 64 and of 128 rows, measured on another box):
+    // kernel / local_few.cu, by rows per expert (even routing; in brackets units of 64 and of 128 rows, measured at another time):
     //   H=7168 I=2048, 32 experts, top-8   20 489 / 425   32 507 / 438 (463, 475)   48 523 / 484 (496, 506)   64 534 / 515 (651, 539)   80 545 / 543
     //   H=2048 I=512, 64, top-4            32 103 / 98    48 107 / 108 (106, 107)   51 110 / 113
     //   H=4096 I=1536, 16, top-2           24 129 / 119   48 139 / 139              64 144 / 147   80 147 / 154

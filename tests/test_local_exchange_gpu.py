@@ -124,6 +124,25 @@ def test_layout_of_many_tokens(T, E, K):
     buf.destroy()
 
 
+@pytest.mark.parametrize("T,E,K,M", [(5, 33, 3, 7), (1, 2, 1, 1), (0, 40, 2, 4)])
+def test_results_of_a_call_do_not_overlap_and_start_as_allocations_do(T, E, K, M):
+    """They lie in one block: every one on a boundary of its own, and writing one leaves the others alone."""
+    idx, w = _routing(T, E, K, seed=3, dtype=torch.int64)
+    buf = tm.Buffer(None, tm.Buffer.get_low_latency_rdma_size_hint(M, 512, 1, E), low_latency_mode=True, explicitly_destroy=True)
+    x = torch.randn(T, 512, device="cuda").to(torch.bfloat16)
+    (_, scales), count, handle, _, _ = buf.low_latency_dispatch(x, idx, M, E)
+    assert scales.shape == (E, M, 4) and scales.stride() == (4 * M, 1, M)
+    per_rank, _, per_expert, in_rank, _ = buf.get_dispatch_layout(idx, E)
+    for block in ((handle.layout_range, count, handle.src_info, handle.entry_row), (per_expert, in_rank)):
+        block = [t for t in block if t.numel()]
+        assert all(t.data_ptr() % 512 == 0 and t.is_contiguous() for t in block)
+        for t in block:
+            before = [o.clone() for o in block if o is not t]
+            t.fill_(1)
+            assert all(torch.equal(o, b) for o, b in zip([o for o in block if o is not t], before))
+    buf.destroy()
+
+
 def _stall(stream, ms=40):
     with torch.cuda.stream(stream):
         torch.cuda._sleep(int(ms * 1.5e6))             # cycles
