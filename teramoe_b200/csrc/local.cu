@@ -10,8 +10,8 @@
 // flight per lane), so that a few hundred rows already fill the SMs.  Through the symmetric arena the same dispatch took a
 // push into the arena, a copy out of it, nine table copies and two waits of the host.  Measured through the API, hidden 7168,
 // top-8, 32 experts: layout + dispatch + combine + cached dispatch + combine with weights at 4096 tokens 1216 -> 96 us (77 launches
-// before), layout + FP8 dispatch + combine at 1003 tokens 736 -> 47 us.
-// The latter is host work: five allocations and four launches, and the wait for the counts, for which the host watches the pinned
+// before), layout + FP8 dispatch + combine at 1003 tokens 736 -> 42 us.
+// The latter is host work: four allocations and four launches, and the wait for the counts, for which the host watches the pinned
 // words that the route kernel writes (an event behind it was seen a few microseconds later).
 #include "local.h"
 

@@ -1,7 +1,7 @@
 // The MoE layer on one rank, see local_layer.h.  Roles of the persistent kernel (74 CTA pairs, 16 warps per CTA):
 //
 //   producer   claims items of the work list, hands them to the pair, loads operand tiles by TMA
-//   issuer     tcgen05 cta_group::2, 256x256 or 256x512 tiles, two accumulators in tensor memory
+//   issuer     tcgen05 cta_group::2, 256x256 or 256x512 tiles (128 rows for a unit of one block), two accumulators in tensor memory
 //   loaders    4 warps: bring the operands that are made of token rows from the caller's tensor (load_rows).  An instance of the kernel
 //              has none: there all warps but the first two copy rows into slot order (copy role), and the producer loads them
 //   epilogue   8 warps: SwiGLU / dSwiGLU / store.  A warp packs 32 rows x 64 columns into shared memory (128-byte swizzle) and
@@ -20,11 +20,11 @@
 // left around the kernel.
 //
 // Forward + backward through the API, several-rank kernels (30 to 38 launches and one host wait per step) -> these:
-//   512 tokens, H=512 I=256, 4 experts, top-2            873 ->    97 us   (was host work and launches)
-//   4096, H=2048 I=2048, 16 experts, top-8              2914 ->  2321 us
-//   8192, H=2048 I=3072, 16 experts, top-6              6192 ->  5030 us
-//   8192, H=7168 I=2048, 32 experts, top-8             16737 -> 15056 us
-//   16384, H=7168 I=512, 32 experts, top-8             10388 ->  8429 us
+//   512 tokens, H=512 I=256, 4 experts, top-2            873 ->    96 us   (was host work and launches)
+//   4096, H=2048 I=2048, 16 experts, top-8              2914 ->  2206 us
+//   8192, H=2048 I=3072, 16 experts, top-6              6192 ->  4780 us
+//   8192, H=7168 I=2048, 32 experts, top-8             16737 -> 14385 us
+//   16384, H=7168 I=512, 32 experts, top-8             10388 ->  8166 us
 // Large layers are bound by the power cap: the SM clock drops to 1.0 to 1.3 GHz, and time is energy (0.86 pJ per FLOP at H=7168 I=2048, of
 // which cuBLAS alone takes 0.74).
 #include "local_layer.h"
@@ -1461,11 +1461,11 @@ LocalLayerPlan local_layer_plan(int T, int K, int E, int H, int I, int keep) {
     // Token rows through the loading warps, or copied into slot order first.  The loading warps load a row again for every tile of the other
     // operand, with more energy per byte than TMA; a copy is written and read once.  us of a step, backward by loaders / by copies, by rows per
     // expert:
-    //   H=7168 I=2048, 32 experts, top-8   16 1918 / 1748   128 2344 / 2150   256 3144 / 2992   512 4682 / 4567   1024 7629 / 7642
-    //   H=7168 I=512, 32, top-8            16 549 / 518     128 701 / 661     256 926 / 919     512 1392 / 1448
-    //   H=4096 I=3072, 16, top-2           32 902 / 808     128 1074 / 964    512 2162 / 2035   1024 3308 / 3243
+    //   H=7168 I=2048, 32 experts, top-8   16 1867 / 1662   128 2309 / 2080   256 3141 / 3001   512 4720 / 4683   1024 7861 / 7822
+    //   H=7168 I=512, 32, top-8            16 554 / 494     128 689 / 650     256 919 / 916     512 1416 / 1476
+    //   H=4096 I=3072, 16, top-2           32 902 / 808     128 1060 / 943    512 2151 / 2086   1024 3386 / 3315
     //   H=4096 I=4096, 16, top-2           32 1172 / 1048   128 1394 / 1248   512 2846 / 2670
-    //   H=2048 I=768, 32, top-4            32 279 / 250     128 333 / 309     512 648 / 671
+    //   H=2048 I=768, 32, top-4            32 279 / 241     128 327 / 306     512 649 / 675
     //   H=4096 I=14336, 8, top-2           128 2385 / 2120  1024 8002 / 7722
     // A forward, by loaders / by copies:
     //   H=7168 I=2048                      17 563 / 561     64 612 / 611      256 994 / 1019    512 1471 / 1507

@@ -431,9 +431,9 @@ ll_combine_recv_kernel(LowLatLayout lay, const uint8_t* arena, const void* topk_
 //
 // Both kernels move a few MB and are bound by how fast enough loads are in flight: a warp owns 256 channels of a token (16
 // bytes per lane), and the grid splits tokens and channels so that a single token still spreads over several SMs.
-// Measured as dispatch + combine through the API, hidden 7168, top-8, 32 experts: 128 tokens, FP8 out and bf16 back 392 -> 52 us
+// Measured as dispatch + combine through the API, hidden 7168, top-8, 32 experts: 128 tokens, FP8 out and bf16 back 392 -> 48 us
 // (the window kernels alone took 301 us: a block per expert found its tokens and cast every row once per expert, and the
-// combine waited for one load after the other); 77 tokens, UE8M0 out and LogFMT-10 back with hooks 580 -> 51 us.
+// combine waited for one load after the other); 77 tokens, UE8M0 out and LogFMT-10 back with hooks 580 -> 48 us.
 // The kernels themselves, us, with 64 experts at 512 tokens: dispatch with FP8 of 16 tokens 3.8, 128 5.9, 512 13.7 (before, with a division per row for the
 // place of its scale, indices of earlier tokens one at a time and a match.any: 4.8, 8.5, 19.7); combine of LogFMT rows of 1 token 3.4, 77 15.1,
 // 512 84 (13.4, 18.0, 99), of bf16 rows 2.7, 3.6, 12.2.
