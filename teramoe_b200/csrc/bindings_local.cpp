@@ -573,17 +573,9 @@ class LocalLayer : public std::enable_shared_from_this<LocalLayer> {
         if (!last_[dir].defined()) return c10::nullopt;
         return last_[dir].narrow(0, last_at_[dir], 48).view(torch::kInt64);
     }
-    // whether the last forward ran in local_few.cu (reads the routing's word back)
-    bool ran_few() {
-        torch::Tensor ws;
-        int64_t at;
-        {
-            std::lock_guard<std::mutex> lock(mutex_);
-            ws = last_[0];
-            at = last_few_;
-        }
-        return ws.defined() && ws[at].item<int>() != 0;
-    }
+    // whether the last forward ran in local_few.cu, and the rows of a unit there (read the workspace back)
+    bool ran_few() { return last_meta(tmoe::kMetaFew) != 0; }
+    int64_t few_unit() { return last_meta(tmoe::kMetaFewUnit); }
 
   private:
     // (with arena_mutex_ held, until the launch)
@@ -597,12 +589,22 @@ class LocalLayer : public std::enable_shared_from_this<LocalLayer> {
         p.status = status_.data_ptr<int>();
         ++launches_;
     }
+    int last_meta(int word) {
+        torch::Tensor ws;
+        int64_t at;
+        {
+            std::lock_guard<std::mutex> lock(mutex_);
+            ws = last_[0];
+            at = last_meta_ + word;
+        }
+        return ws.defined() ? ws[at].item<int>() : 0;
+    }
     void note(int dir, const torch::Tensor& ws, const tmoe::LocalLayerPlan& plan) {
         torch::Tensor before = ws;            // (the one that goes may have to wait for the interpreter: not under the lock)
         std::lock_guard<std::mutex> lock(mutex_);
         std::swap(last_[dir], before);
         last_at_[dir] = plan.stats[dir];
-        if (dir == 0) last_few_ = plan.meta + tmoe::kMetaFew;
+        if (dir == 0) last_meta_ = plan.meta;
     }
     torch::Tensor status_, host_;
     // A backward pass runs without the interpreter's lock, next to a call that replaces the arena.
@@ -611,7 +613,7 @@ class LocalLayer : public std::enable_shared_from_this<LocalLayer> {
     std::atomic<bool> open_{true};
     std::mutex mutex_;
     torch::Tensor last_[2];
-    int64_t last_at_[2] = {0, 0}, last_few_ = 0;
+    int64_t last_at_[2] = {0, 0}, last_meta_ = 0;
 };
 
 // The layer as a native autograd node: a backward pass runs on autograd's worker thread without the interpreter.
@@ -724,6 +726,7 @@ void register_local(pybind11::module_& m) {
         .def("check", &LocalLayer::check)
         .def("stats", &LocalLayer::stats)
         .def("ran_few", &LocalLayer::ran_few, py::call_guard<py::gil_scoped_release>())
+        .def("few_unit", &LocalLayer::few_unit, py::call_guard<py::gil_scoped_release>())
         .def("call", &local_layer_call);
     m.def("local_layer_variant", &local_layer_variant);
     m.def("local_layer_halves", &local_layer_halves);

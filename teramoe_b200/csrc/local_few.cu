@@ -14,7 +14,7 @@
 //   warps 4-7  epilogue: a lane holds one row of weights, so gate and up of a token sit in neighbouring lanes
 //   warps 2-7  at the end of their items: sums of the tokens' expert rows, in the order of their entries
 // Nine stages of 24 KB keep 144 KB of weights per SM on their way; with units of 128 rows, six of 32 KB keep 96 KB, which costs 2 to 4 % where experts
-// have few rows (32 tokens as above 430 / 449) and saves reading weights again where many have more than 64 (256 tokens 651 / 539).
+// have few rows (32 tokens as above 430 / 449) and saves reading weights again where many have more than 64 (256 tokens 651 / 539).  wide_units chooses.
 //
 // Where the host can tell that this kernel takes the call (LocalLayerPlan::routes) it makes the routing tables too, in front of a barrier of the whole grid:
 // a kernel of their own costs 5 us, and a boundary between two kernels of a stream up to 2 us more.  us of a forward, routing kernel / here / here with the
@@ -38,19 +38,24 @@ constexpr int kFewAccs = 4;
 constexpr int kFewThreads = 256;
 constexpr int kFewEpiWarps = 4;
 constexpr int kFewSumWarps = 6;
+constexpr long kFewReadAgain = 64l << 20;                                 // wide_units
 
-// What follows from the rows of a unit
+// Shared memory: the operand stages, barriers, [experts + 1] first unit, [experts] rows, [experts] first slot
 template <int UNIT>
 struct Few {
     static constexpr int kStageBytes = kAStageBytes + UNIT * BK * 2;      // 24 KB, 32 KB
     static constexpr int kStages = UNIT == 64 ? 9 : 6;
-    static constexpr int kBarOffset = kStages * kStageBytes;
-    static constexpr int kUnitsOffset = kBarOffset + 256;                 // [experts + 1] first unit, [experts] rows, [experts] first slot
-    static constexpr int kSmemBytes = kUnitsOffset + (3 * kLocalMaxExperts + 1) * 4 + 1024;
-    static_assert(8 * (2 * kStages + 2 * kFewAccs) <= 248 && kSmemBytes <= 232448, "shared memory");
-    static_assert(kFewThreads == kRouteThreads, "routing");
     static_assert(UNIT % 64 == 0 && 128 % UNIT == 0 && kFewAccs * UNIT <= 512, "units");
 };
+constexpr int kFewMostStages = Few<64>::kStages;
+constexpr int kFewBarOffset = kFewMostStages * Few<64>::kStageBytes;
+constexpr int kFewUnitsOffset = kFewBarOffset + 256;
+constexpr int kFewSmemBytes = kFewUnitsOffset + (3 * kLocalMaxExperts + 1) * 4 + 1024;
+static_assert(Few<128>::kStages * Few<128>::kStageBytes <= kFewBarOffset, "stages");
+static_assert(8 * (2 * kFewMostStages + 2 * kFewAccs) <= 240 && kFewSmemBytes <= 232448, "shared memory");
+// The routing works in the last stages, before they are loaded.
+constexpr int kFewRouteOffset = 7 * Few<64>::kStageBytes;
+static_assert(kFewRouteOffset + route_words(kLocalMaxExperts) * 4 <= kFewBarOffset && kFewThreads == kRouteThreads, "routing");
 
 struct FewArgs {
     alignas(64) CUtensorMap map_wg, map_wd, map_act;
@@ -68,6 +73,7 @@ struct FewArgs {
     int* done2;                          // the same for the second
     unsigned long long* stats;
     int* status;
+    int* ran_unit;                       // for whoever asks: rows of a unit
     const int* wanted;                   // the routing's word for this kernel; null: it takes the call
 };
 
@@ -75,28 +81,30 @@ struct FewItem {
     int second, expert, tile, slot0, rows, n;      // n: columns of the accumulator that are computed
 };
 
-template <int UNIT, bool ROUTES>
-__global__ void __launch_bounds__(kFewThreads, 1) local_few_kernel(const __grid_constant__ FewArgs L, const __grid_constant__ RouteArgs R) {
-    if (L.wanted != nullptr && *L.wanted == 0) return;
-    constexpr int kUnit = UNIT, kFewStages = Few<UNIT>::kStages, kFewStageBytes = Few<UNIT>::kStageBytes;
-    extern __shared__ uint8_t smem_raw[];
-    const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-    uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
-    const uint32_t bar_base = smem_base + Few<UNIT>::kBarOffset;
-    auto full_bar = [&](int s) { return bar_base + 8u * s; };
-    auto empty_bar = [&](int s) { return bar_base + 8u * (kFewStages + s); };
-    auto tfull_bar = [&](int a) { return bar_base + 8u * (2 * kFewStages + a); };
-    auto tempty_bar = [&](int a) { return bar_base + 8u * (2 * kFewStages + kFewAccs + a); };
-    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + Few<UNIT>::kBarOffset + 248);
-    volatile uint32_t* abort_flag = tmem_slot + 1;
-    int* units = reinterpret_cast<int*>(smem_gen + Few<UNIT>::kUnitsOffset);
-    int* counts = units + L.E + 1;
-    int* seg = counts + L.E;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, E = L.E;
+// What both kernels have in shared memory
+struct FewShared {
+    uint32_t base, bars;
+    uint8_t* gen;
+    volatile uint32_t* words;                // [0] address in tensor memory, [1] abort flag, [2] rows of a unit
+    int *units, *counts, *seg;
 
-    if (threadIdx.x == 0) {
-        *abort_flag = 0u;
-        for (int s = 0; s < kFewStages; ++s) {
+    __device__ __forceinline__ FewShared(uint8_t* raw, int E) {
+        base = (smem_u32(raw) + 1023u) & ~1023u;
+        gen = raw + (base - smem_u32(raw));
+        bars = base + kFewBarOffset;
+        words = reinterpret_cast<volatile uint32_t*>(gen + kFewBarOffset + 240);
+        units = reinterpret_cast<int*>(gen + kFewUnitsOffset);
+        counts = units + E + 1;
+        seg = counts + E;
+    }
+    __device__ __forceinline__ uint32_t full_bar(int s) const { return bars + 8u * s; }
+    __device__ __forceinline__ uint32_t empty_bar(int s) const { return bars + 8u * (kFewMostStages + s); }
+    __device__ __forceinline__ uint32_t tfull_bar(int a) const { return bars + 8u * (2 * kFewMostStages + a); }
+    __device__ __forceinline__ uint32_t tempty_bar(int a) const { return bars + 8u * (2 * kFewMostStages + kFewAccs + a); }
+
+    __device__ __forceinline__ void init(const FewArgs& L) const {
+        words[1] = 0u;
+        for (int s = 0; s < kFewMostStages; ++s) {
             mbar_init(full_bar(s), 1 + 32);                  // the producer, and every lane of a loading warp
             mbar_init(empty_bar(s), 1);
         }
@@ -109,33 +117,12 @@ __global__ void __launch_bounds__(kFewThreads, 1) local_few_kernel(const __grid_
         tma_prefetch_desc(&L.map_wd);
         tma_prefetch_desc(&L.map_act);
     }
-    if (warp == 2) tmem_alloc(smem_u32((const void*)tmem_slot), kFewAccs * kUnit);
-    // Routing in the same launch: a few blocks write the tables, the others only count.  All know the units then, and those others have the weights
-    // of their first item on their way while they wait for the tables.  (The stages that the routing works in, the last ones, are left out.)
-    constexpr int kRouteStages = 2;
-    static_assert(route_words(kLocalMaxExperts) * 4 <= kRouteStages * kFewStageBytes, "routing");
-    int* route = reinterpret_cast<int*>(smem_gen + (kFewStages - kRouteStages) * kFewStageBytes);
-    bool counts_only = false;
-    if constexpr (ROUTES) {
-        __shared__ int bound[4];
-        clear_counters(R);
-        const int blocks = R.p.chunks + kRouteTableBlocks;
-        counts_only = (int)blockIdx.x >= blocks;
-        if (counts_only) {
-            for (int i = threadIdx.x; i < 2 * E + 1; i += kFewThreads) route[route_totals(E) + i] = 0;
-            __syncthreads();
-            count_entries(R, route + route_totals(E), nullptr, 0);
-        }
-        for (int b = blockIdx.x; b < blocks; b += gridDim.x) {
-            __syncthreads();
-            route_assign<true>(R, route, bound, b, blocks);
-        }
-        __syncthreads();
-    }
-    if (warp == 1) {
+    // One warp: units of 64 or 128 rows and slots of every expert, from its rows
+    __device__ __forceinline__ void lay_out(const int* rows, int E, int unit, int lane) const {
+        const int log_unit = unit == 64 ? 6 : 7;
         int run = 0, run_s = 0;
         for (int e0 = 0; e0 < E; e0 += 32) {
-            const int e = e0 + lane, c = e < E ? (ROUTES ? route[route_totals(E) + e] : L.counts[e]) : 0, own = (c + kUnit - 1) / kUnit, own_s = (c + 127) & ~127;
+            const int e = e0 + lane, c = e < E ? rows[e] : 0, own = (c + unit - 1) >> log_unit, own_s = (c + 127) & ~127;
             int v = own, s = own_s;
             for (int o = 1; o < 32; o <<= 1) {
                 const int u = __shfl_up_sync(0xffffffffu, v, o), us = __shfl_up_sync(0xffffffffu, s, o);
@@ -154,10 +141,20 @@ __global__ void __launch_bounds__(kFewThreads, 1) local_few_kernel(const __grid_
         }
         if (lane == 0) units[E] = run;
     }
-    tcgen05_fence_before();
-    __syncthreads();
-    tcgen05_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
+};
+
+// The layer, once the units are known.  ROUTES: the tables are being written; counts_only: not by this block.  (The body of the kernels, for each size of a unit.)
+template <int UNIT, bool ROUTES>
+__device__ __forceinline__ void few_layer(const FewArgs& L, const FewShared& sh, uint32_t tmem_base, bool counts_only) {
+    constexpr int kUnit = UNIT, kFewStages = Few<UNIT>::kStages, kFewStageBytes = Few<UNIT>::kStageBytes;
+    const uint32_t smem_base = sh.base;
+    auto full_bar = [&](int s) { return sh.full_bar(s); };
+    auto empty_bar = [&](int s) { return sh.empty_bar(s); };
+    auto tfull_bar = [&](int a) { return sh.tfull_bar(a); };
+    auto tempty_bar = [&](int a) { return sh.tempty_bar(a); };
+    volatile uint32_t* abort_flag = sh.words + 1;
+    const int *units = sh.units, *counts = sh.counts, *seg = sh.seg;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, E = L.E;
 
     const int n1 = 2 * L.I / BM, n2 = (L.H + BM - 1) / BM, U = units[E], items = U * (n1 + n2);
     auto decode = [&](int i) {
@@ -182,9 +179,10 @@ __global__ void __launch_bounds__(kFewThreads, 1) local_few_kernel(const __grid_
     const int nk1 = L.H / BK, nk2 = L.I / BK;
     int primed = 0;                                              // steps of this block's first item whose weights are on their way
     if constexpr (ROUTES) {
+        // Blocks that do not write the tables have the weights of their first item on their way while they wait for them.
         fence_proxy_async_smem();                                // what the routing wrote is written over by copies
         if (counts_only && (int)blockIdx.x < U * n1) {
-            primed = min(nk1, kFewStages - kRouteStages);
+            primed = min(nk1, kFewRouteOffset / kFewStageBytes);
             if (warp == 0 && lane == 0) {
                 const FewItem q = decode(blockIdx.x);
                 for (int s = 0; s < primed; ++s) {
@@ -296,17 +294,22 @@ __global__ void __launch_bounds__(kFewThreads, 1) local_few_kernel(const __grid_
         for (int i = blockIdx.x; i < U * n1 && ok; i += gridDim.x) {
             const FewItem q = decode(i);
             const int quads = (q.rows + 3) / 4;
-            // of rows lane + 32 c; past the last row that one again, whose copies nobody reads (of all SMs the same row would be one hot line of L2)
-            int token[kUnit / 32];
+            // of rows 4 j + sub, which this lane copies pieces of; past the last row that one again, whose copies nobody reads (of all SMs the same row would be
+            // one hot line of L2).  Asking the other lanes in every step instead, with units of 128 rows the loading warps are what the step waits for: 128 tokens on the
+            // same eight experts, H=7168 I=768, first GEMM 60 / 53 us.
+            int token[kUnit / 4];
 #pragma unroll
-            for (int c = 0; c < kUnit / 32; ++c) token[c] = L.slot_tk[q.slot0 + min(lane + 32 * c, q.rows - 1)] / L.K;
+            for (int c = 0; c < kUnit / 32; ++c) {
+                const int t = L.slot_tk[q.slot0 + min(lane + 32 * c, q.rows - 1)] / L.K;
+#pragma unroll
+                for (int j = 0; j < 8; ++j) token[8 * c + j] = __shfl_sync(0xffffffffu, t, 4 * j + sub);
+            }
             for (; step < nk1; step += 2) {
                 if (!(ok = mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag, L.status, 686))) break;
                 const uint32_t dst = smem_base + stage * kFewStageBytes + kAStageBytes;
                 const uint8_t* src = L.x + step * (BK * 2) + 16 * chunk;
                 auto copy = [&](int j) {
-                    const int t = __shfl_sync(0xffffffffu, token[j >> 3], (4 * j + sub) & 31);
-                    cp_async_16(dst + j * 512 + at[j & 1], src + (long)t * (L.H * 2l));
+                    cp_async_16(dst + j * 512 + at[j & 1], src + (long)token[j] * (L.H * 2l));
                 };
                 if (quads <= 4) {
 #pragma unroll
@@ -433,24 +436,119 @@ __global__ void __launch_bounds__(kFewThreads, 1) local_few_kernel(const __grid_
                                                                                 (int)pack_bf16x2(sum[4], sum[5]), (int)pack_bf16x2(sum[6], sum[7]));
         }
     }
+}
+
+// All units of UNIT rows, tables by a routing kernel
+template <int UNIT>
+__global__ void __launch_bounds__(kFewThreads, 1) local_few_kernel(const __grid_constant__ FewArgs L) {
+    if (L.wanted != nullptr && *L.wanted == 0) return;
+    extern __shared__ uint8_t smem_raw[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const FewShared sh(smem_raw, L.E);
+    if (threadIdx.x == 0) sh.init(L);
+    if (warp == 2) tmem_alloc(smem_u32((const void*)sh.words), kFewAccs * UNIT);
+    if (warp == 1) sh.lay_out(L.counts, L.E, UNIT, lane);
+    if (threadIdx.x == 0 && blockIdx.x == 0) *L.ran_unit = UNIT;
+    tcgen05_fence_before();
+    __syncthreads();
+    tcgen05_fence_after();
+    const uint32_t tmem_base = sh.words[0];
+    few_layer<UNIT, false>(L, sh, tmem_base, false);
     tcgen05_fence_before();
     __syncthreads();
     if (warp == 2) {
         tcgen05_fence_after();
-        tmem_dealloc(tmem_base, kFewAccs * kUnit);
+        tmem_dealloc(tmem_base, kFewAccs * UNIT);
     }
 }
 
-template <int UNIT, bool ROUTES>
-cudaError_t launch(const FewArgs& L, const RouteArgs& R, int num_sms, cudaStream_t stream) {
-    static bool configured[64] = {};
-    if (cudaError_t e = ensure_smem_limit(local_few_kernel<UNIT, ROUTES>, Few<UNIT>::kSmemBytes, configured); e != cudaSuccess) return e;
+// Whether units of 128 rows take less time than those of 64, by one warp from the entries per expert.  With 64 an expert of more rows has its weights multiplied
+// again, from L2; with 128 there are fewer tiles, which may not fill the blocks, and a step of K takes longer: 0.62 + 1.1 rows / 128 of one with 64 rows at most (a
+// first GEMM of one turn, H=7168 I=768, 64 / 80 / 96 / 112 / 128 rows 37 / 43 / 44 / 51 / 53 us).  Compared are the steps of a block: whole turns of its tiles through the grid and
+// as they would be dealt out evenly, half and half, as a last turn runs next to the second GEMM.  us of a forward, H=7168, general kernel / 64 / 128, tokens all
+// on as many experts as they have entries:
+//   128, I=512, top-8   95 / 82 / 97     I=768, 8   101 / 109 / 105     I=768, 4   84 / 74 / 84      I=2048, 8   200 / 222 / 177     I=2048, 4   113 / 114 / 112
+//    96, I=768, top-8   97 / 107 / 91    80, I=3072, 8  275 / 318 / 219                  128 on ten of 32, top-8, I=768 111 / 119 / 104, I=2048 227 / 270 / 206
+//   128 evenly on eight, top-4, I=1024 106 / 100 / 89, I=3072 262 / 232 / 211; on sixteen, top-8, I=2048 334 / 338 / 284
+// Below 64 MB the weights that are read again cost less than the larger unit's steps (H=2048 I=512, 128 on ten of 32, top-8, 60 MB 52 / 43 / 50).
+__device__ __forceinline__ bool wide_units(const FewArgs& L, const int* totals, int lane) {
+    uint32_t all = 0, most = 0, narrow = 0, wide = 0;
+    for (int e = lane; e < L.E; e += 32) {
+        const uint32_t n = (uint32_t)totals[e];
+        all += n;
+        most = max(most, n);
+        narrow += (n + 63) / 64;
+        wide += (n + 127) / 128;
+    }
+    narrow = __reduce_add_sync(0xffffffffu, narrow);
+    wide = __reduce_add_sync(0xffffffffu, wide);
+    all = __reduce_add_sync(0xffffffffu, all);
+    most = __reduce_max_sync(0xffffffffu, most);
+    const float blocks = (float)gridDim.x, rows = 0.5f * (min(most, 128u) + (float)all / wide);
+    auto steps = [&](uint32_t units) {
+        auto turns = [&](int tiles) {
+            const float n = (float)(units * tiles) / blocks;
+            return 0.5f * (ceilf(n) + fmaxf(n, 1.f));
+        };
+        return turns(2 * L.I / BM) * (L.H / BK) + turns((L.H + BM - 1) / BM) * (L.I / BK);
+    };
+    return (narrow - wide) * 6l * L.H * L.I > kFewReadAgain && steps(wide) * (0.62f + 1.1f * rows / 128.f) < steps(narrow);
+}
+
+// Routing in the same launch: a few blocks write the tables, the others only count.  All know the units then.
+__global__ void __launch_bounds__(kFewThreads, 1) local_few_routes_kernel(const __grid_constant__ FewArgs L, const __grid_constant__ RouteArgs R) {
+    extern __shared__ uint8_t smem_raw[];
+    __shared__ int bound[4];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, E = L.E;
+    const FewShared sh(smem_raw, E);
+    if (threadIdx.x == 0) sh.init(L);
+    if (warp == 2) tmem_alloc(smem_u32((const void*)sh.words), 512);
+    int* route = reinterpret_cast<int*>(sh.gen + kFewRouteOffset);
+    int* totals = route + route_totals(E);
+    clear_counters(R);
+    const int blocks = R.p.chunks + kRouteTableBlocks;
+    const bool counts_only = (int)blockIdx.x >= blocks;
+    if (counts_only) {
+        for (int i = threadIdx.x; i < 2 * E + 1; i += kFewThreads) totals[i] = 0;
+        __syncthreads();
+        count_entries(R, totals, nullptr, 0);
+    }
+    for (int b = blockIdx.x; b < blocks; b += gridDim.x) {
+        __syncthreads();
+        route_assign<true>(R, route, bound, b, blocks);
+    }
+    __syncthreads();
+    if (warp == 1) {
+        const bool wide = wide_units(L, totals, lane);
+        sh.lay_out(totals, E, wide ? 128 : 64, lane);
+        if (lane == 0) {
+            sh.words[2] = wide ? 128u : 64u;
+            if (blockIdx.x == 0) *L.ran_unit = wide ? 128 : 64;
+        }
+    }
+    tcgen05_fence_before();
+    __syncthreads();
+    tcgen05_fence_after();
+    const uint32_t tmem_base = sh.words[0];
+    if (sh.words[2] == 64u) few_layer<64, true>(L, sh, tmem_base, counts_only);
+    else few_layer<128, true>(L, sh, tmem_base, counts_only);
+    tcgen05_fence_before();
+    __syncthreads();
+    if (warp == 2) {
+        tcgen05_fence_after();
+        tmem_dealloc(tmem_base, 512);
+    }
+}
+
+template <typename... Args>
+cudaError_t launch(void (*kernel)(Args...), bool (&configured)[64], int num_sms, cudaStream_t stream, const Args&... args) {
+    if (cudaError_t e = ensure_smem_limit(kernel, kFewSmemBytes, configured); e != cudaSuccess) return e;
     const int sms = default_sms(num_sms) & ~1;
     if (sms < 4) return cudaErrorInvalidConfiguration;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(sms);
     cfg.blockDim = dim3(kFewThreads);
-    cfg.dynamicSmemBytes = Few<UNIT>::kSmemBytes;
+    cfg.dynamicSmemBytes = kFewSmemBytes;
     cfg.stream = stream;
     // blocks wait for tiles of other blocks: all of them have to be resident
     cudaLaunchAttribute at[1];
@@ -458,7 +556,7 @@ cudaError_t launch(const FewArgs& L, const RouteArgs& R, int num_sms, cudaStream
     at[0].val.cooperative = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, local_few_kernel<UNIT, ROUTES>, L, R);
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
 }  // namespace
@@ -491,10 +589,12 @@ cudaError_t local_few_launch(const LocalLayerParams& q, cudaStream_t stream) {
     L.done2 = q.ws + p.done2[0];
     L.stats = reinterpret_cast<unsigned long long*>(q.ws + p.stats[0]);
     L.status = q.status;
+    L.ran_unit = q.ws + p.meta + kMetaFewUnit;
     L.wanted = p.few == 2 ? q.ws + p.meta + kMetaFew : nullptr;
-    if (!p.routes) return p.few_unit == 64 ? launch<64, false>(L, {}, q.num_sms, stream) : launch<128, false>(L, {}, q.num_sms, stream);
-    const RouteArgs R = local_route_args(q);
-    return p.few_unit == 64 ? launch<64, true>(L, R, q.num_sms, stream) : launch<128, true>(L, R, q.num_sms, stream);
+    static bool configured[3][64] = {};
+    if (p.routes) return launch(local_few_routes_kernel, configured[0], q.num_sms, stream, L, local_route_args(q));
+    return p.few_unit == 64 ? launch(local_few_kernel<64>, configured[1], q.num_sms, stream, L)
+                            : launch(local_few_kernel<128>, configured[2], q.num_sms, stream, L);
 }
 
 }  // namespace tmoe

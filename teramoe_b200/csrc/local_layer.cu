@@ -1444,15 +1444,15 @@ LocalLayerPlan local_layer_plan(int T, int K, int E, int H, int I, int keep) {
     // I=256, 8 experts, top-4, 50 rows 39 / 29, H=1024 I=3072, 4, top-2, 32 rows 51 / 37, H=7168 I=768, 16, top-8, 64 rows 139 / 131).  With I >= 4096 it
     // stays at 16 rows: the rows of act that a tile reads are long there (H=1024 I=14336, 4 experts, 48 rows 138 / 131, 64 rows 139 / 149).
     // An expert of more rows than a unit takes its weights again for every unit.  The host cannot see one, but that it matters takes tokens and a
-    // large layer: if all T tokens chose the same K experts, K * (T / 64 - 1) units would read 6 H I bytes each.  Up to 128 tokens, or with up to 16 rows
-    // on average 96 MB, the kernel is ahead on any routing or close to it; us, general kernel / local_few.cu: 512 tokens on two experts, H=2048 I=512,
-    // 84 MB 49 / 41; H=7168, 128 tokens on two experts, I=2048 92 / 77, on four 122 / 114, on eight, I=1024 130 / 123, I=768 114 / 114, 96 tokens on
-    // eight, I=768 103 / 110, 128 tokens with 32 rows on average on eight of 32, I=768 102 / 112 (the worst that was found).  Beyond, the routing decides on
+    // large layer: if all T tokens chose the same K experts, K * (T / 64 - 1) units would read 6 H I bytes each.  Up to 128 tokens the kernel chooses units of 64 or 128
+    // rows by the routing (wide_units), and with up to 16 rows on average 96 MB are not much: there it is ahead on any routing or close to it.  us, general kernel /
+    // local_few.cu: 512 tokens on two experts, H=2048 I=512, 84 MB 49 / 41; H=7168, 128 tokens on two experts, I=2048 87 / 76, I=3072 93 / 96 (the only one of 120 spreads
+    // of 80 to 128 tokens, with one more, that was slower by more than 3 %: on eight, I=768 102 / 109, I=1024 117 / 118).  Beyond, the routing decides on
     // the GPU: both kernels are launched, and one returns at once, for 5 us (256 tokens, H=4096 I=768, 64 experts, top-4 268 / 215; all on two experts,
     // H=7168 I=2048 95 / 98).  Units beyond an expert's first may be 1 / few_again of the experts with rows: with 48 rows on average, hottest expert three
     // times the mean, H=7168 I=2048 524 / 512, with 64 543 / 560.
     const bool sixteen = entries <= 16l * E;
-    p.few_unit = entries <= 40l * E || T <= 64 ? 64 : 128;
+    p.few_unit = entries <= 40l * E ? 64 : 128;
     p.few_again = sixteen ? 1 : p.few_unit == 64 ? 3 : 8;
     const long again = (long)K * ((T + 63) / 64 - 1) * 6 * H * I, area = (long)I * E;
     const bool few = sixteen || (I < 4096 && (T <= 128 ? entries <= 80l * E : (entries <= 40l * E && 10 * entries <= area) || (entries <= 64l * E && 32 * entries <= area)));

@@ -11,7 +11,7 @@ namespace tmoe {
 constexpr int kLocalMaxExperts = 512;    // the routing kernels keep 23 words per expert in shared memory
 
 // words of the meta block
-enum { kMetaUnits = 0, kMetaSlots = 1, kMetaWork = 2, kMetaRows = 4, kMetaFew = 5, kMetaWords = 8 };
+enum { kMetaUnits = 0, kMetaSlots = 1, kMetaWork = 2, kMetaRows = 4, kMetaFew = 5, kMetaFewUnit = 6, kMetaWords = 8 };
 
 // Word offsets of the tables of one call inside its int32 workspace.  Capacities follow from the sizes alone (T * K entries in
 // at most min(E, T * K) segments padded to 128 rows), so the host never has to read the layout back.
@@ -19,7 +19,7 @@ struct LocalLayerPlan {
     int T, K, E, H, I, keep;             // keep: tables of the backward pass too
     int copies[2];                       // per direction: token rows are copied into slot order, not loaded by the slot table
     int few;                             // a forward with few rows per expert: 1 local_few.cu, 2 local_few.cu if the routing says so (kMetaFew)
-    int few_unit;                        // rows of an expert that it multiplies at a time: 64 or 128
+    int few_unit;                        // rows of an expert that it multiplies at a time: 64 or 128; with `routes` it chooses itself
     int few_again;                       // with few = 2: most units beyond an expert's first, as a share of the experts with rows: 1 / few_again
     int routes;                          // local_few.cu makes the routing tables itself: there is no routing kernel
     int halves;                          // units of one 128-row block are multiplied as 128 rows

@@ -265,6 +265,40 @@ def test_forward_with_up_to_eighty_rows_per_expert(counts, E, T, H, I, few, ran,
     buf.destroy()
 
 
+@pytest.mark.parametrize("counts,H,I,unit", [
+    ([128, 128, 127, 97, 96, 95, 66, 65], 4096, 1024, 128),      # one turn of 128-row tiles, two of 64-row tiles
+    ([128, 128, 127, 97, 96, 95, 66, 65], 4096, 512, 64),        # one turn of either
+    ([128, 128, 128, 128, 0, 0, 0, 0], 7168, 512, 64),           # neither fills one
+    ([128, 65, 64, 64, 33, 1, 0, 16], 4096, 1024, 64),           # few tiles more, and a large unit's steps
+    ([70, 70, 70, 70, 70, 70, 70, 70], 1024, 1024, 64),          # small weights
+])
+def test_units_of_up_to_128_tokens_follow_the_routing(counts, H, I, unit, monkeypatch):
+    """The kernel that routes by itself chooses the rows of a unit from the entries per expert."""
+    from teramoe_b200 import engine
+    from teramoe_b200._build import load_ext
+    T, K, E = 128, 8, 16
+    assert load_ext().local_layer_variant(T, K, E, H, I, False)["few"] == 1
+    gen = torch.Generator().manual_seed(2)
+    idx = torch.full((T, K), -1, dtype=torch.int64)
+    for e, n in enumerate(counts):
+        idx[torch.randperm(T, generator=gen)[:n], e] = 2 * e
+    prob = make_problem(1, T, H, I, E, K, seed=8, dtype=torch.bfloat16, device="cuda", x_scale=0.1, w_scale=0.02)
+    r = prob["ranks"][0]
+    idx = idx.cuda()
+    buf = tm.Buffer(None, int(64e6), explicitly_destroy=True)
+    call = lambda: buf.teramoe_forward(r["x"], idx, r["w"], prob["W_gateup"], prob["W_down"], E)
+    with monkeypatch.context() as m:
+        m.setattr(engine, "_LOCAL_LAYER_MODE", "0")
+        for name in ("_FUSED_DISPATCH_MODE", "_FUSED_MODE", "_LAYER_KERNEL_MODE"):
+            m.setattr(engine, name, "1")
+        want = call()
+    for _ in range(2):
+        assert torch.equal(call(), want)
+        assert buf._engine.native.ran_few() and buf._engine.native.few_unit() == unit
+    buf.check_status()
+    buf.destroy()
+
+
 @pytest.mark.parametrize("counts,H,I,few", [
     ([64] * 20 + [8] * 10, 4096, 1024, True),            # no second unit
     ([129] * 6 + [64] * 6, 4096, 1024, True),            # as many as experts with rows
