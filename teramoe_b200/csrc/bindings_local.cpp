@@ -2,6 +2,7 @@
 // allocations and launches instead of a Python pipeline.
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/CUDAEvent.h>
+#include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <pybind11/stl.h>
@@ -71,14 +72,20 @@ void use_tables(const c10::cuda::CUDAStream& writer, unsigned long long capture,
     now.block(stream);
 }
 
-// A tensor of its own over part of another one's memory, from byte `at` on.  An allocation costs the host about a microsecond, this a tenth of it: small
-// results and tables of one call lie in one block.
+// A tensor of its own over part of another one's memory, from byte `at` on.  An allocation costs the host about a microsecond, this a tenth of it: the
+// tables of one handle, and the counts of one layout, lie in one block.  It lives as long as any of them, is saved or shared with another process as a
+// whole, and resizing one of them would take its neighbour's memory: what a program keeps, saves or changes by itself has an allocation of its own.
 torch::Tensor piece(const torch::Tensor& block, int64_t at, at::IntArrayRef sizes, at::ScalarType type) {
     auto t = at::detail::make_tensor<c10::TensorImpl>(c10::Storage(block.storage()), c10::DispatchKeySet(c10::DispatchKey::CUDA),
                                                       c10::scalarTypeToTypeMeta(type));
     t.unsafeGetTensorImpl()->set_sizes_contiguous(sizes);
     t.unsafeGetTensorImpl()->set_storage_offset(at / (int64_t)c10::elementSize(type));
     return t;
+}
+
+// Memory that the kernels of this call write in full, past torch.empty's dispatcher (which adds to the host's time what the allocation itself takes)
+torch::Tensor written(at::IntArrayRef sizes, const torch::Tensor& like, at::ScalarType type) {
+    return torch::Tensor(at::detail::empty_cuda(sizes, type, like.device(), c10::nullopt));
 }
 
 // Where the next part of a block starts: on a boundary as an allocation has it.
@@ -122,10 +129,11 @@ ll_local_dispatch(torch::Tensor x, torch::Tensor topk_idx, int64_t M, int64_t E,
     auto recv = torch::empty({E, M, H}, on(x, wire > 0 ? torch::kFloat8_e4m3fn : torch::kBFloat16));
     c10::optional<torch::Tensor> scales;
     if (wire > 0) scales = wire == 3 ? torch::empty({E, G / 4, M}, on(x, torch::kInt32)) : torch::empty({E, G, M}, on(x, torch::kFloat32));
-    const int64_t at_count = behind(0, 8 * E), at_src = behind(at_count, 4 * E), at_entry = behind(at_src, 4 * E * M);
-    const auto block = torch::empty({at_entry + 4 * (int64_t)tk.T * tk.K}, on(x, torch::kUInt8));
-    const auto range = piece(block, 0, {E, 1}, torch::kInt64), count = piece(block, at_count, {E}, torch::kInt32);
-    const auto src_info = piece(block, at_src, {E, M}, torch::kInt32), entry = piece(block, at_entry, {tk.T, tk.K}, torch::kInt32);
+    const auto count = written({E}, x, torch::kInt32);          // (a program keeps it without the handle)
+    const int64_t at_src = behind(0, 8 * E), at_entry = behind(at_src, 4 * E * M);
+    const auto block = torch::empty({at_entry + 4 * (int64_t)tk.T * tk.K}, on(x, torch::kUInt8));      // (src_info is not written in full)
+    const auto range = piece(block, 0, {E, 1}, torch::kInt64), src_info = piece(block, at_src, {E, M}, torch::kInt32);
+    const auto entry = piece(block, at_entry, {tk.T, tk.K}, torch::kInt32);
     TM_CHECK_CUDA(tmoe::ll_local_dispatch(local_layout(E, M, H, (int)wire, false), x.data_ptr(), tk.ptr, tk.is64, tk.T, tk.K, recv.data_ptr(),
                                           scales.has_value() ? scales->data_ptr() : nullptr, src_info.data_ptr<int>(),
                                           reinterpret_cast<long long*>(range.data_ptr<int64_t>()), count.data_ptr<int>(), stats,
@@ -163,15 +171,15 @@ torch::Tensor ll_local_combine(torch::Tensor x, torch::Tensor topk_idx, torch::T
 
 // ------------------------------------------------------------------------------------------------ un-fused exchange
 struct Scratch {
-    torch::Tensor all;                       // int32: totals [E + 2], row_local [T], chunk_base, and [T] for whoever asks
+    torch::Tensor all;                       // int32: totals [E + 2], row_local [T], chunk_base, and, with `rows`, [T] more
     int *totals, *row_local, *chunk_base;
     int64_t extra;                           // byte of the last part
 };
-Scratch route_scratch(const torch::Tensor& idx, const TopK& tk, int64_t E) {
+Scratch route_scratch(const torch::Tensor& idx, const TopK& tk, int64_t E, bool rows) {
     const int64_t chunks = std::max<int64_t>(1, (tk.T + tmoe::kLocalChunk - 1) / tmoe::kLocalChunk);
     Scratch s;
     s.extra = behind(0, 4 * (E + 2 + tk.T + chunks));
-    s.all = torch::empty({s.extra / 4 + tk.T}, on(idx, torch::kInt32));
+    s.all = written({s.extra / 4 + (rows ? tk.T : 0)}, idx, torch::kInt32);
     s.totals = s.all.data_ptr<int>();
     s.row_local = s.totals + E + 2;
     s.chunk_base = s.row_local + tk.T;
@@ -187,8 +195,8 @@ std::tuple<torch::Tensor, torch::Tensor, torch::Tensor> local_counts(torch::Tens
     c10::cuda::CUDAGuard guard(topk_idx.device());
     topk_idx = topk_idx.contiguous();
     const TopK tk = topk_of(topk_idx);
-    const auto s = route_scratch(topk_idx, tk, E);
-    const auto in_rank = piece(s.all, s.extra, {tk.T, 1}, torch::kBool);
+    const auto s = route_scratch(topk_idx, tk, E, false);
+    const auto in_rank = written({tk.T, 1}, topk_idx, torch::kBool);
     TM_CHECK_CUDA(tmoe::local_route(tk.ptr, tk.is64, tk.T, tk.K, (int)E, s.totals, s.row_local, s.chunk_base,
                                     reinterpret_cast<uint8_t*>(in_rank.data_ptr<bool>()), nullptr, 0, cur_stream()));
     return {piece(s.all, 4 * E, {1}, torch::kInt32), piece(s.all, 0, {E}, torch::kInt32), in_rank};
@@ -270,7 +278,7 @@ class LocalExchange {
             const auto w = weights_of(topk_weights);
             TORCH_CHECK(w.is_cuda() && w.numel() == (int64_t)tk.T * tk.K, "topk_weights must have one weight per entry");
             TORCH_CHECK(!parts.empty() && parts.size() <= tmoe::kLocalMaxParts, "one or two payloads");
-            const auto s = route_scratch(topk_idx, tk, E);
+            const auto s = route_scratch(topk_idx, tk, E, true);
             const int64_t cap = worst_rows > 0 ? worst_rows : tk.T;
             std::vector<tmoe::LocalPart> lp;
             for (auto& p : parts) {

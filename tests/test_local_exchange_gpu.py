@@ -143,6 +143,23 @@ def test_results_of_a_call_do_not_overlap_and_start_as_allocations_do(T, E, K, M
     buf.destroy()
 
 
+def test_what_a_program_keeps_of_a_call_has_memory_of_its_own():
+    """The received counts and the ranks of the tokens hold no other result's memory, and taking more does not reach into one."""
+    T, E, K, M = 200, 16, 4, 256
+    idx, w = _routing(T, E, K, seed=3, dtype=torch.int64)
+    buf = tm.Buffer(None, tm.Buffer.get_low_latency_rdma_size_hint(M, 512, 1, E), low_latency_mode=True, explicitly_destroy=True)
+    x = torch.randn(T, 512, device="cuda").to(torch.bfloat16)
+    _, count, handle, _, _ = buf.low_latency_dispatch(x, idx, M, E)
+    per_rank, _, per_expert, in_rank, _ = buf.get_dispatch_layout(idx, E)
+    others = [handle.layout_range, handle.src_info, handle.entry_row, per_rank, per_expert]
+    before = [t.clone() for t in others]
+    for t in (count, in_rank):
+        assert t.untyped_storage().nbytes() == t.numel() * t.element_size()
+        t.resize_(1 << 16).fill_(1)
+    assert all(torch.equal(t, b) for t, b in zip(others, before))
+    buf.destroy()
+
+
 def _stall(stream, ms=40):
     with torch.cuda.stream(stream):
         torch.cuda._sleep(int(ms * 1.5e6))             # cycles
