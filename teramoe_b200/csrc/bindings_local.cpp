@@ -409,6 +409,12 @@ py::dict local_layer_variant(int64_t T, int64_t K, int64_t E, int64_t H, int64_t
     return d;
 }
 
+// columns per tile, for tests that are about wide ones: [direction][first GEMM, second GEMM, dW_down, dW_gateup]
+std::vector<std::vector<int>> local_layer_columns(int64_t T, int64_t K, int64_t E, int64_t H, int64_t I) {
+    const tmoe::LocalLayerPlan p = tmoe::local_layer_plan((int)T, (int)K, (int)E, (int)H, (int)I, 1);
+    return {{p.cols[0][0], p.cols[0][1]}, {std::begin(p.cols[1]), std::end(p.cols[1])}};
+}
+
 // whether units of one 128-row block are multiplied as 128 rows
 bool local_layer_halves(int64_t T, int64_t K, int64_t E, int64_t H, int64_t I) {
     return tmoe::local_layer_plan((int)T, (int)K, (int)E, (int)H, (int)I, 0).halves != 0;
@@ -738,6 +744,7 @@ void register_local(pybind11::module_& m) {
         .def("call", &local_layer_call);
     m.def("local_layer_variant", &local_layer_variant);
     m.def("local_layer_halves", &local_layer_halves);
+    m.def("local_layer_columns", &local_layer_columns);
     m.def("local_counts", &local_counts);
     m.def("local_scatter", &local_scatter);
     m.def("local_combine", &local_combine);

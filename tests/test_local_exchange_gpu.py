@@ -58,6 +58,24 @@ def test_low_latency_local_kernels_match_window_kernels(T, H, E, K, M, wire):
         assert torch.equal(a, b), f"output {i} differs"
 
 
+# top-k of 1 to 4: a block takes 8, 4 or 2 channel steps of 256; nine and ten of them leave a short last block behind full ones
+@pytest.mark.parametrize("T,H,E,K,M", [(5, 2304, 4, 1, 8), (6, 2304, 8, 2, 8), (7, 2560, 8, 3, 8), (77, 2304, 16, 4, 128), (3, 256, 8, 4, 4)])
+def test_logfmt_combine_of_few_entries_matches_window_kernels(T, H, E, K, M):
+    idx, w = _routing(T, E, K, seed=T)
+    x = torch.zeros(T, H, dtype=torch.bfloat16, device="cuda")
+    y = (torch.randn(E, M, H, generator=torch.Generator().manual_seed(H)) * 0.2).to(torch.bfloat16).cuda()
+    y[:, :, :128] *= 8.0                    # groups that LogFMT leaves as they are
+    got = []
+    for shrink in (False, True):            # local kernels, window kernels
+        buf = tm.Buffer(None, 0, low_latency_mode=True, explicitly_destroy=True, enable_shrink=shrink)
+        handle = buf.low_latency_dispatch(x, idx, M, E, use_fp8=False)[2]
+        assert (handle.entry_row is None) == shrink
+        got.append(buf.low_latency_combine(y, idx, w, handle, use_logfmt=True)[0].clone())
+        buf.check_status()
+        buf.destroy()
+    assert torch.equal(*got) and bool(got[0].any())
+
+
 # chunks of 128 tokens: one, a full one, one more token, several; rows of 2 KB segments: a short one, several, odd byte counts (fp8 scales)
 @pytest.mark.parametrize("T,H,E,K", [(0, 256, 4, 2), (1, 128, 4, 1), (128, 1024, 8, 4), (129, 1032, 300, 8), (1003, 7168, 32, 8), (1024, 128, 40, 8), (1025, 128, 40, 8),
                                       (5000, 256, 40, 32)])

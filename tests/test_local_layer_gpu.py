@@ -130,6 +130,29 @@ def test_last_units_of_experts(counts, H, I, halves, monkeypatch):
     buf.destroy()
 
 
+def test_last_units_of_experts_with_wide_tiles(monkeypatch):
+    """Half units where every GEMM takes 512-column tiles (1344 = 2 * 512 + 320: a last one and a quarter): 1, 64, 65 and 128 rows in the last block."""
+    from teramoe_b200 import engine
+    from teramoe_b200._build import load_ext
+    H, I, counts = 2048, 1344, [3840 + r for r in (1, 64, 65, 128, 0, 63, 96, 127, 1, 32, 33, 128)] + [2, 7700]
+    E, T = len(counts), sum(counts)
+    assert load_ext().local_layer_halves(T, 1, E, H, I) and load_ext().local_layer_columns(T, 1, E, H, I) == [[512] * 2, [512] * 4]
+    prob = make_problem(1, T, H, I, E, 1, seed=3, dtype=torch.bfloat16, device="cuda", x_scale=0.1, w_scale=0.02)
+    order = torch.randperm(T, generator=torch.Generator().manual_seed(1))
+    idx = torch.repeat_interleave(torch.arange(E), torch.tensor(counts))[order].view(T, 1).to(prob["ranks"][0]["idx"])
+    buf = tm.Buffer(None, int(64e6), explicitly_destroy=True)
+    res = {}
+    for mode in ("0", "auto"):
+        monkeypatch.setattr(engine, "_LOCAL_LAYER_MODE", mode)
+        for name in ("_FUSED_DISPATCH_MODE", "_FUSED_MODE", "_LAYER_KERNEL_MODE"):
+            monkeypatch.setattr(engine, name, "1" if mode == "0" else "auto")
+        res[mode] = _run(buf, prob, idx, E)
+    for name, got in res["auto"].items():
+        assert torch.equal(got, res["0"][name]), f"{name}: differs from the general kernels"
+    buf.check_status()
+    buf.destroy()
+
+
 @pytest.mark.parametrize("batch", [1024, 2048, 4096])
 def test_batches_end_where_experts_do(batch, monkeypatch):
     """Experts of 9, 4, 1, 0, 2, 8, 3, 5 and 1 units of 256 rows in nominal batches of 4, 8 and 16: ends that move to an expert's, that stay inside
@@ -227,6 +250,30 @@ def test_forward_with_few_rows_per_expert(counts, empty, H, I, K, monkeypatch):
     for got, want in zip(res["auto"], res["0"]):
         assert torch.equal(got, want)
     assert bool(res["auto"][0].any()) and not bool(res["auto"][2].any())
+    buf.check_status()
+    buf.destroy()
+
+
+@pytest.mark.parametrize("T,K,E,total_sms", [(700, 2, 100, 6), (4096, 1, 256, 8)])
+def test_few_rows_kernel_routes_on_a_grid_smaller_than_the_routing(T, K, E, total_sms, monkeypatch):
+    """Eleven and twenty-four shares of the routing on six and eight blocks: each takes several, one after the other; tokens without an expert."""
+    from teramoe_b200 import engine
+    from teramoe_b200._build import load_ext
+    H, I = 192, 128
+    assert load_ext().local_layer_variant(T, K, E, H, I, False)["few"] == 1
+    prob = make_problem(1, T, H, I, E, K, seed=T, dtype=torch.bfloat16, device="cuda", x_scale=0.1, w_scale=0.02)
+    r = prob["ranks"][0]
+    idx = r["idx"].clone()
+    idx[5::7] = -1
+    buf = tm.Buffer(None, int(64e6), explicitly_destroy=True)
+    call = lambda **kw: buf.teramoe_forward(r["x"], idx, r["w"], prob["W_gateup"], prob["W_down"], E, **kw)
+    with monkeypatch.context() as m:
+        m.setattr(engine, "_LOCAL_LAYER_MODE", "0")
+        for name in ("_FUSED_DISPATCH_MODE", "_FUSED_MODE", "_LAYER_KERNEL_MODE"):
+            m.setattr(engine, name, "1")
+        want = call()
+    for kw in (dict(total_sms=total_sms, num_dispatch_sms=2, num_combine_sms=2), {}):
+        assert torch.equal(call(**kw), want) and buf._engine.native.ran_few()
     buf.check_status()
     buf.destroy()
 
