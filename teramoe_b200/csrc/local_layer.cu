@@ -1478,7 +1478,11 @@ LocalLayerPlan local_layer_plan(int T, int K, int E, int H, int I, int keep) {
     // 736 / 680, 275 1209 / 1129, 325 1187 / 1222, 525 1645 / 1754, 750 1973 / 2026, H=4096 I=1536, 16, top-2 312 307 / 289; steps: 16 1829 / 1715, 64 1972 /
     // 1834, 275 3466 / 3367, 2048 14940 / 15192, H=4096 I=14336, 8, top-2 375 3762 / 3925, H=2048 I=768, 16, top-4 325 284 / 277, H=2048 I=2048, 16, top-8 2048
     // 2277 / 2262, H=2048 I=3072, 16, top-6 3072 5169 / 5136.  Where an expert has whole units besides, a half one runs ahead of them through the weights that
-    // they share, and on a long K what it has fetched is gone from L2 before they come: hence only few rows, or short tiles.
+    // they share, and on a long K what it has fetched is gone from L2 before they come: with H=7168 they gain up to 300 rows only.  The other line, H=2048 I=3072, is
+    // where the first measurements ended, on the safe side: what lies beyond gains 1 to 9 % more up to about 1000 rows and -1 to 2 % at 1800 (forward, 312 / 550 / 800 rows:
+    // H=2048 I=4096 376 / 341, 517 / 491, 678 / 650; H=3072 I=3072 421 / 399, 587 / 559, 739 / 716; H=4096 I=3072 563 / 519, 759 / 748, 944 / 943).
+    // The average decides, whatever the routing: with 275 rows on average that all go to 8, 16 or unevenly (Zipf, 1.0) to 32 of 32 experts, H=7168 I=2048, forwards
+    // take 780 / 755, 938 / 896, 1047 / 998, steps 2646 / 2623, 2932 / 2838, 3195 / 3107; by every expert's own rows instead it would be 774, 941, 1016 and 2626, 2943, 3130.
     p.halves = entries <= 300l * E || (H <= 2048 && I <= 3072);
     const bool large_i = I >= 4096;
     p.copies[0] = large_i && p.few != 1;          // (local_few.cu gathers rows from x itself)
@@ -1527,7 +1531,6 @@ LocalLayerPlan local_layer_plan(int T, int K, int E, int H, int I, int keep) {
     }
     p.zero_words = at;
     p.meta = take(kMetaWords);
-    p.seg = take(E + 1);
     p.counts = take(E);
     p.slot_tk = take(p.slots_cap);
     p.slot_w = take(p.slots_cap);

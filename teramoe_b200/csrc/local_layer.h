@@ -1,5 +1,5 @@
 // The MoE layer on one rank (local_layer.cu): routing preparation in one launch or two (by the number of entries), then ONE cooperative persistent kernel per
-// direction; a forward with few rows per expert has its own (local_few.cu).  Every sum has the terms and the order that it has in the kernel
+// direction; a forward with few rows per expert has its own (local_few.cu), which with up to 4096 entries prepares the routing itself.  Every sum has the terms and the order that it has in the kernel
 // for several ranks (layer.h), so both give the same bits; what differs is where batches of the work list end, slices of K that are
 // all padding, and everything that only a second rank needs (peer tables, completion flags, landing rows).
 #pragma once
@@ -27,10 +27,10 @@ struct LocalLayerPlan {
     int slots_cap, blocks_cap, units_cap;
     int work_cap[2];                     // items of the forward / backward list
     int cols[2][4];                      // columns per tile: [direction][first GEMM, second GEMM, dW_down, dW_gateup]
-    // zero-filled by local_layer_route
+    // zero-filled by local_layer_route, or with `routes` by local_few.cu
     long stats[2], sync[2], done1[2], done2[2], arrived[2], zero_words;
-    // written by it
-    long meta, seg, counts, slot_tk, slot_w, token_order, order_slot, chunk_hist, chunk_last, work[2], words;
+    // written by the same
+    long meta, counts, slot_tk, slot_w, token_order, order_slot, chunk_hist, chunk_last, work[2], words;
 };
 LocalLayerPlan local_layer_plan(int T, int K, int E, int H, int I, int keep);
 

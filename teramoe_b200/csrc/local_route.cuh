@@ -28,7 +28,8 @@ __device__ __forceinline__ void load_experts(const void* idx, int is64, long t, 
 // assign: every block adds up all chunk histograms, which gives it the segment table and its own bases, so no block waits for
 // another and no scan kernel sits in between.  With few entries (kDirectEntries) every block counts all of them itself and
 // clears a share of the counters: one launch instead of two.  us on the GPU, one launch / two with the gap between them (32 experts, top-8), by
-// entries: 1024 6.1 / 10.8, 4096 8.8 / 12.9, 8192 10.6 / 13.3, 24008 17.2 / 14.2.
+// entries: 1024 6.1 / 10.8, 4096 8.8 / 12.9, 8192 10.6 / 13.3, 24008 17.2 / 14.2.  (So one launch is ahead up to 12 thousand or so; the
+// line stands where the test of a call's launches has it.)
 // What bounds them is a chain of latencies, so a chunk's slots and the work lists are written by different blocks, a token's indices and weights
 // are requested together before anything else, and what follows from the schedule alone is computed on the host.  Before (one block after the
 // other, an index and a weight at a time behind a match.any of 550 to 700 cycles, 64-bit divisions), assign, us, forward / with backward's lists:
@@ -194,9 +195,9 @@ __device__ __forceinline__ void route_assign(const RouteArgs& a, int* sh, int (&
         if (lane == 0) {
             seg[E] = run_s;
             ub[E] = run_u;
-            // Units beyond an expert's first, each of which takes its weights again, from L2: as many as experts with rows at most.  us, general
-            // kernel / local_few.cu (64 experts, top-4, H=7168 I=768, all tokens on four experts): 128 tokens, one such unit per expert, 88 / 76,
-            // 256 tokens, three, 95 / 115.
+            // Units beyond an expert's first, each of which takes its weights again, from L2: 1 / few_again of the experts with rows at most.  (As many of units of 64
+            // rows with up to 16 rows on average.  us, general kernel / local_few.cu, 64 experts, top-4, H=7168 I=768, all tokens on four experts, where every call of 128
+            // and of 256 tokens has one and three per expert: 88 / 76, 95 / 115.  The other shares: local_layer_plan.)
             *few_word = a.p.few == 1 || (a.p.few == 2 && (few_units - hit) * a.p.few_again <= hit);
         }
     }
@@ -222,7 +223,6 @@ __device__ __forceinline__ void route_assign(const RouteArgs& a, int* sh, int (&
         const int helper = block - a.p.chunks, helpers = blocks - a.p.chunks;
         // ---- tables
         if (helper == 0) {
-            for (int e = tid; e <= E; e += kRouteThreads) a.ws[a.p.seg + e] = seg[e];
             for (int e = tid; e < E; e += kRouteThreads) a.ws[a.p.counts + e] = totals[e];
             if (tid == 0) {
                 meta[kMetaUnits] = U;
