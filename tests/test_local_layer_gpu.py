@@ -320,7 +320,7 @@ def test_forward_with_up_to_eighty_rows_per_expert(counts, E, T, H, I, few, ran,
     ([70, 70, 70, 70, 70, 70, 70, 70], 1024, 1024, 64),          # small weights
 ])
 def test_units_of_up_to_128_tokens_follow_the_routing(counts, H, I, unit, monkeypatch):
-    """The kernel that routes by itself chooses the rows of a unit from the entries per expert."""
+    """The kernel that routes by itself chooses the rows of a unit from the entries per expert, also when a captured call is replayed with other ones."""
     from teramoe_b200 import engine
     from teramoe_b200._build import load_ext
     T, K, E = 128, 8, 16
@@ -331,17 +331,25 @@ def test_units_of_up_to_128_tokens_follow_the_routing(counts, H, I, unit, monkey
         idx[torch.randperm(T, generator=gen)[:n], e] = 2 * e
     prob = make_problem(1, T, H, I, E, K, seed=8, dtype=torch.bfloat16, device="cuda", x_scale=0.1, w_scale=0.02)
     r = prob["ranks"][0]
-    idx = idx.cuda()
+    idx, even = idx.cuda(), (torch.arange(T * K, device="cuda") % E).view(T, K)      # even: 64 rows per expert
     buf = tm.Buffer(None, int(64e6), explicitly_destroy=True)
-    call = lambda: buf.teramoe_forward(r["x"], idx, r["w"], prob["W_gateup"], prob["W_down"], E)
+    call = lambda i: buf.teramoe_forward(r["x"], i, r["w"], prob["W_gateup"], prob["W_down"], E)
     with monkeypatch.context() as m:
         m.setattr(engine, "_LOCAL_LAYER_MODE", "0")
         for name in ("_FUSED_DISPATCH_MODE", "_FUSED_MODE", "_LAYER_KERNEL_MODE"):
             m.setattr(engine, name, "1")
-        want = call()
+        want, want_even = call(idx), call(even)
     for _ in range(2):
-        assert torch.equal(call(), want)
+        assert torch.equal(call(idx), want)
         assert buf._engine.native.ran_few() and buf._engine.native.few_unit() == unit
+    static = even.clone()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = call(static)
+    for i, ref, rows in ((idx, want, unit), (even, want_even, 64), (idx, want, unit)):
+        static.copy_(i)
+        graph.replay()
+        assert torch.equal(out, ref) and buf._engine.native.few_unit() == rows
     buf.check_status()
     buf.destroy()
 
